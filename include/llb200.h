@@ -22,7 +22,7 @@
 extern "C" {
 #endif
 
-#define LL_ABI_VERSION 17
+#define LL_ABI_VERSION 18
 
 #define LL_OK 0
 #define LL_ERR_ARG (-1)         /* bad shape / dtype / null pointer */
@@ -411,6 +411,23 @@ LL_API int ll_latent_attn_terms(const void* q_lat, long long qs_h, long long qs_
                                 const void* cache, void* out, long long os_h, long long os_m, int dtype, int B, int T, int n_head,
                                 int kv_rank, int rot_dim, int rot_dims, int cache_len, int window, float scale, int splits,
                                 int weight_terms, float* scratch, ll_stream stream);
+/* Prompts in bf16 on tcgen05 with the rows expanded per head: k_nope (slot r, head h) at k_nope[(b * cache_len + r) * k_row + h * k_head],
+ * v alike, both products of the cache rows with the up-projections; the rotated key part is read from the cache rows.  q: row m at
+ * m * q_stride, head h's [nope | rot_dim] at h * q_head_stride, the rotary part not yet rotated (its rotated copy goes to q_rot
+ * [B*T][n_head][rot_dim]).  gate: null, or one logit per head at gate[m * gate_stride + h].
+ *   y[m * y_stride + h * v_dim + i] = sigmoid(gate) * sum_j softmax_j((q_nope . k_nope_j + rot(q_rot) . k_rot_j) * scale) v_j[i]
+ * Slots that hold no position of the sequence may hold anything, in the cache and in the expanded rows.  weight_terms as above.
+ * ll_latent_prompt_supported: sizes and strides the form takes (operands on 16-byte boundaries besides). */
+LL_API int ll_latent_prompt_supported(int nope, int rot_dim, int v_dim, int kv_rank, int q_stride, int q_head_stride, int y_stride);
+LL_API int ll_latent_prompt_attn(const void* q, int q_stride, int nope, int q_head_stride, const void* gate, int gate_stride,
+                                 const float* rope, const int32_t* pos_ids, const void* k_nope, long long k_row, long long k_head,
+                                 const void* v, long long v_row, long long v_head, const void* cache, void* q_rot, void* y, int y_stride,
+                                 int B, int T, int n_head, int kv_rank, int rot_dim, int rot_dims, int v_dim, int cache_len, int window,
+                                 float scale, int weight_terms, ll_stream stream);
+/* 0, or the code of the first bounded wait that ran out in the tcgen05 attention kernel (csrc/attn_tc.cuh) as launched by
+ * ll_latent_prompt_attn / ll_softmax_attn*.  Both synchronise the device. */
+LL_API int ll_latent_prompt_error(void);
+LL_API int ll_softmax_attn_tc_error(void);
 LL_API size_t ll_latent_attn_scratch_bytes(int M, int n_head, int kv_rank, int splits);
 
 /* ---------------------------------------------------------------------------------------

@@ -11,6 +11,7 @@
 // Rotation pairs dimension 2i with 2i+1 (interleaved) on the first rot_dims dimensions of the rotated
 // part; the (cos, sin) table is [positions][rot_dims / 2][2] fp32.  Scores, softmax weights and sums
 // are fp32; T is the dtype of activations and of the cache.
+#include "attn_tc.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -577,6 +578,32 @@ static int latent_attn_heads_per_block(int H, int KR, int Dk) {
   return hg;
 }
 
+// Rotated query parts of a prompt, [M][H][rot_dim]: eight numbers (four pairs) per thread.
+__global__ void latent_rotate_q_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, int col0, int q_head_stride,
+                                       const float* __restrict__ rope, const int32_t* __restrict__ pos_ids, __nv_bfloat16* __restrict__ out,
+                                       int Tn, int H, int rot_dim, int rot_dims, long long pieces) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pieces) return;
+  const int per = rot_dim / 8, d0 = (int)(i % per) * 8;
+  const long long mh = i / per;
+  const int h = (int)(mh % H);
+  const long long m = mh / H;
+  const uint4 u = *reinterpret_cast<const uint4*>(q + m * q_stride + col0 + (long long)h * q_head_stride + d0);
+  const float* cs = rope + (size_t)pos_ids[m % Tn] * rot_dims;         // [rot_dims / 2][2]
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float a = bf16_bits_to_f32(w[e] & 0xffffu), b = bf16_bits_to_f32(w[e] >> 16);
+    o[e] = w[e];
+    if (d0 + 2 * e < rot_dims) {
+      const float c = cs[d0 + 2 * e], s = cs[d0 + 2 * e + 1];
+      o[e] = pack_bf16(a * c - b * s, b * c + a * s);
+    }
+  }
+  *reinterpret_cast<uint4*>(out + mh * rot_dim + d0) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 }  // namespace llb
 
 using namespace llb;
@@ -696,5 +723,41 @@ int ll_latent_attn_terms(const void* q_lat, long long qs_h, long long qs_m, cons
   }
   return LL_OK;
 }
+
+int ll_latent_prompt_supported(int nope, int rot_dim, int v_dim, int kv_rank, int q_stride, int q_head_stride, int y_stride) {
+  return nope > 0 && nope % 8 == 0 && nope <= 128 && rot_dim > 0 && rot_dim % 8 == 0 && rot_dim <= 64 && v_dim > 0 && v_dim % 8 == 0 &&
+         v_dim <= 128 && kv_rank > 0 && kv_rank % 8 == 0 && q_stride % 8 == 0 && q_head_stride % 8 == 0 && y_stride % 8 == 0;
+}
+
+int ll_latent_prompt_attn(const void* q, int q_stride, int nope, int q_head_stride, const void* gate, int gate_stride, const float* rope,
+                          const int32_t* pos_ids, const void* k_nope, long long k_row, long long k_head, const void* v, long long v_row,
+                          long long v_head, const void* cache, void* q_rot, void* y, int y_stride, int B, int T, int n_head, int kv_rank,
+                          int rot_dim, int rot_dims, int v_dim, int cache_len, int window, float scale, int weight_terms, ll_stream stream) {
+  LL_CHECK_ARG(q && rope && pos_ids && k_nope && v && cache && q_rot && y, "latent_prompt_attn: null pointer");
+  LL_CHECK_ARG(B > 0 && T > 0 && n_head > 0 && cache_len > 0 && rot_dims >= 0 && rot_dims <= rot_dim && rot_dims % 2 == 0 && scale > 0.f &&
+                   ll_latent_prompt_supported(nope, rot_dim, v_dim, kv_rank, q_stride, q_head_stride, y_stride),
+               "bad latent_prompt_attn arguments");
+  const int row = kv_rank + rot_dim;
+  AttnTcArgs a{};
+  a.q = {q, nope, q_head_stride, q_stride, (long long)T * q_stride};
+  a.q2 = {q_rot, rot_dim, rot_dim, (long long)n_head * rot_dim, (long long)T * n_head * rot_dim};
+  a.k = {k_nope, nope, k_head, k_row, (long long)cache_len * k_row};
+  a.k2 = {(const __nv_bfloat16*)cache + kv_rank, rot_dim, row, row, (long long)cache_len * row};
+  a.v = {v, v_dim, v_head, v_row, (long long)cache_len * v_row};
+  a.pos_ids = pos_ids;
+  a.gate = gate, a.gate_ld = gate_stride, a.gate_per_head = 1;
+  a.scale = scale;
+  a.B = B, a.T = T, a.H = n_head, a.G = n_head, a.window = window > 0 ? window : 0, a.ring = cache_len;
+  a.terms = weight_terms;
+  a.y = y, a.y_ld = y_stride;
+  LL_CHECK_ARG(attn_tc_supported(a), "latent_prompt_attn: operands must start on 16-byte boundaries");
+  const long long pieces = (long long)B * T * n_head * (rot_dim / 8);
+  latent_rotate_q_kernel<<<(unsigned)((pieces + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)q, q_stride, nope, q_head_stride, rope, pos_ids, (__nv_bfloat16*)q_rot, T, n_head, rot_dim, rot_dims, pieces);
+  LL_LAUNCH_OK("latent_rotate_q_kernel");
+  return attn_tc_launch<AT_LATENT>(a, (cudaStream_t)stream);
+}
+
+int ll_latent_prompt_error(void) { return attn_tc_error(); }
 
 }  // extern "C"

@@ -18,6 +18,7 @@
 //             likewise, and every map is a softmax attention of its own over the SAME value row of head g.  Two maps are
 //             combined as a difference, o = a_0 - lambda * a_1, then divided by the root mean square of o over the head's
 //             values (eps inside the root) and multiplied by `post`; the gate, if any, follows.
+#include "attn_tc.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -883,6 +884,14 @@ int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, int gate
       y_stride % 2 == 0) {
     const int d = dim > vdim ? dim : vdim;
     if (maps == 1) {           // one map: key and value rows padded alike
+      AttnTcArgs a{};
+      a.q = {q, dim, dim, q_stride, (long long)T * q_stride};
+      a.k = {kc, dim, dim, (long long)G * dim, (long long)ring * G * dim};
+      a.v = {vc, vdim, vdim, (long long)G * vdim, (long long)ring * G * vdim};
+      a.pos_ids = pos_ids, a.sink = sink, a.slopes = slopes, a.gate = gate, a.gate_ld = gate_stride;
+      a.scale = scale, a.softcap = softcap, a.B = B, a.T = T, a.H = H, a.G = G, a.window = window, a.chunk = chunk, a.ring = ring;
+      a.terms = 2, a.y = y, a.y_ld = y_stride;
+      if (attn_tc_supported(a)) return attn_tc_launch<AT_ROTARY>(a, st);
 #define LL_TM_B(DD, BB)                                                                                                               \
   tm_launch<DD, DD, 1, BB>(q, q_stride, gate, gate_stride, kc, vc, pos_ids, sink, slopes, scale, softcap, B, T, H, G, dim, vdim, window, \
                            chunk, ring, dm, y, y_stride, st)
@@ -934,5 +943,7 @@ int ll_softmax_attn(const void* q, int q_stride, const void* gate, int gate_stri
   return ll_softmax_attn_maps(q, q_stride, gate, gate_stride, kc, vc, dtype, pos_ids, sink, scale, softcap, B, T, H, G, dim, vdim,
                               window, chunk, ring, splits, form, 1, 0.f, 1.f, 0.f, scratch, y, stream);
 }
+
+int ll_softmax_attn_tc_error(void) { return attn_tc_error(); }
 
 }  // extern "C"

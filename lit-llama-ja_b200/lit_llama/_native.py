@@ -114,6 +114,11 @@ EXPORTS = {
     "ll_glu_unit_rows": ([vp, i32, i32, vp, C.c_float, C.c_float, C.c_float, vp, i32, i32, i32, vp], C.c_int),
     "ll_latent_attn_terms": ([vp, i64, i64, vp, i32, i32, i32, i32, vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, i32, i32, i32,
                               i32, C.c_float, i32, i32, vp, vp], C.c_int),
+    "ll_latent_prompt_supported": ([i32, i32, i32, i32, i32, i32, i32], C.c_int),
+    "ll_latent_prompt_attn": ([vp, i32, i32, i32, vp, i32, vp, vp, vp, i64, i64, vp, i64, i64, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32,
+                               i32, i32, C.c_float, i32, vp], C.c_int),
+    "ll_latent_prompt_error": ([], C.c_int),
+    "ll_softmax_attn_tc_error": ([], C.c_int),
     "ll_latent_kv_append": ([vp, i32, i32, i32, vp, C.c_float, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_latent_attn": ([vp, i64, i64, vp, i32, i32, i32, i32, vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, i32, i32, i32,
                         i32, C.c_float, i32, vp, vp], C.c_int),
@@ -178,7 +183,7 @@ EXPORTS = {
 }
 _fn = {name: _proto(name, a, r) for name, (a, r) in EXPORTS.items()}
 
-ABI_VERSION = 17
+ABI_VERSION = 18
 if _fn["ll_abi_version"]() != ABI_VERSION:
     raise ImportError("libllb200.so ABI version mismatch; rebuild with lit-llama-ja_b200/build.py")
 
