@@ -156,6 +156,17 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
   return r;
 }
 
+// One lane of the warp, the same one every time.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)::"memory");
+  return r != 0;
+}
+
 // A wait that ends: on its phase, when another role has given up, or after the limit.
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
   for (uint32_t i = 0; i < AT_WAIT_LIMIT; ++i) {
@@ -164,6 +175,18 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
   }
   *fail = 1;
   atomicCAS(&g_attn_tc_error, 0, code);
+  return false;
+}
+
+// The same for a whole warp, which leaves together.  The MMA warp's control flow and operands have to be uniform in the compiler's
+// eyes (votes, shuffles): from a divergent branch an MMA costs its thread about 100 clocks to issue, more than it takes to run.
+__device__ __forceinline__ bool at_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+  for (uint32_t i = 0; i < AT_WAIT_LIMIT; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if ((i & 255u) == 255u && __any_sync(0xffffffffu, *fail != 0)) return false;
+  }
+  *fail = 1;
+  if (elect_one()) atomicCAS(&g_attn_tc_error, 0, code);
   return false;
 }
 
@@ -223,13 +246,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   uint64_t* v_empty = v_full + VS;
   uint64_t* s_full = v_empty + VS;                    // [tile][buffer] scores are there
   uint64_t* p_full = s_full + 4;                      // [tile][buffer] weights are there
-  uint64_t* o_full = p_full + 4;                      // [tile] P V is done
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t* o_full = p_full + 4;                      // [tile][buffer] P V is done
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_full + 4);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
   int* s_range = s_fail + 1;                          // per tile: smallest and largest position
   float* s_x = reinterpret_cast<float*>(s_range + 4); // [tile][half][row]: what the two threads of a row tell one another
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // the last queries see the most keys: they go first, so that the long blocks do not end up as the tail
   const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * AT_Q, h = blockIdx.y, b = blockIdx.z, g = h / p.group;
 
@@ -240,9 +263,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     mbar_init(q_full, 1);
     for (int i = 0; i < KS; ++i) mbar_init(&k_full[i], 1), mbar_init(&k_empty[i], 1);
     for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 1);
-    for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1), mbar_init(&p_full[i], AT_WARPS / 2);
+    for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1), mbar_init(&p_full[i], AT_WARPS / 2), mbar_init(&o_full[i], 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&o_full[i], 1);
       s_range[2 * i] = INT_MAX;
       s_range[2 * i + 1] = -1;
     }
@@ -253,7 +275,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_ptr;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   // positions of the tiles' queries
   const int tile = warp >> 3, half = (warp >> 2) & 1, row = (int)(threadIdx.x & (AT_Q - 1)), t = t0 + tile * AT_Q + row;
   int qp = 0;
@@ -264,13 +286,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   }
   __syncthreads();
   // what every role walks: key blocks from kt0 to the last visible key; per tile the part of it that its rows see
-  const int step_last = p.slots ? p.ring - 1 : p.pos_ids[p.T - 1];     // rows after this key hold nothing of this step
+  const int step_last = p.slots ? p.ring - 1 : __shfl_sync(0xffffffffu, p.pos_ids[p.T - 1], 0);     // rows after this key hold nothing of this step
   int lo[2], hi[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
-    const bool any = s_range[2 * i + 1] >= 0;
-    lo[i] = any ? at_first_visible(s_range[2 * i], p.window, p.chunk) : INT_MAX;
-    hi[i] = any ? (p.slots ? min(s_range[2 * i + 1], p.ring - 1) : s_range[2 * i + 1]) : -1;
+    const int first = __shfl_sync(0xffffffffu, s_range[2 * i], 0), end = __shfl_sync(0xffffffffu, s_range[2 * i + 1], 0);
+    lo[i] = end >= 0 ? at_first_visible(first, p.window, p.chunk) : INT_MAX;
+    hi[i] = end >= 0 && p.slots ? min(end, p.ring - 1) : end;
   }
   const int kt0 = min(lo[0], lo[1]), last = max(hi[0], hi[1]);
 
@@ -308,12 +330,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     // an MMA issued before
     auto scores = [&](int n, int kt, int rows) {
       const int ks = n % KS;
-      if (!at_wait(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
+      if (!at_wait_warp(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
       tc_fence_after();
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         if (kt + rows - 1 < lo[i] || kt > hi[i]) continue;
-        if (lane == 0) {
+        if (elect_one()) {
           const uint32_t d = tmem + TM_S + 128u * i + 64u * (ns[i] & 1u);
 #pragma unroll
           for (int c = 0; c < NB; ++c) {
@@ -326,10 +348,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         }
         ++ns[i];
       }
-      if (lane == 0) umma_commit(&k_empty[ks]);
+      if (elect_one()) umma_commit(&k_empty[ks]);
       return true;
     };
-    bool ok = at_wait(q_full, 0, s_fail, 3);
+    bool ok = at_wait_warp(q_full, 0, s_fail, 3);
     int rows = at_rows(kt0, last, p.ring);
     if (ok) ok = scores(0, kt0, rows);
     int n = 0;
@@ -337,7 +359,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       const int nkt = kt + rows, nrows = nkt <= last ? at_rows(nkt, last, p.ring) : 0;
       if (nkt <= last && !(ok = scores(n + 1, nkt, nrows))) break;
       const int vs = n % VS;
-      if (!(ok = at_wait(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
+      if (!(ok = at_wait_warp(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
       const int keep = step_last - kt + 1;                      // value rows from here on belong to no key of this step
       if (keep < AT_K) {
         const int pieces = (AT_K - keep) * 8;
@@ -352,9 +374,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       for (int i = 0; i < 2; ++i) {
         if (!ok || kt + rows - 1 < lo[i] || kt > hi[i]) continue;
         const uint32_t buf = np[i] & 1u;
-        if (!(ok = at_wait(&p_full[2 * i + (int)buf], (np[i] >> 1) & 1u, s_fail, 6))) continue;
+        if (!(ok = at_wait_warp(&p_full[2 * i + (int)buf], (np[i] >> 1) & 1u, s_fail, 6))) continue;
         tc_fence_after();
-        if (lane == 0) {
+        if (elect_one()) {
           const uint64_t vdesc = smem_desc_mn_sw128(smem_u32(sv + vs * NBV * AT_KBOX));
 #pragma unroll
           for (int term = 0; term < TERMS; ++term)
@@ -362,12 +384,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             for (int k = 0; k < AT_K / UMMA_K; ++k)            // 16 keys: 8 columns of packed weights, two groups of eight rows
               umma_ts(tmem + TM_O + 128u * i, tmem + TM_S + 128u * i + 64u * buf + 32u * term + 8u * k, vdesc + (uint64_t)(128 * k), idesc_o,
                       (np[i] != 0u || (term | k) != 0) ? 1u : 0u);
-          umma_commit(&o_full[i]);
+          umma_commit(&o_full[2 * i + (int)buf]);
         }
         ++np[i];
       }
       if (!ok) break;
-      if (lane == 0) umma_commit(&v_empty[vs]);
+      if (elect_one()) umma_commit(&v_empty[vs]);
       kt = nkt;
       rows = nrows;
     }
@@ -440,7 +462,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           ref = nref;
           sum2[0] = f2_mul(sum2[0], f2_of(f, f));
           sum2[1] = f2_mul(sum2[1], f2_of(f, f));
-          if (n > 0) ok = at_wait(&o_full[tile], (n - 1u) & 1u, s_fail, 8);
+          if (n > 0) ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, 8);
           __syncwarp();
           tc_fence_after();
           if (at_any(1 + tile, !ok)) {                                      // (also: both threads of a row have read the other's)
@@ -517,8 +539,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       kt += rows;
     }
     if (ok && n > 0 && t0 + tile * AT_Q < p.T) {
-      // the last scores came after P V of two blocks before was issued: one phase may be open before the last one
-      ok = (n < 2u || at_wait(&o_full[tile], (n - 2u) & 1u, s_fail, 9)) && at_wait(&o_full[tile], (n - 1u) & 1u, s_fail, 9);
+      ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, 9);
       __syncwarp();
       tc_fence_after();
       float s0, s1;

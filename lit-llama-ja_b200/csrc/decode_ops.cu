@@ -672,19 +672,45 @@ int launch_attn_pf(const void* q, const void* k_cache, const void* v_cache, cons
 }
 
 // ---------------------------------------------------------------- elementwise
-template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, size_t n) {
+struct SiluMul {
+  template <typename T> static __device__ __forceinline__ float of(float a, float b) {
+    return __fmul_rn(dt<T>::rd(a / (1.0f + expf(-a))), b);
+  }
+};
+struct Add {
+  template <typename T> static __device__ __forceinline__ float of(float a, float b) { return __fadd_rn(a, b); }
+};
+template <typename T, typename OP>
+__global__ void binary_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, size_t n) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const float av = dt<T>::ld(a, i);
-    const float s = dt<T>::rd(av / (1.0f + expf(-av)));
-    dt<T>::st(y, i, __fmul_rn(s, dt<T>::ld(b, i)));
+  if (i < n) dt<T>::st(y, i, OP::template of<T>(dt<T>::ld(a, i), dt<T>::ld(b, i)));
+}
+// The same with 16 bytes per access (the form above asks for two bytes at a time and stays at the rate of its instructions).  The last
+// thread also does the n % V numbers that fill no piece.
+template <typename T, typename OP>
+__global__ void __launch_bounds__(256) binary_vec_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, size_t n) {
+  constexpr int V = 16 / sizeof(T);
+  const size_t pieces = n / V, i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < pieces) {
+    const uint4 ua = __ldcs(reinterpret_cast<const uint4*>(a) + i), ub = __ldcs(reinterpret_cast<const uint4*>(b) + i);
+    uint4 uy;
+    const T *pa = reinterpret_cast<const T*>(&ua), *pb = reinterpret_cast<const T*>(&ub);
+    T* py = reinterpret_cast<T*>(&uy);
+#pragma unroll
+    for (int e = 0; e < V; ++e) dt<T>::st(py, e, OP::template of<T>(dt<T>::ld(pa, e), dt<T>::ld(pb, e)));
+    reinterpret_cast<uint4*>(y)[i] = uy;
+  } else if (i == pieces) {
+    for (size_t e = pieces * V; e < n; ++e) dt<T>::st(y, e, OP::template of<T>(dt<T>::ld(a, e), dt<T>::ld(b, e)));
   }
 }
-template <typename T>
-__global__ void add_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ y, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dt<T>::st(y, i, __fadd_rn(dt<T>::ld(a, i), dt<T>::ld(b, i)));
+template <typename T, typename OP>
+void launch_binary(const void* a, const void* b, void* y, size_t n, cudaStream_t st) {
+  if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)y) & 15) == 0) {      // (a column slice or an odd offset takes the plain form)
+    const size_t threads = n / (16 / sizeof(T)) + 1;
+    binary_vec_kernel<T, OP><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n);
+  } else {
+    binary_kernel<T, OP><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const T*)a, (const T*)b, (T*)y, n);
+  }
 }
 // A position past the RoPE table (ref: model.py:101 rope_cache.index_select raises) stops the kernel: the error
 // surfaces at the next synchronisation instead of an out-of-bounds read in the c_attn epilogue.
@@ -897,24 +923,22 @@ int ll_decode_attn_digits(const void* q, const void* k_cache, const void* v_cach
 int ll_silu_mul(const void* a, const void* b, void* y, int dtype, size_t n, ll_stream stream) {
   LL_CHECK_ARG(a && b && y, "null pointer");
   if (n == 0) return LL_OK;
-  const unsigned blocks = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == LL_F32) silu_mul_kernel<float><<<blocks, 256, 0, st>>>((const float*)a, (const float*)b, (float*)y, n);
-  else if (dtype == LL_BF16) silu_mul_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, n);
+  if (dtype == LL_F32) launch_binary<float, SiluMul>(a, b, y, n, st);
+  else if (dtype == LL_BF16) launch_binary<__nv_bfloat16, SiluMul>(a, b, y, n, st);
   else { set_error("silu_mul: unsupported dtype %d", dtype); return LL_ERR_UNSUPPORTED; }
-  LL_LAUNCH_OK("silu_mul_kernel");
+  LL_LAUNCH_OK("silu_mul");
   return LL_OK;
 }
 
 int ll_add(const void* a, const void* b, void* y, int dtype, size_t n, ll_stream stream) {
   LL_CHECK_ARG(a && b && y, "null pointer");
   if (n == 0) return LL_OK;
-  const unsigned blocks = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == LL_F32) add_kernel<float><<<blocks, 256, 0, st>>>((const float*)a, (const float*)b, (float*)y, n);
-  else if (dtype == LL_BF16) add_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, n);
+  if (dtype == LL_F32) launch_binary<float, Add>(a, b, y, n, st);
+  else if (dtype == LL_BF16) launch_binary<__nv_bfloat16, Add>(a, b, y, n, st);
   else { set_error("add: unsupported dtype %d", dtype); return LL_ERR_UNSUPPORTED; }
-  LL_LAUNCH_OK("add_kernel");
+  LL_LAUNCH_OK("add");
   return LL_OK;
 }
 
