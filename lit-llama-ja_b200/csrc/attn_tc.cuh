@@ -5,7 +5,8 @@
 //                     memory, scale, cap, mask, exponentiate, write the weights back over the scores as packed bf16 (one term, or
 //                     two: hi and what hi left over) and keep the row's sum; at the end they normalise and store the row
 //   warp 16         : TMA producer (queries once, then key and value blocks into rings)
-//   warp 17         : one thread issues the MMAs: the scores of the next key block first, then P V of this one
+//   warps 17, 18    : one thread each issues the MMAs of a tile: the scores of the next key block first, then P V of this one (an MMA
+//                     costs its thread 40 to 70 clocks to issue: one thread for both tiles would set the pace)
 // Scores have two buffers per tile, so that the tensor cores form the next block's scores while a block's weights are made; the
 // weights lie where the scores were (MMAs of one thread run in issue order).  The running maximum only moves when a row's scores
 // outgrow it by 2^8: the accumulator is then rescaled in place, which after the first blocks of a row hardly ever happens; the
@@ -49,7 +50,7 @@ struct AttnTcArgs {
   int y_ld;
 };
 
-constexpr int AT_Q = 128, AT_K = 64, AT_C = AT_K / 2, AT_WARPS = 16, AT_THREADS = (AT_WARPS + 2) * 32;
+constexpr int AT_Q = 128, AT_K = 64, AT_C = AT_K / 2, AT_WARPS = 16, AT_THREADS = (AT_WARPS + 3) * 32;
 constexpr int AT_QBOX = AT_Q * 64 * 2, AT_KBOX = AT_K * 64 * 2;      // TMA boxes: rows of 64 bf16
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 constexpr float AT_LOG2E = 1.4426950408889634f;
@@ -214,10 +215,10 @@ __device__ __forceinline__ int at_first_visible(int i, int window, int chunk) {
 // Rows of the key block that starts at position kt: up to 64, ending at the last key and where the ring wraps.
 __device__ __forceinline__ int at_rows(int kt, int last, int ring) { return min(min(AT_K, last - kt + 1), ring - kt % ring); }
 
-// tanh(x) = 1 - 2 / (1 + e^(2x)); for |x| < 1/2 as x P(x^2), P the polynomial through tanh(sqrt(u)) / sqrt(u) at the five Chebyshev
-// points of [0, 1/4] (largest relative error 1.3e-8), which leaves the exponential unit to the softmax
-constexpr float AT_T0 = 0.999999986757f, AT_T1 = -0.333330679444f, AT_T2 = 0.133247505048f, AT_T3 = -0.0529842388285f, AT_T4 = 0.0171313444313f;
-constexpr float AT_TANH_SMALL = 0.5f;
+// tanh(x) = 1 - 2 / (1 + e^(2x)); for |x| < 1/4 as x P(x^2), P the parabola through tanh(sqrt(u)) / sqrt(u) at the three Chebyshev
+// points of [0, 1/16] (largest relative error 4e-7, as the exponential form's), which leaves the exponential unit to the softmax
+constexpr float AT_T0 = 0.999999603463f, AT_T1 = -0.33321896989f, AT_T2 = 0.128414339271f;
+constexpr float AT_TANH_SMALL = 0.25f;
 
 // NB1 / NB2: blocks of 64 dimensions of the two parts of a key row; NBV: of a value row.  KS / VS: stages of key / value blocks.
 template <int NB1, int NB2, int NBV>
@@ -247,7 +248,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   uint64_t* s_full = v_empty + VS;                    // [tile][buffer] scores are there
   uint64_t* p_full = s_full + 4;                      // [tile][buffer] weights are there
   uint64_t* o_full = p_full + 4;                      // [tile][buffer] P V is done
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(o_full + 4);
+  uint64_t* v_clear = o_full + 4;                     // value rows of no key are zero
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(v_clear + 1);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
   int* s_range = s_fail + 1;                          // per tile: smallest and largest position
   float* s_x = reinterpret_cast<float*>(s_range + 4); // [tile][half][row]: what the two threads of a row tell one another
@@ -261,8 +263,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
     mbar_init(q_full, 1);
-    for (int i = 0; i < KS; ++i) mbar_init(&k_full[i], 1), mbar_init(&k_empty[i], 1);
-    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 1);
+    mbar_init(v_clear, 1);
+    for (int i = 0; i < KS; ++i) mbar_init(&k_full[i], 1), mbar_init(&k_empty[i], 2);
+    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 2);
     for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1), mbar_init(&p_full[i], AT_WARPS / 2), mbar_init(&o_full[i], 1);
     for (int i = 0; i < 2; ++i) {
       s_range[2 * i] = INT_MAX;
@@ -321,34 +324,38 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       if (!ok)                       // copies already issued land before the block leaves
         for (int w = 0; w < 2048; ++w) __nanosleep(512);
     }
-  } else if (warp == AT_WARPS + 1) {
-    // ===================== MMA issuer =====================
+  } else if (warp > AT_WARPS) {
+    // ===================== MMA issuers, one per tile =====================
     constexpr uint32_t idesc_s = instr_desc_bf16(AT_Q, AT_K);
     constexpr uint32_t idesc_o = instr_desc_bf16(AT_Q, DV) | (1u << 16);      // V is MN-major
-    uint32_t ns[2] = {0u, 0u}, np[2] = {0u, 0u};      // key blocks whose scores / weighted sum a tile has been given
-    // S = Q K^T of the n-th key block for both tiles: a tile's score buffer is free, its weights two blocks back are in use by
-    // an MMA issued before
+    const int i = warp - AT_WARPS - 1;
+    const int mylo = i == 0 ? lo[0] : lo[1], myhi = i == 0 ? hi[0] : hi[1];
+    const uint32_t tm_s = tmem + TM_S + 128u * i, tm_o = tmem + TM_O + 128u * i;
+    const uint64_t qdesc = smem_desc_sw128(smem_u32(sq + i * NB * AT_QBOX));
+    const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sk)), vdesc0 = smem_desc_mn_sw128(smem_u32(sv));
+    uint32_t ns = 0u, np = 0u, nc = 0u;      // key blocks whose scores / weighted sum the tile has been given; blocks cleared
+    // S = Q K^T of the n-th key block: the tile's score buffer is free, its weights two blocks back are in use by an MMA issued before
     auto scores = [&](int n, int kt, int rows) {
       const int ks = n % KS;
       if (!at_wait_warp(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
       tc_fence_after();
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (kt + rows - 1 < lo[i] || kt > hi[i]) continue;
+      if (kt + rows - 1 >= mylo && kt <= myhi) {
         if (elect_one()) {
-          const uint32_t d = tmem + TM_S + 128u * i + 64u * (ns[i] & 1u);
+          const uint32_t d = tm_s + 64u * (ns & 1u);
+          const uint64_t kdesc = kdesc0 + (uint64_t)(ks * NB * (AT_KBOX >> 4));
 #pragma unroll
-          for (int c = 0; c < NB; ++c) {
-            const uint64_t qdesc = smem_desc_sw128(smem_u32(sq + (i * NB + c) * AT_QBOX));
-            const uint64_t kdesc = smem_desc_sw128(smem_u32(sk + (ks * NB + c) * AT_KBOX));
+          for (int c = 0; c < NB; ++c)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_bf16(d, qdesc + (uint64_t)(2 * k), kdesc + (uint64_t)(2 * k), idesc_s, (c | k) != 0 ? 1u : 0u);
-          }
-          umma_commit(&s_full[2 * i + (int)(ns[i] & 1u)]);
+            for (int k = 0; k < 4; ++k)
+              umma_bf16(d, qdesc + (uint64_t)(c * (AT_QBOX >> 4) + 2 * k), kdesc + (uint64_t)(c * (AT_KBOX >> 4) + 2 * k), idesc_s,
+                        (c | k) != 0 ? 1u : 0u);
+          umma_commit(&s_full[2 * i + (int)(ns & 1u)]);
+          umma_commit(&k_empty[ks]);
         }
-        ++ns[i];
+        ++ns;
+      } else if (elect_one()) {
+        mbar_arrive(&k_empty[ks]);
       }
-      if (elect_one()) umma_commit(&k_empty[ks]);
       return true;
     };
     bool ok = at_wait_warp(q_full, 0, s_fail, 3);
@@ -362,34 +369,39 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       if (!(ok = at_wait_warp(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
       const int keep = step_last - kt + 1;                      // value rows from here on belong to no key of this step
       if (keep < AT_K) {
-        const int pieces = (AT_K - keep) * 8;
-        for (int e = lane; e < pieces * NBV; e += 32) {
-          const int c = e / pieces, r = e - c * pieces;
-          *reinterpret_cast<uint4*>(sv + (vs * NBV + c) * AT_KBOX + keep * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+        if (i == 0) {
+          const int pieces = (AT_K - keep) * 8;
+          for (int e = lane; e < pieces * NBV; e += 32) {
+            const int c = e / pieces, r = e - c * pieces;
+            *reinterpret_cast<uint4*>(sv + (vs * NBV + c) * AT_KBOX + keep * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (elect_one()) mbar_arrive(v_clear);
+        } else if (!(ok = at_wait_warp(v_clear, nc & 1u, s_fail, 10))) {
+          break;
         }
-        fence_proxy_async();
-        __syncwarp();
+        ++nc;
       }
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        if (!ok || kt + rows - 1 < lo[i] || kt > hi[i]) continue;
-        const uint32_t buf = np[i] & 1u;
-        if (!(ok = at_wait_warp(&p_full[2 * i + (int)buf], (np[i] >> 1) & 1u, s_fail, 6))) continue;
+      if (kt + rows - 1 >= mylo && kt <= myhi) {
+        const uint32_t buf = np & 1u;
+        if (!(ok = at_wait_warp(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, 6))) break;
         tc_fence_after();
         if (elect_one()) {
-          const uint64_t vdesc = smem_desc_mn_sw128(smem_u32(sv + vs * NBV * AT_KBOX));
+          const uint64_t vdesc = vdesc0 + (uint64_t)(vs * NBV * (AT_KBOX >> 4));
 #pragma unroll
           for (int term = 0; term < TERMS; ++term)
 #pragma unroll
             for (int k = 0; k < AT_K / UMMA_K; ++k)            // 16 keys: 8 columns of packed weights, two groups of eight rows
-              umma_ts(tmem + TM_O + 128u * i, tmem + TM_S + 128u * i + 64u * buf + 32u * term + 8u * k, vdesc + (uint64_t)(128 * k), idesc_o,
-                      (np[i] != 0u || (term | k) != 0) ? 1u : 0u);
+              umma_ts(tm_o, tm_s + 64u * buf + 32u * term + 8u * k, vdesc + (uint64_t)(128 * k), idesc_o,
+                      (np != 0u || (term | k) != 0) ? 1u : 0u);
           umma_commit(&o_full[2 * i + (int)buf]);
+          umma_commit(&v_empty[vs]);
         }
-        ++np[i];
+        ++np;
+      } else if (elect_one()) {
+        mbar_arrive(&v_empty[vs]);
       }
-      if (!ok) break;
-      if (elect_one()) umma_commit(&v_empty[vs]);
       kt = nkt;
       rows = nrows;
     }
@@ -495,12 +507,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
           }
         } else if (poly) {
-          const f2 t0c = f2_of(cap2 * AT_T0, cap2 * AT_T0), t1c = f2_of(cap2 * AT_T1, cap2 * AT_T1), t2c = f2_of(cap2 * AT_T2, cap2 * AT_T2),
-                   t3c = f2_of(cap2 * AT_T3, cap2 * AT_T3), t4c = f2_of(cap2 * AT_T4, cap2 * AT_T4);
+          const float m3 = mul * mul * mul, c0p = cap2 * AT_T0 * mul, c1p = cap2 * AT_T1 * m3, c2p = cap2 * AT_T2 * (m3 * mul * mul);
+          const f2 p0c = f2_of(c0p, c0p), p1c = f2_of(c1p, c1p), p2c = f2_of(c2p, c2p);
 #pragma unroll
           for (int e = 0; e < AT_C; e += 2) {
-            const f2 x = f2_mul(f2_of(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), mul2), u = f2_mul(x, x);
-            const f2 a = f2_fma(x, f2_fma(f2_fma(f2_fma(f2_fma(t4c, u, t3c), u, t2c), u, t1c), u, t0c), sub2);
+            const f2 x = f2_of(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), u = f2_mul(x, x);
+            const f2 a = f2_fma(x, f2_fma(f2_fma(p2c, u, p1c), u, p0c), sub2);
             float a0, a1;
             f2_split(a, a0, a1);
             sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
