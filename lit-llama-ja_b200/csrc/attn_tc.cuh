@@ -5,8 +5,8 @@
 //                     memory, scale, cap, mask, exponentiate, write the weights back over the scores as packed bf16 (one term, or
 //                     two: hi and what hi left over) and keep the row's sum; at the end they normalise and store the row
 //   warp 16         : TMA producer (queries once, then key and value blocks into rings)
-//   warps 17, 18    : one thread each issues the MMAs of a tile: the scores of the next key block first, then P V of this one (an MMA
-//                     costs its thread 40 to 70 clocks to issue: one thread for both tiles would set the pace)
+//   warps 17, 18    : one thread each issues the MMAs of a tile: the scores of the next key block first, then P V of this one
+//   warp 19         : clears value rows that belong to no key
 // Scores have two buffers per tile, so that the tensor cores form the next block's scores while a block's weights are made; the
 // weights lie where the scores were (MMAs of one thread run in issue order).  The running maximum only moves when a row's scores
 // outgrow it by 2^8: the accumulator is then rescaled in place, which after the first blocks of a row hardly ever happens; the
@@ -50,7 +50,7 @@ struct AttnTcArgs {
   int y_ld;
 };
 
-constexpr int AT_Q = 128, AT_K = 64, AT_C = AT_K / 2, AT_WARPS = 16, AT_THREADS = (AT_WARPS + 3) * 32;
+constexpr int AT_Q = 128, AT_K = 64, AT_C = AT_K / 2, AT_WARPS = 16, AT_THREADS = (AT_WARPS + 4) * 32;
 constexpr int AT_QBOX = AT_Q * 64 * 2, AT_KBOX = AT_K * 64 * 2;      // TMA boxes: rows of 64 bf16
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 constexpr float AT_LOG2E = 1.4426950408889634f;
@@ -142,6 +142,11 @@ __device__ __forceinline__ f2 f2_of(float a, float b) {
 }
 __device__ __forceinline__ void f2_split(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+#ifdef AT_SCALAR
+  float a0, a1, b0, b1, c0, c1;
+  f2_split(a, a0, a1), f2_split(b, b0, b1), f2_split(c, c0, c1);
+  return f2_of(fmaf(a0, b0, c0), fmaf(a1, b1, c1));
+#endif
   f2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
@@ -170,24 +175,13 @@ __device__ __forceinline__ bool elect_one() {
 
 // A wait that ends: on its phase, when another role has given up, or after the limit.
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
   for (uint32_t i = 0; i < AT_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255u) == 255u && *fail) return false;
   }
   *fail = 1;
   atomicCAS(&g_attn_tc_error, 0, code);
-  return false;
-}
-
-// The same for a whole warp, which leaves together.  The MMA warp's control flow and operands have to be uniform in the compiler's
-// eyes (votes, shuffles): from a divergent branch an MMA costs its thread about 100 clocks to issue, more than it takes to run.
-__device__ __forceinline__ bool at_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
-  for (uint32_t i = 0; i < AT_WAIT_LIMIT; ++i) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    if ((i & 255u) == 255u && __any_sync(0xffffffffu, *fail != 0)) return false;
-  }
-  *fail = 1;
-  if (elect_one()) atomicCAS(&g_attn_tc_error, 0, code);
   return false;
 }
 
@@ -212,8 +206,20 @@ __device__ __forceinline__ int at_first_visible(int i, int window, int chunk) {
   return lo;
 }
 
-// Rows of the key block that starts at position kt: up to 64, ending at the last key and where the ring wraps.
-__device__ __forceinline__ int at_rows(int kt, int last, int ring) { return min(min(AT_K, last - kt + 1), ring - kt % ring); }
+// The key block that starts at position kt, slot kt % ring: up to 64 rows, ending at the last key and where the ring wraps.
+struct AtBlock {
+  int kt, slot, rows, last, ring;
+  __device__ __forceinline__ AtBlock(int first, int last_, int ring_) : kt(first), slot(first % ring_), last(last_), ring(ring_) { size(); }
+  __device__ __forceinline__ void size() { rows = min(min(AT_K, last - kt + 1), ring - slot); }
+  __device__ __forceinline__ bool any() const { return kt <= last; }
+  __device__ __forceinline__ bool meets(int lo, int hi) const { return kt + rows - 1 >= lo && kt <= hi; }
+  __device__ __forceinline__ void next() {      // (no division: this stands in every role's loop)
+    kt += rows;
+    slot += rows;
+    if (slot == ring) slot = 0;
+    size();
+  }
+};
 
 // tanh(x) = 1 - 2 / (1 + e^(2x)); for |x| < 1/4 as x P(x^2), P the parabola through tanh(sqrt(u)) / sqrt(u) at the three Chebyshev
 // points of [0, 1/16] (largest relative error 4e-7, as the exponential form's), which leaves the exponential unit to the softmax
@@ -265,7 +271,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     mbar_init(q_full, 1);
     mbar_init(v_clear, 1);
     for (int i = 0; i < KS; ++i) mbar_init(&k_full[i], 1), mbar_init(&k_empty[i], 2);
-    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 2);
+    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 3);
     for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1), mbar_init(&p_full[i], AT_WARPS / 2), mbar_init(&o_full[i], 1);
     for (int i = 0; i < 2; ++i) {
       s_range[2 * i] = INT_MAX;
@@ -301,7 +307,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 
   if (warp == AT_WARPS) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
+    if (elect_one()) {
       const int tiles = t0 + AT_Q < p.T ? 2 : 1;
       mbar_expect_tx(q_full, (uint32_t)(tiles * NB * AT_QBOX));
       for (int i = 0; i < tiles; ++i) {
@@ -310,37 +316,38 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       }
       int n = 0;
       bool ok = true;
-      for (int kt = kt0; kt <= last; ++n) {
-        const int ks = n % KS, vs = n % VS, slot = kt % p.ring;
+      for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next(), ++n) {
+        const int ks = n % KS, vs = n % VS;
         if (!(ok = at_wait(&k_empty[ks], ((n / KS) & 1) ^ 1, s_fail, 1))) break;
         mbar_expect_tx(&k_full[ks], (uint32_t)(NB * AT_KBOX));
-        for (int c = 0; c < NB1; ++c) tma_box4(sk + (ks * NB + c) * AT_KBOX, &map_k, c * 64, g, slot, b, &k_full[ks]);
-        for (int c = 0; c < NB2; ++c) tma_box4(sk + (ks * NB + NB1 + c) * AT_KBOX, &map_k2, c * 64, 0, slot, b, &k_full[ks]);
+        for (int c = 0; c < NB1; ++c) tma_box4(sk + (ks * NB + c) * AT_KBOX, &map_k, c * 64, g, blk.slot, b, &k_full[ks]);
+        for (int c = 0; c < NB2; ++c) tma_box4(sk + (ks * NB + NB1 + c) * AT_KBOX, &map_k2, c * 64, 0, blk.slot, b, &k_full[ks]);
         if (!(ok = at_wait(&v_empty[vs], ((n / VS) & 1) ^ 1, s_fail, 2))) break;
         mbar_expect_tx(&v_full[vs], (uint32_t)(NBV * AT_KBOX));
-        for (int c = 0; c < NBV; ++c) tma_box4(sv + (vs * NBV + c) * AT_KBOX, &map_v, c * 64, g, slot, b, &v_full[vs]);
-        kt += at_rows(kt, last, p.ring);
+        for (int c = 0; c < NBV; ++c) tma_box4(sv + (vs * NBV + c) * AT_KBOX, &map_v, c * 64, g, blk.slot, b, &v_full[vs]);
       }
       if (!ok)                       // copies already issued land before the block leaves
         for (int w = 0; w < 2048; ++w) __nanosleep(512);
     }
-  } else if (warp > AT_WARPS) {
-    // ===================== MMA issuers, one per tile =====================
-    constexpr uint32_t idesc_s = instr_desc_bf16(AT_Q, AT_K);
-    constexpr uint32_t idesc_o = instr_desc_bf16(AT_Q, DV) | (1u << 16);      // V is MN-major
-    const int i = warp - AT_WARPS - 1;
-    const int mylo = i == 0 ? lo[0] : lo[1], myhi = i == 0 ? hi[0] : hi[1];
-    const uint32_t tm_s = tmem + TM_S + 128u * i, tm_o = tmem + TM_O + 128u * i;
-    const uint64_t qdesc = smem_desc_sw128(smem_u32(sq + i * NB * AT_QBOX));
-    const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sk)), vdesc0 = smem_desc_mn_sw128(smem_u32(sv));
-    uint32_t ns = 0u, np = 0u, nc = 0u;      // key blocks whose scores / weighted sum the tile has been given; blocks cleared
-    // S = Q K^T of the n-th key block: the tile's score buffer is free, its weights two blocks back are in use by an MMA issued before
-    auto scores = [&](int n, int kt, int rows) {
-      const int ks = n % KS;
-      if (!at_wait_warp(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
-      tc_fence_after();
-      if (kt + rows - 1 >= mylo && kt <= myhi) {
-        if (elect_one()) {
+  } else if (warp == AT_WARPS + 1 || warp == AT_WARPS + 2) {
+    // ===================== MMA issuers, one thread per tile =====================
+    // (one branch of one elected thread around the whole role: an MMA then takes its thread 40 clocks to issue, and 75 from branches
+    // inside the loop or from `lane == 0`, which is more than the 50 to 64 clocks it runs)
+    if (elect_one()) {
+      constexpr uint32_t idesc_s = instr_desc_bf16(AT_Q, AT_K);
+      constexpr uint32_t idesc_o = instr_desc_bf16(AT_Q, DV) | (1u << 16);      // V is MN-major
+      const int i = warp - AT_WARPS - 1;
+      const int mylo = i == 0 ? lo[0] : lo[1], myhi = i == 0 ? hi[0] : hi[1];
+      const uint32_t tm_s = tmem + TM_S + 128u * i, tm_o = tmem + TM_O + 128u * i;
+      const uint64_t qdesc = smem_desc_sw128(smem_u32(sq + i * NB * AT_QBOX));
+      const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sk)), vdesc0 = smem_desc_mn_sw128(smem_u32(sv));
+      uint32_t ns = 0u, np = 0u, nc = 0u;      // key blocks whose scores / weighted sum the tile has been given; blocks cleared
+      // S = Q K^T of the n-th key block: the tile's score buffer is free, its weights two blocks back are in use by an MMA issued before
+      auto scores = [&](int n, const AtBlock& blk) {
+        const int ks = n % KS;
+        if (!at_wait(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
+        tc_fence_after();
+        if (blk.meets(mylo, myhi)) {
           const uint32_t d = tm_s + 64u * (ns & 1u);
           const uint64_t kdesc = kdesc0 + (uint64_t)(ks * NB * (AT_KBOX >> 4));
 #pragma unroll
@@ -351,43 +358,28 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                         (c | k) != 0 ? 1u : 0u);
           umma_commit(&s_full[2 * i + (int)(ns & 1u)]);
           umma_commit(&k_empty[ks]);
+          ++ns;
+        } else {
+          mbar_arrive(&k_empty[ks]);
         }
-        ++ns;
-      } else if (elect_one()) {
-        mbar_arrive(&k_empty[ks]);
-      }
-      return true;
-    };
-    bool ok = at_wait_warp(q_full, 0, s_fail, 3);
-    int rows = at_rows(kt0, last, p.ring);
-    if (ok) ok = scores(0, kt0, rows);
-    int n = 0;
-    for (int kt = kt0; ok && kt <= last; ++n) {
-      const int nkt = kt + rows, nrows = nkt <= last ? at_rows(nkt, last, p.ring) : 0;
-      if (nkt <= last && !(ok = scores(n + 1, nkt, nrows))) break;
-      const int vs = n % VS;
-      if (!(ok = at_wait_warp(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
-      const int keep = step_last - kt + 1;                      // value rows from here on belong to no key of this step
-      if (keep < AT_K) {
-        if (i == 0) {
-          const int pieces = (AT_K - keep) * 8;
-          for (int e = lane; e < pieces * NBV; e += 32) {
-            const int c = e / pieces, r = e - c * pieces;
-            *reinterpret_cast<uint4*>(sv + (vs * NBV + c) * AT_KBOX + keep * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
-          }
-          fence_proxy_async();
-          __syncwarp();
-          if (elect_one()) mbar_arrive(v_clear);
-        } else if (!(ok = at_wait_warp(v_clear, nc & 1u, s_fail, 10))) {
-          break;
+        return true;
+      };
+      bool ok = at_wait(q_full, 0, s_fail, 3);
+      AtBlock blk(kt0, last, p.ring), nxt = blk;
+      if (ok) ok = scores(0, blk);
+      for (int n = 0; ok && blk.any(); blk = nxt, ++n) {
+        nxt.next();
+        if (nxt.any() && !(ok = scores(n + 1, nxt))) break;
+        const int vs = n % VS;
+        if (!(ok = at_wait(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
+        if (step_last - blk.kt + 1 < AT_K) {
+          if (!(ok = at_wait(v_clear, nc & 1u, s_fail, 10))) break;
+          ++nc;
         }
-        ++nc;
-      }
-      if (kt + rows - 1 >= mylo && kt <= myhi) {
-        const uint32_t buf = np & 1u;
-        if (!(ok = at_wait_warp(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, 6))) break;
-        tc_fence_after();
-        if (elect_one()) {
+        if (blk.meets(mylo, myhi)) {
+          const uint32_t buf = np & 1u;
+          if (!(ok = at_wait(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, 6))) break;
+          tc_fence_after();
           const uint64_t vdesc = vdesc0 + (uint64_t)(vs * NBV * (AT_KBOX >> 4));
 #pragma unroll
           for (int term = 0; term < TERMS; ++term)
@@ -397,13 +389,31 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                       (np != 0u || (term | k) != 0) ? 1u : 0u);
           umma_commit(&o_full[2 * i + (int)buf]);
           umma_commit(&v_empty[vs]);
+          ++np;
+        } else {
+          mbar_arrive(&v_empty[vs]);
         }
-        ++np;
-      } else if (elect_one()) {
-        mbar_arrive(&v_empty[vs]);
       }
-      kt = nkt;
-      rows = nrows;
+    }
+  } else if (warp == AT_WARPS + 3) {
+    // ===================== value rows of no key =====================
+    // a block that reaches past the step's last key holds rows that may hold anything: their weights are 0, and 0 * NaN is not
+    int n = 0;
+    bool ok = true;
+    for (AtBlock blk(kt0, last, p.ring); ok && blk.any(); blk.next(), ++n) {
+      const int keep = step_last - blk.kt + 1, vs = n % VS;
+      ok = __all_sync(0xffffffffu, at_wait(&v_full[vs], (n / VS) & 1, s_fail, 11));
+      if (ok && keep < AT_K) {
+        const int pieces = (AT_K - keep) * 8;
+        for (int e = lane; e < pieces * NBV; e += 32) {
+          const int c = e / pieces, r = e - c * pieces;
+          *reinterpret_cast<uint4*>(sv + (vs * NBV + c) * AT_KBOX + keep * 128 + r * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(v_clear);
+      }
+      if (lane == 0) mbar_arrive(&v_empty[vs]);      // (every block: a wait may not fall two phases behind)
     }
   } else {
     // ===================== softmax, then the epilogue =====================
@@ -423,9 +433,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     f2 sum2[2] = {f2_of(0.f, 0.f), f2_of(0.f, 0.f)};
     uint32_t n = 0;
     bool ok = true;
-    for (int kt = kt0; kt <= last;) {
-      const int rows = at_rows(kt, last, p.ring);
-      if (kt + rows - 1 >= mylo && kt <= myhi) {
+    for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next()) {
+      if (blk.meets(mylo, myhi)) {
         const uint32_t ts = ts0 + 64u * (n & 1u);
         ok = at_wait(&s_full[2 * tile + (int)(n & 1u)], (n >> 1) & 1u, s_fail, 7);
         __syncwarp();
@@ -434,13 +443,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         tmem_ld32_async(ts + (uint32_t)(AT_C * half), sr);
         tmem_wait_ld();
         tie32(sr);
-        const int c0 = kt + AT_C * half;                                    // position of the thread's first column
+        const int c0 = blk.kt + AT_C * half;                                    // position of the thread's first column
         if (BIAS) {
           const float d0 = (float)(c0 - qp), k = p.scale * bias_unit;
 #pragma unroll
           for (int e = 0; e < AT_C; ++e) sr[e] = __float_as_uint(fmaf(slope, d0 + (float)e, __uint_as_float(sr[e]) * k));
         }
-        const int cmin = qlo - c0, cmax = min(rows - 1 - AT_C * half, qhi - c0);          // visible columns of this row
+        const int cmin = qlo - c0, cmax = min(blk.rows - 1 - AT_C * half, qhi - c0);          // visible columns of this row
         const bool masked = __any_sync(0xffffffffu, cmin > 0 || cmax < AT_C - 1);
         float amx = 0.f;
         if (masked) {
@@ -548,7 +557,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         if (lane == 0) mbar_arrive(&p_full[2 * tile + (int)(n & 1u)]);
         ++n;
       }
-      kt += rows;
     }
     if (ok && n > 0 && t0 + tile * AT_Q < p.T) {
       ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, 9);
