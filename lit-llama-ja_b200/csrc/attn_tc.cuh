@@ -65,7 +65,7 @@ struct AtParams {
   const __nv_bfloat16* gate;
   __nv_bfloat16* y;
   float scale, softcap;
-  int T, H, group, vdim, window, chunk, ring, slots, gate_ld, gate_per_head, y_ld;
+  int T, H, group, vdim, window, chunk, ring, slots, gate_ld, gate_per_head, gate_vec, y_ld;
 };
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -125,6 +125,13 @@ __device__ __forceinline__ float at_rcp(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+// 1 / (1 + e^-x), relative error about 1e-6: the products it enters are rounded to bf16
+__device__ __forceinline__ float at_sigmoid(float x) { return at_rcp(1.f + at_exp2(-AT_LOG2E * x)); }
+__device__ __forceinline__ uint4 at_load8(const __nv_bfloat16* p, int vec) {
+  if (vec) return *reinterpret_cast<const uint4*>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 __device__ __forceinline__ void tma_box4(void* dst, const CUtensorMap* map, int x, int h, int row, int b, uint64_t* bar) {
   asm volatile(
@@ -254,8 +261,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   uint64_t* s_full = v_empty + VS;                    // [tile][buffer] scores are there
   uint64_t* p_full = s_full + 4;                      // [tile][buffer] weights are there
   uint64_t* o_full = p_full + 4;                      // [tile][buffer] P V is done
-  uint64_t* v_clear = o_full + 4;                     // value rows of no key are zero
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(v_clear + 1);
+  uint64_t* v_clear = o_full + 4;                     // [VS] value rows of no key are zero: at most two blocks of a walk have such
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(v_clear + VS);  // rows (the last one, and one that the wrap cut off before it)
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
   int* s_range = s_fail + 1;                          // per tile: smallest and largest position
   float* s_x = reinterpret_cast<float*>(s_range + 4); // [tile][half][row]: what the two threads of a row tell one another
@@ -269,9 +276,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
     mbar_init(q_full, 1);
-    mbar_init(v_clear, 1);
     for (int i = 0; i < KS; ++i) mbar_init(&k_full[i], 1), mbar_init(&k_empty[i], 2);
-    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 3);
+    for (int i = 0; i < VS; ++i) mbar_init(&v_full[i], 1), mbar_init(&v_empty[i], 3), mbar_init(&v_clear[i], 1);
     for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1), mbar_init(&p_full[i], AT_WARPS / 2), mbar_init(&o_full[i], 1);
     for (int i = 0; i < 2; ++i) {
       s_range[2 * i] = INT_MAX;
@@ -341,7 +347,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       const uint32_t tm_s = tmem + TM_S + 128u * i, tm_o = tmem + TM_O + 128u * i;
       const uint64_t qdesc = smem_desc_sw128(smem_u32(sq + i * NB * AT_QBOX));
       const uint64_t kdesc0 = smem_desc_sw128(smem_u32(sk)), vdesc0 = smem_desc_mn_sw128(smem_u32(sv));
-      uint32_t ns = 0u, np = 0u, nc = 0u;      // key blocks whose scores / weighted sum the tile has been given; blocks cleared
+      uint32_t ns = 0u, np = 0u;      // key blocks whose scores / weighted sum the tile has been given
       // S = Q K^T of the n-th key block: the tile's score buffer is free, its weights two blocks back are in use by an MMA issued before
       auto scores = [&](int n, const AtBlock& blk) {
         const int ks = n % KS;
@@ -372,10 +378,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         if (nxt.any() && !(ok = scores(n + 1, nxt))) break;
         const int vs = n % VS;
         if (!(ok = at_wait(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
-        if (step_last - blk.kt + 1 < AT_K) {
-          if (!(ok = at_wait(v_clear, nc & 1u, s_fail, 10))) break;
-          ++nc;
-        }
+        if (step_last - blk.kt + 1 < AT_K && !(ok = at_wait(&v_clear[vs], 0, s_fail, 10))) break;
         if (blk.meets(mylo, myhi)) {
           const uint32_t buf = np & 1u;
           if (!(ok = at_wait(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, 6))) break;
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         }
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(v_clear);
+        if (lane == 0) mbar_arrive(&v_clear[vs]);
       }
       if (lane == 0) mbar_arrive(&v_empty[vs]);      // (every block: a wait may not fall two phases behind)
     }
@@ -571,33 +574,33 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         float fin = den > 0.f ? 1.f / den : 0.f;
         const size_t m = (size_t)b * p.T + t;
         const bool live = t < p.T;
-        if (live && p.gate && p.gate_per_head) fin *= 1.f / (1.f + expf(-__bfloat162float(p.gate[m * p.gate_ld + h])));
+        if (live && p.gate && p.gate_per_head) fin *= at_sigmoid(__bfloat162float(p.gate[m * p.gate_ld + h]));
         __nv_bfloat16* dst = p.y + m * p.y_ld + (size_t)h * p.vdim;
         const __nv_bfloat16* gt = p.gate && !p.gate_per_head ? p.gate + m * p.gate_ld + (size_t)h * p.vdim : nullptr;
 #pragma unroll 1
         for (int c = 32 * half; c < DV; c += 64) {
+          // the row's gate numbers are asked for before the accumulator is waited for, 16 bytes at a time (two at a time, one after
+          // the other, took as long as half of the keys)
+          uint4 gu[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (gt && live && c + 8 * e < p.vdim) gu[e] = at_load8(gt + c + 8 * e, p.gate_vec);
           uint32_t o[32];
           tmem_ld32_async(to + (uint32_t)c, o);
           tmem_wait_ld();
           tie32(o);
-          if (live) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
-              if (c + e >= p.vdim) break;           // (vdim is a multiple of 8)
-              float f[8];
+          for (int e = 0; e < 4; ++e) {
+            if (!live || c + 8 * e >= p.vdim) continue;           // (vdim is a multiple of 8)
+            const uint32_t gw[4] = {gu[e].x, gu[e].y, gu[e].z, gu[e].w};
+            uint32_t w[4];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(o[e + j]) * fin;
-              if (gt) {
-#pragma unroll
-                for (int j = 0; j < 8; j += 2) {
-                  const __nv_bfloat162 gg = *reinterpret_cast<const __nv_bfloat162*>(gt + c + e + j);
-                  f[j] *= 1.f / (1.f + expf(-__bfloat162float(gg.x)));
-                  f[j + 1] *= 1.f / (1.f + expf(-__bfloat162float(gg.y)));
-                }
-              }
-              *reinterpret_cast<uint4*>(dst + c + e) =
-                  make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+            for (int j = 0; j < 4; ++j) {
+              float a = __uint_as_float(o[8 * e + 2 * j]) * fin, z = __uint_as_float(o[8 * e + 2 * j + 1]) * fin;
+              if (gt) a *= at_sigmoid(bf16_bits_to_f32(gw[j] & 0xffffu)), z *= at_sigmoid(bf16_bits_to_f32(gw[j] >> 16));
+              w[j] = pack_bf16(a, z);
             }
+            *reinterpret_cast<uint4*>(dst + c + 8 * e) = make_uint4(w[0], w[1], w[2], w[3]);
           }
           __syncwarp();
         }
@@ -672,7 +675,8 @@ enum AttnTcKind { AT_PLAIN, AT_ROTARY, AT_LATENT };     // which forms a file in
 template <AttnTcKind KIND>
 int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
   const AtParams p{a.pos_ids, a.sink, a.slopes, (const __nv_bfloat16*)a.gate, (__nv_bfloat16*)a.y, a.scale, a.softcap, a.T, a.H, a.H / a.G,
-                   a.v.dim, a.window, a.chunk, a.ring, a.slots, a.gate_ld, a.gate_per_head, a.y_ld};
+                   a.v.dim, a.window, a.chunk, a.ring, a.slots, a.gate_ld, a.gate_per_head,
+                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
   const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \

@@ -34,8 +34,8 @@ from torch.nn import functional as F
 from . import _native as N
 from .rotary import RotarySpec
 
-EXPAND_MIN_TOKENS = 64               # tokens a step appends from which its rows are expanded per head
-EXPAND_MAX_SLOTS_PER_TOKEN = 4       # ring slots per such token
+EXPAND_MIN_TOKENS = 16               # tokens a step appends from which its rows are expanded per head
+EXPAND_MAX_SLOTS_PER_TOKEN = 64      # ring slots per such token
 EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
 
 
@@ -200,13 +200,10 @@ class LatentAttention(nn.Module):
             q = F.linear(cq, self.w_uq)                                       # [M, heads * q_head]
         else:
             q = proj
-        if out is None:
-            out = torch.empty((M, s.heads * s.v_dim), dtype=proj.dtype, device=dev)
-        if self._takes_expanded(q, out, cache, B, T, splits):
-            self._attend_expanded(proj, q, B, T, pos_ids, rope, cache, out)
+        if T >= EXPAND_MIN_TOKENS and splits == 1 and self._takes_expanded(q, out, cache, B, T):
+            o = self._attend_expanded(proj, q, B, T, pos_ids, rope, cache, out)
         else:
-            self._attend_latent(proj, q, B, T, pos_ids, rope, cache, splits, out)
-        o = out
+            o = self._attend_latent(proj, q, B, T, pos_ids, rope, cache, splits, out)
         if s.gate == "element":
             N.call("ll_sigmoid_gate_mul", N.ptr(o), o.stride(0), N.ptr_at(proj, self.gate_col0), proj.stride(0), N.ptr(o), o.stride(0), dt,
                    M, s.heads * s.v_dim, st)
@@ -214,34 +211,37 @@ class LatentAttention(nn.Module):
             raise NotImplementedError("a gate per head beside latent queries")
         return o
 
-    def _takes_expanded(self, q, out, cache, B: int, T: int, splits: int) -> bool:
-        """Whether a step expands the cache rows per head (one up-projection of every ring slot) and attends over plain keys and
-        values on the tcgen05 kernel: bf16, sizes that kernel takes, and enough queries for the ring's length."""
+    def _takes_expanded(self, q, out, cache, B: int, T: int) -> bool:
+        """Whether a step of several tokens expands the cache rows per head (one up-projection of every ring slot) and attends over plain
+        keys and values on the tcgen05 kernel: bf16, sizes that kernel takes, a ring that is not too long for the queries.  Both sides
+        measured (16 heads, 128 + 64 dimensions, rank 512, window 1024; device time of the whole layer): 16 tokens after 0 / 1000
+        positions 38 / 111 -> 29 / 47 us, 128 after 8000 119 -> 82 us, 2048 after 0 611 -> 97 us."""
         s = self.spec
         S = cache.shape[1]
-        if T < EXPAND_MIN_TOKENS or splits != 1 or S > EXPAND_MAX_SLOTS_PER_TOKEN * T:
-            return False
-        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0
+        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0 and S <= EXPAND_MAX_SLOTS_PER_TOKEN * T
                 and 2 * B * S * s.heads * (s.nope_dim + s.v_dim) <= EXPAND_MAX_BYTES
-                and N.has("ll_latent_prompt_attn") and cache.is_contiguous() and out.stride(1) == 1
+                and N.has("ll_latent_prompt_attn") and cache.is_contiguous() and (out is None or (out.stride(1) == 1 and out.data_ptr() % 16 == 0))
                 and bool(N.call_ret("ll_latent_prompt_supported", s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, q.stride(0), s.q_head,
-                                    out.stride(0)))
-                and (q.data_ptr() | out.data_ptr() | cache.data_ptr()) % 16 == 0)
+                                    s.heads * s.v_dim if out is None else out.stride(0)))
+                and (q.data_ptr() | cache.data_ptr()) % 16 == 0)
 
-    def _attend_expanded(self, proj, q, B: int, T: int, pos_ids, rope, cache, out) -> None:
+    def _attend_expanded(self, proj, q, B: int, T: int, pos_ids, rope, cache, out) -> torch.Tensor:
         s = self.spec
         S = cache.shape[1]
+        if out is None:
+            out = torch.empty((B * T, s.heads * s.v_dim), dtype=proj.dtype, device=proj.device)
         c = cache.view(B * S, s.row)[:, : s.kv_rank]
         k = F.linear(c, self.w_uk.view(s.heads * s.nope_dim, s.kv_rank))                # [B * S, heads * nope]
-        v = torch.matmul(c, self.w_uv_t)                                                # [heads, B * S, v_dim]
+        v = torch.bmm(c.expand(s.heads, B * S, s.kv_rank), self.w_uv_t)                 # [heads, B * S, v_dim]
         q_rot = torch.empty((B * T, s.heads, s.rot_dim), dtype=q.dtype, device=q.device)
         gate = N.ptr_at(proj, self.gate_col0) if s.gate == "head" and s.q_rank is None else None
         N.call("ll_latent_prompt_attn", N.ptr(q), q.stride(0), s.nope_dim, s.q_head, gate, proj.stride(0), N.ptr(rope), N.ptr(pos_ids),
                N.ptr(k), k.stride(0), s.nope_dim, N.ptr(v), s.v_dim, B * S * s.v_dim, N.ptr(cache), N.ptr(q_rot), N.ptr(out), out.stride(0),
                B, T, s.heads, s.kv_rank, s.rot_dim, s.rot_dims, s.v_dim, S, s.window if s.window is not None else 0, float(s.scale),
                2 if s.exact_weights else 1, N.stream())
+        return out
 
-    def _attend_latent(self, proj, q, B: int, T: int, pos_ids, rope, cache, splits: int, out) -> None:
+    def _attend_latent(self, proj, q, B: int, T: int, pos_ids, rope, cache, splits: int, out) -> torch.Tensor:
         s = self.spec
         M, S, dev = B * T, cache.shape[1], proj.device
         q_nope = q[:, : self.q_cols].view(M, s.heads, s.q_head)[:, :, : s.nope_dim].transpose(0, 1)   # [H, M, nope] view
@@ -256,4 +256,7 @@ class LatentAttention(nn.Module):
                head_gate, N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), N.ptr(o_lat), M * s.kv_rank, s.kv_rank, N.dtype_code(proj.dtype), B, T,
                s.heads, s.kv_rank, s.rot_dim, s.rot_dims, S, s.window if s.window is not None else 0, float(s.scale), splits,
                2 if s.exact_weights else 1, N.ptr(scratch), N.stream())
+        if out is None:
+            return torch.bmm(o_lat, self.w_uv_t).transpose(0, 1).reshape(M, s.heads * s.v_dim)
         torch.bmm(o_lat, self.w_uv_t, out=out.view(M, s.heads, s.v_dim).transpose(0, 1))   # the heads' products land in the rows
+        return out
