@@ -202,7 +202,9 @@ LAUNCHES = 0   # kernels launched through this binding (bench.py's gpu_launches 
 
 def call(name: str, *args) -> None:
     global LAUNCHES
-    check(_fn[name](*args), name)
+    rc = _fn[name](*args)
+    if rc != 0:
+        check(rc, name)
     LAUNCHES += 1
 
 
@@ -232,12 +234,21 @@ def dtype_code(dt: torch.dtype) -> int:
         raise RuntimeError(f"unsupported dtype {dt}") from None
 
 
-def ptr(t) -> C.c_void_p:
-    return C.c_void_p(0 if t is None else t.data_ptr())
+# Addresses and streams go to the library as plain integers (the prototypes above convert them): a small step is a dozen calls of a dozen
+# arguments, and a c_void_p object for each, with a Stream object per call, was a third of its host time.
+def ptr(t) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
-def stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
+def stream() -> int:
+    """The current stream of the current device."""
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def gemv_plan(N: int, K: int, group: int, nmat: int, M: int, grid: int = 0):
@@ -286,8 +297,7 @@ class Workspace:
 
     @classmethod
     def get(cls, device) -> "Workspace":
-        key = (device.index if device.index is not None else torch.cuda.current_device(),
-               torch.cuda.current_stream().cuda_stream)
+        key = (device.index if device.index is not None else torch.cuda.current_device(), stream())
         ws = cls._cache.get(key)
         if ws is None:
             ws = cls._cache[key] = Workspace(device)
@@ -301,7 +311,7 @@ class Workspace:
         return self
 
 
-def ptr_at(t: torch.Tensor, elem_offset: int) -> C.c_void_p:
+def ptr_at(t: torch.Tensor, elem_offset: int) -> int:
     """Address of element ``elem_offset`` (counted in elements of ``t``'s dtype) past ``t``'s first: a column slice of a
     row-major matrix handed to a kernel that takes the row stride separately."""
-    return C.c_void_p(t.data_ptr() + elem_offset * t.element_size())
+    return t.data_ptr() + elem_offset * t.element_size()

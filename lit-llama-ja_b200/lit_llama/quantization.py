@@ -115,8 +115,8 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         return N.STREAM_W8 if self.bits == 8 else N.stream_kind(self.out_features, self.in_features, self.tile_cols, M)
 
     def _state_key(self):
-        return (self.quant_weight.data_ptr(), self.scales.data_ptr(), self.zeros.data_ptr(),
-                self.quant_weight._version, self.scales._version, self.zeros._version)
+        q, s, z = self.quant_weight, self.scales, self.zeros
+        return (q.data_ptr(), s.data_ptr(), z.data_ptr(), q._version, s._version, z._version)
 
     def prepare(self, M: int = 1):
         """Build (once per stream kind) the fragment-ordered weight stream the int4 GEMV reads at batch ``M`` (a derived
@@ -352,7 +352,7 @@ _INT8_WS: dict = {}
 
 def _int8_workspace(device, nbytes: int) -> torch.Tensor:
     """Per-(device, stream) scratch of the int8 linear (kernels on one stream are ordered)."""
-    key = (device.index, torch.cuda.current_stream().cuda_stream)
+    key = (device.index, N.stream())
     ws = _INT8_WS.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = _INT8_WS[key] = torch.empty(nbytes + 256, dtype=torch.uint8, device=device)
