@@ -11,9 +11,13 @@
 // part runs on the tensor cores (mma.sync m16n8k32 s8) with the weights as the A operand straight from
 // global memory in 16-byte loads; K is split across CTAs and combined with int32 atomics (integer addition
 // is associative: bit-deterministic).
+//
+// Prompts (M > 64): the same arithmetic per block of 64 rows (a feature is an outlier for a block of 64 rows, as in the passes above), all
+// blocks at once: row statistics, quantised rows, outlier lists, then ONE product on the 5th-generation tensor cores (tcgen05 kind::i8,
+// int32 accumulators in tensor memory: the same exact sums) and one finishing kernel.  See int8_gemm_tc_kernel.
 #include <stdlib.h>
 
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace llb {
 namespace {
@@ -415,6 +419,373 @@ Ws carve(void* base, int M, int N, int K) {
   return w;
 }
 
+// eight neighbouring activations as x.half() values in fp32 (16-byte aligned)
+template <typename T> __device__ __forceinline__ void int8_load8(const T* p, float (&v)[8]) {
+  constexpr int P = 16 / sizeof(T);
+#pragma unroll
+  for (int i = 0; i < 8; i += P) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p + i);
+    const T* t = reinterpret_cast<const T*>(&u);
+#pragma unroll
+    for (int e = 0; e < P; ++e) v[i + e] = to_half_f32<T>(t[e]);
+  }
+}
+
+// ================================================================================================== prompts: M > 64
+// a16 as above without storing it: sca[m] = absmax over the entries of row m below thr; flag[block of 64 rows][k] = 1 where any
+// |entry| >= thr.  One CTA per row.
+template <typename T>
+__global__ void __launch_bounds__(256) int8_row_stats_kernel(const T* __restrict__ x, uint8_t* __restrict__ flag, float* __restrict__ sca, int K,
+                                                            float thr) {
+  __shared__ float red[8];
+  const int m = blockIdx.x;
+  const T* row = x + (size_t)m * K;
+  uint8_t* fl = flag + (size_t)(m / 64) * K;
+  float mx = 0.f;
+  for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {      // (K is a multiple of 128)
+    float v[8];
+    int8_load8<T>(row + k, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float a = fabsf(v[e]);
+      if (a >= thr) fl[k + e] = 1;
+      else mx = fmaxf(mx, a);
+    }
+  }
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w]);
+    sca[m] = mx;
+  }
+}
+
+// CA[m][k], eight entries per thread
+template <typename T>
+__global__ void __launch_bounds__(256) int8_row_quant_kernel(const T* __restrict__ x, const uint8_t* __restrict__ flag, const float* __restrict__ sca,
+                                                            int8_t* __restrict__ ca, int K, float thr, long long pieces) {
+  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (i >= pieces) return;
+  const int per = K / 8, m = (int)(i / per), k = (int)(i - (long long)m * per) * 8;
+  float v[8];
+  int8_load8<T>(x + (size_t)m * K + k, v);
+  const uint2 f = *reinterpret_cast<const uint2*>(flag + (size_t)(m / 64) * K + k);
+  const float s = sca[m], inv = __fdiv_rn(127.f, s == 0.f ? 1.f : s);
+  uint32_t o[2] = {0u, 0u};
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const uint32_t out = ((e < 4 ? f.x : f.y) >> (8 * (e & 3))) & 0xffu;
+    float q = 0.f;
+    if (out == 0u && fabsf(v[e]) < thr) q = fminf(fmaxf(rintf(__fmul_rn(v[e], inv)), -127.f), 127.f);
+    o[e >> 2] |= ((uint32_t)(int)q & 0xffu) << (8 * (e & 3));
+  }
+  *reinterpret_cast<uint2*>(ca + (size_t)m * K + k) = make_uint2(o[0], o[1]);
+}
+
+// ascending outlier list of every block of 64 rows; one CTA per block
+__global__ void __launch_bounds__(1024) int8_lists_kernel(const uint8_t* __restrict__ flag, int32_t* __restrict__ idx, int32_t* __restrict__ count, int K) {
+  __shared__ int s_warp[32];
+  const uint8_t* fl = flag + (size_t)blockIdx.x * K;
+  int32_t* list = idx + (size_t)blockIdx.x * K;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int base = 0;
+  for (int k0 = 0; k0 < K; k0 += 4096) {             // a thread looks at four neighbouring columns
+    const int k = k0 + threadIdx.x * 4;
+    const uint32_t f = k < K ? *reinterpret_cast<const uint32_t*>(fl + k) : 0u;
+    const int n = __popc(f);
+    int incl = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    int at = base + incl - n, total = 0;
+    for (int w = 0; w < 32; ++w) {
+      if (w < warp) at += s_warp[w];
+      total += s_warp[w];
+    }
+    for (int e = 0; e < 4; ++e)
+      if ((f >> (8 * e)) & 1u) list[at++] = k + e;
+    base += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = base;
+}
+
+// C32[M][N] = CA[M][K] . CB[N][K]^T on tcgen05 (kind::i8, K = 32 an instruction).  A CTA owns 128 x 128 outputs: TMA producer, one issuing
+// thread, four epilogue warps; tiles of 128 x 128 bytes in a ring of three, so that two CTAs share an SM (one's first loads and epilogue run
+// under the other's products).  A 7B feed-forward of 512 rows: 24 passes of 64 rows through mma.sync, four kernels each, took 1435 us on the
+// device (the weights read eight times, the accumulator added up by atomics); three products of 40 us and 28 us around each make 211 us.
+// Every wait is bounded; one that runs out records a code, the roles stop and tensor memory is freed.
+constexpr int I8_BN = 128, I8_STAGES = 3, I8_BOX = 128 * 128;
+constexpr uint32_t I8_WAIT_LIMIT = 1u << 20;
+__device__ int g_int8_tc_error = 0;
+
+__device__ __forceinline__ bool i8_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+  for (uint32_t i = 0; i < I8_WAIT_LIMIT; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && *fail) return false;
+  }
+  *fail = 1;
+  atomicCAS(&g_int8_tc_error, 0, code);
+  return false;
+}
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ bool i8_elect() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r)::"memory");
+  return r != 0;
+}
+__device__ __forceinline__ void i8_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
+               "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+               : "memory");
+}
+
+__global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                                             int32_t* __restrict__ c, int M, int N, int K) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
+  uint8_t *sa = base, *sb = base + I8_STAGES * I8_BOX;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sb + I8_STAGES * I8_BOX);
+  uint64_t* empty = full + I8_STAGES;
+  uint64_t* done = empty + I8_STAGES;
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done + 1);
+  int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * I8_BN, nkb = K / 128;      // (x runs over the rows: CTAs side by side share weights)
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_a);
+    prefetch_tensormap(&map_b);
+    for (int i = 0; i < I8_STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
+    mbar_init(done, 1);
+    *s_fail = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_ptr, I8_BN);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  if (warp == 0) {
+    if (i8_elect()) {
+      bool ok = true;
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % I8_STAGES;
+        if (!(ok = i8_wait(&empty[s], ((kb / I8_STAGES) & 1) ^ 1, s_fail, 1))) break;
+        mbar_expect_tx(&full[s], 2 * I8_BOX);
+        i8_box(sa + s * I8_BOX, &map_a, kb * 128, m0, &full[s]);
+        i8_box(sb + s * I8_BOX, &map_b, kb * 128, n0, &full[s]);
+      }
+      if (!ok)                       // copies already issued land before the CTA leaves
+        for (int w = 0; w < 2048; ++w) __nanosleep(512);
+    }
+  } else if (warp == 1) {
+    if (i8_elect()) {
+      // D = int32 (2 at bit 4), A = B = signed int8 (1 at bits 7 and 10), both K-major
+      constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
+      bool ok = true;
+      for (int kb = 0; kb < nkb; ++kb) {
+        const int s = kb % I8_STAGES;
+        if (!(ok = i8_wait(&full[s], (kb / I8_STAGES) & 1, s_fail, 2))) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          umma_i8(tmem, ad + (uint64_t)(s * (I8_BOX >> 4) + 2 * k), bd + (uint64_t)(s * (I8_BOX >> 4) + 2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+        umma_commit(&empty[s]);
+      }
+      umma_commit(done);             // also after a failure: the epilogue's wait ends
+    }
+  } else {
+    const int quarter = warp & 3, m = m0 + quarter * 32 + lane;
+    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, 3));
+    tc_fence_after();
+    if (ok && *(volatile int*)s_fail == 0) {
+#pragma unroll 1
+      for (int c0 = 0; c0 < I8_BN; c0 += 32) {
+        if (n0 + c0 >= N) break;
+        uint32_t v[32];
+        tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+        if (m >= M) continue;
+        int32_t* dst = c + (size_t)m * N + n0 + c0;
+        if (n0 + c0 + 32 <= N && (N & 3) == 0) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 4)
+            *reinterpret_cast<int4*>(dst + e) = make_int4((int)v[e], (int)v[e + 1], (int)v[e + 2], (int)v[e + 3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (n0 + c0 + e < N) dst[e] = (int)v[e];
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, I8_BN);
+  }
+}
+
+// out = fp16(C32 SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part, for 64 columns x 64 rows (one outlier list) per CTA: a thread owns
+// four columns of four rows; the weights and activations of up to 32 outliers at a time are staged as fp32, already rounded.
+constexpr int I8F_L = 32;
+template <typename T>
+__global__ void __launch_bounds__(256) int8_finish_rows_kernel(const int32_t* __restrict__ c32, const float* __restrict__ sca,
+                                                              const float* __restrict__ scb, const T* __restrict__ bias, const T* __restrict__ x,
+                                                              const int8_t* __restrict__ cb, const int8_t* __restrict__ cbt,
+                                                              const int32_t* __restrict__ idx, const int32_t* __restrict__ count,
+                                                              T* __restrict__ y, int M, int N, int K) {
+  __shared__ __align__(16) float w_s[I8F_L][64], a_s[I8F_L][64];
+  const int n0 = blockIdx.x * 64, blk = blockIdx.y, m0 = blk * 64;
+  const int col = (threadIdx.x & 15) * 4, r0 = (threadIdx.x >> 4) * 4;
+  const int cnt = count[blk];
+  const int32_t* list = idx + (size_t)blk * K;
+  float acc[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+  for (int b = 0; b < cnt; b += I8F_L) {
+    const int ni = min(I8F_L, cnt - b);
+    __syncthreads();
+    for (int e = threadIdx.x; e < ni * 64; e += 256) {
+      const int i = e >> 6, j = e & 63, k = list[b + i], n = n0 + j;
+      float wv = 0.f;
+      if (n < N) {
+        const int8_t q = cbt != nullptr ? cbt[(size_t)k * N + n] : cb[(size_t)n * K + k];
+        wv = __half2float(__float2half_rn(__fmul_rn((float)q, __fdiv_rn(scb[n], 127.f))));
+      }
+      w_s[i][j] = wv;
+      a_s[i][j] = m0 + j < M ? to_half_f32<T>(x[(size_t)(m0 + j) * K + k]) : 0.f;
+    }
+    __syncthreads();
+    for (int i = 0; i < ni; ++i) {
+      const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]), a = *reinterpret_cast<const float4*>(&a_s[i][r0]);
+      const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        acc[r][0] = fmaf(av[r], w.x, acc[r][0]);
+        acc[r][1] = fmaf(av[r], w.y, acc[r][1]);
+        acc[r][2] = fmaf(av[r], w.z, acc[r][2]);
+        acc[r][3] = fmaf(av[r], w.w, acc[r][3]);
+      }
+    }
+  }
+  const int n = n0 + col;
+  if (n >= N) return;
+  float sb[4], bv[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    sb[j] = n + j < N ? scb[n + j] : 0.f;
+    bv[j] = n + j < N && bias != nullptr ? to_half_f32<T>(bias[n + j]) : 0.f;
+  }
+  const bool vec = n + 4 <= N && (N & 3) == 0;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int m = m0 + r0 + r;
+    if (m >= M) break;
+    const float sa = sca[m];
+    const size_t at = (size_t)m * N + n;
+    int cv[4];
+    if (vec) {
+      const int4 v = __ldcs(reinterpret_cast<const int4*>(c32 + at));
+      cv[0] = v.x, cv[1] = v.y, cv[2] = v.z, cv[3] = v.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) cv[j] = n + j < N ? c32[at + j] : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (n + j >= N) break;
+      float out = __fmul_rn(__fmul_rn(__fmul_rn((float)cv[j], sa), sb[j]), 1.0f / (127.0f * 127.0f));
+      if (bias != nullptr) out = __fadd_rn(out, bv[j]);
+      out = __half2float(__float2half_rn(out));
+      if (cnt > 0) out = __half2float(__float2half_rn(__fadd_rn(out, __half2float(__float2half_rn(acc[r][j])))));
+      dt<T>::st(y, at + j, out);
+    }
+  }
+}
+
+constexpr int I8_PASS = 1024;        // rows of one pass: bounds the int32 product (57 MB at 13824 columns)
+struct WsRows {
+  int8_t* ca; int32_t* c32; uint8_t* flag; int32_t* idx; float* sca; int32_t* count;
+  size_t flag_bytes, total;
+};
+WsRows carve_rows(void* base, int M, int N, int K) {
+  WsRows w;
+  const int rows = M < I8_PASS ? M : I8_PASS, blocks = (rows + 63) / 64;
+  size_t o = 0;
+  auto take = [&](size_t b) { size_t r = o; o += (b + 255) & ~(size_t)255; return r; };
+  uint8_t* p = (uint8_t*)base;
+  w.ca = (int8_t*)(p + take((size_t)rows * K));
+  w.c32 = (int32_t*)(p + take((size_t)rows * N * 4));
+  w.flag_bytes = (size_t)blocks * K;
+  w.flag = (uint8_t*)(p + take(w.flag_bytes));
+  w.idx = (int32_t*)(p + take((size_t)blocks * K * 4));
+  w.sca = (float*)(p + take((size_t)rows * 4));
+  w.count = (int32_t*)(p + take((size_t)blocks * 4));
+  w.total = o;
+  return w;
+}
+
+// [rows][K] int8 row-major -> 2-D map, boxes of 128 rows x 128 bytes, 128-byte swizzle, rows past the end zero
+int make_map_i8(const void* base, int rows, int K, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled entry point not available");
+    return LL_ERR_CUDA;
+  }
+  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)K};
+  cuuint32_t box[2] = {128, 128}, estr[2] = {1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d): int8 rows=%d K=%d", (int)r, rows, K);
+    return LL_ERR_CUDA;
+  }
+  return LL_OK;
+}
+
+template <typename T>
+int int8_rows_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* scb, const T* bias, T* y, int M, int N, int K, float thr,
+                void* ws_base, cudaStream_t st) {
+  constexpr int smem = 2 * I8_STAGES * I8_BOX + (2 * I8_STAGES + 1) * 8 + 16 + 1024;
+  LL_CUDA(cudaFuncSetAttribute(int8_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const WsRows w = carve_rows(ws_base, M, N, K);
+  CUtensorMap ma, mb;
+  if (int r = make_map_i8(cb, N, K, &mb)) return r;
+  for (int r0 = 0; r0 < M; r0 += I8_PASS) {
+    const int rows = min(I8_PASS, M - r0), blocks = (rows + 63) / 64;
+    const T* xp = x + (size_t)r0 * K;
+    LL_CUDA(cudaMemsetAsync(w.flag, 0, w.flag_bytes, st));
+    int8_row_stats_kernel<T><<<rows, 256, 0, st>>>(xp, w.flag, w.sca, K, thr);
+    const long long pieces = (long long)rows * (K / 8);
+    int8_row_quant_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(xp, w.flag, w.sca, w.ca, K, thr, pieces);
+    int8_lists_kernel<<<blocks, 1024, 0, st>>>(w.flag, w.idx, w.count, K);
+    if (int r = make_map_i8(w.ca, rows, K, &ma)) return r;
+    int8_gemm_tc_kernel<<<dim3((rows + BM - 1) / BM, (N + I8_BN - 1) / I8_BN), 192, smem, st>>>(ma, mb, w.c32, rows, N, K);
+    int8_finish_rows_kernel<T><<<dim3((N + 63) / 64, blocks), 256, 0, st>>>(w.c32, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count,
+                                                                           y + (size_t)r0 * N, rows, N, K);
+    LL_LAUNCH_OK("int8 linear kernels (prompts)");
+  }
+  return LL_OK;
+}
+
 }  // namespace
 }  // namespace llb
 
@@ -465,7 +836,17 @@ static int int8_linear_t(const T* x, const int8_t* cb, const int8_t* cbt, const 
 
 extern "C" {
 
-size_t ll_int8_workspace_bytes(int M, int N, int K) { return carve(nullptr, M, N, K).total; }
+size_t ll_int8_workspace_bytes(int M, int N, int K) {
+  const size_t pass = carve(nullptr, M < 64 ? M : 64, N, K).total;
+  if (M <= 64) return pass;
+  const size_t rows = carve_rows(nullptr, M, N, K).total;
+  return rows > pass ? rows : pass;
+}
+
+int ll_int8_tc_error(void) {
+  int v = 0;
+  return cudaMemcpyFromSymbol(&v, g_int8_tc_error, sizeof(int)) == cudaSuccess ? v : -1;
+}
 
 int ll_int8_quantize_weight(const void* w, int w_dtype, int8_t* cb, float* scb, int N, int K, ll_stream stream) {
   LL_CHECK_ARG(w && cb && scb && N > 0 && K > 0, "bad int8_quantize_weight arguments");
@@ -488,6 +869,15 @@ int ll_int8_linear(const void* x, int act_dtype, const int8_t* cb, const int8_t*
   LL_CHECK_ARG(((uintptr_t)cb & 15) == 0 && ((uintptr_t)workspace & 255) == 0, "cb must be 16-byte, workspace 256-byte aligned");
   LL_CHECK_ARG(workspace_bytes >= ll_int8_workspace_bytes(M < 64 ? M : 64, N, K), "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
+  // prompts go through the tensor-core form; a workspace that only holds a pass of 64 rows, or rows off 16-byte boundaries, through passes
+  if (M > 64 && workspace_bytes >= ll_int8_workspace_bytes(M, N, K) && ((uintptr_t)x & 15) == 0) {
+    if (act_dtype == LL_BF16)
+      return int8_rows_t<__nv_bfloat16>((const __nv_bfloat16*)x, cb, cbt, scb, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, M, N, K, threshold, workspace, st);
+    if (act_dtype == LL_F16)
+      return int8_rows_t<__half>((const __half*)x, cb, cbt, scb, (const __half*)bias, (__half*)y, M, N, K, threshold, workspace, st);
+    if (act_dtype == LL_F32)
+      return int8_rows_t<float>((const float*)x, cb, cbt, scb, (const float*)bias, (float*)y, M, N, K, threshold, workspace, st);
+  }
   if (act_dtype == LL_BF16)
     return int8_linear_t<__nv_bfloat16>((const __nv_bfloat16*)x, cb, cbt, scb, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, M, N, K, threshold, workspace, st);
   if (act_dtype == LL_F16)

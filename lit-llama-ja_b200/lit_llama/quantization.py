@@ -336,7 +336,7 @@ class Linear8bitLt(torch.nn.Module):
         if M == 0:
             return inp.new_empty(inp.shape[:-1] + (Nout,))
         y = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
-        need = N._fn["ll_int8_workspace_bytes"](min(M, 64), Nout, K)
+        need = N._fn["ll_int8_workspace_bytes"](M, Nout, K)
         ws = _int8_workspace(x.device, need)
         bias = None if self.bias is None else self.bias.to(x.dtype)
         cbt = getattr(self, "_cbt", None)

@@ -1,0 +1,59 @@
+"""llm.int8 prompts (M > 64, one product on the tensor cores) against the passes of 64 rows that the same call makes with a workspace for 64
+rows: the same integer sums and roundings, so the same numbers."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 64, 128), (127, 130, 256), (128, 128, 128), (129, 257, 384), (200, 1000, 512), (1023, 96, 256), (1025, 33, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("outliers,bias,transposed", [(0, False, True), (5, True, True), (40, True, False)])
+def test_rows_against_passes(M, N, K, dtype, outliers, bias, transposed):
+    from lit_llama import _native as NV
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    x = torch.randn((M, K), generator=g, device="cuda")
+    cols = torch.randperm(K, generator=g, device="cuda")[:outliers]
+    rows = torch.rand(M, generator=g, device="cuda") < 0.3            # a feature stands out in some blocks of 64 rows and not in others
+    rows[64:] &= torch.arange(64, M, device="cuda") < 2 * M // 3
+    x[:, cols] = torch.where(rows[:, None], x[:, cols] * 30.0, x[:, cols])
+    x[M // 2] = 0.0                                                    # a row without a scale
+    x = x.to(dtype)
+    w = (torch.randn((N, K), generator=g, device="cuda") * 0.05).to(dtype)
+    cb, scb = torch.empty((N, K), dtype=torch.int8, device="cuda"), torch.empty(N, device="cuda")
+    NV.call("ll_int8_quantize_weight", NV.ptr(w), NV.dtype_code(dtype), NV.ptr(cb), NV.ptr(scb), N, K, NV.stream())
+    cbt = cb.t().contiguous() if transposed else None
+    b = torch.randn(N, generator=g, device="cuda").to(dtype) if bias else None
+    outs = []
+    for m in (M, 64):
+        ws = torch.full((NV.call_ret("ll_int8_workspace_bytes", m, N, K),), 0x5A, dtype=torch.uint8, device="cuda")
+        y = torch.empty((M, N), dtype=dtype, device="cuda")
+        NV.call("ll_int8_linear", NV.ptr(x), NV.dtype_code(dtype), NV.ptr(cb), NV.ptr(cbt), NV.ptr(scb), NV.ptr(b), NV.ptr(y), M, N, K, 6.0, NV.ptr(ws),
+                ws.numel(), NV.stream())
+        outs.append(y)
+    torch.cuda.synchronize()
+    assert NV.call_ret("ll_int8_tc_error") == 0
+    # up to 64 outliers a block are summed in the same order on both sides
+    assert torch.equal(outs[0], outs[1])
+
+
+def test_more_outliers_than_one_stage():
+    from lit_llama.quantization import Linear8bitLt
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    M, N, K = 150, 200, 1024
+    lin = Linear8bitLt(K, N, bias=False, device="cuda", dtype=torch.float32)
+    lin.load_state_dict({"weight": torch.randn((N, K), generator=g, device="cuda") * 0.05})
+    x = torch.randn((M, K), generator=g, device="cuda") * 0.5
+    x[:, ::3] = torch.sign(x[:, ::3]) * (7.0 + x[:, ::3].abs())        # 342 outlier features: several stages of the finishing kernel
+    y = lin(x).double()
+    a, cb, scb = x.half().double(), lin.weight.CB.double(), lin.weight.SCB.double()
+    cols = torch.zeros(K, dtype=torch.bool, device="cuda")
+    cols[::3] = True
+    rest = a.masked_fill(cols[None], 0.0)
+    sca = rest.abs().amax(1)
+    ca = torch.round((rest.float() * (127.0 / sca.float())[:, None]).double())
+    want = (ca @ cb.t()) * sca[:, None] * scb[None] / 127.0 ** 2 + a[:, cols] @ (cb[:, cols] * scb[:, None] / 127.0).half().double().t()
+    # fp16 roundings of the two parts and of their sum (2^-11 each of the largest value)
+    assert (y - want).abs().max() <= 4 * 2.0 ** -11 * want.abs().max()
