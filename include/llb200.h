@@ -576,6 +576,12 @@ LL_API int ll_decay_chunked(const void* q, int q_stride, const void* k, int k_st
                             const float* a, int a_constant, int act_silu, const float* ks, const float* skip, float qs, float* state,
                             const int32_t* pos_ids, float* y, int B, int T, int H, int qk_heads, int n, int p, float* scratch,
                             ll_stream stream);
+/* The same for a recurrence whose last of p columns per head is the constant 1 and not in v (v holds p - 1 columns per head): a decay per
+ * head and token, ks per head and token, no skip.  p - 1 in multiples of 8.  state [B][H][n][p] and y [B*T][H*p] need no alignment. */
+LL_API size_t ll_decay_chunked_unit_scratch_bytes(int B, int T, int H, int n, int p);
+LL_API int ll_decay_chunked_unit(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int dtype, const float* a,
+                                 const float* ks, float qs, float* state, const int32_t* pos_ids, float* y, int B, int T, int H, int qk_heads,
+                                 int n, int p, float* scratch, ll_stream stream);
 /* Gated delta rule (csrc/delta_rule.cu), per sequence b and head h with S an n x p matrix, q and k of head h / (H / qk_heads):
  *   k^ = k / sqrt(|k|^2 + unit_eps),  q^ = q / sqrt(|q|^2 + unit_eps) * qs
  *   g = exp(-exp(a_log[h]) * softplus(raw_a + dt_bias[h])),  beta = sigmoid(raw_b)

@@ -23,7 +23,7 @@ FLAGS = [
 FAMILY_SOURCES = {
     "Lepalorn": ["quant_pack", "decode_ops", "sampling", "residual_ops", "latent_attn", "moe_ops", "moe_gemm_tc"],
     "Bededra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "window_attn", "moe_ops", "moe_gemm_tc"],
-    "Tebodra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "rotary_attn"],
+    "Tebodra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "rotary_attn"],
     "Livasun": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "rotary_attn", "moe_ops", "moe_gemm_tc"],
     "Zekonex": ["quant_pack", "residual_ops", "short_conv", "delta_rule", "delta_chunk", "rotary_attn", "latent_attn"],
     "Bumulix": ["quant_pack", "residual_ops", "rotary_attn", "latent_attn"],

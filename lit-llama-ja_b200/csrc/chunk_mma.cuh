@@ -63,6 +63,14 @@ struct DcTile {
       if (i < UNITS && s < len && ch < cols) u[it] = *(const uint4*)(base + (size_t)s * stride + ch);
     }
   }
+  // column `col` (a multiple of 8, not one of those loaded) becomes 1 in the rows there are
+  __device__ __forceinline__ void one(int col, int len) {
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      const int i = it * DC_THREADS + threadIdx.x, s = i / (PAD / 8), ch = (i % (PAD / 8)) * 8;
+      if (i < UNITS && s < len && ch == col) u[it].x = 0x3f80u;
+    }
+  }
   template <bool SILU>
   __device__ __forceinline__ void store(__nv_bfloat16* smem, int ld) const {
 #pragma unroll

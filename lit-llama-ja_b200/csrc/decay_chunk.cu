@@ -10,6 +10,12 @@
 // e^(..) ks k enters D as three bf16 terms (24 bits: what is carried on is as exact as the walk's fp32), the chunk's weights and
 // the state meet v and q as two terms (16 bits, the sum of both products in fp32).  Sums of log a are formed in fp64, so that the
 // difference of two of them keeps its digits whatever lies before it in the chunk.  The state handed on is fp32.
+//
+// UNIT: the last of the p columns of every head is the constant 1 and not part of v (the normaliser of a matrix memory rides in the same
+// products).  p is then one more than a multiple of 8: the chunks' states are kept with rows of p + 3 numbers, the caller's state and y are
+// read and written one number at a time, and what meets v and q has three terms (24 bits), as the walk this form replaces is fp32.
+// 2048 tokens, 8 heads of 128 x 257: the walk took 496 us (a chain of 2048 steps), collect + pass + read take 24 + 14 + 51.  Column tiles of
+// 64: with three terms of the state a tile of 128 leaves one block per SM.
 #include "chunk_mma.cuh"
 
 namespace llb {
@@ -32,13 +38,14 @@ __device__ __forceinline__ void dc_log_sums(const float* __restrict__ a, int a_r
 
 // grid (chunks * p tiles, H, B): D_c into dst[((b * H + h) * chunks + c)][n][p], e^(G_last) into total[(b * H + h) * chunks + c].
 // NP: n rounded up to 16, 32, 64 or 128.
-template <int NP, int PT, bool SILU>
+template <int NP, int PT, bool SILU, bool UNIT>
 __global__ void __launch_bounds__(DC_THREADS, 2) decay_collect_kernel(const __nv_bfloat16* __restrict__ k, int k_stride,
                                                                       const __nv_bfloat16* __restrict__ v, int v_stride,
                                                                       const float* __restrict__ a, int a_row, const float* __restrict__ ks,
                                                                       float* __restrict__ dst, float* __restrict__ total, int Tn, int H,
                                                                       int qk_heads, int n, int p, int ptiles) {
   constexpr int LK = NP + 8, LV = PT + 8, NF = PT / 16;        // NF: 8-column fragments of a warp's half
+  const int pv = UNIT ? p - 1 : p, pp = UNIT ? p + 3 : p;      // columns of v; numbers in a row of a chunk's state
   extern __shared__ __align__(16) unsigned char dc_smem[];
   __nv_bfloat16* Ks = (__nv_bfloat16*)dc_smem;                // [3 terms][64][LK]
   __nv_bfloat16* Vs = Ks + 3 * DC_L * LK;                     // [64][LV]
@@ -50,7 +57,8 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_collect_kernel(const __nv
   DcTile<NP> kt;
   DcTile<PT> vt;
   kt.load(k + m0 * k_stride + (size_t)g * n, k_stride, len, n);
-  vt.load(v + m0 * v_stride + (size_t)h * p + p0, v_stride, len, p - p0);
+  vt.load(v + m0 * v_stride + (size_t)h * pv + p0, v_stride, len, pv - p0);
+  if (UNIT) vt.one(pv - p0, len);
   const float ksv = (tid < len && ks) ? ks[(m0 + tid) * H + h] : 1.f;
   dc_log_sums(a, a_row, h, m0, len, G);
   vt.template store<SILU>(Vs, LV);
@@ -78,7 +86,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_collect_kernel(const __nv
   }
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31, c0 = (warp >> 2) * (PT / 2);
-  float* D = dst + (((size_t)b * H + h) * chunks + c) * (size_t)n * p;
+  float* D = dst + (((size_t)b * H + h) * chunks + c) * (size_t)n * pp;
 #pragma unroll 1
   for (int mt = warp & 3; mt < NP / 16; mt += 4) {
     if (mt * 16 >= n) break;
@@ -107,23 +115,32 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_collect_kernel(const __nv
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int i = mt * 16 + (lane >> 2) + e * 8, col = p0 + c0 + f * 8 + (lane & 3) * 2;
-        if (i < n && col < p) *(float2*)(D + (size_t)i * p + col) = make_float2(acc[f][2 * e], acc[f][2 * e + 1]);
+        if (i < n && col < p) *(float2*)(D + (size_t)i * pp + col) = make_float2(acc[f][2 * e], acc[f][2 * e + 1]);
       }
   }
 }
 
 // Per (sequence, head), two neighbouring elements of the state a thread: D_c is replaced by the state before chunk c, the state
 // after the last chunk goes back to `state`.
+template <bool UNIT>
 __global__ void __launch_bounds__(128) decay_pass_kernel(float* __restrict__ chunk_state, const float* __restrict__ total,
                                                          float* __restrict__ state, const int32_t* __restrict__ pos_ids, int chunks,
-                                                         int np2) {
+                                                         int np2, int n, int p) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= np2) return;
   const size_t bh = blockIdx.y;
   float2* D = (float2*)chunk_state + bh * chunks * np2 + i;
-  float2* S = (float2*)state + bh * np2 + i;
+  // UNIT: where the pair sits in the caller's rows of p numbers, and whether its two numbers are there at all
+  const int r = UNIT ? (2 * i) / (p + 3) : 0, c = UNIT ? 2 * i - r * (p + 3) : 0;
+  float* S = UNIT ? state + bh * ((size_t)n * p) + (size_t)r * p + c : state + (bh * np2 + i) * 2;
+  const bool in0 = !UNIT || c < p, in1 = !UNIT || c + 1 < p;
+  if (!in0) return;
   const float* tot = total + bh * chunks;
-  float2 s = pos_ids[0] == 0 ? make_float2(0.f, 0.f) : *S;
+  float2 s = make_float2(0.f, 0.f);
+  if (pos_ids[0] != 0) {
+    if (UNIT) s = make_float2(S[0], in1 ? S[1] : 0.f);
+    else s = *(const float2*)S;
+  }
   constexpr int AHEAD = 16;                                   // chunks whose loads are in flight together
   for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
     float2 d[AHEAD];
@@ -137,22 +154,28 @@ __global__ void __launch_bounds__(128) decay_pass_kernel(float* __restrict__ chu
         s = make_float2(w * s.x + d[j].x, w * s.y + d[j].y);
       }
   }
-  *S = s;
+  if (UNIT) {
+    S[0] = s.x;
+    if (in1) S[1] = s.y;
+  } else {
+    *(float2*)S = s;
+  }
 }
 
 // grid (chunks * p tiles, H, B).  A warp owns 16 consecutive tokens and half of the block's columns; its queries come from global
 // memory straight into fragments.
-template <int NP, int PT, bool SILU>
+template <int NP, int PT, bool SILU, bool UNIT>
 __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
     const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k, int k_stride, const __nv_bfloat16* __restrict__ v,
     int v_stride, const float* __restrict__ a, int a_row, const float* __restrict__ ks, const float* __restrict__ skip, float qs,
     const float* __restrict__ chunk_state, const int32_t* __restrict__ pos_ids, float* __restrict__ y, int Tn, int H, int qk_heads, int n,
     int p, int ptiles) {
-  constexpr int LK = NP + 8, LV = PT + 8, NF = PT / 16;
+  constexpr int LK = NP + 8, LV = PT + 8, NF = PT / 16, ZT = UNIT ? 3 : 2;      // ZT: bf16 terms of a weight and of the state
+  const int pv = UNIT ? p - 1 : p, pp = UNIT ? p + 3 : p;
   extern __shared__ __align__(16) unsigned char dc_smem[];
   __nv_bfloat16* Ks = (__nv_bfloat16*)dc_smem;                // [64][LK]
   __nv_bfloat16* Vs = Ks + DC_L * LK;                         // [64][LV]
-  __nv_bfloat16* Ss = Vs + DC_L * LV;                         // [2 terms][NP][LV]
+  __nv_bfloat16* Ss = Vs + DC_L * LV;                         // [ZT terms][NP][LV]
   __shared__ double G[DC_L];
   __shared__ float kw[DC_L];
   const int c = blockIdx.x / ptiles, p0 = (blockIdx.x - c * ptiles) * PT, h = blockIdx.y, b = blockIdx.z, g = h / (H / qk_heads);
@@ -160,11 +183,12 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row0 = (warp & 3) * 16, c0 = (warp >> 2) * (PT / 2);
   const size_t m0 = (size_t)b * Tn + t0;
   const bool has_state = c > 0 || pos_ids[0] != 0;
-  const float* S = chunk_state + (((size_t)b * H + h) * chunks + c) * (size_t)n * p;
+  const float* S = chunk_state + (((size_t)b * H + h) * chunks + c) * (size_t)n * pp;
   DcTile<NP> kt;
   DcTile<PT> vt;
   kt.load(k + m0 * k_stride + (size_t)g * n, k_stride, len, n);
-  vt.load(v + m0 * v_stride + (size_t)h * p + p0, v_stride, len, p - p0);
+  vt.load(v + m0 * v_stride + (size_t)h * pv + p0, v_stride, len, pv - p0);
+  if (UNIT) vt.one(pv - p0, len);
   const float ksv = (tid < len && ks) ? ks[(m0 + tid) * H + h] : 1.f;
   // the state's rows in rounds of eight 16-byte units per thread: the first round is requested with the keys and values
   constexpr int SU = NP * (PT / 4), SR = (SU + 8 * DC_THREADS - 1) / (8 * DC_THREADS);
@@ -174,7 +198,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
     for (int it = 0; it < 8; ++it) {
       const int i = (rd * 8 + it) * DC_THREADS + tid, r = i / (PT / 4), col = (i % (PT / 4)) * 4;
       sv[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (i < SU && r < n && p0 + col < p) sv[it] = *(const float4*)(S + (size_t)r * p + p0 + col);
+      if (i < SU && r < n && p0 + col < p) sv[it] = *(const float4*)(S + (size_t)r * pp + p0 + col);
     }
   };
   if (has_state) state_load(0);
@@ -188,9 +212,11 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
         const int i = (rd * 8 + it) * DC_THREADS + tid, r = i / (PT / 4), col = (i % (PT / 4)) * 4;
         if (i >= SU) break;
         float4 f = sv[it];
-        const uint32_t h0 = dc_term(f.x, f.y), h1 = dc_term(f.z, f.w);
-        *(uint2*)&Ss[r * LV + col] = make_uint2(h0, h1);
-        *(uint2*)&Ss[(NP + r) * LV + col] = make_uint2(pack_bf16(f.x, f.y), pack_bf16(f.z, f.w));
+        uint32_t z0[ZT], z1[ZT];
+        dc_terms<ZT>(f.x, f.y, z0);
+        dc_terms<ZT>(f.z, f.w, z1);
+#pragma unroll
+        for (int z = 0; z < ZT; ++z) *(uint2*)&Ss[(z * NP + r) * LV + col] = make_uint2(z0[z], z1[z]);
       }
       if (rd + 1 < SR) state_load(rd + 1);
     }
@@ -217,7 +243,7 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
 #pragma unroll
     for (int kk = 0; kk < NP / 16; ++kk)
 #pragma unroll
-      for (int z = 1; z >= 0; --z)
+      for (int z = ZT - 1; z >= 0; --z)
 #pragma unroll
         for (int d = 0; d < NF / 2; ++d) {
           uint32_t bf[4];
@@ -249,20 +275,25 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
         const int s = st * 16 + j * 8 + (lane & 3) * 2 + (e & 1), r = r0 + (e >> 1) * 8;
         sc[j][e] = s <= r ? sc[j][e] * (expf((float)((e >> 1 ? g1 : g0) - G[s])) * kw[s]) : 0.f;
       }
-    uint32_t ah[4], al[4];
+    uint32_t at[ZT][4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      ah[2 * j] = dc_term(sc[j][0], sc[j][1]), al[2 * j] = pack_bf16(sc[j][0], sc[j][1]);
-      ah[2 * j + 1] = dc_term(sc[j][2], sc[j][3]), al[2 * j + 1] = pack_bf16(sc[j][2], sc[j][3]);
-    }
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        uint32_t z0[ZT];
+        dc_terms<ZT>(sc[j][2 * e], sc[j][2 * e + 1], z0);
+#pragma unroll
+        for (int z = 0; z < ZT; ++z) at[z][2 * j + e] = z0[z];
+      }
 #pragma unroll
     for (int d = 0; d < NF / 2; ++d) {
       uint32_t bf[4];
       dc_ldmatrix_trans(bf, &Vs[(st * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LV + c0 + d * 16 + (lane >> 4) * 8]);
-      mma_bf16_16816(o[2 * d], al[0], al[1], al[2], al[3], bf[0], bf[1]);
-      mma_bf16_16816(o[2 * d + 1], al[0], al[1], al[2], al[3], bf[2], bf[3]);
-      mma_bf16_16816(o[2 * d], ah[0], ah[1], ah[2], ah[3], bf[0], bf[1]);
-      mma_bf16_16816(o[2 * d + 1], ah[0], ah[1], ah[2], ah[3], bf[2], bf[3]);
+#pragma unroll
+      for (int z = ZT - 1; z >= 0; --z) {
+        mma_bf16_16816(o[2 * d], at[z][0], at[z][1], at[z][2], at[z][3], bf[0], bf[1]);
+        mma_bf16_16816(o[2 * d + 1], at[z][0], at[z][1], at[z][2], at[z][3], bf[2], bf[3]);
+      }
     }
   }
   const float sk = skip ? skip[h] : 0.f;
@@ -280,33 +311,38 @@ __global__ void __launch_bounds__(DC_THREADS, 2) decay_read_kernel(
         v0 += sk * __bfloat162float(Vs[r * LV + c0 + col]);
         v1 += sk * __bfloat162float(Vs[r * LV + c0 + col + 1]);
       }
-      *(float2*)(yr + col) = make_float2(v0, v1);
+      if (UNIT) {
+        yr[col] = v0;
+        if (p0 + c0 + col + 1 < p) yr[col + 1] = v1;
+      } else {
+        *(float2*)(yr + col) = make_float2(v0, v1);
+      }
     }
   }
 }
 
-template <int NP, int PT, bool SILU>
+template <int NP, int PT, bool SILU, bool UNIT = false>
 static int decay_chunked_launch(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, const float* a,
                                 int a_row, const float* ks, const float* skip, float qs, float* state, const int32_t* pos_ids, float* y,
                                 int B, int Tn, int H, int qk_heads, int n, int p, float* scratch, cudaStream_t st) {
-  const int chunks = (Tn + DC_L - 1) / DC_L, ptiles = (p + PT - 1) / PT, np2 = n * p / 2;
+  const int chunks = (Tn + DC_L - 1) / DC_L, ptiles = (p + PT - 1) / PT, pp = UNIT ? p + 3 : p, np2 = n * pp / 2;
   float* chunk_state = scratch;
-  float* total = scratch + (size_t)B * H * chunks * n * p;
+  float* total = scratch + (size_t)B * H * chunks * n * pp;
   const dim3 grid(chunks * ptiles, H, B);
-  constexpr int smem_c = (3 * DC_L * (NP + 8) + DC_L * (PT + 8)) * 2, smem_r = (DC_L * (NP + 8) + DC_L * (PT + 8) + 2 * NP * (PT + 8)) * 2;
+  constexpr int smem_c = (3 * DC_L * (NP + 8) + DC_L * (PT + 8)) * 2, smem_r = (DC_L * (NP + 8) + DC_L * (PT + 8) + (UNIT ? 3 : 2) * NP * (PT + 8)) * 2;
   static bool sized = false;
   if (!sized) {
-    LL_CUDA(cudaFuncSetAttribute(decay_collect_kernel<NP, PT, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_c));
-    LL_CUDA(cudaFuncSetAttribute(decay_read_kernel<NP, PT, SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_r));
+    LL_CUDA(cudaFuncSetAttribute(decay_collect_kernel<NP, PT, SILU, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_c));
+    LL_CUDA(cudaFuncSetAttribute(decay_read_kernel<NP, PT, SILU, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_r));
     sized = true;
   }
   typedef const __nv_bfloat16* in_t;
-  decay_collect_kernel<NP, PT, SILU><<<grid, DC_THREADS, smem_c, st>>>((in_t)k, k_stride, (in_t)v, v_stride, a, a_row, ks, chunk_state, total, Tn, H,
+  decay_collect_kernel<NP, PT, SILU, UNIT><<<grid, DC_THREADS, smem_c, st>>>((in_t)k, k_stride, (in_t)v, v_stride, a, a_row, ks, chunk_state, total, Tn, H,
                                                                   qk_heads, n, p, ptiles);
   LL_LAUNCH_OK("decay_collect_kernel");
-  decay_pass_kernel<<<dim3((np2 + 127) / 128, B * H), 128, 0, st>>>(chunk_state, total, state, pos_ids, chunks, np2);
+  decay_pass_kernel<UNIT><<<dim3((np2 + 127) / 128, B * H), 128, 0, st>>>(chunk_state, total, state, pos_ids, chunks, np2, n, p);
   LL_LAUNCH_OK("decay_pass_kernel");
-  decay_read_kernel<NP, PT, SILU><<<grid, DC_THREADS, smem_r, st>>>((in_t)q, q_stride, (in_t)k, k_stride, (in_t)v, v_stride, a, a_row, ks, skip, qs,
+  decay_read_kernel<NP, PT, SILU, UNIT><<<grid, DC_THREADS, smem_r, st>>>((in_t)q, q_stride, (in_t)k, k_stride, (in_t)v, v_stride, a, a_row, ks, skip, qs,
                                                                chunk_state, pos_ids, y, Tn, H, qk_heads, n, p, ptiles);
   LL_LAUNCH_OK("decay_read_kernel");
   return LL_OK;
@@ -353,6 +389,31 @@ int ll_decay_chunked(const void* q, int q_stride, const void* k, int k_stride, c
   LL_DC(16) LL_DC(32) LL_DC(64) LL_DC(128)
 #undef LL_DC
 #undef LL_DC_S
+  return LL_ERR_UNSUPPORTED;
+}
+
+size_t ll_decay_chunked_unit_scratch_bytes(int B, int T, int H, int n, int p) {
+  return ll_decay_chunked_scratch_bytes(B, T, H, n, p + 3);
+}
+
+int ll_decay_chunked_unit(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int dtype, const float* a,
+                          const float* ks, float qs, float* state, const int32_t* pos_ids, float* y, int B, int T, int H, int qk_heads, int n,
+                          int p, float* scratch, ll_stream stream) {
+  LL_CHECK_ARG(q && k && v && a && state && pos_ids && y && scratch, "decay_chunked_unit: null pointer");
+  LL_CHECK_ARG(B >= 0 && T >= 0 && H > 0 && qk_heads > 0 && H % qk_heads == 0 && n > 0 && p > 1, "bad decay_chunked_unit arguments");
+  if (B == 0 || T == 0) return LL_OK;
+  const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)scratch;
+  if (!ll_decay_chunked_supported(dtype, T, n, p - 1, q_stride, k_stride, v_stride) || (at & 15) != 0 || (long long)B * H > 65535) {
+    set_error("decay_chunked_unit: bf16, at least %d tokens, n and p - 1 in multiples of 8 (n up to 128), rows on 16-byte boundaries", DC_L);
+    return LL_ERR_UNSUPPORTED;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+#define LL_DCU(NP)                                                                                                                        \
+  if (n <= NP)                                                                                                                            \
+    return decay_chunked_launch<NP, 64, false, true>(q, q_stride, k, k_stride, v, v_stride, a, H, ks, nullptr, qs, state, pos_ids, y, B, T, H, \
+                                                     qk_heads, n, p, scratch, st);
+  LL_DCU(16) LL_DCU(32) LL_DCU(64) LL_DCU(128)
+#undef LL_DCU
   return LL_ERR_UNSUPPORTED;
 }
 

@@ -72,6 +72,13 @@ def decay_scan(q, q_col, k, k_col, v, v_col, decay, per_channel, kscale, skip, q
     if not per_channel and not unit_col and takes_chunks(T, H, n, p, (q, q_col), (k, k_col), (v, v_col)):
         _decay_chunked(q, q_col, k, k_col, v, v_col, decay, False, False, kscale, skip, qscale, state, pos_ids, y, B, T, H, qk_heads, n, p)
         return y
+    if unit_col and not per_channel and skip is None and N.has("ll_decay_chunked_unit") \
+            and takes_chunks(T, H, n, p - 1, (q, q_col), (k, k_col), (v, v_col)):
+        scratch = torch.empty(N.call_ret("ll_decay_chunked_unit_scratch_bytes", B, T, H, n, p) // 4, dtype=torch.float32, device=v.device)
+        N.call("ll_decay_chunked_unit", N.ptr_at(q, q_col), q.stride(0), N.ptr_at(k, k_col), k.stride(0), N.ptr_at(v, v_col), v.stride(0),
+               N.dtype_code(v.dtype), N.ptr(decay), N.ptr(kscale), float(qscale), N.ptr(state), N.ptr(pos_ids), N.ptr(y), B, T, H, qk_heads, n,
+               p, N.ptr(scratch), N.stream())
+        return y
     N.call("ll_decay_scan", N.ptr_at(q, q_col), q.stride(0), N.ptr_at(k, k_col), k.stride(0), N.ptr_at(v, v_col), v.stride(0),
            N.dtype_code(v.dtype), N.ptr(decay), 1 if per_channel else 0, N.ptr(kscale), N.ptr(skip), float(qscale), N.ptr(state),
            N.ptr(pos_ids), N.ptr(y), B, T, H, qk_heads, n, p, 1 if unit_col else 0, N.stream())
