@@ -183,6 +183,13 @@ LL_API int ll_int4_gemv(const ll_gemv_args* args /* host */, ll_stream stream);
  * ------------------------------------------------------------------------------------- */
 LL_API int ll_gemm_bf16_tc(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, ll_stream stream);
 
+/* Many rows (prompts): y[M][N] = x[M][K] . W^T (+ bias) in bf16 with W de-quantised in the main loop from the CHECKPOINT bytes [K/2][N]
+ * (scales / zeros bf16 [N][K / group]), with the reference's bf16 rounding steps: what ll_get_weight + ll_gemm_bf16_tc compute, without the
+ * bf16 copy of W.  N % 16 == 0, group % 128 == 0, K % group == 0.  ll_int4_rows_error: as the other tcgen05 kernels' error queries. */
+LL_API int ll_int4_rows_supported(int N, int K, int group);
+LL_API int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K,
+                        int group, ll_stream stream);
+LL_API int ll_int4_rows_error(void);
 /* Fused int4 de-quantise + GEMM on tcgen05 for 1 <= M <= 128 rows (batched decode, short prefill; the HBM-bound regime):
  * y[M][N] (bf16) = x[M][K] (bf16) . W^T (+ bias), W de-quantised INSIDE the main loop from the packed stream
  * (w_stream = ll_int4_prepare(..., LL_STREAM_U8, ...), the batch-1 GEMV's stream) with the reference's bf16 rounding steps

@@ -4,7 +4,8 @@
 // get_weight(dtype=bf16), quantization.py:390-409), so the result is the reference's fallback branch
 // F.linear(inp, get_weight(inp.dtype)) (quantization.py:420-421) with fp32 accumulation - the branch the
 // reference takes for every grouped checkpoint and the semantics of its Triton kernel for per-row ones.
-// Used for prefill and batched decode (M >= 17); replaces Triton's mma.sync kernel (quantization.py:185-280).
+// Used for prefill of layers the many-row kernel (int4_rows.cu) does not take; replaces Triton's mma.sync kernel
+// (quantization.py:185-280).
 //
 // Structure (one 128 x BN output tile per CTA, 192 threads):
 //   warp 0   : TMA producer - 2-D tiled loads (128B swizzle) of X[128 x 64] and W[BN x 64] into a ring
@@ -167,10 +168,7 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, __nv_bfloat16* C, 
 // y[M][N] = x[M][K] . dequant(W)^T for 9 <= M <= 128 (batched decode, short prefill): the regime where the weights are
 // the traffic (HBM-bound), so they are streamed ONCE in their packed form and de-quantised inside the main loop - what the
 // reference's Triton kernel does (ref quantization.py:259-267: load nibble, (q - zero) * scale, tl.dot) - instead of
-// writing a bf16 copy of W to HBM and reading it back.  (For M in the thousands the same idea is counter-productive on
-// this machine: the tensor cores consume a 128-row tile's weights in K/16 * ~8 clk while de-quantising them costs
-// ~0.06 clk per weight of ALU time per SM, so every 128-row block of M would pay the de-quantisation again; there the
-// two-pass path above is within 3 % of the GEMM alone.  DESIGN.md section 3.)
+// writing a bf16 copy of W to HBM and reading it back.  (More rows: int4_rows.cu.)
 //
 //  * operand roles are swapped: the WEIGHTS are the A operand (128 output columns = the 128 TMEM lanes) and live in TENSOR
 //    MEMORY: each of 128 de-quantising threads owns one output column, reads its nibbles from the packed stream (kind 1,

@@ -152,9 +152,18 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         return buf if ok else None
 
     FUSED_GEMM_MAX_M = 128       # rows one ll_int4_gemm_tc call takes
-    # rows up to which the fused kernel is looped over 128-row blocks (each block streams the packed weights again) instead of
-    # unpacking W to bf16 once and running the plain tcgen05 GEMM (measured cross-over: profiles/r02_fused_gemm.md)
-    FUSED_GEMM_LOOP_MAX_M = int(__import__("os").environ.get("LLB200_FUSED_GEMM_MAX_M", 256))
+    # rows from which the weights are de-quantised in the main loop of the many-row kernel, from the checkpoint bytes.  Both sides measured
+    # (11008 x 4096, group 128): 130 rows 27 us against 61 in two passes of the small-row kernel and 87 with a bf16 copy of W; 512 rows
+    # 49 against 112; 2048 rows 137 against 220.
+    ROWS_MIN_M = 129
+
+    def _rows_eligible(self, x) -> bool:
+        """More than 128 bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns."""
+        s, z = self.scales, self.zeros
+        return (self.bits == 4 and x.dtype == torch.bfloat16 and s.dtype == torch.bfloat16 and z.dtype == torch.bfloat16
+                and (self.bias is None or self.bias.dtype == torch.bfloat16) and s.is_contiguous() and z.is_contiguous()
+                and (self.quant_weight.data_ptr() | x.data_ptr()) % 16 == 0
+                and bool(N.call_ret("ll_int4_rows_supported", self.out_features, self.in_features, self.tile_cols)))
 
     def _fused_gemm_eligible(self, x) -> bool:
         """9 <= M <= 128 bf16 rows on a layer whose scale groups are multiples of 128: the fused tcgen05 de-quantise + GEMM."""
@@ -192,9 +201,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             fast = self.prepare(M) is not None
         if fast:
             self._gemv(x, y)
-        elif M <= max(self.FUSED_GEMM_MAX_M, self.FUSED_GEMM_LOOP_MAX_M) and self.FUSED_GEMM_MAX_M > 0 \
-                and self._fused_gemm_eligible(x) and self._fused_gemm(x, y):
+        elif M <= self.FUSED_GEMM_MAX_M and self._fused_gemm_eligible(x) and self._fused_gemm(x, y):
             pass
+        elif M >= self.ROWS_MIN_M and self._rows_eligible(x):
+            N.call("ll_int4_rows", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), M, Nout, K,
+                   self.tile_cols, N.stream())
         elif M <= 16:
             assert inp.dtype in (torch.float32, torch.bfloat16)
             N.call("ll_qlinear_simt", N.ptr(x), N.dtype_code(x.dtype), M, N.ptr(qw), N.ptr(self.scales.contiguous()),
@@ -216,14 +227,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             w = self._prepare_kind(N.STREAM_U8)
         if w is None:
             return False
-        step = self.FUSED_GEMM_MAX_M
-        for r0 in range(0, x.shape[0], step):
-            xb, yb = x[r0:r0 + step], y[r0:r0 + step]
-            M = xb.shape[0]
-            nbytes = N.call_ret("ll_int4_gemm_tc_scratch_bytes", M, self.out_features, self.in_features)
-            scratch = _int8_workspace(x.device, nbytes) if nbytes else None
-            N.call("ll_int4_gemm_tc", N.ptr(w), N.ptr(xb), N.ptr(self.bias), N.ptr(yb), N.ptr(scratch), M, self.out_features,
-                   self.in_features, self.tile_cols, N.stream())
+        M = x.shape[0]
+        nbytes = N.call_ret("ll_int4_gemm_tc_scratch_bytes", M, self.out_features, self.in_features)
+        scratch = _int8_workspace(x.device, nbytes) if nbytes else None
+        N.call("ll_int4_gemm_tc", N.ptr(w), N.ptr(x), N.ptr(self.bias), N.ptr(y), N.ptr(scratch), M, self.out_features, self.in_features,
+               self.tile_cols, N.stream())
         return True
 
     def _gemv(self, x, y, *, pdl=False, grid=0):
@@ -238,7 +246,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
 
 def dequant_gemm(lin: ColBlockQuantizedLinear, x: torch.Tensor) -> torch.Tensor:
-    """Large-M path (prefill, batched decode): bit-exact de-quantisation of W into a bf16 scratch (the
+    """Large-M path of layers the many-row kernel does not take: bit-exact de-quantisation of W into a bf16 scratch (the
     reference's ``get_weight``) followed by the tcgen05/TMEM tensor-core GEMM - the reference's fallback
     branch (quantization.py:420-421) on the 5th-generation tensor cores.  fp32 activations (tests scale
     only) use the library GEMM."""

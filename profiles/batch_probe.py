@@ -17,7 +17,7 @@ dev = torch.device("cuda:0")
 model = bench.build_model(dev)
 if os.environ.get("LLB200_FUSED_GEMM") == "0":
     ColBlockQuantizedLinear.FUSED_GEMM_MAX_M = 0
-    ColBlockQuantizedLinear.FUSED_GEMM_LOOP_MAX_M = 0
+    ColBlockQuantizedLinear.ROWS_MIN_M = 1 << 30
 S, POS = 768, 640
 wbytes, _ = bench.algorithmic_bytes(model, 0)
 out = []
