@@ -224,8 +224,8 @@ LL_API int ll_int8_quantize_weight(const void* w /*[N][K]*/, int w_dtype, int8_t
 
 /* ref: bnb MatMul8bitLt forward (has_fp16_weights=False, threshold) as reached through quantization.py:36-45:
  * y[M][N] = int8 matmul of the row-quantised non-outlier part + fp16 outlier-column part (+ bias), in the
- * activation dtype.  K % 128 == 0.  workspace: ll_int8_workspace_bytes(M, N, K) bytes, 256-byte aligned; with those of min(M, 64) rows,
- * or x off 16-byte boundaries, M > 64 runs as passes of 64 rows (the same results: a feature is an outlier for a block of 64 rows). */
+ * activation dtype.  K % 128 == 0.  workspace: ll_int8_workspace_bytes(M, N, K) bytes, 256-byte aligned; with those of min(M, 64) rows
+ * M > 64 runs as passes of 64 rows (the same results: a feature is an outlier for a block of 64 rows). */
 LL_API size_t ll_int8_workspace_bytes(int M, int N, int K);
 /* 0, or the code of the first bounded wait that ran out in the tcgen05 product of ll_int8_linear (M > 64).  Synchronises the device. */
 LL_API int ll_int8_tc_error(void);

@@ -38,6 +38,44 @@ def test_rows_against_passes(M, N, K, dtype, outliers, bias, transposed):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("M", [1, 15, 16, 17, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("N,K", [(33, 128), (128, 384), (1000, 1024), (256, 4096 * 10)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_small_batches_against_64_bits(M, N, K, offset):
+    """Up to 64 rows: every padded row count, a last column tile that is not full, one and many ranges of k, a K whose preparation does not
+    fit a resident grid, activations off 16-byte boundaries."""
+    from lit_llama import _native as NV
+
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.empty(M * K + 8, dtype=torch.float16, device="cuda")[offset: offset + M * K].view(M, K)
+    x.copy_(torch.randn((M, K), generator=g, device="cuda"))
+    x[:, 5::97] *= 9.0
+    cb = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    scb = torch.rand(N, generator=g, device="cuda") + 0.5
+    ws = torch.full((NV.call_ret("ll_int8_workspace_bytes", M, N, K),), 0x5A, dtype=torch.uint8, device="cuda")
+    y = torch.empty((M, N), dtype=torch.float32, device="cuda")
+    xf = x.float()
+    ya, yf = torch.empty((M, N), dtype=torch.float16, device="cuda"), y
+    NV.call("ll_int8_linear", NV.ptr(x), NV.LL_F16, NV.ptr(cb), None, NV.ptr(scb), None, NV.ptr(ya), M, N, K, 6.0, NV.ptr(ws), ws.numel(), NV.stream())
+    NV.call("ll_int8_linear", NV.ptr(xf), NV.LL_F32, NV.ptr(cb), None, NV.ptr(scb), None, NV.ptr(yf), M, N, K, 6.0, NV.ptr(ws), ws.numel(), NV.stream())
+    torch.cuda.synchronize()
+    assert NV.call_ret("ll_int8_tc_error") == 0
+    assert torch.equal(ya.float(), yf)                                 # x.half() either way
+    a = x.double()
+    big = a.abs() >= 6.0
+    cols = big.any(0)
+    rest = a.masked_fill(big, 0.0)
+    sca = rest.abs().amax(1)
+    # (a tensor over a tensor: a number over a tensor is a product with its reciprocal, which may end on another code)
+    ca = torch.round((rest.float() * (torch.full_like(sca, 127.0).float() / sca.float())[:, None]).double()).masked_fill(cols[None], 0.0)
+    want = (ca @ cb.double().t()) * sca[:, None] * scb.double()[None] / 127.0 ** 2
+    wo = (cb.double()[:, cols] * scb.double()[:, None] / 127.0).half().double()
+    odd, size = a[:, cols] @ wo.t(), a[:, cols].abs() @ wo.abs().t()
+    # both parts and their sum rounded to fp16 (2^-11 of each); an outlier's weight may round to the other fp16 neighbour, where its fp32
+    # product (one rounding of SCB / 127, one of the product) sits on the other side of the middle: 2^-10 of the term
+    assert ((yf.double() - want - odd).abs() <= 2.0 ** -11 * (want.abs() + odd.abs() + (want + odd).abs()) * 1.01 + 2.0 ** -10 * size + 1e-4).all()
+
+
 def test_more_outliers_than_one_stage():
     from lit_llama.quantization import Linear8bitLt
 
@@ -53,7 +91,7 @@ def test_more_outliers_than_one_stage():
     cols[::3] = True
     rest = a.masked_fill(cols[None], 0.0)
     sca = rest.abs().amax(1)
-    ca = torch.round((rest.float() * (127.0 / sca.float())[:, None]).double())
+    ca = torch.round((rest.float() * (torch.full_like(sca, 127.0).float() / sca.float())[:, None]).double())
     want = (ca @ cb.t()) * sca[:, None] * scb[None] / 127.0 ** 2 + a[:, cols] @ (cb[:, cols] * scb[:, None] / 127.0).half().double().t()
     # fp16 roundings of the two parts and of their sum (2^-11 each of the largest value)
     assert (y - want).abs().max() <= 4 * 2.0 ** -11 * want.abs().max()
