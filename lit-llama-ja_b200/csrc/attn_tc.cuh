@@ -169,17 +169,6 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
   return r;
 }
 
-// One lane of the warp, the same one every time.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)::"memory");
-  return r != 0;
-}
-
 // A wait that ends: on its phase, when another role has given up, or after the limit.
 __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
   if (mbar_try_wait(bar, parity)) return true;

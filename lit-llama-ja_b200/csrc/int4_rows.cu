@@ -61,15 +61,6 @@ __device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, volatile
   atomicCAS(&g_r4_error, 0, code);
   return false;
 }
-__device__ __forceinline__ bool r4_elect() {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)::"memory");
-  return r != 0;
-}
 __device__ __forceinline__ void r4_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
                "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
@@ -140,7 +131,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
   const int steps = p.steps;
 
   if (warp == 0 || warp == 2) {
-    if (r4_elect()) {
+    if (elect_one()) {
       bool ok = true;
       int s = 0;
       uint32_t ph = 1;
@@ -167,7 +158,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
         for (int w = 0; w < 2048; ++w) __nanosleep(512);
     }
   } else if (warp == 1) {
-    if (r4_elect()) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc_bf16(R4_N, BN);
       const uint64_t xd = smem_desc_sw128(smem_u32(sx));
       bool ok = true;

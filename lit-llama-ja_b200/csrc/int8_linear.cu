@@ -176,15 +176,6 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ bool i8_elect() {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(r)::"memory");
-  return r != 0;
-}
 __device__ __forceinline__ void i8_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
                "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
@@ -217,7 +208,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   if (warp == 0) {
-    if (i8_elect()) {
+    if (elect_one()) {
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % I8_STAGES;
@@ -230,7 +221,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
         for (int w = 0; w < 2048; ++w) __nanosleep(512);
     }
   } else if (warp == 1) {
-    if (i8_elect()) {
+    if (elect_one()) {
       // D = int32 (2 at bit 4), A = B = signed int8 (1 at bits 7 and 10), both K-major
       constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
@@ -543,7 +534,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   if (warp == 0) {
-    if (i8_elect()) {
+    if (elect_one()) {
       bool ok = true;
       int s = 0;
       uint32_t ph = 1;
@@ -558,7 +549,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
         for (int w = 0; w < 2048; ++w) __nanosleep(512);
     }
   } else if (warp == 1) {
-    if (i8_elect()) {
+    if (elect_one()) {
       constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(MP >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       const uint64_t wd = smem_desc_sw128(smem_u32(sw)), xd = smem_desc_sw128(smem_u32(sx));
       bool ok = true;

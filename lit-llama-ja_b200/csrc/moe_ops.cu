@@ -17,13 +17,20 @@
 
 namespace llb {
 
-constexpr int RT_TOK = 4;        // tokens per routing block
 constexpr int RT_THREADS = 256;
+constexpr int RT_WIDE_M = 8 * 148, RT_NARROW_M = 149;
+constexpr size_t RT_WIDE_SMEM = 100 * 1024;   // two blocks a SM
 constexpr int RT_EG = 4;         // experts a warp accumulates side by side
 enum { SCORE_CHOSEN = 0, SCORE_ALL = 1, SCORE_SIGMOID = 2 };
 
-template <typename T>
-__global__ void __launch_bounds__(RT_THREADS) moe_route_kernel(const T* __restrict__ x, const float* __restrict__ w_router,
+// One block routes RT_TOK tokens and reads the whole router for them: bound by the latency of those reads while the blocks fit
+// the chip at once, and by their number (X * dim * 4 bytes a block, from L2) for long prompts.  So a token to a block while
+// every token gets its own SM (M < RT_NARROW_M), eight once every SM has a block of eight (RT_WIDE_M), four between; the sums
+// are the same numbers in every form.  32 experts of width 2048, us by M (one / four / eight tokens a block):
+// 148: 8.7 / 12.5, 300: 12.6 with four, 15.5 with eight, 1183: 15.2 / 17.2, 2048: 37 with four, 19 with eight; four tokens a
+// block at every M, with weights loaded where they are used: 16 at M = 1, 34 at 2048.
+template <typename T, int RT_TOK>
+__global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kernel(const T* __restrict__ x, const float* __restrict__ w_router,
                                                                const float* __restrict__ bias, int M, int dim, int X, int top,
                                                                int score, const float* __restrict__ correction, float out_scale,
                                                                int n_groups, int keep_groups, int group_top,
@@ -37,7 +44,17 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_kernel(const T* __restri
   const int m0 = blockIdx.x * RT_TOK;
   const int nt = min(RT_TOK, M - m0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int idx = tid; idx < nt * dim; idx += RT_THREADS) xs[idx] = dt<T>::ld(x, (size_t)m0 * dim + idx);
+  constexpr int V = 16 / sizeof(T);
+  const T* xr = x + (size_t)m0 * dim;
+  if (dim % V == 0 && ((uintptr_t)xr & 15) == 0) {      // 16-byte reads of the rows
+    for (int i = tid; i < nt * dim / V; i += RT_THREADS) {
+      const uint4 u = reinterpret_cast<const uint4*>(xr)[i];
+#pragma unroll
+      for (int j = 0; j < V; ++j) xs[i * V + j] = dt<T>::ld(reinterpret_cast<const T*>(&u), j);
+    }
+  } else {
+    for (int idx = tid; idx < nt * dim; idx += RT_THREADS) xs[idx] = dt<T>::ld(xr, idx);
+  }
   for (int idx = nt * dim + tid; idx < RT_TOK * dim; idx += RT_THREADS) xs[idx] = 0.f;
   __syncthreads();
   const bool vec4 = (dim % 4 == 0) && (((uintptr_t)w_router & 15) == 0);
@@ -48,18 +65,35 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_kernel(const T* __restri
     for (int g = 0; g < RT_EG; ++g)
 #pragma unroll
       for (int t = 0; t < RT_TOK; ++t) a[g][t] = 0.f;
-    if (vec4) {          // 16-byte weight loads, four steps unrolled: 16 independent loads in flight per lane
-#pragma unroll 4
-      for (int i4 = lane; i4 < dim / 4; i4 += 32) {
-        float4 w[RT_EG];
+    if (vec4) {          // 16-byte weight loads, the next group's in flight under the sums of this one
+      constexpr int U = RT_TOK > 1 ? 1 : 2;
+      const int n4 = dim / 4;
+      float4 w[2][U][RT_EG];
+      auto fetch = [&](float4 (&d)[U][RT_EG], int i0) {
 #pragma unroll
-        for (int g = 0; g < RT_EG; ++g) w[g] = ((const float4*)(w_router + (size_t)min(e0 + g, X - 1) * dim))[i4];
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int t = 0; t < RT_TOK; ++t) {
-          const float4 xv = ((const float4*)(xs + t * dim))[i4];
+          for (int g = 0; g < RT_EG; ++g)
+            d[u][g] = __ldg((const float4*)(w_router + (size_t)min(e0 + g, X - 1) * dim) + min(i0 + 32 * u, n4 - 1));
+      };
+      auto add = [&](const float4 (&d)[U][RT_EG], int i0) {
 #pragma unroll
-          for (int g = 0; g < RT_EG; ++g) a[g][t] += w[g].x * xv.x + w[g].y * xv.y + w[g].z * xv.z + w[g].w * xv.w;
+        for (int u = 0; u < U; ++u) {
+          if (i0 + 32 * u >= n4) break;
+#pragma unroll
+          for (int t = 0; t < RT_TOK; ++t) {
+            const float4 xv = ((const float4*)(xs + t * dim))[i0 + 32 * u];
+#pragma unroll
+            for (int g = 0; g < RT_EG; ++g) a[g][t] += d[u][g].x * xv.x + d[u][g].y * xv.y + d[u][g].z * xv.z + d[u][g].w * xv.w;
+          }
         }
+      };
+      fetch(w[0], lane);
+      for (int i = lane; i < n4; i += 64 * U) {
+        fetch(w[1], i + 32 * U);
+        add(w[0], i);
+        fetch(w[0], i + 64 * U);
+        add(w[1], i + 32 * U);
       }
     } else {
 #pragma unroll 4
@@ -147,13 +181,16 @@ __global__ void __launch_bounds__(RT_THREADS) moe_route_kernel(const T* __restri
         z[bi] = -INFINITY;
         expert_idx[(size_t)m * top + k] = bi;
         expert_w[(size_t)m * top + k] = p;                       // normalised below
-        rank[(size_t)m * top + k] = atomicAdd(&counts[bi], 1);
       }
       __syncwarp();
     }
     __syncwarp();
     if (score != SCORE_CHOSEN) denom += 1e-20f;
-    for (int k = lane; k < top; k += 32) expert_w[(size_t)m * top + k] = expert_w[(size_t)m * top + k] / denom * out_scale;
+    for (int k = lane; k < top; k += 32) {      // the places of all choices at once: one round trip to the counters
+      const size_t at = (size_t)m * top + k;
+      expert_w[at] = expert_w[at] / denom * out_scale;
+      rank[at] = atomicAdd(&counts[expert_idx[at]], 1);
+    }
   }
 }
 
@@ -428,6 +465,54 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
   }
 }
 
+// 16 bytes per access, the same sums: 2048 tokens of width 2048 with four choices and a shared expert, 21 us -> 9 (40 MB).
+template <typename T>
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const T* __restrict__ y, const float* __restrict__ expert_w, int top,
+                                                              const T* __restrict__ shared_y, int shared_ld,
+                                                              const T* __restrict__ shared_gate, int gate_ld, T* __restrict__ out, int M,
+                                                              int dim) {
+  constexpr int V = 16 / sizeof(T);
+  const int pieces = dim / V;
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (size_t)M * pieces) return;
+  const int m = (int)(idx / pieces), c = (int)(idx - (size_t)m * pieces) * V;
+  float v[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) v[j] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < top; ++k) {
+    const float w = expert_w[(size_t)m * top + k];
+    const uint4 u = __ldcs(reinterpret_cast<const uint4*>(y + ((size_t)m * top + k) * dim + c));
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] += w * dt<T>::ld(reinterpret_cast<const T*>(&u), j);
+  }
+  if (shared_y) {
+    const float sg = shared_gate ? 1.f / (1.f + expf(-dt<T>::ld(shared_gate, (size_t)m * gate_ld))) : 1.f;
+    const uint4 u = *reinterpret_cast<const uint4*>(shared_y + (size_t)m * shared_ld + c);
+#pragma unroll
+    for (int j = 0; j < V; ++j) v[j] += sg * dt<T>::ld(reinterpret_cast<const T*>(&u), j);
+  }
+  uint4 o;
+#pragma unroll
+  for (int j = 0; j < V; ++j) dt<T>::st(reinterpret_cast<T*>(&o), j, v[j]);
+  *reinterpret_cast<uint4*>(out + (size_t)m * dim + c) = o;
+}
+
+// Rows in whole 16-byte pieces take the wide form; odd widths and shifted rows go element by element.
+template <typename T>
+static void launch_combine(const void* y, const float* expert_w, int top, const void* shared_y, int shared_ld, const void* shared_gate,
+                           int gate_ld, void* out, int M, int dim, cudaStream_t st) {
+  constexpr int V = 16 / sizeof(T);
+  if (dim % V == 0 && (!shared_y || shared_ld % V == 0) && (((uintptr_t)y | (uintptr_t)shared_y | (uintptr_t)out) & 15) == 0) {
+    const size_t n = (size_t)M * (dim / V);
+    moe_combine_vec_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const T*)y, expert_w, top, (const T*)shared_y, shared_ld,
+                                                                        (const T*)shared_gate, gate_ld, (T*)out, M, dim);
+  } else {
+    moe_combine_kernel<T><<<M, dim >= 1024 ? 256 : 128, 0, st>>>((const T*)y, expert_w, top, (const T*)shared_y, shared_ld,
+                                                                (const T*)shared_gate, gate_ld, (T*)out, dim);
+  }
+}
+
 template <typename T, int TM, int MODE>
 static int launch_grouped(const void* a, int lda, const void* w, const int32_t* offsets, const int32_t* perm, int top, int X, int N,
                           int K, float limit, float alpha, float shift, void* c, int ldc, int n_rows, cudaStream_t st) {
@@ -477,18 +562,22 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
                "moe_route: %d groups (keep %d) of %d experts cannot give %d choices", n_groups, keep_groups, n_experts, top);
   if (M == 0) return LL_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t smem =
-      sizeof(float) * RT_TOK * ((size_t)dim + (score == SCORE_SIGMOID ? 2 : 1) * (size_t)n_experts + 2 * (size_t)n_groups);
-  if (smem > 200 * 1024) {
+  const size_t per_token =
+      sizeof(float) * ((size_t)dim + (score == SCORE_SIGMOID ? 2 : 1) * (size_t)n_experts + 2 * (size_t)n_groups);
+  if (4 * per_token > 200 * 1024) {
     set_error("moe_route: width %d with %d experts does not fit shared memory", dim, n_experts);
     return LL_ERR_UNSUPPORTED;
   }
   LL_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * n_experts, st));
-  const int blocks = (M + RT_TOK - 1) / RT_TOK;
+  const int tok = M >= RT_WIDE_M && 8 * per_token <= RT_WIDE_SMEM ? 8 : M < RT_NARROW_M ? 1 : 4;
+  const int blocks = (M + tok - 1) / tok;
+  const size_t smem = tok * per_token;
+#define LL_RT_TOK(T, TOK)                                                                                                            \
+  LL_CUDA(cudaFuncSetAttribute(moe_route_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));                  \
+  moe_route_kernel<T, TOK><<<blocks, RT_THREADS, smem, st>>>((const T*)x, w_router, bias, M, dim, n_experts, top, score, correction,  \
+                                                             out_scale, n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank)
 #define LL_RT(T)                                                                                                                     \
-  LL_CUDA(cudaFuncSetAttribute(moe_route_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));                       \
-  moe_route_kernel<T><<<blocks, RT_THREADS, smem, st>>>((const T*)x, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, \
-                                                        n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank)
+  if (tok == 8) { LL_RT_TOK(T, 8); } else if (tok == 4) { LL_RT_TOK(T, 4); } else { LL_RT_TOK(T, 1); }
   if (dtype == LL_F32) {
     LL_RT(float);
   } else if (dtype == LL_BF16) {
@@ -498,6 +587,7 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
     return LL_ERR_UNSUPPORTED;
   }
 #undef LL_RT
+#undef LL_RT_TOK
   LL_LAUNCH_OK("moe_route_kernel");
   const int n_pairs = M * top;
   moe_permute_kernel<<<(n_pairs + 255) / 256, 256, sizeof(int32_t) * (n_experts + 1), st>>>(expert_idx, rank, counts, n_pairs,
@@ -540,14 +630,10 @@ int ll_moe_combine(const void* y, const float* expert_w, int top, const void* sh
   LL_CHECK_ARG(y && expert_w && out && top > 0 && M >= 0 && dim > 0, "bad moe_combine arguments");
   if (M == 0) return LL_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int threads = dim >= 1024 ? 256 : 128;
   if (dtype == LL_F32)
-    moe_combine_kernel<float><<<M, threads, 0, st>>>((const float*)y, expert_w, top, (const float*)shared_y, shared_ld,
-                                                    (const float*)shared_gate, gate_ld, (float*)out, dim);
+    launch_combine<float>(y, expert_w, top, shared_y, shared_ld, shared_gate, gate_ld, out, M, dim, st);
   else if (dtype == LL_BF16)
-    moe_combine_kernel<__nv_bfloat16><<<M, threads, 0, st>>>((const __nv_bfloat16*)y, expert_w, top, (const __nv_bfloat16*)shared_y,
-                                                            shared_ld, (const __nv_bfloat16*)shared_gate, gate_ld,
-                                                            (__nv_bfloat16*)out, dim);
+    launch_combine<__nv_bfloat16>(y, expert_w, top, shared_y, shared_ld, shared_gate, gate_ld, out, M, dim, st);
   else {
     set_error("moe_combine: unsupported dtype %d", dtype);
     return LL_ERR_UNSUPPORTED;
