@@ -44,7 +44,6 @@ struct AttnTcArgs {
   int gate_ld, gate_per_head;
   float scale, softcap;
   int B, T, H, G, window, chunk, ring;
-  int slots;                   // 1: key slot s is visible where s <= position (a cache that is not a ring of positions)
   int terms;                   // bf16 terms of a softmax weight: 1 or 2
   void* y;                     // bf16 [B * T] rows, head h at column h * v.dim
   int y_ld;
@@ -65,7 +64,7 @@ struct AtParams {
   const __nv_bfloat16* gate;
   __nv_bfloat16* y;
   float scale, softcap;
-  int T, H, group, vdim, window, chunk, ring, slots, gate_ld, gate_per_head, gate_vec, y_ld;
+  int T, H, group, vdim, window, chunk, ring, gate_ld, gate_per_head, gate_vec, y_ld;
 };
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -290,13 +289,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   }
   __syncthreads();
   // what every role walks: key blocks from kt0 to the last visible key; per tile the part of it that its rows see
-  const int step_last = p.slots ? p.ring - 1 : __shfl_sync(0xffffffffu, p.pos_ids[p.T - 1], 0);     // rows after this key hold nothing of this step
+  const int step_last = __shfl_sync(0xffffffffu, p.pos_ids[p.T - 1], 0);     // rows after this key hold nothing of this step
   int lo[2], hi[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int first = __shfl_sync(0xffffffffu, s_range[2 * i], 0), end = __shfl_sync(0xffffffffu, s_range[2 * i + 1], 0);
     lo[i] = end >= 0 ? at_first_visible(first, p.window, p.chunk) : INT_MAX;
-    hi[i] = end >= 0 && p.slots ? min(end, p.ring - 1) : end;
+    hi[i] = end;
   }
   const int kt0 = min(lo[0], lo[1]), last = max(hi[0], hi[1]);
 
@@ -413,7 +412,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     const uint32_t ts0 = tmem + lanes + TM_S + 128u * tile, to = tmem + lanes + TM_O + 128u * tile;
     const int mylo = tile == 0 ? lo[0] : lo[1], myhi = tile == 0 ? hi[0] : hi[1];
     const int qlo = at_first_visible(qp, p.window, p.chunk);
-    const int qhi = p.slots ? min(qp, p.ring - 1) : qp;
     const float cap2 = CAP ? p.softcap * AT_LOG2E : 0.f;
     // what a raw score is multiplied by: to the argument of tanh, or to units of log2 (a biased score has been brought there)
     const float mul = BIAS ? 1.f : CAP ? p.scale / p.softcap : p.scale * AT_LOG2E;
@@ -441,7 +439,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
           for (int e = 0; e < AT_C; ++e) sr[e] = __float_as_uint(fmaf(slope, d0 + (float)e, __uint_as_float(sr[e]) * k));
         }
-        const int cmin = qlo - c0, cmax = min(blk.rows - 1 - AT_C * half, qhi - c0);          // visible columns of this row
+        const int cmin = qlo - c0, cmax = min(blk.rows - 1 - AT_C * half, qp - c0);          // visible columns of this row
         const bool masked = __any_sync(0xffffffffu, cmin > 0 || cmax < AT_C - 1);
         float amx = 0.f;
         if (masked) {
@@ -659,21 +657,19 @@ bool attn_tc_supported(const AttnTcArgs& a) {
          a.y_ld % 8 == 0 && ((uintptr_t)a.y & 15) == 0 && (a.terms == 1 || a.terms == 2);
 }
 
-enum AttnTcKind { AT_PLAIN, AT_ROTARY, AT_LATENT };     // which forms a file instantiates
+enum AttnTcKind { AT_ROTARY, AT_LATENT };     // which forms a file instantiates
 
 template <AttnTcKind KIND>
 int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
   const AtParams p{a.pos_ids, a.sink, a.slopes, (const __nv_bfloat16*)a.gate, (__nv_bfloat16*)a.y, a.scale, a.softcap, a.T, a.H, a.H / a.G,
-                   a.v.dim, a.window, a.chunk, a.ring, a.slots, a.gate_ld, a.gate_per_head,
+                   a.v.dim, a.window, a.chunk, a.ring, a.gate_ld, a.gate_per_head,
                    a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
   const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \
   if (nb == N1 && two == (N2 > 0) && nbv == NV && a.terms == TERMS && cap == CC && bias == BB) return at_launch<N1, N2, NV, TERMS, CC, BB>(a, p, st);
 #define LL_AT_SIZES(N2, TERMS, CC, BB) LL_AT(1, N2, 1, TERMS, CC, BB) LL_AT(1, N2, 2, TERMS, CC, BB) LL_AT(2, N2, 1, TERMS, CC, BB) LL_AT(2, N2, 2, TERMS, CC, BB)
-  if constexpr (KIND == AT_PLAIN) {
-    LL_AT(1, 0, 1, 1, false, false) LL_AT(2, 0, 2, 1, false, false)
-  } else if constexpr (KIND == AT_ROTARY) {
+  if constexpr (KIND == AT_ROTARY) {
     LL_AT_SIZES(0, 2, false, false) LL_AT_SIZES(0, 2, true, false) LL_AT_SIZES(0, 2, false, true) LL_AT_SIZES(0, 2, true, true)
   } else {
     LL_AT_SIZES(1, 1, false, false) LL_AT_SIZES(1, 2, false, false)
