@@ -155,7 +155,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     # rows from which the weights are de-quantised in the main loop of the many-row kernel, from the checkpoint bytes.  Both sides measured
     # (11008 x 4096, group 128): 130 rows 27 us against 61 in two passes of the small-row kernel and 87 with a bf16 copy of W; 512 rows
     # 49 against 112; 2048 rows 137 against 220.
-    ROWS_MIN_M = 129
+    # Past 8192 rows a long run of products is held by the power limit, and a tile of W is de-quantised again for every 256 rows: the
+    # bf16 copy, written once, then costs less.  us, this kernel / copy and product, 150 ms of each in turn: 13824 x 5120 at 8192 rows
+    # 1067 / 1342, at 16384 2350 / 2618; 5120 x 13824: 1033 / 1160 and 2365 / 2245; 4096 x 11008: 682 / 713 and 1522 / 1380; 11008 x 4096:
+    # 741 / 856 and 1746 / 1678.
+    ROWS_MIN_M, ROWS_MAX_M = 129, 8192
 
     def _rows_eligible(self, x) -> bool:
         """More than 128 bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns."""
@@ -203,7 +207,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             self._gemv(x, y)
         elif M <= self.FUSED_GEMM_MAX_M and self._fused_gemm_eligible(x) and self._fused_gemm(x, y):
             pass
-        elif M >= self.ROWS_MIN_M and self._rows_eligible(x):
+        elif self.ROWS_MIN_M <= M <= self.ROWS_MAX_M and self._rows_eligible(x):
             N.call("ll_int4_rows", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), M, Nout, K,
                    self.tile_cols, N.stream())
         elif M <= 16:

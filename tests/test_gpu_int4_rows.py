@@ -54,3 +54,19 @@ def test_module_route_and_refusals():
     x = torch.randn((300, 256), generator=g, device="cuda").to(torch.bfloat16)
     want = x.float() @ lin.get_weight(torch.float32).t()
     assert (lin(x).float() - want).abs().max() <= 2.0 ** -7 * want.abs().max()
+
+
+@pytest.mark.parametrize("M", [8192, 8193])
+def test_longest_steps(M):
+    """The last step of the kernel and the first one of the unpacked copy."""
+    from lit_llama.quantization import ColBlockQuantizedLinear
+
+    g = torch.Generator(device="cuda").manual_seed(M)
+    lin = ColBlockQuantizedLinear(256, 144, False, bits=4, tile_cols=128).to("cuda", torch.bfloat16)
+    lin.quant_weight.copy_(torch.randint(0, 256, lin.quant_weight.shape, generator=g, device="cuda", dtype=torch.uint8))
+    lin.scales.fill_(0.01)
+    lin.zeros.fill_(8.0)
+    x = torch.randn((M, 256), generator=g, device="cuda").to(torch.bfloat16)
+    w = lin.get_weight(torch.bfloat16).double()
+    want, size = x.double() @ w.t(), x.double().abs() @ w.abs().t()
+    assert ((lin(x).double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 256 * 2.0 ** -24 + 1e-30).all()
