@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ 
                                                           T* __restrict__ y, int n_head, int S, int nsplit,
                                                           float* __restrict__ scratch, int32_t* __restrict__ counters,
                                                           int use_pdl, unsigned long long* __restrict__ trace) {
-#ifdef LLB_TRACE  // tuning build: %globaltimer stamps per CTA (profiles/attn_trace.py)
+#ifdef LLB_TRACE  // tuning build: %globaltimer stamps per CTA
 #define ATRACE(i)                                                                                     \
   do {                                                                                                \
     if (trace != nullptr && threadIdx.x == 0) {                                                       \

@@ -90,7 +90,7 @@ __device__ __forceinline__ unsigned long long gtimer() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// stage stamps for profiles/gemv_trace.py: only in the tuning build (build.py --variant trace LLB_TRACE=1) - the
+// stage stamps: only in the tuning build (build.py --variant trace LLB_TRACE=1) - the
 // stamps are code every launch would have to fetch
 #ifdef LLB_TRACE
 #define TRACE(i)                                                                   \
