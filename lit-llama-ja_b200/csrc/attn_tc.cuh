@@ -530,11 +530,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         for (int e = 0; e < 16; ++e) {
           const float p0 = at_exp2(__uint_as_float(sr[2 * e])), p1 = at_exp2(__uint_as_float(sr[2 * e + 1]));
           const f2 pp = f2_of(p0, p1);
-          sum2[e & 1] = f2_add(sum2[e & 1], pp);
           ph[e] = pack_bf16(p0, p1);
+          const f2 hi = f2_of(__uint_as_float(ph[e] << 16), __uint_as_float(ph[e] & 0xffff0000u));
+          // the sum is of the weights as the product sees them: with one term (8 bits) their rounding would not cancel in the quotient
+          sum2[e & 1] = f2_add(sum2[e & 1], TERMS == 1 ? hi : pp);
           if (TERMS == 2) {
             float l0, l1;
-            f2_split(f2_fma(f2_of(__uint_as_float(ph[e] << 16), __uint_as_float(ph[e] & 0xffff0000u)), f2_of(-1.f, -1.f), pp), l0, l1);
+            f2_split(f2_fma(hi, f2_of(-1.f, -1.f), pp), l0, l1);
             pl[e] = pack_bf16(l0, l1);
           }
         }

@@ -90,3 +90,27 @@ def test_latent_prompt_expanded_against_latent_space(T, past, S, window, terms, 
     # over a row's sum leaves about 2^-8 of it, twice
     assert torch.isfinite(outs[0]).all()
     assert (outs[0] - outs[1]).norm() <= 2.0 ** -6.5 * outs[1].norm()
+
+
+@pytest.mark.parametrize("T,S,window", [(16, 16, 0), (129, 129, 0), (300, 512, 100)])
+@pytest.mark.parametrize("terms", [1, 2])
+@pytest.mark.parametrize("scale", [0.02, 0.2])
+def test_weights_add_up_to_what_they_are_divided_by(T, S, window, terms, scale):
+    """Values that are all 1 come back as 1: the sum a row is divided by is that of the weights the product saw.  The fp32 sums on both sides
+    are off by a few 2^-24 of T numbers, two terms by 2^-17: well inside the half step of bf16 below 1 (2^-9)."""
+    from lit_llama import _native as N
+
+    B, H, nope, rot, v, rank = 2, 3, 64, 32, 64, 64
+    g = torch.Generator(device="cuda").manual_seed(T)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    q, k, cache = rnd(B * T, H * (nope + rot)), rnd(B * S, H * nope), rnd(B, S, rank + rot)
+    ones = torch.ones((H, B * S, v), dtype=torch.bfloat16, device="cuda")
+    pos = torch.arange(T, dtype=torch.int32, device="cuda")
+    rope = torch.tensor([1.0, 0.0], device="cuda").repeat(T, rot // 2).contiguous()
+    q_rot, y = torch.empty((B * T, H, rot), dtype=torch.bfloat16, device="cuda"), torch.zeros((B * T, H * v), dtype=torch.bfloat16, device="cuda")
+    N.call("ll_latent_prompt_attn", N.ptr(q), q.stride(0), nope, nope + rot, None, 0, N.ptr(rope), N.ptr(pos), N.ptr(k), k.stride(0), nope,
+           N.ptr(ones), v, B * S * v, N.ptr(cache), N.ptr(q_rot), N.ptr(y), y.stride(0), B, T, H, rank, rot, rot, v, S, window, scale, terms,
+           N.stream())
+    torch.cuda.synchronize()
+    assert N.call_ret("ll_latent_prompt_error") == 0
+    assert bool((y == 1.0).all())
