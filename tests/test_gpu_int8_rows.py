@@ -95,3 +95,30 @@ def test_more_outliers_than_one_stage():
     want = (ca @ cb.t()) * sca[:, None] * scb[None] / 127.0 ** 2 + a[:, cols] @ (cb[:, cols] * scb[:, None] / 127.0).half().double().t()
     # fp16 roundings of the two parts and of their sum (2^-11 each of the largest value)
     assert (y - want).abs().max() <= 4 * 2.0 ** -11 * want.abs().max()
+
+
+def test_small_batches_on_many_streams():
+    """A call's kernels wait for no block that may not be running: rows of 35840 features on twelve streams at once, more blocks than the
+    device holds together, give what one stream after the other gives."""
+    from lit_llama import _native as NV
+
+    g = torch.Generator(device="cuda").manual_seed(11)
+    M, N, K, S = 5, 40, 35840, 12
+    x = torch.randn((S, M, K), generator=g, device="cuda").to(torch.bfloat16)
+    x[:, 1::2, 7::501] *= 20.0                                         # outliers in some rows
+    cb = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    scb = torch.rand(N, generator=g, device="cuda") + 0.5
+    need = NV.call_ret("ll_int8_workspace_bytes", M, N, K)
+    ws = torch.full((S, (need + 255) // 256 * 256), 0x5A, dtype=torch.uint8, device="cuda")
+    outs = []
+    for streams in ([torch.cuda.Stream() for _ in range(S)], [torch.cuda.current_stream()] * S):
+        y = torch.zeros((S, M, N), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        for _ in range(5):
+            for i, st in enumerate(streams):
+                NV.call("ll_int8_linear", NV.ptr(x[i]), NV.LL_BF16, NV.ptr(cb), None, NV.ptr(scb), None, NV.ptr(y[i]), M, N, K, 6.0, NV.ptr(ws[i]),
+                        ws.shape[1], st.cuda_stream)
+        torch.cuda.synchronize()
+        outs.append(y)
+    assert NV.call_ret("ll_int8_tc_error") == 0
+    assert torch.equal(outs[0], outs[1]) and bool(outs[0].any())
