@@ -269,54 +269,132 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
   }
 }
 
-// out = fp16(C32 SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part, for 64 columns x 16 R rows (of one outlier list) per CTA: a thread
-// owns four columns of R rows; the weights and activations of up to 32 outliers at a time are staged as fp32, already rounded.  C32 is the
-// sum of `parts` partial sums, `part` numbers apart.
-constexpr int I8F_L = 32;
-template <typename T, int R>
-__global__ void __launch_bounds__(256) int8_finish_rows_kernel(const int32_t* __restrict__ c32, int parts, size_t part, const float* __restrict__ sca,
+// out = fp16(C32 SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part, for 64 columns x ROWS rows (of one outlier list) per CTA.  C32 is
+// the sum of `parts` partial sums, `part` numbers apart.
+// Outlier part: the weights and activations of L outliers at a time stand in shared memory as fp32, already rounded; the next L are asked
+// for (all list entries, then all they point to) before these are added.  64 rows: a thread owns four columns of four rows, two 16-byte
+// reads for 16 multiply-adds.  16 rows: a list of up to L is added by a thread per row and four columns; a longer one is shared among the
+// quarters of the threads, four columns of four rows each, a quarter of every L, whose sums are added in order.  Four CTAs an SM:
+// a batch of 64 rows has 688 of them for 11008 columns.
+// Three layers of a 4096-wide feed-forward, 32 rows whose inputs have 6 / 30 / 100 / 200 outlier features (their products up to thousands):
+// 78 / 121 / 424 / 519 us a call on the device.  32 outliers at a time, each weight behind its own list entry: 78 / 259 / 1725 / 2131; the
+// kernel beside the mma.sync product: 123 / 181 / 536 / 647.  (A stage of 128 leaves three CTAs an SM: 87 with 12 outliers, 84 with 64.)
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t* __restrict__ c32, int parts, size_t part, const float* __restrict__ sca,
                                                               const float* __restrict__ scb, const T* __restrict__ bias, const T* __restrict__ x,
                                                               const int8_t* __restrict__ cb, const int8_t* __restrict__ cbt,
                                                               const int32_t* __restrict__ idx, const int32_t* __restrict__ count,
                                                               T* __restrict__ y, int M, int N, int K) {
-  __shared__ __align__(16) float w_s[I8F_L][64], a_s[I8F_L][16 * R];
-  const int n0 = blockIdx.x * 64, m0 = blockIdx.y * 16 * R, blk = m0 / 64;
-  const int col = (threadIdx.x & 15) * 4, r0 = (threadIdx.x >> 4) * R;
+  static_assert(ROWS == 16 || ROWS == 64, "rows of a CTA");
+  constexpr int SL = 64 / ROWS, L = SL == 1 ? 32 : 64, NW = L * 16 / 256, NA = L * ROWS / 256;      // SL: shares of the list
+  __shared__ __align__(16) float w_s[L][64], a_s[L][ROWS];
+  const int tid = threadIdx.x, n0 = blockIdx.x * 64, m0 = blockIdx.y * ROWS, blk = m0 / 64, col = (tid & 15) * 4;
   const int cnt = count[blk];
-  const int32_t* list = idx + (size_t)blk * K;
-  float acc[R][4];
+  float acc[4][4];
 #pragma unroll
-  for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
-  for (int b = 0; b < cnt; b += I8F_L) {
-    const int ni = min(I8F_L, cnt - b);
-    __syncthreads();
-    for (int e = threadIdx.x; e < ni * 64; e += 256) {
-      const int i = e >> 6, j = e & 63, k = list[b + i], n = n0 + j;
-      float wv = 0.f;
-      if (n < N) {
-        const int8_t q = cbt != nullptr ? cbt[(size_t)k * N + n] : cb[(size_t)n * K + k];
-        wv = __half2float(__float2half_rn(__fmul_rn((float)q, __fdiv_rn(scb[n], 127.f))));
+  for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+  if (cnt > 0) {
+    const int32_t* list = idx + (size_t)blk * K;
+    // what a thread brings: four columns of NW outliers' weights, one row of NA outliers' activations.  Entries past the list's end, columns
+    // past N and rows past M repeat the last one: they are never added, or added to what nobody stores.
+    const int wi = tid >> 4, ai = tid / ROWS;
+    const T* xr = x + (size_t)min(m0 + (tid & (ROWS - 1)), M - 1) * K;
+    const bool words = cbt != nullptr && (N & 3) == 0 && ((uintptr_t)cbt & 3) == 0;
+    float sb127[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn(scb[min(n0 + col + j, N - 1)], 127.f);
+    uint32_t q[NW];
+    float av[NA];
+    auto fetch = [&](int b) {
+      int kw[NW], ka[NA];
+#pragma unroll
+      for (int u = 0; u < NW; ++u) kw[u] = __ldg(list + min(b + wi + 16 * u, cnt - 1));
+#pragma unroll
+      for (int u = 0; u < NA; ++u) ka[u] = __ldg(list + min(b + ai + (256 / ROWS) * u, cnt - 1));
+      if (words) {
+        const int8_t* src = cbt + min(n0 + col, N - 4);
+#pragma unroll
+        for (int u = 0; u < NW; ++u) q[u] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)kw[u] * N));
+      } else {
+#pragma unroll
+        for (int u = 0; u < NW; ++u) {
+          q[u] = 0u;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int n = min(n0 + col + j, N - 1);
+            const int8_t v = cbt != nullptr ? __ldg(cbt + (size_t)kw[u] * N + n) : __ldg(cb + (size_t)n * K + kw[u]);
+            q[u] |= (uint32_t)(uint8_t)v << (8 * j);
+          }
+        }
       }
-      w_s[i][j] = wv;
-    }
-    for (int e = threadIdx.x; e < ni * 16 * R; e += 256) {
-      const int i = e / (16 * R), j = e - i * (16 * R);
-      a_s[i][j] = m0 + j < M ? to_half_f32<T>(x[(size_t)(m0 + j) * K + list[b + i]]) : 0.f;
-    }
-    __syncthreads();
-    for (int i = 0; i < ni; ++i) {
-      const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const float a = a_s[i][r0 + r];
-        acc[r][0] = fmaf(a, w.x, acc[r][0]);
-        acc[r][1] = fmaf(a, w.y, acc[r][1]);
-        acc[r][2] = fmaf(a, w.z, acc[r][2]);
-        acc[r][3] = fmaf(a, w.w, acc[r][3]);
+      for (int u = 0; u < NA; ++u) av[u] = to_half_f32<T>(xr[ka[u]]);
+    };
+    auto stage = [&]() {
+#pragma unroll
+      for (int u = 0; u < NW; ++u) {
+        float w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = __half2float(__float2half_rn(__fmul_rn((float)(int8_t)(q[u] >> (8 * j)), sb127[j])));
+        *reinterpret_cast<float4*>(&w_s[wi + 16 * u][col]) = make_float4(w[0], w[1], w[2], w[3]);
+      }
+#pragma unroll
+      for (int u = 0; u < NA; ++u) a_s[ai + (256 / ROWS) * u][tid & (ROWS - 1)] = av[u];
+    };
+    fetch(0);
+    if (SL > 1 && cnt <= L) {
+      stage();
+      __syncthreads();
+      const int row = tid >> 4;
+#pragma unroll 4
+      for (int i = 0; i < cnt; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]);
+        const float a = a_s[i][row];
+        acc[0][0] = fmaf(a, w.x, acc[0][0]);
+        acc[0][1] = fmaf(a, w.y, acc[0][1]);
+        acc[0][2] = fmaf(a, w.z, acc[0][2]);
+        acc[0][3] = fmaf(a, w.w, acc[0][3]);
+      }
+    } else {
+      const int r0 = ((tid >> 4) & (ROWS / 4 - 1)) * 4, sl = tid / (256 / SL);
+      for (int b = 0; b < cnt; b += L) {
+        if (b > 0) __syncthreads();                        // the outliers before have been added
+        stage();
+        __syncthreads();
+        if (b + L < cnt) fetch(b + L);
+        const int i0 = sl * (L / SL), i1 = min(min(L, cnt - b), i0 + L / SL);
+#pragma unroll 4
+        for (int i = i0; i < i1; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]), a4 = *reinterpret_cast<const float4*>(&a_s[i][r0]);
+          const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            acc[r][0] = fmaf(a[r], w.x, acc[r][0]);
+            acc[r][1] = fmaf(a[r], w.y, acc[r][1]);
+            acc[r][2] = fmaf(a[r], w.z, acc[r][2]);
+            acc[r][3] = fmaf(a[r], w.w, acc[r][3]);
+          }
+        }
+      }
+      if (SL > 1) {                                        // every thread finishes one row: its sums come through shared memory
+        __syncthreads();
+        float* sums = &w_s[0][0];                          // [SL][ROWS][64]
+#pragma unroll
+        for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(sums + (sl * ROWS + r0 + r) * 64 + col) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        __syncthreads();
+        const int row = tid >> 4;
+        float4 o = *reinterpret_cast<const float4*>(sums + row * 64 + col);
+#pragma unroll
+        for (int z = 1; z < SL; ++z) {
+          const float4 v = *reinterpret_cast<const float4*>(sums + (z * ROWS + row) * 64 + col);
+          o.x += v.x, o.y += v.y, o.z += v.z, o.w += v.w;
+        }
+        acc[0][0] = o.x, acc[0][1] = o.y, acc[0][2] = o.z, acc[0][3] = o.w;
       }
     }
   }
-  const int n = n0 + col;
+  constexpr int R = ROWS / 16;                             // rows a thread finishes
+  const int n = n0 + col, fr = (tid >> 4) * R;
   if (n >= N) return;
   float sb[4], bv[4];
 #pragma unroll
@@ -327,7 +405,7 @@ __global__ void __launch_bounds__(256) int8_finish_rows_kernel(const int32_t* __
   const bool vec = n + 4 <= N && (N & 3) == 0;             // (then a partial sum starts on a 16-byte boundary too)
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int m = m0 + r0 + r;
+    const int m = m0 + fr + r;
     if (m >= M) break;
     const float sa = sca[m];
     const size_t at = (size_t)m * N + n;
@@ -413,7 +491,7 @@ int int8_rows_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* sc
     int8_lists_kernel<<<blocks, 1024, 0, st>>>(w.flag, w.idx, w.count, K);
     if (int r = make_map_i8(w.ca, rows, K, 128, &ma)) return r;
     int8_gemm_tc_kernel<<<dim3((rows + BM - 1) / BM, (N + I8_BN - 1) / I8_BN), 192, smem, st>>>(ma, mb, w.c32, rows, N, K);
-    int8_finish_rows_kernel<T, 4><<<dim3((N + 63) / 64, blocks), 256, 0, st>>>(w.c32, 1, 0, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count,
+    int8_finish_rows_kernel<T, 64><<<dim3((N + 63) / 64, blocks), 256, 0, st>>>(w.c32, 1, 0, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count,
                                                                            y + (size_t)r0 * N, rows, N, K);
     LL_LAUNCH_OK("int8 linear kernels (prompts)");
   }
@@ -688,7 +766,7 @@ int int8_linear_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* 
     else r = i8c_launch<64>(mw, w, Mp, N, K, sms, st);
     if (r) return r;
     int per;
-    int8_finish_rows_kernel<T, 1><<<dim3((N + 63) / 64, (Mp + 15) / 16), 256, 0, st>>>(
+    int8_finish_rows_kernel<T, 16><<<dim3((N + 63) / 64, (Mp + 15) / 16), 256, 0, st>>>(
         w.part, i8c_ranges(N, K, sms, &per), (size_t)Mp * N, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count, y + (size_t)m0 * N, Mp, N, K);
     LL_LAUNCH_OK("int8_finish_rows_kernel");
   }

@@ -122,3 +122,37 @@ def test_small_batches_on_many_streams():
         outs.append(y)
     assert NV.call_ret("ll_int8_tc_error") == 0
     assert torch.equal(outs[0], outs[1]) and bool(outs[0].any())
+
+
+@pytest.mark.parametrize("M", [1, 16, 33, 64, 70])
+@pytest.mark.parametrize("outliers", [1, 32, 64, 65, 96, 128, 129, 300])
+@pytest.mark.parametrize("N,transposed", [(70, True), (64, False)])
+def test_long_outlier_lists(M, outliers, N, transposed):
+    """Lists that end inside a share, at its end, inside a stage and after several stages."""
+    from lit_llama import _native as NV
+
+    g = torch.Generator(device="cuda").manual_seed(M + outliers)
+    K = 384
+    cols = torch.randperm(K, generator=g, device="cuda")[:outliers]
+    x = torch.randn((M, K), generator=g, device="cuda").clamp(-4, 4)
+    x[:, cols] = torch.sign(x[:, cols]) * (6.0 + 3.0 * x[:, cols].abs())
+    x = x.half()
+    cb = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    cbt = cb.t().contiguous() if transposed else None
+    scb = torch.rand(N, generator=g, device="cuda") + 0.5
+    ws = torch.full((NV.call_ret("ll_int8_workspace_bytes", M, N, K),), 0x5A, dtype=torch.uint8, device="cuda")
+    y = torch.empty((M, N), dtype=torch.float32, device="cuda")
+    xf = x.float()
+    NV.call("ll_int8_linear", NV.ptr(xf), NV.LL_F32, NV.ptr(cb), NV.ptr(cbt), NV.ptr(scb), None, NV.ptr(y), M, N, K, 6.0, NV.ptr(ws),
+            ws.numel(), NV.stream())
+    torch.cuda.synchronize()
+    a, out = x.double(), torch.zeros(K, dtype=torch.bool, device="cuda")
+    out[cols] = True
+    rest = a.masked_fill(out[None], 0.0)
+    sca = rest.abs().amax(1)
+    ca = torch.round((rest.float() * (torch.full_like(sca, 127.0).float() / sca.clamp_min(1e-30).float())[:, None]).double())
+    want = (ca @ cb.double().t()) * sca[:, None] * scb.double()[None] / 127.0 ** 2
+    wo = (cb.double()[:, out] * scb.double()[:, None] / 127.0).half().double()
+    odd, size = a[:, out] @ wo.t(), a[:, out].abs() @ wo.abs().t()
+    # as above: both parts and their sum rounded to fp16, an outlier's weight possibly on its other fp16 neighbour
+    assert ((y.double() - want - odd).abs() <= 2.0 ** -11 * (want.abs() + odd.abs() + (want + odd).abs()) * 1.01 + 2.0 ** -10 * size + 1e-4).all()
