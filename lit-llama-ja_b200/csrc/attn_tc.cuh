@@ -462,6 +462,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           mx *= mul;
           if (CAP) mx = cap2 * (1.f - 2.f * at_rcp(1.f + at_exp2(mx * (2.f * AT_LOG2E))));
         }
+        __syncwarp();      // the stores to tensor memory below are the whole warp's: lanes part above this line and not between it and them
         // one barrier of the tile's warps per block: does any row's reference have to move, has any wait run out?
         if (at_any(1 + tile, !ok || mx > ref + AT_SLACK || (ref == -INFINITY && mx > -INFINITY))) {
           *mine = mx;
@@ -574,6 +575,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
           for (int e = 0; e < 4; ++e)
             if (gt && live && c + 8 * e < p.vdim) gu[e] = at_load8(gt + c + 8 * e, p.gate_vec);
+          __syncwarp();
           uint32_t o[32];
           tmem_ld32_async(to + (uint32_t)c, o);
           tmem_wait_ld();

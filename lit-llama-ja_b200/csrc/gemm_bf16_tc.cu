@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_const
           }
         }
       }
+      __syncwarp();                  // the next load from tensor memory is the whole warp's
     }
     tc_fence_before();
   }
@@ -349,6 +350,10 @@ __global__ void __launch_bounds__(64 + 32 * W4_DW, 1) gemm_w4_tc_kernel(const __
       const float zf = __uint_as_float((sz & 0xffff0000u) ^ 0x80000000u);
       const bool zint = zf == floorf(zf) && zf >= 0.f && zf <= 64.f;
       const uint32_t zc2 = zint ? (uint32_t)(0x4300u + (uint32_t)zf) * 0x00010001u : 0x43004300u;
+      // a column's zero may be whole and its neighbour's not: the warp goes one way (the store below is the whole warp's), a whole zero
+      // then subtracts 0
+      const bool one_step = __all_sync(0xffffffffu, zint);
+      const uint32_t zr2 = zint ? 0u : z2;
       const uint32_t ta = lane_addr + 128u + (uint32_t)buf * 64u;
       constexpr int MPW = 8 * 4 / W4_DW;  // 16-k slices per warp per block
 #pragma unroll
@@ -367,9 +372,9 @@ __global__ void __launch_bounds__(64 + 32 * W4_DW, 1) gemm_w4_tc_kernel(const __
           // the reference's get_weight in bf16 (quantization.py:399-408)
           uint32_t a = w4_sub2(w4_prmt(nib, 0x43434343u, 0x5140u), zc2);
           uint32_t b = w4_sub2(w4_prmt(nib, 0x43434343u, 0x5342u), zc2);
-          if (!zint) {
-            a = w4_sub2(a, z2);
-            b = w4_sub2(b, z2);
+          if (!one_step) {
+            a = w4_sub2(a, zr2);
+            b = w4_sub2(b, zr2);
           }
           r[2 * j] = w4_mul2(a, s2);
           r[2 * j + 1] = w4_mul2(b, s2);
@@ -413,6 +418,7 @@ __global__ void __launch_bounds__(64 + 32 * W4_DW, 1) gemm_w4_tc_kernel(const __
           else p.scratch[(((size_t)tile * p.ksplit + ks) * MPAD + m) * W4_BN + t] = __uint_as_float(v[j]);
         }
       }
+      __syncwarp();
     }
     tc_fence_before();
   }

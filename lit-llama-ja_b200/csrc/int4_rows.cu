@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
         const uint32_t o = odd ? (got >> 16) | (w[e] & 0xffff0000u) : (w[e] & 0xffffu) | (got << 16);
         if (2 * e < left && n < p.N) *reinterpret_cast<uint32_t*>(dst + (size_t)(2 * e) * p.N) = o;
       }
+      __syncwarp();
     };
     // the group's steps: every fourth of all steps of all of the CTA's tiles
     int tile = blockIdx.x, kb = grp, drained = blockIdx.x;
@@ -242,6 +243,10 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
       const float zf = __uint_as_float(zn << 16);
       const bool zint = zf == floorf(zf) && zf >= 0.f && zf <= 64.f;
       const uint32_t zc2 = zint ? (uint32_t)(0x4300u + (uint32_t)zf) * 0x00010001u : 0x43004300u;
+      // a column's zero may be whole and its neighbour's not: the warp goes one way (the store below is the whole warp's), a whole zero
+      // then subtracts 0
+      const bool one_step = __all_sync(0xffffffffu, zint);
+      const uint32_t zr2 = zint ? 0u : z2;
       kb += R4_GROUPS;
       normal();
       params(sn, zn);                        // of the next step, under this one's work
@@ -259,7 +264,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
         for (int j = 0; j < 16; ++j) {
           const uint32_t b = src[(c * 16 + j) * R4_N];
           uint32_t a = r4_sub2(((b * 0x1001u) & 0x000f000fu) | 0x43004300u, zc2);      // bf16 (128 + q) of both halves, minus 128 (+ zero)
-          if (!zint) a = r4_sub2(a, z2);
+          if (!one_step) a = r4_sub2(a, zr2);
           r[j] = r4_mul2(a, s2);
         }
         r4_st16(ta + 16u * c, r);

@@ -247,17 +247,19 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
         if (n0 + c0 >= N) break;
         uint32_t v[32];
         tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-        if (m >= M) continue;
-        int32_t* dst = c + (size_t)m * N + n0 + c0;
-        if (n0 + c0 + 32 <= N && (N & 3) == 0) {
+        if (m < M) {
+          int32_t* dst = c + (size_t)m * N + n0 + c0;
+          if (n0 + c0 + 32 <= N && (N & 3) == 0) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 4)
-            *reinterpret_cast<int4*>(dst + e) = make_int4((int)v[e], (int)v[e + 1], (int)v[e + 2], (int)v[e + 3]);
-        } else {
+            for (int e = 0; e < 32; e += 4)
+              *reinterpret_cast<int4*>(dst + e) = make_int4((int)v[e], (int)v[e + 1], (int)v[e + 2], (int)v[e + 3]);
+          } else {
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (n0 + c0 + e < N) dst[e] = (int)v[e];
+            for (int e = 0; e < 32; ++e)
+              if (n0 + c0 + e < N) dst[e] = (int)v[e];
+          }
         }
+        __syncwarp();                // the next load from tensor memory is the whole warp's
       }
     }
     tc_fence_before();
@@ -690,6 +692,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
 #pragma unroll
         for (int e = 0; e < 32; ++e)
           if (c0 + e < M && n < N) dst[(size_t)(c0 + e) * N] = (int)v[e];
+        __syncwarp();                // the next load from tensor memory is the whole warp's
       }
     }
     tc_fence_before();
