@@ -289,7 +289,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   }
   __syncthreads();
   // what every role walks: key blocks from kt0 to the last visible key; per tile the part of it that its rows see
-  const int step_last = __shfl_sync(0xffffffffu, p.pos_ids[p.T - 1], 0);     // rows after this key hold nothing of this step
   int lo[2], hi[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -298,6 +297,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     hi[i] = end;
   }
   const int kt0 = min(lo[0], lo[1]), last = max(hi[0], hi[1]);
+  // rows after this key hold nothing of this step, or (positions that do not rise) nothing that a row of this block sees: a block of keys
+  // starts at or before it
+  const int step_last = max(__shfl_sync(0xffffffffu, p.pos_ids[p.T - 1], 0), last);
 
   if (warp == AT_WARPS) {
     // ===================== TMA producer =====================

@@ -114,3 +114,27 @@ def test_weights_add_up_to_what_they_are_divided_by(T, S, window, terms, scale):
     torch.cuda.synchronize()
     assert N.call_ret("ll_latent_prompt_error") == 0
     assert bool((y == 1.0).all())
+
+
+def test_positions_that_do_not_rise():
+    """Queries in any order of their positions see the keys up to their own: the same rows as in rising order.  (Nothing is written outside
+    a key block's rows in shared memory, whatever the last query's position is.)"""
+    from lit_llama import _native as N
+
+    T, H, G, dim = 300, 4, 2, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    q, kc, vc = rnd(T, H * dim), rnd(1, T, G * dim), rnd(1, T, G * dim)
+    outs = []
+    for order in (torch.arange(T, device="cuda"), torch.arange(T - 1, -1, -1, device="cuda"), torch.randperm(T, generator=g, device="cuda")):
+        pos, qs = order.to(torch.int32), q[order].contiguous()
+        y = torch.zeros((T, H * dim), dtype=torch.bfloat16, device="cuda")
+        N.call("ll_softmax_attn_rows", N.ptr(qs), H * dim, None, 0, N.ptr(kc), N.ptr(vc), N.LL_BF16, N.ptr(pos), None, None, dim ** -0.5, 0.0, 1, T, H,
+               G, dim, dim, 0, 0, T, 1, 0, 1, 0.0, 1.0, 0.0, None, N.ptr(y), y.stride(0), N.stream())
+        torch.cuda.synchronize()
+        assert N.call_ret("ll_softmax_attn_tc_error") == 0
+        back = torch.empty_like(y)
+        back[order] = y
+        outs.append(back.float())
+    for other in outs[1:]:           # a row's maximum moves elsewhere: the weights' scale differs by a power that is not exact, 2^-16, and bf16 rounds
+        assert ((outs[0] - other).abs() <= outs[0].abs() * 2.0 ** -7 + 2.0 ** -12).all()
