@@ -8,6 +8,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "../../include/llb200.h"
 
 namespace llb {
@@ -37,6 +39,21 @@ int cuda_fail(cudaError_t e, const char* what);
   } while (0)
 
 int sm_count();
+
+// Whether a kernel's attributes have been set on the current device: they belong to a device, not to the process.  Marked after they have
+// been set, so that a second thread sets them again instead of launching without them.
+class PerDevice {
+ public:
+  explicit operator bool() const { return (set_.load(std::memory_order_acquire) & bit()) != 0; }
+  void mark() { set_.fetch_or(bit(), std::memory_order_release); }
+
+ private:
+  static uint64_t bit() {      // 0 (set every time) past the 64th device
+    int d = 0;
+    return cudaGetDevice(&d) == cudaSuccess && d < 64 ? (uint64_t)1 << d : 0;
+  }
+  std::atomic<uint64_t> set_{0};
+};
 
 // ------------------------------------------------------------------ small device helpers
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t b) { return __uint_as_float(b << 16); }

@@ -330,11 +330,11 @@ static int decay_chunked_launch(const void* q, int q_stride, const void* k, int 
   float* total = scratch + (size_t)B * H * chunks * n * pp;
   const dim3 grid(chunks * ptiles, H, B);
   constexpr int smem_c = (3 * DC_L * (NP + 8) + DC_L * (PT + 8)) * 2, smem_r = (DC_L * (NP + 8) + DC_L * (PT + 8) + (UNIT ? 3 : 2) * NP * (PT + 8)) * 2;
-  static bool sized = false;
+  static PerDevice sized;
   if (!sized) {
     LL_CUDA(cudaFuncSetAttribute(decay_collect_kernel<NP, PT, SILU, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_c));
     LL_CUDA(cudaFuncSetAttribute(decay_read_kernel<NP, PT, SILU, UNIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_r));
-    sized = true;
+    sized.mark();
   }
   typedef const __nv_bfloat16* in_t;
   decay_collect_kernel<NP, PT, SILU, UNIT><<<grid, DC_THREADS, smem_c, st>>>((in_t)k, k_stride, (in_t)v, v_stride, a, a_row, ks, chunk_state, total, Tn, H,

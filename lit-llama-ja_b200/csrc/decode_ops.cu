@@ -779,8 +779,8 @@ int ll_rmsnorm(const void* x, const void* w, void* y, int dtype, int rows, int d
 int ll_embed_ssq(const void* wte, const int64_t* idx, void* x, float* ssq, int M, int dim, ll_stream stream) {
   LL_CHECK_ARG(wte && idx && x && M > 0 && dim > 0 && dim % 16 == 0, "bad embed arguments (dim must be a multiple of 16)");
   const int nchunks = (dim + 127) / 128;
-  static bool once = false;
-  if (!once) { prefer_max_smem(embed_ssq_kernel); prefer_max_smem(set_pos_kernel); prefer_max_smem(advance_pos_kernel); once = true; }
+  static PerDevice once;
+  if (!once) { prefer_max_smem(embed_ssq_kernel); prefer_max_smem(set_pos_kernel); prefer_max_smem(advance_pos_kernel); once.mark(); }
   embed_ssq_kernel<<<dim3(nchunks, M), 128, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)wte, idx, (__nv_bfloat16*)x, ssq, dim, dim / 16);
   LL_LAUNCH_OK("embed_ssq_kernel");
   return LL_OK;
@@ -843,11 +843,11 @@ static int decode_attn_impl(const void* q, const void* k_cache, const void* v_ca
   const bool cl = use_cluster && max_splits >= 2 && max_splits <= 8;
 #define ATTN(TT, HS)                                                                                              \
   do {                                                                                                            \
-    static bool once = false;                                                                                     \
+    static PerDevice once;                                                                                     \
     if (!once) {                                                                                                  \
       prefer_max_smem(decode_attn_kernel<TT, HS, false>);                                                         \
       prefer_max_smem(decode_attn_kernel<TT, HS, true>);                                                          \
-      once = true;                                                                                                \
+      once.mark();                                                                                                \
     }                                                                                                             \
     const int pfr = cl ? launch_attn_pf<TT, HS>(q, k_cache, v_cache, pos, y, cache_len, max_splits, grid, block, st, pdl, \
                                                 kflags | (flags & (LL_ATTN_FLAG_MISGUESS | LL_ATTN_FLAG_POISON)), tr,  \

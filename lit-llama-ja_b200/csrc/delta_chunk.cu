@@ -672,10 +672,10 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_read_kernel(const DeltaCh
 template <int NP, int PT, int WARPS>
 static int delta_pass_launch(const DeltaChunkArgs& A, int B, cudaStream_t st) {
   constexpr int smem = (3 * 3 * DC_L * (NP + 8) + (2 * NP + 3 * DC_L) * dx_pitch(PT)) * 2;
-  static bool sized = false;
+  static PerDevice sized;
   if (!sized) {
     LL_CUDA(cudaFuncSetAttribute(delta_pass_kernel<NP, PT, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    sized = true;
+    sized.mark();
   }
   delta_pass_kernel<NP, PT, WARPS><<<dim3((A.p + PT - 1) / PT, A.H, B), WARPS * 32, smem, st>>>(A);
   LL_LAUNCH_OK("delta_pass_kernel");
@@ -685,10 +685,10 @@ static int delta_pass_launch(const DeltaChunkArgs& A, int B, cudaStream_t st) {
 template <int NP, int PT>
 static int delta_prepare_launch(const DeltaChunkArgs& A, int B, cudaStream_t st) {
   constexpr int smem = (DC_L * DX_LD + 32 * DX_TMP) * 4 + DC_L * (3 * (NP + 8) + PT + 8) * 2;
-  static bool sized = false;
+  static PerDevice sized;
   if (!sized) {
     LL_CUDA(cudaFuncSetAttribute(delta_prepare_kernel<NP, PT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    sized = true;
+    sized.mark();
   }
   delta_prepare_kernel<NP, PT><<<dim3(A.chunks, A.H, B), DC_THREADS, smem, st>>>(A);
   LL_LAUNCH_OK("delta_prepare_kernel");
@@ -698,10 +698,10 @@ static int delta_prepare_launch(const DeltaChunkArgs& A, int B, cudaStream_t st)
 template <int NP>
 static int delta_chunked_launch(const DeltaChunkArgs& A, int B, cudaStream_t st) {
   constexpr int smem_r = (DC_L * (NP + 8) + 2 * DC_L * (DC_L + 8) + 2 * (DC_L + NP) * (DX_PT + 8)) * 2;
-  static bool sized = false;
+  static PerDevice sized;
   if (!sized) {
     LL_CUDA(cudaFuncSetAttribute(delta_read_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_r));
-    sized = true;
+    sized.mark();
   }
   int rc = A.p <= 64 ? delta_prepare_launch<NP, 64>(A, B, st) : delta_prepare_launch<NP, 128>(A, B, st);
   if (rc != LL_OK) return rc;

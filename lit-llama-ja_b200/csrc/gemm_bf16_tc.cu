@@ -154,10 +154,10 @@ template <int BN, int STAGES>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, __nv_bfloat16* C, const __nv_bfloat16* bias, int M, int N, int K,
                 cudaStream_t st) {
   constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
-  static bool configured = false;
+  static PerDevice configured;
   if (!configured) {
     LL_CUDA(cudaFuncSetAttribute(gemm_bf16_tc_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
+    configured.mark();
   }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   gemm_bf16_tc_kernel<BN, STAGES><<<grid, 192, smem, st>>>(ma, mb, C, bias, M, N, K);
@@ -471,10 +471,10 @@ int launch_w4(const CUtensorMap& mx, const W4Params& p, cudaStream_t st) {
   constexpr int W4_STAGES = w4_stages(MPAD);
   constexpr size_t stage = ((8 * W4_BLK + 1023) / 1024) * 1024 + 2 * MPAD * 128;
   constexpr size_t smem = W4_STAGES * stage + (2 * W4_STAGES + 5) * 8 + 16 + 1024;
-  static bool configured = false;
+  static PerDevice configured;
   if (!configured) {
     LL_CUDA(cudaFuncSetAttribute(gemm_w4_tc_kernel<MPAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
+    configured.mark();
   }
   gemm_w4_tc_kernel<MPAD><<<(p.N / W4_BN) * p.ksplit, 64 + 32 * W4_DW, smem, st>>>(mx, p);
   LL_LAUNCH_OK("gemm_w4_tc_kernel");

@@ -264,10 +264,10 @@ template <int MODE>
 int launch_moe_tc(const CUtensorMap& ma, const CUtensorMap& mb, const int32_t* offsets, const int32_t* perm, int X, int N, int K,
                   float limit, float alpha, float shift, void* c, int ldc, int n_rows, cudaStream_t st) {
   constexpr size_t smem = (size_t)MT_STAGES * (MT_A_BYTES + MT_B_BYTES) + (2 * MT_STAGES + 5) * 8 + 32 + 1024;
-  static bool configured = false;
+  static PerDevice configured;
   if (!configured) {
     LL_CUDA(cudaFuncSetAttribute(moe_gemm_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
+    configured.mark();
   }
   const int ncols = MODE == 1 ? MT_BN : MT_COLS;
   const long long most = (long long)((N + ncols - 1) / ncols) * ((n_rows + BM - 1) / BM + X);

@@ -438,10 +438,10 @@ static int launch_grouped_mma(const void* a, int lda, const void* w, const int32
                               int K, float limit, float alpha, float shift, void* c, int ldc, int n_rows, cudaStream_t st) {
   constexpr int NB = MODE == MODE_GLU ? 2 : 1;
   const size_t smem = sizeof(__nv_bfloat16) * gm_stages(BM) * (BM + NB * GM_BN) * GM_PITCH;
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     LL_CUDA(cudaFuncSetAttribute(moe_grouped_gemm_mma_kernel<BM, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    once = true;
+    once.mark();
   }
   dim3 grid((n_rows + BM - 1) / BM + X, (N + GM_BN - 1) / GM_BN);
   moe_grouped_gemm_mma_kernel<BM, MODE><<<grid, GM_THREADS, smem, st>>>((const __nv_bfloat16*)a, lda, (const __nv_bfloat16*)w, offsets, perm,

@@ -375,10 +375,10 @@ static int add_row_norm_launch(float* x, const void* a, float s, const float* a_
       set_error("add + norm: rows of %d numbers", dim);
       return LL_ERR_UNSUPPORTED;
     }
-    static bool sized = false;
+    static PerDevice sized;
     if (!sized && smem > 48 * 1024) {
       LL_CUDA(cudaFuncSetAttribute(add_row_norm_kernel<TA, 0, RMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-      sized = true;
+      sized.mark();
     }
     LL_ALN(0, dim >= 512 ? 256 : 128, smem);
   }
@@ -697,10 +697,10 @@ int ll_hyper_mix_norm(const float* src, long long src_row, long long src_copy, f
   }
 #define LL_HYPER(TA, SM)                                                                                                            \
   {                                                                                                                                 \
-    static bool sized = false;                                                                                                      \
+    static PerDevice sized;                                                                                                      \
     if (!sized && smem > 48 * 1024) {                                                                                               \
       LL_CUDA(cudaFuncSetAttribute(hyper_mix_norm_kernel<TA, SM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));        \
-      sized = true;                                                                                                                 \
+      sized.mark();                                                                                                                 \
     }                                                                                                                               \
     hyper_mix_norm_kernel<TA, SM><<<rows, threads, smem, st>>>(src, src_row, src_copy, X, (const TA*)y, ls, r, mix, w_out, w_in, w, eps, \
                                                               h, h_f32, total, S, dim);                                             \

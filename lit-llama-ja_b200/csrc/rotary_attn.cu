@@ -865,10 +865,10 @@ static int tm_launch(const void* q, int q_stride, const void* gate, int gate_str
                      int ring, const DiffMaps& dm, void* y, int y_stride, cudaStream_t st) {
   const dim3 grid((Tn + TM_Q - 1) / TM_Q, H, B);
   constexpr int smem = 2 * TM_K * (DK + 8 + DV + 8) * (int)sizeof(__nv_bfloat16);
-  static bool sized = false;
+  static PerDevice sized;
   if (!sized) {
     LL_CUDA(cudaFuncSetAttribute(softmax_attn_mma_kernel<DK, DV, MAPS, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    sized = true;
+    sized.mark();
   }
   softmax_attn_mma_kernel<DK, DV, MAPS, BIAS><<<grid, TM_THREADS, smem, st>>>(
       (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)gate, gate_stride, (const __nv_bfloat16*)kc, (const __nv_bfloat16*)vc,

@@ -209,11 +209,11 @@ static int launch_sample(const void* logits, int V, float temperature, int top_k
   LL_CHECK_ARG(V > 0 && V <= ST * 64, "vocabulary size %d out of range (max %d)", V, ST * 64);
   LL_CHECK_ARG(temperature > 0.f, "temperature must be positive");
   LL_CHECK_ARG(out_tokens == nullptr || pos != nullptr, "out_tokens needs pos");
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     prefer_max_smem(sample_topk_kernel<32>);
     prefer_max_smem(sample_topk_kernel<64>);
-    once = true;
+    once.mark();
   }
   cudaStream_t st = (cudaStream_t)stream;
   if (V <= ST * 32)

@@ -286,10 +286,10 @@ int ll_tp_allreduce_add(void* x, const uint64_t* peer_parts /* host: world point
     a.part[r] = (const __nv_bfloat16*)(uintptr_t)peer_parts[r];
     a.flags[r] = (int32_t*)(uintptr_t)peer_flags[r];
   }
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     prefer_max_smem(tp_allreduce_add_kernel);
-    once = true;
+    once.mark();
   }
   const bool pdl = (flags & LL_GEMV_PDL) != 0;
   // as a link of the programmatic chain the CTAs are kept small (256 threads each, one 16-byte piece per thread, up to
@@ -339,10 +339,10 @@ int ll_tp_reduce_add(void* x, const void* recv, uint32_t* cnt, int32_t* epoch_co
   LL_CHECK_ARG(x && recv && cnt && epoch_counter, "null pointer");
   LL_CHECK_ARG(world >= 1 && world <= MAX_WORLD && arrivals > 0, "bad world / arrivals (%d / %d)", world, arrivals);
   LL_CHECK_ARG(n > 0 && n % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)recv & 15) == 0, "n must be a multiple of 8, buffers 16-byte aligned");
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     prefer_max_smem(tp_reduce_add_kernel);
-    once = true;
+    once.mark();
   }
   tp_reduce_add_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((__nv_bfloat16*)x, (const __nv_bfloat16*)recv, cnt, epoch_counter, world, n,
                                                             arrivals);

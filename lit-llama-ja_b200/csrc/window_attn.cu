@@ -602,10 +602,10 @@ static bool wm_takes(const WaParams& P, int dtype, size_t* smem) {
 
 template <int HPW>
 static int wm_launch(const WaParams& P, const void* gate, int gate_stride, void* y, size_t smem, cudaStream_t st) {
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     LL_CUDA(cudaFuncSetAttribute(window_attn_mma_kernel<HPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    once = true;
+    once.mark();
   }
   const int tiles = P.B * ((P.T + WM_Q - 1) / WM_Q);
   window_attn_mma_kernel<HPW><<<tiles, WM_THREADS, smem, st>>>(P, (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)y);
@@ -643,11 +643,11 @@ static int window_attn_run(WaParams& P, const void* gate, int gate_stride, void*
     set_error("window_attn: %d heads of %d do not fit shared memory", P.H, P.dim);
     return LL_ERR_UNSUPPORTED;
   }
-  static bool once = false;
+  static PerDevice once;
   if (!once) {
     LL_CUDA(cudaFuncSetAttribute(window_attn_stats_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     LL_CUDA(cudaFuncSetAttribute(window_attn_out_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    once = true;
+    once.mark();
   }
   const int M = P.B * P.T;
   dim3 grid(M, P.splits);

@@ -111,3 +111,12 @@ def test_bench_reference_arm_prints_the_contract_line():
     assert "workload" in d["config"]
     # all the host threads, whatever OMP_NUM_THREADS torchrun exported; and none of this repo's libraries in that process
     assert d["cpu_baseline"]["cores"] == len(os.sched_getaffinity(0))
+
+
+def test_kernel_attributes_are_set_per_device():
+    """A kernel's shared-memory limit and carve-out belong to a device: no process-wide flag may stand in front of setting them (a second
+    device of the process would launch without them)."""
+    import re
+
+    for path in sorted((Path(__file__).resolve().parent.parent / "lit-llama-ja_b200" / "csrc").glob("*.cu*")):
+        assert not re.search(r"static\s+bool\s+\w+\s*=", path.read_text()), path.name
