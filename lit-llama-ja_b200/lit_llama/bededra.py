@@ -293,7 +293,7 @@ class Bededra(PortionedDecoder):
             t.copy_(k)
 
     # ------------------------------------------------------------------ forward
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
         cfg = self.config
         B, T = idx.shape
         M, E = B * T, cfg.width

@@ -305,7 +305,7 @@ class Bumulix(PortionedDecoder):
         self.kv_caches, self._rings, self._batch = saved
 
     # ------------------------------------------------------------------ forward
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
         cfg = self.config
         B, T = idx.shape
         M, E, S = B * T, cfg.width, cfg.copies
@@ -336,7 +336,7 @@ class Bumulix(PortionedDecoder):
                 y = blk.mix(h, B, T, pos_ids, self.kv_caches[at:at + 2], None, splits)
             else:
                 splits = max(1, min(16, (2 * sms) // max(1, M * ((spec.heads + 31) // 32)), (ring + 63) // 64))
-                y = blk.mix(h, B, T, pos_ids, self._rope[astuple(spec.rotary)], self.kv_caches[at], splits)
+                y = blk.mix(h, B, T, pos_ids, self._rope[astuple(spec.rotary)], self.kv_caches[at], splits, end)
             pending = (y, blk.ls1, blk.hc1)
             if blk.mlp is not None:
                 h2 = torch.empty((M, E), dtype=self.dtype, device=dev)

@@ -7,8 +7,8 @@ With h the mixer's input, per token
     score(i, j, head) = (q_nope . (W_uk c_j) + rope(q_rot) . k_rot_j) * scale,   j in the sliding window of i
     out = W_o concat_heads( sigmoid(g) * sum_j softmax_j(score) (W_uv c_j) )
 The kernels work in latent space: W_uk is absorbed into the query (q_lat = W_uk^T q_nope, a batched GEMM over heads) and
-W_uv is applied to the weighted sum of the c_j, so every head reads the same cache row once, in prefill and in decoding
-alike.  A layer built with ``kv_from`` has no down-projection: it reads another layer's rows with its own W_uk, W_uv,
+W_uv is applied to the weighted sum of the c_j, so every head reads the same cache row once.  Prompts in bf16 whose queries
+fill the device by themselves (``splits`` 1) have the visible rows expanded per head instead (``_takes_expanded``).  A layer built with ``kv_from`` has no down-projection: it reads another layer's rows with its own W_uk, W_uv,
 queries and window.
 
 Variations, all parameters of the spec:
@@ -35,7 +35,7 @@ from . import _native as N
 from .rotary import RotarySpec
 
 EXPAND_MIN_TOKENS = 16               # tokens a step appends from which its rows are expanded per head
-EXPAND_MAX_SLOTS_PER_TOKEN = 64      # ring slots per such token
+EXPAND_MAX_SLOTS_PER_TOKEN = 64      # expanded rows per such token
 EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
 
 
@@ -176,15 +176,17 @@ class LatentAttention(nn.Module):
             self.kv_norm.copy_(get("dkv.norm").float())
 
     def forward(self, x_act: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor,
-                splits: int = 1) -> torch.Tensor:
+                splits: int = 1, end: Optional[int] = None) -> torch.Tensor:
         """x_act ``[B*T, width]`` -> ``[B*T, width]``; ``cache`` ``[B, S, row]`` is this layer's or its source's (already
-        appended to by the source in this step)."""
-        return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits), self.w_o)
+        appended to by the source in this step).  ``end``: as in ``attend``."""
+        return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
 
     def attend(self, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor,
-               splits: int = 1, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+               splits: int = 1, out: Optional[torch.Tensor] = None, end: Optional[int] = None) -> torch.Tensor:
         """``proj``: the input projection's output (this mixer's columns first).  Returns the gated heads
-        ``[B*T, heads * v_dim]`` before the output projection, in ``out`` (a column slice) when given."""
+        ``[B*T, heads * v_dim]`` before the output projection, in ``out`` (a column slice) when given.  ``end``: the position after
+        the step's last, when the host knows it (positions are consecutive); then only rows that some query sees are expanded,
+        else every slot of the cache."""
         s = self.spec
         M = B * T
         dt = N.dtype_code(proj.dtype)
@@ -200,8 +202,9 @@ class LatentAttention(nn.Module):
             q = F.linear(cq, self.w_uq)                                       # [M, heads * q_head]
         else:
             q = proj
-        if T >= EXPAND_MIN_TOKENS and splits == 1 and self._takes_expanded(q, out, cache, B, T):
-            o = self._attend_expanded(proj, q, B, T, pos_ids, rope, cache, out)
+        first, rows = self._visible(T, S, end)
+        if T >= EXPAND_MIN_TOKENS and splits == 1 and self._takes_expanded(q, out, cache, B, T, rows):
+            o = self._attend_expanded(proj, q, B, T, pos_ids, rope, cache, out, first, rows)
         else:
             o = self._attend_latent(proj, q, B, T, pos_ids, rope, cache, splits, out)
         if s.gate == "element":
@@ -211,33 +214,48 @@ class LatentAttention(nn.Module):
             raise NotImplementedError("a gate per head beside latent queries")
         return o
 
-    def _takes_expanded(self, q, out, cache, B: int, T: int) -> bool:
-        """Whether a step of several tokens expands the cache rows per head (one up-projection of every ring slot) and attends over plain
-        keys and values on the tcgen05 kernel: bf16, sizes that kernel takes, a ring that is not too long for the queries.  Both sides
-        measured (16 heads, 128 + 64 dimensions, rank 512, window 1024; device time of the whole layer): 16 tokens after 0 / 1000
-        positions 38 / 111 -> 29 / 47 us, 128 after 8000 119 -> 82 us, 2048 after 0 611 -> 97 us."""
+    def _visible(self, T: int, S: int, end: Optional[int]):
+        """(first position, rows) that the queries of a step of ``T`` tokens up to position ``end`` see; (None, S) when that is not known."""
+        if end is None:
+            return None, S
+        first = 0 if self.spec.window is None else max(0, end - T - self.spec.window + 1)
+        return (first, end - first) if end - first <= S else (None, S)
+
+    def _takes_expanded(self, q, out, cache, B: int, T: int, rows: int) -> bool:
+        """Whether a step of several tokens expands ``rows`` cache rows per head (one up-projection of each) and attends over plain keys and
+        values on the tcgen05 kernel: bf16, sizes that kernel takes, not too many rows for the queries.  Both sides measured (128 + 64
+        dimensions, rank 512, graphed ``attend``, us): 16 heads, 16 tokens after 0 / 1000 positions 29 / 101 -> 21 / 39, 200 after 0 / 7000
+        48 / 574 -> 27 / 192, 2048 after 0 734 -> 68; 64 heads, 16 after 1000 102 -> 50, 200 after 7000 1679 -> 267.  Rows that no query
+        sees are not worth forming: with all of 8192 slots expanded, 150 tokens at position 0 took 41 -> 60 (16 heads) and 76 -> 146 (64)."""
         s = self.spec
-        S = cache.shape[1]
-        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0 and S <= EXPAND_MAX_SLOTS_PER_TOKEN * T
-                and 2 * B * S * s.heads * (s.nope_dim + s.v_dim) <= EXPAND_MAX_BYTES
+        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0 and rows <= EXPAND_MAX_SLOTS_PER_TOKEN * T
+                and 2 * B * rows * s.heads * (s.nope_dim + s.v_dim) <= EXPAND_MAX_BYTES
                 and N.has("ll_latent_prompt_attn") and cache.is_contiguous() and (out is None or (out.stride(1) == 1 and out.data_ptr() % 16 == 0))
                 and bool(N.call_ret("ll_latent_prompt_supported", s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, q.stride(0), s.q_head,
                                     s.heads * s.v_dim if out is None else out.stride(0)))
                 and (q.data_ptr() | cache.data_ptr()) % 16 == 0)
 
-    def _attend_expanded(self, proj, q, B: int, T: int, pos_ids, rope, cache, out) -> torch.Tensor:
+    def _attend_expanded(self, proj, q, B: int, T: int, pos_ids, rope, cache, out, first: Optional[int], n: int) -> torch.Tensor:
+        """``n`` rows per sequence from position ``first`` on, in the order of their positions; ``first`` None: the ring as it lies."""
         s = self.spec
         S = cache.shape[1]
         if out is None:
             out = torch.empty((B * T, s.heads * s.v_dim), dtype=proj.dtype, device=proj.device)
-        c = cache.view(B * S, s.row)[:, : s.kv_rank]
-        k = F.linear(c, self.w_uk.view(s.heads * s.nope_dim, s.kv_rank))                # [B * S, heads * nope]
-        v = torch.bmm(c.expand(s.heads, B * S, s.kv_rank), self.w_uv_t)                 # [heads, B * S, v_dim]
+        rope_at = N.ptr(rope)
+        if first is not None:
+            a = first % S
+            cache = cache[:, a: a + n] if a + n <= S else torch.cat([cache[:, a:], cache[:, : a + n - S]], dim=1)
+            cache = cache.contiguous()                            # (one sequence whose rows do not wrap: a view)
+            if first > 0:                                         # the kernel's positions count from the first row
+                pos_ids, rope_at = pos_ids - first, N.ptr_at(rope, first * s.rot_dims)
+        c = cache.view(B * n, s.row)[:, : s.kv_rank]
+        k = F.linear(c, self.w_uk.view(s.heads * s.nope_dim, s.kv_rank))                # [B * n, heads * nope]
+        v = torch.bmm(c.expand(s.heads, B * n, s.kv_rank), self.w_uv_t)                 # [heads, B * n, v_dim]
         q_rot = torch.empty((B * T, s.heads, s.rot_dim), dtype=q.dtype, device=q.device)
         gate = N.ptr_at(proj, self.gate_col0) if s.gate == "head" and s.q_rank is None else None
-        N.call("ll_latent_prompt_attn", N.ptr(q), q.stride(0), s.nope_dim, s.q_head, gate, proj.stride(0), N.ptr(rope), N.ptr(pos_ids),
-               N.ptr(k), k.stride(0), s.nope_dim, N.ptr(v), s.v_dim, B * S * s.v_dim, N.ptr(cache), N.ptr(q_rot), N.ptr(out), out.stride(0),
-               B, T, s.heads, s.kv_rank, s.rot_dim, s.rot_dims, s.v_dim, S, s.window if s.window is not None else 0, float(s.scale),
+        N.call("ll_latent_prompt_attn", N.ptr(q), q.stride(0), s.nope_dim, s.q_head, gate, proj.stride(0), rope_at, N.ptr(pos_ids),
+               N.ptr(k), k.stride(0), s.nope_dim, N.ptr(v), s.v_dim, B * n * s.v_dim, N.ptr(cache), N.ptr(q_rot), N.ptr(out), out.stride(0),
+               B, T, s.heads, s.kv_rank, s.rot_dim, s.rot_dims, s.v_dim, n, s.window if s.window is not None else 0, float(s.scale),
                2 if s.exact_weights else 1, N.stream())
         return out
 

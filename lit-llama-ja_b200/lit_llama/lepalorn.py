@@ -247,7 +247,7 @@ class Lepalorn(PortionedDecoder):
     def _restore_memory(self, saved) -> None:
         self.kv_caches, self._ring = saved
 
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
         cfg = self.config
         B, T = idx.shape
         M, E, L = B * T, cfg.width, cfg.n_layer
@@ -267,7 +267,7 @@ class Lepalorn(PortionedDecoder):
             span = spec.window if spec.window is not None else self._ring
             splits = max(1, min(16, (2 * sms) // max(1, M * ((spec.heads + 31) // 32)), (min(span, self._ring) + 63) // 64))
             rope = self._rope[(spec.rot_base, spec.rot_dims)]
-            y = blk.mix(x_act, B, T, pos_ids, rope, self.kv_caches[self._cache_of[i]], splits)
+            y = blk.mix(x_act, B, T, pos_ids, rope, self.kv_caches[self._cache_of[i]], splits, end)
             nxt = mixed[i & 1]
             if blk.mlp is not None:
                 mid = nxt                                                        # scratch for the stream between the sublayers

@@ -226,7 +226,7 @@ class Livasun(RingStateDecoder):
         return [s for b in self.blocks for s in b.mix.state_shapes(B)]
 
     # ------------------------------------------------------------------ forward
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
         cfg = self.config
         B, T = idx.shape
         M, E = B * T, cfg.width

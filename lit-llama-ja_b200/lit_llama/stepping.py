@@ -70,7 +70,8 @@ class PortionedDecoder(nn.Module):
     def _restore_memory(self, saved) -> None:
         raise NotImplementedError
 
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
+        """``end``: the position after the portion's last (None: only the device knows it, a captured step)."""
         raise NotImplementedError
 
     def _drop_graphs(self) -> None:
@@ -112,7 +113,7 @@ class PortionedDecoder(nn.Module):
                     lg = lg[:, sel]
             else:
                 pos_ids = torch.arange(pos0 + t0, pos0 + t1, dtype=torch.int32, device=idx.device)
-                lg = self._forward_portion(part.contiguous(), pos_ids, sel)
+                lg = self._forward_portion(part.contiguous(), pos_ids, sel, pos0 + t1)
             outs.append(lg)
         if not keep:
             self._restore_memory(saved)

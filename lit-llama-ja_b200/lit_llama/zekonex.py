@@ -260,7 +260,8 @@ class Zekonex(RingStateDecoder):
         return [s for r in self.runs for s in r.block.mix.state_shapes(B)]
 
     # ------------------------------------------------------------------ forward
-    def _mixer(self, run: LayerRun, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, sms: int, out: torch.Tensor) -> None:
+    def _mixer(self, run: LayerRun, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, sms: int, out: torch.Tensor,
+               end: Optional[int]) -> None:
         mix = run.block.mix
         spec = mix.spec
         M = B * T
@@ -272,9 +273,9 @@ class Zekonex(RingStateDecoder):
             mix.attend(proj, B, T, pos_ids, self.kv_caches[run.cache_at:run.cache_at + 2], None, splits, out=out)
         else:
             splits = max(1, min(16, (2 * sms) // max(1, M * ((spec.heads + 31) // 32)), (self._rings[run.ring] + 63) // 64))
-            mix.attend(proj, B, T, pos_ids, self.rope_table(spec.rotary), self.kv_caches[run.cache_at], splits, out=out)
+            mix.attend(proj, B, T, pos_ids, self.rope_table(spec.rotary), self.kv_caches[run.cache_at], splits, out=out, end=end)
 
-    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel) -> torch.Tensor:
+    def _forward_portion(self, idx: torch.Tensor, pos_ids: torch.Tensor, sel, end: Optional[int] = None) -> torch.Tensor:
         cfg = self.config
         B, T = idx.shape
         M, E = B * T, cfg.width
@@ -297,7 +298,7 @@ class Zekonex(RingStateDecoder):
             add_rms_norm(x, pending, r, bias, step, blk.norm1, cfg.eps, h, self.dtype)
             proj = F.linear(h, blk.w_in)
             rows = (torch.zeros if blk.gaps else torch.empty)((M, blk.n_out), dtype=self.dtype, device=dev)
-            self._mixer(run, proj, B, T, pos_ids, sms, rows[:, : blk.mix.out_cols])
+            self._mixer(run, proj, B, T, pos_ids, sms, rows[:, : blk.mix.out_cols], end)
             bias = None
             if blk.mlp is not None:
                 blk.mlp(proj[:, blk.ff_in:], rows[:, blk.ff_out: blk.ff_out + blk.mlp.ff])

@@ -138,3 +138,52 @@ def test_positions_that_do_not_rise():
         outs.append(back.float())
     for other in outs[1:]:           # a row's maximum moves elsewhere: the weights' scale differs by a power that is not exact, 2^-16, and bf16 rounds
         assert ((outs[0] - other).abs() <= outs[0].abs() * 2.0 ** -7 + 2.0 ** -12).all()
+
+
+@pytest.mark.parametrize("T,past,S,window,rows", [(64, 0, 1024, None, 64), (130, 70, 512, None, 200), (257, 100, 400, 50, 306), (100, 300, 256, 64, 163),
+                                                  (129, 500, 200, 50, 178), (33, 8, 41, None, 41)])
+@pytest.mark.parametrize("B", [1, 2])
+def test_only_visible_rows_are_expanded(monkeypatch, T, past, S, window, rows, B):
+    """With the end of the step known, the rows its queries see are formed and no others: rings that are nearly empty, rings that wrap,
+    windows that begin after position 0.  The result is that of the form in latent space."""
+    from lit_llama import _native as N
+    from lit_llama.latent_attention import LatentAttention, LatentAttentionSpec
+
+    H, nope, rot, v, rank = 3, 64, 32, 64, 64
+    spec = LatentAttentionSpec(width=64, heads=H, nope_dim=nope, rot_dim=rot, v_dim=v, kv_rank=rank, window=window, scale=(nope + rot) ** -0.5)
+    m = LatentAttention(spec, torch.bfloat16, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(T)
+    for p in m.parameters():
+        if p.dim() > 1:
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") / math.sqrt(p.shape[-1]))
+    proj = torch.randn((B * T, m.w_in.shape[0]), generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.arange(past, past + T, dtype=torch.int32, device="cuda")
+    rope = spec.rope_table(past + T, "cuda")
+    cache = torch.randn((B, S, spec.row), generator=g, device="cuda").to(torch.bfloat16)
+    used = torch.zeros(S, dtype=torch.bool, device="cuda")
+    used[[p % S for p in range(max(0, past - (window or past + 1) + 1), past + T)]] = True
+    cache[:, ~used] = math.nan
+    formed, call = [], N.call
+    monkeypatch.setattr(N, "call", lambda name, *a: (formed.append(a[25]) if name == "ll_latent_prompt_attn" else None, call(name, *a))[1])
+    got = m.attend(proj, B, T, pos, rope, cache.clone(), 1, end=past + T).double()
+    m._takes_expanded = lambda *a: False
+    want = m.attend(proj, B, T, pos, rope, cache.clone(), 1, end=past + T).double()
+    assert formed == [rows] and N.call_ret("ll_latent_prompt_error") == 0
+    assert torch.isfinite(got).all()
+    assert (got - want).norm() <= 2.0 ** -6.5 * want.norm()      # as above
+
+
+@pytest.mark.parametrize("family", ["lepalorn", "bumulix", "zekonex"])
+def test_models_say_where_a_step_ends(family, monkeypatch, tmp_path):
+    import importlib
+
+    from lit_llama.latent_attention import LatentAttention
+
+    util = importlib.import_module(f"tests.util_{family}")
+    cfg, W = util.case_mixed()
+    m = util.load(util.write_model(tmp_path, cfg, W), torch.bfloat16)
+    ends, attend = [], LatentAttention.attend
+    monkeypatch.setattr(LatentAttention, "attend", lambda self, *a, end=None, **kw: (ends.append((a[2], end)), attend(self, *a, end=end, **kw))[1])
+    util.run_schedule(m, list(range(9)), [5, 3, 1], 64)
+    assert {e for t, e in ends if t == 5} == {5} and {e for t, e in ends if t == 3} == {8}
+    assert {e for t, e in ends if t == 1} <= {None}              # a captured step's position is known to the device alone
