@@ -22,12 +22,13 @@
 extern "C" {
 #endif
 
-#define LL_ABI_VERSION 18
+#define LL_ABI_VERSION 19
 
 #define LL_OK 0
 #define LL_ERR_ARG (-1)         /* bad shape / dtype / null pointer */
 #define LL_ERR_CUDA (-2)        /* a CUDA runtime/driver call failed */
 #define LL_ERR_UNSUPPORTED (-3) /* valid request this build has no kernel for */
+#define LL_ERR_WAIT (-4)        /* a bounded wait inside an earlier launch ran out: see ll_wait_check */
 
 /* element types of activation / parameter buffers */
 #define LL_F32 0
@@ -43,6 +44,12 @@ typedef void* ll_stream; /* cudaStream_t */
 #endif
 
 LL_API const char* ll_last_error(void);
+/* The waits inside the tcgen05 kernels and the chunked delta rule are bounded; a kernel whose wait runs out skips its stores and leaves a
+ * code in host memory (100 + prompt attention's, 200 + int4 rows', 300 + llm.int8's, 400 + grouped experts', 500 + delta rule's).
+ * The next launch through this library fails with LL_ERR_WAIT, or this call does, which looks without launching: after a synchronisation
+ * it speaks for everything before it.  Either clears the code.  ll_wait_report leaves a code as a kernel does. */
+LL_API int ll_wait_check(void);
+LL_API int ll_wait_report(int code);
 LL_API int ll_abi_version(void);
 /* number of SMs of the current device (host query; <0 on error) */
 LL_API int ll_sm_count(void);

@@ -65,6 +65,7 @@ struct AtParams {
   __nv_bfloat16* y;
   float scale, softcap;
   int T, H, group, vdim, window, chunk, ring, gate_ld, gate_per_head, gate_vec, y_ld;
+  int* word;                   // wait_word()
 };
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -169,7 +170,7 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
 }
 
 // A wait that ends: on its phase, when another role has given up, or after the limit.
-__device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+__device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
   if (mbar_try_wait(bar, parity)) return true;
   for (uint32_t i = 0; i < AT_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -177,6 +178,7 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
   }
   *fail = 1;
   atomicCAS(&g_attn_tc_error, 0, code);
+  wait_ran_out(word, 100 + code);
   return false;
 }
 
@@ -314,11 +316,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       bool ok = true;
       for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next(), ++n) {
         const int ks = n % KS, vs = n % VS;
-        if (!(ok = at_wait(&k_empty[ks], ((n / KS) & 1) ^ 1, s_fail, 1))) break;
+        if (!(ok = at_wait(&k_empty[ks], ((n / KS) & 1) ^ 1, s_fail, p.word, 1))) break;
         mbar_expect_tx(&k_full[ks], (uint32_t)(NB * AT_KBOX));
         for (int c = 0; c < NB1; ++c) tma_box4(sk + (ks * NB + c) * AT_KBOX, &map_k, c * 64, g, blk.slot, b, &k_full[ks]);
         for (int c = 0; c < NB2; ++c) tma_box4(sk + (ks * NB + NB1 + c) * AT_KBOX, &map_k2, c * 64, 0, blk.slot, b, &k_full[ks]);
-        if (!(ok = at_wait(&v_empty[vs], ((n / VS) & 1) ^ 1, s_fail, 2))) break;
+        if (!(ok = at_wait(&v_empty[vs], ((n / VS) & 1) ^ 1, s_fail, p.word, 2))) break;
         mbar_expect_tx(&v_full[vs], (uint32_t)(NBV * AT_KBOX));
         for (int c = 0; c < NBV; ++c) tma_box4(sv + (vs * NBV + c) * AT_KBOX, &map_v, c * 64, g, blk.slot, b, &v_full[vs]);
       }
@@ -341,7 +343,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       // S = Q K^T of the n-th key block: the tile's score buffer is free, its weights two blocks back are in use by an MMA issued before
       auto scores = [&](int n, const AtBlock& blk) {
         const int ks = n % KS;
-        if (!at_wait(&k_full[ks], (n / KS) & 1, s_fail, 4)) return false;
+        if (!at_wait(&k_full[ks], (n / KS) & 1, s_fail, p.word, 4)) return false;
         tc_fence_after();
         if (blk.meets(mylo, myhi)) {
           const uint32_t d = tm_s + 64u * (ns & 1u);
@@ -360,18 +362,18 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         }
         return true;
       };
-      bool ok = at_wait(q_full, 0, s_fail, 3);
+      bool ok = at_wait(q_full, 0, s_fail, p.word, 3);
       AtBlock blk(kt0, last, p.ring), nxt = blk;
       if (ok) ok = scores(0, blk);
       for (int n = 0; ok && blk.any(); blk = nxt, ++n) {
         nxt.next();
         if (nxt.any() && !(ok = scores(n + 1, nxt))) break;
         const int vs = n % VS;
-        if (!(ok = at_wait(&v_full[vs], (n / VS) & 1, s_fail, 5))) break;
-        if (step_last - blk.kt + 1 < AT_K && !(ok = at_wait(&v_clear[vs], 0, s_fail, 10))) break;
+        if (!(ok = at_wait(&v_full[vs], (n / VS) & 1, s_fail, p.word, 5))) break;
+        if (step_last - blk.kt + 1 < AT_K && !(ok = at_wait(&v_clear[vs], 0, s_fail, p.word, 10))) break;
         if (blk.meets(mylo, myhi)) {
           const uint32_t buf = np & 1u;
-          if (!(ok = at_wait(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, 6))) break;
+          if (!(ok = at_wait(&p_full[2 * i + (int)buf], (np >> 1) & 1u, s_fail, p.word, 6))) break;
           tc_fence_after();
           const uint64_t vdesc = vdesc0 + (uint64_t)(vs * NBV * (AT_KBOX >> 4));
 #pragma unroll
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     bool ok = true;
     for (AtBlock blk(kt0, last, p.ring); ok && blk.any(); blk.next(), ++n) {
       const int keep = step_last - blk.kt + 1, vs = n % VS;
-      ok = __all_sync(0xffffffffu, at_wait(&v_full[vs], (n / VS) & 1, s_fail, 11));
+      ok = __all_sync(0xffffffffu, at_wait(&v_full[vs], (n / VS) & 1, s_fail, p.word, 11));
       if (ok && keep < AT_K) {
         const int pieces = (AT_K - keep) * 8;
         for (int e = lane; e < pieces * NBV; e += 32) {
@@ -428,7 +430,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next()) {
       if (blk.meets(mylo, myhi)) {
         const uint32_t ts = ts0 + 64u * (n & 1u);
-        ok = at_wait(&s_full[2 * tile + (int)(n & 1u)], (n >> 1) & 1u, s_fail, 7);
+        ok = at_wait(&s_full[2 * tile + (int)(n & 1u)], (n >> 1) & 1u, s_fail, p.word, 7);
         __syncwarp();
         tc_fence_after();
         uint32_t sr[AT_C];
@@ -476,7 +478,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           ref = nref;
           sum2[0] = f2_mul(sum2[0], f2_of(f, f));
           sum2[1] = f2_mul(sum2[1], f2_of(f, f));
-          if (n > 0) ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, 8);
+          if (n > 0) ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, p.word, 8);
           __syncwarp();
           tc_fence_after();
           if (at_any(1 + tile, !ok)) {                                      // (also: both threads of a row have read the other's)
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
       }
     }
     if (ok && n > 0 && t0 + tile * AT_Q < p.T) {
-      ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, 9);
+      ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, p.word, 9);
       __syncwarp();
       tc_fence_after();
       float s0, s1;
@@ -669,7 +671,7 @@ template <AttnTcKind KIND>
 int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
   const AtParams p{a.pos_ids, a.sink, a.slopes, (const __nv_bfloat16*)a.gate, (__nv_bfloat16*)a.y, a.scale, a.softcap, a.T, a.H, a.H / a.G,
                    a.v.dim, a.window, a.chunk, a.ring, a.gate_ld, a.gate_per_head,
-                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld};
+                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, wait_word()};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
   const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \

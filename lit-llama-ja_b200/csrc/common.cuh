@@ -36,9 +36,14 @@ int cuda_fail(cudaError_t e, const char* what);
   do {                                             \
     cudaError_t _e = cudaGetLastError();           \
     if (_e != cudaSuccess) return llb::cuda_fail(_e, name); \
+    if (int _w = llb::wait_check()) return _w;     \
   } while (0)
 
 int sm_count();
+// Where a kernel leaves the code of a bounded wait that ran out: mapped host memory, the same address on every device (null: there is
+// none).  wait_check: LL_OK, or LL_ERR_WAIT with the code in the error text, which is then cleared.
+int* wait_word();
+int wait_check();
 
 // Whether a kernel's attributes have been set on the current device: they belong to a device, not to the process.  Marked after they have
 // been set, so that a second thread sets them again instead of launching without them.
@@ -56,6 +61,11 @@ class PerDevice {
 };
 
 // ------------------------------------------------------------------ small device helpers
+__device__ __forceinline__ void wait_ran_out(int* word, int code) {
+  if (word == nullptr) return;
+  *reinterpret_cast<volatile int*>(word) = code;
+  __threadfence_system();
+}
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t b) { return __uint_as_float(b << 16); }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ uint16_t f32_to_bf16_bits(float x) {

@@ -45,6 +45,7 @@ struct DeltaChunkArgs {
   float* y;
   int T, H, qk_heads, n, p, chunks;
   DeltaScratch sc;
+  int* word;      // wait_word()
 };
 
 // four neighbouring numbers: o += a * x
@@ -376,10 +377,11 @@ __device__ __forceinline__ void dx_columns(uint32_t (&bf)[NF][2], const __nv_bfl
 constexpr uint32_t DX_WAIT_LIMIT = 1u << 22;
 __device__ int g_delta_chunk_error = 0;
 
-__device__ __forceinline__ bool dx_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool dx_wait(uint64_t* bar, uint32_t parity, int* word) {
   for (uint32_t i = 0; i < DX_WAIT_LIMIT; ++i)
     if (mbar_try_wait(bar, parity)) return true;
   atomicCAS(&g_delta_chunk_error, 0, 1);
+  wait_ran_out(word, 501);
   return false;
 }
 
@@ -464,7 +466,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) delta_pass_kernel(const DeltaCh
         *(uint32_t*)&Ss[(NP + row) * LU + cl] = t[1];
       }
     }
-    if (!dx_wait(&full[st], phase)) gave_up = 1;
+    if (!dx_wait(&full[st], phase, A.word)) gave_up = 1;
     __syncthreads();
     if (gave_up) {                     // the copies in flight get time to land before the block leaves; the host sees the code
       for (int i = 0; i < 2048; ++i) __nanosleep(512);
@@ -761,6 +763,7 @@ int ll_delta_chunked(const void* q, int q_stride, const void* k, int k_stride, c
   A.dt_bias = dt_bias, A.a_log = a_log, A.unit_eps = unit_eps, A.qs = qs, A.state = state, A.pos_ids = pos_ids, A.y = y;
   A.T = T, A.H = H, A.qk_heads = qk_heads, A.n = n, A.p = p, A.chunks = (T + DC_L - 1) / DC_L;
   const size_t cells = (size_t)B * H * A.chunks;
+  A.word = wait_word();
   A.sc.fac = scratch;
   A.sc.row = A.sc.fac + cells * DC_L;
   A.sc.tot = A.sc.row + cells * DC_L;

@@ -32,19 +32,21 @@ struct R4Params {
   const __nv_bfloat16* bias;
   __nv_bfloat16* y;
   int M, N, steps, G, steps_per_group, mtiles, tiles;
+  int* word;                     // wait_word()
 };
 
-__device__ __forceinline__ bool r4_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+__device__ __forceinline__ bool r4_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
   for (uint32_t i = 0; i < R4_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255u) == 255u && *fail) return false;
   }
   *fail = 1;
   atomicCAS(&g_r4_error, 0, code);
+  wait_ran_out(word, 200 + code);
   return false;
 }
 // The same without suspending the thread between looks: for the thread that feeds the tensor cores, whose wake-up would be waited for.
-__device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+__device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
   for (uint32_t i = 0; i < 64u * R4_WAIT_LIMIT; ++i) {
     uint32_t ok;
     asm volatile(
@@ -59,6 +61,7 @@ __device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, volatile
   }
   *fail = 1;
   atomicCAS(&g_r4_error, 0, code);
+  wait_ran_out(word, 200 + code);
   return false;
 }
 __device__ __forceinline__ void r4_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
         const int n0 = (tile / p.mtiles) * R4_N, m0 = (tile % p.mtiles) * BN;
         if (warp == 0) {
           for (int kb = 0; kb < steps; ++kb) {
-            if (!(ok = r4_wait(&x_empty[s], ph, s_fail, 1))) break;
+            if (!(ok = r4_wait(&x_empty[s], ph, s_fail, p.word, 1))) break;
             mbar_expect_tx(&x_full[s], XB);
             r4_box(sx + s * XB, &map_x, kb * R4_K, m0, &x_full[s]);
             r4_box(sx + s * XB + XB / 2, &map_x, kb * R4_K + 64, m0, &x_full[s]);
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
           }
         } else {
           for (int kb = 0; kb < steps; ++kb) {
-            if (!(ok = r4_wait(&w_empty[s], ph, s_fail, 2))) break;
+            if (!(ok = r4_wait(&w_empty[s], ph, s_fail, p.word, 2))) break;
             mbar_expect_tx(&w_full[s], R4_WBYTES);
             r4_box(sw + s * R4_WBYTES, &map_w, n0, kb * (R4_K / 2), &w_full[s]);
             if (++s == R4_WST) s = 0, ph ^= 1u;
@@ -165,10 +168,10 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
       int s = 0, tl = 0;
       uint32_t ph = 0, blk = 0;
       for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x, ++tl) {
-        if (tl > 0 && !(ok = r4_wait(d_empty, (uint32_t)(tl - 1) & 1u, s_fail, 3))) break;
+        if (tl > 0 && !(ok = r4_wait(d_empty, (uint32_t)(tl - 1) & 1u, s_fail, p.word, 3))) break;
         for (int kb = 0; ok && kb < steps; ++kb, ++blk) {
           const uint32_t buf = blk % R4_GROUPS;
-          if (!(ok = r4_spin(&x_full[s], ph, s_fail, 5) && r4_spin(&a_ready[buf], (blk / R4_GROUPS) & 1u, s_fail, 4))) break;
+          if (!(ok = r4_spin(&x_full[s], ph, s_fail, p.word, 5) && r4_spin(&a_ready[buf], (blk / R4_GROUPS) & 1u, s_fail, p.word, 4))) break;
           tc_fence_after();
           const uint64_t bd = xd + (uint64_t)(s * (XB >> 4));
 #pragma unroll
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
     bool ok = true;
     // a finished tile: its sums leave tensor memory, then the accumulator is given back, then they are stored
     auto drain = [&](int tile, uint32_t nth) {
-      ok = __all_sync(0xffffffffu, r4_wait(d_full, nth & 1u, s_fail, 6));
+      ok = __all_sync(0xffffffffu, r4_wait(d_full, nth & 1u, s_fail, p.word, 6));
       if (!ok) return;
       tc_fence_after();
       const int n = (tile / p.mtiles) * R4_N + col, m0 = (tile % p.mtiles) * BN + grp * PART;
@@ -251,8 +254,8 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
       normal();
       params(sn, zn);                        // of the next step, under this one's work
       const int s = grp;
-      ok = r4_wait(&w_full[s], round & 1u, s_fail, 7);
-      if (ok && round > 0) ok = r4_wait(&a_free[grp], (round - 1u) & 1u, s_fail, 8);
+      ok = r4_wait(&w_full[s], round & 1u, s_fail, p.word, 7);
+      if (ok && round > 0) ok = r4_wait(&a_free[grp], (round - 1u) & 1u, s_fail, p.word, 8);
       if (!(ok = __all_sync(0xffffffffu, ok))) break;
       tc_fence_after();
       const uint8_t* src = sw + s * R4_WBYTES + col;
@@ -348,6 +351,7 @@ int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const
   R4Params p{};
   p.scales = (const __nv_bfloat16*)scales, p.zeros = (const __nv_bfloat16*)zeros, p.bias = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
+  p.word = wait_word();
   const int sms = sm_count();
   CUtensorMap mw;
   if (int r = r4_weight_map(qw, N, K, &mw)) return r;

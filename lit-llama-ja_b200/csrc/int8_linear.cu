@@ -159,13 +159,14 @@ constexpr int I8_BN = 128, I8_STAGES = 3, I8_BOX = 128 * 128;
 constexpr uint32_t I8_WAIT_LIMIT = 1u << 20;
 __device__ int g_int8_tc_error = 0;
 
-__device__ __forceinline__ bool i8_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+__device__ __forceinline__ bool i8_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
   for (uint32_t i = 0; i < I8_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255u) == 255u && *fail) return false;
   }
   *fail = 1;
   atomicCAS(&g_int8_tc_error, 0, code);
+  wait_ran_out(word, 300 + code);
   return false;
 }
 __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -183,7 +184,7 @@ __device__ __forceinline__ void i8_box(void* dst, const CUtensorMap* map, int x,
 }
 
 __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                                             int32_t* __restrict__ c, int M, int N, int K) {
+                                                             int32_t* __restrict__ c, int M, int N, int K, int* word) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
   uint8_t *sa = base, *sb = base + I8_STAGES * I8_BOX;
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % I8_STAGES;
-        if (!(ok = i8_wait(&empty[s], ((kb / I8_STAGES) & 1) ^ 1, s_fail, 1))) break;
+        if (!(ok = i8_wait(&empty[s], ((kb / I8_STAGES) & 1) ^ 1, s_fail, word, 1))) break;
         mbar_expect_tx(&full[s], 2 * I8_BOX);
         i8_box(sa + s * I8_BOX, &map_a, kb * 128, m0, &full[s]);
         i8_box(sb + s * I8_BOX, &map_b, kb * 128, n0, &full[s]);
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
       bool ok = true;
       for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb % I8_STAGES;
-        if (!(ok = i8_wait(&full[s], (kb / I8_STAGES) & 1, s_fail, 2))) break;
+        if (!(ok = i8_wait(&full[s], (kb / I8_STAGES) & 1, s_fail, word, 2))) break;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -239,9 +240,9 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
     }
   } else {
     const int quarter = warp & 3, m = m0 + quarter * 32 + lane;
-    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, 3));
+    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, word, 3) && *(volatile int*)s_fail == 0);
     tc_fence_after();
-    if (ok && *(volatile int*)s_fail == 0) {
+    if (ok) {
 #pragma unroll 1
       for (int c0 = 0; c0 < I8_BN; c0 += 32) {
         if (n0 + c0 >= N) break;
@@ -492,7 +493,7 @@ int int8_rows_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* sc
     int8_row_quant_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(xp, w.flag, w.sca, w.ca, K, thr, pieces, vec);
     int8_lists_kernel<<<blocks, 1024, 0, st>>>(w.flag, w.idx, w.count, K);
     if (int r = make_map_i8(w.ca, rows, K, 128, &ma)) return r;
-    int8_gemm_tc_kernel<<<dim3((rows + BM - 1) / BM, (N + I8_BN - 1) / I8_BN), 192, smem, st>>>(ma, mb, w.c32, rows, N, K);
+    int8_gemm_tc_kernel<<<dim3((rows + BM - 1) / BM, (N + I8_BN - 1) / I8_BN), 192, smem, st>>>(ma, mb, w.c32, rows, N, K, wait_word());
     int8_finish_rows_kernel<T, 64><<<dim3((N + 63) / 64, blocks), 256, 0, st>>>(w.c32, 1, 0, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count,
                                                                            y + (size_t)r0 * N, rows, N, K);
     LL_LAUNCH_OK("int8 linear kernels (prompts)");
@@ -621,7 +622,7 @@ constexpr int i8c_stages(int mp) { return mp > 32 ? 4 : 5; }
 constexpr int i8c_smem(int mp) { return i8c_stages(mp) * (I8_BOX + mp * 128) + 256 + 1024; }
 template <int MP>
 __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                                                                int32_t* __restrict__ part, int M, int N, int nkb, int per) {
+                                                                int32_t* __restrict__ part, int M, int N, int nkb, int per, int* word) {
   constexpr int STAGES = i8c_stages(MP), XB = MP * 128, COLS = MP <= 32 ? 32 : 64;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
       int s = 0;
       uint32_t ph = 1;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!(ok = i8_wait(&empty[s], ph, s_fail, 5))) break;
+        if (!(ok = i8_wait(&empty[s], ph, s_fail, word, 5))) break;
         mbar_expect_tx(&full[s], I8_BOX + XB);
         i8_box(sw + s * I8_BOX, &map_w, kb * 128, n0, &full[s]);
         i8_box(sx + s * XB, &map_x, kb * 128, 0, &full[s]);
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
       int s = 0;
       uint32_t ph = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!(ok = i8_wait(&full[s], ph, s_fail, 6))) break;
+        if (!(ok = i8_wait(&full[s], ph, s_fail, word, 6))) break;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -681,9 +682,9 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
     }
   } else {
     const int quarter = warp & 3, n = n0 + quarter * 32 + lane;
-    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, 7));
+    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, word, 7) && *(volatile int*)s_fail == 0);
     tc_fence_after();
-    if (ok && *(volatile int*)s_fail == 0) {
+    if (ok) {
       int32_t* dst = part + (size_t)blockIdx.y * M * N + n;
 #pragma unroll
       for (int c0 = 0; c0 < COLS; c0 += 32) {
@@ -743,7 +744,7 @@ int i8c_launch(const CUtensorMap& mw, const Ws& w, int M, int N, int K, int sms,
   LL_CUDA(cudaFuncSetAttribute(int8_columns_tc_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, i8c_smem(MP)));
   int per;
   const int ranges = i8c_ranges(N, K, sms, &per);
-  int8_columns_tc_kernel<MP><<<dim3((N + 127) / 128, ranges), 192, i8c_smem(MP), st>>>(mw, mx, w.part, M, N, K / 128, per);
+  int8_columns_tc_kernel<MP><<<dim3((N + 127) / 128, ranges), 192, i8c_smem(MP), st>>>(mw, mx, w.part, M, N, K / 128, per, wait_word());
   LL_LAUNCH_OK("int8_columns_tc_kernel");
   return LL_OK;
 }

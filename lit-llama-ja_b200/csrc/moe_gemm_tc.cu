@@ -46,13 +46,14 @@ constexpr uint32_t MT_WAIT_LIMIT = 1u << 22;
 __device__ int g_moe_tc_error = 0;
 
 // A wait that ends: on its phase, when another role has given up, or after the limit.
-__device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int code) {
+__device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
   for (uint32_t i = 0; i < MT_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((i & 255u) == 255u && *fail) return false;
   }
   *fail = 1;
   atomicCAS(&g_moe_tc_error, 0, code);
+  wait_ran_out(word, 400 + code);
   return false;
 }
 
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) moe_gemm_tc_kernel(const __grid
                                                                     const __grid_constant__ CUtensorMap map_b,
                                                                     const int32_t* __restrict__ offsets, const int32_t* __restrict__ perm,
                                                                     int X, int N, int K, float limit, float alpha, float shift,
-                                                                    __nv_bfloat16* __restrict__ c, int ldc) {
+                                                                    __nv_bfloat16* __restrict__ c, int ldc, int* word) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
   uint8_t* sa = base;                              // [STAGES][128][64] bf16, swizzled
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) moe_gemm_tc_kernel(const __grid
         const int brow0 = MODE == 1 ? walk.e * 2 * N + n0 : walk.e * N + n0;
         const int brow1 = MODE == 1 ? brow0 + N : brow0 + MT_BN;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mt_wait(&empty[s], phase ^ 1, s_fail, 1)) { ok = false; break; }
+          if (!mt_wait(&empty[s], phase ^ 1, s_fail, word, 1)) { ok = false; break; }
           mbar_expect_tx(&full[s], MT_A_BYTES + MT_B_BYTES);
           tma_box(sa + s * MT_A_BYTES, &map_a, kb * BK, r0, &full[s]);
           tma_box(sb + s * MT_B_BYTES, &map_b, kb * BK, brow0, &full[s]);
@@ -167,10 +168,10 @@ __global__ void __launch_bounds__(MT_THREADS, 1) moe_gemm_tc_kernel(const __grid
       bool ok = true;
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++i) {
         const uint32_t d = tmem_d + (uint32_t)((i & 1) * MT_COLS);
-        if (!mt_wait(&acc_empty[i & 1], ((i >> 1) & 1) ^ 1, s_fail, 4)) break;
+        if (!mt_wait(&acc_empty[i & 1], ((i >> 1) & 1) ^ 1, s_fail, word, 4)) break;
         tc_fence_after();
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mt_wait(&full[s], phase, s_fail, 2)) { ok = false; break; }
+          if (!mt_wait(&full[s], phase, s_fail, word, 2)) { ok = false; break; }
           tc_fence_after();
           const uint64_t adesc = smem_desc_sw128(smem_u32(sa + s * MT_A_BYTES));
           const uint64_t bdesc = smem_desc_sw128(smem_u32(sb + s * MT_B_BYTES));
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(MT_THREADS, 1) moe_gemm_tc_kernel(const __grid
       const bool row_ok = row < walk.end;
       const long long dst_row = !row_ok || MODE != 0 ? (long long)row : (long long)perm[row];
       __nv_bfloat16* dst = c + dst_row * ldc;
-      if (!__all_sync(0xffffffffu, mt_wait(&acc_full[i & 1], (i >> 1) & 1, s_fail, 3))) break;
+      if (!__all_sync(0xffffffffu, mt_wait(&acc_full[i & 1], (i >> 1) & 1, s_fail, word, 3))) break;
       tc_fence_after();
       const uint32_t trow = tmem_d + (uint32_t)((i & 1) * MT_COLS) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
@@ -273,7 +274,7 @@ int launch_moe_tc(const CUtensorMap& ma, const CUtensorMap& mb, const int32_t* o
   const long long most = (long long)((N + ncols - 1) / ncols) * ((n_rows + BM - 1) / BM + X);
   LL_CHECK_ARG(most < (1ll << 30), "moe_grouped_gemm_tc: too many tiles");
   const int grid = (int)std::min<long long>(most, sm_count() > 0 ? sm_count() : 148);
-  moe_gemm_tc_kernel<MODE><<<grid, MT_THREADS, smem, st>>>(ma, mb, offsets, perm, X, N, K, limit, alpha, shift, (__nv_bfloat16*)c, ldc);
+  moe_gemm_tc_kernel<MODE><<<grid, MT_THREADS, smem, st>>>(ma, mb, offsets, perm, X, N, K, limit, alpha, shift, (__nv_bfloat16*)c, ldc, wait_word());
   LL_LAUNCH_OK("moe_gemm_tc_kernel");
   return LL_OK;
 }

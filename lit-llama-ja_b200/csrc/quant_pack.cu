@@ -2,6 +2,8 @@
 // ref: /root/reference/lit_llama/quantization.py:339-421 (ColBlockQuantizedLinear).
 #include <stdarg.h>
 
+#include <mutex>
+
 #include "common.cuh"
 
 namespace llb {
@@ -17,6 +19,36 @@ void set_error(const char* fmt, ...) {
 int cuda_fail(cudaError_t e, const char* what) {
   set_error("CUDA error %d (%s) at %s", (int)e, cudaGetErrorString(e), what);
   return LL_ERR_CUDA;
+}
+static std::atomic<int*> g_wait_word{nullptr};
+int* wait_word() {
+  static std::once_flag once;
+  std::call_once(once, [] {
+    // the first launch may be one that is being captured: this allocation has nothing to do with the capture
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool exchanged = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    int* p = nullptr;
+    if (cudaHostAlloc((void**)&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      *p = 0;
+      g_wait_word.store(p, std::memory_order_release);
+    } else {
+      cudaGetLastError();
+    }
+    if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
+  });
+  return g_wait_word.load(std::memory_order_acquire);
+}
+static std::atomic<int> g_wait_host{0};      // what ll_wait_report leaves where there is no device to share memory with
+int wait_check() {
+  volatile int* p = g_wait_word.load(std::memory_order_acquire);
+  int code = p ? *p : 0;
+  if (code != 0) *p = 0;
+  if (g_wait_host.load(std::memory_order_relaxed) != 0) code = g_wait_host.exchange(0, std::memory_order_relaxed);
+  if (code == 0) return LL_OK;
+  static const char* const where[] = {"", "prompt attention", "int4 rows", "llm.int8", "grouped experts", "delta rule in chunks"};
+  set_error("a bounded wait ran out in an earlier launch (%s, code %d): what it and the launches after it wrote is not valid",
+            code >= 100 && code < 600 ? where[code / 100] : "?", code);
+  return LL_ERR_WAIT;
 }
 int sm_count() {
   static int n = 0;
@@ -194,6 +226,13 @@ extern "C" {
 
 const char* ll_last_error(void) { return g_err; }
 int ll_abi_version(void) { return LL_ABI_VERSION; }
+int ll_wait_check(void) { return wait_check(); }
+int ll_wait_report(int code) {
+  if (int* p = g_wait_word.load(std::memory_order_acquire)) *reinterpret_cast<volatile int*>(p) = code;
+  else g_wait_host.store(code, std::memory_order_relaxed);
+  return LL_OK;
+}
+
 int ll_sm_count(void) {
   int n = sm_count();
   if (n < 0) set_error("no CUDA device");

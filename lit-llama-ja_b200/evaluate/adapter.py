@@ -14,6 +14,7 @@ wd = Path(__file__).absolute().parent.parent
 sys.path.insert(0, str(wd))
 
 from lit_llama import Tokenizer  # noqa: E402
+from lit_llama._native import check_waits  # noqa: E402
 
 
 def _load(rel: str, name: str):
@@ -56,6 +57,7 @@ def run(data_paths, accelerator, adapter_path, checkpoint_path, tokenizer_path, 
         print(f"Perplexity on {path}: {ppl:.2f}")
         total_toks += toks
     torch.cuda.synchronize()
+    check_waits()
     t = time.perf_counter() - t0
     print(f"\n\nTime for inference: {t:.02f} sec total, {total_toks / t:.02f} tokens/sec", file=sys.stderr)
     print(f"Memory used: {torch.cuda.max_memory_reserved() / 1e9:.02f} GB", file=sys.stderr)

@@ -17,6 +17,7 @@ wd = Path(__file__).absolute().parent.parent
 sys.path.insert(0, str(wd))
 
 from lit_llama import LLaMA, Tokenizer  # noqa: E402
+from lit_llama._native import check_waits  # noqa: E402
 from lit_llama.utils import EmptyInitOnDevice, lazy_load, stream_load_state_dict  # noqa: E402
 
 
@@ -78,6 +79,7 @@ def main(
         print(f"Perplexity on {path}: {ppl:.2f}")
         total_toks += toks
     torch.cuda.synchronize()
+    check_waits()
     t = time.perf_counter() - t0
     print(f"\n\nTime for inference: {t:.02f} sec total, {total_toks / t:.02f} tokens/sec", file=sys.stderr)
     print(f"Memory used: {torch.cuda.max_memory_reserved() / 1e9:.02f} GB", file=sys.stderr)

@@ -16,6 +16,7 @@ import torch
 sys.path.insert(0, str(Path(__file__).parent.resolve()))
 
 from lit_llama import LLaMA, HFTokenizer, Tokenizer  # noqa: E402
+from lit_llama._native import check_waits  # noqa: E402
 from lit_llama.utils import EmptyInitOnDevice, lazy_load, llama_model_lookup  # noqa: E402
 
 
@@ -163,6 +164,7 @@ def main(
         t0 = time.perf_counter()
         y = generate(model, encoded, max_new_tokens, temperature=temperature, top_k=top_k)
         torch.cuda.synchronize()
+        check_waits()
         t = time.perf_counter() - t0
         model.reset_cache()
         print(tokenizer.decode(y) if tokenizer is not None else ",".join(str(int(t)) for t in y))

@@ -13,6 +13,7 @@ wd = Path(__file__).absolute().parent.parent
 sys.path.insert(0, str(wd))
 
 from lit_llama import Tokenizer  # noqa: E402
+from lit_llama._native import check_waits  # noqa: E402
 from lit_llama.adapter import LLaMA  # noqa: E402
 from lit_llama.utils import EmptyInitOnDevice, lazy_load, llama_model_lookup, stream_load_state_dict  # noqa: E402
 import generate as _gen  # noqa: E402  (generate.py next to this directory: the module wins over the namespace package)
@@ -67,6 +68,7 @@ def run(prompt, input, adapter_path, pretrained_path, tokenizer_path, quantize, 
     t0 = time.perf_counter()
     y = _gen.generate(model, encoded, max_new_tokens, temperature=temperature, top_k=top_k, eos_id=tokenizer.eos_id)
     torch.cuda.synchronize()
+    check_waits()
     t = time.perf_counter() - t0
     model.reset_cache()
     output = tokenizer.decode(y)

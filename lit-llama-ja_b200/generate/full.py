@@ -12,6 +12,7 @@ wd = Path(__file__).absolute().parent.parent
 sys.path.insert(0, str(wd))
 
 from lit_llama import LLaMA, Tokenizer  # noqa: E402
+from lit_llama._native import check_waits  # noqa: E402
 from lit_llama.utils import EmptyInitOnDevice, lazy_load, stream_load_state_dict  # noqa: E402
 import generate as _gen  # noqa: E402  (generate.py next to this directory: the module wins over the namespace package)
 
@@ -75,6 +76,7 @@ def main(
         t0 = time.perf_counter()
         y = _gen.generate(model, encoded, max_new_tokens, temperature=temperature, top_k=top_k)
         torch.cuda.synchronize()
+        check_waits()
         t = time.perf_counter() - t0
         model.reset_cache()
         print(tokenizer.decode(y))

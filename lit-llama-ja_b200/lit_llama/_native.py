@@ -66,6 +66,8 @@ def _proto(name, argtypes, restype=C.c_int):
 # every symbol include/llb200.h declares
 EXPORTS = {
     "ll_last_error": ([], C.c_char_p),
+    "ll_wait_check": ([], C.c_int),
+    "ll_wait_report": ([i32], C.c_int),
     "ll_abi_version": ([], C.c_int),
     "ll_sm_count": ([], C.c_int),
     "ll_pack_weight": ([vp, i32, vp, vp, i32, vp, i32, i32, i32, i32, vp], C.c_int),
@@ -189,7 +191,7 @@ EXPORTS = {
 }
 _fn = {name: _proto(name, a, r) for name, (a, r) in EXPORTS.items()}
 
-ABI_VERSION = 18
+ABI_VERSION = 19
 if _fn["ll_abi_version"]() != ABI_VERSION:
     raise ImportError("libllb200.so ABI version mismatch; rebuild with lit-llama-ja_b200/build.py")
 
@@ -212,6 +214,12 @@ def call(name: str, *args) -> None:
     if rc != 0:
         check(rc, name)
     LAUNCHES += 1
+
+
+def check_waits() -> None:
+    """Raise if a bounded wait inside an earlier launch ran out (its results are not valid).  Looks at host memory only: call it where the
+    host has synchronised with the work it is about to use.  (Every later launch raises as well.)"""
+    check(_fn["ll_wait_check"](), "an earlier launch")
 
 
 def has(name: str) -> bool:

@@ -92,6 +92,7 @@ class PortionedDecoder(nn.Module):
             pos0, max_seq_length = 0, T
         else:
             pos0 = int(input_pos[0])
+            N.check_waits()                    # (reading the position has waited for the steps before)
             if max_seq_length is None:         # the length the memory was last sized for, unless the sequence outgrows it
                 max_seq_length = max(pos0 + T, self._sized_for)
             self._sized_for = max_seq_length

@@ -156,3 +156,22 @@ def test_long_outlier_lists(M, outliers, N, transposed):
     odd, size = a[:, out] @ wo.t(), a[:, out].abs() @ wo.abs().t()
     # as above: both parts and their sum rounded to fp16, an outlier's weight possibly on its other fp16 neighbour
     assert ((y.double() - want - odd).abs() <= 2.0 ** -11 * (want.abs() + odd.abs() + (want + odd).abs()) * 1.01 + 2.0 ** -10 * size + 1e-4).all()
+
+
+def test_a_wait_that_ran_out_fails_the_next_launch():
+    from lit_llama import _native as NV
+
+    x = torch.ones(64, device="cuda")
+    y = torch.empty_like(x)
+    args = (NV.ptr(x), NV.ptr(x), NV.ptr(y), NV.LL_F32, 64, NV.stream())
+    w = torch.zeros((128, 128), dtype=torch.int8, device="cuda")       # (a launch that shares the word with its kernel)
+    ws = torch.empty(NV.call_ret("ll_int8_workspace_bytes", 1, 128, 128), dtype=torch.uint8, device="cuda")
+    a, o, s = torch.zeros((1, 128), device="cuda"), torch.empty((1, 128), device="cuda"), torch.ones(128, device="cuda")
+    NV.call("ll_int8_linear", NV.ptr(a), NV.LL_F32, NV.ptr(w), None, NV.ptr(s), None, NV.ptr(o), 1, 128, 128, 6.0, NV.ptr(ws), ws.numel(), NV.stream())
+    NV.call("ll_add", *args)
+    NV.call_ret("ll_wait_report", 203)                                 # as a kernel leaves it
+    with pytest.raises(RuntimeError, match="int4 rows, code 203"):
+        NV.call("ll_add", *args)
+    NV.call("ll_add", *args)
+    torch.cuda.synchronize()
+    assert bool((y == 2).all())

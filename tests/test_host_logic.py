@@ -120,3 +120,13 @@ def test_kernel_attributes_are_set_per_device():
 
     for path in sorted((Path(__file__).resolve().parent.parent / "lit-llama-ja_b200" / "csrc").glob("*.cu*")):
         assert not re.search(r"static\s+bool\s+\w+\s*=", path.read_text()), path.name
+
+
+def test_a_wait_that_ran_out_is_raised_once():
+    from lit_llama import _native as N
+
+    N.check_waits()
+    N.call_ret("ll_wait_report", 307)
+    with pytest.raises(RuntimeError, match="llm.int8, code 307"):
+        N.check_waits()
+    N.check_waits()
