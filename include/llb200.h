@@ -196,6 +196,10 @@ LL_API int ll_gemm_bf16_tc(const void* x, const void* w, const void* bias, void*
 LL_API int ll_int4_rows_supported(int N, int K, int group);
 LL_API int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K,
                         int group, ll_stream stream);
+/* The same with tiles of tile_rows rows (128, 192 or 256; 0: the cheapest) on at most `grid` blocks (0: one an SM): which form runs is
+ * otherwise a matter of the sizes. */
+LL_API int ll_int4_rows_form(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N,
+                             int K, int group, int tile_rows, int grid, ll_stream stream);
 LL_API int ll_int4_rows_error(void);
 /* Fused int4 de-quantise + GEMM on tcgen05 for 1 <= M <= 128 rows (batched decode, short prefill; the HBM-bound regime):
  * y[M][N] (bf16) = x[M][K] (bf16) . W^T (+ bias), W de-quantised INSIDE the main loop from the packed stream

@@ -149,11 +149,6 @@ __device__ __forceinline__ f2 f2_of(float a, float b) {
 }
 __device__ __forceinline__ void f2_split(f2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
-#ifdef AT_SCALAR
-  float a0, a1, b0, b1, c0, c1;
-  f2_split(a, a0, a1), f2_split(b, b0, b1), f2_split(c, c0, c1);
-  return f2_of(fmaf(a0, b0, c0), fmaf(a1, b1, c1));
-#endif
   f2 r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;

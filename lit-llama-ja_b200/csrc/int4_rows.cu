@@ -21,7 +21,7 @@ constexpr int R4_N = 128, R4_K = 128, R4_GROUPS = 4, R4_THREADS = (4 + 4 * R4_GR
 constexpr int R4_WBYTES = R4_N * R4_K / 2, R4_WST = R4_GROUPS;         // a stage of packed bytes per group
 constexpr uint32_t R4_WAIT_LIMIT = 1u << 20;
 __host__ __device__ constexpr int r4_xbytes(int bn) { return bn * R4_K * 2; }
-__host__ __device__ constexpr int r4_xst(int bn) { return bn >= 256 ? 3 : bn >= 192 ? 4 : bn >= 128 ? 6 : 8; }
+__host__ __device__ constexpr int r4_xst(int bn) { return bn >= 256 ? 3 : bn >= 192 ? 4 : 6; }
 constexpr int r4_smem(int bn) { return r4_xst(bn) * r4_xbytes(bn) + R4_WST * R4_WBYTES + 512 + 1024; }
 
 __device__ int g_r4_error = 0;
@@ -314,18 +314,19 @@ int r4_weight_map(const void* qw, int N, int K, CUtensorMap* out) {
 }
 
 template <int BN>
-int r4_launch(const CUtensorMap& mw, const void* x, R4Params p, int K, int sms, cudaStream_t st) {
+int r4_launch(const CUtensorMap& mw, const void* x, R4Params p, int K, int grid, cudaStream_t st) {
   CUtensorMap mx;
   if (int r = make_map(x, p.M, K, BN, &mx)) return r;
   LL_CUDA(cudaFuncSetAttribute(int4_rows_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, r4_smem(BN)));
   p.mtiles = (p.M + BN - 1) / BN;
   p.tiles = p.mtiles * ((p.N + R4_N - 1) / R4_N);
-  int4_rows_kernel<BN><<<p.tiles < sms ? p.tiles : sms, R4_THREADS, r4_smem(BN), st>>>(mw, mx, p);
+  int4_rows_kernel<BN><<<p.tiles < grid ? p.tiles : grid, R4_THREADS, r4_smem(BN), st>>>(mw, mx, p);
   LL_LAUNCH_OK("int4_rows_kernel");
   return LL_OK;
 }
 
-// Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time (see the head of the file), plus the drain.
+// Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time (see the head of the file), plus the drain.  (A
+// step takes 600 clocks at least, however few the rows: tiles of 64 never cost less than tiles of 128.)
 long long r4_cost(int M, int N, int steps, int bn, int sms) {
   const long long tiles = (long long)((M + bn - 1) / bn) * ((N + R4_N - 1) / R4_N);
   return (tiles + sms - 1) / sms * ((long long)steps * (4 * bn > 600 ? 4 * bn : 600) + 1200);
@@ -342,6 +343,11 @@ int ll_int4_rows_supported(int N, int K, int group) { return N > 0 && N % 16 == 
 
 int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K, int group,
                  ll_stream stream) {
+  return ll_int4_rows_form(qw, scales, zeros, x, bias, y, M, N, K, group, 0, 0, stream);
+}
+
+int ll_int4_rows_form(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K,
+                      int group, int tile_rows, int grid, ll_stream stream) {
   LL_CHECK_ARG(qw && scales && zeros && x && y && M > 0, "int4_rows: null pointer or no rows");
   if (!ll_int4_rows_supported(N, K, group)) {
     set_error("int4_rows needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
@@ -352,17 +358,19 @@ int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const
   p.scales = (const __nv_bfloat16*)scales, p.zeros = (const __nv_bfloat16*)zeros, p.bias = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
   p.word = wait_word();
-  const int sms = sm_count();
+  LL_CHECK_ARG((tile_rows == 0 || tile_rows == 128 || tile_rows == 192 || tile_rows == 256) && grid >= 0, "int4_rows: tiles of 128, 192 or 256 rows");
+  if (grid == 0) grid = sm_count();
   CUtensorMap mw;
   if (int r = r4_weight_map(qw, N, K, &mw)) return r;
-  int best = 256;
-  for (int bn = 192; bn >= 64; bn -= 64)
-    if (r4_cost(M, N, p.steps, bn, sms) < r4_cost(M, N, p.steps, best, sms)) best = bn;
+  if (tile_rows == 0) {
+    tile_rows = 256;
+    for (int bn = 192; bn >= 128; bn -= 64)
+      if (r4_cost(M, N, p.steps, bn, grid) < r4_cost(M, N, p.steps, tile_rows, grid)) tile_rows = bn;
+  }
   cudaStream_t st = (cudaStream_t)stream;
-  if (best == 256) return r4_launch<256>(mw, x, p, K, sms, st);
-  if (best == 192) return r4_launch<192>(mw, x, p, K, sms, st);
-  if (best == 128) return r4_launch<128>(mw, x, p, K, sms, st);
-  return r4_launch<64>(mw, x, p, K, sms, st);
+  if (tile_rows == 256) return r4_launch<256>(mw, x, p, K, grid, st);
+  if (tile_rows == 192) return r4_launch<192>(mw, x, p, K, grid, st);
+  return r4_launch<128>(mw, x, p, K, grid, st);
 }
 
 // 0, or the code of the first bounded wait that ran out in this file's kernel.  Synchronises the device.

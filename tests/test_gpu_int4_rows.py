@@ -1,5 +1,5 @@
-"""The many-row int4 kernel (weights de-quantised into tensor memory) against the unpacked weights through plain fp32 products: edges of row
-tiles (64, 128, 192, 256), a last column tile that is not full, one and many steps of 128 k, several groups a row, fractional zeros, a bias."""
+"""The many-row int4 kernel (weights de-quantised into tensor memory) against the unpacked weights through 64-bit products: edges of row
+tiles (128, 192, 256) and several tiles a block, a last column tile that is not full, one and many steps of 128 k, several groups a row, fractional zeros, a bias."""
 import pytest
 import torch
 
@@ -70,3 +70,32 @@ def test_longest_steps(M):
     w = lin.get_weight(torch.bfloat16).double()
     want, size = x.double() @ w.t(), x.double().abs() @ w.abs().t()
     assert ((lin(x).double() - want).abs() <= want.abs() * 2.0 ** -8 + size * 256 * 2.0 ** -24 + 1e-30).all()
+
+
+@pytest.mark.parametrize("tile_rows", [128, 192, 256])
+@pytest.mark.parametrize("grid", [1, 2, 5])
+@pytest.mark.parametrize("M,N,K,group", [(513, 400, 128, 128), (700, 272, 384, 128), (260, 1040, 640, 640), (513, 528, 1280, 256)])
+def test_blocks_that_walk_several_tiles(tile_rows, grid, M, N, K, group):
+    """Every tile size with few blocks, so that each walks three tiles and more: one, three, five and ten steps a tile (the four groups take
+    every fourth step, across tiles), partial last tiles of rows and columns, fractional zeros, a bias."""
+    from lit_llama import _native as NV
+    from lit_llama.quantization import ColBlockQuantizedLinear
+
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    lin = ColBlockQuantizedLinear(K, N, True, bits=4, tile_cols=group).to("cuda", torch.bfloat16)
+    lin.quant_weight.copy_(torch.randint(0, 256, lin.quant_weight.shape, generator=g, device="cuda", dtype=torch.uint8))
+    lin.scales.copy_(torch.rand(lin.scales.shape, generator=g, device="cuda") * 0.02 + 0.005)
+    z = torch.randint(0, 16, lin.zeros.shape, generator=g, device="cuda").float()
+    z[::3] += 0.37                                                     # whole zeros beside fractional ones
+    lin.zeros.copy_(z)
+    lin.bias.copy_(torch.randn(N, generator=g, device="cuda"))
+    x = torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16)
+    y = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert ((M + tile_rows - 1) // tile_rows) * ((N + 127) // 128) >= 3 * grid or grid == 5
+    NV.call("ll_int4_rows_form", NV.ptr(lin.quant_weight), NV.ptr(lin.scales), NV.ptr(lin.zeros), NV.ptr(x), NV.ptr(lin.bias), NV.ptr(y), M, N, K,
+            group, tile_rows, grid, NV.stream())
+    torch.cuda.synchronize()
+    assert NV.call_ret("ll_int4_rows_error") == 0 and bool((y[M] == 7.0).all())
+    w = lin.get_weight(dtype=torch.bfloat16).double()
+    want, size = x.double() @ w.t() + lin.bias.double(), x.double().abs() @ w.abs().t()
+    assert ((y[:M].double() - want).abs() <= want.abs() * 2.0 ** -8 + size * K * 2.0 ** -24 + 1e-30).all()
