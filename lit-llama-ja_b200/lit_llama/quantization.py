@@ -363,12 +363,14 @@ _INT8_WS: dict = {}
 
 
 def _int8_workspace(device, nbytes: int) -> torch.Tensor:
-    """Per-(device, stream) scratch of the int8 linear (kernels on one stream are ordered)."""
+    """Per-(device, stream) scratch of the int8 linear (kernels on one stream are ordered).  An outgrown buffer stays: a graph captured with
+    its address writes to it at every replay.  Each is at least twice the one before, so that together they stay below twice the largest."""
     key = (device.index, N.stream())
-    ws = _INT8_WS.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = _INT8_WS[key] = torch.empty(nbytes + 256, dtype=torch.uint8, device=device)
-    return ws
+    held = _INT8_WS.get(key)
+    if held is None or held[-1].numel() < nbytes:
+        held = _INT8_WS.setdefault(key, [])
+        held.append(torch.empty(max(nbytes + 256, 2 * held[-1].numel() if held else 0), dtype=torch.uint8, device=device))
+    return held[-1]
 
 
 # --------------------------------------------------------------------------------------- row Z

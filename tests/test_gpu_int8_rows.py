@@ -175,3 +175,29 @@ def test_a_wait_that_ran_out_fails_the_next_launch():
     NV.call("ll_add", *args)
     torch.cuda.synchronize()
     assert bool((y == 2).all())
+
+
+def test_a_captured_call_keeps_its_workspace():
+    """A step captured with a small workspace is replayed after a longer prompt on its stream needed a larger one: it still writes to its own."""
+    from lit_llama.quantization import Linear8bitLt
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    K, Nout, st = 1024, 2048, torch.cuda.Stream()
+    lin = Linear8bitLt(K, Nout, bias=False, device="cuda", dtype=torch.float32)
+    lin.load_state_dict({"weight": torch.randn((Nout, K), generator=g, device="cuda") * 0.05})
+    x, long = torch.randn((8, K), generator=g, device="cuda"), torch.randn((900, K), generator=g, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(st):
+        want = lin(x)
+        st.synchronize()
+        with torch.cuda.graph(graph, stream=st):
+            y = lin(x)
+        lin(long)
+        st.synchronize()
+        others = [torch.full((n,), 0x33, dtype=torch.uint8, device="cuda") for n in (1 << 17, 1 << 18, 1 << 19, 1 << 20, 1 << 21, 3 << 20) for _ in range(8)]
+        for _ in range(3):
+            graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    assert all(bool((o == 0x33).all()) for o in others)
