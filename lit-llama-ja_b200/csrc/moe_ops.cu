@@ -18,14 +18,13 @@
 namespace llb {
 
 constexpr int RT_THREADS = 256;
-constexpr int RT_WIDE_M = 8 * 148, RT_NARROW_M = 149;
 constexpr size_t RT_WIDE_SMEM = 100 * 1024;   // two blocks a SM
 constexpr int RT_EG = 4;         // experts a warp accumulates side by side
 enum { SCORE_CHOSEN = 0, SCORE_ALL = 1, SCORE_SIGMOID = 2 };
 
 // One block routes RT_TOK tokens and reads the whole router for them: bound by the latency of those reads while the blocks fit
 // the chip at once, and by their number (X * dim * 4 bytes a block, from L2) for long prompts.  So a token to a block while
-// every token gets its own SM (M < RT_NARROW_M), eight once every SM has a block of eight (RT_WIDE_M), four between; the sums
+// every token gets its own SM, eight once every SM has a block of eight, four between; the sums
 // are the same numbers in every form.  32 experts of width 2048, us by M (one / four / eight tokens a block):
 // 148: 8.7 / 12.5, 300: 12.6 with four, 15.5 with eight, 1183: 15.2 / 17.2, 2048: 37 with four, 19 with eight; four tokens a
 // block at every M, with weights loaded where they are used: 16 at M = 1, 34 at 2048.
@@ -569,7 +568,8 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
     return LL_ERR_UNSUPPORTED;
   }
   LL_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * n_experts, st));
-  const int tok = M >= RT_WIDE_M && 8 * per_token <= RT_WIDE_SMEM ? 8 : M < RT_NARROW_M ? 1 : 4;
+  const int sms = sm_count();
+  const int tok = M >= 8 * sms && 8 * per_token <= RT_WIDE_SMEM ? 8 : M <= sms ? 1 : 4;
   const int blocks = (M + tok - 1) / tok;
   const size_t smem = tok * per_token;
 #define LL_RT_TOK(T, TOK)                                                                                                            \
