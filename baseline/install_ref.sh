@@ -1,6 +1,6 @@
 #!/bin/bash
-# Installs the UNMODIFIED reference (if001/lit-llama-ja) into baseline/_ref (git-ignored; it travels to the GPU box with
-# the gpurun snapshot).  The reference tree is read-only and its setup.py lists git dependencies, so the wheel is built from
+# Installs the UNMODIFIED reference (if001/lit-llama-ja) into baseline/_ref (git-ignored; it goes wherever the built
+# tree is copied).  The reference tree is read-only and its setup.py lists git dependencies, so the wheel is built from
 # a copy under /tmp with --no-deps.  generate.py is a top-level script outside the package: it is copied next to it as
 # ref_generate.py so that bench.py --impl reference can time the reference's own generate() loop.
 #   bash baseline/install_ref.sh          (run where /root/reference exists)

@@ -4,7 +4,7 @@
 Both packages are called ``lit_llama`` and the reference imports itself by absolute name, so it is imported first with
 baseline/_ref at the head of ``sys.path`` and its modules are then taken OUT of ``sys.modules`` (they keep working through
 the references they hold to each other); whatever ``lit_llama`` modules were loaded before are put back.  ``lightning``
-(absent from the image; the reference needs two class names from it, lit_llama/utils.py:13) is stubbed - SURVEY.md App. A.
+(absent from the image; the reference needs two class names from it, lit_llama/utils.py:13) is stubbed.
 
 Used only by tests/ and by bench.py's reference legs; nothing in the product imports it.
 """

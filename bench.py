@@ -3,7 +3,7 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
 A "step" is one pass of the hot path over one synthetic input: ``generate()`` of NEW_TOKENS tokens
-after a PROMPT_LEN-token prompt (BASELINE.json configs[1]; the reference prints the same
+after a PROMPT_LEN-token prompt (the reference prints the same
 tokens/sec, generate.py:146-153, prefill included).  Prints ONE JSON line (rank 0).
 
 * ``value``: tokens/s with the prompt already resident in HBM, device-timed (CUDA events).
@@ -108,7 +108,7 @@ class ClockSampler:
 
 # ----------------------------------------------------------------------------- synthetic model
 def build_model(device, name=MODEL, group=GROUP, seed=0, mode="gptq.int4"):
-    """Random-init LLaMA of the named size, RTN-quantised per group on the device (SURVEY 8d config 2)."""
+    """Random-init LLaMA of the named size, RTN-quantised per group on the device."""
     import torch
     from lit_llama import LLaMA
     from lit_llama.quantization import ColBlockQuantizedLinear, rtn_quantize_
@@ -252,7 +252,7 @@ def run_reference(args, rank, world):
 
 # ----------------------------------------------------------------------------- B200 arm
 def algorithmic_bytes(model, n_positions_avg):
-    """bytes one decoded token must move - packed weights + scale/zero tables (+ KV)."""
+    """Bytes one decoded token must move - packed weights + scale/zero tables (+ KV)."""
     from lit_llama.quantization import ColBlockQuantizedLinear
 
     wbytes = 0
@@ -442,7 +442,7 @@ def tp_decode_step_metrics(model, device, world, dist, name):
 
 
 def tp_65b_probe(device, rank, world, dist):
-    """BASELINE.json configs[4]: LLaMA-65B int4 group 128, batch-1 tensor-parallel decode step on `world` GPUs."""
+    """LLaMA-65B int4 group 128, batch-1 tensor-parallel decode step on `world` GPUs."""
     import torch
     from lit_llama.tensor_parallel import tensor_parallelize_
 
@@ -459,10 +459,10 @@ def tp_65b_probe(device, rank, world, dist):
 
 
 def reference_gpu(model, device):
-    """SURVEY section 0's bar: the reference's own GPU path on this B200, identical weights (the model's state dict loaded
+    """The bar: the reference's own GPU path on this B200, identical weights (the model's state dict loaded
     into the unmodified reference's LLaMA from baseline/_ref): decode tokens/s of its LLaMA.forward with KV cache, batch 1.
     Group 128 takes its get_weight + F.linear branch (ref quantization.py:420-421); its Triton kernel only serves per-row
-    scales (measured by profiles/parity_7b.py --per-row; numbers in BASELINE.md)."""
+    scales (measured by profiles/parity_7b.py --per-row)."""
     import torch
 
     try:

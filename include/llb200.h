@@ -7,7 +7,7 @@
  * Return value: LL_OK or a negative LL_ERR_* code; ll_last_error() then holds a message
  * (thread-local).  Nothing throws across this boundary.
  *
- * "ref:" citations are into /root/reference (if001/lit-llama-ja); each entry point names
+ * "ref:" citations are into if001/lit-llama-ja; each entry point names
  * the reference interface it replaces.  The reference has no native code on this path: its
  * FFI-equivalent is the Triton launcher + the PyTorch fallback inside
  * lit_llama/quantization.py, bitsandbytes for llm.int8, and ATen ops in lit_llama/model.py.

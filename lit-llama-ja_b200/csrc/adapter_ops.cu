@@ -1,4 +1,4 @@
-// LLaMA-Adapter inference ops (SURVEY 8f #3; ref: lit_llama/adapter.py:145-165, lit_llama/adapter_v2.py:29-32).
+// LLaMA-Adapter inference ops (ref: lit_llama/adapter.py:145-165, lit_llama/adapter_v2.py:29-32).
 //
 // The reference adds, to every attention output of the adapted layers,
 //     gating_factor[h] * softmax(q . prefix_k^T / sqrt(hs)) . prefix_v

@@ -1,6 +1,6 @@
 // model.py kernels around the quantized Linears: RMSNorm, embedding (+ sum-of-squares partials),
 // RoPE + in-place KV-cache write, split-KV decode attention, SwiGLU product, residual add.
-// ref: /root/reference/lit_llama/model.py:110, 162-175, 192-243, 257-260, 276-283, 312-329.
+// ref: lit_llama/model.py:110, 162-175, 192-243, 257-260, 276-283, 312-329.
 // Every kernel mirrors torch's rounding points (each elementwise op rounds to the activation dtype).
 #include <stdlib.h>
 

@@ -4,7 +4,7 @@
 // get_weight(dtype=bf16), quantization.py:390-409), so the result is the reference's fallback branch
 // F.linear(inp, get_weight(inp.dtype)) (quantization.py:420-421) with fp32 accumulation - the branch the
 // reference takes for every grouped checkpoint and the semantics of its Triton kernel for per-row ones.
-// Used for prefill of layers the many-row kernel (int4_rows.cu) does not take; replaces Triton's mma.sync kernel
+// Used for prefill of layers the many-row kernel (int4_rows.cu) does not take and for steps of more than 8192 rows; replaces Triton's mma.sync kernel
 // (quantization.py:185-280).
 //
 // Structure (one 128 x BN output tile per CTA, 192 threads):

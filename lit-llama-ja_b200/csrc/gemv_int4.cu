@@ -29,7 +29,7 @@
 //    plain store, residual add, RoPE + KV-cache write (c_attn), SwiGLU (c_fc1/c_fc2 as two matrices
 //    of one launch), or peer stores for the tensor-parallel push.  The decode chain's configuration
 //    gets one instantiation per (epilogue, norm, batch 1): less cold code per launch.
-//  * Measurements, ablations and rejected variants: profiles/r01_gemv_experiments.md, DESIGN.md section 3.
+//  * Measurements, ablations and rejected variants: profiles/r01_gemv_experiments.md.
 //    Tuning switches (-D): LLB_XPRED, LLB_SHIFT_FMA, LLB_XSTAGE_TMA, LLB_TRACE, LLB_ABL_* (timing
 //    ablations, wrong sums) - build with `build.py --variant`, select with LLB200_LIB.
 #include <stdlib.h>
@@ -160,7 +160,7 @@ __device__ __forceinline__ void mbar_wait_u32(uint32_t bar, uint32_t parity) {
 // configuration gets one specialised kernel per layer kind: less code to fetch cold at every launch - the kernel
 // runs its prologue and epilogue once - and no epilogue dispatch); -1: taken from the arguments.
 // MM > 0: the batch (rows of x) is the compile-time constant MM (batch-1 decode: every per-row loop folds away).
-// (A neighbour stream-K split of the boundary tiles was built and measured in round 2: q 311 -> 361, p 131 -> 199, f 423 -> 519,
+// (A neighbour stream-K split of the boundary tiles was built and measured: q 311 -> 361, p 131 -> 199, f 423 -> 519,
 // d 277 -> 325 us per 32 layers - slower than the 7-14 % tile imbalance it removes; taken out, profiles/r02_gemv_experiments.md.)
 template <int W, int KSP, int BPW, int EPI = -1, int NORM = -1, int MM = 0>
 __global__ void __launch_bounds__((W + 1) * 32, (W >= 12 ? 1 : 2)) gemv_int4_kernel(const __grid_constant__ Params p) {

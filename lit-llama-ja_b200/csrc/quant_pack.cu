@@ -1,5 +1,5 @@
 // GPTQ column-block storage kernels: pack, unpack, reference-semantics linear.
-// ref: /root/reference/lit_llama/quantization.py:339-421 (ColBlockQuantizedLinear).
+// ref: lit_llama/quantization.py:339-421 (ColBlockQuantizedLinear).
 #include <stdarg.h>
 
 #include <mutex>

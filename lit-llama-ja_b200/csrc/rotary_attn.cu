@@ -997,7 +997,11 @@ int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, int gate
   if (form == 0 && !(slopes && maps > 1) && tm_supported(dtype, T, dim, vdim, q_stride, gate ? gate_stride : 0, splits) &&
       y_stride % 2 == 0) {
     const int d = dim > vdim ? dim : vdim;
-    if (maps == 1) {           // one map: key and value rows padded alike
+    // One map: the tcgen05 form wherever its maps take the rows (16-byte boundaries), from 16 tokens on; the mma.sync form serves shifted
+    // rows.  Both sides measured, us, mma.sync / tcgen05, 16 heads over 4 of 128, after 0 / 2000 / 8000 positions: 16 tokens 18 / 10,
+    // 162 / 41, 602 / 135; 256 tokens 33 / 16, 184 / 51, 621 / 152; 1024 tokens 101 / 29, 273 / 66, 778 / 167.  (8 and 32 heads, heads
+    // of 64, caps, windows and batches alike: 0.74 of the time at most.)
+    if (maps == 1) {           // (mma.sync: key and value rows padded alike)
       AttnTcArgs a{};
       a.q = {q, dim, dim, q_stride, (long long)T * q_stride};
       a.k = {kc, dim, dim, (long long)G * dim, (long long)ring * G * dim};

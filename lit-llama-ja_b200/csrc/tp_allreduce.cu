@@ -1,7 +1,7 @@
 // One-shot all-reduce over NVLink peer memory for the tensor-parallel decode step, fused with the residual add:
 //   x[i] = bf16( x[i] + bf16( sum_r part_r[i] ) )        (r in rank order on every rank: identical bits everywhere)
 // ref: none - the reference is single-device (generate.py:122); this is the one exchange step of the sharded path
-// (SURVEY 8e): [B, n_embd] bf16 after each row-parallel GEMV (16 KB at batch 1 for 65B), latency-bound.  NCCL's
+// [B, n_embd] bf16 after each row-parallel GEMV (16 KB at batch 1 for 65B), latency-bound.  NCCL's
 // all-reduce costs a launch + protocol round per call and does not sit well inside a captured graph next to PDL
 // kernels; here every rank pushes nothing - it only raises a flag, then PULLS the peers' partial sums straight out of
 // their HBM through the NVSwitch (P2P loads on symmetric-memory mappings), so one small kernel is the whole
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(1024) tp_allreduce_add_kernel(const __grid_con
                                                                 int32_t* __restrict__ epoch_counter, int rank, int world, int n,
                                                                 int use_pdl) {
   __shared__ int s_epoch;
-  // use_pdl (round 2): a link of the programmatic-launch chain.  Round 1 launched this kernel plainly because an early
+  // use_pdl: a link of the programmatic-launch chain.  It was once launched plainly because an early
   // launch behind it cost time - the cause was CTA placement (a 148-CTA GEMV grid released while a fat CTA holds an SM
   // doubles up elsewhere, profiles/r02_gemv_experiments.md section 6), cured by the EVEN / ODD GEMV footprints.  With them
   // the next GEMV's CTAs can start (barriers, norm weights, ring fill from HBM) while the flags and partial sums travel,

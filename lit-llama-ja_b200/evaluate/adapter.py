@@ -1,4 +1,4 @@
-"""Perplexity of a LLaMA-Adapter fine-tune (ref: /root/reference/evaluate/adapter.py:50-160): as evaluate/full.py, on
+"""Perplexity of a LLaMA-Adapter fine-tune (ref: evaluate/adapter.py:50-160): as evaluate/full.py, on
 ``lit_llama.adapter.LLaMA`` with the pretrained and the adapter checkpoint loaded non-strictly, the text wrapped in the Alpaca
 instruction template first (the reference's ``instruction_tuning = True``, evaluate/adapter.py:24).  Text comes from local
 files (``--data_paths a.txt,b.txt``): there is no network for ``datasets``."""

@@ -1,4 +1,4 @@
-"""Perplexity of a LLaMA-Adapter v2 fine-tune (ref: /root/reference/evaluate/adapter_v2.py): as evaluate/adapter.py, with the
+"""Perplexity of a LLaMA-Adapter v2 fine-tune (ref: evaluate/adapter_v2.py): as evaluate/adapter.py, with the
 per-Linear ``adapter_bias`` / ``adapter_scale`` parameters added before the checkpoints are loaded."""
 import importlib.util
 from pathlib import Path

@@ -1,4 +1,4 @@
-"""Perplexity of a (quantized) checkpoint, GPTQ-style (ref: /root/reference/evaluate/full.py:45-141): the
+"""Perplexity of a (quantized) checkpoint, GPTQ-style (ref: evaluate/full.py:45-141): the
 text is tokenised once, cut into windows of 2048 tokens, each window goes through ``model(inp)`` WITHOUT a KV cache - the
 prefill path (large-M quantized Linear: fused de-quantise + tcgen05 GEMM up to 256 rows, unpack + tcgen05 GEMM beyond) -
 and the summed next-token negative log-likelihood gives exp(nll / tokens).

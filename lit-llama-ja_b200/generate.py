@@ -1,4 +1,4 @@
-"""Text generation with the B200-native quantized LLaMA (ref: /root/reference/generate.py).
+"""Text generation with the B200-native quantized LLaMA (ref: generate.py).
 
 Same ``generate(model, idx, max_new_tokens, *, max_seq_length, temperature, top_k, eos_id)``
 signature and sampling semantics, same ``main`` flags (``--quantize gptq.int4|llm.int8`` ...).

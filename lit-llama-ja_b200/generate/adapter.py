@@ -1,4 +1,4 @@
-"""Sampling from a LLaMA-Adapter fine-tune (ref: /root/reference/generate/adapter.py:20-106): the same
+"""Sampling from a LLaMA-Adapter fine-tune (ref: generate/adapter.py:20-106): the same
 flags; the pretrained checkpoint and the adapter checkpoint are loaded into ``lit_llama.adapter.LLaMA`` built under
 ``quantization(mode)``, the instruction goes through the Alpaca template, and the text after "### Response:" is printed."""
 import importlib.util

@@ -1,4 +1,4 @@
-"""Sampling from a LLaMA-Adapter v2 fine-tune (ref: /root/reference/generate/adapter_v2.py:22-108): as
+"""Sampling from a LLaMA-Adapter v2 fine-tune (ref: generate/adapter_v2.py:22-108): as
 generate/adapter.py, with the per-Linear ``adapter_bias`` / ``adapter_scale`` parameters added to the model before the two
 checkpoints are loaded (ref :71-73)."""
 import importlib.util

@@ -1,4 +1,4 @@
-"""Sampling from a fully fine-tuned checkpoint (ref: /root/reference/generate/full.py:21-91): the same flags,
+"""Sampling from a fully fine-tuned checkpoint (ref: generate/full.py:21-91): the same flags,
 the Alpaca instruction template around the prompt (ref scripts/prepare_alpaca.py:111-125), the model built under
 ``quantization(mode)`` and decoded by this repository's ``generate()`` (device-side sampling loop, fused decode step)."""
 import sys

@@ -1,4 +1,4 @@
-"""LLaMA-Adapter for inference on B200 (SURVEY 8f #3; ref: lit_llama/adapter.py:47-313): the reference's module tree,
+"""LLaMA-Adapter for inference on B200 (ref: lit_llama/adapter.py:47-313): the reference's module tree,
 state-dict keys and call signatures over this package's kernels.
 
 What the adapter adds to an attention layer (``block_idx >= adapter_start_layer``): the queries also attend to a learned

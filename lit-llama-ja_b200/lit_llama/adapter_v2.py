@@ -1,4 +1,4 @@
-"""LLaMA-Adapter v2 for inference on B200 (SURVEY 8f #3; ref: lit_llama/adapter_v2.py:1-45): every Linear gets a learned
+"""LLaMA-Adapter v2 for inference on B200 (ref: lit_llama/adapter_v2.py:1-45): every Linear gets a learned
 per-output-column ``adapter_bias`` and ``adapter_scale`` applied after its matrix product,
 ``y = adapter_scale * (linear(x) + adapter_bias)``.
 

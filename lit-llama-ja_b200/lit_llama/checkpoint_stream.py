@@ -1,6 +1,6 @@
-"""Lazy checkpoint streaming with the one-time weight repack inside the load (SURVEY 8f #2).
+"""Lazy checkpoint streaming with the one-time weight repack inside the load.
 
-ref: /root/reference/lit_llama/utils.py:198-376 (``NotYetLoadedTensor``, ``LazyLoadingUnpickler``, ``lazy_load``): the
+ref: lit_llama/utils.py:198-376 (``NotYetLoadedTensor``, ``LazyLoadingUnpickler``, ``lazy_load``): the
 reference unpickles a ``torch.save`` archive into placeholders and lets ``torch._C.PyTorchFileReader`` materialise one
 tensor when torch first touches it, so that ``model.load_state_dict`` never holds the whole checkpoint on the host.
 

@@ -4,7 +4,7 @@
 What differs from the reference, by design:
 * every op between the Linears is one kernel call through the C-ABI (RMSNorm, RoPE + in-place
   KV-cache write, split-KV decode attention, SwiGLU product, residual add) instead of 5-16 ATen
-  launches each (SURVEY 2b);
+  launches each;
 * the KV cache is written IN PLACE; the reference's roll-when-full (model.py:221-225) becomes a
   ring slot ``pos % max_seq_length`` - attention is order-independent over the slots;
 * single-token steps of an int4/bf16 model run through the fused, CUDA-graph-captured decode

@@ -155,8 +155,8 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     # rows from which the weights are de-quantised in the main loop of the many-row kernel, from the checkpoint bytes.  Both sides measured
     # (11008 x 4096, group 128): 130 rows 27 us against 61 in two passes of the small-row kernel and 87 with a bf16 copy of W; 512 rows
     # 49 against 112; 2048 rows 137 against 220.
-    # Past 8192 rows a long run of products is held by the power limit, and a tile of W is de-quantised again for every 256 rows: the
-    # bf16 copy, written once, then costs less.  us, this kernel / copy and product, 150 ms of each in turn: 13824 x 5120 at 8192 rows
+    # Past 8192 rows the bf16 copy, written once, costs less than a tile of W de-quantised again for every 256 rows.  us, this kernel / copy
+    # and product, 150 ms of each in turn: 13824 x 5120 at 8192 rows
     # 1067 / 1342, at 16384 2350 / 2618; 5120 x 13824: 1033 / 1160 and 2365 / 2245; 4096 x 11008: 682 / 713 and 1522 / 1380; 11008 x 4096:
     # 741 / 856 and 1746 / 1678.
     ROWS_MIN_M, ROWS_MAX_M = 129, 8192
@@ -250,7 +250,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
 
 def dequant_gemm(lin: ColBlockQuantizedLinear, x: torch.Tensor) -> torch.Tensor:
-    """Large-M path of layers the many-row kernel does not take: bit-exact de-quantisation of W into a bf16 scratch (the
+    """Large-M path of layers the many-row kernel does not take, and of steps of more than ROWS_MAX_M rows: bit-exact de-quantisation of W into a bf16 scratch (the
     reference's ``get_weight``) followed by the tcgen05/TMEM tensor-core GEMM - the reference's fallback
     branch (quantization.py:420-421) on the 5th-generation tensor cores.  fp32 activations (tests scale
     only) use the library GEMM."""
@@ -402,7 +402,7 @@ def quantize_weight(x, scale, zero, maxq):
 def rtn_quantize_(lin: ColBlockQuantizedLinear, weight: torch.Tensor) -> ColBlockQuantizedLinear:
     """Round-to-nearest quantisation of ``weight`` into ``lin`` (per group of ``lin.tile_cols``):
     parameters from ``find_params_weight``, on-grid weights from ``quantize_weight``, bytes from
-    ``pack_weight`` - the grouped fixture of SURVEY 8c/8d, all on the module's device."""
+    ``pack_weight`` - all on the module's device."""
     maxq = 2 ** lin.bits - 1
     w = weight.to(device=lin.quant_weight.device, dtype=torch.float32)
     n, k = w.shape

@@ -1,6 +1,6 @@
-"""Tensor-parallel quantized LLaMA over one NVSwitch node (BASELINE.json config 5: LLaMA-65B int4 at 2/4/8 GPUs).
+"""Tensor-parallel quantized LLaMA over one NVSwitch node (LLaMA-65B int4 at 2/4/8 GPUs).
 
-The reference is single-device (generate.py:122 ``devices=1``; SURVEY 8e): sharding is new here and is validated
+The reference is single-device (generate.py:122 ``devices=1``): sharding is new here and is validated
 against the unsharded result on identical weights.  Megatron-style, one exchange per row-parallel layer:
 
 * column-parallel (split the output rows N of ``quant_weight`` / ``scales`` / ``zeros``): ``attn.c_attn`` (by HEAD
@@ -13,7 +13,7 @@ against the unsharded result on identical weights.  Megatron-style, one exchange
   is not worth a second collective).
 
 The pure index helpers below are exercised on CPU with world-size-2 ``gloo`` (tests/test_tp_gloo.py) against the
-oracle; the CUDA path is exercised with ``gpurun --gpus 2`` (tests/test_gpu_tp.py, launched by torchrun).
+oracle; the CUDA path is exercised on 2 GPUs by tests/test_gpu_tp.py, launched by torchrun.
 """
 from __future__ import annotations
 

@@ -1,4 +1,4 @@
-"""GPTQ checkpoint writer for the B200-native LLaMA (ref: /root/reference/quantize/gptq.py).
+"""GPTQ checkpoint writer for the B200-native LLaMA (ref: quantize/gptq.py).
 
 Same entry points: ``llama_blockwise_quantization(model, sample_inputs, working_device, *, bits, groupsize)`` and
 ``main(checkpoint_path, output_path, tokenizer_path, n_samples, dtype, quantize)``; the written state dict has the

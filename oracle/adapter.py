@@ -1,7 +1,7 @@
 """Numpy restatement of the reference's LLaMA-Adapter (v1 and v2) forward.
 
-TEST INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).  Citations are into ``/root/reference/lit_llama/adapter.py`` and
-``/root/reference/lit_llama/adapter_v2.py``.  Parity: **pinned** against outputs of the unmodified reference run in the
+TEST INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).  Citations are into ``lit_llama/adapter.py`` and
+``lit_llama/adapter_v2.py``.  Parity: **pinned** against outputs of the unmodified reference run in the
 build container (``tests/golden/make_golden_adapter.py`` -> ``tests/golden/adapter_tiny.npz``).
 """
 from __future__ import annotations

@@ -1,7 +1,7 @@
 """Numpy restatement of the reference LLaMA decode path around the quantized Linears.
 
 TEST INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).  Citations are into
-``/root/reference/lit_llama/model.py`` and ``/root/reference/generate.py``.
+``lit_llama/model.py`` and ``generate.py``.
 Values live in float32 arrays; ``dtype="bf16"`` rounds after each op where torch would.
 """
 from __future__ import annotations

@@ -1,7 +1,7 @@
 """Numpy restatement of the reference's quantized-Linear arithmetic.
 
 TEST INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).  Citations are into
-``/root/reference/lit_llama/quantization.py`` unless another file is named.
+``lit_llama/quantization.py`` unless another file is named.
 
 dtype handling: the reference computes in whatever dtype the tensors carry
 (fp32 under ``32-true``, bf16 under ``bf16-true``).  The oracle keeps every value
@@ -75,7 +75,7 @@ def quantize_weight(x, scale, zero, maxq: int) -> np.ndarray:
 
 def rtn_quantize(W: np.ndarray, bits: int, groupsize: int = -1):
     """Round-to-nearest on-grid weights + params per group: the grouped fixture of
-    SURVEY.md section 8c (find_params_weight per column slice, quantize_weight).
+    (find_params_weight per column slice, quantize_weight).
     Returns (W_on_grid[N,K], scales[N,G], zeros[N,G])."""
     W = np.asarray(W, dtype=F32)
     N, K = W.shape

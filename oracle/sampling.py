@@ -1,4 +1,4 @@
-"""Numpy restatement of the sampling tail of the reference's ``generate`` (/root/reference/generate.py:62-75).
+"""Numpy restatement of the sampling tail of the reference's ``generate`` (generate.py:62-75).
 
 TEST INFRASTRUCTURE ONLY (see ``oracle/__init__.py``).  The reference computes, on the last position's logits,
 

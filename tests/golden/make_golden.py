@@ -5,7 +5,7 @@ absent there); the ``*.npz`` files it writes are committed beside it.
     python tests/golden/make_golden.py
 
 The reference imports once ``lightning`` is stubbed (it is needed only for two class
-names at lit_llama/utils.py:13) - SURVEY.md appendix A.
+names at lit_llama/utils.py:13).
 """
 import importlib.util
 import io
@@ -187,7 +187,7 @@ def tiny_weights(cfg):
 
 
 def golden_model(qz, utils, model, gen, gptq):
-    """Tiny LLaMA: fp32 forward / KV-cache decode / generate,
+    """Tiny LLaMA (the smallest configuration): fp32 forward / KV-cache decode / generate,
     the reference GPTQ writer's int4 checkpoint and its forward + generate, and a
     group-32 RTN int4 model in fp32 and bf16 (rows M, A, K, S, Q, L)."""
     out = {}

@@ -1,4 +1,4 @@
-"""Golden vectors for the LLaMA-Adapter callers (SURVEY 8f #3), produced by running the UNMODIFIED reference
+"""Golden vectors for the LLaMA-Adapter callers, produced by running the UNMODIFIED reference
 (/root/reference/lit_llama/adapter.py, adapter_v2.py) in the build container on the weights of
 ``tests/util_tiny.adapter_tiny_weights``.  Not runnable on the GPU box (the reference is absent there); the file it
 writes, ``adapter_tiny.npz``, is committed beside it.

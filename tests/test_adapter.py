@@ -1,4 +1,4 @@
-"""LLaMA-Adapter callers of the quantized-inference boundary (SURVEY 8f #3): lit_llama/adapter.py, adapter_v2.py and
+"""LLaMA-Adapter callers of the quantized-inference boundary: lit_llama/adapter.py, adapter_v2.py and
 generate/adapter*.py.  The oracle (oracle/adapter.py) is pinned against outputs of the unmodified reference
 (tests/golden/adapter_tiny.npz, written by tests/golden/make_golden_adapter.py); the CUDA path is compared with the
 goldens (fp32) and with the oracle (int4 weights, bf16 activations)."""

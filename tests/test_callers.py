@@ -1,4 +1,4 @@
-"""The other callers of the quantized-inference boundary (SURVEY 8f #3): generate/full.py and evaluate/full.py."""
+"""The other callers of the quantized-inference boundary: generate/full.py and evaluate/full.py."""
 import importlib.util
 import math
 from pathlib import Path

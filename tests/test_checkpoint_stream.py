@@ -1,4 +1,4 @@
-"""Lazy checkpoint streaming (SURVEY 8f #2; ref lit_llama/utils.py:198-376).  CPU: the archive index and the placeholders
+"""Lazy checkpoint streaming (ref lit_llama/utils.py:198-376).  CPU: the archive index and the placeholders
 against ``torch.load`` on the same file.  GPU: the disk -> pinned -> HBM pipeline with the repack inside the load."""
 import numpy as np
 import pytest

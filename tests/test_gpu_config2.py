@@ -1,4 +1,4 @@
-"""Parity at the HEADLINE configuration's layer shapes (SURVEY 8d "Correctness gates"):
+"""Parity at the HEADLINE configuration's layer shapes (7B int4 group 128):
 LLaMA-7B dimensions (n_embd 4096, 32 heads of 128, n_hidden 11008, vocab 32000), GPTQ int4 group 128 (and per-row), bf16,
 a 512-token prompt then teacher-forced single-token steps - the shapes that select the SHIPPED decode kernels
 (`gemv_w4a8_kernel<{ROPE_KV,RESIDUAL,SWIGLU,STORE},{norm}>` at batch 1, `gemv_int4_kernel<8,4,2,...>` at batch 2,
@@ -13,7 +13,7 @@ Three references on identical weights and tokens:
 
 Layer count is 2 here; the full depth (32 layers, 512 + 256 steps on the reference's greedy stream, and the reference's own
 fp32 result on the same tokens) is run by profiles/parity_7b.py -> profiles/r02_parity_config2_*.json.  The stated
-tolerance is in TOL below and in DESIGN.md section 1.
+tolerance is in TOL below.
 """
 import ctypes as C
 import os
@@ -30,7 +30,7 @@ DEV = "cuda"
 CFG2 = dict(block_size=2048, vocab_size=32000, n_layer=2, n_head=32, n_embd=4096)
 PROMPT = 512
 
-# Stated bf16 tolerance (DESIGN.md section 1).  The reference's one stated tolerance is atol 5e-3 / rtol 1e-3 on logits of
+# Stated bf16 tolerance.  The reference's one stated tolerance is atol 5e-3 / rtol 1e-3 on logits of
 # an fp32 16-layer E=32 model (ref tests/test_model.py:131).  Under bf16-true every op rounds to 2^-9 relative and the two
 # numerics the reference itself has for a quantized Linear (bf16-rounded de-quantised weights in the fallback branch, exact
 # (q - zero) * scale in the Triton branch) already differ by that much per layer, so the bar is relative to the logit
@@ -48,7 +48,7 @@ def _lin_names(n_layer):
 
 
 def build_cfg2_model(group, n_layer=2, seed=0, mode="gptq.int4"):
-    """Random-init model of 7B layer shapes, RTN-quantised on-grid per group (SURVEY 8d config 2), norm scales 1 +- 0.1."""
+    """Random-init model of 7B layer shapes, RTN-quantised on-grid per group, norm scales 1 +- 0.1."""
     from lit_llama import LLaMA, LLaMAConfig
     from lit_llama.quantization import ColBlockQuantizedLinear, rtn_quantize_
     from lit_llama.utils import EmptyInitOnDevice, quantization
@@ -599,7 +599,7 @@ def test_q8_gemv_epilogues_at_7b_shapes(monkeypatch):
 @pytest.mark.parametrize("M", [1, 2])
 @pytest.mark.parametrize("N_,K", [(4096, 4096), (1040, 11008)])
 def test_gemv_writes_nothing_outside_its_output(M, N_, K):
-    """compute-sanitizer is closed on this pool (profiles/r02_sanitizer_closed.txt): stray stores are looked for directly -
+    """Stray stores are looked for directly -
     the output rows sit between canary rows that must come back untouched (both kernels, a ragged last CTA share)."""
     from lit_llama import _native as NV
     from oracle import quant as OQ

@@ -1,4 +1,4 @@
-"""GPTQ solver on the device (row Z2 / SURVEY 8f #1): ll_gptq_block + GPTQQuantizer against oracle/quant.py
+"""GPTQ solver on the device (row Z2): ll_gptq_block + GPTQQuantizer against oracle/quant.py
 (itself pinned to the reference's GPTQQuantizer outputs in tests/golden/gptq_solver.npz)."""
 import sys
 from pathlib import Path

@@ -1,5 +1,5 @@
 """GPU parity of the llm.int8 path (Linear8bitLt) against the oracle's restatement of LLM.int8().
-bitsandbytes is un-vendored/unpinned in the reference and absent here: parity is "unpinned" (DESIGN.md section 1)."""
+bitsandbytes is un-vendored/unpinned in the reference and absent here: parity is "unpinned"."""
 import numpy as np
 import pytest
 import torch

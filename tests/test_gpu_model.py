@@ -1,4 +1,4 @@
-"""GPU parity at model level: tiny LLaMA vs the reference's goldens and the
+"""GPU parity at model level: tiny LLaMA (the smallest configuration) vs the reference's goldens and the
 oracle; fused decode engine vs the per-module path; generate loop."""
 import sys
 

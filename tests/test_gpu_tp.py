@@ -1,6 +1,6 @@
 """Tensor-parallel decode on 2 GPUs (NCCL): sharded tiny int4/bf16 LLaMA == the unsharded one within the bf16
 tolerance, through both the per-module path (prefill) and the fused CUDA-graph engine (decode).
-Skipped on a 1-GPU box; run with `gpurun --gpus 2`."""
+Skipped on a 1-GPU box."""
 import os
 import socket
 import sys
@@ -56,7 +56,7 @@ def _worker(rank, world, port, out):
         dist.destroy_process_group()
 
 
-@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs (gpurun --gpus 2)")
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs")
 def test_tp2_decode_matches_single_gpu():
     import torch.multiprocessing as mp
 
@@ -111,7 +111,7 @@ def _worker_7b(rank, world, port, out):
         dist.destroy_process_group()
 
 
-@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs (gpurun --gpus 2)")
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs 2 GPUs")
 def test_tp2_decode_at_7b_shapes_matches_single_gpu():
     import torch.multiprocessing as mp
 

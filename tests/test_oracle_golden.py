@@ -54,7 +54,7 @@ def test_pack_unpack_forward_bit_exact(golden, dt):
 
 
 def test_truncation_quirk_is_reproduced(golden):
-    """pack_weight truncates x/scale+zero (SURVEY row P): some codes land one below the
+    """pack_weight truncates x/scale+zero: some codes land one below the
     RTN code; the oracle must reproduce the reference's bytes, not 'fix' them."""
     g = golden["quant"]
     n_off = 0

@@ -46,7 +46,7 @@ def test_pack_unpack_round_trip_and_code_range(case):
     assert codes.shape == (N, K) and codes.min() >= 0 and codes.max() <= 2**bits - 1
     w = OQ.get_weight(packed, s, z, bits, tc, "fp32")
     # pack(get_weight(p)): pack_weight TRUNCATES (quantization.py:383), so a code whose fp32 `(c - z) * s / s + z` lands
-    # at c - eps comes back as c - 1 (SURVEY 8a row P); never upward, never by more than one
+    # at c - eps comes back as c - 1; never upward, never by more than one
     again = OQ.unpack_codes(OQ.pack_weight(w, s, z, bits, tc, "fp32"), bits).astype(np.int32)
     d = codes.astype(np.int32) - again
     assert d.min() >= 0 and d.max() <= 1

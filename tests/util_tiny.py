@@ -1,4 +1,4 @@
-"""Shared builders for the tiny LLaMA used by CPU and GPU tests.
+"""Shared builders for the tiny LLaMA (the smallest configuration) used by CPU and GPU tests.
 ``tiny_weights`` replays tests/golden/make_golden.py's generator (numpy legacy RNG)."""
 import numpy as np
 
@@ -58,7 +58,7 @@ def oracle_q_model(g, prefix, tile_cols, dtype):
     return OM.LLaMA(OM.Config(**TINY), lin, W["transformer.wte.weight"], norms, dtype)
 
 
-# --------------------------------------------------------------------------- LLaMA-Adapter (SURVEY 8f #3)
+# --------------------------------------------------------------------------- LLaMA-Adapter
 ADAPTER_TINY = dict(block_size=64, vocab_size=128, n_layer=3, n_head=4, n_embd=128, adapter_prompt_length=10,
                     adapter_start_layer=1)
 
