@@ -319,8 +319,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         mbar_expect_tx(&v_full[vs], (uint32_t)(NBV * AT_KBOX));
         for (int c = 0; c < NBV; ++c) tma_box4(sv + (vs * NBV + c) * AT_KBOX, &map_v, c * 64, g, blk.slot, b, &v_full[vs]);
       }
-      if (!ok)                       // copies already issued land before the block leaves
-        for (int w = 0; w < 2048; ++w) __nanosleep(512);
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == AT_WARPS + 1 || warp == AT_WARPS + 2) {
     // ===================== MMA issuers, one thread per tile =====================
@@ -384,6 +383,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           mbar_arrive(&v_empty[vs]);
         }
       }
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == AT_WARPS + 3) {
     // ===================== value rows of no key =====================

@@ -157,8 +157,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
           }
         }
       }
-      if (!ok)                         // copies already issued land before the CTA leaves
-        for (int w = 0; w < 2048; ++w) __nanosleep(512);
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -183,6 +182,7 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
         }
         if (ok) umma_commit(d_full);
       }
+      if (!ok) let_issued_work_end();
     }
   } else if (warp >= 4) {
     const int quarter = warp & 3, grp = (warp >> 2) - 1, col = quarter * 32 + lane;

@@ -218,8 +218,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
         i8_box(sa + s * I8_BOX, &map_a, kb * 128, m0, &full[s]);
         i8_box(sb + s * I8_BOX, &map_b, kb * 128, n0, &full[s]);
       }
-      if (!ok)                       // copies already issued land before the CTA leaves
-        for (int w = 0; w < 2048; ++w) __nanosleep(512);
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -237,6 +236,7 @@ __global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_const
         umma_commit(&empty[s]);
       }
       umma_commit(done);             // also after a failure: the epilogue's wait ends
+      if (!ok) let_issued_work_end();
     }
   } else {
     const int quarter = warp & 3, m = m0 + quarter * 32 + lane;
@@ -662,8 +662,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
         i8_box(sx + s * XB, &map_x, kb * 128, 0, &full[s]);
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
-      if (!ok)                       // copies already issued land before the CTA leaves
-        for (int w = 0; w < 2048; ++w) __nanosleep(512);
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == 1) {
     if (elect_one()) {
@@ -682,6 +681,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
       umma_commit(done);             // also after a failure: the epilogue's wait ends
+      if (!ok) let_issued_work_end();
     }
   } else {
     const int quarter = warp & 3, n = n0 + quarter * 32 + lane;

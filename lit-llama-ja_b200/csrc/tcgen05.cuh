@@ -114,6 +114,11 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(r)::"memory");
   return r != 0;
 }
+// For a role that gives up: copies and products it has issued end (a millisecond is a hundred times as long as the ring's worth of either)
+// before the block lets go of its shared and tensor memory.
+__device__ __forceinline__ void let_issued_work_end() {
+  for (int w = 0; w < 2048; ++w) __nanosleep(512);
+}
 __device__ __forceinline__ void mbar_wait_parity(uint64_t* bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n"

@@ -130,3 +130,13 @@ def test_a_wait_that_ran_out_is_raised_once():
     with pytest.raises(RuntimeError, match="llm.int8, code 307"):
         N.check_waits()
     N.check_waits()
+
+
+def test_roles_that_give_up_let_their_work_end():
+    """In every tcgen05 kernel with bounded waits, the roles that issue copies or products wait for them (bounded) after a wait has run out,
+    before tensor memory is freed.  (A wait cannot be made to run out on a GPU in a test: the statement is read off the source.)"""
+    csrc = Path(__file__).resolve().parent.parent / "lit-llama-ja_b200" / "csrc"
+    for name, roles in (("attn_tc.cuh", 2), ("int4_rows.cu", 2), ("int8_linear.cu", 4)):
+        text = (csrc / name).read_text()
+        assert text.count("if (!ok) let_issued_work_end();") == roles, name
+        assert text.count("if (elect_one()) {") == roles, name         # one such role each
