@@ -45,9 +45,9 @@ int wait_check() {
   if (code != 0) *p = 0;
   if (g_wait_host.load(std::memory_order_relaxed) != 0) code = g_wait_host.exchange(0, std::memory_order_relaxed);
   if (code == 0) return LL_OK;
-  static const char* const where[] = {"", "prompt attention", "int4 rows", "llm.int8", "grouped experts", "delta rule in chunks"};
+  static const char* const where[] = {"", "prompt attention", "int4 rows", "llm.int8", "grouped experts", "delta rule in chunks", "dense products"};
   set_error("a bounded wait ran out in an earlier launch (%s, code %d): what it and the launches after it wrote is not valid",
-            code >= 100 && code < 600 ? where[code / 100] : "?", code);
+            code >= 100 && code < 700 ? where[code / 100] : "?", code);
   return LL_ERR_WAIT;
 }
 int sm_count() {
@@ -157,6 +157,66 @@ __global__ void __launch_bounds__(256) get_weight_int4_bf16_kernel(const uint8_t
       o[i] = (uint32_t)f32_to_bf16_bits(lo) | ((uint32_t)f32_to_bf16_bits(hi) << 16);
     }
     *reinterpret_cast<uint4*>(out + (size_t)n * K + kb) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// The same for bf16 scales: 64 columns x 512 k a block, every thread's 16-byte loads in flight together; ldmatrix transposes the bytes, so that
+// a thread holds four of a column's (8 k: one 16-byte store), and a whole zero (every RTN / GPTQ checkpoint) is taken off in one exact
+// subtraction of packed pairs: bound by the bytes written.  13824 x 5120, group 128: 64 us as above (2.8 TB/s of
+// bytes read and written), here 44 (4.1).
+constexpr int GW_DEEP = 4;
+__global__ void __launch_bounds__(256) get_weight_int4_pairs_kernel(const uint8_t* __restrict__ qw, const __nv_bfloat16* __restrict__ scales,
+                                                                    const __nv_bfloat16* __restrict__ zeros, __nv_bfloat16* __restrict__ out, int N, int K,
+                                                                    int tile, int G) {
+  __shared__ __align__(16) uint8_t raw[GW_DEEP][64][80];      // 80: the rows ldmatrix reads lie in different banks
+  const int n0 = blockIdx.x * 64, kb0 = blockIdx.y * GW_DEEP, deep = min(GW_DEEP, K / 128 - kb0);
+  {
+    const int r = threadIdx.x >> 2, seg = threadIdx.x & 3;
+    uint4 v[GW_DEEP];
+#pragma unroll
+    for (int d = 0; d < GW_DEEP; ++d)
+      if (d < deep) v[d] = __ldcs(reinterpret_cast<const uint4*>(qw + (size_t)((kb0 + d) * 64 + r) * N + n0 + seg * 16));
+#pragma unroll
+    for (int d = 0; d < GW_DEEP; ++d)
+      if (d < deep) *reinterpret_cast<uint4*>(&raw[d][r][seg * 16]) = v[d];
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c16 = (warp & 3) * 16, half = warp >> 2;
+#pragma unroll
+  for (int d = 0; d < GW_DEEP; ++d) {
+    if (d >= deep) break;
+    uint32_t w[4];
+    asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                 : "r"(smem_u32(&raw[d][half * 32 + lane][c16])));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {            // i & 1: column lane / 4 or + 8; i >> 1: the half's first or last 32 k
+      const int n = n0 + c16 + (lane >> 2) + (i & 1) * 8, k = (kb0 + d) * 128 + half * 64 + (i >> 1) * 32 + (lane & 3) * 8;
+      const size_t at = (size_t)n * G + k / tile;
+      const __nv_bfloat16 sc = scales[at];
+      const float z = __bfloat162float(zeros[at]);
+      uint32_t o[4];
+      if (z == floorf(z) && z >= 0.f && z <= 64.f) {
+        const uint32_t s2 = (uint32_t)__bfloat16_as_ushort(sc) * 0x00010001u, z2 = (0x4300u + (uint32_t)z) * 0x00010001u;
+        const uint32_t lo = w[i] & 0x0f0f0f0fu, hi = (w[i] >> 4) & 0x0f0f0f0fu;
+        const uint32_t p = __byte_perm(lo, hi, 0x5140), q = __byte_perm(lo, hi, 0x7362);
+        const uint32_t v[4] = {__byte_perm(p, 0x43u, 0x4140), __byte_perm(p, 0x43u, 0x4342), __byte_perm(q, 0x43u, 0x4140), __byte_perm(q, 0x43u, 0x4342)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {        // bf16 (128 + q) - (128 + zero), exact; times the scale, rounded
+          uint32_t t;
+          asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(v[e]), "r"(z2));
+          asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(o[e]) : "r"(t), "r"(s2));
+        }
+      } else {
+        const float s = __bfloat162float(sc);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t b = (w[i] >> (8 * e)) & 0xffu;
+          o[e] = pack_bf16(__fmul_rn(bf16r(__fsub_rn((float)(b & 15u), z)), s), __fmul_rn(bf16r(__fsub_rn((float)(b >> 4), z)), s));
+        }
+      }
+      *reinterpret_cast<uint4*>(out + (size_t)n * K + k) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
   }
 }
 
@@ -272,7 +332,8 @@ int ll_get_weight(const uint8_t* qw, const void* scales, const void* zeros, int 
       ((uintptr_t)qw & 15) == 0 && ((uintptr_t)out & 15) == 0 && (pdt == LL_BF16 || pdt == LL_F32)) {
     dim3 fgrid(N / 64, K / 128);
     if (pdt == LL_BF16)
-      get_weight_int4_bf16_kernel<__nv_bfloat16><<<fgrid, 256, 0, st>>>(qw, (const __nv_bfloat16*)scales, (const __nv_bfloat16*)zeros, (__nv_bfloat16*)out, N, K, tile, G);
+      get_weight_int4_pairs_kernel<<<dim3(N / 64, (K / 128 + GW_DEEP - 1) / GW_DEEP), 256, 0, st>>>(qw, (const __nv_bfloat16*)scales, (const __nv_bfloat16*)zeros,
+                                                                                               (__nv_bfloat16*)out, N, K, tile, G);
     else
       get_weight_int4_bf16_kernel<float><<<fgrid, 256, 0, st>>>(qw, (const float*)scales, (const float*)zeros, (__nv_bfloat16*)out, N, K, tile, G);
     LL_LAUNCH_OK("get_weight_int4_bf16_kernel");
