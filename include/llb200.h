@@ -22,7 +22,7 @@
 extern "C" {
 #endif
 
-#define LL_ABI_VERSION 19
+#define LL_ABI_VERSION 20
 
 #define LL_OK 0
 #define LL_ERR_ARG (-1)         /* bad shape / dtype / null pointer */
@@ -189,6 +189,14 @@ LL_API int ll_int4_gemv(const ll_gemv_args* args /* host */, ll_stream stream);
  * K % 8 == 0; any M, N (tails are zero-filled by TMA and masked on store).
  * ------------------------------------------------------------------------------------- */
 LL_API int ll_gemm_bf16_tc(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, ll_stream stream);
+/* The same with tiles of 256 rows x tile_columns (128 or 256) columns a pair of CTAs; 0: the cheaper one by the sizes, as ll_gemm_bf16_tc. */
+LL_API int ll_gemm_bf16_tc_form(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int tile_columns, ll_stream stream);
+/* Two layers that read the same x, and their gated product: h[M][N] = silu(x . W1^T (+ bias1)) * (x . W2^T (+ bias2)), every step rounded to
+ * bf16 as ll_gemm_bf16_tc twice and ll_silu_mul round it. */
+LL_API int ll_gemm_bf16_gated(const void* x, const void* w1, const void* bias1, const void* w2, const void* bias2, void* h, int M, int N, int K,
+                              ll_stream stream);
+/* 0, or the code of the first bounded wait that ran out in the pairs' kernel.  Synchronises the device. */
+LL_API int ll_gemm_bf16_tc_error(void);
 
 /* Many rows (prompts): y[M][N] = x[M][K] . W^T (+ bias) in bf16 with W de-quantised in the main loop from the CHECKPOINT bytes [K/2][N]
  * (scales / zeros bf16 [N][K / group]), with the reference's bf16 rounding steps: what ll_get_weight + ll_gemm_bf16_tc compute, without the

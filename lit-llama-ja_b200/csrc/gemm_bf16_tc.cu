@@ -4,164 +4,259 @@
 // get_weight(dtype=bf16), quantization.py:390-409), so the result is the reference's fallback branch
 // F.linear(inp, get_weight(inp.dtype)) (quantization.py:420-421) with fp32 accumulation - the branch the
 // reference takes for every grouped checkpoint and the semantics of its Triton kernel for per-row ones.
-// Used for prefill of layers the many-row kernel (int4_rows.cu) does not take and for steps of more than 8192 rows; replaces Triton's mma.sync kernel
+// Used for prefill of layers the many-row kernel (int4_rows.cu) does not take and for steps of more than 6144 rows; replaces Triton's mma.sync kernel
 // (quantization.py:185-280).
 //
-// Structure (one 128 x BN output tile per CTA, 192 threads):
-//   warp 0   : TMA producer - 2-D tiled loads (128B swizzle) of X[128 x 64] and W[BN x 64] into a ring
-//   warp 1   : TMEM allocation; one elected thread issues tcgen05.mma (128 x BN x 16, kind::f16, bf16 inputs,
-//              fp32 accumulator in TMEM); tcgen05.commit releases ring slots / signals the epilogue
-//   warps 2-5: epilogue - tcgen05.ld (32 lanes x 32 columns per instruction), bias, bf16, global stores
 #include "tcgen05.cuh"
 
 namespace llb {
 namespace {
 
 
-template <int BN, int STAGES>
-__global__ void __launch_bounds__(192, 1) gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                              const __grid_constant__ CUtensorMap map_b,
-                                                              __nv_bfloat16* __restrict__ C,
-                                                              const __nv_bfloat16* __restrict__ bias, int M, int N, int K) {
-  constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
+// ==================================================================================== pairs of CTAs
+// Tiles of 256 rows x BN columns a pair (tcgen05 cta_group::2: a CTA has 128 rows of x, half of the tile's rows of W and
+// the sums of its 128 rows), persistent, with two accumulators in tensor memory, so that a tile's epilogue runs under the next one's products.
+// A CTA of its own takes 128 x 256 and reads 1.5 times the operand bytes per product from L2; one tile per CTA leaves its prologue and
+// epilogue in the open.
+//   GP_GATED: the two layers of a gated feed-forward that read the same x: the tile's columns are 128 of W1 (brought by rank 0) and the same
+//   128 of W2 (rank 1), and y = silu(x W1^T) * (x W2^T), each step rounded as the separate kernels round it.
+//   warp 0   : TMA producer;  warp 1 : in rank 0, one thread issues the products;  warps 2-5: epilogue, a row per thread, boxes of 32 rows x
+//   64 columns stored by TMA from a staging place per warp
+// Bound by the products: us, a tile of 128 x 256 per CTA / pairs: 13824 x 5120 at 512, 2048, 16384 rows 86 / 56, 277 / 182, 2161 / 1452
+// (1.60 PFLOP/s, as the library's); 4096 x 11008 at 512 rows 51 / 38.  The gated form of 16384 rows: 2864 for both layers and their product.
+// Tiles are walked in blocks of GP_BAND row tiles, columns outermost within a block: what the pairs work on at a time is about as many row
+// tiles as column tiles, so that W and x come from HBM once a block, not once a row tile.
+// Every wait is bounded, as in the other tcgen05 kernels.
+constexpr int GP_BAND = 8, GP_OUT = 32 * 128, GP_SMEM = 192 * 1024 + 4 * 2 * GP_OUT + 512 + 1024;
+constexpr uint32_t GP_WAIT_LIMIT = 1u << 22;
+__device__ int g_gp_error = 0;
+
+struct GpParams {
+  __nv_bfloat16* y;
+  const __nv_bfloat16* bias[2];
+  int M, N, nkb, mtiles, ntiles, boxes;      // boxes: y's rows are multiples of 16 bytes, TMA can store them
+  int* word;
+};
+struct GpFail {
+  volatile int* here;
+  uint32_t there;
+  int* word;
+};
+__device__ __forceinline__ bool gp_wait(uint64_t* bar, uint32_t parity, const GpFail& f, int code) {
+  for (uint32_t i = 0; i < GP_WAIT_LIMIT; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && *f.here) return false;
+  }
+  *f.here = 1;
+  store_cluster_u32(f.there, 1u);
+  atomicCAS(&g_gp_error, 0, code);
+  wait_ran_out(f.word, 600 + code);
+  return false;
+}
+__device__ __forceinline__ void gp_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void gp_tile(const GpParams& p, int t, int& mt, int& nt) {
+  const int per = GP_BAND * p.ntiles, blk = t / per, r = t - blk * per, rows = min(GP_BAND, p.mtiles - blk * GP_BAND);
+  nt = r / rows;
+  mt = blk * GP_BAND + (r - nt * rows);
+}
+
+template <int BN, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+    gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                     const __grid_constant__ CUtensorMap map_y, const GpParams p) {
+  constexpr int A_BYTES = 128 * BK * 2, B_BYTES = BN / 2 * BK * 2, STAGES = 192 * 1024 / (A_BYTES + B_BYTES);
+  constexpr int COLS = GATED ? BN / 2 : BN;            // outputs of a tile
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sa = base;                      // [STAGES][128][64] bf16, swizzled
-  uint8_t* sb = base + STAGES * A_BYTES;   // [STAGES][BN][64]
-  uint64_t* full = reinterpret_cast<uint64_t*>(sb + STAGES * B_BYTES);
+  uint8_t *sa = base, *sb = base + STAGES * A_BYTES, *so = base + 192 * 1024;
+  uint64_t* full = reinterpret_cast<uint64_t*>(so + 4 * 2 * GP_OUT);        // used in rank 0
   uint64_t* empty = full + STAGES;
-  uint64_t* tmem_full = empty + STAGES;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(tmem_full + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n_blk = blockIdx.x, m_blk = blockIdx.y;
-  const int nkb = (K + BK - 1) / BK;
-
-  if (warp == 0 && lane == 0) {
-    prefetch_tensormap(&map_a);
-    prefetch_tensormap(&map_b);
-    for (int i = 0; i < STAGES; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 1);
-    }
-    mbar_init(tmem_full, 1);
+  uint64_t* acc_full = empty + STAGES;                 // [2]
+  uint64_t* acc_empty = acc_full + 2;                  // [2], used in rank 0: both CTAs' warps arrive
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_x);
+    prefetch_tensormap(&map_w0);
+    prefetch_tensormap(&map_w1);
+    prefetch_tensormap(&map_y);
+    for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 8);
+    *s_fail = 0;
     fence_barrier_init();
   }
-  if (warp == 1) tmem_alloc(tmem_ptr, BN);  // BN fp32 accumulator columns (power of two >= 32)
+  if (warp == 1) pair_tmem_alloc(tmem_ptr, 2 * BN);
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   tc_fence_after();
-  const uint32_t tmem_d = *tmem_ptr;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  const GpFail fail{s_fail, cluster_addr(s_fail, (uint32_t)(rank ^ 1)), p.word};
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, tiles = p.mtiles * p.ntiles, nkb = p.nkb;
+  pdl_wait();
+  pdl_launch_dependents();
 
   if (warp == 0) {
-    // ===================== TMA producer =====================
-    if (lane == 0) {
-      const uint64_t pol_keep = 0;  // default policy (both operands are re-read by other CTAs through L2)
-      (void)pol_keep;
+    if (elect_one()) {
+      bool ok = true;
       int s = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < nkb; ++kb) {
-        mbar_wait_parity(&empty[s], phase ^ 1);
-        mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
-        asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                smem_u32(sa + s * A_BYTES)),
-            "l"(&map_a), "r"(kb * BK), "r"(m_blk * BM), "r"(smem_u32(&full[s]))
-            : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                smem_u32(sb + s * B_BYTES)),
-            "l"(&map_b), "r"(kb * BK), "r"(n_blk * BN), "r"(smem_u32(&full[s]))
-            : "memory");
-        if (++s == STAGES) {
-          s = 0;
-          phase ^= 1u;
+      uint32_t ph = 1;
+      for (int t = pair; ok && t < tiles; t += pairs) {
+        int mt, nt;
+        gp_tile(p, t, mt, nt);
+        const int m0 = mt * 256 + rank * 128, n0 = nt * COLS + (GATED ? 0 : rank * (BN / 2));
+        const CUtensorMap* mw = GATED && rank == 1 ? &map_w1 : &map_w0;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = gp_wait(&empty[s], ph, fail, 1))) break;
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * (A_BYTES + B_BYTES));      // both CTAs' operands
+          const uint32_t bar = cluster_addr(&full[s], 0);
+          pair_box(sa + s * A_BYTES, &map_x, kb * BK, m0, bar);
+          pair_box(sb + s * B_BYTES, mw, kb * BK, n0, bar);
+          if (++s == STAGES) s = 0, ph ^= 1u;
         }
       }
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == 1) {
-    // ===================== MMA issuer =====================
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
-      int s = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < nkb; ++kb) {
-        mbar_wait_parity(&full[s], phase);
+    if (elect_one()) {
+      constexpr uint32_t idesc = instr_desc_bf16(256, BN);
+      const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
+      bool ok = true;
+      int s = 0, i = 0;
+      uint32_t ph = 0;
+      for (int t = pair; rank == 0 && ok && t < tiles; t += pairs, ++i) {
+        const uint32_t d = tmem + (uint32_t)((i & 1) * BN);
+        if (!(ok = gp_wait(&acc_empty[i & 1], (uint32_t)((i >> 1) & 1) ^ 1u, fail, 4))) break;
         tc_fence_after();
-        const uint64_t adesc = smem_desc_sw128(smem_u32(sa + s * A_BYTES));
-        const uint64_t bdesc = smem_desc_sw128(smem_u32(sb + s * B_BYTES));
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = gp_wait(&full[s], ph, fail, 2))) break;
+          tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          // advance 16 elements = 32 bytes along K inside the swizzle atom: +2 in the (>>4) address field
-          umma_bf16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            gp_mma(d, ad + (uint64_t)(s * (A_BYTES >> 4) + 2 * k), bd + (uint64_t)(s * (B_BYTES >> 4) + 2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+          pair_commit(&empty[s]);
+          if (++s == STAGES) s = 0, ph ^= 1u;
         }
-        umma_commit(&empty[s]);  // frees the ring slot when these MMAs have read it
-        if (++s == STAGES) {
-          s = 0;
-          phase ^= 1u;
-        }
+        if (ok) pair_commit(&acc_full[i & 1]);
       }
-      umma_commit(tmem_full);  // accumulator complete
+      if (!ok) let_issued_work_end();
     }
   } else {
-    // ===================== epilogue (warps 2..5) =====================
-    const int quarter = warp & 3;  // a warp may only touch TMEM lanes [32 * (warpid % 4), +32)
-    const int row = m_blk * BM + quarter * 32 + lane;
-    mbar_wait_parity(tmem_full, 0);
-    tc_fence_after();
+    const int quarter = warp & 3;
+    uint8_t* out = so + quarter * 2 * GP_OUT;
+    int i = 0;
+    uint32_t boxes = 0;
+    for (int t = pair; t < tiles; t += pairs, ++i) {
+      int mt, nt;
+      gp_tile(p, t, mt, nt);
+      const int r0 = mt * 256 + rank * 128 + quarter * 32, n0 = nt * COLS;
+      if (!__all_sync(0xffffffffu, gp_wait(&acc_full[i & 1], (uint32_t)(i >> 1) & 1u, fail, 3))) break;
+      tc_fence_after();
+      const uint32_t td = tmem + (uint32_t)((i & 1) * BN) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-      uint32_t v[32];
-      tmem_ld_32x32(tmem_d + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-      const int col = n_blk * BN + c0;
-      if (row < M && col < N) {
-        __nv_bfloat16* dst = C + (size_t)row * N + col;
-        if (col + 32 <= N && (N & 7) == 0) {
+      for (int c0 = 0; c0 < COLS; c0 += 64) {
+        uint32_t o[32];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t pk[4];
+        for (int h = 0; h < 2; ++h) {
+          const int cc = c0 + 32 * h;
+          uint32_t v[32];
+          tmem_ld_32x32(td + (uint32_t)cc, v);
+          if (p.bias[0] != nullptr) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float f0 = __uint_as_float(v[j * 8 + 2 * e]), f1 = __uint_as_float(v[j * 8 + 2 * e + 1]);
-              if (bias != nullptr) {
-                f0 += __bfloat162float(bias[col + j * 8 + 2 * e]);
-                f1 += __bfloat162float(bias[col + j * 8 + 2 * e + 1]);
-              }
-              pk[e] = (uint32_t)f32_to_bf16_bits(f0) | ((uint32_t)f32_to_bf16_bits(f1) << 16);
+            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + (n0 + cc + e < p.N ? __bfloat162float(p.bias[0][n0 + cc + e]) : 0.f));
+          }
+          if (GATED) {
+            uint32_t u[32];
+            tmem_ld_32x32(td + (uint32_t)(BN / 2 + cc), u);
+            if (p.bias[1] != nullptr) {
+#pragma unroll
+              for (int e = 0; e < 32; ++e) u[e] = __float_as_uint(__uint_as_float(u[e]) + (n0 + cc + e < p.N ? __bfloat162float(p.bias[1][n0 + cc + e]) : 0.f));
             }
-            *reinterpret_cast<uint4*>(dst + j * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) {
+              v[e] = __float_as_uint(__fmul_rn(silu_act<__nv_bfloat16>(bf16r(__uint_as_float(v[e]))), bf16r(__uint_as_float(u[e]))));
+            }
           }
-        } else {
-          for (int j = 0; j < 32 && col + j < N; ++j) {
-            float f = __uint_as_float(v[j]);
-            if (bias != nullptr) f += __bfloat162float(bias[col + j]);
-            dst[j] = __float2bfloat16_rn(f);
-          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) o[16 * h + e] = pack_bf16(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
         }
+        if (c0 + 64 >= COLS) {               // the sums have left tensor memory
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[i & 1], 0));
+        }
+        if (p.boxes) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the box before the last has left
+          __syncwarp();
+          uint8_t* box = out + (boxes & 1u) * GP_OUT;
+          ++boxes;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) * 16)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            if (r0 < p.M && n0 + c0 < p.N)
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&map_y), "r"(n0 + c0), "r"(r0),
+                           "r"(smem_u32(box))
+                           : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        } else if (r0 + lane < p.M) {
+          __nv_bfloat16* dst = p.y + (size_t)(r0 + lane) * p.N + n0 + c0;
+#pragma unroll
+          for (int e = 0; e < 64; ++e)
+            if (n0 + c0 + e < p.N) dst[e] = __ushort_as_bfloat16((uint16_t)(o[e >> 1] >> (16 * (e & 1))));
+        }
+        __syncwarp();                        // the next load from tensor memory is the whole warp's
       }
-      __syncwarp();                  // the next load from tensor memory is the whole warp's
     }
     tc_fence_before();
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   }
   __syncthreads();
+  cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_d, BN);
+    pair_tmem_dealloc(tmem, 2 * BN);
   }
 }
 
-template <int BN, int STAGES>
-int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, __nv_bfloat16* C, const __nv_bfloat16* bias, int M, int N, int K,
-                cudaStream_t st) {
-  constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + (2 * STAGES + 1) * 8 + 16 + 1024;
+template <int BN, bool GATED>
+int launch_pair(const void* x, const void* w0, const void* w1, const void* b0, const void* b1, void* y, int M, int N, int K, cudaStream_t st) {
+  constexpr int COLS = GATED ? BN / 2 : BN;
+  GpParams p;
+  p.y = (__nv_bfloat16*)y, p.bias[0] = (const __nv_bfloat16*)b0, p.bias[1] = (const __nv_bfloat16*)b1;
+  p.M = M, p.N = N, p.nkb = (K + BK - 1) / BK, p.mtiles = (M + 255) / 256, p.ntiles = (N + COLS - 1) / COLS, p.boxes = N % 8 == 0;
+  p.word = wait_word();
+  const long long tiles = (long long)p.mtiles * p.ntiles;
+  LL_CHECK_ARG(tiles < (1ll << 30), "gemm_pair: too many tiles");
+  CUtensorMap mx, m0, m1, my;
+  if (int r = make_map(x, M, K, 128, &mx)) return r;
+  if (int r = make_map(w0, N, K, BN / 2, &m0)) return r;
+  if (int r = make_map(w1, N, K, BN / 2, &m1)) return r;
+  if (p.boxes) {
+    if (int r = make_map(y, M, N, 32, &my)) return r;
+  } else {
+    my = mx;
+  }
   static PerDevice configured;
   if (!configured) {
-    LL_CUDA(cudaFuncSetAttribute(gemm_bf16_tc_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LL_CUDA(cudaFuncSetAttribute(gemm_pair_kernel<BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, GP_SMEM));
     configured.mark();
   }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  gemm_bf16_tc_kernel<BN, STAGES><<<grid, 192, smem, st>>>(ma, mb, C, bias, M, N, K);
-  LL_LAUNCH_OK("gemm_bf16_tc_kernel");
+  const int pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  LL_CUDA(launch(gemm_pair_kernel<BN, GATED>, dim3(2 * (unsigned)(tiles < pairs ? tiles : pairs)), dim3(192), GP_SMEM, st, true, mx, m0, m1, my, p));
+  LL_LAUNCH_OK("gemm_pair_kernel");
   return LL_OK;
 }
 
@@ -504,20 +599,38 @@ using namespace llb;
 extern "C" {
 
 int ll_gemm_bf16_tc(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, ll_stream stream) {
+  return ll_gemm_bf16_tc_form(x, w, bias, y, M, N, K, 0, stream);
+}
+
+int ll_gemm_bf16_gated(const void* x, const void* w1, const void* bias1, const void* w2, const void* bias2, void* h, int M, int N, int K,
+                       ll_stream stream) {
+  LL_CHECK_ARG(x && w1 && w2 && h, "null pointer");
+  LL_CHECK_ARG(M > 0 && N > 0 && K > 0, "bad shape M=%d N=%d K=%d", M, N, K);
+  LL_CHECK_ARG(K % 8 == 0, "K must be a multiple of 8 (16-byte rows for TMA), got %d", K);
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)h) & 15) == 0, "x, the weights and h must be 16-byte aligned");
+  return launch_pair<256, true>(x, w1, w2, bias1, bias2, h, M, N, K, (cudaStream_t)stream);
+}
+
+int ll_gemm_bf16_tc_error(void) {
+  int v = 0;
+  return cudaMemcpyFromSymbol(&v, g_gp_error, sizeof(int)) == cudaSuccess ? v : -1;
+}
+
+int ll_gemm_bf16_tc_form(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, int tile_columns, ll_stream stream) {
   LL_CHECK_ARG(x && w && y, "null pointer");
   LL_CHECK_ARG(M > 0 && N > 0 && K > 0, "bad shape M=%d N=%d K=%d", M, N, K);
   LL_CHECK_ARG(K % 8 == 0, "K must be a multiple of 8 (16-byte rows for TMA), got %d", K);
   LL_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)y & 15) == 0, "x/w/y must be 16-byte aligned");
-  const int sms = sm_count();
-  // wide tiles once they fill the machine; narrower ones for small M (prefill of a few hundred tokens)
-  const long tiles256 = (long)((M + BM - 1) / BM) * ((N + 255) / 256);
-  const bool wide = tiles256 >= sms;
-  CUtensorMap ma, mb;
-  if (int r = make_map(x, M, K, BM, &ma)) return r;
-  if (int r = make_map(w, N, K, wide ? 256 : 128, &mb)) return r;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (wide) return launch_gemm<256, 4>(ma, mb, (__nv_bfloat16*)y, (const __nv_bfloat16*)bias, M, N, K, st);
-  return launch_gemm<128, 6>(ma, mb, (__nv_bfloat16*)y, (const __nv_bfloat16*)bias, M, N, K, st);
+  LL_CHECK_ARG(tile_columns == 0 || tile_columns == 128 || tile_columns == 256, "gemm_bf16_tc: tiles of 128 or 256 columns");
+  if (tile_columns == 0) {
+    // a tile of 128 columns takes 0.53 (many tiles a pair) to 0.67 (one) of the time of 256: what the waves cost.  us, 256 / 128 columns:
+    // 11008 x 4096 at 512 rows 45 / 42 (2 waves / 3), 2048 rows 119 / 133 (5 / 10); 4096 x 11008 at 512 rows 57 / 38 (1 / 1).
+    const long long pairs = sm_count() > 1 ? sm_count() / 2 : 1, mt = (M + 255) / 256;
+    const long long wide = (mt * ((N + 255) / 256) + pairs - 1) / pairs, narrow = (mt * ((N + 127) / 128) + pairs - 1) / pairs;
+    tile_columns = 3 * narrow < 5 * wide ? 128 : 256;
+  }
+  if (tile_columns == 256) return launch_pair<256, false>(x, w, w, bias, nullptr, y, M, N, K, (cudaStream_t)stream);
+  return launch_pair<128, false>(x, w, w, bias, nullptr, y, M, N, K, (cudaStream_t)stream);
 }
 
 size_t ll_int4_gemm_tc_scratch_bytes(int M, int N, int K) {

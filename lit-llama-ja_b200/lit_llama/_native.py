@@ -82,6 +82,9 @@ EXPORTS = {
     "ll_int4_gemv_plan": ([i32, i32, i32, i32, i32, i32, C.POINTER(sz_t), C.POINTER(C.c_int32)], C.c_int),
     "ll_int4_gemv": ([C.POINTER(GemvArgs), vp], C.c_int),
     "ll_gemm_bf16_tc": ([vp, vp, vp, vp, i32, i32, i32, vp], C.c_int),
+    "ll_gemm_bf16_tc_form": ([vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),
+    "ll_gemm_bf16_gated": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, vp], C.c_int),
+    "ll_gemm_bf16_tc_error": ([], C.c_int),
     "ll_int4_rows_supported": ([i32, i32, i32], C.c_int),
     "ll_int4_rows": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_form": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
@@ -192,7 +195,7 @@ EXPORTS = {
 }
 _fn = {name: _proto(name, a, r) for name, (a, r) in EXPORTS.items()}
 
-ABI_VERSION = 19
+ABI_VERSION = 20
 if _fn["ll_abi_version"]() != ABI_VERSION:
     raise ImportError("libllb200.so ABI version mismatch; rebuild with lit-llama-ja_b200/build.py")
 
