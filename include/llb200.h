@@ -204,10 +204,15 @@ LL_API int ll_gemm_bf16_tc_error(void);
 LL_API int ll_int4_rows_supported(int N, int K, int group);
 LL_API int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K,
                         int group, ll_stream stream);
-/* The same with tiles of tile_rows rows (128, 192 or 256; 0: the cheapest) on at most `grid` blocks (0: one an SM): which form runs is
- * otherwise a matter of the sizes. */
+/* The same with tiles of tile_rows rows (128 to 256, a multiple of 32; 0: the cheapest) on at most `grid` blocks (rounded up to pairs; 0: one
+ * an SM): which form runs is otherwise a matter of the sizes. */
 LL_API int ll_int4_rows_form(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N,
                              int K, int group, int tile_rows, int grid, ll_stream stream);
+/* Two layers that read the same x, and their gated product: h[M][N] = silu(x . W1^T (+ bias1)) * (x . W2^T (+ bias2)), every step rounded to
+ * bf16 as ll_int4_rows twice and ll_silu_mul round it.  Sizes as for ll_int4_rows, tile_rows and grid as for ll_int4_rows_form. */
+LL_API int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2,
+                              const void* scales2, const void* zeros2, const void* bias2, const void* x, void* h, int M, int N, int K, int group,
+                              int tile_rows, int grid, ll_stream stream);
 LL_API int ll_int4_rows_error(void);
 /* Fused int4 de-quantise + GEMM on tcgen05 for 1 <= M <= 128 rows (batched decode, short prefill; the HBM-bound regime):
  * y[M][N] (bf16) = x[M][K] (bf16) . W^T (+ bias), W de-quantised INSIDE the main loop from the packed stream

@@ -1,67 +1,80 @@
-// Many rows through an int4 layer on tcgen05 (prompts): y[M][N] = x[M][K] . dequant(W)^T, the weights read in their packed checkpoint form
+// Many rows through int4 layers on tcgen05 (prompts): y[M][N] = x[M][K] . dequant(W)^T, the weights read in their packed checkpoint form
 // (bytes [K/2][N], even k in the low half) and de-quantised inside the main loop with the reference's two bf16 roundings
-// (ref: lit_llama/quantization.py:399-408), so that no bf16 copy of W is written and read back.
+// (ref: lit_llama/quantization.py:399-408), so that no bf16 copy of W is written and read back.  A second form takes the two layers of a
+// gated feed-forward that read the same x: h = silu(x W1^T) * (x W2^T), each step rounded as the separate kernels round it.
 //
-// Operand roles are swapped: the weights are the A operand (128 output columns = the 128 TMEM lanes) and live in tensor memory, where the
-// threads that de-quantise them put them; the activations are the B operand, tiles of BN rows x 64 k loaded by TMA.
-//   warps 0, 2 : TMA producers: 128 k of BN rows of x; 64 x 128 packed bytes
-//   warp 1     : one thread issues 128 x BN x 16 MMAs (A from tensor memory)
+// Operand roles are swapped: the weights are the A operand and live in tensor memory, where the threads that de-quantise them put them; the
+// activations are the B operand, tiles of bn rows x 128 k loaded by TMA.  A pair of CTAs forms one product of 256 weight columns (128 = the
+// TMEM lanes of each) x bn rows, and each CTA brings half of the rows: of a CTA of its own x takes 72 KB a step of 128 k at 256 rows from L2,
+// 46 bytes a clock and SM; the pair needs 40 KB.  Unpacking reads the bytes by transposing loads (64 single-byte loads a thread before) and
+// the scales from shared memory; nothing of the loop may spill or miss in what is left of L1 (a spilled register doubled a step's time).
+// us, one CTA a tile / pairs: 11008 x 4096 at 150, 512, 1100 rows 28 / 24, 51 / 46, 82 / 69; 4096 x 11008 at 150, 512 rows 53 / 48, 87 / 54;
+// 32000 x 4096 at 512 rows 140 / 103.  Bound by products at 256 rows a tile (0.84 us a step with all SMs busy, 0.76 at the rate of a large
+// dense product), below that by unpacking.
+//   warps 0, 2 : TMA producers: 128 k of bn / 2 rows of x; 64 x 128 packed bytes
+//   warp 1     : in the CTA of rank 0, one thread issues 256 x bn x 16 MMAs (A from tensor memory) for both
+//   warp 3     : scales and zeros, several steps ahead
 //   warps 4-19 : de-quantise in four groups of four warps (a warp per TMEM lane quarter); group g makes every fourth step of 128 k into
 //                A buffer g, so that four steps are in the making at a time (one step's chain of waits, loads and stores is 1500 clocks
-//                long however many warps share it); then the epilogue, a quarter of the rows per group
-// Persistent: a CTA walks tiles with a stride of the grid; a group drains a tile after its first step of the next one, and gives the
+//                long however many warps share it); then the epilogue, every fourth 16 rows per group
+// Gated form: a CTA's 128 columns are 64 of W1 and the same 64 of W2; the warps of the first hand their sums, rounded, to those of the
+// second through shared memory.  (13824 x 5120, 1100 rows: 241 us; two layers and their product 274 before.)
+// Persistent: a pair walks tiles with a stride of the grid; a group drains a tile after its first step of the next one, and gives the
 // accumulator back as soon as it is in registers, so that the tensor cores wait for the drain alone.
-// Every wait is bounded; one that runs out records a code, all roles stop, copies in flight are waited for, tensor memory is freed.
+// Every wait is bounded; one that runs out records a code, all roles of both CTAs stop, copies in flight are waited for, tensor memory is
+// freed.
 #include "tcgen05.cuh"
 
 namespace llb {
 namespace {
 
-constexpr int R4_N = 128, R4_K = 128, R4_GROUPS = 4, R4_THREADS = (4 + 4 * R4_GROUPS) * 32;
-constexpr int R4_WBYTES = R4_N * R4_K / 2, R4_WST = R4_GROUPS;         // a stage of packed bytes per group
+constexpr int R4_K = 128, R4_GROUPS = 4, R4_THREADS = (4 + 4 * R4_GROUPS) * 32;
+constexpr int R4_WBYTES = 128 * R4_K / 2, R4_WST = 6;                  // stages of packed bytes
+constexpr int R4_SZ = 128 * 8 + 16;                                    // their columns' scales and zeros, and a word per 32 columns: all zeros whole
+constexpr int R4_XBYTES = 128 * 1024, R4_XST = 8;                      // the ring of x: as many stages of two halves [bn / 2 rows][64 k] as fit
+constexpr int R4_BOX = 16 * 64, R4_OUT = 2 * R4_BOX;                   // a warp stores 16 rows of 32 columns at a time, from two places in turn
+constexpr int R4_SWAP = 64 * 16 * 4;                                   // gated form: what a group hands over at a time, 64 columns x 32 rows of bf16
 constexpr uint32_t R4_WAIT_LIMIT = 1u << 20;
-__host__ __device__ constexpr int r4_xbytes(int bn) { return bn * R4_K * 2; }
-__host__ __device__ constexpr int r4_xst(int bn) { return bn >= 256 ? 3 : bn >= 192 ? 4 : 6; }
-constexpr int r4_smem(int bn) { return r4_xst(bn) * r4_xbytes(bn) + R4_WST * R4_WBYTES + 512 + 1024; }
+constexpr int R4_SMEM = R4_XBYTES + R4_WST * (R4_WBYTES + R4_SZ) + 4 * R4_GROUPS * R4_OUT + 512 + 1024;   // (gated: half the warps store, the rest is for the swap)
+static_assert(8 * R4_OUT >= R4_GROUPS * R4_SWAP, "the gated form's second half of the staging space");
 
 __device__ int g_r4_error = 0;
 
 struct R4Params {
-  const __nv_bfloat16* scales;   // [N][G]
-  const __nv_bfloat16* zeros;
-  const __nv_bfloat16* bias;
+  const __nv_bfloat16* scales[2];   // [N][G]; the second set: the gated form's W2
+  const __nv_bfloat16* zeros[2];
+  const __nv_bfloat16* bias[2];
   __nv_bfloat16* y;
-  int M, N, steps, G, steps_per_group, mtiles, tiles;
+  int M, N, steps, G, steps_per_group, wide, bn, xst, mtiles, tiles;
   int* word;                     // wait_word()
 };
 
-__device__ __forceinline__ bool r4_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
+struct R4Fail {                  // the flag that stops all roles, here and in the other CTA
+  volatile int* here;
+  uint32_t there;
+  int* word;
+};
+__device__ __forceinline__ void r4_give_up(const R4Fail& f, int code) {
+  *f.here = 1;
+  store_cluster_u32(f.there, 1u);
+  atomicCAS(&g_r4_error, 0, code);
+  wait_ran_out(f.word, 200 + code);
+}
+__device__ __forceinline__ bool r4_wait(uint64_t* bar, uint32_t parity, const R4Fail& f, int code) {
   for (uint32_t i = 0; i < R4_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && *fail) return false;
+    if ((i & 255u) == 255u && *f.here) return false;
   }
-  *fail = 1;
-  atomicCAS(&g_r4_error, 0, code);
-  wait_ran_out(word, 200 + code);
+  r4_give_up(f, code);
   return false;
 }
 // The same without suspending the thread between looks: for the thread that feeds the tensor cores, whose wake-up would be waited for.
-__device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
+__device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, const R4Fail& f, int code) {
   for (uint32_t i = 0; i < 64u * R4_WAIT_LIMIT; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((i & 255u) == 255u && *fail) return false;
+    if (mbar_test_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && *f.here) return false;
   }
-  *fail = 1;
-  atomicCAS(&g_r4_error, 0, code);
-  wait_ran_out(word, 200 + code);
+  r4_give_up(f, code);
   return false;
 }
 __device__ __forceinline__ void r4_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -73,16 +86,37 @@ __device__ __forceinline__ void r4_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ void r4_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                 "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+               : "r"(taddr)
+               : "memory");
+}
+// 32 k-pairs x 16 columns of packed bytes, four bytes of a column's k-pairs in a word: r[0], r[1] (r[2], r[3]: the next 16 k-pairs) hold
+// columns lane / 4 and lane / 4 + 8 and the k-pairs whose rows the lanes 4 (lane % 4) .. + 3 point at
+__device__ __forceinline__ void r4_ldt(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+// 16 lanes x 32 columns of tensor memory: of every 8 columns a thread writes columns 2 (lane % 4), + 1 of lanes lane / 4 and lane / 4 + 8
 __device__ __forceinline__ void r4_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
+      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
       "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
       "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
       : "memory");
+}
+__device__ __forceinline__ uint32_t r4_prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
 }
 __device__ __forceinline__ uint32_t r4_sub2(uint32_t a, uint32_t b) {
   uint32_t r;
@@ -95,64 +129,107 @@ __device__ __forceinline__ uint32_t r4_mul2(uint32_t a, uint32_t b) {
   return r;
 }
 
-template <int BN>
-__global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                                                                  const R4Params p) {
-  constexpr int XST = r4_xst(BN), XB = r4_xbytes(BN), PART = BN / R4_GROUPS;      // PART: rows a group drains
-  constexpr uint32_t TM_A = 256;                       // D: columns [0, BN); A buffers of 64 columns from 256 on
+// four bytes of a column -> the bf16 pairs of their k: (128 + q) - (128 + zero), exact for a whole zero; FRACTION: minus 128, minus zr (which is
+// 0 in columns whose zero is whole), each rounded as the reference does; times the scale
+template <bool FRACTION>
+__device__ __forceinline__ void r4_unpack(uint32_t w, uint32_t s2, uint32_t zc2, uint32_t zr2, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
+  const uint32_t lo = w & 0x0f0f0f0fu, hi = (w >> 4) & 0x0f0f0f0fu;
+  const uint32_t p = r4_prmt(lo, hi, 0x5140), q = r4_prmt(lo, hi, 0x7362);
+  uint32_t v[4] = {r4_prmt(p, 0x43u, 0x4140), r4_prmt(p, 0x43u, 0x4342), r4_prmt(q, 0x43u, 0x4140), r4_prmt(q, 0x43u, 0x4342)};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[i] = r4_sub2(v[i], zc2);
+    if (FRACTION) v[i] = r4_sub2(v[i], zr2);
+    v[i] = r4_mul2(v[i], s2);
+  }
+  o0 = v[0], o1 = v[1], o2 = v[2], o3 = v[3];
+}
+// what r4_ldt brought, as r4_st16 stores it; n: the numbers of columns lane / 4 and lane / 4 + 8
+template <bool FRACTION>
+__device__ __forceinline__ void r4_unpack16(const uint32_t (&w)[4], const uint2 (&n)[2], uint32_t (&r)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint2 v = n[i & 1];
+    const int o = (i >> 1) * 8 + (i & 1) * 2;
+    r4_unpack<FRACTION>(w[i], r4_prmt(v.x, 0u, 0x1010), r4_prmt(v.x, 0u, 0x3232), v.y, r[o], r[o + 1], r[o + 4], r[o + 5]);
+  }
+}
+
+template <bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
+    int4_rows_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_x,
+                     const __grid_constant__ CUtensorMap map_y, const R4Params p) {
+  constexpr uint32_t TM_A = 256;                       // D: columns [0, bn); A buffers of 64 columns from 256 on
+  constexpr int TILE_N = GATED ? 128 : 256;            // outputs of a pair
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sx = base;                                  // [XST][2][BN][64] bf16, swizzled
-  uint8_t* sw = base + XST * XB;                       // [WST][64][128] packed bytes
-  uint64_t* x_full = reinterpret_cast<uint64_t*>(sw + R4_WST * R4_WBYTES);
-  uint64_t* x_empty = x_full + XST;
-  uint64_t* w_full = x_empty + XST;
+  uint8_t* sx = base;                                  // [xst][2][bn / 2][64] bf16, swizzled
+  uint8_t* sw = base + R4_XBYTES;                      // [WST][2][64][64] packed bytes: two boxes of 64 columns, swizzled
+  uint8_t* so = sw + R4_WST * R4_WBYTES;               // [16 warps][2][16 rows][32 columns] bf16, swizzled
+  uint8_t* swap = so + 8 * R4_OUT;                     // gated form: [GROUPS][16 pairs of rows][64 columns]
+  uint8_t* sz = so + 4 * R4_GROUPS * R4_OUT;           // [WST][128] (scale | magic number of the zero << 16, rest), [4] whole
+  uint64_t* x_full = reinterpret_cast<uint64_t*>(sz + R4_WST * R4_SZ);               // used in rank 0
+  uint64_t* x_empty = x_full + R4_XST;
+  uint64_t* w_full = x_empty + R4_XST;
   uint64_t* w_empty = w_full + R4_WST;
-  uint64_t* a_ready = w_empty + R4_WST;
+  uint64_t* a_ready = w_empty + R4_WST;                // used in rank 0: both CTAs' warps arrive
   uint64_t* a_free = a_ready + R4_GROUPS;
   uint64_t* d_full = a_free + R4_GROUPS;
-  uint64_t* d_empty = d_full + 1;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(d_empty + 1);
+  uint64_t* d_empty = d_full + 1;                      // used in rank 0: both CTAs' warps arrive
+  uint64_t* g_full = d_empty + 1;                      // gated form: a group's first sums are there
+  uint64_t* g_empty = g_full + R4_GROUPS;              // and have been taken
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(g_empty + R4_GROUPS);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
   if (threadIdx.x == 0) {
-    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_w0);
+    prefetch_tensormap(&map_w1);
     prefetch_tensormap(&map_x);
-    for (int i = 0; i < XST; ++i) mbar_init(&x_full[i], 1), mbar_init(&x_empty[i], 1);
-    for (int i = 0; i < R4_WST; ++i) mbar_init(&w_full[i], 1), mbar_init(&w_empty[i], 4);
-    for (int i = 0; i < R4_GROUPS; ++i) mbar_init(&a_ready[i], 4), mbar_init(&a_free[i], 1);
+    prefetch_tensormap(&map_y);
+    for (int i = 0; i < R4_XST; ++i) mbar_init(&x_full[i], 1), mbar_init(&x_empty[i], 1);
+    for (int i = 0; i < R4_WST; ++i) mbar_init(&w_full[i], 2), mbar_init(&w_empty[i], 4);
+    for (int i = 0; i < R4_GROUPS; ++i) mbar_init(&a_ready[i], 8), mbar_init(&a_free[i], 1), mbar_init(&g_full[i], 2), mbar_init(&g_empty[i], 2);
     mbar_init(d_full, 1);
-    mbar_init(d_empty, 4 * R4_GROUPS);
+    mbar_init(d_empty, 2 * 4 * R4_GROUPS);
     *s_fail = 0;
     fence_barrier_init();
   }
-  if (warp == 1) tmem_alloc(tmem_ptr, 512);
+  if (warp == 1) pair_tmem_alloc(tmem_ptr, 512);
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
-  const int steps = p.steps;
+  const R4Fail fail{s_fail, cluster_addr(s_fail, (uint32_t)(rank ^ 1)), p.word};
+  const int steps = p.steps, bn = p.bn, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int xb = bn * 128, xst = p.xst;                // bytes of a stage of x in a CTA, stages
+  pdl_wait();                                          // (what comes before it runs under the kernel before)
+  pdl_launch_dependents();
 
   if (warp == 0 || warp == 2) {
     if (elect_one()) {
       bool ok = true;
       int s = 0;
       uint32_t ph = 1;
-      for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x) {
-        const int n0 = (tile / p.mtiles) * R4_N, m0 = (tile % p.mtiles) * BN;
+      for (int tile = pair; ok && tile < p.tiles; tile += pairs) {
+        const int n0 = (tile / p.mtiles) * TILE_N, m0 = (tile % p.mtiles) * bn + rank * (bn >> 1);
         if (warp == 0) {
           for (int kb = 0; kb < steps; ++kb) {
-            if (!(ok = r4_wait(&x_empty[s], ph, s_fail, p.word, 1))) break;
-            mbar_expect_tx(&x_full[s], XB);
-            r4_box(sx + s * XB, &map_x, kb * R4_K, m0, &x_full[s]);
-            r4_box(sx + s * XB + XB / 2, &map_x, kb * R4_K + 64, m0, &x_full[s]);
-            if (++s == XST) s = 0, ph ^= 1u;
+            if (!(ok = r4_wait(&x_empty[s], ph, fail, 1))) break;
+            if (rank == 0) mbar_expect_tx(&x_full[s], 2u * (uint32_t)xb);      // both CTAs' rows
+            const uint32_t bar = cluster_addr(&x_full[s], 0);
+            pair_box(sx + s * xb, &map_x, kb * R4_K, m0, bar);
+            pair_box(sx + s * xb + (xb >> 1), &map_x, kb * R4_K + 64, m0, bar);
+            if (++s == xst) s = 0, ph ^= 1u;
           }
         } else {
+          const int c0 = n0 + rank * (TILE_N / 2), c1 = GATED ? c0 : c0 + 64;
           for (int kb = 0; kb < steps; ++kb) {
-            if (!(ok = r4_wait(&w_empty[s], ph, s_fail, p.word, 2))) break;
+            if (!(ok = r4_wait(&w_empty[s], ph, fail, 2))) break;
             mbar_expect_tx(&w_full[s], R4_WBYTES);
-            r4_box(sw + s * R4_WBYTES, &map_w, n0, kb * (R4_K / 2), &w_full[s]);
+            r4_box(sw + s * R4_WBYTES, &map_w0, c0, kb * (R4_K / 2), &w_full[s]);
+            r4_box(sw + s * R4_WBYTES + R4_WBYTES / 2, GATED ? &map_w1 : &map_w0, c1, kb * (R4_K / 2), &w_full[s]);
             if (++s == R4_WST) s = 0, ph ^= 1u;
           }
         }
@@ -161,141 +238,240 @@ __global__ void __launch_bounds__(R4_THREADS, 1) int4_rows_kernel(const __grid_c
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = instr_desc_bf16(R4_N, BN);
+      const uint32_t idesc = instr_desc_bf16(256, bn);
       const uint64_t xd = smem_desc_sw128(smem_u32(sx));
       bool ok = true;
       int s = 0, tl = 0;
       uint32_t ph = 0, blk = 0;
-      for (int tile = blockIdx.x; ok && tile < p.tiles; tile += gridDim.x, ++tl) {
-        if (tl > 0 && !(ok = r4_wait(d_empty, (uint32_t)(tl - 1) & 1u, s_fail, p.word, 3))) break;
+      for (int tile = pair; rank == 0 && ok && tile < p.tiles; tile += pairs, ++tl) {
+        if (tl > 0 && !(ok = r4_wait(d_empty, (uint32_t)(tl - 1) & 1u, fail, 3))) break;
         for (int kb = 0; ok && kb < steps; ++kb, ++blk) {
           const uint32_t buf = blk % R4_GROUPS;
-          if (!(ok = r4_spin(&x_full[s], ph, s_fail, p.word, 5) && r4_spin(&a_ready[buf], (blk / R4_GROUPS) & 1u, s_fail, p.word, 4))) break;
+          if (!(ok = r4_spin(&x_full[s], ph, fail, 5) && r4_spin(&a_ready[buf], (blk / R4_GROUPS) & 1u, fail, 4))) break;
           tc_fence_after();
-          const uint64_t bd = xd + (uint64_t)(s * (XB >> 4));
+          const uint64_t bd = xd + (uint64_t)(s * (xb >> 4));
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            r4_mma(tmem, tmem + TM_A + 64u * buf + 8u * k, bd + (uint64_t)((k >> 2) * (XB >> 5) + 2 * (k & 3)), idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit(&a_free[buf]);
-          umma_commit(&x_empty[s]);
-          if (++s == XST) s = 0, ph ^= 1u;
+            r4_mma(tmem, tmem + TM_A + 64u * buf + 8u * k, bd + (uint64_t)((k >> 2) * (xb >> 5) + 2 * (k & 3)), idesc, (kb | k) != 0 ? 1u : 0u);
+          pair_commit(&a_free[buf]);
+          pair_commit(&x_empty[s]);
+          if (++s == xst) s = 0, ph ^= 1u;
         }
-        if (ok) umma_commit(d_full);
+        if (ok) pair_commit(d_full);
       }
       if (!ok) let_issued_work_end();
     }
-  } else if (warp >= 4) {
-    const int quarter = warp & 3, grp = (warp >> 2) - 1, col = quarter * 32 + lane;
-    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+  } else if (warp == 3) {
+    // scales and zeros, four steps ahead of their use at least: the groups of four steps lie side by side.  A column's numbers as the unpacking
+    // threads want them: its scale, and 128 + zero for one exact subtraction if the zero is whole (every RTN / GPTQ checkpoint), else 128 and
+    // the zero.  (Loaded by those threads one step ahead, 64 lines a warp and no L1 to speak of, they were half of a step's time.)
     bool ok = true;
+    int s = 0;
+    uint32_t ph = 1;
+    auto four = [&](const __nv_bfloat16* src, size_t row, int kb) {      // the numbers of steps kb .. kb + 3, in one load where rows allow it
+      const uint16_t* at = reinterpret_cast<const uint16_t*>(src) + row;
+      if (p.wide == 4) return *reinterpret_cast<const uint2*>(at + kb);
+      if (p.wide == 2)
+        return make_uint2(*reinterpret_cast<const uint32_t*>(at + kb), *reinterpret_cast<const uint32_t*>(at + min(kb + 2, p.G - 2)));
+      uint32_t v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = at[min(kb + j, steps - 1) / p.steps_per_group];
+      return make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+    };
+    auto fetch = [&](int tile, int kb, uint2 (&sv)[4], uint2 (&zv)[4]) {
+      const int n0 = (tile / p.mtiles) * TILE_N;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool second = GATED && q >= 2;
+        const int n = n0 + (GATED ? rank * 64 + (q & 1) * 32 : rank * 128 + q * 32) + lane;
+        const size_t row = (size_t)min(n, p.N - 1) * p.G;
+        sv[q] = four(second ? p.scales[1] : p.scales[0], row, kb);
+        zv[q] = four(second ? p.zeros[1] : p.zeros[0], row, kb);
+      }
+    };
+    uint2 sv[4], zv[4];
+    fetch(pair, 0, sv, zv);
+    for (int tile = pair; ok && tile < p.tiles; tile += pairs) {
+      for (int kb = 0; ok && kb < steps; kb += 4) {
+        uint2 sn[4], zn[4];
+        const bool last = kb + 4 >= steps;
+        if (!last || tile + pairs < p.tiles) fetch(last ? tile + pairs : tile, last ? 0 : kb + 4, sn, zn);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (kb + j >= steps) break;
+          ok = __all_sync(0xffffffffu, r4_wait(&w_empty[s], ph, fail, 11));
+          if (!ok) break;
+          uint2* dst = reinterpret_cast<uint2*>(sz + s * R4_SZ);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t sc = ((j < 2 ? sv[q].x : sv[q].y) >> (16 * (j & 1))) & 0xffffu, ze = ((j < 2 ? zv[q].x : zv[q].y) >> (16 * (j & 1))) & 0xffffu;
+            const float zf = __uint_as_float(ze << 16);
+            const bool whole = zf == floorf(zf) && zf >= 0.f && zf <= 64.f;
+            dst[q * 32 + lane] = make_uint2(sc | ((whole ? 0x4300u + (uint32_t)zf : 0x4300u) << 16), whole ? 0u : ze * 0x00010001u);
+            const bool all = __all_sync(0xffffffffu, whole);
+            if (lane == 0) reinterpret_cast<uint32_t*>(dst + 128)[q] = all ? 1u : 0u;
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&w_full[s]);
+          if (++s == R4_WST) s = 0, ph ^= 1u;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sv[q] = sn[q], zv[q] = zn[q];
+      }
+    }
+  } else {
+    const int quarter = warp & 3, grp = (warp - 4) >> 2, half = quarter >> 1;        // half: the CTA's first or last 64 columns
+    const int col = (GATED ? rank * 64 : rank * 128 + half * 64) + (quarter & 1) * 32 + lane;      // within the pair's outputs
+    const bool second = GATED && half == 1;             // columns of W2
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    const uint32_t a_ready0 = cluster_addr(&a_ready[grp], 0), d_empty0 = cluster_addr(d_empty, 0);
+    bool ok = true;
+    uint32_t boxes = 0, swaps = 0;
     // a finished tile: its sums leave tensor memory, then the accumulator is given back, then they are stored
     auto drain = [&](int tile, uint32_t nth) {
-      ok = __all_sync(0xffffffffu, r4_wait(d_full, nth & 1u, s_fail, p.word, 6));
+      ok = __all_sync(0xffffffffu, r4_wait(d_full, nth & 1u, fail, 6));
       if (!ok) return;
       tc_fence_after();
-      const int n = (tile / p.mtiles) * R4_N + col, m0 = (tile % p.mtiles) * BN + grp * PART;
-      const float bias = p.bias != nullptr && n < p.N ? __bfloat162float(p.bias[n]) : 0.f;
-      uint32_t w[PART / 2];
+      const int n = (tile / p.mtiles) * TILE_N + col, m0 = (tile % p.mtiles) * bn;
+      const __nv_bfloat16* b = second ? p.bias[1] : p.bias[0];
+      const float bias = b != nullptr && n < p.N ? __bfloat162float(b[n]) : 0.f;
+      uint32_t w[4][8];
 #pragma unroll
-      for (int c = 0; c < PART; c += 16) {
-        uint32_t v[16];
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-            "tcgen05.wait::ld.sync.aligned;"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-              "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tmem + lanes + (uint32_t)(grp * PART + c))
-            : "memory");
+      for (int c = 0; c < 4; c += 2) {       // (bn is a multiple of 32 above 64: pairs of chunks, and only the last chunk of a group can be missing)
+        if ((grp + 4 * c) * 16 >= bn) break;
+        const bool two = (grp + 4 * (c + 1)) * 16 < bn;
+        uint32_t v[32];
+        r4_ld16(tmem + lanes + (uint32_t)((grp + 4 * c) * 16), v);
+        if (two) r4_ld16(tmem + lanes + (uint32_t)((grp + 4 * c + 4) * 16), v + 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int e = 0; e < 16; e += 2) w[(c + e) / 2] = pack_bf16(__uint_as_float(v[e]) + bias, __uint_as_float(v[e + 1]) + bias);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(d_empty);
-      // a lane holds two rows of its column in a word; neighbours swap, so that a lane stores two columns of one row
-      const bool odd = (lane & 1) != 0;
-      __nv_bfloat16* dst = p.y + (size_t)(m0 + (odd ? 1 : 0)) * p.N + (n & ~1);
-      const int left = p.M - m0 - (odd ? 1 : 0);
+        for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(v[e]), "+r"(v[e + 16]));       // (the loads' results are there from here on)
 #pragma unroll
-      for (int e = 0; e < PART / 2; ++e) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, w[e], 1);
-        const uint32_t o = odd ? (got >> 16) | (w[e] & 0xffff0000u) : (w[e] & 0xffffu) | (got << 16);
-        if (2 * e < left && n < p.N) *reinterpret_cast<uint32_t*>(dst + (size_t)(2 * e) * p.N) = o;
-      }
-      __syncwarp();
-    };
-    // the group's steps: every fourth of all steps of all of the CTA's tiles
-    int tile = blockIdx.x, kb = grp, drained = blockIdx.x;
-    uint32_t nth = 0;
-    auto normal = [&]() {
-      while (kb >= steps && tile < p.tiles) kb -= steps, tile += gridDim.x;
-    };
-    auto params = [&](uint32_t& sv, uint32_t& zv) {
-      if (tile >= p.tiles) return;
-      const size_t at = (size_t)min((tile / p.mtiles) * R4_N + col, p.N - 1) * p.G + kb / p.steps_per_group;
-      sv = *reinterpret_cast<const uint16_t*>(p.scales + at);
-      zv = *reinterpret_cast<const uint16_t*>(p.zeros + at);
-    };
-    uint32_t sn = 0, zn = 0, round = 0;      // round: the group's how-many-th step
-    normal();
-    params(sn, zn);
-    while (ok && tile < p.tiles) {
-      const int cur = tile;
-      const uint32_t s2 = sn * 0x00010001u, z2 = zn * 0x00010001u;
-      // an integer zero (every RTN / GPTQ checkpoint): (128 + q) - (128 + zero) in ONE exact subtraction
-      const float zf = __uint_as_float(zn << 16);
-      const bool zint = zf == floorf(zf) && zf >= 0.f && zf <= 64.f;
-      const uint32_t zc2 = zint ? (uint32_t)(0x4300u + (uint32_t)zf) * 0x00010001u : 0x43004300u;
-      // a column's zero may be whole and its neighbour's not: the warp goes one way (the store below is the whole warp's), a whole zero
-      // then subtracts 0
-      const bool one_step = __all_sync(0xffffffffu, zint);
-      const uint32_t zr2 = zint ? 0u : z2;
-      kb += R4_GROUPS;
-      normal();
-      params(sn, zn);                        // of the next step, under this one's work
-      const int s = grp;
-      ok = r4_wait(&w_full[s], round & 1u, s_fail, p.word, 7);
-      if (ok && round > 0) ok = r4_wait(&a_free[grp], (round - 1u) & 1u, s_fail, p.word, 8);
-      if (!(ok = __all_sync(0xffffffffu, ok))) break;
-      tc_fence_after();
-      const uint8_t* src = sw + s * R4_WBYTES + col;
-      const uint32_t ta = tmem + lanes + TM_A + 64u * grp;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t r[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const uint32_t b = src[(c * 16 + j) * R4_N];
-          uint32_t a = r4_sub2(((b * 0x1001u) & 0x000f000fu) | 0x43004300u, zc2);      // bf16 (128 + q) of both halves, minus 128 (+ zero)
-          if (!one_step) a = r4_sub2(a, zr2);
-          r[j] = r4_mul2(a, s2);
+        for (int e = 0; e < 8; ++e) {
+          w[c][e] = pack_bf16(__uint_as_float(v[2 * e]) + bias, __uint_as_float(v[2 * e + 1]) + bias);
+          w[c + 1][e] = pack_bf16(__uint_as_float(v[16 + 2 * e]) + bias, __uint_as_float(v[17 + 2 * e]) + bias);
         }
-        r4_st16(ta + 16u * c, r);
       }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&w_empty[s]), mbar_arrive(&a_ready[grp]);
-      ++round;
-      while (ok && drained < cur) {
-        drain(drained, nth++);
-        drained += gridDim.x;
+      if (lane == 0) mbar_arrive_cluster(d_empty0);
+      const bool odd = (lane & 1) != 0;
+      uint8_t* const out = so + (GATED ? grp * 2 + (quarter & 1) : grp * 4 + quarter) * R4_OUT;
+#pragma unroll
+      for (int c = 0; c < 4; c += 2) {
+        if ((grp + 4 * c) * 16 >= bn) break;
+        if (GATED) {
+          // (each lane of the second half meets the words of the same column in the first)
+          uint32_t* sums = reinterpret_cast<uint32_t*>(swap + grp * R4_SWAP) + (quarter & 1) * 32 + lane;
+          if (half == 0) {
+            if (swaps > 0) ok = __all_sync(0xffffffffu, r4_wait(&g_empty[grp], (swaps - 1u) & 1u, fail, 9));
+            if (!ok) return;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {   // (the first half forms the silu, the second the product and the boxes)
+              const uint32_t g = w[c + (e >> 3)][e & 7];
+              sums[e * 64] = pack_bf16(silu_fast(__uint_as_float(g << 16)), silu_fast(__uint_as_float(g & 0xffff0000u)));
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&g_full[grp]);
+            ++swaps;
+            continue;
+          }
+          ok = __all_sync(0xffffffffu, r4_wait(&g_full[grp], swaps & 1u, fail, 10));
+          if (!ok) return;
+          ++swaps;
+#pragma unroll
+          for (int e = 0; e < 16; ++e) w[c + (e >> 3)][e & 7] = r4_mul2(sums[e * 64], w[c + (e >> 3)][e & 7]);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&g_empty[grp]);
+        }
+        // a lane holds two rows of its column in a word; neighbours swap, so that a lane has two columns of one row; 16 rows x 32 columns go
+        // out as one box while the warp is back at its next step (rows past M and columns past N stay out)
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+          const int r0 = m0 + (grp + 4 * (c + d)) * 16, nb = n - lane;
+          if (r0 >= m0 + bn) break;
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the box before the last has left
+          __syncwarp();
+          uint8_t* box = out + (boxes & 1u) * R4_BOX;
+          ++boxes;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const uint32_t v = w[c + d][e], got = __shfl_xor_sync(0xffffffffu, v, 1);
+            const uint32_t o = odd ? (got >> 16) | (v & 0xffff0000u) : (v & 0xffffu) | (got << 16);
+            *reinterpret_cast<uint32_t*>(box + (2 * e + (odd ? 1 : 0)) * 64 + ((((lane >> 3) ^ e) & 3) * 16) + ((lane >> 1) & 3) * 4) = o;
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            if (r0 < p.M && nb < p.N)
+              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&map_y), "r"(nb), "r"(r0), "r"(smem_u32(box))
+                           : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
       }
-    }
+    };
+    // the group's steps: every fourth of all steps of all of the pair's tiles
+    int tile = pair, kb = grp, drained = pair, s = grp;
+    uint32_t nth = 0, round = 0, wph = 0;    // round: the group's how-many-th step
+    while (kb >= steps && tile < p.tiles) kb -= steps, tile += pairs;
+    // the row of packed bytes (64 of them, 16-byte pieces swizzled) a lane points at: of 16 k-pairs, four lanes name those of which the threads
+    // of one lane % 4 write two and two tensor-memory columns
+    const int li = lane & 15, krow = (lane >> 4) * 16 + (li >> 2) * 2 + (li & 1) + (li & 2) * 4;
+    const uint32_t row_at = (uint32_t)(krow * 64), turn = (uint32_t)(((krow >> 1) & 3) * 16);
     while (ok && drained < p.tiles) {
-      drain(drained, nth++);
-      drained += gridDim.x;
+      const int upto = min(tile, p.tiles);   // tiles before this one can be drained
+      bool step = tile < p.tiles;
+      if (step) {
+        ok = r4_wait(&w_full[s], wph, fail, 7);
+        if (ok && round > 0) ok = r4_wait(&a_free[grp], (round - 1u) & 1u, fail, 8);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        // a tile that is done already (for the group whose step was its last) is drained before the step, others after it
+        step = drained >= upto || !__any_sync(0xffffffffu, mbar_test_wait(d_full, nth & 1u));
+      }
+      if (step) {
+        tc_fence_after();
+        const uint32_t src = smem_u32(sw + s * R4_WBYTES + half * (R4_WBYTES / 2)) + row_at;
+        const uint32_t ta = tmem + lanes + TM_A + 64u * grp, nums = smem_u32(sz + s * R4_SZ) + (uint32_t)((quarter * 32 + (lane >> 2)) * 8);
+        const bool whole = reinterpret_cast<const uint32_t*>(sz + s * R4_SZ + 128 * 8)[quarter] != 0u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {        // 16 of the warp's 32 columns
+          const uint2 n[2] = {lds64(nums + h * 128), lds64(nums + h * 128 + 64)};
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {      // 32 of the step's 64 k-pairs
+            uint32_t w[4], r[16];
+            r4_ldt(src + ((uint32_t)((quarter & 1) * 32 + h * 16) ^ turn) + (uint32_t)(c * 32 * 64), w);
+            if (whole) r4_unpack16<false>(w, n, r);
+            else r4_unpack16<true>(w, n, r);
+            r4_st16(ta + ((uint32_t)(16 * h) << 16) + 32u * c, r);
+          }
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&w_empty[s]), mbar_arrive_cluster(a_ready0);
+        kb += R4_GROUPS;
+        while (kb >= steps && tile < p.tiles) kb -= steps, tile += pairs;
+        ++round;
+        if ((s += R4_GROUPS) >= R4_WST) s -= R4_WST, wph ^= 1u;
+      }
+      while (ok && drained < upto) {
+        drain(drained, nth++);
+        drained += pairs;
+      }
     }
     tc_fence_before();
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   }
   __syncthreads();
+  cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    pair_tmem_dealloc(tmem, 512);
   }
 }
 
-// packed bytes [K/2][N] as a 2-D map, boxes of 128 columns x 64 rows
+// packed bytes [K/2][N] as a 2-D map, boxes of 64 columns x 64 rows
 int r4_weight_map(const void* qw, int N, int K, CUtensorMap* out) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) {
@@ -303,9 +479,9 @@ int r4_weight_map(const void* qw, int N, int K, CUtensorMap* out) {
     return LL_ERR_CUDA;
   }
   cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)(K / 2)}, strides[1] = {(cuuint64_t)N};
-  cuuint32_t box[2] = {R4_N, R4_K / 2}, estr[2] = {1, 1};
+  cuuint32_t box[2] = {64, R4_K / 2}, estr[2] = {1, 1};
   const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)qw, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled failed (%d): packed weights N=%d K=%d", (int)r, N, K);
     return LL_ERR_CUDA;
@@ -313,23 +489,65 @@ int r4_weight_map(const void* qw, int N, int K, CUtensorMap* out) {
   return LL_OK;
 }
 
-template <int BN>
-int r4_launch(const CUtensorMap& mw, const void* x, R4Params p, int K, int grid, cudaStream_t st) {
-  CUtensorMap mx;
-  if (int r = make_map(x, p.M, K, BN, &mx)) return r;
-  LL_CUDA(cudaFuncSetAttribute(int4_rows_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, r4_smem(BN)));
-  p.mtiles = (p.M + BN - 1) / BN;
-  p.tiles = p.mtiles * ((p.N + R4_N - 1) / R4_N);
-  int4_rows_kernel<BN><<<p.tiles < grid ? p.tiles : grid, R4_THREADS, r4_smem(BN), st>>>(mw, mx, p);
-  LL_LAUNCH_OK("int4_rows_kernel");
+// the output, boxes of 16 rows x 32 columns
+int r4_out_map(const void* y, int M, int N, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled entry point not available");
+    return LL_ERR_CUDA;
+  }
+  cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M}, strides[1] = {(cuuint64_t)N * 2};
+  cuuint32_t box[2] = {32, 16}, estr[2] = {1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d): output M=%d N=%d", (int)r, M, N);
+    return LL_ERR_CUDA;
+  }
   return LL_OK;
 }
 
-// Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time (see the head of the file), plus the drain.  (A
-// step takes 600 clocks at least, however few the rows: tiles of 64 never cost less than tiles of 128.)
-long long r4_cost(int M, int N, int steps, int bn, int sms) {
-  const long long tiles = (long long)((M + bn - 1) / bn) * ((N + R4_N - 1) / R4_N);
-  return (tiles + sms - 1) / sms * ((long long)steps * (4 * bn > 600 ? 4 * bn : 600) + 1200);
+// Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time, plus the drain.  A step costs its products, or, with
+// few rows, its unpacking (us a step of 13824 x 5120, 900 rows, tiles of 128 / 160 / 192 / 224 / 256 rows: .54 / .56 / .61 / .66 / .78).
+long long r4_cost(int M, int N, int tile_n, int steps, int bn, int pairs) {
+  const long long tiles = (long long)((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n);
+  const int products = 4 * bn, unpack = 530 + 7 * bn / 5;
+  return (tiles + pairs - 1) / pairs * ((long long)steps * (products > unpack ? products : unpack) + 1500);
+}
+
+template <bool GATED>
+int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p, int K, int tile_rows, int grid, cudaStream_t st) {
+  constexpr int TILE_N = GATED ? 128 : 256;
+  const int sms = grid > 0 ? grid : sm_count();
+  const int pairs = sms > 1 ? (grid > 0 ? (sms + 1) / 2 : sms / 2) : 1;
+  p.bn = tile_rows;
+  if (tile_rows == 0) {
+    p.bn = 256;
+    for (int bn = 224; bn >= 128; bn -= 32)
+      if (r4_cost(p.M, p.N, TILE_N, p.steps, bn, pairs) < r4_cost(p.M, p.N, TILE_N, p.steps, p.bn, pairs)) p.bn = bn;
+  }
+  p.xst = R4_XBYTES / (p.bn * 128);
+  // steps whose scales (and zeros) one load takes: a row of groups of 128 starts on its boundary, and no load passes a row's end
+  const uintptr_t at = (uintptr_t)p.scales[0] | (uintptr_t)p.scales[1] | (uintptr_t)p.zeros[0] | (uintptr_t)p.zeros[1];
+  p.wide = p.steps_per_group != 1 ? 1 : p.G % 4 == 0 && at % 8 == 0 ? 4 : p.G % 2 == 0 && at % 4 == 0 ? 2 : 1;
+  CUtensorMap mw0, mw1, mx, my;
+  if (int r = r4_weight_map(qw0, p.N, K, &mw0)) return r;
+  if (int r = r4_weight_map(qw1, p.N, K, &mw1)) return r;
+  if (int r = make_map(x, p.M, K, p.bn / 2, &mx)) return r;
+  if (int r = r4_out_map(p.y, p.M, p.N, &my)) return r;
+  static PerDevice configured;
+  if (!configured) {
+    LL_CUDA(cudaFuncSetAttribute(int4_rows_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, R4_SMEM));
+    configured.mark();
+  }
+  p.mtiles = (p.M + p.bn - 1) / p.bn;
+  const long long tiles = (long long)p.mtiles * ((p.N + TILE_N - 1) / TILE_N);
+  LL_CHECK_ARG(tiles < (1ll << 30), "int4_rows: too many tiles");
+  p.tiles = (int)tiles;
+  p.word = wait_word();
+  LL_CUDA(launch(int4_rows_kernel<GATED>, dim3(2 * (p.tiles < pairs ? p.tiles : pairs)), dim3(R4_THREADS), R4_SMEM, st, true, mw0, mw1, mx, my, p));
+  LL_LAUNCH_OK("int4_rows_kernel");
+  return LL_OK;
 }
 
 }  // namespace
@@ -354,23 +572,33 @@ int ll_int4_rows_form(const uint8_t* qw, const void* scales, const void* zeros, 
     return LL_ERR_UNSUPPORTED;
   }
   LL_CHECK_ARG((((uintptr_t)qw | (uintptr_t)x | (uintptr_t)y) & 15) == 0, "int4_rows: packed weights, x and y must be 16-byte aligned");
+  LL_CHECK_ARG((tile_rows == 0 || (tile_rows % 32 == 0 && tile_rows >= 128 && tile_rows <= 256)) && grid >= 0,
+               "int4_rows: tiles of 128 to 256 rows, a multiple of 32");
   R4Params p{};
-  p.scales = (const __nv_bfloat16*)scales, p.zeros = (const __nv_bfloat16*)zeros, p.bias = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
+  p.scales[0] = p.scales[1] = (const __nv_bfloat16*)scales, p.zeros[0] = p.zeros[1] = (const __nv_bfloat16*)zeros;
+  p.bias[0] = p.bias[1] = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
-  p.word = wait_word();
-  LL_CHECK_ARG((tile_rows == 0 || tile_rows == 128 || tile_rows == 192 || tile_rows == 256) && grid >= 0, "int4_rows: tiles of 128, 192 or 256 rows");
-  if (grid == 0) grid = sm_count();
-  CUtensorMap mw;
-  if (int r = r4_weight_map(qw, N, K, &mw)) return r;
-  if (tile_rows == 0) {
-    tile_rows = 256;
-    for (int bn = 192; bn >= 128; bn -= 64)
-      if (r4_cost(M, N, p.steps, bn, grid) < r4_cost(M, N, p.steps, tile_rows, grid)) tile_rows = bn;
+  return r4_launch<false>(qw, qw, x, p, K, tile_rows, grid, (cudaStream_t)stream);
+}
+
+int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
+                       const void* zeros2, const void* bias2, const void* x, void* h, int M, int N, int K, int group, int tile_rows, int grid,
+                       ll_stream stream) {
+  LL_CHECK_ARG(qw1 && scales1 && zeros1 && qw2 && scales2 && zeros2 && x && h && M > 0, "int4_rows_gated: null pointer or no rows");
+  if (!ll_int4_rows_supported(N, K, group)) {
+    set_error("int4_rows_gated needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
+    return LL_ERR_UNSUPPORTED;
   }
-  cudaStream_t st = (cudaStream_t)stream;
-  if (tile_rows == 256) return r4_launch<256>(mw, x, p, K, grid, st);
-  if (tile_rows == 192) return r4_launch<192>(mw, x, p, K, grid, st);
-  return r4_launch<128>(mw, x, p, K, grid, st);
+  LL_CHECK_ARG((((uintptr_t)qw1 | (uintptr_t)qw2 | (uintptr_t)x | (uintptr_t)h) & 15) == 0,
+               "int4_rows_gated: packed weights, x and h must be 16-byte aligned");
+  LL_CHECK_ARG((tile_rows == 0 || (tile_rows % 32 == 0 && tile_rows >= 128 && tile_rows <= 256)) && grid >= 0,
+               "int4_rows_gated: tiles of 128 to 256 rows, a multiple of 32");
+  R4Params p{};
+  p.scales[0] = (const __nv_bfloat16*)scales1, p.zeros[0] = (const __nv_bfloat16*)zeros1, p.bias[0] = (const __nv_bfloat16*)bias1;
+  p.scales[1] = (const __nv_bfloat16*)scales2, p.zeros[1] = (const __nv_bfloat16*)zeros2, p.bias[1] = (const __nv_bfloat16*)bias2;
+  p.y = (__nv_bfloat16*)h;
+  p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
+  return r4_launch<true>(qw1, qw2, x, p, K, tile_rows, grid, (cudaStream_t)stream);
 }
 
 // 0, or the code of the first bounded wait that ran out in this file's kernel.  Synchronises the device.

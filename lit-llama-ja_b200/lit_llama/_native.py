@@ -88,6 +88,7 @@ EXPORTS = {
     "ll_int4_rows_supported": ([i32, i32, i32], C.c_int),
     "ll_int4_rows": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_form": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
+    "ll_int4_rows_gated": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_error": ([], C.c_int),
     "ll_int4_gemm_tc_scratch_bytes": ([i32, i32, i32], sz_t),
     "ll_int4_gemm_tc": ([vp, vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),

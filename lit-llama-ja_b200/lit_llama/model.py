@@ -22,6 +22,7 @@ import torch.nn as nn
 from torch.nn import functional as F
 
 from . import _native as N
+from .quantization import gated_pair
 from .stepping import graph_capture
 from .utils import find_multiple
 
@@ -180,6 +181,9 @@ class MLP(nn.Module):
         self.c_proj = nn.Linear(config.n_hidden, config.n_embd, bias=False)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        h = gated_pair(self.c_fc1, self.c_fc2, x)
+        if h is not None:
+            return self.c_proj(h)
         a, b = self.c_fc1(x).contiguous(), self.c_fc2(x).contiguous()
         h = torch.empty_like(a)
         N.call("ll_silu_mul", N.ptr(a), N.ptr(b), N.ptr(h), N.dtype_code(a.dtype), a.numel(), N.stream())

@@ -153,13 +153,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
     FUSED_GEMM_MAX_M = 128       # rows one ll_int4_gemm_tc call takes
     # rows from which the weights are de-quantised in the main loop of the many-row kernel, from the checkpoint bytes.  Both sides measured
-    # (11008 x 4096, group 128): 130 rows 27 us against 61 in two passes of the small-row kernel and 87 with a bf16 copy of W; 512 rows
-    # 49 against 112; 2048 rows 137 against 220.
-    # Past 8192 rows the bf16 copy, written once, costs less than a tile of W de-quantised again for every 256 rows.  us, this kernel / copy
-    # and product, 150 ms of each in turn: 13824 x 5120 at 8192 rows
-    # 1067 / 1342, at 16384 2350 / 2618; 5120 x 13824: 1033 / 1160 and 2365 / 2245; 4096 x 11008: 682 / 713 and 1522 / 1380; 11008 x 4096:
-    # 741 / 856 and 1746 / 1678.
-    ROWS_MIN_M, ROWS_MAX_M = 129, 8192
+    # (11008 x 4096, group 128): 130 rows 24 us against 61 in two passes of the small-row kernel.
+    # Past 6144 rows a bf16 copy of W, written once, costs less than a tile of W de-quantised again for every 256 rows.  us, feed-forwards of
+    # widths 2048 / 4096 / 5120 (two layers in the gated form, one plain), this kernel and copies with their products: 2048 rows
+    # 128 / 474 / 748 and 137 / 527 / 854, 6000 rows 393 / 1367 / 2159 and 369 / 1409 / 2145, 8192 rows 531 / 1884 / 3098 and 504 / 1827 / 2882.
+    ROWS_MIN_M, ROWS_MAX_M = 129, 6144
 
     def _rows_eligible(self, x) -> bool:
         """More than 128 bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns."""
@@ -168,6 +166,10 @@ class ColBlockQuantizedLinear(torch.nn.Module):
                 and (self.bias is None or self.bias.dtype == torch.bfloat16) and s.is_contiguous() and z.is_contiguous()
                 and (self.quant_weight.data_ptr() | x.data_ptr()) % 16 == 0
                 and bool(N.call_ret("ll_int4_rows_supported", self.out_features, self.in_features, self.tile_cols)))
+
+    def _copy_eligible(self, x) -> bool:
+        """bf16 rows on a layer whose unpacked copy the dense kernel takes."""
+        return x.dtype == torch.bfloat16 and self.in_features % 8 == 0 and (self.bias is None or self.bias.dtype == torch.bfloat16)
 
     def _fused_gemm_eligible(self, x) -> bool:
         """9 <= M <= 128 bf16 rows on a layer whose scale groups are multiples of 128: the fused tcgen05 de-quantise + GEMM."""
@@ -247,6 +249,42 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         a.bias = 0 if self.bias is None else self.bias.data_ptr()
         a.epilogue, a.flags, a.grid = N.EPI_STORE, (N.GEMV_PDL if pdl else 0), grid
         N.gemv(a)
+
+
+def is_plain(m: torch.nn.Module, kind: type) -> bool:
+    """Whether calling ``m`` runs ``kind.forward`` and nothing else: no subclass, no forward set on the instance, no hooks.  Only then may a
+    kernel do the work of several layers without calling them."""
+    g = torch.nn.modules.module
+    return (type(m) is kind and "forward" not in m.__dict__ and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks
+            or m._backward_pre_hooks or g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks
+            or g._global_backward_pre_hooks))
+
+
+def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
+    """``silu(fc1(x)) * fc2(x)`` of two quantized layers of one size in one kernel, rounded as the separate ones round it; ``None``: this step
+    has no such kernel."""
+    if not (is_plain(fc1, ColBlockQuantizedLinear) and is_plain(fc2, ColBlockQuantizedLinear)):
+        return None
+    K, Nout = fc1.in_features, fc1.out_features
+    if (fc2.in_features, fc2.out_features, fc2.tile_cols) != (K, Nout, fc1.tile_cols) or inp.shape[-1] != K or inp.device.type != "cuda":
+        return None
+    x = inp.reshape(-1, K)
+    if not x.is_contiguous():
+        x = x.contiguous()
+    M = x.shape[0]
+    rows = ColBlockQuantizedLinear.ROWS_MIN_M <= M <= ColBlockQuantizedLinear.ROWS_MAX_M and fc1._rows_eligible(x) and fc2._rows_eligible(x)
+    if not rows and not (M > ColBlockQuantizedLinear.ROWS_MAX_M and all(f._copy_eligible(x) for f in (fc1, fc2))):
+        return None
+    h = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
+    if rows:
+        q1, q2 = fc1._packed_ptr_ok(), fc2._packed_ptr_ok()
+        N.require_cuda(q1, q2)
+        N.call("ll_int4_rows_gated", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
+               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), M, Nout, K, fc1.tile_cols, 0, 0, N.stream())
+    else:
+        w1, w2 = fc1.get_weight(dtype=x.dtype), fc2.get_weight(dtype=x.dtype)
+        N.call("ll_gemm_bf16_gated", N.ptr(x), N.ptr(w1), N.ptr(fc1.bias), N.ptr(w2), N.ptr(fc2.bias), N.ptr(h), M, Nout, K, N.stream())
+    return h.view(inp.shape[:-1] + (Nout,))
 
 
 def dequant_gemm(lin: ColBlockQuantizedLinear, x: torch.Tensor) -> torch.Tensor:
