@@ -214,6 +214,16 @@ LL_API int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const voi
                               const void* scales2, const void* zeros2, const void* bias2, const void* x, void* h, int M, int N, int K, int group,
                               int tile_rows, int grid, ll_stream stream);
 LL_API int ll_int4_rows_error(void);
+/* Batches of 1 to 128 rows from the same checkpoint bytes: y = x . W^T (+ bias), or, of two layers that read the same x, the gated product as
+ * ll_int4_rows_gated rounds it.  Sizes as for ll_int4_rows; scratch: ll_int4_batch_scratch_bytes (layers: 1, or 2 for the gated form) on a
+ * 16-byte boundary, of any contents; grid: ranges that the work is cut into at most (0: one an SM). */
+LL_API size_t ll_int4_batch_scratch_bytes(int M, int N, int K, int layers, int grid);
+LL_API int ll_int4_batch(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch, int M,
+                         int N, int K, int group, int grid, ll_stream stream);
+LL_API int ll_int4_batch_gated(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2,
+                               const void* scales2, const void* zeros2, const void* bias2, const void* x, void* h, void* scratch, int M, int N,
+                               int K, int group, int grid, ll_stream stream);
+LL_API int ll_int4_batch_error(void);
 /* Fused int4 de-quantise + GEMM on tcgen05 for 1 <= M <= 128 rows (batched decode, short prefill; the HBM-bound regime):
  * y[M][N] (bf16) = x[M][K] (bf16) . W^T (+ bias), W de-quantised INSIDE the main loop from the packed stream
  * (w_stream = ll_int4_prepare(..., LL_STREAM_U8, ...), the batch-1 GEMV's stream) with the reference's bf16 rounding steps

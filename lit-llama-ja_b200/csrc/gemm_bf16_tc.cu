@@ -261,6 +261,8 @@ int launch_pair(const void* x, const void* w0, const void* w1, const void* b0, c
 }
 
 // ==================================================================================== fused int4 dequant-GEMM, M <= 128
+// (The layers of this package run int4_batch.cu; this kernel takes the packed stream of callers that hold nothing else, and layers whose
+// checkpoint bytes that one does not take.)
 // y[M][N] = x[M][K] . dequant(W)^T for 9 <= M <= 128 (batched decode, short prefill): the regime where the weights are
 // the traffic (HBM-bound), so they are streamed ONCE in their packed form and de-quantised inside the main loop - what the
 // reference's Triton kernel does (ref quantization.py:259-267: load nibble, (q - zero) * scale, tl.dot) - instead of

@@ -23,14 +23,13 @@
 // accumulator back as soon as it is in registers, so that the tensor cores wait for the drain alone.
 // Every wait is bounded; one that runs out records a code, all roles of both CTAs stop, copies in flight are waited for, tensor memory is
 // freed.
-#include "tcgen05.cuh"
+#include "int4_unpack.cuh"
 
 namespace llb {
 namespace {
 
-constexpr int R4_K = 128, R4_GROUPS = 4, R4_THREADS = (4 + 4 * R4_GROUPS) * 32;
-constexpr int R4_WBYTES = 128 * R4_K / 2, R4_WST = 6;                  // stages of packed bytes
-constexpr int R4_SZ = 128 * 8 + 16;                                    // their columns' scales and zeros, and a word per 32 columns: all zeros whole
+constexpr int R4_GROUPS = 4, R4_THREADS = (4 + 4 * R4_GROUPS) * 32;
+constexpr int R4_WST = 6;                                              // stages of packed bytes
 constexpr int R4_XBYTES = 128 * 1024, R4_XST = 8;                      // the ring of x: as many stages of two halves [bn / 2 rows][64 k] as fit
 constexpr int R4_BOX = 16 * 64, R4_OUT = 2 * R4_BOX;                   // a warp stores 16 rows of 32 columns at a time, from two places in turn
 constexpr int R4_SWAP = 64 * 16 * 4;                                   // gated form: what a group hands over at a time, 64 columns x 32 rows of bf16
@@ -77,11 +76,6 @@ __device__ __forceinline__ bool r4_spin(uint64_t* bar, uint32_t parity, const R4
   r4_give_up(f, code);
   return false;
 }
-__device__ __forceinline__ void r4_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
-               "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-               : "memory");
-}
 __device__ __forceinline__ void r4_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -90,71 +84,6 @@ __device__ __forceinline__ void r4_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void r4_ld16(uint32_t taddr, uint32_t* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                 "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-               : "r"(taddr)
-               : "memory");
-}
-// 32 k-pairs x 16 columns of packed bytes, four bytes of a column's k-pairs in a word: r[0], r[1] (r[2], r[3]: the next 16 k-pairs) hold
-// columns lane / 4 and lane / 4 + 8 and the k-pairs whose rows the lanes 4 (lane % 4) .. + 3 point at
-__device__ __forceinline__ void r4_ldt(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(addr)
-               : "memory");
-}
-// 16 lanes x 32 columns of tensor memory: of every 8 columns a thread writes columns 2 (lane % 4), + 1 of lanes lane / 4 and lane / 4 + 8
-__device__ __forceinline__ void r4_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(r[0]),
-      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
-      "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ uint32_t r4_prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
-}
-__device__ __forceinline__ uint32_t r4_sub2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t r4_mul2(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-
-// four bytes of a column -> the bf16 pairs of their k: (128 + q) - (128 + zero), exact for a whole zero; FRACTION: minus 128, minus zr (which is
-// 0 in columns whose zero is whole), each rounded as the reference does; times the scale
-template <bool FRACTION>
-__device__ __forceinline__ void r4_unpack(uint32_t w, uint32_t s2, uint32_t zc2, uint32_t zr2, uint32_t& o0, uint32_t& o1, uint32_t& o2, uint32_t& o3) {
-  const uint32_t lo = w & 0x0f0f0f0fu, hi = (w >> 4) & 0x0f0f0f0fu;
-  const uint32_t p = r4_prmt(lo, hi, 0x5140), q = r4_prmt(lo, hi, 0x7362);
-  uint32_t v[4] = {r4_prmt(p, 0x43u, 0x4140), r4_prmt(p, 0x43u, 0x4342), r4_prmt(q, 0x43u, 0x4140), r4_prmt(q, 0x43u, 0x4342)};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[i] = r4_sub2(v[i], zc2);
-    if (FRACTION) v[i] = r4_sub2(v[i], zr2);
-    v[i] = r4_mul2(v[i], s2);
-  }
-  o0 = v[0], o1 = v[1], o2 = v[2], o3 = v[3];
-}
-// what r4_ldt brought, as r4_st16 stores it; n: the numbers of columns lane / 4 and lane / 4 + 8
-template <bool FRACTION>
-__device__ __forceinline__ void r4_unpack16(const uint32_t (&w)[4], const uint2 (&n)[2], uint32_t (&r)[16]) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const uint2 v = n[i & 1];
-    const int o = (i >> 1) * 8 + (i & 1) * 2;
-    r4_unpack<FRACTION>(w[i], r4_prmt(v.x, 0u, 0x1010), r4_prmt(v.x, 0u, 0x3232), v.y, r[o], r[o + 1], r[o + 4], r[o + 5]);
-  }
-}
-
 template <bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
     int4_rows_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_x,
@@ -164,10 +93,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
   uint8_t* sx = base;                                  // [xst][2][bn / 2][64] bf16, swizzled
-  uint8_t* sw = base + R4_XBYTES;                      // [WST][2][64][64] packed bytes: two boxes of 64 columns, swizzled
+  uint8_t* sw = base + R4_XBYTES;                      // [WST][64][128] packed bytes (gated: [2][64][64]), swizzled
   uint8_t* so = sw + R4_WST * R4_WBYTES;               // [16 warps][2][16 rows][32 columns] bf16, swizzled
   uint8_t* swap = so + 8 * R4_OUT;                     // gated form: [GROUPS][16 pairs of rows][64 columns]
-  uint8_t* sz = so + 4 * R4_GROUPS * R4_OUT;           // [WST][128] (scale | magic number of the zero << 16, rest), [4] whole
+  uint8_t* sz = so + 4 * R4_GROUPS * R4_OUT;           // [WST][128] scale | zero << 16
   uint64_t* x_full = reinterpret_cast<uint64_t*>(sz + R4_WST * R4_SZ);               // used in rank 0
   uint64_t* x_empty = x_full + R4_XST;
   uint64_t* w_full = x_empty + R4_XST;
@@ -224,12 +153,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
             if (++s == xst) s = 0, ph ^= 1u;
           }
         } else {
-          const int c0 = n0 + rank * (TILE_N / 2), c1 = GATED ? c0 : c0 + 64;
+          const int c0 = n0 + rank * (TILE_N / 2);
           for (int kb = 0; kb < steps; ++kb) {
             if (!(ok = r4_wait(&w_empty[s], ph, fail, 2))) break;
             mbar_expect_tx(&w_full[s], R4_WBYTES);
             r4_box(sw + s * R4_WBYTES, &map_w0, c0, kb * (R4_K / 2), &w_full[s]);
-            r4_box(sw + s * R4_WBYTES + R4_WBYTES / 2, GATED ? &map_w1 : &map_w0, c1, kb * (R4_K / 2), &w_full[s]);
+            if (GATED) r4_box(sw + s * R4_WBYTES + R4_WBYTES / 2, &map_w1, c0, kb * (R4_K / 2), &w_full[s]);
             if (++s == R4_WST) s = 0, ph ^= 1u;
           }
         }
@@ -262,22 +191,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
       if (!ok) let_issued_work_end();
     }
   } else if (warp == 3) {
-    // scales and zeros, four steps ahead of their use at least: the groups of four steps lie side by side.  A column's numbers as the unpacking
-    // threads want them: its scale, and 128 + zero for one exact subtraction if the zero is whole (every RTN / GPTQ checkpoint), else 128 and
-    // the zero.  (Loaded by those threads one step ahead, 64 lines a warp and no L1 to speak of, they were half of a step's time.)
+    // scales and zeros, four steps ahead of their use at least: the groups of four steps lie side by side.  (Loaded by the unpacking threads one
+    // step ahead, 64 lines a warp and no L1 to speak of, they were half of a step's time.)
     bool ok = true;
     int s = 0;
     uint32_t ph = 1;
-    auto four = [&](const __nv_bfloat16* src, size_t row, int kb) {      // the numbers of steps kb .. kb + 3, in one load where rows allow it
-      const uint16_t* at = reinterpret_cast<const uint16_t*>(src) + row;
-      if (p.wide == 4) return *reinterpret_cast<const uint2*>(at + kb);
-      if (p.wide == 2)
-        return make_uint2(*reinterpret_cast<const uint32_t*>(at + kb), *reinterpret_cast<const uint32_t*>(at + min(kb + 2, p.G - 2)));
-      uint32_t v[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) v[j] = at[min(kb + j, steps - 1) / p.steps_per_group];
-      return make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
-    };
     auto fetch = [&](int tile, int kb, uint2 (&sv)[4], uint2 (&zv)[4]) {
       const int n0 = (tile / p.mtiles) * TILE_N;
 #pragma unroll
@@ -285,8 +203,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
         const bool second = GATED && q >= 2;
         const int n = n0 + (GATED ? rank * 64 + (q & 1) * 32 : rank * 128 + q * 32) + lane;
         const size_t row = (size_t)min(n, p.N - 1) * p.G;
-        sv[q] = four(second ? p.scales[1] : p.scales[0], row, kb);
-        zv[q] = four(second ? p.zeros[1] : p.zeros[0], row, kb);
+        sv[q] = r4_four(second ? p.scales[1] : p.scales[0], row, kb, steps, p.G, p.steps_per_group, p.wide);
+        zv[q] = r4_four(second ? p.zeros[1] : p.zeros[0], row, kb, steps, p.G, p.steps_per_group, p.wide);
       }
     };
     uint2 sv[4], zv[4];
@@ -301,16 +219,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
           if (kb + j >= steps) break;
           ok = __all_sync(0xffffffffu, r4_wait(&w_empty[s], ph, fail, 11));
           if (!ok) break;
-          uint2* dst = reinterpret_cast<uint2*>(sz + s * R4_SZ);
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t sc = ((j < 2 ? sv[q].x : sv[q].y) >> (16 * (j & 1))) & 0xffffu, ze = ((j < 2 ? zv[q].x : zv[q].y) >> (16 * (j & 1))) & 0xffffu;
-            const float zf = __uint_as_float(ze << 16);
-            const bool whole = zf == floorf(zf) && zf >= 0.f && zf <= 64.f;
-            dst[q * 32 + lane] = make_uint2(sc | ((whole ? 0x4300u + (uint32_t)zf : 0x4300u) << 16), whole ? 0u : ze * 0x00010001u);
-            const bool all = __all_sync(0xffffffffu, whole);
-            if (lane == 0) reinterpret_cast<uint32_t*>(dst + 128)[q] = all ? 1u : 0u;
-          }
+          for (int q = 0; q < 4; ++q) reinterpret_cast<uint32_t*>(sz + s * R4_SZ)[q * 32 + lane] = r4_word(j, sv[q], zv[q]);
           __syncwarp();
           if (lane == 0) mbar_arrive(&w_full[s]);
           if (++s == R4_WST) s = 0, ph ^= 1u;
@@ -415,10 +325,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
     int tile = pair, kb = grp, drained = pair, s = grp;
     uint32_t nth = 0, round = 0, wph = 0;    // round: the group's how-many-th step
     while (kb >= steps && tile < p.tiles) kb -= steps, tile += pairs;
-    // the row of packed bytes (64 of them, 16-byte pieces swizzled) a lane points at: of 16 k-pairs, four lanes name those of which the threads
-    // of one lane % 4 write two and two tensor-memory columns
-    const int li = lane & 15, krow = (lane >> 4) * 16 + (li >> 2) * 2 + (li & 1) + (li & 2) * 4;
-    const uint32_t row_at = (uint32_t)(krow * 64), turn = (uint32_t)(((krow >> 1) & 3) * 16);
+    constexpr int WIDTH = GATED ? 64 : 128;
+    const R4Row<WIDTH> row(lane);
     while (ok && drained < p.tiles) {
       const int upto = min(tile, p.tiles);   // tiles before this one can be drained
       bool step = tile < p.tiles;
@@ -431,21 +339,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
       }
       if (step) {
         tc_fence_after();
-        const uint32_t src = smem_u32(sw + s * R4_WBYTES + half * (R4_WBYTES / 2)) + row_at;
-        const uint32_t ta = tmem + lanes + TM_A + 64u * grp, nums = smem_u32(sz + s * R4_SZ) + (uint32_t)((quarter * 32 + (lane >> 2)) * 8);
-        const bool whole = reinterpret_cast<const uint32_t*>(sz + s * R4_SZ + 128 * 8)[quarter] != 0u;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {        // 16 of the warp's 32 columns
-          const uint2 n[2] = {lds64(nums + h * 128), lds64(nums + h * 128 + 64)};
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {      // 32 of the step's 64 k-pairs
-            uint32_t w[4], r[16];
-            r4_ldt(src + ((uint32_t)((quarter & 1) * 32 + h * 16) ^ turn) + (uint32_t)(c * 32 * 64), w);
-            if (whole) r4_unpack16<false>(w, n, r);
-            else r4_unpack16<true>(w, n, r);
-            r4_st16(ta + ((uint32_t)(16 * h) << 16) + 32u * c, r);
-          }
-        }
+        r4_unpack_step<WIDTH>(smem_u32(sw + s * R4_WBYTES + (GATED ? half * (R4_WBYTES / 2) : 0)), (uint32_t)((GATED ? quarter & 1 : quarter) * 32), row,
+                              smem_u32(sz + s * R4_SZ) + (uint32_t)(quarter * 128), tmem + lanes + TM_A + 64u * grp);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         tc_fence_before();
         __syncwarp();
@@ -469,24 +364,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
     tc_fence_after();
     pair_tmem_dealloc(tmem, 512);
   }
-}
-
-// packed bytes [K/2][N] as a 2-D map, boxes of 64 columns x 64 rows
-int r4_weight_map(const void* qw, int N, int K, CUtensorMap* out) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) {
-    set_error("cuTensorMapEncodeTiled entry point not available");
-    return LL_ERR_CUDA;
-  }
-  cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)(K / 2)}, strides[1] = {(cuuint64_t)N};
-  cuuint32_t box[2] = {64, R4_K / 2}, estr[2] = {1, 1};
-  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)qw, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed (%d): packed weights N=%d K=%d", (int)r, N, K);
-    return LL_ERR_CUDA;
-  }
-  return LL_OK;
 }
 
 // the output, boxes of 16 rows x 32 columns
@@ -527,12 +404,10 @@ int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p,
       if (r4_cost(p.M, p.N, TILE_N, p.steps, bn, pairs) < r4_cost(p.M, p.N, TILE_N, p.steps, p.bn, pairs)) p.bn = bn;
   }
   p.xst = R4_XBYTES / (p.bn * 128);
-  // steps whose scales (and zeros) one load takes: a row of groups of 128 starts on its boundary, and no load passes a row's end
-  const uintptr_t at = (uintptr_t)p.scales[0] | (uintptr_t)p.scales[1] | (uintptr_t)p.zeros[0] | (uintptr_t)p.zeros[1];
-  p.wide = p.steps_per_group != 1 ? 1 : p.G % 4 == 0 && at % 8 == 0 ? 4 : p.G % 2 == 0 && at % 4 == 0 ? 2 : 1;
+  p.wide = r4_wide(p.scales[0], p.zeros[0], p.scales[1], p.zeros[1], p.G, p.steps_per_group);
   CUtensorMap mw0, mw1, mx, my;
-  if (int r = r4_weight_map(qw0, p.N, K, &mw0)) return r;
-  if (int r = r4_weight_map(qw1, p.N, K, &mw1)) return r;
+  if (int r = r4_weight_map(qw0, p.N, K, GATED ? 64 : 128, &mw0)) return r;
+  if (int r = r4_weight_map(qw1, p.N, K, GATED ? 64 : 128, &mw1)) return r;
   if (int r = make_map(x, p.M, K, p.bn / 2, &mx)) return r;
   if (int r = r4_out_map(p.y, p.M, p.N, &my)) return r;
   static PerDevice configured;

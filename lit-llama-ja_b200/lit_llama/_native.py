@@ -90,6 +90,10 @@ EXPORTS = {
     "ll_int4_rows_form": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_gated": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_error": ([], C.c_int),
+    "ll_int4_batch_scratch_bytes": ([i32, i32, i32, i32, i32], sz_t),
+    "ll_int4_batch": ([vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp], C.c_int),
+    "ll_int4_batch_gated": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp], C.c_int),
+    "ll_int4_batch_error": ([], C.c_int),
     "ll_int4_gemm_tc_scratch_bytes": ([i32, i32, i32], sz_t),
     "ll_int4_gemm_tc": ([vp, vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_gemm_tc_static": ([vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),

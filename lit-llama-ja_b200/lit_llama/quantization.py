@@ -7,6 +7,7 @@ strides, state-dict keys, constructor protocol) so GPTQ checkpoints written by t
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
@@ -18,6 +19,24 @@ def _entries_per_byte(bits: int) -> int:
     epb = 8 // bits
     assert epb > 0 and epb * bits == 8, f"bits must be 1, 2, 4 or 8, got {bits}"
     return epb
+
+
+# What the library says of sizes alone: asked once for each, not on every call.
+@functools.lru_cache(maxsize=4096)
+def _rows_supported(Nout: int, K: int, group: int) -> bool:
+    return bool(N.call_ret("ll_int4_rows_supported", Nout, K, group))
+
+
+@functools.lru_cache(maxsize=4096)
+def _batch_scratch_bytes(M: int, Nout: int, K: int, layers: int) -> int:
+    return N.call_ret("ll_int4_batch_scratch_bytes", M, Nout, K, layers, 0)
+
+
+@functools.lru_cache(maxsize=4096)
+def _gemv_supported(bits: int, Nout: int, K: int, group: int, nmat: int, M: int) -> bool:
+    if bits == 8:
+        return bool(N.call_ret("ll_q8_gemv_supported", Nout, K, group, nmat, M))
+    return bits == 4 and N.gemv_supported(Nout, K, group, nmat, M)
 
 
 class ColBlockQuantizedLinear(torch.nn.Module):
@@ -107,9 +126,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
     def gemv_ok(self, M: int, nmat: int = 1) -> bool:
         """The tensor-core GEMV takes this layer at batch ``M`` (4-bit: M <= 8; 8-bit weights: batch 1)."""
-        if self.bits == 8:
-            return bool(N.call_ret("ll_q8_gemv_supported", self.out_features, self.in_features, self.tile_cols, nmat, M))
-        return self.bits == 4 and N.gemv_supported(self.out_features, self.in_features, self.tile_cols, nmat, M)
+        return _gemv_supported(self.bits, self.out_features, self.in_features, self.tile_cols, nmat, M)
 
     def _kind(self, M: int) -> int:
         return N.STREAM_W8 if self.bits == 8 else N.stream_kind(self.out_features, self.in_features, self.tile_cols, M)
@@ -151,7 +168,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         self._streams[kind] = (self._state_key(), buf, ok)
         return buf if ok else None
 
-    FUSED_GEMM_MAX_M = 128       # rows one ll_int4_gemm_tc call takes
+    FUSED_GEMM_MAX_M = 128       # rows one ll_int4_batch (or ll_int4_gemm_tc) call takes
     # rows from which the weights are de-quantised in the main loop of the many-row kernel, from the checkpoint bytes.  Both sides measured
     # (11008 x 4096, group 128): 130 rows 24 us against 61 in two passes of the small-row kernel.
     # Past 6144 rows a bf16 copy of W, written once, costs less than a tile of W de-quantised again for every 256 rows.  us, feed-forwards of
@@ -160,12 +177,12 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     ROWS_MIN_M, ROWS_MAX_M = 129, 6144
 
     def _rows_eligible(self, x) -> bool:
-        """More than 128 bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns."""
-        s, z = self.scales, self.zeros
-        return (self.bits == 4 and x.dtype == torch.bfloat16 and s.dtype == torch.bfloat16 and z.dtype == torch.bfloat16
-                and (self.bias is None or self.bias.dtype == torch.bfloat16) and s.is_contiguous() and z.is_contiguous()
-                and (self.quant_weight.data_ptr() | x.data_ptr()) % 16 == 0
-                and bool(N.call_ret("ll_int4_rows_supported", self.out_features, self.in_features, self.tile_cols)))
+        """bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns: the kernels that read the checkpoint bytes."""
+        b = self._buffers
+        s, z, bias = b["scales"], b["zeros"], b["bias"]
+        return (self.bits == 4 and x.dtype == s.dtype == z.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)
+                and s.is_contiguous() and z.is_contiguous() and (b["quant_weight"].data_ptr() | x.data_ptr()) % 16 == 0
+                and _rows_supported(self.out_features, self.in_features, self.tile_cols))
 
     def _copy_eligible(self, x) -> bool:
         """bf16 rows on a layer whose unpacked copy the dense kernel takes."""
@@ -207,6 +224,13 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             fast = self.prepare(M) is not None
         if fast:
             self._gemv(x, y)
+        elif M <= self.FUSED_GEMM_MAX_M and self._rows_eligible(x):
+            # the stream that single-token steps read is made here once, with a generation's prompt or first batch, not with its next token
+            if M > 8 and N.STREAM_U8 not in self._streams and self._fused_gemm_eligible(x) and not torch.cuda.is_current_stream_capturing():
+                self._prepare_kind(N.STREAM_U8)
+            scratch = _int8_workspace(x.device, _batch_scratch_bytes(M, Nout, K, 1))
+            N.call("ll_int4_batch", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), N.ptr(scratch), M, Nout, K,
+                   self.tile_cols, 0, N.stream())
         elif M <= self.FUSED_GEMM_MAX_M and self._fused_gemm_eligible(x) and self._fused_gemm(x, y):
             pass
         elif self.ROWS_MIN_M <= M <= self.ROWS_MAX_M and self._rows_eligible(x):
@@ -241,6 +265,9 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         return True
 
     def _gemv(self, x, y, *, pdl=False, grid=0):
+        N.gemv(self._gemv_args(x, y, pdl=pdl, grid=grid))
+
+    def _gemv_args(self, x, y, *, pdl=False, grid=0):
         a = N.GemvArgs()
         w, a.stream_kind = self.stream_for(x.shape[0])
         a.w = w.data_ptr()
@@ -248,7 +275,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         a.x, a.y = x.data_ptr(), y.data_ptr()
         a.bias = 0 if self.bias is None else self.bias.data_ptr()
         a.epilogue, a.flags, a.grid = N.EPI_STORE, (N.GEMV_PDL if pdl else 0), grid
-        N.gemv(a)
+        return a
 
 
 def is_plain(m: torch.nn.Module, kind: type) -> bool:
@@ -272,6 +299,31 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
     if not x.is_contiguous():
         x = x.contiguous()
     M = x.shape[0]
+    if M == 0:
+        return None
+    if x.dtype == torch.bfloat16 and M <= 8 and fc1.bits == fc2.bits == 4 and fc1.bias is None and fc2.bias is None:
+        # few rows: both layers and their product are an epilogue of the GEMV, whose weight streams are made outside a capture
+        if fc1.gemv_ok(M, 2) and (fc1.gemv_ok(M) and fc2.gemv_ok(M)):
+            if torch.cuda.is_current_stream_capturing():
+                streams = fc1.stream_for(M)[0] is not None and fc2.stream_for(M)[0] is not None
+            else:
+                streams = fc1.prepare(M) is not None and fc2.prepare(M) is not None
+            if streams:
+                h = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
+                a = fc1._gemv_args(x, h)
+                a.w2, a.epilogue = fc2.stream_for(M)[0].data_ptr(), N.EPI_SWIGLU
+                N.gemv(a)
+                return h.view(inp.shape[:-1] + (Nout,))
+    if M <= ColBlockQuantizedLinear.FUSED_GEMM_MAX_M:
+        if M <= 8 and fc1.gemv_ok(M) or not (fc1._rows_eligible(x) and fc2._rows_eligible(x)):
+            return None
+        q1, q2 = fc1._packed_ptr_ok(), fc2._packed_ptr_ok()
+        N.require_cuda(q1, q2)
+        h = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
+        scratch = _int8_workspace(x.device, _batch_scratch_bytes(M, Nout, K, 2))
+        N.call("ll_int4_batch_gated", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
+               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), N.ptr(scratch), M, Nout, K, fc1.tile_cols, 0, N.stream())
+        return h.view(inp.shape[:-1] + (Nout,))
     rows = ColBlockQuantizedLinear.ROWS_MIN_M <= M <= ColBlockQuantizedLinear.ROWS_MAX_M and fc1._rows_eligible(x) and fc2._rows_eligible(x)
     if not rows and not (M > ColBlockQuantizedLinear.ROWS_MAX_M and all(f._copy_eligible(x) for f in (fc1, fc2))):
         return None
