@@ -45,7 +45,8 @@ typedef void* ll_stream; /* cudaStream_t */
 
 LL_API const char* ll_last_error(void);
 /* The waits inside the tcgen05 kernels and the chunked delta rule are bounded; a kernel whose wait runs out skips its stores and leaves a
- * code in host memory (100 + prompt attention's, 200 + int4 rows', 300 + llm.int8's, 400 + grouped experts', 500 + delta rule's).
+ * code in host memory (100 + prompt attention's, 200 + int4 rows', 300 + llm.int8's, 400 + grouped experts', 500 + delta rule's,
+ * 600 + dense products').
  * The next launch through this library fails with LL_ERR_WAIT, or this call does, which looks without launching: after a synchronisation
  * it speaks for everything before it.  Either clears the code.  ll_wait_report leaves a code as a kernel does. */
 LL_API int ll_wait_check(void);
@@ -261,6 +262,12 @@ LL_API int ll_int8_quantize_weight(const void* w /*[N][K]*/, int w_dtype, int8_t
  * activation dtype.  K % 128 == 0.  workspace: ll_int8_workspace_bytes(M, N, K) bytes, 256-byte aligned; with those of min(M, 64) rows
  * M > 64 runs as passes of 64 rows (the same results: a feature is an outlier for a block of 64 rows). */
 LL_API size_t ll_int8_workspace_bytes(int M, int N, int K);
+/* Two layers that read the same bf16 x, and their gated product: h[M][N] = silu(x . W1^T (+ bias1)) * (x . W2^T (+ bias2)), every step rounded
+ * as ll_int8_linear twice and ll_silu_mul round it; x is prepared once. */
+LL_API size_t ll_int8_gated_workspace_bytes(int M, int N, int K);
+LL_API int ll_int8_gated(const void* x, const int8_t* cb1, const int8_t* cbt1, const float* scb1, const void* bias1, const int8_t* cb2,
+                         const int8_t* cbt2, const float* scb2, const void* bias2, void* h, int M, int N, int K, float threshold,
+                         void* workspace, size_t workspace_bytes, ll_stream stream);
 /* 0, or the code of the first bounded wait that ran out in the tcgen05 product of ll_int8_linear (M > 64).  Synchronises the device. */
 LL_API int ll_int8_tc_error(void);
 /* cbt: CB transposed, int8 [K][N] (optional, NULL = none): with it an outlier column of the weights is one contiguous row

@@ -10,8 +10,9 @@
 // Up to 64 rows: HBM-bound on the int8 weight read (N*K bytes per layer).  One kernel prepares the activations (row maxima, outlier list,
 // quantised rows), one streams the weights as the A operand of tcgen05 kind::i8 MMAs (128 output columns = the 128 TMEM lanes, int32
 // accumulators) with K cut into ranges whose partial sums are stored, one adds them up (integers: exact in any order) and finishes.
-// Prompts (M > 64): the same arithmetic per block of 64 rows (a feature is an outlier for a block of 64 rows), all blocks at once: row
-// statistics, quantised rows, outlier lists, then one 128 x 128-tiled product and one finishing kernel.  See int8_gemm_tc_kernel.
+// Prompts (M > 64): the same arithmetic per block of 64 rows (a feature is an outlier for a block of 64 rows), all blocks at once: the same
+// preparation, then one kernel for the product and its finish (int8_pair_kernel).
+// Either way the two layers of a gated feed-forward that read the same x go together: x is prepared once, one product over both, one finish.
 #include "tcgen05.cuh"
 
 namespace llb {
@@ -66,96 +67,7 @@ template <typename T> __device__ __forceinline__ void int8_load8(const T* p, flo
   }
 }
 
-// ================================================================================================== prompts: M > 64
-// x.half() without storing it: sca[m] = absmax over the entries of row m below thr; flag[block of 64 rows][k] = 1 where any
-// |entry| >= thr.  One CTA per row.
-template <typename T>
-__global__ void __launch_bounds__(256) int8_row_stats_kernel(const T* __restrict__ x, uint8_t* __restrict__ flag, float* __restrict__ sca, int K,
-                                                            float thr, int vec) {
-  __shared__ float red[8];
-  const int m = blockIdx.x;
-  const T* row = x + (size_t)m * K;
-  uint8_t* fl = flag + (size_t)(m / 64) * K;
-  float mx = 0.f;
-  for (int k = threadIdx.x * 8; k < K; k += 256 * 8) {      // (K is a multiple of 128)
-    float v[8];
-    int8_load8<T>(row + k, v, vec);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float a = fabsf(v[e]);
-      if (a >= thr) fl[k + e] = 1;
-      else mx = fmaxf(mx, a);
-    }
-  }
-  mx = warp_max(mx);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, red[w]);
-    sca[m] = mx;
-  }
-}
-
-// CA[m][k], eight entries per thread
-template <typename T>
-__global__ void __launch_bounds__(256) int8_row_quant_kernel(const T* __restrict__ x, const uint8_t* __restrict__ flag, const float* __restrict__ sca,
-                                                            int8_t* __restrict__ ca, int K, float thr, long long pieces, int vec) {
-  const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (i >= pieces) return;
-  const int per = K / 8, m = (int)(i / per), k = (int)(i - (long long)m * per) * 8;
-  float v[8];
-  int8_load8<T>(x + (size_t)m * K + k, v, vec);
-  const uint2 f = *reinterpret_cast<const uint2*>(flag + (size_t)(m / 64) * K + k);
-  const float s = sca[m], inv = __fdiv_rn(127.f, s == 0.f ? 1.f : s);
-  uint32_t o[2] = {0u, 0u};
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const uint32_t out = ((e < 4 ? f.x : f.y) >> (8 * (e & 3))) & 0xffu;
-    float q = 0.f;
-    if (out == 0u && fabsf(v[e]) < thr) q = fminf(fmaxf(rintf(__fmul_rn(v[e], inv)), -127.f), 127.f);
-    o[e >> 2] |= ((uint32_t)(int)q & 0xffu) << (8 * (e & 3));
-  }
-  *reinterpret_cast<uint2*>(ca + (size_t)m * K + k) = make_uint2(o[0], o[1]);
-}
-
-// ascending outlier list of every block of 64 rows; one CTA per block
-__global__ void __launch_bounds__(1024) int8_lists_kernel(const uint8_t* __restrict__ flag, int32_t* __restrict__ idx, int32_t* __restrict__ count, int K) {
-  __shared__ int s_warp[32];
-  const uint8_t* fl = flag + (size_t)blockIdx.x * K;
-  int32_t* list = idx + (size_t)blockIdx.x * K;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int base = 0;
-  for (int k0 = 0; k0 < K; k0 += 4096) {             // a thread looks at four neighbouring columns
-    const int k = k0 + threadIdx.x * 4;
-    const uint32_t f = k < K ? *reinterpret_cast<const uint32_t*>(fl + k) : 0u;
-    const int n = __popc(f);
-    int incl = n;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, d);
-      if (lane >= d) incl += v;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    int at = base + incl - n, total = 0;
-    for (int w = 0; w < 32; ++w) {
-      if (w < warp) at += s_warp[w];
-      total += s_warp[w];
-    }
-    for (int e = 0; e < 4; ++e)
-      if ((f >> (8 * e)) & 1u) list[at++] = k + e;
-    base += total;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) count[blockIdx.x] = base;
-}
-
-// C32[M][N] = CA[M][K] . CB[N][K]^T on tcgen05 (kind::i8, K = 32 an instruction).  A CTA owns 128 x 128 outputs: TMA producer, one issuing
-// thread, four epilogue warps; tiles of 128 x 128 bytes in a ring of three, so that two CTAs share an SM (one's first loads and epilogue run
-// under the other's products).  A 7B feed-forward of 512 rows: 24 passes of 64 rows through mma.sync, four kernels each, took 1435 us on the
-// device (the weights read eight times, the accumulator added up by atomics); three products of 40 us and 28 us around each make 211 us.
-// Every wait is bounded; one that runs out records a code, the roles stop and tensor memory is freed.
-constexpr int I8_BN = 128, I8_STAGES = 3, I8_BOX = 128 * 128;
+constexpr int I8_BOX = 128 * 128;
 constexpr uint32_t I8_WAIT_LIMIT = 1u << 20;
 __device__ int g_int8_tc_error = 0;
 
@@ -183,212 +95,145 @@ __device__ __forceinline__ void i8_box(void* dst, const CUtensorMap* map, int x,
                : "memory");
 }
 
-__global__ void __launch_bounds__(192, 2) int8_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                                             int32_t* __restrict__ c, int M, int N, int K, int* word) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
-  uint8_t *sa = base, *sb = base + I8_STAGES * I8_BOX;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sb + I8_STAGES * I8_BOX);
-  uint64_t* empty = full + I8_STAGES;
-  uint64_t* done = empty + I8_STAGES;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done + 1);
-  int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
-  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * I8_BN, nkb = K / 128;      // (x runs over the rows: CTAs side by side share weights)
-  if (threadIdx.x == 0) {
-    prefetch_tensormap(&map_a);
-    prefetch_tensormap(&map_b);
-    for (int i = 0; i < I8_STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
-    mbar_init(done, 1);
-    *s_fail = 0;
-    fence_barrier_init();
-  }
-  if (warp == 1) tmem_alloc(tmem_ptr, I8_BN);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
-  if (warp == 0) {
-    if (elect_one()) {
-      bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % I8_STAGES;
-        if (!(ok = i8_wait(&empty[s], ((kb / I8_STAGES) & 1) ^ 1, s_fail, word, 1))) break;
-        mbar_expect_tx(&full[s], 2 * I8_BOX);
-        i8_box(sa + s * I8_BOX, &map_a, kb * 128, m0, &full[s]);
-        i8_box(sb + s * I8_BOX, &map_b, kb * 128, n0, &full[s]);
-      }
-      if (!ok) let_issued_work_end();
-    }
-  } else if (warp == 1) {
-    if (elect_one()) {
-      // D = int32 (2 at bit 4), A = B = signed int8 (1 at bits 7 and 10), both K-major
-      constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-      const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
-      bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % I8_STAGES;
-        if (!(ok = i8_wait(&full[s], (kb / I8_STAGES) & 1, s_fail, word, 2))) break;
-        tc_fence_after();
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          umma_i8(tmem, ad + (uint64_t)(s * (I8_BOX >> 4) + 2 * k), bd + (uint64_t)(s * (I8_BOX >> 4) + 2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-        umma_commit(&empty[s]);
-      }
-      umma_commit(done);             // also after a failure: the epilogue's wait ends
-      if (!ok) let_issued_work_end();
-    }
-  } else {
-    const int quarter = warp & 3, m = m0 + quarter * 32 + lane;
-    const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, word, 3) && *(volatile int*)s_fail == 0);
-    tc_fence_after();
-    if (ok) {
-#pragma unroll 1
-      for (int c0 = 0; c0 < I8_BN; c0 += 32) {
-        if (n0 + c0 >= N) break;
-        uint32_t v[32];
-        tmem_ld_32x32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-        if (m < M) {
-          int32_t* dst = c + (size_t)m * N + n0 + c0;
-          if (n0 + c0 + 32 <= N && (N & 3) == 0) {
-#pragma unroll
-            for (int e = 0; e < 32; e += 4)
-              *reinterpret_cast<int4*>(dst + e) = make_int4((int)v[e], (int)v[e + 1], (int)v[e + 2], (int)v[e + 3]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (n0 + c0 + e < N) dst[e] = (int)v[e];
-          }
-        }
-        __syncwarp();                // the next load from tensor memory is the whole warp's
-      }
-    }
-    tc_fence_before();
-  }
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, I8_BN);
-  }
+// fp16(c SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part where the list is not empty, rounded to fp16
+__device__ __forceinline__ float int8_finish(float c, float sa, float sb, bool has_bias, float bias, int cnt, float odd) {
+  float out = __fmul_rn(__fmul_rn(__fmul_rn(c, sa), sb), 1.0f / (127.0f * 127.0f));
+  if (has_bias) out = __fadd_rn(out, bias);
+  out = __half2float(__float2half_rn(out));
+  if (cnt > 0) out = __half2float(__float2half_rn(__fadd_rn(out, __half2float(__float2half_rn(odd)))));
+  return out;
 }
 
-// out = fp16(C32 SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part, for 64 columns x ROWS rows (of one outlier list) per CTA.  C32 is
-// the sum of `parts` partial sums, `part` numbers apart.
-// Outlier part: the weights and activations of L outliers at a time stand in shared memory as fp32, already rounded; the next L are asked
-// for (all list entries, then all they point to) before these are added.  64 rows: a thread owns four columns of four rows, two 16-byte
-// reads for 16 multiply-adds.  16 rows: a list of up to L is added by a thread per row and four columns; a longer one is shared among the
-// quarters of the threads, four columns of four rows each, a quarter of every L, whose sums are added in order.  Four CTAs an SM:
-// a batch of 64 rows has 688 of them for 11008 columns.
+// One layer's weights, scales and bias as the finishing code reads them (cbt: CB transposed, or null).
+template <typename T>
+struct I8Layer {
+  const int8_t* cb;
+  const int8_t* cbt;
+  const float* scb;
+  const T* bias;
+};
+
+// out = fp16(C32 SCA SCB / 127^2 (+ bias)), plus fp16 of the outlier part, for 64 columns x 16 rows (of one outlier list) per CTA.  C32 is
+// the sum of `parts` partial sums, `part` numbers apart.  GATED: of both layers (the second's partial sums lie `layer` numbers further), and
+// y = silu(out1) * out2, rounded as ll_silu_mul rounds it.
+// Outlier part: the weights and activations of 64 outliers at a time stand in shared memory as fp32, already rounded; the next 64 are asked
+// for (all list entries, then all they point to) before these are added.  A list of up to 64 is added by a thread per row and four columns; a
+// longer one is shared among the quarters of the threads, four columns of four rows each, a quarter of every 64, whose sums are added in
+// order.  Four CTAs an SM: a batch of 64 rows has 688 of them for 11008 columns.
 // Three layers of a 4096-wide feed-forward, 32 rows whose inputs have 6 / 30 / 100 / 200 outlier features (their products up to thousands):
 // 78 / 121 / 424 / 519 us a call on the device.  32 outliers at a time, each weight behind its own list entry: 78 / 259 / 1725 / 2131; the
 // kernel beside the mma.sync product: 123 / 181 / 536 / 647.  (A stage of 128 leaves three CTAs an SM: 87 with 12 outliers, 84 with 64.)
-template <typename T, int ROWS>
-__global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t* __restrict__ c32, int parts, size_t part, const float* __restrict__ sca,
-                                                              const float* __restrict__ scb, const T* __restrict__ bias, const T* __restrict__ x,
-                                                              const int8_t* __restrict__ cb, const int8_t* __restrict__ cbt,
-                                                              const int32_t* __restrict__ idx, const int32_t* __restrict__ count,
+template <typename T, bool GATED>
+__global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t* __restrict__ c32, int parts, size_t part, size_t layer,
+                                                              const float* __restrict__ sca, const I8Layer<T> l0, const I8Layer<T> l1,
+                                                              const T* __restrict__ x, const int32_t* __restrict__ idx, const int32_t* __restrict__ count,
                                                               T* __restrict__ y, int M, int N, int K) {
-  static_assert(ROWS == 16 || ROWS == 64, "rows of a CTA");
-  constexpr int SL = 64 / ROWS, L = SL == 1 ? 32 : 64, NW = L * 16 / 256, NA = L * ROWS / 256, AS = 256 / ROWS;   // SL: shares of the list
+  constexpr int ROWS = 16, SL = 4, L = 64, NW = L * 16 / 256, NA = L * ROWS / 256, AS = 256 / ROWS;   // SL: shares of the list
   __shared__ __align__(16) float w_s[L][64], a_s[L][ROWS];
   const int tid = threadIdx.x, n0 = blockIdx.x * 64, m0 = blockIdx.y * ROWS, blk = m0 / 64, col = (tid & 15) * 4;
-  const int cnt = count[blk];
-  float acc[4][4];
+  const int cnt = count[blk], n = n0 + col, m = m0 + (tid >> 4);
+  const bool vec = n + 4 <= N && (N & 3) == 0;             // (then a partial sum starts on a 16-byte boundary too)
+  float first[4];                                          // GATED: the first layer's outputs
+#pragma unroll 1
+  for (int which = 0; which < (GATED ? 2 : 1); ++which) {
+    const int8_t *cb = which ? l1.cb : l0.cb, *cbt = which ? l1.cbt : l0.cbt;
+    const float* scb = which ? l1.scb : l0.scb;
+    const T* bias = which ? l1.bias : l0.bias;
+    float acc[4][4];
 #pragma unroll
-  for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
-  if (cnt > 0) {
-    const int32_t* list = idx + (size_t)blk * K;
-    // what a thread brings: four columns of NW outliers' weights, one row of NA outliers' activations.  Entries past the list's end, columns
-    // past N and rows past M repeat the last one: they are never added, or added to what nobody stores.  Steps that lie past the end for the
-    // whole CTA are left out (a gather from every row each: 512 rows with six outliers, three layers: 264 us a call with them, 244 without).
-    const int wi = tid >> 4, ai = tid / ROWS;
-    const T* xr = x + (size_t)min(m0 + (tid & (ROWS - 1)), M - 1) * K;
-    const bool words = cbt != nullptr && (N & 3) == 0 && ((uintptr_t)cbt & 3) == 0;
-    float sb127[4];
+    for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+    if (cnt > 0) {
+      if (which) __syncthreads();                          // the first layer's outliers have been added
+      const int32_t* list = idx + (size_t)blk * K;
+      // what a thread brings: four columns of NW outliers' weights, one row of NA outliers' activations.  Entries past the list's end, columns
+      // past N and rows past M repeat the last one: they are never added, or added to what nobody stores.  Steps that lie past the end for the
+      // whole CTA are left out.
+      const int wi = tid >> 4, ai = tid / ROWS;
+      const T* xr = x + (size_t)min(m0 + (tid & (ROWS - 1)), M - 1) * K;
+      const bool words = cbt != nullptr && (N & 3) == 0 && ((uintptr_t)cbt & 3) == 0;
+      float sb127[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn(scb[min(n0 + col + j, N - 1)], 127.f);
-    uint32_t q[NW];
-    float av[NA];
-    auto fetch = [&](int b) {
-      int kw[NW], ka[NA];
+      for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn(scb[min(n + j, N - 1)], 127.f);
+      uint32_t q[NW];
+      float av[NA];
+      auto fetch = [&](int b) {
+        int kw[NW], ka[NA];
 #pragma unroll
-      for (int u = 0; u < NW; ++u) q[u] = 0u, kw[u] = b + 16 * u < cnt ? __ldg(list + min(b + wi + 16 * u, cnt - 1)) : 0;
+        for (int u = 0; u < NW; ++u) q[u] = 0u, kw[u] = b + 16 * u < cnt ? __ldg(list + min(b + wi + 16 * u, cnt - 1)) : 0;
 #pragma unroll
-      for (int u = 0; u < NA; ++u) av[u] = 0.f, ka[u] = b + AS * u < cnt ? __ldg(list + min(b + ai + AS * u, cnt - 1)) : 0;
-      if (words) {
-        const int8_t* src = cbt + min(n0 + col, N - 4);
+        for (int u = 0; u < NA; ++u) av[u] = 0.f, ka[u] = b + AS * u < cnt ? __ldg(list + min(b + ai + AS * u, cnt - 1)) : 0;
+        if (words) {
+          const int8_t* src = cbt + min(n, N - 4);
 #pragma unroll
-        for (int u = 0; u < NW; ++u)
-          if (b + 16 * u < cnt) q[u] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)kw[u] * N));
-      } else {
+          for (int u = 0; u < NW; ++u)
+            if (b + 16 * u < cnt) q[u] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)kw[u] * N));
+        } else {
+#pragma unroll
+          for (int u = 0; u < NW; ++u) {
+            if (b + 16 * u >= cnt) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int c = min(n + j, N - 1);
+              const int8_t v = cbt != nullptr ? __ldg(cbt + (size_t)kw[u] * N + c) : __ldg(cb + (size_t)c * K + kw[u]);
+              q[u] |= (uint32_t)(uint8_t)v << (8 * j);
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < NA; ++u)
+          if (b + AS * u < cnt) av[u] = to_half_f32<T>(xr[ka[u]]);
+      };
+      auto stage = [&]() {
 #pragma unroll
         for (int u = 0; u < NW; ++u) {
-          if (b + 16 * u >= cnt) continue;
+          float w[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int n = min(n0 + col + j, N - 1);
-            const int8_t v = cbt != nullptr ? __ldg(cbt + (size_t)kw[u] * N + n) : __ldg(cb + (size_t)n * K + kw[u]);
-            q[u] |= (uint32_t)(uint8_t)v << (8 * j);
-          }
+          for (int j = 0; j < 4; ++j) w[j] = __half2float(__float2half_rn(__fmul_rn((float)(int8_t)(q[u] >> (8 * j)), sb127[j])));
+          *reinterpret_cast<float4*>(&w_s[wi + 16 * u][col]) = make_float4(w[0], w[1], w[2], w[3]);
         }
-      }
 #pragma unroll
-      for (int u = 0; u < NA; ++u)
-        if (b + AS * u < cnt) av[u] = to_half_f32<T>(xr[ka[u]]);
-    };
-    auto stage = [&]() {
-#pragma unroll
-      for (int u = 0; u < NW; ++u) {
-        float w[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = __half2float(__float2half_rn(__fmul_rn((float)(int8_t)(q[u] >> (8 * j)), sb127[j])));
-        *reinterpret_cast<float4*>(&w_s[wi + 16 * u][col]) = make_float4(w[0], w[1], w[2], w[3]);
-      }
-#pragma unroll
-      for (int u = 0; u < NA; ++u) a_s[ai + AS * u][tid & (ROWS - 1)] = av[u];
-    };
-    fetch(0);
-    if (SL > 1 && cnt <= L) {
-      stage();
-      __syncthreads();
+        for (int u = 0; u < NA; ++u) a_s[ai + AS * u][tid & (ROWS - 1)] = av[u];
+      };
+      fetch(0);
       const int row = tid >> 4;
-#pragma unroll 4
-      for (int i = 0; i < cnt; ++i) {
-        const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]);
-        const float a = a_s[i][row];
-        acc[0][0] = fmaf(a, w.x, acc[0][0]);
-        acc[0][1] = fmaf(a, w.y, acc[0][1]);
-        acc[0][2] = fmaf(a, w.z, acc[0][2]);
-        acc[0][3] = fmaf(a, w.w, acc[0][3]);
-      }
-    } else {
-      const int r0 = ((tid >> 4) & (ROWS / 4 - 1)) * 4, sl = tid / (256 / SL);
-      for (int b = 0; b < cnt; b += L) {
-        if (b > 0) __syncthreads();                        // the outliers before have been added
+      if (cnt <= L) {
         stage();
         __syncthreads();
-        if (b + L < cnt) fetch(b + L);
-        const int i0 = sl * (L / SL), i1 = min(min(L, cnt - b), i0 + L / SL);
 #pragma unroll 4
-        for (int i = i0; i < i1; ++i) {
-          const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]), a4 = *reinterpret_cast<const float4*>(&a_s[i][r0]);
-          const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+        for (int i = 0; i < cnt; ++i) {
+          const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]);
+          const float a = a_s[i][row];
+          acc[0][0] = fmaf(a, w.x, acc[0][0]);
+          acc[0][1] = fmaf(a, w.y, acc[0][1]);
+          acc[0][2] = fmaf(a, w.z, acc[0][2]);
+          acc[0][3] = fmaf(a, w.w, acc[0][3]);
+        }
+      } else {
+        const int r0 = (row & (ROWS / 4 - 1)) * 4, sl = tid / (256 / SL);
+        for (int b = 0; b < cnt; b += L) {
+          if (b > 0) __syncthreads();                      // the outliers before have been added
+          stage();
+          __syncthreads();
+          if (b + L < cnt) fetch(b + L);
+          const int i0 = sl * (L / SL), i1 = min(min(L, cnt - b), i0 + L / SL);
+#pragma unroll 4
+          for (int i = i0; i < i1; ++i) {
+            const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]), a4 = *reinterpret_cast<const float4*>(&a_s[i][r0]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-          for (int r = 0; r < 4; ++r) {
-            acc[r][0] = fmaf(a[r], w.x, acc[r][0]);
-            acc[r][1] = fmaf(a[r], w.y, acc[r][1]);
-            acc[r][2] = fmaf(a[r], w.z, acc[r][2]);
-            acc[r][3] = fmaf(a[r], w.w, acc[r][3]);
+            for (int r = 0; r < 4; ++r) {
+              acc[r][0] = fmaf(a[r], w.x, acc[r][0]);
+              acc[r][1] = fmaf(a[r], w.y, acc[r][1]);
+              acc[r][2] = fmaf(a[r], w.z, acc[r][2]);
+              acc[r][3] = fmaf(a[r], w.w, acc[r][3]);
+            }
           }
         }
-      }
-      if (SL > 1) {                                        // every thread finishes one row: its sums come through shared memory
-        __syncthreads();
+        __syncthreads();                                   // every thread finishes one row: its sums come through shared memory
         float* sums = &w_s[0][0];                          // [SL][ROWS][64]
 #pragma unroll
         for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(sums + (sl * ROWS + r0 + r) * 64 + col) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
         __syncthreads();
-        const int row = tid >> 4;
         float4 o = *reinterpret_cast<const float4*>(sums + row * 64 + col);
 #pragma unroll
         for (int z = 1; z < SL; ++z) {
@@ -398,26 +243,12 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
         acc[0][0] = o.x, acc[0][1] = o.y, acc[0][2] = o.z, acc[0][3] = o.w;
       }
     }
-  }
-  constexpr int R = ROWS / 16;                             // rows a thread finishes
-  const int n = n0 + col, fr = (tid >> 4) * R;
-  if (n >= N) return;
-  float sb[4], bv[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    sb[j] = n + j < N ? scb[n + j] : 0.f;
-    bv[j] = n + j < N && bias != nullptr ? to_half_f32<T>(bias[n + j]) : 0.f;
-  }
-  const bool vec = n + 4 <= N && (N & 3) == 0;             // (then a partial sum starts on a 16-byte boundary too)
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int m = m0 + fr + r;
-    if (m >= M) break;
+    if (n >= N || m >= M) continue;                        // (which takes part in the barriers of the second layer's list)
     const float sa = sca[m];
     const size_t at = (size_t)m * N + n;
     int cv[4] = {0, 0, 0, 0};
     for (int z = 0; z < parts; ++z) {
-      const int32_t* src = c32 + (size_t)z * part + at;
+      const int32_t* src = c32 + (which ? layer : 0) + (size_t)z * part + at;
       if (vec) {
         const int4 v = __ldcs(reinterpret_cast<const int4*>(src));
         cv[0] += v.x, cv[1] += v.y, cv[2] += v.z, cv[3] += v.w;
@@ -429,35 +260,12 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (n + j >= N) break;
-      float out = __fmul_rn(__fmul_rn(__fmul_rn((float)cv[j], sa), sb[j]), 1.0f / (127.0f * 127.0f));
-      if (bias != nullptr) out = __fadd_rn(out, bv[j]);
-      out = __half2float(__float2half_rn(out));
-      if (cnt > 0) out = __half2float(__float2half_rn(__fadd_rn(out, __half2float(__float2half_rn(acc[r][j])))));
-      dt<T>::st(y, at + j, out);
+      const float out = int8_finish((float)cv[j], sa, scb[n + j], bias != nullptr, bias != nullptr ? to_half_f32<T>(bias[n + j]) : 0.f, cnt, acc[0][j]);
+      if (!GATED) dt<T>::st(y, at + j, out);
+      else if (which == 0) first[j] = dt<T>::rd(out);
+      else dt<T>::st(y, at + j, __fmul_rn(silu_act<T>(first[j]), dt<T>::rd(out)));
     }
   }
-}
-
-constexpr int I8_PASS = 1024;        // rows of one pass: bounds the int32 product (57 MB at 13824 columns)
-struct WsRows {
-  int8_t* ca; int32_t* c32; uint8_t* flag; int32_t* idx; float* sca; int32_t* count;
-  size_t flag_bytes, total;
-};
-WsRows carve_rows(void* base, int M, int N, int K) {
-  WsRows w;
-  const int rows = M < I8_PASS ? M : I8_PASS, blocks = (rows + 63) / 64;
-  size_t o = 0;
-  auto take = [&](size_t b) { size_t r = o; o += (b + 255) & ~(size_t)255; return r; };
-  uint8_t* p = (uint8_t*)base;
-  w.ca = (int8_t*)(p + take((size_t)rows * K));
-  w.c32 = (int32_t*)(p + take((size_t)rows * N * 4));
-  w.flag_bytes = (size_t)blocks * K;
-  w.flag = (uint8_t*)(p + take(w.flag_bytes));
-  w.idx = (int32_t*)(p + take((size_t)blocks * K * 4));
-  w.sca = (float*)(p + take((size_t)rows * 4));
-  w.count = (int32_t*)(p + take((size_t)blocks * 4));
-  w.total = o;
-  return w;
 }
 
 // [rows][K] int8 row-major -> 2-D map, boxes of box_rows x 128 bytes, 128-byte swizzle, rows past the end zero
@@ -478,37 +286,12 @@ int make_map_i8(const void* base, int rows, int K, int box_rows, CUtensorMap* ou
   return LL_OK;
 }
 
-template <typename T>
-int int8_rows_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* scb, const T* bias, T* y, int M, int N, int K, float thr,
-                void* ws_base, cudaStream_t st) {
-  constexpr int smem = 2 * I8_STAGES * I8_BOX + (2 * I8_STAGES + 1) * 8 + 16 + 1024;
-  LL_CUDA(cudaFuncSetAttribute(int8_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const WsRows w = carve_rows(ws_base, M, N, K);
-  const int vec = ((uintptr_t)x & 15) == 0;
-  CUtensorMap ma, mb;
-  if (int r = make_map_i8(cb, N, K, 128, &mb)) return r;
-  for (int r0 = 0; r0 < M; r0 += I8_PASS) {
-    const int rows = min(I8_PASS, M - r0), blocks = (rows + 63) / 64;
-    const T* xp = x + (size_t)r0 * K;
-    LL_CUDA(cudaMemsetAsync(w.flag, 0, w.flag_bytes, st));
-    int8_row_stats_kernel<T><<<rows, 256, 0, st>>>(xp, w.flag, w.sca, K, thr, vec);
-    const long long pieces = (long long)rows * (K / 8);
-    int8_row_quant_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>(xp, w.flag, w.sca, w.ca, K, thr, pieces, vec);
-    int8_lists_kernel<<<blocks, 1024, 0, st>>>(w.flag, w.idx, w.count, K);
-    if (int r = make_map_i8(w.ca, rows, K, 128, &ma)) return r;
-    int8_gemm_tc_kernel<<<dim3((rows + BM - 1) / BM, (N + I8_BN - 1) / I8_BN), 192, smem, st>>>(ma, mb, w.c32, rows, N, K, wait_word());
-    int8_finish_rows_kernel<T, 64><<<dim3((N + 63) / 64, blocks), 256, 0, st>>>(w.c32, 1, 0, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count,
-                                                                           y + (size_t)r0 * N, rows, N, K);
-    LL_LAUNCH_OK("int8 linear kernels (prompts)");
-  }
-  return LL_OK;
-}
-
-// ================================================================================================== up to 64 rows
-// One kernel: x.half(), row maxima of the entries below thr, quantised rows, outlier columns as an ascending list.  A CTA owns a row and
+// ================================================================================================== preparation
+// One kernel: x.half(), row maxima of the entries below thr, quantised rows, and for every block of 64 rows the outlier columns as an ascending
+// list.  A CTA owns a row and
 // holds it in registers between its maximum and its codes (up to I8P_HELD * 4096 features; a longer row is read again).  Whether a column
-// stands out in some row is known when every row is done, so the CTA that finishes last makes the list and clears the listed columns'
-// codes.  No CTA waits for another: nothing says that all of them run at the same time.  (A CTA per 64 columns and one wait of the whole
+// stands out in some row is known when the block's rows are done, so the CTA that finishes last of them makes the list and clears the listed
+// columns' codes.  No CTA waits for another: nothing says that all of them run at the same time.  (A CTA per 64 columns and one wait of the whole
 // grid in the middle took 2 us less a layer, and stood still, or went on with counts that were not there, when other streams held the SMs.)
 // 32 rows through a 7B feed-forward, three layers: 78 us on the device; 123 before the product ran on tcgen05.
 constexpr int I8P_THREADS = 512, I8P_HELD = 4;
@@ -519,7 +302,8 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
   constexpr int WARPS = I8P_THREADS / 32, STEP = I8P_THREADS * 8;
   __shared__ float s_max[WARPS];
   __shared__ int s_warp[WARPS], s_last;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, M = gridDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blk = blockIdx.x / 64, m0 = blk * 64, M = min(64, (int)gridDim.x - m0);
+  flag += (size_t)blk * K, idx += (size_t)blk * K;
   const T* row = x + (size_t)blockIdx.x * K;
   float held[I8P_HELD][8], mx = 0.f;
 #pragma unroll
@@ -569,7 +353,7 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
   }
   __threadfence();
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(arrive, 1) == M - 1;
+  if (tid == 0) s_last = atomicAdd(arrive + blk, 1) == M - 1;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
@@ -609,14 +393,15 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
     base += total;
     __syncthreads();
   }
-  if (tid == 0) *count = base;
+  if (tid == 0) count[blk] = base;
   // (the list is complete: a barrier of this CTA, which wrote it, lies behind the last entry)
   for (int i = tid; i < base * M; i += I8P_THREADS) {
     const int m = i / base;
-    ca[(size_t)m * K + idx[i - m * base]] = 0;
+    ca[(size_t)(m0 + m) * K + idx[i - m * base]] = 0;
   }
 }
 
+// ================================================================================================== up to 64 rows
 // part[range][m][n] = the sum over the range's k of CA[m][k] CB[n][k]: the weights are the A operand (128 output columns a CTA), streamed
 // through a ring of 16 KB boxes; two CTAs share an SM.  MP: rows rounded up to 16, 32, 48 or 64.
 // A batch of 32 through a 7B feed-forward: mma.sync straight from global memory, two loads in flight a thread and int32 atomics, took 17.5 us
@@ -624,8 +409,9 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
 constexpr int i8c_stages(int mp) { return mp > 32 ? 4 : 5; }
 constexpr int i8c_smem(int mp) { return i8c_stages(mp) * (I8_BOX + mp * 128) + 256 + 1024; }
 template <int MP>
-__global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                                                                int32_t* __restrict__ part, int M, int N, int nkb, int per, int* word) {
+__global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                                                                const __grid_constant__ CUtensorMap map_x, int32_t* __restrict__ part, int M, int N, int nkb,
+                                                                int per, int tiles, size_t layer, int* word) {
   constexpr int STAGES = i8c_stages(MP), XB = MP * 128, COLS = MP <= 32 ? 32 : 64;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
@@ -636,9 +422,11 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(done + 1);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * 128, kb0 = blockIdx.y * per, kb1 = min(kb0 + per, nkb);
+  const bool second = (int)blockIdx.x >= tiles;              // column tiles of the second layer
+  const int n0 = ((int)blockIdx.x - (second ? tiles : 0)) * 128, kb0 = blockIdx.y * per, kb1 = min(kb0 + per, nkb);
+  const CUtensorMap* map_w = second ? &map_w1 : &map_w0;
   if (threadIdx.x == 0) {
-    prefetch_tensormap(&map_w);
+    prefetch_tensormap(map_w);
     prefetch_tensormap(&map_x);
     for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
     mbar_init(done, 1);
@@ -658,7 +446,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = i8_wait(&empty[s], ph, s_fail, word, 5))) break;
         mbar_expect_tx(&full[s], I8_BOX + XB);
-        i8_box(sw + s * I8_BOX, &map_w, kb * 128, n0, &full[s]);
+        i8_box(sw + s * I8_BOX, map_w, kb * 128, n0, &full[s]);
         i8_box(sx + s * XB, &map_x, kb * 128, 0, &full[s]);
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
@@ -688,7 +476,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
     const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, word, 7) && *(volatile int*)s_fail == 0);
     tc_fence_after();
     if (ok) {
-      int32_t* dst = part + (size_t)blockIdx.y * M * N + n;
+      int32_t* dst = part + (second ? layer : 0) + (size_t)blockIdx.y * M * N + n;
 #pragma unroll
       for (int c0 = 0; c0 < COLS; c0 += 32) {
         uint32_t v[32];
@@ -709,73 +497,523 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
 }
 
 // ranges of k (per: blocks of 128 in each): every CTA of the grid resident at two an SM, if the columns alone do not fill the device
-int i8c_ranges(int N, int K, int sms, int* per) {
-  const int tiles = (N + 127) / 128, nkb = K / 128;
+int i8c_ranges(int N, int K, int layers, int sms, int* per) {
+  const int tiles = layers * ((N + 127) / 128), nkb = K / 128;
   int ranges = 2 * (sms > 0 ? sms : 148) / tiles;
   ranges = ranges < 1 ? 1 : ranges > nkb ? nkb : ranges;
   *per = (nkb + ranges - 1) / ranges;
   return (nkb + *per - 1) / *per;
 }
 
+// What the preparation leaves for a step of M rows, and the partial sums of a step of up to 64 (part_rows).
 struct Ws {
   int8_t* ca; int32_t* part; float* sca; int32_t* idx; uint8_t* flag; int32_t* count; int32_t* arrive;
   size_t zero_off, zero_bytes, total;
 };
-Ws carve(void* base, int M, int N, int K) {
+Ws carve(void* base, int M, int N, int K, int layers, bool partial) {
   Ws w;
+  const size_t blocks = (size_t)(M + 63) / 64;
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o += (b + 255) & ~(size_t)255; return r; };
   uint8_t* p = (uint8_t*)base;
   int per;
   w.ca = (int8_t*)(p + take((size_t)M * K));
-  w.part = (int32_t*)(p + take((size_t)i8c_ranges(N, K, sm_count(), &per) * M * N * 4));
-  w.idx = (int32_t*)(p + take((size_t)K * 4));
-  w.sca = (float*)(p + take(64 * 4));
+  w.part = (int32_t*)(p + take(partial ? (size_t)layers * i8c_ranges(N, K, layers, sm_count(), &per) * M * N * 4 : 0));
+  w.idx = (int32_t*)(p + take(blocks * K * 4));
+  w.sca = (float*)(p + take((size_t)M * 4));
   w.zero_off = o;  // cleared at the start of every call
-  w.flag = p + take((size_t)K);
-  w.count = (int32_t*)(p + take(4));
-  w.arrive = (int32_t*)(p + take(4));
+  w.flag = p + take(blocks * K);
+  w.arrive = (int32_t*)(p + take(blocks * 4));
   w.zero_bytes = o - w.zero_off;
+  w.count = (int32_t*)(p + take(blocks * 4));
   w.total = o;
   return w;
 }
 
+template <typename T>
+int int8_prepare(const T* x, const Ws& w, void* base, int M, int K, float thr, cudaStream_t st) {
+  LL_CUDA(cudaMemsetAsync((uint8_t*)base + w.zero_off, 0, w.zero_bytes, st));
+  int8_prep_kernel<T><<<M, I8P_THREADS, 0, st>>>(x, w.ca, w.sca, w.flag, w.idx, w.count, w.arrive, K, thr, ((uintptr_t)x & 15) == 0);
+  LL_LAUNCH_OK("int8_prep_kernel");
+  return LL_OK;
+}
+
 template <int MP>
-int i8c_launch(const CUtensorMap& mw, const Ws& w, int M, int N, int K, int sms, cudaStream_t st) {
+int i8c_launch(const CUtensorMap& m0, const CUtensorMap& m1, const Ws& w, int M, int N, int K, int layers, int per, int ranges, cudaStream_t st) {
   CUtensorMap mx;
   if (int r = make_map_i8(w.ca, M, K, MP, &mx)) return r;
-  LL_CUDA(cudaFuncSetAttribute(int8_columns_tc_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, i8c_smem(MP)));
-  int per;
-  const int ranges = i8c_ranges(N, K, sms, &per);
-  int8_columns_tc_kernel<MP><<<dim3((N + 127) / 128, ranges), 192, i8c_smem(MP), st>>>(mw, mx, w.part, M, N, K / 128, per, wait_word());
+  static PerDevice configured;
+  if (!configured) {
+    LL_CUDA(cudaFuncSetAttribute(int8_columns_tc_kernel<MP>, cudaFuncAttributeMaxDynamicSharedMemorySize, i8c_smem(MP)));
+    configured.mark();
+  }
+  const int tiles = (N + 127) / 128;
+  int8_columns_tc_kernel<MP><<<dim3(layers * tiles, ranges), 192, i8c_smem(MP), st>>>(m0, m1, mx, w.part, M, N, K / 128, per, tiles, (size_t)ranges * M * N,
+                                                                                    wait_word());
   LL_LAUNCH_OK("int8_columns_tc_kernel");
   return LL_OK;
 }
 
+// up to 64 rows of one layer, or of two whose gated product is wanted
+template <typename T, bool GATED>
+int int8_pass(const T* x, const I8Layer<T>& l0, const I8Layer<T>& l1, T* y, int M, int N, int K, float thr, void* base, cudaStream_t st) {
+  constexpr int layers = GATED ? 2 : 1;
+  const Ws w = carve(base, M, N, K, layers, true);
+  if (int r = int8_prepare<T>(x, w, base, M, K, thr, st)) return r;
+  CUtensorMap m0, m1;
+  if (int r = make_map_i8(l0.cb, N, K, 128, &m0)) return r;
+  if (int r = make_map_i8(l1.cb, N, K, 128, &m1)) return r;
+  int per, r;
+  const int ranges = i8c_ranges(N, K, layers, sm_count(), &per);
+  if (M <= 16) r = i8c_launch<16>(m0, m1, w, M, N, K, layers, per, ranges, st);
+  else if (M <= 32) r = i8c_launch<32>(m0, m1, w, M, N, K, layers, per, ranges, st);
+  else if (M <= 48) r = i8c_launch<48>(m0, m1, w, M, N, K, layers, per, ranges, st);
+  else r = i8c_launch<64>(m0, m1, w, M, N, K, layers, per, ranges, st);
+  if (r) return r;
+  int8_finish_rows_kernel<T, GATED><<<dim3((N + 63) / 64, (M + 15) / 16), 256, 0, st>>>(w.part, ranges, (size_t)M * N, (size_t)ranges * M * N, w.sca, l0, l1, x,
+                                                                                     w.idx, w.count, y, M, N, K);
+  LL_LAUNCH_OK("int8_finish_rows_kernel");
+  return LL_OK;
+}
+
+// ================================================================================================== prompts: M > 64
+// The product and its finish in one kernel, by pairs of CTAs (tcgen05 cta_group::2, kind::i8, K = 32 an instruction): tiles of 256 rows x BN
+// columns a pair, persistent, two int32 accumulators in tensor memory, so that a tile is finished (scales, bias, outlier part, rounding,
+// stores by TMA) under the next one's products.  GATED: the tile's columns are BN / 2 of the first layer (rank 0 brings them) and the same of
+// the second, and y = silu(out1) * out2.
+//   warp 0: TMA producer; warp 1: in rank 0, one thread issues the products; warps 2-9: finish, 32 rows and half of the columns per warp,
+//   32 columns at a time (GATED: 16 of either layer), read from tensor memory so that a thread has four rows of eight columns
+// Outlier part: a warp's 32 rows belong to one block of 64 rows, so to one list.  Its activations (up to 32 a row) are gathered before the
+// tile's sums are there, and so are the scales and the first eight outliers' weights of its columns; the weights of four outliers x 32 columns
+// pass through shared memory as fp32, already rounded.
+// (Four finishing warps, one a scheduler, took 35 us a tile of the gated form, four times as long as its products.)
+// 512 rows through a 7B feed-forward with six outlier features: 53 us for both gated layers and 27 for the third, preparation 24; 127 for three
+// products of 128 x 128 tiles a CTA, 55 for their finish and 45 for preparation and the gated product before.  2048 rows: 305 us a call (701).
+// Bound by the weights' way from memory and, with outliers, by the finish (weights asked for one by one: 10 us a tile instead of 3).
+constexpr int I8R_PASS = 8192;                           // rows of one pass: bounds the workspace
+constexpr int I8R_WARPS = 8, I8R_THREADS = (2 + I8R_WARPS) * 32;                           // finishing warps: two per 32 rows, half of the columns each
+constexpr int I8R_LIST = 32, I8R_OUT = 32 * 64, I8R_W = 6 * 32 * 4;
+constexpr int i8r_stages(int bn) { return bn > 128 ? 5 : 6; }
+constexpr int i8r_smem(int bn) {
+  return i8r_stages(bn) * (I8_BOX + bn * 64) + I8R_WARPS * (2 * I8R_OUT + I8R_LIST * 64 + I8R_LIST * 4 + I8R_W) + 512 + 1024;
+}
+
 template <typename T>
-int int8_linear_t(const T* x, const int8_t* cb, const int8_t* cbt, const float* scb, const T* bias, T* y, int M, int N, int K, float thr,
-                  void* ws_base, cudaStream_t st) {
-  const int sms = sm_count();
-  const int vec = ((uintptr_t)x & 15) == 0;
-  CUtensorMap mw;
-  if (int r = make_map_i8(cb, N, K, 128, &mw)) return r;
-  for (int m0 = 0; m0 < M; m0 += 64) {
-    const int Mp = min(64, M - m0);
-    const Ws w = carve(ws_base, Mp, N, K);
-    const T* xp = x + (size_t)m0 * K;
-    LL_CUDA(cudaMemsetAsync((uint8_t*)ws_base + w.zero_off, 0, w.zero_bytes, st));
-    int8_prep_kernel<T><<<Mp, I8P_THREADS, 0, st>>>(xp, w.ca, w.sca, w.flag, w.idx, w.count, w.arrive, K, thr, vec);
-    LL_LAUNCH_OK("int8_prep_kernel");
-    int r;
-    if (Mp <= 16) r = i8c_launch<16>(mw, w, Mp, N, K, sms, st);
-    else if (Mp <= 32) r = i8c_launch<32>(mw, w, Mp, N, K, sms, st);
-    else if (Mp <= 48) r = i8c_launch<48>(mw, w, Mp, N, K, sms, st);
-    else r = i8c_launch<64>(mw, w, Mp, N, K, sms, st);
+struct I8RParams {
+  I8Layer<T> layer[2];
+  const T* x;
+  const float* sca;
+  const int32_t* idx;
+  const int32_t* count;
+  T* y;
+  int M, N, K, mtiles, ntiles, boxes;                // boxes: TMA stores y
+  int* word;
+};
+struct I8Fail {
+  volatile int* here;
+  uint32_t there;
+  int* word;
+};
+__device__ __forceinline__ bool i8r_wait(uint64_t* bar, uint32_t parity, const I8Fail& f, int code) {
+  for (uint32_t i = 0; i < I8_WAIT_LIMIT; ++i) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 255u) == 255u && *f.here) return false;
+  }
+  *f.here = 1;
+  store_cluster_u32(f.there, 1u);
+  atomicCAS(&g_int8_tc_error, 0, code);
+  wait_ran_out(f.word, 300 + code);
+  return false;
+}
+__device__ __forceinline__ void i8r_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 16 lanes x 16 columns: of every 8 columns a thread gets columns 2 (lane % 4), + 1 of lanes lane / 4 and lane / 4 + 8
+__device__ __forceinline__ void i8r_ld16(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+// two outputs in the activation dtype, packed (16-bit dtypes)
+template <typename T> __device__ __forceinline__ uint32_t i8r_pack(float a, float b);
+template <> __device__ __forceinline__ uint32_t i8r_pack<__nv_bfloat16>(float a, float b) { return pack_bf16(a, b); }
+template <> __device__ __forceinline__ uint32_t i8r_pack<__half>(float a, float b) {
+  const __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+template <> __device__ __forceinline__ uint32_t i8r_pack<float>(float, float) { return 0u; }
+
+template <typename T, int BN, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
+    int8_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
+                     const __grid_constant__ CUtensorMap map_y, const I8RParams<T> p) {
+  constexpr int STAGES = i8r_stages(BN), B_BYTES = BN * 64, COLS = GATED ? BN / 2 : BN, CH = GATED ? 16 : 32, NCH = COLS / 2 / CH;
+  // COLS: outputs of a tile, CH: outputs a thread forms at a time, NCH: how many times
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
+  uint8_t *sa = base, *sb = base + STAGES * I8_BOX, *so = sb + STAGES * B_BYTES;
+  uint8_t* s_list = so + I8R_WARPS * 2 * I8R_OUT;      // per warp: [LIST][32] fp16 activations
+  uint8_t* s_idx = s_list + I8R_WARPS * I8R_LIST * 64; //           [LIST] columns
+  uint8_t* s_w = s_idx + I8R_WARPS * I8R_LIST * 4;     //           [4][32] fp32 weights, [32] scales, [32] biases
+  uint64_t* full = reinterpret_cast<uint64_t*>(s_w + I8R_WARPS * I8R_W);      // used in rank 0
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;                 // [2]
+  uint64_t* acc_empty = acc_full + 2;                  // [2], used in rank 0: both CTAs' warps arrive
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_x);
+    prefetch_tensormap(&map_w0);
+    prefetch_tensormap(&map_w1);
+    prefetch_tensormap(&map_y);
+    for (int i = 0; i < STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * I8R_WARPS);
+    *s_fail = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) pair_tmem_alloc(tmem_ptr, 2 * BN);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  const I8Fail fail{s_fail, cluster_addr(s_fail, (uint32_t)(rank ^ 1)), p.word};
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, tiles = p.mtiles * p.ntiles, nkb = p.K / 128;
+  pdl_wait();
+  pdl_launch_dependents();
+
+  if (warp == 0) {
+    if (elect_one()) {
+      bool ok = true;
+      int s = 0;
+      uint32_t ph = 1;
+      for (int t = pair; ok && t < tiles; t += pairs) {
+        const int m0 = (t % p.mtiles) * 256 + rank * 128, n0 = (t / p.mtiles) * COLS + (GATED ? 0 : rank * (BN / 2));
+        const CUtensorMap* mw = GATED && rank == 1 ? &map_w1 : &map_w0;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = i8r_wait(&empty[s], ph, fail, 1))) break;
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * (I8_BOX + B_BYTES));      // both CTAs' operands
+          const uint32_t bar = cluster_addr(&full[s], 0);
+          pair_box(sa + s * I8_BOX, &map_x, kb * 128, m0, bar);
+          pair_box(sb + s * B_BYTES, mw, kb * 128, n0, bar);
+          if (++s == STAGES) s = 0, ph ^= 1u;
+        }
+      }
+      if (!ok) let_issued_work_end();
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      // D = int32 (2 at bit 4), A = B = signed int8 (1 at bits 7 and 10), both K-major
+      constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+      const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
+      bool ok = true;
+      int s = 0, i = 0;
+      uint32_t ph = 0;
+      for (int t = pair; rank == 0 && ok && t < tiles; t += pairs, ++i) {
+        if (!(ok = i8r_wait(&acc_empty[i & 1], (uint32_t)((i >> 1) & 1) ^ 1u, fail, 4))) break;
+        tc_fence_after();
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!(ok = i8r_wait(&full[s], ph, fail, 2))) break;
+          tc_fence_after();
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            i8r_mma(tmem + (uint32_t)((i & 1) * BN), ad + (uint64_t)(s * (I8_BOX >> 4) + 2 * k), bd + (uint64_t)(s * (B_BYTES >> 4) + 2 * k), idesc,
+                    (kb | k) != 0 ? 1u : 0u);
+          pair_commit(&empty[s]);
+          if (++s == STAGES) s = 0, ph ^= 1u;
+        }
+        if (ok) pair_commit(&acc_full[i & 1]);
+      }
+      if (!ok) let_issued_work_end();
+    }
+  } else {
+    const int quarter = warp & 3, ew = warp - 2, part = ew >> 2;
+    uint8_t* out = so + ew * 2 * I8R_OUT;
+    __half* a_s = reinterpret_cast<__half*>(s_list + ew * I8R_LIST * 64);      // [LIST][8][4]: rows g, g + 8, g + 16, g + 24 side by side
+    int* k_s = reinterpret_cast<int*>(s_idx + ew * I8R_LIST * 4);
+    float* w_s = reinterpret_cast<float*>(s_w + ew * I8R_W);
+    // what a thread finishes: rows g, g + 8, .. of the warp's 32, columns 2 t4, + 1 of every 8 (as tensor memory is read in 16 x 256-bit pieces)
+    const int g = lane >> 2, t4 = lane & 3;
+    // the weight column a lane brings, and its place among those that the threads of one t4 read
+    const int place = ((lane & 7) >> 1) * 8 + (lane >> 3) * 2 + (lane & 1);
+    const bool second = GATED && lane >= 16;
+    const int lcol = GATED ? lane & 15 : lane;
+    const int8_t *cb = second ? p.layer[1].cb : p.layer[0].cb, *cbt = second ? p.layer[1].cbt : p.layer[0].cbt;
+    const float* scb = second ? p.layer[1].scb : p.layer[0].scb;
+    const T* bias = second ? p.layer[1].bias : p.layer[0].bias;
+    const bool any_bias = p.layer[0].bias != nullptr || (GATED && p.layer[1].bias != nullptr);
+    int i = 0;
+    uint32_t boxes = 0;
+    for (int t = pair; t < tiles; t += pairs, ++i) {
+      const int r0 = (t % p.mtiles) * 256 + rank * 128 + quarter * 32, n0 = (t / p.mtiles) * COLS, m = min(r0 + lane, p.M - 1);
+      // the block's list and this row's activations of its first entries
+      const int cnt = r0 < p.M ? p.count[r0 / 64] : 0;
+      const int32_t* list = p.idx + (size_t)(r0 / 64) * p.K;
+      const T* xr = p.x + (size_t)m * p.K;
+      __syncwarp();
+      if (lane < cnt) k_s[lane] = __ldg(list + lane);
+      __syncwarp();
+      for (int l = 0; l < min(cnt, I8R_LIST); l += 4) {
+        T v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = xr[k_s[min(l + j, cnt - 1)]];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a_s[(l + j) * 32 + (lane & 7) * 4 + (lane >> 3)] = __float2half_rn(to_half_f32<T>(v[j]));
+      }
+      float sca[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) sca[r] = p.sca[min(r0 + g + 8 * r, p.M - 1)];
+      // the weights of outliers l .. l + 3 in the lane's column of the chunk at cc, all loads in flight together (past the list's end the last
+      // one again: never added)
+      auto fetch = [&](int cc, int l) {
+        const int n = min(n0 + cc + lcol, p.N - 1);
+        const int8_t* src = cbt != nullptr ? cbt + n : cb + (size_t)n * p.K;
+        const size_t step = cbt != nullptr ? (size_t)p.N : 1;
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int at = min(l + j, cnt - 1);
+          v[j] = (uint8_t)__ldg(src + (size_t)(l < I8R_LIST ? k_s[at] : __ldg(list + at)) * step);
+        }
+        return v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
+      };
+      // what the tile's chunks want of their columns, asked for before the sums are there: scales, weights of the first eight outliers
+      const int c_end = (part + 1) * (COLS / 2);
+      float scale[NCH];
+      uint32_t q0[NCH], q1[NCH];
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        const int cc = part * (COLS / 2) + c * CH;
+        scale[c] = __ldg(scb + min(n0 + cc + lcol, p.N - 1));
+        q0[c] = q1[c] = 0u;
+      }
+      if (cnt > 0) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) q0[c] = fetch(part * (COLS / 2) + c * CH, 0);
+      }
+      if (cnt > 4) {
+#pragma unroll
+        for (int c = 0; c < NCH; ++c) q1[c] = fetch(part * (COLS / 2) + c * CH, 4);
+      }
+      if (!__all_sync(0xffffffffu, i8r_wait(&acc_full[i & 1], (uint32_t)(i >> 1) & 1u, fail, 3))) break;
+      tc_fence_after();
+      const uint32_t td = tmem + (uint32_t)((i & 1) * BN) + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll 1
+      for (int cc = part * (COLS / 2); cc < c_end; cc += CH) {
+        // scales and biases of the chunk's columns for every lane to read
+        const int n = min(n0 + cc + lcol, p.N - 1);
+        const float sb = scale[0], sb127 = __fdiv_rn(sb, 127.f);
+        __syncwarp();
+        w_s[4 * 32 + place] = sb;
+        w_s[5 * 32 + place] = bias != nullptr ? to_half_f32<T>(bias[n]) : 0.f;
+        float odd[32];                       // [row half of 16][8 columns][g, g + 8][2 t4, + 1]
+#pragma unroll
+        for (int e = 0; e < 32; ++e) odd[e] = 0.f;
+        uint32_t q = q0[0], qn = q1[0];
+#pragma unroll 1
+        for (int l = 0; l < cnt; l += 4) {
+          const uint32_t w4 = q;
+          q = qn;
+          if (l + 8 < cnt) qn = fetch(cc, l + 8);
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) w_s[j * 32 + place] = __half2float(__float2half_rn(__fmul_rn((float)(int8_t)(w4 >> (8 * j)), sb127)));
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (l + j >= cnt) break;
+            float a[4];
+            if (l + j < I8R_LIST) {
+              const uint2 h = *reinterpret_cast<const uint2*>(a_s + (l + j) * 32 + g * 4);
+              const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
+              a[0] = lo.x, a[1] = lo.y, a[2] = hi.x, a[3] = hi.y;
+            } else {
+              const int k = __ldg(list + l + j);
+#pragma unroll
+              for (int r = 0; r < 4; ++r) a[r] = to_half_f32<T>(p.x[(size_t)min(r0 + g + 8 * r, p.M - 1) * p.K + k]);
+            }
+            const float4 w0 = *reinterpret_cast<const float4*>(w_s + j * 32 + t4 * 8), w1 = *reinterpret_cast<const float4*>(w_s + j * 32 + t4 * 8 + 4);
+            const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int e = 0; e < 32; ++e) odd[e] = fmaf(a[(e >> 4) * 2 + ((e >> 1) & 1)], w[((e >> 2) & 3) * 2 + (e & 1)], odd[e]);
+          }
+        }
+        __syncwarp();
+        uint32_t v[32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          i8r_ld16(td + ((uint32_t)(16 * h) << 16) + (uint32_t)cc, v + 16 * h);
+          i8r_ld16(td + ((uint32_t)(16 * h) << 16) + (uint32_t)(GATED ? BN / 2 + cc : cc + 16), v + 16 * h + 8);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 32; ++e) asm volatile("" : "+r"(v[e]));          // (the loads' results are there from here on)
+        if (cc + CH >= c_end) {              // the warp's sums have left tensor memory
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[i & 1], 0));
+        }
+        const float4 s0 = *reinterpret_cast<const float4*>(w_s + 4 * 32 + t4 * 8), s1 = *reinterpret_cast<const float4*>(w_s + 4 * 32 + t4 * 8 + 4);
+        const float sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+        float o[32];
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {    // int8_finish, two columns at a time (the sum of two fp16 numbers rounds to fp16 the same from fp32)
+          const int b = (e >> 2) & 3;
+          const float sa = sca[(e >> 4) * 2 + ((e >> 1) & 1)];
+          float f0 = __fmul_rn(__fmul_rn(__fmul_rn((float)(int)v[e], sa), sv[b * 2]), 1.0f / (127.0f * 127.0f));
+          float f1 = __fmul_rn(__fmul_rn(__fmul_rn((float)(int)v[e + 1], sa), sv[b * 2 + 1]), 1.0f / (127.0f * 127.0f));
+          if (any_bias) {
+            const float2 bv = *reinterpret_cast<const float2*>(w_s + 5 * 32 + t4 * 8 + b * 2);
+            f0 = __fadd_rn(f0, bv.x), f1 = __fadd_rn(f1, bv.y);
+          }
+          __half2 h = __floats2half2_rn(f0, f1);
+          if (cnt > 0) h = __hadd2_rn(h, __floats2half2_rn(odd[e], odd[e + 1]));
+          const float2 r = __half22float2(h);
+          o[e] = r.x, o[e + 1] = r.y;
+        }
+        if (GATED) {                         // columns b of the first layer and b + 2 of the second: the product takes the first's place
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if ((e & 8) == 0) o[e] = __fmul_rn(silu_act<T>(dt<T>::rd(o[e])), dt<T>::rd(o[e + 8]));
+        }
+        if (p.boxes) {                       // boxes of 32 rows x 32 columns (GATED: in two halves)
+          const int half = GATED ? (cc >> 4) & 1 : 0;
+          const bool last = !GATED || half == 1;
+          uint8_t* box = out + (boxes & 1u) * I8R_OUT;
+          if (half == 0) {
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the box before the last has left
+            __syncwarp();
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            if (GATED && (e & 8) != 0) continue;
+            const int row = (e >> 4) * 16 + ((e >> 1) & 1) * 8 + g, piece = half * 2 + ((e >> 2) & 3);
+            *reinterpret_cast<uint32_t*>(box + row * 64 + ((piece ^ ((row >> 1) & 3)) * 16) + t4 * 4) = i8r_pack<T>(o[e], o[e + 1]);
+          }
+          if (last) {
+            fence_proxy_async();
+            __syncwarp();
+            const int c0 = n0 + (cc & ~31);
+            if (lane == 0) {
+              if (r0 < p.M && c0 < p.N)
+                asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&map_y), "r"(c0), "r"(r0),
+                             "r"(smem_u32(box))
+                             : "memory");
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+            ++boxes;
+          }
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            if (GATED && (e & 8) != 0) continue;
+            const int row = r0 + (e >> 4) * 16 + ((e >> 1) & 1) * 8 + g, c = n0 + cc + ((e >> 2) & 3) * 8 + 2 * t4 + (e & 1);
+            if (row < p.M && c < p.N) dt<T>::st(p.y, (size_t)row * p.N + c, o[e]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c + 1 < NCH; ++c) scale[c] = scale[c + 1], q0[c] = q0[c + 1], q1[c] = q1[c + 1];
+        __syncwarp();                        // the next load from tensor memory is the whole warp's
+      }
+    }
+    tc_fence_before();
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+  }
+  __syncthreads();
+  cluster_sync();
+  if (warp == 1) {
+    tc_fence_after();
+    pair_tmem_dealloc(tmem, 2 * BN);
+  }
+}
+
+// the output as a map of boxes of 32 rows x 32 numbers of two bytes (their type does not matter to a copy)
+int i8r_out_map(const void* y, int M, int N, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled entry point not available");
+    return LL_ERR_CUDA;
+  }
+  cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M}, strides[1] = {(cuuint64_t)N * 2};
+  cuuint32_t box[2] = {32, 32}, estr[2] = {1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)y, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d): output M=%d N=%d", (int)r, M, N);
+    return LL_ERR_CUDA;
+  }
+  return LL_OK;
+}
+
+template <typename T, int BN, bool GATED>
+int i8r_launch(const I8RParams<T>& q, cudaStream_t st, const int8_t* ca) {
+  constexpr int COLS = GATED ? BN / 2 : BN;
+  I8RParams<T> p = q;
+  p.mtiles = (p.M + 255) / 256, p.ntiles = (p.N + COLS - 1) / COLS;
+  p.boxes = sizeof(T) == 2 && p.N % 8 == 0 && ((uintptr_t)p.y & 15) == 0;
+  p.word = wait_word();
+  const long long tiles = (long long)p.mtiles * p.ntiles;
+  LL_CHECK_ARG(tiles < (1ll << 30), "int8 linear: too many tiles");
+  CUtensorMap mx, m0, m1, my;
+  if (int r = make_map_i8(ca, p.M, p.K, 128, &mx)) return r;
+  if (int r = make_map_i8(p.layer[0].cb, p.N, p.K, BN / 2, &m0)) return r;
+  if (int r = make_map_i8(p.layer[GATED ? 1 : 0].cb, p.N, p.K, BN / 2, &m1)) return r;
+  my = mx;
+  if (p.boxes) {
+    if (int r = i8r_out_map(p.y, p.M, p.N, &my)) return r;
+  }
+  static PerDevice configured;
+  if (!configured) {
+    LL_CUDA(cudaFuncSetAttribute(int8_pair_kernel<T, BN, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, i8r_smem(BN)));
+    configured.mark();
+  }
+  const int pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  LL_CUDA(launch(int8_pair_kernel<T, BN, GATED>, dim3(2 * (unsigned)(tiles < pairs ? tiles : pairs)), dim3(I8R_THREADS), i8r_smem(BN), st, true, mx, m0, m1, my, p));
+  LL_LAUNCH_OK("int8_pair_kernel");
+  return LL_OK;
+}
+
+template <typename T, bool GATED>
+int int8_rows(const T* x, const I8Layer<T>& l0, const I8Layer<T>& l1, T* y, int M, int N, int K, float thr, void* base, cudaStream_t st) {
+  for (int r0 = 0; r0 < M; r0 += I8R_PASS) {
+    const int rows = min(I8R_PASS, M - r0);
+    const Ws w = carve(base, rows, N, K, 1, false);
+    const T* xp = x + (size_t)r0 * K;
+    if (int r = int8_prepare<T>(xp, w, base, rows, K, thr, st)) return r;
+    I8RParams<T> p{};
+    p.layer[0] = l0, p.layer[1] = l1, p.x = xp, p.sca = w.sca, p.idx = w.idx, p.count = w.count, p.y = y + (size_t)r0 * N;
+    p.M = rows, p.N = N, p.K = K;
+    // tiles of half the columns take 0.6 of the time: what the waves cost (as the dense products' rule)
+    const long long pairs = sm_count() > 1 ? sm_count() / 2 : 1, mt = (rows + 255) / 256, wide = GATED ? 128 : 256;
+    const long long w256 = (mt * ((N + wide - 1) / wide) + pairs - 1) / pairs, w128 = (mt * ((2 * N + wide - 1) / wide) + pairs - 1) / pairs;
+    const int r = 3 * w128 < 5 * w256 ? i8r_launch<T, 128, GATED>(p, st, w.ca) : i8r_launch<T, 256, GATED>(p, st, w.ca);
     if (r) return r;
-    int per;
-    int8_finish_rows_kernel<T, 16><<<dim3((N + 63) / 64, (Mp + 15) / 16), 256, 0, st>>>(
-        w.part, i8c_ranges(N, K, sms, &per), (size_t)Mp * N, w.sca, scb, bias, xp, cb, cbt, w.idx, w.count, y + (size_t)m0 * N, Mp, N, K);
-    LL_LAUNCH_OK("int8_finish_rows_kernel");
+  }
+  return LL_OK;
+}
+
+size_t i8_workspace_bytes(int M, int N, int K, int layers) {
+  const size_t pass = carve(nullptr, M < 64 ? M : 64, N, K, layers, true).total;
+  if (M <= 64) return pass;
+  const size_t rows = carve(nullptr, M < I8R_PASS ? M : I8R_PASS, N, K, layers, false).total;
+  return rows > pass ? rows : pass;
+}
+
+// prompts go through one product; with a workspace that only holds a pass of 64 rows, through passes
+template <typename T, bool GATED>
+int int8_run(const void* x, const I8Layer<T>& l0, const I8Layer<T>& l1, void* y, int M, int N, int K, float thr, void* base, size_t bytes, cudaStream_t st) {
+  if (M > 64 && bytes >= i8_workspace_bytes(M, N, K, GATED ? 2 : 1)) return int8_rows<T, GATED>((const T*)x, l0, l1, (T*)y, M, N, K, thr, base, st);
+  for (int m0 = 0; m0 < M; m0 += 64) {
+    const int r = int8_pass<T, GATED>((const T*)x + (size_t)m0 * K, l0, l1, (T*)y + (size_t)m0 * N, min(64, M - m0), N, K, thr, base, st);
+    if (r) return r;
   }
   return LL_OK;
 }
@@ -787,12 +1025,8 @@ using namespace llb;
 
 extern "C" {
 
-size_t ll_int8_workspace_bytes(int M, int N, int K) {
-  const size_t pass = carve(nullptr, M < 64 ? M : 64, N, K).total;
-  if (M <= 64) return pass;
-  const size_t rows = carve_rows(nullptr, M, N, K).total;
-  return rows > pass ? rows : pass;
-}
+size_t ll_int8_workspace_bytes(int M, int N, int K) { return i8_workspace_bytes(M, N, K, 1); }
+size_t ll_int8_gated_workspace_bytes(int M, int N, int K) { return i8_workspace_bytes(M, N, K, 2); }
 
 int ll_int8_tc_error(void) {
   int v = 0;
@@ -820,23 +1054,29 @@ int ll_int8_linear(const void* x, int act_dtype, const int8_t* cb, const int8_t*
   LL_CHECK_ARG(((uintptr_t)cb & 15) == 0 && ((uintptr_t)workspace & 255) == 0, "cb must be 16-byte, workspace 256-byte aligned");
   LL_CHECK_ARG(workspace_bytes >= ll_int8_workspace_bytes(M < 64 ? M : 64, N, K), "workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
-  // prompts go through one product; with a workspace that only holds a pass of 64 rows, through passes
-  if (M > 64 && workspace_bytes >= ll_int8_workspace_bytes(M, N, K)) {
-    if (act_dtype == LL_BF16)
-      return int8_rows_t<__nv_bfloat16>((const __nv_bfloat16*)x, cb, cbt, scb, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, M, N, K, threshold, workspace, st);
-    if (act_dtype == LL_F16)
-      return int8_rows_t<__half>((const __half*)x, cb, cbt, scb, (const __half*)bias, (__half*)y, M, N, K, threshold, workspace, st);
-    if (act_dtype == LL_F32)
-      return int8_rows_t<float>((const float*)x, cb, cbt, scb, (const float*)bias, (float*)y, M, N, K, threshold, workspace, st);
-  }
-  if (act_dtype == LL_BF16)
-    return int8_linear_t<__nv_bfloat16>((const __nv_bfloat16*)x, cb, cbt, scb, (const __nv_bfloat16*)bias, (__nv_bfloat16*)y, M, N, K, threshold, workspace, st);
-  if (act_dtype == LL_F16)
-    return int8_linear_t<__half>((const __half*)x, cb, cbt, scb, (const __half*)bias, (__half*)y, M, N, K, threshold, workspace, st);
-  if (act_dtype == LL_F32)
-    return int8_linear_t<float>((const float*)x, cb, cbt, scb, (const float*)bias, (float*)y, M, N, K, threshold, workspace, st);
+#define LL_I8(T)                                                        \
+  do {                                                                  \
+    const I8Layer<T> l{cb, cbt, scb, (const T*)bias};                   \
+    return int8_run<T, false>(x, l, l, y, M, N, K, threshold, workspace, workspace_bytes, st); \
+  } while (0)
+  if (act_dtype == LL_BF16) LL_I8(__nv_bfloat16);
+  if (act_dtype == LL_F16) LL_I8(__half);
+  if (act_dtype == LL_F32) LL_I8(float);
+#undef LL_I8
   set_error("int8_linear: unsupported activation dtype %d", act_dtype);
   return LL_ERR_UNSUPPORTED;
+}
+
+int ll_int8_gated(const void* x, const int8_t* cb1, const int8_t* cbt1, const float* scb1, const void* bias1, const int8_t* cb2, const int8_t* cbt2,
+                  const float* scb2, const void* bias2, void* h, int M, int N, int K, float threshold, void* workspace, size_t workspace_bytes,
+                  ll_stream stream) {
+  LL_CHECK_ARG(x && cb1 && scb1 && cb2 && scb2 && h && workspace, "null pointer");
+  LL_CHECK_ARG(M > 0 && N > 0 && K > 0 && K % 128 == 0, "int8 linear needs K %% 128 == 0 (M=%d N=%d K=%d)", M, N, K);
+  LL_CHECK_ARG((((uintptr_t)cb1 | (uintptr_t)cb2) & 15) == 0 && ((uintptr_t)workspace & 255) == 0, "cb must be 16-byte, workspace 256-byte aligned");
+  LL_CHECK_ARG(workspace_bytes >= ll_int8_gated_workspace_bytes(M < 64 ? M : 64, N, K), "workspace too small");
+  typedef __nv_bfloat16 T;
+  const I8Layer<T> l0{cb1, cbt1, scb1, (const T*)bias1}, l1{cb2, cbt2, scb2, (const T*)bias2};
+  return int8_run<T, true>(x, l0, l1, h, M, N, K, threshold, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 }  // extern "C"

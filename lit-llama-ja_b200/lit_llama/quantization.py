@@ -291,7 +291,7 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
     """``silu(fc1(x)) * fc2(x)`` of two quantized layers of one size in one kernel, rounded as the separate ones round it; ``None``: this step
     has no such kernel."""
     if not (is_plain(fc1, ColBlockQuantizedLinear) and is_plain(fc2, ColBlockQuantizedLinear)):
-        return None
+        return _int8_gated_pair(fc1, fc2, inp) if is_plain(fc1, Linear8bitLt) and is_plain(fc2, Linear8bitLt) else None
     K, Nout = fc1.in_features, fc1.out_features
     if (fc2.in_features, fc2.out_features, fc2.tile_cols) != (K, Nout, fc1.tile_cols) or inp.shape[-1] != K or inp.device.type != "cuda":
         return None
@@ -438,15 +438,41 @@ class Linear8bitLt(torch.nn.Module):
         if M == 0:
             return inp.new_empty(inp.shape[:-1] + (Nout,))
         y = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
-        need = N._fn["ll_int8_workspace_bytes"](M, Nout, K)
-        ws = _int8_workspace(x.device, need)
-        bias = None if self.bias is None else self.bias.to(x.dtype)
-        cbt = getattr(self, "_cbt", None)
-        if cbt is not None and (cbt.device != x.device or cbt.shape != (K, Nout)):
-            cbt = None
-        N.call("ll_int8_linear", N.ptr(x), N.dtype_code(x.dtype), N.ptr(self.weight.CB), N.ptr(cbt), N.ptr(self.weight.SCB), N.ptr(bias),
-               N.ptr(y), M, Nout, K, float(self.threshold), N.ptr(ws), ws.numel(), N.stream())
+        ws = _int8_workspace(x.device, _int8_workspace_bytes(M, Nout, K, 1))
+        cb, cbt, scb, bias = self._operands(x)
+        N.call("ll_int8_linear", N.ptr(x), N.dtype_code(x.dtype), N.ptr(cb), N.ptr(cbt), N.ptr(scb), N.ptr(bias), N.ptr(y), M, Nout, K,
+               float(self.threshold), N.ptr(ws), ws.numel(), N.stream())
         return y.reshape(inp.shape[:-1] + (Nout,))
+
+    def _operands(self, x):
+        """(CB, CB transposed or None, SCB, bias in x's dtype or None)"""
+        w, bias, cbt = self.weight, self.bias, getattr(self, "_cbt", None)
+        if cbt is not None and (cbt.device != x.device or cbt.shape != (self.in_features, self.out_features)):
+            cbt = None
+        return w.CB, cbt, w.SCB, None if bias is None else bias.to(x.dtype)
+
+
+@functools.lru_cache(maxsize=4096)
+def _int8_workspace_bytes(M: int, Nout: int, K: int, layers: int) -> int:
+    return N.call_ret("ll_int8_gated_workspace_bytes" if layers == 2 else "ll_int8_workspace_bytes", M, Nout, K)
+
+
+def _int8_gated_pair(fc1: Linear8bitLt, fc2: Linear8bitLt, inp: torch.Tensor):
+    """``gated_pair`` of two llm.int8 layers: x is prepared once."""
+    K, Nout = fc1.in_features, fc1.out_features
+    if (fc2.in_features, fc2.out_features, fc2.threshold) != (K, Nout, fc1.threshold) or inp.dtype != torch.bfloat16 or inp.shape[-1] != K:
+        return None
+    N.require_cuda(inp, fc1.weight, fc2.weight)
+    x = inp.reshape(-1, K).contiguous()
+    M = x.shape[0]
+    if M == 0:
+        return None
+    h = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
+    ws = _int8_workspace(x.device, _int8_workspace_bytes(M, Nout, K, 2))
+    (cb1, cbt1, scb1, b1), (cb2, cbt2, scb2, b2) = fc1._operands(x), fc2._operands(x)
+    N.call("ll_int8_gated", N.ptr(x), N.ptr(cb1), N.ptr(cbt1), N.ptr(scb1), N.ptr(b1), N.ptr(cb2), N.ptr(cbt2), N.ptr(scb2), N.ptr(b2), N.ptr(h),
+           M, Nout, K, float(fc1.threshold), N.ptr(ws), ws.numel(), N.stream())
+    return h.view(inp.shape[:-1] + (Nout,))
 
 
 _INT8_WS: dict = {}
