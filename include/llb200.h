@@ -528,6 +528,18 @@ LL_API int ll_moe_grouped_gemm_tc(const void* a, const void* w, const int32_t* o
                                   int n_experts, int N, int K, float limit, float alpha, void* c, int ldc, ll_stream stream);
 LL_API int ll_moe_tc_error(void);
 
+/* A step of 1 to 8 tokens (x [M][width] bf16, widths in multiples of 8) in three launches: the router as ll_moe_route_choice, the chosen experts' and the
+ * shared expert's first projections with their unit, the second projections with the combination; what ll_moe_route_choice, two
+ * ll_moe_grouped_gemm, the shared expert's dense layers and ll_moe_combine compute, in the same roundings.  w_gu [X][2 ff or ff][width],
+ * w_down [X][width][ff]; ws_in [2 shared_ff or shared_ff, then the gate's row if shared_gate][width], ws_down [width][shared_ff] (shared_ff 0:
+ * none); mode: 1, 2 the gated unit with and without the shift of the up branch, 3 relu^2.  scratch: ll_moe_step_scratch_bytes, of any
+ * contents, on a 16-byte boundary. */
+LL_API int ll_moe_step_supported(int M, int width, int ff, int shared_ff);
+LL_API size_t ll_moe_step_scratch_bytes(int M, int n_experts, int top, int ff, int shared_ff);
+LL_API int ll_moe_step(const void* x, const float* w_router, const float* bias, const float* correction, int score, float out_scale,
+                       int n_groups, int keep_groups, int group_top, const void* w_gu, const void* w_down, const void* ws_in, const void* ws_down,
+                       int M, int width, int n_experts, int top, int ff, int shared_ff, int shared_gate, int mode, float limit, float alpha,
+                       float shared_limit, void* out, void* scratch, ll_stream stream);
 /* out[m] = sum_k expert_w[m][k] * y[m * top + k]  (+ sigmoid(shared_gate[m * gate_ld]) * shared_y[m], when shared_y is
  * given; shared_gate NULL: the shared expert is added as it is). */
 LL_API int ll_moe_combine(const void* y, const float* expert_w, int top, const void* shared_y, int shared_ld,

@@ -21,10 +21,10 @@ FLAGS = [
 # The kernels a folder-loaded model family is served with (build_only): what a first run in a fresh checkout has to compile
 # for that family, and no more.  quant_pack carries the library's error plumbing and version.
 FAMILY_SOURCES = {
-    "Lepalorn": ["quant_pack", "decode_ops", "sampling", "residual_ops", "latent_attn", "moe_ops", "moe_gemm_tc"],
-    "Bededra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "window_attn", "moe_ops", "moe_gemm_tc"],
+    "Lepalorn": ["quant_pack", "decode_ops", "sampling", "residual_ops", "latent_attn", "moe_ops", "moe_gemm_tc", "moe_step"],
+    "Bededra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "window_attn", "moe_ops", "moe_gemm_tc", "moe_step"],
     "Tebodra": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "rotary_attn"],
-    "Livasun": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "rotary_attn", "moe_ops", "moe_gemm_tc"],
+    "Livasun": ["quant_pack", "residual_ops", "short_conv", "decay_scan", "decay_chunk", "rotary_attn", "moe_ops", "moe_gemm_tc", "moe_step"],
     "Zekonex": ["quant_pack", "residual_ops", "short_conv", "delta_rule", "delta_chunk", "rotary_attn", "latent_attn"],
     "Bumulix": ["quant_pack", "residual_ops", "rotary_attn", "latent_attn"],
 }

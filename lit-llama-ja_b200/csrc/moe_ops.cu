@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kern
                                                                int n_groups, int keep_groups, int group_top,
                                                                int32_t* __restrict__ expert_idx, float* __restrict__ expert_w,
                                                                int32_t* __restrict__ counts, int32_t* __restrict__ rank) {
+  pdl_launch_dependents();             // (a step of a few tokens: the shared expert's blocks start beside this one)
   extern __shared__ float sm[];
   float* xs = sm;                      // [RT_TOK][dim]
   float* zs = xs + RT_TOK * dim;       // [RT_TOK][X]
@@ -528,6 +529,65 @@ static int launch_grouped_f32(A... args) { return launch_grouped<float, TM, MODE
 template <int TM, int MODE, typename... A>
 static int launch_grouped_bf16(A... args) { return launch_grouped<__nv_bfloat16, TM, MODE>(args...); }
 
+static size_t route_smem(int dim, int n_experts, int score, int n_groups) {      // of one token
+  return sizeof(float) * ((size_t)dim + (score == SCORE_SIGMOID ? 2 : 1) * (size_t)n_experts + 2 * (size_t)n_groups);
+}
+static int route_check(int M, int dim, int n_experts, int top, int score, const float* correction, int n_groups, int keep_groups, int group_top) {
+  LL_CHECK_ARG(M >= 0 && dim > 0 && n_experts > 0 && top > 0 && top <= n_experts, "bad moe_route arguments");
+  LL_CHECK_ARG(score >= SCORE_CHOSEN && score <= SCORE_SIGMOID && (!correction || score == SCORE_SIGMOID) && (group_top == 1 || group_top == 2),
+               "moe_route: score %d, group score of %d", score, group_top);
+  LL_CHECK_ARG(n_groups >= 1 && keep_groups >= 1 && keep_groups <= n_groups && n_experts % n_groups == 0 &&
+                   top <= keep_groups * (n_experts / n_groups),
+               "moe_route: %d groups (keep %d) of %d experts cannot give %d choices", n_groups, keep_groups, n_experts, top);
+  if (M > 0 && 4 * route_smem(dim, n_experts, score, n_groups) > 200 * 1024) {
+    set_error("moe_route: width %d with %d experts does not fit shared memory", dim, n_experts);
+    return LL_ERR_UNSUPPORTED;
+  }
+  return LL_OK;
+}
+// The router: choices and weights of every token (counts: how many choices an expert has, added to what is there; rank: a choice's place).
+static int route_launch(const void* x, int dtype, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score,
+                        const float* correction, float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx,
+                        float* expert_w, int32_t* counts, int32_t* rank, cudaStream_t st) {
+  const size_t per_token = route_smem(dim, n_experts, score, n_groups);
+  const int sms = sm_count();
+  const int tok = M >= 8 * sms && 8 * per_token <= RT_WIDE_SMEM ? 8 : M <= sms ? 1 : 4;
+  const int blocks = (M + tok - 1) / tok;
+  const size_t smem = tok * per_token;
+#define LL_RT_TOK(T, TOK)                                                                                                            \
+  {                                                                                                                                  \
+    static PerDevice configured;                                                                                                     \
+    if (!configured) {                                                                                                               \
+      LL_CUDA(cudaFuncSetAttribute(moe_route_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));              \
+      configured.mark();                                                                                                             \
+    }                                                                                                                                \
+  }                                                                                                                                  \
+  moe_route_kernel<T, TOK><<<blocks, RT_THREADS, smem, st>>>((const T*)x, w_router, bias, M, dim, n_experts, top, score, correction,  \
+                                                             out_scale, n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank)
+#define LL_RT(T)                                                                                                                     \
+  if (tok == 8) { LL_RT_TOK(T, 8); } else if (tok == 4) { LL_RT_TOK(T, 4); } else { LL_RT_TOK(T, 1); }
+  if (dtype == LL_F32) {
+    LL_RT(float);
+  } else if (dtype == LL_BF16) {
+    LL_RT(__nv_bfloat16);
+  } else {
+    set_error("moe_route: unsupported dtype %d", dtype);
+    return LL_ERR_UNSUPPORTED;
+  }
+#undef LL_RT
+#undef LL_RT_TOK
+  LL_LAUNCH_OK("moe_route_kernel");
+  return LL_OK;
+}
+
+int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   cudaStream_t st) {
+  if (int r = route_check(M, dim, n_experts, top, score, correction, n_groups, keep_groups, group_top)) return r;
+  return route_launch(x, LL_BF16, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
+                      expert_w, counts, rank, st);
+}
+
 }  // namespace llb
 
 using namespace llb;
@@ -553,42 +613,13 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
                         int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank, int32_t* offsets, int32_t* perm,
                         ll_stream stream) {
   LL_CHECK_ARG(x && w_router && expert_idx && expert_w && counts && rank && offsets && perm, "moe_route: null pointer");
-  LL_CHECK_ARG(M >= 0 && dim > 0 && n_experts > 0 && top > 0 && top <= n_experts, "bad moe_route arguments");
-  LL_CHECK_ARG(score >= SCORE_CHOSEN && score <= SCORE_SIGMOID && (!correction || score == SCORE_SIGMOID) && (group_top == 1 || group_top == 2),
-               "moe_route: score %d, group score of %d", score, group_top);
-  LL_CHECK_ARG(n_groups >= 1 && keep_groups >= 1 && keep_groups <= n_groups && n_experts % n_groups == 0 &&
-                   top <= keep_groups * (n_experts / n_groups),
-               "moe_route: %d groups (keep %d) of %d experts cannot give %d choices", n_groups, keep_groups, n_experts, top);
-  if (M == 0) return LL_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t per_token =
-      sizeof(float) * ((size_t)dim + (score == SCORE_SIGMOID ? 2 : 1) * (size_t)n_experts + 2 * (size_t)n_groups);
-  if (4 * per_token > 200 * 1024) {
-    set_error("moe_route: width %d with %d experts does not fit shared memory", dim, n_experts);
-    return LL_ERR_UNSUPPORTED;
-  }
+  if (int r = route_check(M, dim, n_experts, top, score, correction, n_groups, keep_groups, group_top)) return r;
+  if (M == 0) return LL_OK;
   LL_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * n_experts, st));
-  const int sms = sm_count();
-  const int tok = M >= 8 * sms && 8 * per_token <= RT_WIDE_SMEM ? 8 : M <= sms ? 1 : 4;
-  const int blocks = (M + tok - 1) / tok;
-  const size_t smem = tok * per_token;
-#define LL_RT_TOK(T, TOK)                                                                                                            \
-  LL_CUDA(cudaFuncSetAttribute(moe_route_kernel<T, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));                  \
-  moe_route_kernel<T, TOK><<<blocks, RT_THREADS, smem, st>>>((const T*)x, w_router, bias, M, dim, n_experts, top, score, correction,  \
-                                                             out_scale, n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank)
-#define LL_RT(T)                                                                                                                     \
-  if (tok == 8) { LL_RT_TOK(T, 8); } else if (tok == 4) { LL_RT_TOK(T, 4); } else { LL_RT_TOK(T, 1); }
-  if (dtype == LL_F32) {
-    LL_RT(float);
-  } else if (dtype == LL_BF16) {
-    LL_RT(__nv_bfloat16);
-  } else {
-    set_error("moe_route: unsupported dtype %d", dtype);
-    return LL_ERR_UNSUPPORTED;
-  }
-#undef LL_RT
-#undef LL_RT_TOK
-  LL_LAUNCH_OK("moe_route_kernel");
+  if (int r = route_launch(x, dtype, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
+                           expert_w, counts, rank, st))
+    return r;
   const int n_pairs = M * top;
   moe_permute_kernel<<<(n_pairs + 255) / 256, 256, sizeof(int32_t) * (n_experts + 1), st>>>(expert_idx, rank, counts, n_pairs,
                                                                                           n_experts, offsets, perm);

@@ -21,6 +21,7 @@ GEMM's epilogue); small steps use the mma.sync / FMA kernels that take rows in p
 """
 from __future__ import annotations
 
+import functools
 import os
 from dataclasses import dataclass
 from typing import Optional
@@ -35,6 +36,19 @@ from .feed_forward import glu_unit, relu_squared_
 # the tcgen05 path: at least this many (token, choice) rows in the step, and on average per expert
 TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "1024"))
 TC_MIN_ROWS_PER_EXPERT = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "48"))
+
+
+STEP_MAX_TOKENS, STEP_SMALL_EXPERT = 8, 1 << 22       # tokens of a step; ff * width
+
+
+@functools.lru_cache(maxsize=1024)
+def _step_supported(M: int, width: int, ff: int, shared_ff: int) -> bool:
+    return bool(N.call_ret("ll_moe_step_supported", M, width, ff, shared_ff))
+
+
+@functools.lru_cache(maxsize=1024)
+def _step_scratch_bytes(M: int, experts: int, top: int, ff: int, shared_ff: int) -> int:
+    return N.call_ret("ll_moe_step_scratch_bytes", M, experts, top, ff, shared_ff)
 
 
 @dataclass
@@ -145,9 +159,34 @@ class MoE(nn.Module):
         return (x_act.dtype == torch.bfloat16 and s.width % 8 == 0 and s.ff % 8 == 0 and x_act.stride(0) % 8 == 0
                 and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts and N.has("ll_moe_grouped_gemm_tc"))
 
+    def _step(self, x_act: torch.Tensor, M: int) -> torch.Tensor:
+        """A few tokens in three launches (``ll_moe_step``)."""
+        s, p, dev = self.spec, self._parameters, x_act.device
+        sff = s.shared_ff or 0
+        out = torch.empty((M, s.width), dtype=x_act.dtype, device=dev)
+        scratch = torch.empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff), dtype=torch.uint8, device=dev)
+        N.call("ll_moe_step", N.ptr(x_act), N.ptr(p["w_router"]), N.ptr(self.b_router), N.ptr(self.correction), _SCORES[s.score],
+               float(s.weight_scale), s.groups, s.keep_groups if s.groups > 1 else 1, s.group_top, N.ptr(p["w_gu"]), N.ptr(p["w_down"]),
+               N.ptr(p["w_shared_in"]) if sff else None, N.ptr(p["w_shared_down"]) if sff else None, M, s.width, s.experts, s.top, s.ff, sff,
+               1 if s.shared_gate else 0, self.up_mode, float(s.limit), float(s.alpha), float(s.shared_limit if s.shared_limit is not None else s.limit),
+               N.ptr(out), N.ptr(scratch), N.stream())
+        return out
+
+    def _takes_step(self, x_act: torch.Tensor, M: int) -> bool:
+        """A few bf16 tokens.  A choice's weights are read for its token alone, where the grouped GEMM reads an expert's once for all of its
+        tokens: more than four tokens only where experts are small.  us, grouped / here: 32 experts of 2048 x 1024, four chosen, at 4, 6, 8
+        tokens 97 / 62, 99 / 78, 128 / 94; of 4096 x 2048 212 / 168, 229 / 247, 286 / 320."""
+        s = self.spec
+        most = STEP_MAX_TOKENS if s.ff * s.width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
+        return (1 <= M <= most and x_act.dtype == torch.bfloat16 and x_act.is_cuda and self._parameters["w_gu"].dtype == torch.bfloat16
+                and x_act.is_contiguous() and x_act.data_ptr() % 16 == 0
+                and N.has("ll_moe_step") and _step_supported(M, s.width, s.ff, s.shared_ff or 0))
+
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:
         s = self.spec
         M, dev, dtype = x_act.shape[0], x_act.device, x_act.dtype
+        if self._takes_step(x_act, M):
+            return self._step(x_act, M)
         dt, st = N.dtype_code(dtype), N.stream()
         _, w, offsets, perm = self.route(x_act)
         n = M * s.top
