@@ -751,6 +751,23 @@ LL_API int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, i
                                 int splits, int form, int maps, float diff_lambda, float diff_post, float eps, float* scratch,
                                 void* y, int y_stride, ll_stream stream);
 
+/* One token of 1 to 8 sequences (bf16) through a whole attention layer in one call: the input projection, the step's cache rows, attention and
+ * the output projection, in the roundings of the separate calls and dense layers.  x [B][width], w_in [n_in][width], w_o [width][heads * v_dim].
+ * Latent: w_uk [heads][nope][kv_rank], w_uv_t [heads][kv_rank][v_dim]; columns of the projection: queries first, gate_col0 (one logit a head;
+ * < 0: none), kv_col0; kv_norm NULL: the cache is another layer's and already holds the rows.  Softmax (one score map, queries and keys that
+ * turn or are normed): columns of queries, keys, values (< 0: the un-rotated keys) and gate (< 0: none).  Sizes in multiples of 8; scratch of
+ * the given bytes, any contents, 256-byte aligned. */
+LL_API size_t ll_latent_step_scratch_bytes(int B, int n_in, int heads, int kv_rank, int v_dim, int splits);
+LL_API int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm,
+                          float eps, const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim,
+                          int rot_dims, int v_dim, int kv_rank, int cache_len, int gate_col0, int kv_col0, int window, float scale, int splits,
+                          int weight_terms, void* out, void* scratch, ll_stream stream);
+LL_API size_t ll_softmax_step_scratch_bytes(int B, int n_in, int H, int dim, int vdim, int splits);
+LL_API int ll_softmax_step(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col,
+                           const float* q_norm, const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc,
+                           void* vc, const float* sink, const float* slopes, float scale, float softcap, int B, int width, int H, int G, int dim,
+                           int vdim, int window, int chunk, int ring, int splits, int form, void* out, void* scratch, ll_stream stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -12,6 +12,7 @@
 // part; the (cos, sin) table is [positions][rot_dims / 2][2] fp32.  Scores, softmax weights and sums
 // are fp32; T is the dtype of activations and of the cache.
 #include "attn_tc.cuh"
+#include "small_rows.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -722,6 +723,58 @@ int ll_latent_attn_terms(const void* q_lat, long long qs_h, long long qs_m, cons
     LL_LAUNCH_OK("latent_attn_combine_kernel");
   }
   return LL_OK;
+}
+
+// One token per sequence: what the layer holds between its launches.
+namespace {
+struct LatentStepScratch {
+  void *proj, *q_lat, *o_lat, *o;
+  float* split;
+  size_t total;
+};
+LatentStepScratch latent_step_carve(void* base, int B, int n_in, int heads, int kv_rank, int v_dim, int splits) {
+  LatentStepScratch s;
+  size_t o = 0;
+  auto take = [&](size_t b) { void* r = (uint8_t*)base + o; o += (b + 255) & ~(size_t)255; return r; };
+  s.proj = take((size_t)B * n_in * 2);
+  s.q_lat = take((size_t)B * heads * kv_rank * 2);
+  s.o_lat = take((size_t)B * heads * kv_rank * 2);
+  s.o = take((size_t)B * heads * v_dim * 2);
+  s.split = (float*)take(ll_latent_attn_scratch_bytes(B, heads, kv_rank, splits));
+  s.total = o;
+  return s;
+}
+}  // namespace
+
+size_t ll_latent_step_scratch_bytes(int B, int n_in, int heads, int kv_rank, int v_dim, int splits) {
+  return latent_step_carve(nullptr, B, n_in, heads, kv_rank, v_dim, splits).total;
+}
+
+int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm, float eps,
+                   const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim, int rot_dims, int v_dim,
+                   int kv_rank, int cache_len, int gate_col0, int kv_col0, int window, float scale, int splits, int weight_terms, void* out,
+                   void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_in && w_uk && w_uv_t && w_o && rope && pos_ids && cache && out && scratch, "latent_step: null pointer");
+  LL_CHECK_ARG(heads > 0 && nope > 0 && kv_rank > 0 && v_dim > 0 && splits >= 1, "bad latent_step arguments");
+  if (B < 1 || B > SR_MAX || width % 8 != 0 || n_in % 8 != 0 || kv_rank % 8 != 0 || v_dim % 8 != 0 || kv_rank > 1024 || nope > 1024) {
+    set_error("latent_step takes 1 to %d sequences and sizes in multiples of 8 (B=%d width=%d rank=%d v=%d)", SR_MAX, B, width, kv_rank, v_dim);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_uk | (uintptr_t)w_uv_t | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0,
+               "latent_step: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const LatentStepScratch s = latent_step_carve(scratch, B, n_in, heads, kv_rank, v_dim, splits);
+  const long long lat_h = (long long)B * kv_rank, q_head = nope + rot_dim;
+  if (int r = small_linear(x, width, w_in, s.proj, n_in, B, n_in, width, st)) return r;
+  if (kv_norm != nullptr)
+    if (int r = ll_latent_kv_append(s.proj, LL_BF16, n_in, kv_col0, kv_norm, eps, rope, pos_ids, cache, B, 1, kv_rank, rot_dim, rot_dims, cache_len, stream))
+      return r;
+  if (int r = small_heads(s.proj, q_head, n_in, w_uk, s.q_lat, lat_h, kv_rank, heads, B, kv_rank, nope, st)) return r;
+  if (int r = ll_latent_attn_terms(s.q_lat, lat_h, kv_rank, s.proj, n_in, nope, (int)q_head, gate_col0, rope, pos_ids, cache, s.o_lat, lat_h, kv_rank,
+                                   LL_BF16, B, 1, heads, kv_rank, rot_dim, rot_dims, cache_len, window, scale, splits, weight_terms, s.split, stream))
+    return r;
+  if (int r = small_heads(s.o_lat, lat_h, kv_rank, w_uv_t, s.o, v_dim, (long long)heads * v_dim, heads, B, v_dim, kv_rank, st)) return r;
+  return small_linear(s.o, heads * v_dim, w_o, out, width, B, width, heads * v_dim, st);
 }
 
 int ll_latent_prompt_supported(int nope, int rot_dim, int v_dim, int kv_rank, int q_stride, int q_head_stride, int y_stride) {

@@ -9,7 +9,7 @@
 // copy rate.  The shared expert's blocks come first and do not wait for the router.
 // us a call (graphed), sorted and grouped with dense layers for the shared expert / here: that size at 1, 2, 4, 8 tokens 155 (69) / 32 (28),
 // 125 (73) / 40 (38), 97 (76) / 62 (59), 128 (113) / 94 (91).
-#include "common.cuh"
+#include "small_rows.cuh"
 
 namespace llb {
 
@@ -31,29 +31,10 @@ struct MsParams {
   float limit, alpha, slimit;
 };
 
-// 16 bytes of weights, read once (asm volatile: the loads stay together ahead of the sums; left to the compiler they went one by one)
-__device__ __forceinline__ uint4 ms_ld(const __nv_bfloat16* row, int piece) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(reinterpret_cast<const uint4*>(row) + piece));
-  return v;
-}
 __device__ __forceinline__ float ms_unit(float g, float u, const MsParams& p, float limit) {
   if (p.mode == 3) return fmaxf(u, 0.f) * fmaxf(u, 0.f);
   g = fminf(g, limit), u = fminf(fmaxf(u, -limit), limit);
   return g / (1.f + expf(-p.alpha * g)) * (u + (p.mode == 1 ? 1.f : 0.f));
-}
-__device__ __forceinline__ void ms_floats(const uint4& u, float (&x)[8]) {
-  x[0] = __uint_as_float(u.x << 16), x[1] = __uint_as_float(u.x & 0xffff0000u), x[2] = __uint_as_float(u.y << 16), x[3] = __uint_as_float(u.y & 0xffff0000u);
-  x[4] = __uint_as_float(u.z << 16), x[5] = __uint_as_float(u.z & 0xffff0000u), x[6] = __uint_as_float(u.w << 16), x[7] = __uint_as_float(u.w & 0xffff0000u);
-}
-// acc += the products of eight bf16 numbers with eight of x
-__device__ __forceinline__ void ms_dot(float& acc, const uint4& w, const float (&x)[8]) {
-  float f[8];
-  ms_floats(w, f);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc = fmaf(f[i], x[i], acc);
 }
 // This lane's part of the dot products of R rows with R vectors (or all with the first: SAME) of n numbers; U 16-byte loads of every row in
 // flight.  Past the end a lane takes the last piece again, times zero.
@@ -67,15 +48,17 @@ __device__ __forceinline__ void ms_rows(const __nv_bfloat16* const (&row)[R], co
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r) w[r][u] = ms_ld(row[r], min(i + 32 * u, pieces - 1));
+      for (int r = 0; r < R; ++r) w[r][u] = sr_ld(row[r], min(i + 32 * u, pieces - 1));
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool in = i + 32 * u < pieces;
       float xf[8];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        if (r == 0 || !SAME) ms_floats(in ? reinterpret_cast<const uint4*>(x[r])[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
-        ms_dot(part[r], w[r][u], xf);
+        if (r == 0 || !SAME) sr_floats(in ? reinterpret_cast<const uint4*>(x[r])[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
+        float wf[8];
+        sr_floats(w[r][u], wf);
+        sr_dot(part[r], wf, xf);
       }
     }
   }

@@ -19,6 +19,7 @@
 //             combined as a difference, o = a_0 - lambda * a_1, then divided by the root mean square of o over the head's
 //             values (eps inside the root) and multiplied by `post`; the gate, if any, follows.
 #include "attn_tc.cuh"
+#include "small_rows.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -1037,6 +1038,54 @@ int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, int gate
                                       chunk, ring, splits, dm, scratch, y, y_stride, st);
   set_error("softmax_attn: unsupported dtype %d", dtype);
   return LL_ERR_UNSUPPORTED;
+}
+
+namespace {
+struct SoftmaxStepScratch {
+  void *proj, *q, *y;
+  float* split;
+  size_t total;
+};
+SoftmaxStepScratch softmax_step_carve(void* base, int B, int n_in, int H, int dim, int vdim, int splits) {
+  SoftmaxStepScratch s;
+  size_t o = 0;
+  auto take = [&](size_t b) { void* r = (uint8_t*)base + o; o += (b + 255) & ~(size_t)255; return r; };
+  s.proj = take((size_t)B * n_in * 2);
+  s.q = take((size_t)B * H * dim * 2);
+  s.y = take((size_t)B * H * vdim * 2);
+  s.split = (float*)take(splits > 1 ? ll_softmax_attn_scratch_bytes(B, H, vdim, splits) : 0);
+  s.total = o;
+  return s;
+}
+}  // namespace
+
+size_t ll_softmax_step_scratch_bytes(int B, int n_in, int H, int dim, int vdim, int splits) {
+  return softmax_step_carve(nullptr, B, n_in, H, dim, vdim, splits).total;
+}
+
+int ll_softmax_step(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col, const float* q_norm,
+                    const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc, void* vc, const float* sink,
+                    const float* slopes, float scale, float softcap, int B, int width, int H, int G, int dim, int vdim, int window, int chunk, int ring,
+                    int splits, int form, void* out, void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_in && w_o && pos_ids && kc && vc && out && scratch, "softmax_step: null pointer");
+  LL_CHECK_ARG(H > 0 && G > 0 && dim > 0 && vdim > 0 && splits >= 1 && q_col >= 0 && k_col >= 0, "bad softmax_step arguments");
+  if (B < 1 || B > SR_MAX || width % 8 != 0 || n_in % 8 != 0 || (H * vdim) % 8 != 0) {
+    set_error("softmax_step takes 1 to %d sequences and widths in multiples of 8 (B=%d width=%d heads %d x %d)", SR_MAX, B, width, H, vdim);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0, "softmax_step: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const SoftmaxStepScratch s = softmax_step_carve(scratch, B, n_in, H, dim, vdim, splits);
+  const __nv_bfloat16* proj = (const __nv_bfloat16*)s.proj;
+  if (int r = small_linear(x, width, w_in, s.proj, n_in, B, n_in, width, st)) return r;
+  if (int r = ll_qk_rotary_append_maps(proj + q_col, n_in, proj + k_col, n_in, v_col >= 0 ? proj + v_col : nullptr, n_in, LL_BF16, q_norm, k_norm, eps, freq,
+                                       rot_dims, pos_ids, s.q, kc, vc, B, 1, H, G, dim, vdim, ring, 1, stream))
+    return r;
+  if (int r = ll_softmax_attn_rows(s.q, H * dim, gate_col >= 0 ? proj + gate_col : nullptr, gate_col >= 0 ? n_in : 0, kc, vc, LL_BF16, pos_ids, sink, slopes,
+                                   scale, softcap, B, 1, H, G, dim, vdim, window, chunk, ring, splits, form, 1, 0.f, 1.f, eps, splits > 1 ? s.split : nullptr,
+                                   s.y, H * vdim, stream))
+    return r;
+  return small_linear(s.y, H * vdim, w_o, out, width, B, width, H * vdim, st);
 }
 
 int ll_softmax_attn_biased(const void* q, int q_stride, const void* gate, int gate_stride, const void* kc, const void* vc, int dtype,

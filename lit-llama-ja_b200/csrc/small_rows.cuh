@@ -1,0 +1,159 @@
+// Products of a few rows (decoding: one or two) with bf16 weights that are read once, on CUDA cores: bound by the weights' way from memory, so what
+// counts is 16-byte loads in flight.  Two forms: weights [N][K] (a warp per output row), and weights [K][N] per head (partial sums over
+// k in a block).  Both start under the kernel before them and wait for it before they read anything.
+// One or two rows only: every weight meets every row's sums in registers, and from three rows on the conversions cost more than the loads.  Both
+// projections of an attention layer, us, here / the library's products: one row of width 2048 12.7 / 12.7, of 4096 21.7 / 27.3; four rows (when
+// this form still took them) 21.4 / 11.4 and 51.9 / 27.1.  Two rows of w a warp halve the warps in flight: 8.4 for the first projection against 5.5.
+#pragma once
+#include "common.cuh"
+
+namespace llb {
+namespace {
+
+constexpr int SR_MAX = 2, SR_THREADS = 256, SR_WARPS = SR_THREADS / 32;
+
+// 16 bytes of weights, read once (asm volatile: the loads stay together ahead of the sums; left to the compiler they went one by one)
+__device__ __forceinline__ uint4 sr_ld(const __nv_bfloat16* row, int piece) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(reinterpret_cast<const uint4*>(row) + piece));
+  return v;
+}
+__device__ __forceinline__ void sr_floats(const uint4& u, float (&x)[8]) {
+  x[0] = __uint_as_float(u.x << 16), x[1] = __uint_as_float(u.x & 0xffff0000u), x[2] = __uint_as_float(u.y << 16), x[3] = __uint_as_float(u.y & 0xffff0000u);
+  x[4] = __uint_as_float(u.z << 16), x[5] = __uint_as_float(u.z & 0xffff0000u), x[6] = __uint_as_float(u.w << 16), x[7] = __uint_as_float(u.w & 0xffff0000u);
+}
+// acc += the products of eight bf16 numbers with eight of x
+__device__ __forceinline__ void sr_dot(float& acc, const float (&w)[8], const float (&x)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc = fmaf(w[i], x[i], acc);
+}
+
+// y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; past the end of k a lane takes the last piece again,
+// times zero.  K, ldx multiples of 8, rows on 16-byte boundaries.
+template <int MT>
+__global__ void __launch_bounds__(SR_THREADS) small_linear_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ w,
+                                                                  __nv_bfloat16* __restrict__ y, int ldy, int N, int K) {
+  constexpr int U = 8;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int n = (int)blockIdx.x * SR_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31, pieces = K / 8;
+  if (n >= N) return;
+  const __nv_bfloat16* row = w + (size_t)n * K;
+  float acc[MT];
+#pragma unroll
+  for (int m = 0; m < MT; ++m) acc[m] = 0.f;
+  for (int i = lane; i < pieces; i += 32 * U) {
+    uint4 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u] = sr_ld(row, min(i + 32 * u, pieces - 1));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool in = i + 32 * u < pieces;
+      float wf[8];
+      sr_floats(q[u], wf);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        float xf[8];
+        sr_floats(in ? reinterpret_cast<const uint4*>(x + (size_t)m * ldx)[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
+        sr_dot(acc[m], wf, xf);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+    const float v = warp_sum(acc[m]);
+    if (lane == 0) y[(size_t)m * ldy + n] = __float2bfloat16_rn(v);
+  }
+}
+
+// y(h, m, n) = sum_k x(h, m, k) w[h][k][n]: a block takes 32 columns of a head, four threads side by side eight columns each, 64 of them one
+// k apart; their sums meet by shuffles and in shared memory.  N a multiple of 8 (K of any size), rows of w on 16-byte boundaries.
+template <int MT>
+__global__ void __launch_bounds__(SR_THREADS) small_heads_kernel(const __nv_bfloat16* __restrict__ x, long long xs_h, long long xs_m,
+                                                                 const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, long long ys_h,
+                                                                 long long ys_m, int M, int N, int K) {
+  extern __shared__ float sr_x[];                      // [MT][K]
+  __shared__ float part[SR_WARPS][MT][32];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int h = blockIdx.y, tid = threadIdx.x, n = (int)blockIdx.x * 32 + (tid & 3) * 8, kg = tid >> 2, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < MT * K; i += SR_THREADS) {
+    const int m = i / K, k = i - m * K;
+    sr_x[i] = m < M ? __bfloat162float(x[h * xs_h + m * xs_m + k]) : 0.f;
+  }
+  const __nv_bfloat16* wh = w + (size_t)h * K * N + min(n, N - 8);
+  float acc[MT][8];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[m][e] = 0.f;
+  constexpr int U = 8;
+  bool first = true;
+  for (int k0 = kg; k0 < K + kg; k0 += 64 * U) {       // (the same number of turns for every thread: a barrier lies in the first)
+    uint4 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u] = sr_ld(wh + (size_t)min(k0 + 64 * u, K - 1) * N, 0);
+    if (first) __syncthreads();
+    first = false;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 + 64 * u;
+      if (k >= K) break;
+      float wf[8];
+      sr_floats(q[u], wf);
+#pragma unroll
+      for (int m = 0; m < MT; ++m) {
+        const float xv = sr_x[m * K + k];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[m][e] = fmaf(xv, wf[e], acc[m][e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float v = acc[m][e];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < 4) part[warp][m][lane * 8 + e] = v;
+    }
+  __syncthreads();
+  for (int i = tid; i < MT * 32; i += SR_THREADS) {
+    const int m = i / 32, c = i & 31;
+    float v = 0.f;
+#pragma unroll
+    for (int z = 0; z < SR_WARPS; ++z) v += part[z][m][c];
+    if (m < M && (int)blockIdx.x * 32 + c < N) y[h * ys_h + m * ys_m + blockIdx.x * 32 + c] = __float2bfloat16_rn(v);
+  }
+}
+
+inline int small_linear(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, cudaStream_t st) {
+  typedef const __nv_bfloat16* B;
+  const dim3 grid((N + SR_WARPS - 1) / SR_WARPS);
+  if (M == 1)
+    LL_CUDA(launch(small_linear_kernel<1>, grid, dim3(SR_THREADS), 0, st, true, (B)x, ldx, (B)w, (__nv_bfloat16*)y, ldy, N, K));
+  else
+    LL_CUDA(launch(small_linear_kernel<2>, grid, dim3(SR_THREADS), 0, st, true, (B)x, ldx, (B)w, (__nv_bfloat16*)y, ldy, N, K));
+  LL_LAUNCH_OK("small_linear_kernel");
+  return LL_OK;
+}
+
+inline int small_heads(const void* x, long long xs_h, long long xs_m, const void* w, void* y, long long ys_h, long long ys_m, int H, int M, int N, int K,
+                       cudaStream_t st) {
+  typedef const __nv_bfloat16* B;
+  const dim3 grid((N + 31) / 32, H);
+#define LL_SH(MT)                                                                                                                               \
+  LL_CUDA(launch(small_heads_kernel<MT>, grid, dim3(SR_THREADS), sizeof(float) * MT * K, st, true, (B)x, xs_h, xs_m, (B)w, (__nv_bfloat16*)y, ys_h, \
+                 ys_m, M, N, K))
+  if (M == 1) LL_SH(1);
+  else LL_SH(2);
+#undef LL_SH
+  LL_LAUNCH_OK("small_heads_kernel");
+  return LL_OK;
+}
+
+}  // namespace
+}  // namespace llb

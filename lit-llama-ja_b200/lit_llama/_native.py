@@ -147,6 +147,11 @@ EXPORTS = {
     "ll_moe_gather_rows": ([vp, i32, vp, i32, i32, i32, vp, vp], C.c_int),
     "ll_moe_grouped_gemm_tc": ([vp, vp, vp, vp, i32, i32, i32, i32, i32, C.c_float, C.c_float, vp, i32, vp], C.c_int),
     "ll_moe_tc_error": ([], C.c_int),
+    "ll_latent_step_scratch_bytes": ([i32] * 6, sz_t),
+    "ll_latent_step": ([vp, vp, i32, vp, vp, vp, vp, C.c_float, vp, vp, vp] + [i32] * 12 + [C.c_float, i32, i32, vp, vp, vp], C.c_int),
+    "ll_softmax_step_scratch_bytes": ([i32] * 6, sz_t),
+    "ll_softmax_step": ([vp, vp, i32, vp, i32, i32, i32, i32, vp, vp, C.c_float, vp, i32, vp, vp, vp, vp, vp, C.c_float, C.c_float] + [i32] * 11
+                        + [vp, vp, vp], C.c_int),
     "ll_moe_step_supported": ([i32, i32, i32, i32], C.c_int),
     "ll_moe_step_scratch_bytes": ([i32, i32, i32, i32, i32], sz_t),
     "ll_moe_step": ([vp, vp, vp, vp, i32, C.c_float, i32, i32, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, C.c_float,

@@ -24,6 +24,7 @@ Variations, all parameters of the spec:
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass
 from typing import Optional
 
@@ -37,6 +38,17 @@ from .rotary import RotarySpec
 EXPAND_MIN_TOKENS = 16               # tokens a step appends from which its rows are expanded per head
 EXPAND_MAX_SLOTS_PER_TOKEN = 64      # expanded rows per such token
 EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
+
+
+# Sequences of a step that takes the layer's one call.  us a call, before and after: one token of width 2048 over 1024 of 2048 rows 88 -> 45, of 4096 over 300 104 -> 58, two sequences 102 -> 61; replayed as a graph 40.5 -> 33.2, 53.9 -> 51.2 and
+# 60.4 -> 55.4.
+# From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
+STEP_MAX_ROWS = 2
+
+
+@functools.lru_cache(maxsize=1024)
+def _step_scratch_bytes(B: int, n_in: int, heads: int, kv_rank: int, v_dim: int, splits: int) -> int:
+    return N.call_ret("ll_latent_step_scratch_bytes", B, n_in, heads, kv_rank, v_dim, splits)
 
 
 @dataclass
@@ -179,7 +191,28 @@ class LatentAttention(nn.Module):
                 splits: int = 1, end: Optional[int] = None) -> torch.Tensor:
         """x_act ``[B*T, width]`` -> ``[B*T, width]``; ``cache`` ``[B, S, row]`` is this layer's or its source's (already
         appended to by the source in this step).  ``end``: as in ``attend``."""
+        if T == 1 and self._takes_step(x_act, B, cache):
+            return self._step(x_act, B, pos_ids, rope, cache, splits)
         return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
+
+    def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor) -> bool:
+        """One bf16 token of one or two sequences, plain queries, at most a gate per head: the whole layer in one call."""
+        s, w = self.spec, self._parameters.get("w_in")
+        return (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
+                and x_act.dtype == w.dtype == cache.dtype == torch.bfloat16 and x_act.is_contiguous() and cache.is_contiguous()
+                and x_act.data_ptr() % 16 == 0 and (s.width | s.kv_rank | s.v_dim) % 8 == 0 and s.kv_rank <= 1024 and s.nope_dim <= 1024
+                and N.has("ll_latent_step"))
+
+    def _step(self, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
+        s, p = self.spec, self._parameters
+        n_in = p["w_in"].shape[0]
+        out = torch.empty((B, s.width), dtype=x_act.dtype, device=x_act.device)
+        scratch = torch.empty(_step_scratch_bytes(B, n_in, s.heads, s.kv_rank, s.v_dim, splits), dtype=torch.uint8, device=x_act.device)
+        N.call("ll_latent_step", N.ptr(x_act), N.ptr(p["w_in"]), n_in, N.ptr(p["w_uk"]), N.ptr(p["w_uv_t"]), N.ptr(p["w_o"]),
+               N.ptr(self.kv_norm) if self.owns_cache else None, float(s.eps), N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), B, s.width, s.heads, s.nope_dim,
+               s.rot_dim, s.rot_dims, s.v_dim, s.kv_rank, cache.shape[1], self.gate_col0 if s.gate == "head" else -1, self.kv_col0,
+               s.window if s.window is not None else 0, float(s.scale), splits, 2 if s.exact_weights else 1, N.ptr(out), N.ptr(scratch), N.stream())
+        return out
 
     def attend(self, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor,
                splits: int = 1, out: Optional[torch.Tensor] = None, end: Optional[int] = None) -> torch.Tensor:

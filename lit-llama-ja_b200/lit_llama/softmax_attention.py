@@ -34,6 +34,7 @@ Cache: ``[B, R, G * maps * dim]`` keys and ``[B, R, G * vdim]`` values, position
 """
 from __future__ import annotations
 
+import functools
 from dataclasses import dataclass, field
 from typing import List, Optional, Tuple
 
@@ -48,6 +49,17 @@ from .short_conv import ShortConv
 
 def pad8(n: int) -> int:
     return (n + 7) // 8 * 8
+
+
+# Sequences of a step that takes the layer's one call.  us a call, before and after: one token of width 2048 over 1000 keys 66 -> 39 (with the walk over the keys several at a time), two sequences 67 -> 43; replayed as a graph
+# 57 -> 32 and 59 -> 36.
+# From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
+STEP_MAX_ROWS = 2
+
+
+@functools.lru_cache(maxsize=1024)
+def _step_scratch_bytes(B: int, n_in: int, heads: int, dim: int, vdim: int, splits: int) -> int:
+    return N.call_ret("ll_softmax_step_scratch_bytes", B, n_in, heads, dim, vdim, splits)
 
 
 @dataclass
@@ -207,7 +219,29 @@ class SoftmaxAttention(nn.Module):
 
     def forward(self, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
                 form: int = 0) -> torch.Tensor:
+        if T == 1 and self._takes_step(u, B, caches):
+            return self._step(u, B, pos_ids, caches, splits, form)
         return F.linear(self.attend(F.linear(u, self.w_in), B, T, pos_ids, caches, conv_state, splits, form), self.w_o)
+
+    def _takes_step(self, u: torch.Tensor, B: int, caches) -> bool:
+        """One bf16 token of one or two sequences on a layer with its own ring, one score map, no short convolution and nothing prepared head by
+        head: the whole layer in one call."""
+        s, w = self.spec, self._parameters.get("w_in")
+        return (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and self.conv is None and s.maps == 1 and not s.by_head
+                and not self.plain_q and u.is_cuda and u.dtype == w.dtype == caches[0].dtype == torch.bfloat16 and u.is_contiguous()
+                and u.data_ptr() % 16 == 0 and (s.width | (s.heads * s.vdim)) % 8 == 0 and N.has("ll_softmax_step"))
+
+    def _step(self, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
+        s, p, c = self.spec, self._parameters, self.cols
+        kc, vc = caches
+        n_in = p["w_in"].shape[0]
+        out = torch.empty((B, s.width), dtype=u.dtype, device=u.device)
+        scratch = torch.empty(_step_scratch_bytes(B, n_in, s.heads, s.dim, s.vdim, splits), dtype=torch.uint8, device=u.device)
+        N.call("ll_softmax_step", N.ptr(u), N.ptr(p["w_in"]), n_in, N.ptr(p["w_o"]), c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1,
+               N.ptr(self.q_norm), N.ptr(self.k_norm), float(s.eps), N.ptr(self.freq), s.rotary.dims, N.ptr(pos_ids), N.ptr(kc), N.ptr(vc),
+               N.ptr(self.sink), N.ptr(self.slopes), float(s.scale), float(s.softcap), B, s.width, s.heads, s.kv_heads, s.dim, s.vdim, s.window or 0,
+               s.chunk or 0, kc.shape[1], splits, form, N.ptr(out), N.ptr(scratch), N.stream())
+        return out
 
     def attend(self, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
                form: int = 0, first_values: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
