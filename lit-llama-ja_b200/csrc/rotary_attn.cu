@@ -367,6 +367,45 @@ __device__ __forceinline__ void sa_load8<__nv_bfloat16>(const __nv_bfloat16* __r
   }
 }
 
+// Eight dimensions of a key or value row as they lie in memory, so that several rows can be on their way at once.
+template <typename T>
+struct SaRow;
+template <>
+struct SaRow<float> {
+  float v[8];
+  __device__ __forceinline__ void load(const float* __restrict__ row, int e0, int n, bool vec) { sa_load8<float>(row, e0, n, vec, v); }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o[i] = v[i];
+  }
+};
+template <>
+struct SaRow<__nv_bfloat16> {
+  uint4 v;
+  __device__ __forceinline__ void load(const __nv_bfloat16* __restrict__ row, int e0, int n, bool vec) {
+    if (vec && e0 + 8 <= n) {
+      v = *(const uint4*)(row + e0);
+    } else {
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = e0 + i < n ? (uint32_t)reinterpret_cast<const uint16_t*>(row)[e0 + i] : 0u;
+      v = make_uint4(w[0] | w[1] << 16, w[2] | w[3] << 16, w[4] | w[5] << 16, w[6] | w[7] << 16);
+    }
+  }
+  __device__ __forceinline__ void get(float (&o)[8]) const {
+    o[0] = bf16_bits_to_f32(v.x & 0xffffu), o[1] = bf16_bits_to_f32(v.x >> 16), o[2] = bf16_bits_to_f32(v.y & 0xffffu), o[3] = bf16_bits_to_f32(v.y >> 16);
+    o[4] = bf16_bits_to_f32(v.z & 0xffffu), o[5] = bf16_bits_to_f32(v.z >> 16), o[6] = bf16_bits_to_f32(v.w & 0xffffu), o[7] = bf16_bits_to_f32(v.w >> 16);
+  }
+};
+// Keys a group has on their way at once: what waits in registers stays within 64 of them.  One key at a time the walk is a chain that waits for
+// memory once a key; in us, before and after, 16 heads over 4 of 128 after 1000 positions with the layer's other kernels: one bf16 token without
+// splits 255 -> 95, in 16 ranges 30 -> 20, 8 sequences in 4 ranges 74 -> 34, one fp32 token 253 -> 115, 512 fp32 tokens 620 -> 520.
+template <typename T>
+constexpr int sa_keys(int r, int rv) {
+  const int regs = (r + rv) * (int)sizeof(T) * 2;
+  return regs <= 16 ? 4 : regs <= 32 ? 2 : 1;
+}
+
 __device__ __forceinline__ int sa_first_visible(int i, int window, int chunk) {
   int lo = 0;
   if (window > 0) lo = max(lo, i - window + 1);
@@ -410,35 +449,63 @@ __global__ void __launch_bounds__(SA_WARPS * 32) softmax_attn_kernel(
   const T* kbase = kc + ((size_t)b * ring * GK + gk) * dim;
   const T* vbase = vc + ((size_t)b * ring * G + g) * vdim;
   const unsigned gmask = 0xffu << (grp * 8);
-  for (int j = j0 + grp; j < j1; j += 4) {
-    const size_t slot = (size_t)(j % ring);
-    const T* krow = kbase + slot * GK * dim;
-    float s = 0.f;
+  // U keys at a time: their rows are asked for together, and the running maximum moves once for all of them.
+  constexpr int U = sa_keys<T>(R, RV);
+  for (int j = j0 + grp; j < j1; j += 4 * U) {
+    SaRow<T> kr[U][R], vr[U][RV];
+    float s[U];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      float kk[8];
-      sa_load8<T>(krow, r * 64 + sub * 8, dim, kvec, kk);
+    for (int u = 0; u < U; ++u) {                // past the range's end: the group's first row again, with no weight
+      const size_t slot = (size_t)((j + 4 * u < j1 ? j + 4 * u : j) % ring);
+      const T *krow = kbase + slot * GK * dim, *vrow = vbase + slot * G * vdim;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s = fmaf(qr[r][e], kk[e], s);
+      for (int r = 0; r < R; ++r) kr[u][r].load(krow, r * 64 + sub * 8, dim, kvec);
+#pragma unroll
+      for (int r = 0; r < RV; ++r) vr[u][r].load(vrow, r * 64 + sub * 8, vdim, vvec);
     }
-    s += __shfl_xor_sync(gmask, s, 1);          // the groups' trip counts differ: only the group's own lanes meet here
-    s += __shfl_xor_sync(gmask, s, 2);
-    s += __shfl_xor_sync(gmask, s, 4);
-    s *= scale;
-    if (slopes) s -= slope * (float)(i - j);
-    if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-    const float mn = fmaxf(mx, s);
-    const float corr = expf(mx - mn), p = expf(s - mn);
+    float mn = mx;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      s[u] = 0.f;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float kk[8];
+        kr[u][r].get(kk);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[u] = fmaf(qr[r][e], kk[e], s[u]);
+      }
+    }
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1)             // the groups' trip counts differ: only the group's own lanes meet here
+#pragma unroll
+      for (int u = 0; u < U; ++u) s[u] += __shfl_xor_sync(gmask, s[u], o);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      s[u] *= scale;
+      if (slopes) s[u] -= slope * (float)(i - j - 4 * u);
+      if (softcap > 0.f) s[u] = softcap * tanhf(s[u] * inv_cap);
+      if (j + 4 * u < j1) mn = fmaxf(mn, s[u]);
+    }
+    const float corr = expf(mx - mn);
     mx = mn;
-    l = l * corr + p;
-    const T* vrow = vbase + slot * G * vdim;
+    l *= corr;
 #pragma unroll
-    for (int r = 0; r < RV; ++r) {
-      float vv[8];
-      sa_load8<T>(vrow, r * 64 + sub * 8, vdim, vvec, vv);
+    for (int r = 0; r < RV; ++r)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(p, vv[e], acc[r][e] * corr);
-    }
+      for (int e = 0; e < 8; ++e) acc[r][e] *= corr;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (j + 4 * u < j1) {
+        const float p = expf(s[u] - mn);
+        l += p;
+#pragma unroll
+        for (int r = 0; r < RV; ++r) {
+          float vv[8];
+          vr[u][r].get(vv);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[r][e] = fmaf(p, vv[e], acc[r][e]);
+        }
+      }
   }
   // the four groups of the warp hold disjoint keys: merge them (lanes 8 and 16 apart hold the same dimensions).  The
   // trip counts differ between groups, so the shuffles wait until the whole warp is here.
