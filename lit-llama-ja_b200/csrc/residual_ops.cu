@@ -395,6 +395,8 @@ static int add_row_norm_launch(float* x, const void* a, float s, const float* a_
 // A part of y spans y_gs >= C / groups numbers (the rest is skipped), except with `stab`: then number C / groups of every
 // part is a normaliser's product nq and stab[m][part] a stabiliser mx, and the part is first divided by
 // max(|nq|, exp(-mx)) + 1e-6 (the read-out of a matrix memory with exponential gates).
+// Parts of up to 256 numbers stay in a lane's registers between the two sweeps, every load of theirs asked for at once (y's parts with a normaliser
+// beside them start on any number, so the loads are single ones).  2048 rows of 8 parts of 256 (+ 1): 17.5 -> 13.0 us.
 template <typename TA>
 __global__ void gated_group_norm_kernel(const float* __restrict__ y, int y_gs, const float* __restrict__ stab,
                                         const TA* __restrict__ gate, int gate_stride, const float* __restrict__ w, int w_shared,
@@ -405,8 +407,36 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, int y_gs, c
   for (int g = warp; g < groups; g += nw) {
     const float* yr = y + ((size_t)m * groups + g) * y_gs;
     const TA* gr = gate + (size_t)m * gate_stride + (size_t)g * gs;
+    float yv8[8], g8[8], w8[8];
+    const bool held = gs <= 256;
+    if (held) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int i = lane + 32 * e;
+        yv8[e] = i < gs ? yr[i] : 0.f;
+        g8[e] = i < gs ? dt<TA>::ld(gr, i) : 0.f;
+        w8[e] = i < gs ? w[w_shared ? i : g * gs + i] : 0.f;
+      }
+    }
     const float pre = stab ? 1.f / (fmaxf(fabsf(yr[gs]), expf(-stab[(size_t)m * groups + g])) + 1e-6f) : 1.f;
     float ss = 0.f;
+    if (held) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        yv8[e] *= pre;
+        g8[e] = (gate_sigmoid ? 1.f : g8[e]) / (1.f + expf(-g8[e]));
+        const float v = gate_first ? yv8[e] * g8[e] : yv8[e];
+        if (lane + 32 * e < gs) ss += v * v;
+      }
+      ss = warp_sum(ss);
+      const float k = 1.f / sqrtf(ss / (float)gs + eps);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float v = gate_first ? (yv8[e] * g8[e]) * k * w8[e] : yv8[e] * k * w8[e] * g8[e];
+        if (lane + 32 * e < gs) dt<TA>::st(out, (size_t)m * out_stride + (size_t)g * gs + lane + 32 * e, v);
+      }
+      continue;
+    }
     for (int i = lane; i < gs; i += 32) {
       float v = yr[i] * pre;
       if (gate_first) {
