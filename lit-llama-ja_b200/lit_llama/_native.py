@@ -314,6 +314,12 @@ def gemv(args: GemvArgs) -> None:
     check(_fn["ll_int4_gemv"](C.byref(args), stream()), "ll_int4_gemv")
 
 
+def step_rows(*tensors: torch.Tensor) -> bool:
+    """Whether the step's kernels can read these rows (dense, on 16-byte boundaries), and nothing that a gradient is wanted for is among them."""
+    grad = torch.is_grad_enabled()
+    return all(t.is_contiguous() and t.data_ptr() % 16 == 0 and not (grad and t.requires_grad) for t in tensors)
+
+
 def attn_scratch_bytes(B, n_head, hs, splits) -> int:
     return _fn["ll_decode_attn_scratch_bytes"](B, n_head, hs, splits)
 

@@ -200,8 +200,8 @@ class LatentAttention(nn.Module):
         s, w = self.spec, self._parameters.get("w_in")
         return (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
                 and x_act.dtype == w.dtype == cache.dtype == torch.bfloat16 and x_act.is_contiguous() and cache.is_contiguous()
-                and x_act.data_ptr() % 16 == 0 and (s.width | s.kv_rank | s.v_dim) % 8 == 0 and s.kv_rank <= 1024 and s.nope_dim <= 1024
-                and N.has("ll_latent_step"))
+                and x_act.shape == (B, s.width) and (s.width | s.kv_rank | s.v_dim | w.shape[0]) % 8 == 0 and s.kv_rank <= 1024
+                and s.nope_dim <= 1024 and N.step_rows(x_act, w, self.w_uk, self.w_uv_t, self.w_o) and N.has("ll_latent_step"))
 
     def _step(self, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
         s, p = self.spec, self._parameters

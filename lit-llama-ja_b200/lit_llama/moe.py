@@ -179,7 +179,7 @@ class MoE(nn.Module):
         s = self.spec
         most = STEP_MAX_TOKENS if s.ff * s.width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
         return (1 <= M <= most and x_act.dtype == torch.bfloat16 and x_act.is_cuda and self._parameters["w_gu"].dtype == torch.bfloat16
-                and x_act.is_contiguous() and x_act.data_ptr() % 16 == 0
+                and x_act.shape == (M, s.width) and x_act.is_contiguous() and x_act.data_ptr() % 16 == 0
                 and N.has("ll_moe_step") and _step_supported(M, s.width, s.ff, s.shared_ff or 0))
 
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:

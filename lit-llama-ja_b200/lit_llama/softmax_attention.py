@@ -229,7 +229,8 @@ class SoftmaxAttention(nn.Module):
         s, w = self.spec, self._parameters.get("w_in")
         return (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and self.conv is None and s.maps == 1 and not s.by_head
                 and not self.plain_q and u.is_cuda and u.dtype == w.dtype == caches[0].dtype == torch.bfloat16 and u.is_contiguous()
-                and u.data_ptr() % 16 == 0 and (s.width | (s.heads * s.vdim)) % 8 == 0 and N.has("ll_softmax_step"))
+                and u.shape == (B, s.width) and (s.width | (s.heads * s.vdim) | w.shape[0]) % 8 == 0 and N.step_rows(u, w, self.w_o)
+                and N.has("ll_softmax_step"))
 
     def _step(self, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
         s, p, c = self.spec, self._parameters, self.cols

@@ -43,6 +43,7 @@ def test_latent_step(B, width, heads, nope, rot, v, rank, window, past, gate, sp
     got = mix(x, B, 1, pos, rope, cache, splits)
     want = F.linear(mix.attend(F.linear(x, mix.w_in), B, 1, pos, rope, other, splits), mix.w_o)
     _close(got, want, [cache], [other])
+    assert not mix._takes_step(x[:, :-8].contiguous(), B, cache) and not mix._takes_step(x.unsqueeze(1), B, cache)
     assert not mix._takes_step(x.float(), B, cache) and not mix._takes_step(x.repeat(3, 1), 3, cache)
     assert not mix._takes_step(torch.empty((B, 2 * width), dtype=torch.bfloat16, device="cuda")[:, :width], B, cache) or B == 1
 
@@ -67,6 +68,7 @@ def test_softmax_step(B, width, heads, kv_heads, dim, window, chunk, past, cap, 
     got = mix(u, B, 1, pos, caches, None, splits)
     want = F.linear(mix.attend(F.linear(u, mix.w_in), B, 1, pos, others, None, splits), mix.w_o)
     _close(got, want, caches, others)
+    assert not mix._takes_step(u[:, :-8].contiguous(), B, caches) and not mix._takes_step(u.unsqueeze(1), B, caches)
     assert not mix._takes_step(u.float(), B, caches) and not mix._takes_step(u.repeat(3, 1), 3, caches)
 
 
