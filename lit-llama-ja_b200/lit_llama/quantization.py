@@ -178,10 +178,11 @@ class ColBlockQuantizedLinear(torch.nn.Module):
 
     def _rows_eligible(self, x) -> bool:
         """bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns: the kernels that read the checkpoint bytes."""
-        b = self._buffers
-        s, z, bias = b["scales"], b["zeros"], b["bias"]
-        return (self.bits == 4 and x.dtype == s.dtype == z.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)
-                and s.is_contiguous() and z.is_contiguous() and (b["quant_weight"].data_ptr() | x.data_ptr()) % 16 == 0
+        if self.bits != 4 or x.dtype != torch.bfloat16:
+            return False
+        s, z, bias = self.scales, self.zeros, self.bias          # (buffers, or what qlinear_4bit_weight was given)
+        return (s.dtype == z.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)
+                and s.is_contiguous() and z.is_contiguous() and (self.quant_weight.data_ptr() | x.data_ptr()) % 16 == 0
                 and _rows_supported(self.out_features, self.in_features, self.tile_cols))
 
     def _copy_eligible(self, x) -> bool:
