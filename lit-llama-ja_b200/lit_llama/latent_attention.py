@@ -196,12 +196,16 @@ class LatentAttention(nn.Module):
         return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
 
     def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor) -> bool:
-        """One bf16 token of one or two sequences, plain queries, at most a gate per head: the whole layer in one call."""
-        s, w = self.spec, self._parameters.get("w_in")
+        """One bf16 token of one or two sequences, plain queries, at most a gate per head: the whole layer in one call, if its weights are
+        what the layer was built with."""
+        s, p = self.spec, self._parameters
+        w = p.get("w_in")
         return (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
-                and x_act.dtype == w.dtype == cache.dtype == torch.bfloat16 and x_act.is_contiguous() and cache.is_contiguous()
-                and x_act.shape == (B, s.width) and (s.width | s.kv_rank | s.v_dim | w.shape[0]) % 8 == 0 and s.kv_rank <= 1024
-                and s.nope_dim <= 1024 and N.step_rows(x_act, w, self.w_uk, self.w_uv_t, self.w_o) and N.has("ll_latent_step"))
+                and x_act.dtype == cache.dtype == torch.bfloat16 and cache.is_contiguous() and cache.device == x_act.device
+                and x_act.shape == (B, s.width) and w.shape[0] >= self.n_in and (s.width | s.kv_rank | s.v_dim | w.shape[0]) % 8 == 0
+                and s.kv_rank <= 1024 and s.nope_dim <= 1024 and N.has("ll_latent_step")
+                and N.step_rows(x_act, (w, (w.shape[0], s.width)), (p.get("w_uk"), (s.heads, s.nope_dim, s.kv_rank)),
+                                (p.get("w_uv_t"), (s.heads, s.kv_rank, s.v_dim)), (p.get("w_o"), (s.width, s.heads * s.v_dim))))
 
     def _step(self, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
         s, p = self.spec, self._parameters

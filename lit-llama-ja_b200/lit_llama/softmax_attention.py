@@ -225,12 +225,14 @@ class SoftmaxAttention(nn.Module):
 
     def _takes_step(self, u: torch.Tensor, B: int, caches) -> bool:
         """One bf16 token of one or two sequences on a layer with its own ring, one score map, no short convolution and nothing prepared head by
-        head: the whole layer in one call."""
-        s, w = self.spec, self._parameters.get("w_in")
+        head: the whole layer in one call, if its weights are what the layer was built with."""
+        s, p = self.spec, self._parameters
+        w = p.get("w_in")
         return (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and self.conv is None and s.maps == 1 and not s.by_head
-                and not self.plain_q and u.is_cuda and u.dtype == w.dtype == caches[0].dtype == torch.bfloat16 and u.is_contiguous()
-                and u.shape == (B, s.width) and (s.width | (s.heads * s.vdim) | w.shape[0]) % 8 == 0 and N.step_rows(u, w, self.w_o)
-                and N.has("ll_softmax_step"))
+                and not self.plain_q and u.is_cuda and u.dtype == caches[0].dtype == caches[1].dtype == torch.bfloat16
+                and caches[0].device == caches[1].device == u.device and u.shape == (B, s.width) and w.shape[0] >= self.n_in
+                and (s.width | (s.heads * s.vdim) | w.shape[0]) % 8 == 0 and N.has("ll_softmax_step")
+                and N.step_rows(u, (w, (w.shape[0], s.width)), (p.get("w_o"), (s.width, s.heads * s.vdim))))
 
     def _step(self, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
         s, p, c = self.spec, self._parameters, self.cols

@@ -88,3 +88,87 @@ def test_projections_against_64_bits(M, width, heads, v):
     want, size = o @ mix.w_o.double().t(), o.abs() @ mix.w_o.double().abs().t()
     # o is rounded to bf16 (2^-9 of each term, 2^-8 beside the other neighbour), the output once more
     assert ((got - want).abs() <= size * 2.0 ** -8 + want.abs() * 2.0 ** -8 + 1e-6).all()
+
+
+def _latent(width=64, heads=2, nope=16, rot=8, v=24, rank=40):
+    from lit_llama.latent_attention import LatentAttention, LatentAttentionSpec
+
+    spec = LatentAttentionSpec(width=width, heads=heads, nope_dim=nope, rot_dim=rot, v_dim=v, kv_rank=rank, window=None, scale=(nope + rot) ** -0.5)
+    mix = _fill(LatentAttention(spec, torch.bfloat16, "cuda"), 3)
+    args = dict(B=1, T=1, pos_ids=torch.tensor([4], dtype=torch.int32, device="cuda"), rope=spec.rope_table(8, "cuda"))
+    return mix, args, lambda: torch.zeros((1, 8, rank + rot), dtype=torch.bfloat16, device="cuda")
+
+
+def _softmax(width=64, heads=4, kv_heads=2, dim=16):
+    from lit_llama.rotary import RotarySpec
+    from lit_llama.softmax_attention import SoftmaxAttention, SoftmaxAttentionSpec
+
+    spec = SoftmaxAttentionSpec(width=width, heads=heads, kv_heads=kv_heads, dim=dim, vdim=dim, scale=dim ** -0.5, eps=1e-5, rotary=RotarySpec(dim // 2))
+    mix = _fill(SoftmaxAttention(spec, torch.bfloat16, "cuda"), 4)
+    args = dict(B=1, T=1, pos_ids=torch.tensor([4], dtype=torch.int32, device="cuda"))
+    return mix, args, lambda: [torch.zeros((1, 8, kv_heads * dim), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+
+
+def _call(mix, x, args, held):
+    return mix(x, args["B"], args["T"], args["pos_ids"], args["rope"], held, 1) if "rope" in args else mix(x, args["B"], args["T"], args["pos_ids"], held, None, 1)
+
+
+LAYERS = [(_latent, ("w_in", "w_uk", "w_uv_t", "w_o")), (_softmax, ("w_in", "w_o"))]
+
+
+@pytest.mark.parametrize("make,name", [(m, n) for m, names in LAYERS for n in names])
+@pytest.mark.parametrize("other", ["fp32", "fp16", "cpu"])
+def test_weights_of_another_kind_are_refused(make, name, other):
+    """The dense layers refuse weights of another dtype or on another device than the step's rows, and so does the layer."""
+    mix, args, held = make()
+    x = torch.ones((1, 64), dtype=torch.bfloat16, device="cuda")
+    assert mix._takes_step(x, 1, held())
+    w = getattr(mix, name)
+    new = w.detach().float() if other == "fp32" else w.detach().half() if other == "fp16" else w.detach().cpu()
+    setattr(mix, name, torch.nn.Parameter(new, requires_grad=False))
+    assert not mix._takes_step(x, 1, held())
+    with pytest.raises(RuntimeError):
+        _call(mix, x, args, held())
+
+
+@pytest.mark.parametrize("make,names", LAYERS)
+def test_weights_of_another_shape(make, names):
+    """A narrower output projection is refused where its rows do not fit, and serves where they do, as a dense layer of its own."""
+    mix, args, held = make()
+    x = torch.randn((1, 64), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda").to(torch.bfloat16)
+    whole = _call(mix, x, args, held())
+    w_o = mix.w_o.detach()
+    mix.w_o = torch.nn.Parameter(w_o[:40].clone(), requires_grad=False)
+    assert not mix._takes_step(x, 1, held())
+    part = _call(mix, x, args, held())
+    assert part.shape == (1, 40) and (part.double() - whole[:, :40].double()).norm() <= 0.01 * whole[:, :40].double().norm()
+    mix.w_o = torch.nn.Parameter(w_o[:, :-8].clone(), requires_grad=False)
+    assert not mix._takes_step(x, 1, held())
+    with pytest.raises(RuntimeError):
+        _call(mix, x, args, held())
+
+
+@pytest.mark.parametrize("make,name", [(m, n) for m, names in LAYERS for n in names])
+@pytest.mark.parametrize("how", ["shifted", "strided", "plain", "grad"])
+def test_weights_that_the_step_cannot_read(make, name, how):
+    """Weights off 16-byte boundaries or in strided rows, and tensors that are no parameters, go through the dense layers: the same numbers up to
+    the order of sums.  So does a weight that a gradient is wanted for."""
+    mix, args, held = make()
+    x = torch.randn((1, 64), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").to(torch.bfloat16)
+    want = _call(mix, x, args, held()).double()
+    w = getattr(mix, name).detach()
+    if how == "shifted":
+        new = torch.empty(w.numel() + 1, dtype=w.dtype, device="cuda")[1:].view(w.shape).copy_(w)
+    elif how == "strided":
+        new = torch.empty(w.shape[:-1] + (2 * w.shape[-1],), dtype=w.dtype, device="cuda")[..., : w.shape[-1]].copy_(w)
+    else:
+        new = w.clone()
+    if how == "plain":
+        delattr(mix, name)
+        object.__setattr__(mix, name, new)
+    else:
+        setattr(mix, name, torch.nn.Parameter(new, requires_grad=how == "grad"))
+    assert not mix._takes_step(x, 1, held())
+    got = _call(mix, x, args, held())
+    assert got.requires_grad == (how == "grad" and name in ("w_uv_t", "w_o"))
+    assert (got.detach().double() - want).norm() <= 0.01 * want.norm()
