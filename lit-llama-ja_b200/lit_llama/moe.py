@@ -165,7 +165,7 @@ class MoE(nn.Module):
         sff = s.shared_ff or 0
         out = torch.empty((M, s.width), dtype=x_act.dtype, device=dev)
         scratch = torch.empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff), dtype=torch.uint8, device=dev)
-        N.call("ll_moe_step", N.ptr(x_act), N.ptr(p["w_router"]), N.ptr(self.b_router), N.ptr(self.correction), _SCORES[s.score],
+        N.call("ll_moe_step", N.ptr(x_act), N.ptr(self.w_router), N.ptr(self.b_router), N.ptr(self.correction), _SCORES[s.score],
                float(s.weight_scale), s.groups, s.keep_groups if s.groups > 1 else 1, s.group_top, N.ptr(p["w_gu"]), N.ptr(p["w_down"]),
                N.ptr(p["w_shared_in"]) if sff else None, N.ptr(p["w_shared_down"]) if sff else None, M, s.width, s.experts, s.top, s.ff, sff,
                1 if s.shared_gate else 0, self.up_mode, float(s.limit), float(s.alpha), float(s.shared_limit if s.shared_limit is not None else s.limit),
@@ -178,9 +178,17 @@ class MoE(nn.Module):
         tokens 97 / 62, 99 / 78, 128 / 94; of 4096 x 2048 212 / 168, 229 / 247, 286 / 320."""
         s = self.spec
         most = STEP_MAX_TOKENS if s.ff * s.width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
-        return (1 <= M <= most and x_act.dtype == torch.bfloat16 and x_act.is_cuda and self._parameters["w_gu"].dtype == torch.bfloat16
-                and x_act.shape == (M, s.width) and x_act.is_contiguous() and x_act.data_ptr() % 16 == 0
-                and N.has("ll_moe_step") and _step_supported(M, s.width, s.ff, s.shared_ff or 0))
+        if not (1 <= M <= most and x_act.dtype == torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width) and N.has("ll_moe_step")
+                and _step_supported(M, s.width, s.ff, s.shared_ff or 0)):
+            return False
+        p = self._parameters
+        rows = 1 if s.unit == "relu2" else 2
+        weights = [(p.get("w_gu"), (s.experts, rows * s.ff, s.width)), (p.get("w_down"), (s.experts, s.width, s.ff))]
+        if s.shared_ff:
+            w = p.get("w_shared_in")
+            weights += [(w, (w.shape[0] if w is not None and w.shape[0] >= rows * s.shared_ff + (1 if s.shared_gate else 0) else 0, s.width)),
+                        (p.get("w_shared_down"), (s.width, s.shared_ff))]
+        return N.step_rows(x_act, *weights)
 
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:
         s = self.spec

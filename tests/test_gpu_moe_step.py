@@ -81,3 +81,41 @@ def test_route_of_a_module():
     x = torch.zeros((5, 4096), dtype=torch.bfloat16, device="cuda")
     assert wide._takes_step(x[:4], 4) and not wide._takes_step(x, 5)
     assert not _module(36, 4, 2, 64, 0, "glu", 1.0, True, "chosen", 2)._takes_step(torch.zeros((2, 36), dtype=torch.bfloat16, device="cuda"), 2)
+
+
+@pytest.mark.parametrize("name,how", [("w_gu", "shifted"), ("w_down", "shifted"), ("w_shared_in", "shifted"), ("w_shared_down", "shifted"),
+                                      ("w_shared_in", "strided"), ("w_shared_down", "strided"), ("w_down", "plain"), ("w_shared_in", "plain")])
+def test_weights_that_the_step_cannot_read(name, how):
+    """Weights off 16-byte boundaries, a shared expert's in strided rows and tensors that are no parameters take the grouped kernels and dense
+    layers: the same numbers up to rounding."""
+    mix = _module(256, 8, 2, 64, 32, "glu", 1.0, True, "chosen", 5)
+    x = torch.randn((3, 256), generator=torch.Generator(device="cuda").manual_seed(5), device="cuda").to(torch.bfloat16)
+    assert mix._takes_step(x, 3)
+    want = mix(x).double()
+    w = getattr(mix, name).detach()
+    if how == "shifted":
+        new = torch.empty(w.numel() + 1, dtype=w.dtype, device="cuda")[1:].view(w.shape).copy_(w)
+    elif how == "strided":
+        new = torch.empty(w.shape[:-1] + (2 * w.shape[-1],), dtype=w.dtype, device="cuda")[..., : w.shape[-1]].copy_(w)
+    else:
+        new = w.clone()
+    if how == "plain":
+        delattr(mix, name)
+        object.__setattr__(mix, name, new)
+    else:
+        setattr(mix, name, torch.nn.Parameter(new, requires_grad=False))
+    assert not mix._takes_step(x, 3)
+    assert (mix(x).double() - want).norm() <= 0.01 * want.norm()
+
+
+@pytest.mark.parametrize("name", ["w_shared_in", "w_shared_down"])
+@pytest.mark.parametrize("other", ["fp32", "cpu", "narrow"])
+def test_shared_weights_of_another_kind_are_refused(name, other):
+    """The dense layers refuse a shared expert of another dtype, on another device or of other widths, and so does the module."""
+    mix = _module(256, 8, 2, 64, 32, "glu", 1.0, True, "chosen", 6)
+    x = torch.ones((2, 256), dtype=torch.bfloat16, device="cuda")
+    w = getattr(mix, name).detach()
+    setattr(mix, name, torch.nn.Parameter(w.float() if other == "fp32" else w.cpu() if other == "cpu" else w[:, :-8].clone(), requires_grad=False))
+    assert not mix._takes_step(x, 2)
+    with pytest.raises(RuntimeError):
+        mix(x)
