@@ -172,3 +172,26 @@ def test_weights_that_the_step_cannot_read(make, name, how):
     got = _call(mix, x, args, held())
     assert got.requires_grad == (how == "grad" and name in ("w_uv_t", "w_o"))
     assert (got.detach().double() - want).norm() <= 0.01 * want.norm()
+
+
+def _same_kinds(a, b):
+    """Infinities of the same sign and no numbers in the same places, and numbers close to each other."""
+    return torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf()) and torch.equal(a[a.isinf()].sign(), b[b.isinf()].sign()) \
+        and bool(((a - b).abs()[a.isfinite()] <= 0.02 * b[b.isfinite()].abs().amax()).all())
+
+
+@pytest.mark.parametrize("width", [64, 264, 2056])
+@pytest.mark.parametrize("make,gate_row", [(_latent, lambda m: m.gate_col0 + 1), (_softmax, lambda m: m.cols["g"] + 3)])
+def test_infinite_weights_at_the_end_of_a_row(make, gate_row, width):
+    """A row's last weights are infinite and its length fills no whole round of the warp's loads: sums are infinite, or no numbers, exactly where the
+    dense layers' are."""
+    mix, args, held = make(width=width)
+    x = torch.randn((1, width), generator=torch.Generator(device="cuda").manual_seed(width), device="cuda").to(torch.bfloat16)
+    with torch.no_grad():
+        mix.w_o[1, -1], mix.w_o[5, -3] = float("inf"), -float("inf")
+        mix.w_in[gate_row(mix), -2] = float("inf")
+    assert mix._takes_step(x, 1, held())
+    got = _call(mix, x, args, held()).double()
+    attend = (args["B"], args["T"], args["pos_ids"]) + ((args["rope"], held()) if "rope" in args else (held(),))
+    want = F.linear(mix.attend(F.linear(x, mix.w_in), *attend), mix.w_o).double()
+    assert want.isinf().any() and _same_kinds(got, want)

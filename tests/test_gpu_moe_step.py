@@ -119,3 +119,22 @@ def test_shared_weights_of_another_kind_are_refused(name, other):
     assert not mix._takes_step(x, 2)
     with pytest.raises(RuntimeError):
         mix(x)
+
+
+@pytest.mark.parametrize("width,ff,shared", [(72, 40, 24), (264, 1032, 16), (2048, 1024, 1536)])
+def test_infinite_weights_at_the_end_of_a_row(width, ff, shared):
+    """A row's last weights are infinite: outputs are infinite where the grouped kernels' are, and no numbers nowhere else either."""
+    mix = _module(width, 4, 2, ff, shared, "glu", 1.0, True, "chosen", 7)
+    with torch.no_grad():
+        mix.w_down[:, 1, -1], mix.w_down[:, 6, -2] = float("inf"), -float("inf")
+        mix.w_shared_down[3, -1] = float("inf")
+        mix.w_shared_in[mix.shared_cols, -1] = float("inf")
+    x = torch.randn((2, width), generator=torch.Generator(device="cuda").manual_seed(7), device="cuda").to(torch.bfloat16)
+    assert mix._takes_step(x, 2)
+    got = mix(x).double()
+    mix._takes_step = lambda *a: False
+    want = mix(x).double()
+    assert want.isinf().any() and torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()].sign(), want[want.isinf()].sign())
+    ok = want.isfinite()
+    assert (got[ok] - want[ok]).norm() <= 0.01 * want[ok].norm()
