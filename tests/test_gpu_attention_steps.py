@@ -190,6 +190,7 @@ def test_infinite_weights_at_the_end_of_a_row(make, gate_row, width):
     with torch.no_grad():
         mix.w_o[1, -1], mix.w_o[5, -3] = float("inf"), -float("inf")
         mix.w_in[gate_row(mix), -2] = float("inf")
+        x[0, -2] = 1.0                       # (that gate is open)
     assert mix._takes_step(x, 1, held())
     got = _call(mix, x, args, held()).double()
     attend = (args["B"], args["T"], args["pos_ids"]) + ((args["rope"], held()) if "rope" in args else (held(),))
