@@ -314,22 +314,28 @@ def gemv(args: GemvArgs) -> None:
     check(_fn["ll_int4_gemv"](C.byref(args), stream()), "ll_int4_gemv")
 
 
-def step_rows(x: torch.Tensor, *weights) -> bool:
-    """Whether a kernel can do the dense layers' work on the rows ``x`` with these (weight, shape) pairs: plain tensors, as a dense layer takes
-    them (of x's dtype, on x's device, of the layer's shape), in rows that it can read (dense, on 16-byte boundaries), and nothing that a
-    gradient is wanted for among them.  Otherwise the step goes through the dense layers, which take more and refuse the rest."""
-    grad = torch.is_grad_enabled()
-    if type(x) not in _PLAIN or not x.is_contiguous() or x.data_ptr() % 16 or (grad and x.requires_grad):
-        return False
-    dtype, dev = x.dtype, x.device
-    for t, shape in weights:
-        if (type(t) not in _PLAIN or t.dtype != dtype or t.device != dev or t.shape != shape or not t.is_contiguous() or t.data_ptr() % 16
-                or (grad and t.requires_grad)):
-            return False
-    return True
-
-
 _PLAIN = (torch.nn.Parameter, torch.Tensor)
+
+
+def step_rows(x: torch.Tensor, weights, shapes):
+    """The addresses of the rows ``x`` and of the weights, if a kernel can do the dense layers' work with them: plain tensors, as a dense layer
+    takes them (of x's dtype, on x's device, of the layer's shape), in rows that it can read (dense, on 16-byte boundaries), and nothing that a
+    gradient is wanted for among them.  Otherwise ``None``: the step goes through the dense layers, which take more and refuse the rest."""
+    if type(x) not in _PLAIN or not x.is_contiguous():
+        return None
+    grad, dtype, dev, a = torch.is_grad_enabled(), x.dtype, x.get_device(), x.data_ptr()
+    if a & 15 or (grad and x.requires_grad):
+        return None
+    at = [a]
+    for t, shape in zip(weights, shapes):
+        if (type(t) not in _PLAIN or t.dtype is not dtype or t.shape != shape or t.get_device() != dev or not t.is_contiguous()
+                or (grad and t.requires_grad)):
+            return None
+        a = t.data_ptr()
+        if a & 15:
+            return None
+        at.append(a)
+    return at
 
 
 def attn_scratch_bytes(B, n_head, hs, splits) -> int:

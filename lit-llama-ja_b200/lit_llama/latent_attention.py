@@ -191,31 +191,39 @@ class LatentAttention(nn.Module):
                 splits: int = 1, end: Optional[int] = None) -> torch.Tensor:
         """x_act ``[B*T, width]`` -> ``[B*T, width]``; ``cache`` ``[B, S, row]`` is this layer's or its source's (already
         appended to by the source in this step).  ``end``: as in ``attend``."""
-        if T == 1 and self._takes_step(x_act, B, cache):
-            return self._step(x_act, B, pos_ids, rope, cache, splits)
+        if T == 1:
+            at = self._takes_step(x_act, B, cache)
+            if at:
+                return self._step(at, x_act, B, pos_ids, rope, cache, splits)
         return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
 
-    def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor) -> bool:
+    def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor):
         """One bf16 token of one or two sequences, plain queries, at most a gate per head: the whole layer in one call, if its weights are
-        what the layer was built with."""
+        what the layer was built with.  Their addresses, or ``None``."""
         s, p = self.spec, self._parameters
         w = p.get("w_in")
-        return (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
-                and x_act.dtype == cache.dtype == torch.bfloat16 and cache.is_contiguous() and cache.device == x_act.device
-                and x_act.shape == (B, s.width) and w.shape[0] >= self.n_in and (s.width | s.kv_rank | s.v_dim | w.shape[0]) % 8 == 0
-                and s.kv_rank <= 1024 and s.nope_dim <= 1024 and N.has("ll_latent_step")
-                and N.step_rows(x_act, (w, (w.shape[0], s.width)), (p.get("w_uk"), (s.heads, s.nope_dim, s.kv_rank)),
-                                (p.get("w_uv_t"), (s.heads, s.kv_rank, s.v_dim)), (p.get("w_o"), (s.width, s.heads * s.v_dim))))
+        if not (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
+                and x_act.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and cache.is_contiguous()
+                and cache.get_device() == x_act.get_device() and x_act.shape == (B, s.width) and s.kv_rank <= 1024 and s.nope_dim <= 1024
+                and N.has("ll_latent_step")):
+            return None
+        n_in = w.shape[0]
+        if n_in < self.n_in or (s.width | s.kv_rank | s.v_dim | n_in) % 8:
+            return None
+        return N.step_rows(x_act, (w, p.get("w_uk"), p.get("w_uv_t"), p.get("w_o")),
+                           ((n_in, s.width), (s.heads, s.nope_dim, s.kv_rank), (s.heads, s.kv_rank, s.v_dim), (s.width, s.heads * s.v_dim)))
 
-    def _step(self, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
+    def _step(self, at, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
         s, p = self.spec, self._parameters
+        x, w_in, w_uk, w_uv_t, w_o = at
         n_in = p["w_in"].shape[0]
-        out = torch.empty((B, s.width), dtype=x_act.dtype, device=x_act.device)
-        scratch = torch.empty(_step_scratch_bytes(B, n_in, s.heads, s.kv_rank, s.v_dim, splits), dtype=torch.uint8, device=x_act.device)
-        N.call("ll_latent_step", N.ptr(x_act), N.ptr(p["w_in"]), n_in, N.ptr(p["w_uk"]), N.ptr(p["w_uv_t"]), N.ptr(p["w_o"]),
-               N.ptr(self.kv_norm) if self.owns_cache else None, float(s.eps), N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), B, s.width, s.heads, s.nope_dim,
-               s.rot_dim, s.rot_dims, s.v_dim, s.kv_rank, cache.shape[1], self.gate_col0 if s.gate == "head" else -1, self.kv_col0,
-               s.window if s.window is not None else 0, float(s.scale), splits, 2 if s.exact_weights else 1, N.ptr(out), N.ptr(scratch), N.stream())
+        norm = None if not self.owns_cache else p["kv_norm"] if "kv_norm" in p else self.kv_norm
+        out = torch.empty_like(x_act)
+        scratch = x_act.new_empty(_step_scratch_bytes(B, n_in, s.heads, s.kv_rank, s.v_dim, splits) // 2)          # (whole pieces of 128 bytes or more)
+        N.call("ll_latent_step", x, w_in, n_in, w_uk, w_uv_t, w_o, N.ptr(norm), float(s.eps), N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), B, s.width,
+               s.heads, s.nope_dim, s.rot_dim, s.rot_dims, s.v_dim, s.kv_rank, cache.shape[1], self.gate_col0 if s.gate == "head" else -1,
+               self.kv_col0, s.window if s.window is not None else 0, float(s.scale), splits, 2 if s.exact_weights else 1, N.ptr(out),
+               N.ptr(scratch), N.stream())
         return out
 
     def attend(self, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor,

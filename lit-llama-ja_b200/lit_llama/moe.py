@@ -159,42 +159,46 @@ class MoE(nn.Module):
         return (x_act.dtype == torch.bfloat16 and s.width % 8 == 0 and s.ff % 8 == 0 and x_act.stride(0) % 8 == 0
                 and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts and N.has("ll_moe_grouped_gemm_tc"))
 
-    def _step(self, x_act: torch.Tensor, M: int) -> torch.Tensor:
+    def _step(self, at, x_act: torch.Tensor, M: int) -> torch.Tensor:
         """A few tokens in three launches (``ll_moe_step``)."""
-        s, p, dev = self.spec, self._parameters, x_act.device
+        s, p = self.spec, self._parameters
         sff = s.shared_ff or 0
-        out = torch.empty((M, s.width), dtype=x_act.dtype, device=dev)
-        scratch = torch.empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff), dtype=torch.uint8, device=dev)
-        N.call("ll_moe_step", N.ptr(x_act), N.ptr(self.w_router), N.ptr(self.b_router), N.ptr(self.correction), _SCORES[s.score],
-               float(s.weight_scale), s.groups, s.keep_groups if s.groups > 1 else 1, s.group_top, N.ptr(p["w_gu"]), N.ptr(p["w_down"]),
-               N.ptr(p["w_shared_in"]) if sff else None, N.ptr(p["w_shared_down"]) if sff else None, M, s.width, s.experts, s.top, s.ff, sff,
+        x, w_gu, w_down, ws_in, ws_down = at if sff else (*at, None, None)
+        router, bias, correction = (p[n] if n in p else getattr(self, n) for n in ("w_router", "b_router", "correction"))
+        out = torch.empty_like(x_act)
+        scratch = x_act.new_empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff) // 2)          # (whole pieces of 128 bytes or more)
+        N.call("ll_moe_step", x, N.ptr(router), N.ptr(bias), N.ptr(correction), _SCORES[s.score], float(s.weight_scale), s.groups,
+               s.keep_groups if s.groups > 1 else 1, s.group_top, w_gu, w_down, ws_in, ws_down, M, s.width, s.experts, s.top, s.ff, sff,
                1 if s.shared_gate else 0, self.up_mode, float(s.limit), float(s.alpha), float(s.shared_limit if s.shared_limit is not None else s.limit),
                N.ptr(out), N.ptr(scratch), N.stream())
         return out
 
-    def _takes_step(self, x_act: torch.Tensor, M: int) -> bool:
-        """A few bf16 tokens.  A choice's weights are read for its token alone, where the grouped GEMM reads an expert's once for all of its
+    def _takes_step(self, x_act: torch.Tensor, M: int):
+        """A few bf16 tokens, and weights that are what the module was built with: their addresses, or ``None``.  A choice's weights are read for its token alone, where the grouped GEMM reads an expert's once for all of its
         tokens: more than four tokens only where experts are small.  us, grouped / here: 32 experts of 2048 x 1024, four chosen, at 4, 6, 8
         tokens 97 / 62, 99 / 78, 128 / 94; of 4096 x 2048 212 / 168, 229 / 247, 286 / 320."""
         s = self.spec
         most = STEP_MAX_TOKENS if s.ff * s.width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
-        if not (1 <= M <= most and x_act.dtype == torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width) and N.has("ll_moe_step")
+        if not (1 <= M <= most and x_act.dtype is torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width) and N.has("ll_moe_step")
                 and _step_supported(M, s.width, s.ff, s.shared_ff or 0)):
-            return False
+            return None
         p = self._parameters
-        rows = 1 if s.unit == "relu2" else 2
-        weights = [(p.get("w_gu"), (s.experts, rows * s.ff, s.width)), (p.get("w_down"), (s.experts, s.width, s.ff))]
-        if s.shared_ff:
-            w = p.get("w_shared_in")
-            weights += [(w, (w.shape[0] if w is not None and w.shape[0] >= rows * s.shared_ff + (1 if s.shared_gate else 0) else 0, s.width)),
-                        (p.get("w_shared_down"), (s.width, s.shared_ff))]
-        return N.step_rows(x_act, *weights)
+        branches = 1 if s.unit == "relu2" else 2
+        up, down = (s.experts, branches * s.ff, s.width), (s.experts, s.width, s.ff)
+        if not s.shared_ff:
+            return N.step_rows(x_act, (p.get("w_gu"), p.get("w_down")), (up, down))
+        w = p.get("w_shared_in")
+        if w is None or w.shape[0] < branches * s.shared_ff + (1 if s.shared_gate else 0):
+            return None
+        return N.step_rows(x_act, (p.get("w_gu"), p.get("w_down"), w, p.get("w_shared_down")),
+                           (up, down, (w.shape[0], s.width), (s.width, s.shared_ff)))
 
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:
         s = self.spec
         M, dev, dtype = x_act.shape[0], x_act.device, x_act.dtype
-        if self._takes_step(x_act, M):
-            return self._step(x_act, M)
+        at = self._takes_step(x_act, M)
+        if at:
+            return self._step(at, x_act, M)
         dt, st = N.dtype_code(dtype), N.stream()
         _, w, offsets, perm = self.route(x_act)
         n = M * s.top

@@ -219,31 +219,41 @@ class SoftmaxAttention(nn.Module):
 
     def forward(self, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
                 form: int = 0) -> torch.Tensor:
-        if T == 1 and self._takes_step(u, B, caches):
-            return self._step(u, B, pos_ids, caches, splits, form)
+        if T == 1:
+            at = self._takes_step(u, B, caches)
+            if at:
+                return self._step(at, u, B, pos_ids, caches, splits, form)
         return F.linear(self.attend(F.linear(u, self.w_in), B, T, pos_ids, caches, conv_state, splits, form), self.w_o)
 
-    def _takes_step(self, u: torch.Tensor, B: int, caches) -> bool:
+    def _takes_step(self, u: torch.Tensor, B: int, caches):
         """One bf16 token of one or two sequences on a layer with its own ring, one score map, no short convolution and nothing prepared head by
-        head: the whole layer in one call, if its weights are what the layer was built with."""
+        head: the whole layer in one call, if its weights are what the layer was built with.  Their addresses, or ``None``."""
         s, p = self.spec, self._parameters
         w = p.get("w_in")
-        return (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and self.conv is None and s.maps == 1 and not s.by_head
-                and not self.plain_q and u.is_cuda and u.dtype == caches[0].dtype == caches[1].dtype == torch.bfloat16
-                and caches[0].device == caches[1].device == u.device and u.shape == (B, s.width) and w.shape[0] >= self.n_in
-                and (s.width | (s.heads * s.vdim) | w.shape[0]) % 8 == 0 and N.has("ll_softmax_step")
-                and N.step_rows(u, (w, (w.shape[0], s.width)), (p.get("w_o"), (s.width, s.heads * s.vdim))))
+        if not (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and s.conv_taps == 0 and s.maps == 1 and not s.by_head
+                and not self.plain_q and u.is_cuda and u.dtype is torch.bfloat16 and u.shape == (B, s.width) and N.has("ll_softmax_step")):
+            return None
+        dev, n_in = u.get_device(), w.shape[0]
+        for c in caches:
+            if c.dtype is not torch.bfloat16 or c.get_device() != dev:
+                return None
+        hv = s.heads * s.vdim
+        if n_in < self.n_in or (s.width | hv | n_in) % 8:
+            return None
+        return N.step_rows(u, (w, p.get("w_o")), ((n_in, s.width), (s.width, hv)))
 
-    def _step(self, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
+    def _step(self, at, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
         s, p, c = self.spec, self._parameters, self.cols
         kc, vc = caches
+        x, w_in, w_o = at
         n_in = p["w_in"].shape[0]
-        out = torch.empty((B, s.width), dtype=u.dtype, device=u.device)
-        scratch = torch.empty(_step_scratch_bytes(B, n_in, s.heads, s.dim, s.vdim, splits), dtype=torch.uint8, device=u.device)
-        N.call("ll_softmax_step", N.ptr(u), N.ptr(p["w_in"]), n_in, N.ptr(p["w_o"]), c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1,
-               N.ptr(self.q_norm), N.ptr(self.k_norm), float(s.eps), N.ptr(self.freq), s.rotary.dims, N.ptr(pos_ids), N.ptr(kc), N.ptr(vc),
-               N.ptr(self.sink), N.ptr(self.slopes), float(s.scale), float(s.softcap), B, s.width, s.heads, s.kv_heads, s.dim, s.vdim, s.window or 0,
-               s.chunk or 0, kc.shape[1], splits, form, N.ptr(out), N.ptr(scratch), N.stream())
+        q_norm, k_norm, sink = (p[n] if n in p else getattr(self, n) for n in ("q_norm", "k_norm", "sink"))
+        out = torch.empty_like(u)
+        scratch = u.new_empty(_step_scratch_bytes(B, n_in, s.heads, s.dim, s.vdim, splits) // 2)          # (whole pieces of 128 bytes or more)
+        N.call("ll_softmax_step", x, w_in, n_in, w_o, c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1, N.ptr(q_norm), N.ptr(k_norm),
+               float(s.eps), N.ptr(self.freq), s.rotary.dims, N.ptr(pos_ids), N.ptr(kc), N.ptr(vc), N.ptr(sink), N.ptr(self.slopes), float(s.scale),
+               float(s.softcap), B, s.width, s.heads, s.kv_heads, s.dim, s.vdim, s.window or 0, s.chunk or 0, kc.shape[1], splits, form, N.ptr(out),
+               N.ptr(scratch), N.stream())
         return out
 
     def attend(self, proj: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
