@@ -180,9 +180,13 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         """bf16 rows on a 4-bit layer whose scale groups are multiples of 128 columns: the kernels that read the checkpoint bytes."""
         if self.bits != 4 or x.dtype != torch.bfloat16:
             return False
-        s, z, bias = self.scales, self.zeros, self.bias          # (buffers, or what qlinear_4bit_weight was given)
+        b = self._buffers
+        try:
+            q, s, z, bias = b["quant_weight"], b["scales"], b["zeros"], b["bias"]
+        except KeyError:                       # no buffers (qlinear_4bit_weight's layer)
+            q, s, z, bias = self.quant_weight, self.scales, self.zeros, self.bias
         return (s.dtype == z.dtype == torch.bfloat16 and (bias is None or bias.dtype == torch.bfloat16)
-                and s.is_contiguous() and z.is_contiguous() and (self.quant_weight.data_ptr() | x.data_ptr()) % 16 == 0
+                and s.is_contiguous() and z.is_contiguous() and (q.data_ptr() | x.data_ptr()) % 16 == 0
                 and _rows_supported(self.out_features, self.in_features, self.tile_cols))
 
     def _copy_eligible(self, x) -> bool:
