@@ -131,8 +131,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
   constexpr int ROWS = 16, SL = 4, L = 64, NW = L * 16 / 256, NA = L * ROWS / 256, AS = 256 / ROWS;   // SL: shares of the list
   __shared__ __align__(16) float w_s[L][64], a_s[L][ROWS];
   const int tid = threadIdx.x, n0 = blockIdx.x * 64, m0 = blockIdx.y * ROWS, blk = m0 / 64, col = (tid & 15) * 4;
-  const int cnt = count[blk], n = n0 + col, m = m0 + (tid >> 4);
-  const bool vec = n + 4 <= N && (N & 3) == 0;             // (then a partial sum starts on a 16-byte boundary too)
+  const int cnt = count[blk];
   float first[4];                                          // GATED: the first layer's outputs
 #pragma unroll 1
   for (int which = 0; which < (GATED ? 2 : 1); ++which) {
@@ -153,7 +152,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
       const bool words = cbt != nullptr && (N & 3) == 0 && ((uintptr_t)cbt & 3) == 0;
       float sb127[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn(scb[min(n + j, N - 1)], 127.f);
+      for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn(scb[min(n0 + col + j, N - 1)], 127.f);
       uint32_t q[NW];
       float av[NA];
       auto fetch = [&](int b) {
@@ -163,7 +162,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
 #pragma unroll
         for (int u = 0; u < NA; ++u) av[u] = 0.f, ka[u] = b + AS * u < cnt ? __ldg(list + min(b + ai + AS * u, cnt - 1)) : 0;
         if (words) {
-          const int8_t* src = cbt + min(n, N - 4);
+          const int8_t* src = cbt + min(n0 + col, N - 4);
 #pragma unroll
           for (int u = 0; u < NW; ++u)
             if (b + 16 * u < cnt) q[u] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)kw[u] * N));
@@ -173,7 +172,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
             if (b + 16 * u >= cnt) continue;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const int c = min(n + j, N - 1);
+              const int c = min(n0 + col + j, N - 1);
               const int8_t v = cbt != nullptr ? __ldg(cbt + (size_t)kw[u] * N + c) : __ldg(cb + (size_t)c * K + kw[u]);
               q[u] |= (uint32_t)(uint8_t)v << (8 * j);
             }
@@ -243,9 +242,17 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
         acc[0][0] = o.x, acc[0][1] = o.y, acc[0][2] = o.z, acc[0][3] = o.w;
       }
     }
+    const int n = n0 + col, m = m0 + (tid >> 4);
+    const bool vec = n + 4 <= N && (N & 3) == 0;           // (then a partial sum starts on a 16-byte boundary too)
     if (n >= N || m >= M) continue;                        // (which takes part in the barriers of the second layer's list)
     const float sa = sca[m];
     const size_t at = (size_t)m * N + n;
+    float sb[4], bv[4];                                    // (asked for before the sums are there)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      sb[j] = n + j < N ? scb[n + j] : 0.f;
+      bv[j] = n + j < N && bias != nullptr ? to_half_f32<T>(bias[n + j]) : 0.f;
+    }
     int cv[4] = {0, 0, 0, 0};
     for (int z = 0; z < parts; ++z) {
       const int32_t* src = c32 + (which ? layer : 0) + (size_t)z * part + at;
@@ -260,7 +267,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       if (n + j >= N) break;
-      const float out = int8_finish((float)cv[j], sa, scb[n + j], bias != nullptr, bias != nullptr ? to_half_f32<T>(bias[n + j]) : 0.f, cnt, acc[0][j]);
+      const float out = int8_finish((float)cv[j], sa, sb[j], bias != nullptr, bv[j], cnt, acc[0][j]);
       if (!GATED) dt<T>::st(y, at + j, out);
       else if (which == 0) first[j] = dt<T>::rd(out);
       else dt<T>::st(y, at + j, __fmul_rn(silu_act<T>(first[j]), dt<T>::rd(out)));
@@ -355,6 +362,9 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
   __syncthreads();
   if (tid == 0) s_last = atomicAdd(arrive + blk, 1) == M - 1;
   __syncthreads();
+  // The next kernel's CTAs come while the lists are made.  (Let in from the start on they pile up on the SMs that have no row: 130 rows with long
+  // lists 2300 us instead of 1280.)
+  pdl_launch_dependents();
   if (!s_last) return;
   __threadfence();
   int base = 0;
@@ -505,9 +515,11 @@ int i8c_ranges(int N, int K, int layers, int sms, int* per) {
   return (nkb + *per - 1) / *per;
 }
 
-// What the preparation leaves for a step of M rows, and the partial sums of a step of up to 64 (part_rows).
+// What the preparation leaves for a step of M rows, the partial sums of a step of up to 64 (partial) and the outlier parts of a longer one.
+int i8r_pitch(int N) { return (N + 255) & ~255; }      // of an outlier part's rows: whole tiles
 struct Ws {
-  int8_t* ca; int32_t* part; float* sca; int32_t* idx; uint8_t* flag; int32_t* count; int32_t* arrive;
+  int8_t* ca; int32_t* part; __half* odd; float* sca; int32_t* idx; uint8_t* flag; int32_t* count; int32_t* arrive;
+  int32_t* next;                 // of int8_outlier_rows_kernel's tiles
   size_t zero_off, zero_bytes, total;
 };
 Ws carve(void* base, int M, int N, int K, int layers, bool partial) {
@@ -519,11 +531,13 @@ Ws carve(void* base, int M, int N, int K, int layers, bool partial) {
   int per;
   w.ca = (int8_t*)(p + take((size_t)M * K));
   w.part = (int32_t*)(p + take(partial ? (size_t)layers * i8c_ranges(N, K, layers, sm_count(), &per) * M * N * 4 : 0));
+  w.odd = (__half*)(p + take(partial ? 0 : (size_t)layers * M * i8r_pitch(N) * 2));
   w.idx = (int32_t*)(p + take(blocks * K * 4));
   w.sca = (float*)(p + take((size_t)M * 4));
   w.zero_off = o;  // cleared at the start of every call
   w.flag = p + take(blocks * K);
   w.arrive = (int32_t*)(p + take(blocks * 4));
+  w.next = (int32_t*)(p + take(4));
   w.zero_bytes = o - w.zero_off;
   w.count = (int32_t*)(p + take(blocks * 4));
   w.total = o;
@@ -583,19 +597,137 @@ int int8_pass(const T* x, const I8Layer<T>& l0, const I8Layer<T>& l1, T* y, int 
 // the second, and y = silu(out1) * out2.
 //   warp 0: TMA producer; warp 1: in rank 0, one thread issues the products; warps 2-9: finish, 32 rows and half of the columns per warp,
 //   32 columns at a time (GATED: 16 of either layer), read from tensor memory so that a thread has four rows of eight columns
-// Outlier part: a warp's 32 rows belong to one block of 64 rows, so to one list.  Its activations (up to 32 a row) are gathered before the
-// tile's sums are there, and so are the scales and the first eight outliers' weights of its columns; the weights of four outliers x 32 columns
-// pass through shared memory as fp32, already rounded.
+// Outlier part: a warp's 32 rows belong to one block of 64 rows, so to one list.  Of a short list (i8r_limit) its activations are gathered before
+// the tile's sums are there, and so are the scales and the first eight outliers' weights of its columns; the weights of four outliers x 32
+// columns pass through shared memory as fp32, already rounded.  The parts of longer lists a kernel before this one has left as fp16
+// (int8_outlier_rows_kernel: a warp has no other warp's rows to share a list's weights with).  us a call, a feed-forward of 4096 x 11008 whose
+// input has 6 and 30 outlier features, and its hidden state more of them: a warp reading its lists to the end / three products with their finish by 64 rows / here:
+// 512 rows 582 / 326 / 234, 1900 / 725 / 667 and, of one layer alone with 64, 300, 1000 outliers, 175 / 105 / 87, 773 / 263 / 258, 2265 / 729 / 732;
+// 2048 rows 2043 / 1061 / 690 and 7235 / 2432 / 2116, alone 522 / 357 / 266, 2543 / 950 / 887, 7377 / 2691 / 2620.
 // (Four finishing warps, one a scheduler, took 35 us a tile of the gated form, four times as long as its products.)
 // 512 rows through a 7B feed-forward with six outlier features: 53 us for both gated layers and 27 for the third, preparation 24; 127 for three
 // products of 128 x 128 tiles a CTA, 55 for their finish and 45 for preparation and the gated product before.  2048 rows: 305 us a call (701).
 // Bound by the weights' way from memory and, with outliers, by the finish (weights asked for one by one: 10 us a tile instead of 3).
-constexpr int I8R_PASS = 8192;                           // rows of one pass: bounds the workspace
+constexpr int I8R_PASS = 8192;                           // rows of one pass: bounds the workspace (outlier parts of a gated pair: 453 MB at 13824 columns)
 constexpr int I8R_WARPS = 8, I8R_THREADS = (2 + I8R_WARPS) * 32;                           // finishing warps: two per 32 rows, half of the columns each
 constexpr int I8R_LIST = 32, I8R_OUT = 32 * 64, I8R_W = 6 * 32 * 4;
 constexpr int i8r_stages(int bn) { return bn > 128 ? 5 : 6; }
 constexpr int i8r_smem(int bn) {
   return i8r_stages(bn) * (I8_BOX + bn * 64) + I8R_WARPS * (2 * I8R_OUT + I8R_LIST * 64 + I8R_LIST * 4 + I8R_W) + 512 + 1024;
+}
+
+// The outlier part of blocks of 64 rows whose lists are longer than `limit`, rounded to fp16 as the finish adds it: 64 rows x 64 columns of a
+// layer at a time.  The weights and activations of 32 outliers stand in shared memory as fp32, already rounded, and the next 32 are asked for
+// (all list entries, then all they point to) before these are added; a thread owns four columns of four rows, two 16-byte reads for 16
+// multiply-adds, and adds in the order of the list.  WORDS: CB transposed is there, on 4-byte boundaries.
+template <typename T, bool WORDS>
+__global__ void __launch_bounds__(256, 4) int8_outlier_rows_kernel(const I8Layer<T> l0, const I8Layer<T> l1, const T* __restrict__ x, const int32_t* __restrict__ idx,
+                                                              const int32_t* __restrict__ count, int32_t* __restrict__ next, __half* __restrict__ odd,
+                                                              int M, int N, int K, int layers, int pitch, int limit) {
+  constexpr int L = 32, NW = L * 16 / 256, NA = L * 64 / 256;
+  __shared__ __align__(16) float w_s[L][64], a_s[L][64];
+  __shared__ int s_item, s_blk[I8R_PASS / 64];
+  pdl_launch_dependents();                                 // (what follows waits for this kernel's end, and this one for the preparation's)
+  pdl_wait();
+  const int tid = threadIdx.x, col = (tid & 15) * 4;
+  const int tiles = (N + 63) / 64, per = layers * tiles, blocks = (M + 63) / 64;
+  const bool single = (int)gridDim.x >= blocks * per;      // a CTA per tile of every block
+  if (!single) {                                           // the blocks with long lists, in order
+    if (tid < 32) {
+      int n = 0;
+      for (int b0 = 0; b0 < blocks; b0 += 32) {
+        const uint32_t any = __ballot_sync(0xffffffffu, b0 + tid < blocks && count[b0 + tid] > limit);
+        if ((any >> tid) & 1u) s_blk[n + __popc(any & ((1u << tid) - 1u))] = b0 + tid;
+        n += __popc(any);
+      }
+      if (tid == 0) s_item = n;
+    }
+    __syncthreads();
+  }
+  const int items = single ? blocks * per : s_item * per;
+  for (int item = blockIdx.x; item < items;) {
+    const int m0 = (single ? item / per : s_blk[item / per]) * 64, cnt = count[m0 / 64];
+    if (cnt <= limit) break;                               // (single)
+    const bool second = item % per >= tiles;
+    const int n = item % per % tiles * 64 + col;
+    const int32_t* list = idx + (size_t)(m0 / 64) * K;
+    // what a thread brings: four columns of NW outliers' weights, one row of NA outliers' activations.  Entries past the list's end, columns
+    // past N and rows past M repeat the last one: they are never added, or added to what nobody stores or reads.
+    const T* xr = x + (size_t)min(m0 + (tid & 63), M - 1) * K;
+    const int8_t* src = WORDS ? (second ? l1.cbt : l0.cbt) + min(n, N - 4) : nullptr;
+    uint32_t q[NW];
+    float av[NA], acc[4][4], sb127[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sb127[j] = __fdiv_rn((second ? l1.scb : l0.scb)[min(n + j, N - 1)], 127.f);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+    auto fetch = [&](int b) {
+      int kw[NW], ka[NA];
+#pragma unroll
+      for (int u = 0; u < NW; ++u) kw[u] = __ldg(list + min(b + (tid >> 4) + 16 * u, cnt - 1));
+#pragma unroll
+      for (int u = 0; u < NA; ++u) ka[u] = __ldg(list + min(b + (tid >> 6) + 4 * u, cnt - 1));
+#pragma unroll
+      for (int u = 0; u < NW; ++u) {
+        if (WORDS) {
+          q[u] = __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)kw[u] * N));
+        } else {
+          const I8Layer<T>& l = second ? l1 : l0;
+          q[u] = 0u;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int c = min(n + j, N - 1);
+            const int8_t v = l.cbt != nullptr ? __ldg(l.cbt + (size_t)kw[u] * N + c) : __ldg(l.cb + (size_t)c * K + kw[u]);
+            q[u] |= (uint32_t)(uint8_t)v << (8 * j);
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < NA; ++u) av[u] = to_half_f32<T>(xr[ka[u]]);
+    };
+    fetch(0);
+    const int r0 = (tid >> 4) * 4;
+    for (int b = 0; b < cnt; b += L) {
+      __syncthreads();                                     // the outliers before have been added
+#pragma unroll
+      for (int u = 0; u < NW; ++u) {
+        float w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = __half2float(__float2half_rn(__fmul_rn((float)(int8_t)(q[u] >> (8 * j)), sb127[j])));
+        *reinterpret_cast<float4*>(&w_s[(tid >> 4) + 16 * u][col]) = make_float4(w[0], w[1], w[2], w[3]);
+      }
+#pragma unroll
+      for (int u = 0; u < NA; ++u) a_s[(tid >> 6) + 4 * u][tid & 63] = av[u];
+      __syncthreads();
+      if (b + L < cnt) fetch(b + L);
+      const int end = min(L, cnt - b);
+#pragma unroll 4
+      for (int i = 0; i < end; ++i) {
+        const float4 w = *reinterpret_cast<const float4*>(&w_s[i][col]), a4 = *reinterpret_cast<const float4*>(&a_s[i][r0]);
+        const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          acc[r][0] = fmaf(a[r], w.x, acc[r][0]);
+          acc[r][1] = fmaf(a[r], w.y, acc[r][1]);
+          acc[r][2] = fmaf(a[r], w.z, acc[r][2]);
+          acc[r][3] = fmaf(a[r], w.w, acc[r][3]);
+        }
+      }
+    }
+    __half* dst = odd + (size_t)(second ? M : 0) * pitch + n;          // (n < pitch: a row is whole tiles)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (m0 + r0 + r >= M) break;
+      const __half2 lo = __floats2half2_rn(acc[r][0], acc[r][1]), hi = __floats2half2_rn(acc[r][2], acc[r][3]);
+      *reinterpret_cast<uint2*>(dst + (size_t)(m0 + r0 + r) * pitch) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    if (single) break;
+    __syncthreads();                                       // the item has been read by all
+    if (tid == 0) s_item = (int)gridDim.x + atomicAdd(next, 1);
+    __syncthreads();
+    item = s_item;
+  }
 }
 
 template <typename T>
@@ -605,8 +737,9 @@ struct I8RParams {
   const float* sca;
   const int32_t* idx;
   const int32_t* count;
+  const __half* odd;                                 // [layer][M][pitch] outlier parts of blocks with longer lists than a warp holds
   T* y;
-  int M, N, K, mtiles, ntiles, boxes;                // boxes: TMA stores y
+  int M, N, K, pitch, limit, mtiles, ntiles, boxes;  // limit: of what a warp adds itself; boxes: TMA stores y
   int* word;
 };
 struct I8Fail {
@@ -754,14 +887,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
     uint32_t boxes = 0;
     for (int t = pair; t < tiles; t += pairs, ++i) {
       const int r0 = (t % p.mtiles) * 256 + rank * 128 + quarter * 32, n0 = (t / p.mtiles) * COLS, m = min(r0 + lane, p.M - 1);
-      // the block's list and this row's activations of its first entries
-      const int cnt = r0 < p.M ? p.count[r0 / 64] : 0;
+      // the block's list and this row's activations of its entries; the outlier part of a longer list is there already
+      const int all = r0 < p.M ? p.count[r0 / 64] : 0, cnt = all <= p.limit ? all : 0;
       const int32_t* list = p.idx + (size_t)(r0 / 64) * p.K;
       const T* xr = p.x + (size_t)m * p.K;
       __syncwarp();
       if (lane < cnt) k_s[lane] = __ldg(list + lane);
       __syncwarp();
-      for (int l = 0; l < min(cnt, I8R_LIST); l += 4) {
+      for (int l = 0; l < cnt; l += 4) {
         T v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) v[j] = xr[k_s[min(l + j, cnt - 1)]];
@@ -779,10 +912,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
         const size_t step = cbt != nullptr ? (size_t)p.N : 1;
         uint32_t v[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int at = min(l + j, cnt - 1);
-          v[j] = (uint8_t)__ldg(src + (size_t)(l < I8R_LIST ? k_s[at] : __ldg(list + at)) * step);
-        }
+        for (int j = 0; j < 4; ++j) v[j] = (uint8_t)__ldg(src + (size_t)k_s[min(l + j, cnt - 1)] * step);
         return v[0] | (v[1] << 8) | (v[2] << 16) | (v[3] << 24);
       };
       // what the tile's chunks want of their columns, asked for before the sums are there: scales, weights of the first eight outliers
@@ -830,20 +960,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if (l + j >= cnt) break;
-            float a[4];
-            if (l + j < I8R_LIST) {
-              const uint2 h = *reinterpret_cast<const uint2*>(a_s + (l + j) * 32 + g * 4);
-              const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
-              a[0] = lo.x, a[1] = lo.y, a[2] = hi.x, a[3] = hi.y;
-            } else {
-              const int k = __ldg(list + l + j);
-#pragma unroll
-              for (int r = 0; r < 4; ++r) a[r] = to_half_f32<T>(p.x[(size_t)min(r0 + g + 8 * r, p.M - 1) * p.K + k]);
-            }
+            const uint2 h = *reinterpret_cast<const uint2*>(a_s + (l + j) * 32 + g * 4);
+            const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&h.x)), hi = __half22float2(*reinterpret_cast<const __half2*>(&h.y));
+            const float a[4] = {lo.x, lo.y, hi.x, hi.y};
             const float4 w0 = *reinterpret_cast<const float4*>(w_s + j * 32 + t4 * 8), w1 = *reinterpret_cast<const float4*>(w_s + j * 32 + t4 * 8 + 4);
             const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
             for (int e = 0; e < 32; ++e) odd[e] = fmaf(a[(e >> 4) * 2 + ((e >> 1) & 1)], w[((e >> 2) & 3) * 2 + (e & 1)], odd[e]);
+          }
+        }
+        if (all > p.limit) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 2) {
+            const int b = (e >> 2) & 3, row = min(r0 + (e >> 4) * 16 + ((e >> 1) & 1) * 8 + g, p.M - 1);
+            const __half* src = p.odd + (size_t)((GATED && b >= 2 ? p.M : 0) + row) * p.pitch + n0 + cc + (GATED ? b & 1 : b) * 8 + 2 * t4;
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(src));
+            odd[e] = f.x, odd[e + 1] = f.y;
           }
         }
         __syncwarp();
@@ -875,7 +1007,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
             f0 = __fadd_rn(f0, bv.x), f1 = __fadd_rn(f1, bv.y);
           }
           __half2 h = __floats2half2_rn(f0, f1);
-          if (cnt > 0) h = __hadd2_rn(h, __floats2half2_rn(odd[e], odd[e + 1]));
+          if (all > 0) h = __hadd2_rn(h, __floats2half2_rn(odd[e], odd[e + 1]));
           const float2 r = __half22float2(h);
           o[e] = r.x, o[e + 1] = r.y;
         }
@@ -981,15 +1113,26 @@ int i8r_launch(const I8RParams<T>& q, cudaStream_t st, const int8_t* ca) {
   return LL_OK;
 }
 
+// Entries of a list up to which the finishing warps add the outlier part themselves.  us, here / in the kernel before, one layer of 11008 x 4096
+// with 18, 26, 30 outliers: 65 rows 36 / 32, 41 / 33, 43 / 33; 512 rows 55 / 60, 67 / 64, 73 / 65; 2048 rows 143 / 175, 175 / 183, 191 / 187.
+int i8r_limit(int rows) { return rows <= 384 ? 16 : 28; }
 template <typename T, bool GATED>
 int int8_rows(const T* x, const I8Layer<T>& l0, const I8Layer<T>& l1, T* y, int M, int N, int K, float thr, void* base, cudaStream_t st) {
   for (int r0 = 0; r0 < M; r0 += I8R_PASS) {
     const int rows = min(I8R_PASS, M - r0);
-    const Ws w = carve(base, rows, N, K, 1, false);
+    const Ws w = carve(base, rows, N, K, GATED ? 2 : 1, false);
     const T* xp = x + (size_t)r0 * K;
     if (int r = int8_prepare<T>(xp, w, base, rows, K, thr, st)) return r;
+    // a CTA per tile where that is a few rounds of four an SM; more tiles are taken one by one by that many CTAs, so that passing over blocks with
+    // short lists stays cheap (2048 x 11008: 1.5 us instead of 6.5).
+    const int items = (rows + 63) / 64 * ((N + 63) / 64) * (GATED ? 2 : 1), ctas = 4 * (sm_count() > 0 ? sm_count() : 148), limit = i8r_limit(rows);
+    const bool words = l0.cbt != nullptr && l1.cbt != nullptr && (N & 3) == 0 && (((uintptr_t)l0.cbt | (uintptr_t)l1.cbt) & 3) == 0;
+    LL_CUDA(launch(words ? int8_outlier_rows_kernel<T, true> : int8_outlier_rows_kernel<T, false>, dim3(items <= 4 * ctas ? items : ctas), dim3(256), 0, st,
+                   true, l0, l1, xp, (const int32_t*)w.idx, (const int32_t*)w.count, w.next, w.odd, rows, N, K, GATED ? 2 : 1, i8r_pitch(N), limit));
+    LL_LAUNCH_OK("int8_outlier_rows_kernel");
     I8RParams<T> p{};
     p.layer[0] = l0, p.layer[1] = l1, p.x = xp, p.sca = w.sca, p.idx = w.idx, p.count = w.count, p.y = y + (size_t)r0 * N;
+    p.odd = w.odd, p.pitch = i8r_pitch(N), p.limit = limit;
     p.M = rows, p.N = N, p.K = K;
     // tiles of half the columns take 0.6 of the time: what the waves cost (as the dense products' rule)
     const long long pairs = sm_count() > 1 ? sm_count() / 2 : 1, mt = (rows + 255) / 256, wide = GATED ? 128 : 256;

@@ -201,3 +201,58 @@ def test_a_captured_call_keeps_its_workspace():
     torch.cuda.synchronize()
     assert torch.equal(y, want)
     assert all(bool((o == 0x33).all()) for o in others)
+
+
+@pytest.mark.parametrize("M,N", [(65, 70), (200, 64), (385, 300), (640, 260), (2100, 5000)])
+@pytest.mark.parametrize("transposed", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_prompts_with_long_and_short_lists(M, N, transposed, dtype):
+    """Every block of 64 rows has a list of its own length: none, what the finishing warps add themselves, one more, several stages, half of all
+    features; few tiles (one a CTA) and more than the CTAs that take them one by one.  Against 64 bits, and both gated layers against each alone."""
+    from lit_llama import _native as NV
+
+    K = 384
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn((M, K), generator=g, device="cuda").clamp(-4, 4)
+    lists = [0, 5, 16, 17, 28, 29, 32, 33, 64, 65, 190]
+    for b in range((M + 63) // 64):
+        cols = torch.randperm(K, generator=g, device="cuda")[: lists[(7 * b + M) % len(lists)]]
+        rows = slice(64 * b, min(64 * b + 64, M))
+        x[rows, cols] = torch.sign(x[rows, cols]) * (6.5 + 3.0 * x[rows, cols].abs())
+    x = x.to(dtype).half().to(dtype)
+    layers = []
+    for i in range(2):
+        cb = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+        layers.append((cb, cb.t().contiguous() if transposed else None, (torch.rand(N, generator=g, device="cuda") + 0.5) * 0.05,
+                       torch.randn(N, generator=g, device="cuda").to(torch.bfloat16).to(dtype)))      # (a number of every dtype)
+    ws = torch.full((NV.call_ret("ll_int8_gated_workspace_bytes", M, N, K),), 0x5A, dtype=torch.uint8, device="cuda")
+    outs = []
+    for cb, cbt, scb, bias in layers:
+        y = torch.empty((M, N), dtype=dtype, device="cuda")
+        NV.call("ll_int8_linear", NV.ptr(x), NV.dtype_code(dtype), NV.ptr(cb), NV.ptr(cbt), NV.ptr(scb), NV.ptr(bias), NV.ptr(y), M, N, K, 6.0, NV.ptr(ws),
+                ws.numel(), NV.stream())
+        outs.append(y)
+    if dtype == torch.bfloat16:
+        h, want_h = torch.empty_like(outs[0]), torch.empty_like(outs[0])
+        ws.fill_(0x5A)
+        NV.call("ll_int8_gated", NV.ptr(x), *(NV.ptr(t) for layer in layers for t in layer), NV.ptr(h), M, N, K, 6.0, NV.ptr(ws), ws.numel(), NV.stream())
+        NV.call("ll_silu_mul", NV.ptr(outs[0]), NV.ptr(outs[1]), NV.ptr(want_h), NV.LL_BF16, M * N, NV.stream())
+        # (silu comes from a fast exponential and division: now and then on the other bf16 neighbour, a rounding each of it and of the product)
+        assert ((h.double() - want_h.double()).abs() <= want_h.double().abs() * 2.0 ** -7).all() and (h == want_h).float().mean() >= 0.99
+    for y, (cb, cbt, scb, bias) in zip(outs, layers):
+        for b in range((M + 63) // 64):
+            rows = slice(64 * b, min(64 * b + 64, M))
+            a = x[rows].double()
+            out = (a.abs() >= 6.0).any(0)
+            rest = a.masked_fill(out[None], 0.0)
+            sca = rest.abs().amax(1)
+            ca = torch.round((rest.float() * (torch.full_like(sca, 127.0).float() / sca.float())[:, None]).double())
+            want = (ca @ cb.double().t()) * sca[:, None] * scb.double()[None] / 127.0 ** 2 + bias.double()[None]
+            wo = (cb.double()[:, out] * scb.double()[:, None] / 127.0).half().double()
+            odd, size = a[:, out] @ wo.t(), a[:, out].abs() @ wo.abs().t()
+            # both parts and their sum rounded to fp16, an outlier's weight possibly on its other fp16 neighbour, the result to the dtype (bf16:
+            # eight significant bits, half a unit in the last place is up to 2^-8 of the number)
+            bound = 2.0 ** -11 * (want.abs() + odd.abs() + (want + odd).abs()) * 1.01 + 2.0 ** -10 * size + 1e-4
+            bound = bound + ((want + odd).abs() * 2.0 ** -8 * 1.01 if dtype == torch.bfloat16 else 0.0)
+            assert ((y[rows].double() - want - odd).abs() <= bound).all()
+    assert NV.call_ret("ll_int8_tc_error") == 0
