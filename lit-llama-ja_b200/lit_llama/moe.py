@@ -164,7 +164,9 @@ class MoE(nn.Module):
         s, p = self.spec, self._parameters
         sff = s.shared_ff or 0
         x, w_gu, w_down, ws_in, ws_down = at if sff else (*at, None, None)
-        router, bias, correction = (p[n] if n in p else getattr(self, n) for n in ("w_router", "b_router", "correction"))
+        router = p["w_router"] if "w_router" in p else self.w_router
+        bias = p["b_router"] if "b_router" in p else self.b_router
+        correction = p["correction"] if "correction" in p else self.correction
         out = torch.empty_like(x_act)
         scratch = x_act.new_empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff) // 2)          # (whole pieces of 128 bytes or more)
         N.call("ll_moe_step", x, N.ptr(router), N.ptr(bias), N.ptr(correction), _SCORES[s.score], float(s.weight_scale), s.groups,
@@ -194,11 +196,11 @@ class MoE(nn.Module):
                            (up, down, (w.shape[0], s.width), (s.width, s.shared_ff)))
 
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:
-        s = self.spec
-        M, dev, dtype = x_act.shape[0], x_act.device, x_act.dtype
-        at = self._takes_step(x_act, M)
+        s, M = self.spec, x_act.shape[0]
+        at = self._takes_step(x_act, M) if M <= STEP_MAX_TOKENS else None
         if at:
             return self._step(at, x_act, M)
+        dev, dtype = x_act.device, x_act.dtype
         dt, st = N.dtype_code(dtype), N.stream()
         _, w, offsets, perm = self.route(x_act)
         n = M * s.top

@@ -247,7 +247,9 @@ class SoftmaxAttention(nn.Module):
         kc, vc = caches
         x, w_in, w_o = at
         n_in = p["w_in"].shape[0]
-        q_norm, k_norm, sink = (p[n] if n in p else getattr(self, n) for n in ("q_norm", "k_norm", "sink"))
+        q_norm = p["q_norm"] if "q_norm" in p else self.q_norm
+        k_norm = p["k_norm"] if "k_norm" in p else self.k_norm
+        sink = p["sink"] if "sink" in p else self.sink
         out = torch.empty_like(u)
         scratch = u.new_empty(_step_scratch_bytes(B, n_in, s.heads, s.dim, s.vdim, splits) // 2)          # (whole pieces of 128 bytes or more)
         N.call("ll_softmax_step", x, w_in, n_in, w_o, c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1, N.ptr(q_norm), N.ptr(k_norm),
