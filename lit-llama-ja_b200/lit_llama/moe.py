@@ -39,11 +39,25 @@ TC_MIN_ROWS_PER_EXPERT = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT",
 
 
 STEP_MAX_TOKENS, STEP_SMALL_EXPERT = 8, 1 << 22       # tokens of a step; ff * width
+STEP_REPEAT_BYTES = 300 << 20                         # of weights that a step reads for one token after another
 
 
 @functools.lru_cache(maxsize=1024)
-def _step_supported(M: int, width: int, ff: int, shared_ff: int) -> bool:
-    return bool(N.call_ret("ll_moe_step_supported", M, width, ff, shared_ff))
+def step_pays(M: int, width: int, ff: int, shared_ff: int, experts: int, top: int, branches: int) -> bool:
+    """Whether ``M`` tokens go through ``ll_moe_step``: sizes that it takes, and no fewer microseconds in the grouped kernels.
+
+    A step reads a choice's weights for its token alone, the grouped kernels read an expert's once for all of its tokens and take 40 to 60 us
+    more around that.  So what counts is what is read again: the choices less the distinct experts they can be expected to name, times an
+    expert's bytes; 300 MB of it are those 40 us.  Graphed, us, grouped / step (repeated MB): experts of 4096 x 1024, 16 of them and four
+    chosen, 6 tokens 106 / 99 (273), 8 tokens 107 / 127 (443); 32 and four, 8 tokens 158 / 139 (277); 64 and eight, 5 tokens 197 / 180 (222),
+    6 tokens 205 / 211 (320); of 2048 x 2048 the same to 5 us; of 2048 x 1024, 64 and eight, 8 tokens 160 / 143 (277); of 4096 x 2048, 16 and
+    four, 4 tokens 173 / 136 (255).  More than four tokens of larger experts keep the grouped kernels: 16 and four at 6 tokens 179 / 198, 32
+    and four at 8 tokens 247 / 263."""
+    most = STEP_MAX_TOKENS if ff * width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
+    if not 1 <= M <= most or not N.has("ll_moe_step") or not N.call_ret("ll_moe_step_supported", M, width, ff, shared_ff):
+        return False
+    distinct = experts * (1.0 - (1.0 - top / experts) ** M)
+    return (M * top - distinct) * (branches + 1) * ff * width * 2 <= STEP_REPEAT_BYTES
 
 
 @functools.lru_cache(maxsize=1024)
@@ -176,16 +190,13 @@ class MoE(nn.Module):
         return out
 
     def _takes_step(self, x_act: torch.Tensor, M: int):
-        """A few bf16 tokens, and weights that are what the module was built with: their addresses, or ``None``.  A choice's weights are read for its token alone, where the grouped GEMM reads an expert's once for all of its
-        tokens: more than four tokens only where experts are small.  us, grouped / here: 32 experts of 2048 x 1024, four chosen, at 4, 6, 8
-        tokens 97 / 62, 99 / 78, 128 / 94; of 4096 x 2048 212 / 168, 229 / 247, 286 / 320."""
+        """A few bf16 tokens (``step_pays``), and weights that are what the module was built with: their addresses, or ``None``."""
         s = self.spec
-        most = STEP_MAX_TOKENS if s.ff * s.width <= STEP_SMALL_EXPERT else STEP_MAX_TOKENS // 2
-        if not (1 <= M <= most and x_act.dtype is torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width) and N.has("ll_moe_step")
-                and _step_supported(M, s.width, s.ff, s.shared_ff or 0)):
+        branches = 1 if s.unit == "relu2" else 2
+        if not (x_act.dtype is torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width)
+                and step_pays(M, s.width, s.ff, s.shared_ff or 0, s.experts, s.top, branches)):
             return None
         p = self._parameters
-        branches = 1 if s.unit == "relu2" else 2
         up, down = (s.experts, branches * s.ff, s.width), (s.experts, s.width, s.ff)
         if not s.shared_ff:
             return N.step_rows(x_act, (p.get("w_gu"), p.get("w_down")), (up, down))
