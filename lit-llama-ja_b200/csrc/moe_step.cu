@@ -37,34 +37,33 @@ __device__ __forceinline__ float ms_unit(float g, float u, const MsParams& p, fl
   return g / (1.f + expf(-p.alpha * g)) * (u + (p.mode == 1 ? 1.f : 0.f));
 }
 // This lane's part of the dot products of R rows with R vectors (or all with the first: SAME) of n numbers; U 16-byte loads of every row in
-// flight.  In the last round a lane past the end loads the last piece again and adds zeros.
+// flight.  Past the end a lane takes the last piece again and drops its sum.
 template <int R, int U, bool SAME>
 __device__ __forceinline__ void ms_rows(const __nv_bfloat16* const (&row)[R], const __nv_bfloat16* const (&x)[R], int n, float (&part)[R]) {
   const int lane = threadIdx.x & 31, pieces = n / 8;
 #pragma unroll
   for (int r = 0; r < R; ++r) part[r] = 0.f;
-  auto round = [&](int i, bool whole) {        // whole: no lane's pieces lie past the end
+  for (int i = lane; i < pieces; i += 32 * U) {
     uint4 w[R][U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r) w[r][u] = sr_ld(row[r], whole ? i + 32 * u : min(i + 32 * u, pieces - 1));
+      for (int r = 0; r < R; ++r) w[r][u] = sr_ld(row[r], min(i + 32 * u, pieces - 1));
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool in = whole || i + 32 * u < pieces;
+      const bool in = i + 32 * u < pieces;
       float xf[8];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r == 0 || !SAME) sr_floats(in ? reinterpret_cast<const uint4*>(x[r])[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
         float wf[8];
-        sr_floats(in ? w[r][u] : make_uint4(0u, 0u, 0u, 0u), wf);
-        sr_dot(part[r], wf, xf);
+        sr_floats(w[r][u], wf);
+        float sum = part[r];
+        sr_dot(sum, wf, xf);
+        part[r] = in ? sum : part[r];
       }
     }
-  };
-  int i = lane;
-  for (const int end = pieces / (32 * U) * (32 * U); i < end; i += 32 * U) round(i, true);
-  if (i < pieces) round(i, false);
+  }
 }
 
 // blockIdx.y: token and choice, the shared expert's first; blockIdx.x: 2 outputs a warp

@@ -30,8 +30,9 @@ __device__ __forceinline__ void sr_dot(float& acc, const float (&w)[8], const fl
   for (int i = 0; i < 8; ++i) acc = fmaf(w[i], x[i], acc);
 }
 
-// y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; in the last round a lane past the end of k
-// loads the last piece again and adds zeros (zero times an infinite weight would be no number).  K, ldx multiples of 8, rows on 16-byte boundaries.
+// y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; past the end of k a lane takes the last piece again and
+// drops its sum (times zero an infinite weight would be no number; zeroed weights, or rounds without a check before the last, are slower).
+// K, ldx multiples of 8, rows on 16-byte boundaries.
 template <int MT>
 __global__ void __launch_bounds__(SR_THREADS) small_linear_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ w,
                                                                   __nv_bfloat16* __restrict__ y, int ldy, int N, int K) {
@@ -44,26 +45,25 @@ __global__ void __launch_bounds__(SR_THREADS) small_linear_kernel(const __nv_bfl
   float acc[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-  auto round = [&](int i, bool whole) {        // whole: no lane's pieces lie past the end
+  for (int i = lane; i < pieces; i += 32 * U) {
     uint4 q[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) q[u] = sr_ld(row, whole ? i + 32 * u : min(i + 32 * u, pieces - 1));
+    for (int u = 0; u < U; ++u) q[u] = sr_ld(row, min(i + 32 * u, pieces - 1));
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool in = whole || i + 32 * u < pieces;
+      const bool in = i + 32 * u < pieces;
       float wf[8];
-      sr_floats(in ? q[u] : make_uint4(0u, 0u, 0u, 0u), wf);
+      sr_floats(q[u], wf);
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         float xf[8];
         sr_floats(in ? reinterpret_cast<const uint4*>(x + (size_t)m * ldx)[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
-        sr_dot(acc[m], wf, xf);
+        float sum = acc[m];
+        sr_dot(sum, wf, xf);
+        acc[m] = in ? sum : acc[m];
       }
     }
-  };
-  int i = lane;
-  for (const int end = pieces / (32 * U) * (32 * U); i < end; i += 32 * U) round(i, true);
-  if (i < pieces) round(i, false);
+  }
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
     const float v = warp_sum(acc[m]);
