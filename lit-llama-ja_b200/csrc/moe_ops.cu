@@ -175,7 +175,9 @@ __global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kern
         if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
       }
       if (k == 0) v0 = best;
-      const float p = score == SCORE_SIGMOID ? sg[bi] : score == SCORE_ALL ? expf(best - zmax) / zsum : expf(best - v0);
+      const bool none = bi >= X;         // only scores that are no numbers are left: a valid expert, whose weight is none either
+      if (none) bi = X - 1;
+      const float p = none ? NAN : score == SCORE_SIGMOID ? sg[bi] : score == SCORE_ALL ? expf(best - zmax) / zsum : expf(best - v0);
       denom += p;
       if (lane == 0) {
         z[bi] = -INFINITY;

@@ -145,3 +145,25 @@ def test_rotated_rows(dim, rot, norm, values, shift):
         rest = torch.ones(ring, dtype=torch.bool)
         rest[at.cpu()] = False
         assert not kc[:, rest.cuda()].any() and not vc[:, rest.cuda()].any()
+
+
+@pytest.mark.parametrize("M", [1, 3, 9, 300, 1400])
+@pytest.mark.parametrize("score", ["chosen", "all", "sigmoid"])
+def test_a_row_of_no_numbers(M, score):
+    """A token of NaNs has no expert to choose: it is routed to a valid one, comes out as NaNs, and the other tokens as without it."""
+    from lit_llama.moe import MoE, MoESpec
+
+    mix = MoE(MoESpec(64, 8, 2, 32, 7.0, 16, 7.0, score=score, router_bias=False), torch.bfloat16, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(M)
+    with torch.no_grad():
+        for p in mix.parameters():
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") * p.shape[-1] ** -0.5)
+    x = torch.randn((M, 64), generator=g, device="cuda").to(torch.bfloat16)
+    want = mix(x)
+    x[M // 2] = float("nan")
+    idx, w, offsets, perm = mix.route(x)
+    assert bool(((idx >= 0) & (idx < 8)).all()) and int(offsets[-1]) == 2 * M and torch.equal(perm.sort().values, torch.arange(2 * M, device="cuda", dtype=perm.dtype))
+    assert bool(w[M // 2].isnan().all())
+    got = mix(x)
+    keep = torch.arange(M, device="cuda") != M // 2
+    assert bool(got[M // 2].isnan().all()) and torch.equal(got[keep], want[keep])
