@@ -199,6 +199,12 @@ class ColBlockQuantizedLinear(torch.nn.Module):
                 and self.out_features % 128 == 0 and self.tile_cols % 128 == 0 and self.in_features % self.tile_cols == 0
                 and (self.bias is None or self.bias.dtype == torch.bfloat16))
 
+    def _make_step_stream(self, x) -> None:
+        """The stream that single-token steps read is made with a layer's first batch of 9 to 128 rows, once: neither its next token pays for it,
+        nor does a capture that follows find none and take another kernel."""
+        if x.shape[0] > 8 and N.STREAM_U8 not in self._streams and self._fused_gemm_eligible(x) and not torch.cuda.is_current_stream_capturing():
+            self._prepare_kind(N.STREAM_U8)
+
     def stream_for(self, M: int):
         """(prepared stream, its kind) for batch ``M`` WITHOUT building it (safe under CUDA-graph capture), or (None, kind)."""
         kind = self._kind(M)
@@ -230,9 +236,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         if fast:
             self._gemv(x, y)
         elif M <= self.FUSED_GEMM_MAX_M and self._rows_eligible(x):
-            # the stream that single-token steps read is made here once, with a generation's prompt or first batch, not with its next token
-            if M > 8 and N.STREAM_U8 not in self._streams and self._fused_gemm_eligible(x) and not torch.cuda.is_current_stream_capturing():
-                self._prepare_kind(N.STREAM_U8)
+            self._make_step_stream(x)
             scratch = _int8_workspace(x.device, _batch_scratch_bytes(M, Nout, K, 1))
             N.call("ll_int4_batch", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), N.ptr(scratch), M, Nout, K,
                    self.tile_cols, 0, N.stream())
@@ -324,6 +328,8 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
             return None
         q1, q2 = fc1._packed_ptr_ok(), fc2._packed_ptr_ok()
         N.require_cuda(q1, q2)
+        fc1._make_step_stream(x)
+        fc2._make_step_stream(x)
         h = torch.empty((M, Nout), device=x.device, dtype=x.dtype)
         scratch = _int8_workspace(x.device, _batch_scratch_bytes(M, Nout, K, 2))
         N.call("ll_int4_batch_gated", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
