@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
     for (int j = 0; j < 4; ++j) {
       if (n + j >= N) break;
       const float out = int8_finish((float)cv[j], sa, sb[j], bias != nullptr, bv[j], cnt, acc[0][j]);
-      if (!GATED) dt<T>::st(y, at + j, out);
+      if constexpr (!GATED) dt<T>::st(y, at + j, out);
       else if (which == 0) first[j] = dt<T>::rd(out);
       else dt<T>::st(y, at + j, __fmul_rn(silu_act<T>(first[j]), dt<T>::rd(out)));
     }
@@ -1011,7 +1011,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(I8R_THREADS, 1)
           const float2 r = __half22float2(h);
           o[e] = r.x, o[e + 1] = r.y;
         }
-        if (GATED) {                         // columns b of the first layer and b + 2 of the second: the product takes the first's place
+        if constexpr (GATED) {               // columns b of the first layer and b + 2 of the second: the product takes the first's place
 #pragma unroll
           for (int e = 0; e < 32; ++e)
             if ((e & 8) == 0) o[e] = __fmul_rn(silu_act<T>(dt<T>::rd(o[e])), dt<T>::rd(o[e + 8]));

@@ -9,7 +9,7 @@
 // copy rate.  The shared expert's blocks come first and do not wait for the router.
 // us a call (graphed), sorted and grouped with dense layers for the shared expert / here: that size at 1, 2, 4, 8 tokens 155 (69) / 32 (28),
 // 125 (73) / 40 (38), 97 (76) / 62 (59), 128 (113) / 94 (91).
-#include "small_rows.cuh"
+#include "row_loads.cuh"
 
 namespace llb {
 

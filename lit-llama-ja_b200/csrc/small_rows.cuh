@@ -5,30 +5,12 @@
 // projections of an attention layer, us, here / the library's products: one row of width 2048 12.7 / 12.7, of 4096 21.7 / 27.3; four rows (when
 // this form still took them) 21.4 / 11.4 and 51.9 / 27.1.  Two rows of w a warp halve the warps in flight: 8.4 for the first projection against 5.5.
 #pragma once
-#include "common.cuh"
+#include "row_loads.cuh"
 
 namespace llb {
 namespace {
 
 constexpr int SR_MAX = 2, SR_THREADS = 256, SR_WARPS = SR_THREADS / 32;
-
-// 16 bytes of weights, read once (asm volatile: the loads stay together ahead of the sums; left to the compiler they went one by one)
-__device__ __forceinline__ uint4 sr_ld(const __nv_bfloat16* row, int piece) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(reinterpret_cast<const uint4*>(row) + piece));
-  return v;
-}
-__device__ __forceinline__ void sr_floats(const uint4& u, float (&x)[8]) {
-  x[0] = __uint_as_float(u.x << 16), x[1] = __uint_as_float(u.x & 0xffff0000u), x[2] = __uint_as_float(u.y << 16), x[3] = __uint_as_float(u.y & 0xffff0000u);
-  x[4] = __uint_as_float(u.z << 16), x[5] = __uint_as_float(u.z & 0xffff0000u), x[6] = __uint_as_float(u.w << 16), x[7] = __uint_as_float(u.w & 0xffff0000u);
-}
-// acc += the products of eight bf16 numbers with eight of x
-__device__ __forceinline__ void sr_dot(float& acc, const float (&w)[8], const float (&x)[8]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) acc = fmaf(w[i], x[i], acc);
-}
 
 // y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; past the end of k a lane takes the last piece again and
 // drops its sum (times zero an infinite weight would be no number; zeroed weights, or rounds without a check before the last, are slower).
