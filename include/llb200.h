@@ -217,7 +217,7 @@ LL_API int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const voi
 LL_API int ll_int4_rows_error(void);
 /* Batches of 1 to 128 rows from the same checkpoint bytes: y = x . W^T (+ bias), or, of two layers that read the same x, the gated product as
  * ll_int4_rows_gated rounds it.  Sizes as for ll_int4_rows; scratch: ll_int4_batch_scratch_bytes (layers: 1, or 2 for the gated form) on a
- * 16-byte boundary, of any contents; grid: ranges that the work is cut into at most (0: one an SM). */
+ * 16-byte boundary, of any contents; grid: ranges that the work is cut into at most (0: one an SM), the same for the size and the launch. */
 LL_API size_t ll_int4_batch_scratch_bytes(int M, int N, int K, int layers, int grid);
 LL_API int ll_int4_batch(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch, int M,
                          int N, int K, int group, int grid, ll_stream stream);
@@ -260,7 +260,8 @@ LL_API int ll_int8_quantize_weight(const void* w /*[N][K]*/, int w_dtype, int8_t
 /* ref: bnb MatMul8bitLt forward (has_fp16_weights=False, threshold) as reached through quantization.py:36-45:
  * y[M][N] = int8 matmul of the row-quantised non-outlier part + fp16 outlier-column part (+ bias), in the
  * activation dtype.  K % 128 == 0.  workspace: ll_int8_workspace_bytes(M, N, K) bytes, 256-byte aligned; with those of min(M, 64) rows
- * M > 64 runs as passes of 64 rows (the same results: a feature is an outlier for a block of 64 rows). */
+ * M > 64 runs as passes of 64 rows (the same results, but for the order of sums of more than 64 outliers: a feature is an outlier for a block
+ * of 64 rows).  More than 64 rows take up to 8192 at a time; with 16-bit room for the outlier part of each output. */
 LL_API size_t ll_int8_workspace_bytes(int M, int N, int K);
 /* Two layers that read the same bf16 x, and their gated product: h[M][N] = silu(x . W1^T (+ bias1)) * (x . W2^T (+ bias2)), every step rounded
  * as ll_int8_linear twice and ll_silu_mul round it; x is prepared once. */
@@ -751,12 +752,12 @@ LL_API int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, i
                                 int splits, int form, int maps, float diff_lambda, float diff_post, float eps, float* scratch,
                                 void* y, int y_stride, ll_stream stream);
 
-/* One token of 1 to 8 sequences (bf16) through a whole attention layer in one call: the input projection, the step's cache rows, attention and
+/* One token of 1 or 2 sequences (bf16) through a whole attention layer in one call: the input projection, the step's cache rows, attention and
  * the output projection, in the roundings of the separate calls and dense layers.  x [B][width], w_in [n_in][width], w_o [width][heads * v_dim].
  * Latent: w_uk [heads][nope][kv_rank], w_uv_t [heads][kv_rank][v_dim]; columns of the projection: queries first, gate_col0 (one logit a head;
  * < 0: none), kv_col0; kv_norm NULL: the cache is another layer's and already holds the rows.  Softmax (one score map, queries and keys that
- * turn or are normed): columns of queries, keys, values (< 0: the un-rotated keys) and gate (< 0: none).  Sizes in multiples of 8; scratch of
- * the given bytes, any contents, 256-byte aligned. */
+ * turn or are normed): columns of queries, keys, values (< 0: the un-rotated keys) and gate (< 0: none).  Widths, ranks and value sizes in
+ * multiples of 8, kv_rank and nope up to 1024; scratch of the given bytes, any contents, 256-byte aligned.  Other sizes: LL_ERR_UNSUPPORTED. */
 LL_API size_t ll_latent_step_scratch_bytes(int B, int n_in, int heads, int kv_rank, int v_dim, int splits);
 LL_API int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm,
                           float eps, const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim,

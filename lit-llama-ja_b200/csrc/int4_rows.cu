@@ -7,7 +7,8 @@
 // activations are the B operand, tiles of bn rows x 128 k loaded by TMA.  A pair of CTAs forms one product of 256 weight columns (128 = the
 // TMEM lanes of each) x bn rows, and each CTA brings half of the rows: of a CTA of its own x takes 72 KB a step of 128 k at 256 rows from L2,
 // 46 bytes a clock and SM; the pair needs 40 KB.  Unpacking reads the bytes by transposing loads (64 single-byte loads a thread before) and
-// the scales from shared memory; nothing of the loop may spill or miss in what is left of L1 (a spilled register doubled a step's time).
+// the scales from shared memory; the loop's registers may not spill or miss in what is left of L1 (that doubled a step's time; of the plain form
+// ptxas spills one register, stored and loaded once each).
 // us, one CTA a tile / pairs: 11008 x 4096 at 150, 512, 1100 rows 28 / 24, 51 / 46, 82 / 69; 4096 x 11008 at 150, 512 rows 53 / 48, 87 / 54;
 // 32000 x 4096 at 512 rows 140 / 103.  Bound by products at 256 rows a tile (0.84 us a step with all SMs busy, 0.76 at the rate of a large
 // dense product), below that by unpacking.
@@ -385,7 +386,7 @@ int r4_out_map(const void* y, int M, int N, CUtensorMap* out) {
 }
 
 // Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time, plus the drain.  A step costs its products, or, with
-// few rows, its unpacking (us a step of 13824 x 5120, 900 rows, tiles of 128 / 160 / 192 / 224 / 256 rows: .54 / .56 / .61 / .66 / .78).
+// few rows, its unpacking (us a step of 13824 x 5120, 900 rows, tiles of 128 / 160 / 192 / 224 / 256 rows: .54 / .56 / .61 / .66 / .78, the last with six pairs idle in its third wave).
 long long r4_cost(int M, int N, int tile_n, int steps, int bn, int pairs) {
   const long long tiles = (long long)((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n);
   const int products = 4 * bn, unpack = 530 + 7 * bn / 5;

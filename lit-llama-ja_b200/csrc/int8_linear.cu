@@ -11,7 +11,7 @@
 // quantised rows), one streams the weights as the A operand of tcgen05 kind::i8 MMAs (128 output columns = the 128 TMEM lanes, int32
 // accumulators) with K cut into ranges whose partial sums are stored, one adds them up (integers: exact in any order) and finishes.
 // Prompts (M > 64): the same arithmetic per block of 64 rows (a feature is an outlier for a block of 64 rows), all blocks at once: the same
-// preparation, then one kernel for the product and its finish (int8_pair_kernel).
+// preparation, a kernel for the outlier parts of long lists, then one for the product and its finish (int8_pair_kernel).
 // Either way the two layers of a gated feed-forward that read the same x go together: x is prepared once, one product over both, one finish.
 #include "tcgen05.cuh"
 

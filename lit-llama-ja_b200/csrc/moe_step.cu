@@ -7,8 +7,8 @@
 //
 // Bound by the weights' way from memory: 69 MB for one token of width 2048 (4 of 32 experts of 1024, a shared one of 1536), 10.6 us at the
 // copy rate.  The shared expert's blocks come first and do not wait for the router.
-// us a call (graphed), sorted and grouped with dense layers for the shared expert / here: that size at 1, 2, 4, 8 tokens 155 (69) / 32 (28),
-// 125 (73) / 40 (38), 97 (76) / 62 (59), 128 (113) / 94 (91).
+// us a call (graphed), sorted and grouped with dense layers for the shared expert / here: that size at 1, 2, 4, 8 tokens 98 (72) / 25 (23),
+// 97 (77) / 34 (32), 99 (80) / 51 (49), 122 (108) / 80 (77).  Which steps come here: by what they read again (the module's rule).
 #include "row_loads.cuh"
 
 namespace llb {

@@ -21,7 +21,8 @@ def _entries_per_byte(bits: int) -> int:
     return epb
 
 
-# What the library says of sizes alone: asked once for each, not on every call.
+# What the library says of sizes alone: asked once for each, not on every call.  (It counts the SMs of a device once a process: the sizes asked for
+# here and the launches go by the same number.)
 @functools.lru_cache(maxsize=4096)
 def _rows_supported(Nout: int, K: int, group: int) -> bool:
     return bool(N.call_ret("ll_int4_rows_supported", Nout, K, group))
@@ -174,6 +175,10 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     # Past 6144 rows a bf16 copy of W, written once, costs less than a tile of W de-quantised again for every 256 rows.  us, feed-forwards of
     # widths 2048 / 4096 / 5120 (two layers in the gated form, one plain), this kernel and copies with their products: 2048 rows
     # 128 / 474 / 748 and 137 / 527 / 854, 6000 rows 393 / 1367 / 2159 and 369 / 1409 / 2145, 8192 rows 531 / 1884 / 3098 and 504 / 1827 / 2882.
+    # The line is flat: single layers, this kernel / copy, at 4096, 6144, 8192 rows 4096 x 4096 102 / 107, 148 / 154, 198 / 190; 11008 x 4096
+    # 300 / 312, 399 / 394, 602 / 549; 4096 x 11008 334 / 355, 434 / 469, 516 / 522; 5120 x 13824 422 / 467, 732 / 719, 925 / 1042;
+    # 5632 x 2048 94 / 82, 128 / 117, 158 / 153.  Of the gated pairs alone the copies are the faster ones from about 4000 rows on (11008 x 4096
+    # 627 / 583, 933 / 798, 1316 / 1116; 5632 x 2048 207 / 156, 274 / 214, 396 / 279).
     ROWS_MIN_M, ROWS_MAX_M = 129, 6144
 
     def _rows_eligible(self, x) -> bool:
@@ -194,7 +199,8 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         return x.dtype == torch.bfloat16 and self.in_features % 8 == 0 and (self.bias is None or self.bias.dtype == torch.bfloat16)
 
     def _fused_gemm_eligible(self, x) -> bool:
-        """9 <= M <= 128 bf16 rows on a layer whose scale groups are multiples of 128: the fused tcgen05 de-quantise + GEMM."""
+        """bf16 rows on a layer whose scale groups are multiples of 128: the fused tcgen05 de-quantise + GEMM on the packed stream.  (It still
+        runs for layers that the byte kernel leaves: zeros of another dtype than the scales, parameters in strided rows.)"""
         return (self.bits == 4 and x.dtype == torch.bfloat16 and self.scales.dtype == torch.bfloat16
                 and self.out_features % 128 == 0 and self.tile_cols % 128 == 0 and self.in_features % self.tile_cols == 0
                 and (self.bias is None or self.bias.dtype == torch.bfloat16))
@@ -214,8 +220,10 @@ class ColBlockQuantizedLinear(torch.nn.Module):
     # ------------------------------------------------------------------ row F
     def forward(self, inp):
         """ref: quantization.py:411-421.  M <= 8 bf16 rows: TMA-streamed int4 GEMV (exact (q - zero) * scale,
-        fp32 accumulation); small M in other dtypes / bit widths: reference-semantics SIMT kernel;
-        large M: dequant-GEMM."""
+        fp32 accumulation); more rows of 4-bit layers with groups in multiples of 128: from the checkpoint bytes, up to 128 rows
+        (and fewer than 9 that the GEMV does not take, or whose stream a capture does not find) ``ll_int4_batch``, up to
+        ROWS_MAX_M ``ll_int4_rows``; small M in other dtypes / bit widths: reference-semantics SIMT kernel; the rest:
+        dequant-GEMM."""
         qw = self._packed_ptr_ok()
         N.require_cuda(inp, qw)
         K, Nout = self.in_features, self.out_features

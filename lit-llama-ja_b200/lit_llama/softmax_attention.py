@@ -51,8 +51,10 @@ def pad8(n: int) -> int:
     return (n + 7) // 8 * 8
 
 
-# Sequences of a step that takes the layer's one call.  us a call, before and after: one token of width 2048 over 1000 keys 66 -> 39 (with the walk over the keys several at a time), two sequences 67 -> 43; replayed as a graph
-# 57 -> 32 and 59 -> 36.
+# Sequences of a step that takes the layer's one call.  us, separate calls / one, replayed as a graph (called), every layer's weights and keys from
+# memory, one token over 100, 1000 and 4000 keys in ranges of 64: width 1024 34 / 26 (72 / 37), 36 / 29 (57 / 36), 56 / 52 (67 / 55); 2048
+# 38 / 31 (51 / 35), 41 / 35 (58 / 40), 60 / 54 (72 / 60); 4096 55 / 47 (65 / 52), 59 / 51 (71 / 58), 79 / 65 (88 / 71).  Two sequences 33 / 28 to
+# 55 / 55, 37 / 33 to 59 / 59, 55 / 53 to 80 / 74; 32 key heads over 4000 keys 90 / 92 (100 / 98).
 # From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
 
