@@ -462,7 +462,7 @@ def reference_gpu(model, device):
     """The bar: the reference's own GPU path on this B200, identical weights (the model's state dict loaded
     into the unmodified reference's LLaMA from baseline/_ref): decode tokens/s of its LLaMA.forward with KV cache, batch 1.
     Group 128 takes its get_weight + F.linear branch (ref quantization.py:420-421); its Triton kernel only serves per-row
-    scales (measured by profiles/parity_7b.py --per-row)."""
+    scales, and at 512 rows returns wrong values on this image's Triton."""
     import torch
 
     try:

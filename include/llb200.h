@@ -138,7 +138,7 @@ LL_API int ll_q8_prepare(const uint8_t* qw, const void* scales, const void* zero
 /* Footprint parity of a batch-1 launch inside a PDL chain (stream kind 1 only).  Consecutive GEMVs of a chain alternate
  * EVEN / ODD: an EVEN launch asks for 116 KB of shared memory (two EVEN CTAs cannot share an SM), an ODD launch carries
  * two idle warps (two ODD CTAs exceed the register file), an EVEN + ODD pair fits - so the block scheduler can never put
- * two CTAs of the SAME GEMV on one SM, whatever else is resident (profiles/r02_gemv_experiments.md section 6). */
+ * two CTAs of the SAME GEMV on one SM, whatever else is resident. */
 #define LL_GEMV_EVEN 4
 #define LL_GEMV_ODD 2
 

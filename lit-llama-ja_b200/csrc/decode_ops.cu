@@ -194,8 +194,7 @@ template <> struct vec_ld<float> {
 };
 
 // Registers: 151 at the natural allocation.  Capping the kernel at 128 (so that two CTAs fit an SM next to a GEMV
-// CTA) costs 10 % of its time and does not remove the penalty of overlapping it with the neighbouring GEMVs
-// (profiles/r01_gemv_experiments.md).
+// CTA) costs 10 % of its time and does not remove the penalty of overlapping it with the neighbouring GEMVs.
 // CL: the splits of one (batch, head) form a thread-block cluster (nsplit <= 8) and hand their partial states to the
 // cluster's first CTA through distributed shared memory - no global scratch, fence, atomic or reload on the way.
 template <typename T, int HS, bool CL>
@@ -365,7 +364,7 @@ __global__ void __launch_bounds__(128) decode_attn_kernel(const T* __restrict__ 
 
 // ---------------------------------------------------------------- decode attention, K/V staged ahead of the wait
 // The kernel above is latency-bound: after the c_attn GEMV retires it pays position -> K/V rows -> combine as dependent
-// memory round trips (3.2 us of its 9.4 us per layer at position 640, profiles/r02_gemv_experiments.md).  Only ONE row of
+// memory round trips (3.2 us of its 9.4 us per layer at position 640).  Only ONE row of
 // the layer's cache changes in this step - the slot the c_attn epilogue writes - so everything else can be in shared
 // memory before the producer finishes.  As a programmatic dependent this kernel
 //   1. BEFORE griddepcontrol.wait: reads the position (a guess: the kernel that advanced it may formally still be running),

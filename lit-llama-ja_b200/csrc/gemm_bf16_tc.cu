@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(64 + 32 * W4_DW, 1) gemm_w4_tc_kernel(const __
     tc_fence_after();
     tmem_dealloc(tmem_base, 256);
   }
-  // (Measured, profiles/r02_fused_gemm.md: reducing inside the kernel - the last k-split to arrive sums the tile - and two
+  // (Measured: reducing inside the kernel - the last k-split to arrive sums the tile - and two
   // CTAs per SM were both SLOWER than a separate reduce kernel and one CTA per SM: 2.95 -> 3.76 ms per 161 Linears at
   // batch 32.  The code stays behind a constant for the record.)
   if (W4_REDUCE_IN_KERNEL && p.ksplit > 1) {

@@ -29,7 +29,6 @@
 //    plain store, residual add, RoPE + KV-cache write (c_attn), SwiGLU (c_fc1/c_fc2 as two matrices
 //    of one launch), or peer stores for the tensor-parallel push.  The decode chain's configuration
 //    gets one instantiation per (epilogue, norm, batch 1): less cold code per launch.
-//  * Measurements, ablations and rejected variants: profiles/r01_gemv_experiments.md.
 //    Tuning switches (-D): LLB_XPRED, LLB_SHIFT_FMA, LLB_XSTAGE_TMA, LLB_TRACE, LLB_ABL_* (timing
 //    ablations, wrong sums) - build with `build.py --variant`, select with LLB200_LIB.
 #include <stdlib.h>
@@ -161,7 +160,7 @@ __device__ __forceinline__ void mbar_wait_u32(uint32_t bar, uint32_t parity) {
 // runs its prologue and epilogue once - and no epilogue dispatch); -1: taken from the arguments.
 // MM > 0: the batch (rows of x) is the compile-time constant MM (batch-1 decode: every per-row loop folds away).
 // (A neighbour stream-K split of the boundary tiles was built and measured: q 311 -> 361, p 131 -> 199, f 423 -> 519,
-// d 277 -> 325 us per 32 layers - slower than the 7-14 % tile imbalance it removes; taken out, profiles/r02_gemv_experiments.md.)
+// d 277 -> 325 us per 32 layers - slower than the 7-14 % tile imbalance it removes; taken out.)
 template <int W, int KSP, int BPW, int EPI = -1, int NORM = -1, int MM = 0>
 __global__ void __launch_bounds__((W + 1) * 32, (W >= 12 ? 1 : 2)) gemv_int4_kernel(const __grid_constant__ Params p) {
   const int epilogue = EPI >= 0 ? EPI : p.epilogue;
@@ -551,7 +550,7 @@ __global__ void __launch_bounds__((W + 1) * 32, (W >= 12 ? 1 : 2)) gemv_int4_ker
         for (int i = 0; i < 4; ++i) t[b][i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
       }
       // the folds come after all of the chunk's MMAs (measured: folding block b behind block b+1's MMAs and
-      // handing the slot back before the last fold is 7 % slower, profiles/r01_gemv_experiments.md)
+      // handing the slot back before the last fold is 7 % slower)
 #pragma unroll
       for (int b = 0; b < BPW; ++b) {
         const float s0 = __uint_as_float(sz[b].x << 16), zn0 = __uint_as_float(sz[b].x & 0xffff0000u);
@@ -729,7 +728,7 @@ __global__ void int4_repack_kernel(const uint8_t* __restrict__ qw, const P* __re
 
 // ==================================================================================== batch-1 kernel, integer MMA
 // The decode chain's kernel (M = 1, scale groups of a multiple of 128): the same ring / tile split / epilogues as above with
-// a cheaper main loop.  profiles/r02_gemv_experiments.md: the bf16 loop above is bound by instruction ISSUE (ALU-pipe
+// a cheaper main loop: the bf16 loop above is bound by instruction ISSUE (ALU-pipe
 // instructions hold the issue port for two cycles: 7 of them per 8 weights + bookkeeping = 24 slots per 32-bit word), not
 // by HBM or the tensor pipe.  Here:
 //  * stream kind 1 (ll_int4_prepare kind = 1): a 32-bit word holds 4 k-consecutive nibbles of output column g in the LOW
@@ -1386,7 +1385,7 @@ void consumer_config(int M, int KSP, int* W, int* BPW) {
       }
     }
   }
-  // measured on the 7B decode chain (profiles/r01_step_probe.md): 8 warps x 2 blocks beats 12 x 1 by 6 %
+  // measured on the 7B decode chain: 8 warps x 2 blocks beats 12 x 1 by 6 %
   if (M <= 2) { *W = 8; *BPW = KSP == 4 ? 2 : 1; } else if (M <= 4) { *W = 8; *BPW = 1; } else { *W = 4; *BPW = 1; }
   if (M <= 2 && KSP == 4 && env_w > 0) { *W = env_w; *BPW = env_b; }
 }

@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(1024) tp_allreduce_add_kernel(const __grid_con
   __shared__ int s_epoch;
   // use_pdl: a link of the programmatic-launch chain.  It was once launched plainly because an early
   // launch behind it cost time - the cause was CTA placement (a 148-CTA GEMV grid released while a fat CTA holds an SM
-  // doubles up elsewhere, profiles/r02_gemv_experiments.md section 6), cured by the EVEN / ODD GEMV footprints.  With them
+  // doubles up elsewhere), cured by the EVEN / ODD GEMV footprints.  With them
   // the next GEMV's CTAs can start (barriers, norm weights, ring fill from HBM) while the flags and partial sums travel,
   // and this kernel's own launch latency hides behind the row-parallel GEMV.  Everything that touches data comes after
   // the wait.

@@ -90,11 +90,11 @@ class DecodeEngine:
         self.rope = model._rope_f32
         self.use_pdl = _env_flag("LLB200_PDL", True)
         self.use_graph = _env_flag("LLB200_GRAPH", True)
-        # measured (profiles/r01_step_probe.md): launching the attention kernel itself with the programmatic
+        # measured: launching the attention kernel itself with the programmatic
         # attribute costs ~8 us per block (its 512 waiting CTAs crowd the SMs the GEMV pair shares)
         # LLB200_GEMV_PARITY=1: consecutive GEMVs alternate EVEN / ODD footprints (include/llb200.h) so that two CTAs of the
         # same GEMV can never share an SM; the attention kernel can then be a programmatic dependent too
-        # (measured, profiles/r02_gemv_experiments.md section 6: every SM then holds exactly one CTA of each GEMV and the
+        # (measured: every SM then holds exactly one CTA of each GEMV and the
         # 7B step drops 1360 -> 1339 us).  Default: on where every Linear of the chain takes the integer-MMA kernel (the
         # only one with the two footprints) on one GPU, and under tensor parallelism when the exchange kernel joins
         # the programmatic chain (below); with a plainly launched exchange kernel the GEMVs are separated anyway.
@@ -242,7 +242,7 @@ class DecodeEngine:
         signals arrival; a small kernel reduces from local memory (compute and the first half of the collective in
         one kernel; correct, but measured 4 % slower at 65B TP2: the system-scope release at the end of every GEMV
         CTA costs more than the pull it saves).  Both sit inside the step graph.  "nccl": dist.all_reduce + ll_add, run eagerly (a captured NCCL
-        collective next to programmatic-launch kernels stalled on the 2-GPU box, profiles/r01_tp.md)."""
+        collective next to programmatic-launch kernels stalled on two GPUs)."""
         import os
         B, E = self.x.shape
         rank, world, group = self.model._tp

@@ -11,9 +11,8 @@ Three references on identical weights and tokens:
       LLaMA.forward over ColBlockQuantizedLinear.forward - for group 128 its get_weight + F.linear branch
       (ref quantization.py:390-421), for per-row its Triton kernel (ref quantization.py:185-331; opt-in, see below).
 
-Layer count is 2 here; the full depth (32 layers, 512 + 256 steps on the reference's greedy stream, and the reference's own
-fp32 result on the same tokens) is run by profiles/parity_7b.py -> profiles/r02_parity_config2_*.json.  The stated
-tolerance is in TOL below.
+Layer count is 2 here; at full depth (32 layers, 512 + 256 steps on the reference's greedy stream, beside the reference's own
+fp32 result on the same tokens) the same comparison was made once.  The stated tolerance is in TOL below.
 """
 import ctypes as C
 import os
