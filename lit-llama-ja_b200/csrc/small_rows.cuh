@@ -12,8 +12,8 @@ namespace {
 
 constexpr int SR_MAX = 2, SR_THREADS = 256, SR_WARPS = SR_THREADS / 32;
 
-// y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; past the end of k a lane takes the last piece again and
-// drops its sum (times zero an infinite weight would be no number; zeroed weights, or rounds without a check before the last, are slower).
+// y[m][n] = x[m] . w[n], m < MT: a warp per row of w, eight 16-byte loads of it in flight; in the last round a lane past the end of k takes the last
+// piece again and zeros in its place (zero times an infinite weight would be no number; a check in every round costs the layer 2 %).
 // K, ldx multiples of 8, rows on 16-byte boundaries.
 template <int MT>
 __global__ void __launch_bounds__(SR_THREADS) small_linear_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const __nv_bfloat16* __restrict__ w,
@@ -27,25 +27,26 @@ __global__ void __launch_bounds__(SR_THREADS) small_linear_kernel(const __nv_bfl
   float acc[MT];
 #pragma unroll
   for (int m = 0; m < MT; ++m) acc[m] = 0.f;
-  for (int i = lane; i < pieces; i += 32 * U) {
+  auto round = [&](int i, bool whole) {        // whole: no lane's pieces lie past the end
     uint4 q[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) q[u] = sr_ld(row, min(i + 32 * u, pieces - 1));
+    for (int u = 0; u < U; ++u) q[u] = sr_ld(row, whole ? i + 32 * u : min(i + 32 * u, pieces - 1));
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const bool in = i + 32 * u < pieces;
+      const bool in = whole || i + 32 * u < pieces;
       float wf[8];
-      sr_floats(q[u], wf);
+      sr_floats(in ? q[u] : make_uint4(0u, 0u, 0u, 0u), wf);
 #pragma unroll
       for (int m = 0; m < MT; ++m) {
         float xf[8];
         sr_floats(in ? reinterpret_cast<const uint4*>(x + (size_t)m * ldx)[i + 32 * u] : make_uint4(0u, 0u, 0u, 0u), xf);
-        float sum = acc[m];
-        sr_dot(sum, wf, xf);
-        acc[m] = in ? sum : acc[m];
+        sr_dot(acc[m], wf, xf);
       }
     }
-  }
+  };
+  int i = lane;
+  for (const int end = pieces / (32 * U) * (32 * U); i < end; i += 32 * U) round(i, true);
+  if (i < pieces) round(i, false);
 #pragma unroll
   for (int m = 0; m < MT; ++m) {
     const float v = warp_sum(acc[m]);

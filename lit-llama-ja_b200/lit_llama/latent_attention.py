@@ -42,8 +42,8 @@ EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
 
 # Sequences of a step that takes the layer's one call.  us a call, separate calls / one: one token of width 2048 over 1024 of 2048 rows 88 / 45, of
 # 4096 over 300 104 / 58, two sequences 102 / 61; replayed as a graph 40.5 / 33.2, 53.9 / 51.2 and 60.4 / 55.4.  Graphed, every layer's weights
-# and rows from memory, over 300 and 2000 rows: width 1024 48 / 42 and 47 / 41, 2048 50 / 46 and 51 / 46, 4096 63 / 61 and 64 / 60; two sequences
-# 48 / 45 and 49 / 45, 52 / 49 and 52 / 50, 67 / 66 and 67 / 64.
+# and rows from memory, over 300 and 2000 rows: width 1024 48 / 42 and 47 / 41, 2048 50 / 46 and 50 / 45, 4096 63 / 59 and 63 / 58; two sequences
+# 48 / 43 and 50 / 44, 52 / 48 and 52 / 48, 66 / 63 and 66 / 62.
 # From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
 

@@ -52,9 +52,9 @@ def pad8(n: int) -> int:
 
 
 # Sequences of a step that takes the layer's one call.  us, separate calls / one, replayed as a graph (called), every layer's weights and keys from
-# memory, one token over 100, 1000 and 4000 keys in ranges of 64: width 1024 34 / 26 (72 / 37), 36 / 29 (57 / 36), 56 / 52 (67 / 55); 2048
-# 38 / 31 (51 / 35), 41 / 35 (58 / 40), 60 / 54 (72 / 60); 4096 55 / 47 (65 / 52), 59 / 51 (71 / 58), 79 / 65 (88 / 71).  Two sequences 33 / 28 to
-# 55 / 55, 37 / 33 to 59 / 59, 55 / 53 to 80 / 74; 32 key heads over 4000 keys 90 / 92 (100 / 98).
+# memory, one token over 100, 1000 and 4000 keys in ranges of 64: width 1024 34 / 26 (70 / 36), 36 / 29 (56 / 35), 56 / 52 (67 / 55); 2048
+# 38 / 31 (50 / 35), 42 / 35 (56 / 40), 60 / 53 (72 / 58); 4096 55 / 45 (63 / 50), 58 / 49 (71 / 56), 77 / 62 (87 / 68).  Two sequences 33 / 27 to
+# 55 / 53, 37 / 32 to 59 / 57, 55 / 50 to 80 / 71; with 32 key heads of width 4096 62 / 61 (69 / 65) to 90 / 93 (99 / 100).
 # From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
 
