@@ -1,34 +1,25 @@
-// Grouped expert GEMM of the mixture-of-experts feed-forward on the 5th-generation tensor cores
-// (tcgen05 + TMEM + TMA), for steps with many rows per expert (prefill).
+// Grouped expert GEMM of the mixture-of-experts feed-forward on the 5th-generation tensor cores (tcgen05 + TMEM + TMA).
 //
-// The (token, choice) pairs are sorted by expert (ll_moe_route) and the rows of the activations are
-// gathered into that order once (ll_moe_gather_rows), so every operand is a plain row-major matrix
-// that TMA can tile:
+// The (token, choice) pairs are sorted by expert (ll_moe_route) and the rows of the activations are gathered into that order once
+// (ll_moe_gather_rows), so every operand is a matrix that TMA can tile:
 //   mode 1 (GLU) : h[r][n] = glu(xs[r] . gate_e[n], xs[r] . up_e[n])     w [X][2N][K] = [gate; up]
 //   mode 3 (relu^2): h[r][n] = relu(xs[r] . up_e[n])^2                    w [X][N][K]
 //   mode 0 (down): y[perm[r]][n] = h[r] . down_e[n]                       w [X][N][K]
-// for the sorted rows r of expert e.  A CTA owns 128 sorted rows of ONE expert (found from the device-side
-// offsets, as in the mma.sync form: no host synchronisation) x 256 accumulator columns in TMEM:
-//   GLU : columns 0..127 = gate tile, 128..255 = up tile of the same 128 outputs; the clamped gated unit is
-//         the epilogue, applied to the two accumulators as they are read back from TMEM;
-//   relu^2: columns 0..255 = 256 outputs, squared as they are read back;
-//   down: columns 0..255 = 256 outputs, scattered to (token, choice) order by the epilogue.
-// A row tile may run past its expert's last row: those rows (the next expert's, or zero fill) are
-// computed and never stored.
-// One CTA per SM walks the tiles t = blockIdx.x, + gridDim.x, ... (column tiles first, so the tiles in flight share their
-// experts' weights and their rows in L2):
-//   warp 0   : TMA producer (A box 128 x 64, two B boxes 128 x 64, 128-byte swizzle) into a 4-stage ring that runs on across
-//              tiles
-//   warp 1   : TMEM allocation, one elected thread issues tcgen05.mma 128 x 256 x 16 (bf16 in, fp32 accumulate)
-//   warps 2-9: epilogue, one accumulator row and half of its columns per thread
-// Two accumulators of 256 TMEM columns alternate, so the epilogue of a tile (an exponential, a division and scattered rows
-// of stores, about half as long as the main loop) and the search for the next one run under the main loop of the next.  One
-// tile per CTA, two CTAs per SM, left both in the open and dealt out whole tiles in three rounds where 2.2 would do:
-// 8192 rows of 32 experts, width 2048, ff 1024: gate and up 137 us -> 96 (0.72 PFLOP/s of rows that count), down 73 -> 56.
-// What bounds it now: 128-row tiles that are not full (a fifth of the products) and the operands' way from L2 (96 bytes a
-// clock and SM at the full rate of the products).
-// Every wait on an mbarrier is bounded; a wait that runs out records a code in g_moe_tc_error, the roles
-// stop, the CTA waits for its copies and products in flight (bounded), frees its TMEM and returns.
+// for the sorted rows r of expert e (found from the device-side offsets: no host synchronisation).
+//
+// The products are turned round: the WEIGHTS are the operand of 256 rows (a pair of CTAs, tcgen05 cta_group::2, 128 rows and accumulator lanes
+// each) and an expert's tokens are the columns, 32 to 256 of them in steps of 32.  An expert's weights always fill whole tiles, and the
+// tokens it happens to have are rounded up to 32 instead of 128; an expert of more than 256 tokens gets equal tiles.  The pair shares the
+// tokens (each CTA brings half of them).  GLU: a CTA's 128 rows are eight of gate and eight of up in turn (one box of a five-dimensional map),
+// so that a thread finds both numbers of an output in one load from tensor memory.
+// One pair per two SMs walks the tiles t = pair, + pairs, ... (an expert's token tiles innermost: they read the same weights):
+//   warp 0   : TMA producer (128 rows of w, half of the tokens, 64 k each, 128-byte swizzle) into a six-stage ring that runs on across tiles
+//   warp 1   : TMEM allocation; in rank 0 one elected thread issues tcgen05.mma 256 x n x 16 (bf16 in, fp32 accumulate)
+//   warps 2-9: epilogue, 32 tokens at a time: 16x256b loads from tensor memory, the unit, a transposing store into the warp's staging
+//              place (tokens of 32 or 64 bytes), whole sectors from there
+// Two accumulators of 256 TMEM columns alternate, so the epilogue of a tile runs under the main loop of the next.
+// Every wait on an mbarrier is bounded; a wait that runs out records a code in g_moe_tc_error, the roles of both CTAs
+// stop, copies and products in flight end, TMEM is freed.
 #include <algorithm>
 
 #include "tcgen05.cuh"
@@ -36,219 +27,281 @@
 namespace llb {
 namespace {
 
-constexpr int MT_BN = 128;                 // rows of one B box
-constexpr int MT_STAGES = 4;
-constexpr int MT_A_BYTES = BM * BK * 2, MT_B_BYTES = 2 * MT_BN * BK * 2;
-constexpr int MT_COLS = 256, MT_TMEM_COLS = 2 * MT_COLS;      // two accumulators
-constexpr int MT_EPI_WARPS = 8, MT_THREADS = 64 + 32 * MT_EPI_WARPS;
+constexpr int MT_STAGES = 6, MT_NMAX = 256, MT_NSTEP = 32;
+constexpr int MT_A_BYTES = 128 * BK * 2, MT_B_BYTES = MT_NMAX / 2 * BK * 2;
+constexpr int MT_EPI_WARPS = 8, MT_THREADS = 64 + 32 * MT_EPI_WARPS, MT_OUT = 32 * 64;      // staging of a warp: 32 tokens of 64 bytes
+constexpr size_t MT_SMEM = (size_t)MT_STAGES * (MT_A_BYTES + MT_B_BYTES) + MT_EPI_WARPS * MT_OUT + (2 * MT_STAGES + 4) * 8 + 32 + 1024;
 constexpr uint32_t MT_WAIT_LIMIT = 1u << 22;
 
 __device__ int g_moe_tc_error = 0;
 
+struct MtParams {
+  const int32_t* offsets;
+  const int32_t* perm;
+  __nv_bfloat16* c;
+  int X, N, nkb, ldc, vec;          // vec: rows of c are whole 16-byte pieces
+  int boxes;                        // GLU with N no multiple of 8: gate and up rows come in boxes of eight from a flat map
+  float limit, alpha, shift;
+  int* word;
+};
+struct MtFail {
+  volatile int* here;
+  uint32_t there;
+  int* word;
+};
+
 // A wait that ends: on its phase, when another role has given up, or after the limit.
-__device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, volatile int* fail, int* word, int code) {
+__device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, const MtFail& f, int code) {
   for (uint32_t i = 0; i < MT_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && *fail) return false;
+    if ((i & 255u) == 255u && *f.here) return false;
   }
-  *fail = 1;
+  *f.here = 1;
+  store_cluster_u32(f.there, 1u);
   atomicCAS(&g_moe_tc_error, 0, code);
-  wait_ran_out(word, 400 + code);
+  wait_ran_out(f.word, 400 + code);
   return false;
 }
 
-// Walk over the row tiles (128 sorted rows of one expert) in rising order; every role that needs them keeps its own.
+// Walk over the tiles in rising order; every role keeps its own.  Tile: 256 weight rows (column tile `ct`) x `cnt` sorted rows from `r0` on,
+// `n` columns of the product.
 struct MtWalk {
-  int e = -1, first = 0, next = 0;      // expert, its first row tile, the one after its last
-  int row = 0, end = 0;                 // its sorted rows
-  __device__ __forceinline__ bool seek(const int32_t* __restrict__ offsets, int X, int rt) {
-    while (rt >= next) {
+  int e = -1, first = 0, next = 0;      // expert, its first tile, the one after its last
+  int row = 0, count = 0, tiles = 1, step = 0;
+  int ct = 0, r0 = 0, cnt = 0, n = 0;
+  __device__ __forceinline__ bool seek(const int32_t* __restrict__ offsets, int X, int ncol, int t) {
+    while (t >= next) {
       if (++e >= X) return false;
       row = __ldg(offsets + e);
-      end = __ldg(offsets + e + 1);
+      count = __ldg(offsets + e + 1) - row;
+      tiles = (count + MT_NMAX - 1) / MT_NMAX;
       first = next;
-      next += (end - row + BM - 1) / BM;
+      next += tiles * ncol;
+      if (count > 0) step = ((count + tiles - 1) / tiles + MT_NSTEP - 1) / MT_NSTEP * MT_NSTEP;
     }
+    const int q = t - first;
+    ct = q / tiles;
+    const int at = (q - ct * tiles) * step;
+    r0 = row + at;
+    cnt = min(step, count - at);
+    n = (cnt + MT_NSTEP - 1) / MT_NSTEP * MT_NSTEP;
     return true;
   }
-  __device__ __forceinline__ int r0(int rt) const { return row + (rt - first) * BM; }
 };
 
-// 2-D tiled TMA load, default L2 policy (both operands are re-read by other CTAs through L2)
-__device__ __forceinline__ void tma_box(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                   smem_u32(dst)),
-               "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void pair_box3(void* dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void pair_box5(void* dst, const CUtensorMap* map, int x, int chunk, int e, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
+          smem_u32(dst)),
+      "l"(map), "r"(x), "r"(0), "r"(0), "r"(chunk), "r"(e), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void mt_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// 16 lanes x 32 columns: v[4 i + j] is lane (lane / 4) + 8 * (j / 2), column 8 i + 2 (lane % 4) + j % 2
+__device__ __forceinline__ void tmem_ld_16x32(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+        "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// four 8 x 8 blocks of packed pairs, transposed: the lane's address is the place of eight numbers of token `lane`
+__device__ __forceinline__ void store_tokens(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(MT_THREADS, 1) moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
-                                                                    const __grid_constant__ CUtensorMap map_b,
-                                                                    const int32_t* __restrict__ offsets, const int32_t* __restrict__ perm,
-                                                                    int X, int N, int K, float limit, float alpha, float shift,
-                                                                    __nv_bfloat16* __restrict__ c, int ldc, int* word) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
+    moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_t64,
+                         const __grid_constant__ CUtensorMap map_t16, const MtParams p) {
+  constexpr int OUTS = MODE == 1 ? 64 : 128;             // outputs of a CTA's 128 rows
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
   uint8_t* sa = base;                              // [STAGES][128][64] bf16, swizzled
-  uint8_t* sb = base + MT_STAGES * MT_A_BYTES;     // [STAGES][256][64]
-  uint64_t* full = reinterpret_cast<uint64_t*>(sb + MT_STAGES * MT_B_BYTES);
+  uint8_t* sb = sa + MT_STAGES * MT_A_BYTES;       // [STAGES][up to 128][64]
+  uint8_t* so = sb + MT_STAGES * MT_B_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(so + MT_EPI_WARPS * MT_OUT);      // used in rank 0
   uint64_t* empty = full + MT_STAGES;
   uint64_t* acc_full = empty + MT_STAGES;          // [2]
-  uint64_t* acc_empty = acc_full + 2;              // [2]
-  uint64_t* drained = acc_empty + 2;
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(drained + 1);
-  int* s_tiles = reinterpret_cast<int*>(tmem_ptr + 1);
-  volatile int* s_fail = s_tiles + 1;
+  uint64_t* acc_empty = acc_full + 2;              // [2], used in rank 0: both CTAs' warps arrive
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int NCOL = MODE == 1 ? MT_BN : MT_COLS;      // outputs of a tile
-  const int ncol = (N + NCOL - 1) / NCOL;
-  const int nkb = (K + BK - 1) / BK;
-  if (warp == 0) {
-    int n = 0;
-    for (int e = lane; e < X; e += 32) n += (offsets[e + 1] - offsets[e] + BM - 1) / BM;
-    n = __reduce_add_sync(0xffffffffu, n);
-    if (lane == 0) {
-      *s_tiles = n * ncol;
-      *s_fail = 0;
-      prefetch_tensormap(&map_a);
-      prefetch_tensormap(&map_b);
-      for (int i = 0; i < MT_STAGES; ++i) {
-        mbar_init(&full[i], 1);
-        mbar_init(&empty[i], 1);
-      }
-      for (int i = 0; i < 2; ++i) {
-        mbar_init(&acc_full[i], 1);
-        mbar_init(&acc_empty[i], MT_EPI_WARPS);
-      }
-      mbar_init(drained, 1);
-      fence_barrier_init();
-    }
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int rank = (int)cluster_rank();
+  if (threadIdx.x == 0) {
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_t64);
+    prefetch_tensormap(&map_t16);
+    for (int i = 0; i < MT_STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * MT_EPI_WARPS);
+    *s_fail = 0;
+    fence_barrier_init();
   }
-  if (warp == 1) tmem_alloc(tmem_ptr, MT_TMEM_COLS);
+  if (warp == 1) pair_tmem_alloc(tmem_ptr, 2 * MT_NMAX);
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   tc_fence_after();
-  const uint32_t tmem_d = *tmem_ptr;
-  const int tiles = *s_tiles;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  const MtFail fail{s_fail, cluster_addr(s_fail, (uint32_t)(rank ^ 1)), p.word};
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, nkb = p.nkb;
+  const int ncol = (p.N + 2 * OUTS - 1) / (2 * OUTS);
+  pdl_wait();
+  pdl_launch_dependents();
 
   if (warp == 0) {
     if (elect_one()) {
       MtWalk walk;
-      int s = 0, issued = 0;
-      uint32_t phase = 0;
+      int s = 0;
+      uint32_t ph = 1;
       bool ok = true;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int rt = t / ncol, n0 = (t - rt * ncol) * NCOL;
-        if (!walk.seek(offsets, X, rt)) break;
-        const int r0 = walk.r0(rt);
-        // rows of the expert's weight matrix under the two B boxes
-        const int brow0 = MODE == 1 ? walk.e * 2 * N + n0 : walk.e * N + n0;
-        const int brow1 = MODE == 1 ? brow0 + N : brow0 + MT_BN;
+      for (int t = pair; ok && walk.seek(p.offsets, p.X, ncol, t); t += pairs) {
+        const int half = walk.n / 2, r0 = walk.r0 + rank * half, n0 = (walk.ct * 2 + rank) * OUTS;
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mt_wait(&empty[s], phase ^ 1, s_fail, word, 1)) { ok = false; break; }
-          mbar_expect_tx(&full[s], MT_A_BYTES + MT_B_BYTES);
-          tma_box(sa + s * MT_A_BYTES, &map_a, kb * BK, r0, &full[s]);
-          tma_box(sb + s * MT_B_BYTES, &map_b, kb * BK, brow0, &full[s]);
-          tma_box(sb + s * MT_B_BYTES + MT_BN * BK * 2, &map_b, kb * BK, brow1, &full[s]);
-          issued = 1;
-          if (++s == MT_STAGES) { s = 0; phase ^= 1u; }
+          if (!(ok = mt_wait(&empty[s], ph, fail, 1))) break;
+          if (rank == 0) mbar_expect_tx(&full[s], (uint32_t)(2 * (MT_A_BYTES + half * BK * 2)));      // both CTAs' operands
+          const uint32_t bar = cluster_addr(&full[s], 0);
+          uint8_t *da = sa + s * MT_A_BYTES, *db = sb + s * MT_B_BYTES;
+          if (MODE != 1) {
+            pair_box3(da, &map_w, kb * BK, n0, walk.e, bar);
+          } else if (!p.boxes) {
+            pair_box5(da, &map_w, kb * BK, n0 / 8, walk.e, bar);
+          } else {
+            const int y = walk.e * 2 * p.N + n0;
+            for (int j = 0; j < 8; ++j) {
+              pair_box(da + j * 2048, &map_w, kb * BK, y + 8 * j, bar);
+              pair_box(da + j * 2048 + 1024, &map_w, kb * BK, y + p.N + 8 * j, bar);
+            }
+          }
+          int r = 0;
+          for (; r + 64 <= half; r += 64) pair_box(db + r * BK * 2, &map_t64, kb * BK, r0 + r, bar);
+          for (; r < half; r += 16) pair_box(db + r * BK * 2, &map_t16, kb * BK, r0 + r, bar);
+          if (++s == MT_STAGES) s = 0, ph ^= 1u;
         }
       }
-      if (!ok && issued) {   // give the copies already issued time to land before the CTA leaves
-        for (int w = 0; w < 2048; ++w) __nanosleep(512);
-      }
+      if (!ok) let_issued_work_end();
     }
   } else if (warp == 1) {
     if (elect_one()) {
-      constexpr uint32_t idesc = instr_desc_bf16(BM, 2 * MT_BN);
-      int s = 0, i = 0;
-      uint32_t phase = 0;
+      const uint64_t ad = smem_desc_sw128(smem_u32(sa)), bd = smem_desc_sw128(smem_u32(sb));
+      MtWalk walk;
       bool ok = true;
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++i) {
-        const uint32_t d = tmem_d + (uint32_t)((i & 1) * MT_COLS);
-        if (!mt_wait(&acc_empty[i & 1], ((i >> 1) & 1) ^ 1, s_fail, word, 4)) break;
+      int s = 0, i = 0;
+      uint32_t ph = 0;
+      for (int t = pair; rank == 0 && ok && walk.seek(p.offsets, p.X, ncol, t); t += pairs, ++i) {
+        const uint32_t d = tmem + (uint32_t)((i & 1) * MT_NMAX), idesc = instr_desc_bf16(256, 0) | ((uint32_t)(walk.n >> 3) << 17);
+        if (!(ok = mt_wait(&acc_empty[i & 1], (uint32_t)((i >> 1) & 1) ^ 1u, fail, 4))) break;
         tc_fence_after();
         for (int kb = 0; kb < nkb; ++kb) {
-          if (!mt_wait(&full[s], phase, s_fail, word, 2)) { ok = false; break; }
+          if (!(ok = mt_wait(&full[s], ph, fail, 2))) break;
           tc_fence_after();
-          const uint64_t adesc = smem_desc_sw128(smem_u32(sa + s * MT_A_BYTES));
-          const uint64_t bdesc = smem_desc_sw128(smem_u32(sb + s * MT_B_BYTES));
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_bf16(d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
-          umma_commit(&empty[s]);
-          if (++s == MT_STAGES) { s = 0; phase ^= 1u; }
+            mt_mma(d, ad + (uint64_t)(s * (MT_A_BYTES >> 4) + 2 * k), bd + (uint64_t)(s * (MT_B_BYTES >> 4) + 2 * k), idesc, (kb | k) != 0 ? 1u : 0u);
+          pair_commit(&empty[s]);
+          if (++s == MT_STAGES) s = 0, ph ^= 1u;
         }
-        if (ok) umma_commit(&acc_full[i & 1]);
+        if (ok) pair_commit(&acc_full[i & 1]);
       }
-      umma_commit(drained);      // on every path: nothing is in flight when the TMEM goes back
-      for (uint32_t w = 0; w < MT_WAIT_LIMIT && !mbar_try_wait(drained, 0); ++w) {
-      }
+      if (!ok) let_issued_work_end();
     }
   } else {
     const int quarter = warp & 3, part = (warp - 2) >> 2;   // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
-    const int rt_row = quarter * 32 + lane;
+    constexpr int DIMS = OUTS / 4, CHUNKS = DIMS / 8;       // outputs of a quarter, 16-byte pieces of a token
+    const uint32_t stage = smem_u32(so + (warp - 2) * MT_OUT);
+    // where the lane's token lies; pieces of neighbouring tokens change places so that eight tokens cover all banks
+    const int turn = MODE == 1 ? (lane >> 2) & 1 : (lane >> 1) & 3;
+    const uint32_t mine = stage + (uint32_t)(lane * DIMS * 2);
     MtWalk walk;
     int i = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++i) {
-      const int rt = t / ncol, n0 = (t - rt * ncol) * NCOL;
-      if (!walk.seek(offsets, X, rt)) break;
-      const int row = walk.r0(rt) + rt_row;
-      const bool row_ok = row < walk.end;
-      const long long dst_row = !row_ok || MODE != 0 ? (long long)row : (long long)perm[row];
-      __nv_bfloat16* dst = c + dst_row * ldc;
-      if (!__all_sync(0xffffffffu, mt_wait(&acc_full[i & 1], (i >> 1) & 1, s_fail, word, 3))) break;
+    for (int t = pair; walk.seek(p.offsets, p.X, ncol, t); t += pairs, ++i) {
+      const int n0 = (walk.ct * 2 + rank) * OUTS + quarter * DIMS;
+      if (!__all_sync(0xffffffffu, mt_wait(&acc_full[i & 1], (uint32_t)(i >> 1) & 1u, fail, 3))) break;
       tc_fence_after();
-      const uint32_t trow = tmem_d + (uint32_t)((i & 1) * MT_COLS) + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t td = tmem + (uint32_t)((i & 1) * MT_NMAX) + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c0 = part * (NCOL / 2); c0 < (part + 1) * (NCOL / 2); c0 += 32) {
-        if (n0 + c0 >= N) break;            // uniform over the warp
-        uint32_t v[32];
-        tmem_ld_32x32(trow + (uint32_t)c0, v);
-        float f[32];
-        if (MODE == 1) {
-          uint32_t u[32];
-          tmem_ld_32x32(trow + (uint32_t)(MT_BN + c0), u);
+      for (int c0 = part * 32; c0 < walk.cnt; c0 += 64) {
+        const int tok = c0 + lane;
+        int row = walk.r0 + tok;
+        if (MODE == 0 && tok < walk.cnt) row = p.perm[row];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float g = fminf(__uint_as_float(v[j]), limit);
-            const float up = fminf(fmaxf(__uint_as_float(u[j]), -limit), limit);
-            f[j] = g / (1.f + expf(-alpha * g)) * (up + shift);
-          }
-        } else {
+        for (int hl = 0; hl < 2; ++hl) {
+          uint32_t v[16];
+          tmem_ld_16x32(td + ((uint32_t)(16 * hl) << 16) + (uint32_t)c0, v);
+          if (MODE == 1) {
+            uint32_t o[4];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            f[j] = __uint_as_float(v[j]);
-            if (MODE == 3) f[j] = fmaxf(f[j], 0.f) * fmaxf(f[j], 0.f);
+            for (int j = 0; j < 4; ++j) {
+              float f[2];
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const float g = fminf(__uint_as_float(v[4 * j + q]), p.limit);
+                const float up = fminf(fmaxf(__uint_as_float(v[4 * j + 2 + q]), -p.limit), p.limit);
+                f[q] = g / (1.f + expf(-p.alpha * g)) * (up + p.shift);
+              }
+              o[j] = pack_bf16(f[0], f[1]);
+            }
+            store_tokens(mine + (uint32_t)((hl ^ turn) * 16), o[0], o[1], o[2], o[3]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              uint32_t o[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                float f0 = __uint_as_float(v[4 * j + 2 * q]), f1 = __uint_as_float(v[4 * j + 2 * q + 1]);
+                if (MODE == 3) f0 = fmaxf(f0, 0.f) * fmaxf(f0, 0.f), f1 = fmaxf(f1, 0.f) * fmaxf(f1, 0.f);
+                o[j] = pack_bf16(f0, f1);
+              }
+              store_tokens(mine + (uint32_t)(((2 * hl + q) ^ turn) * 16), o[0], o[1], o[2], o[3]);
+            }
           }
         }
-        const int col = n0 + c0;
-        if (row_ok && col + 32 <= N && (ldc & 7) == 0) {
+        __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t pk[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              pk[q] = (uint32_t)f32_to_bf16_bits(f[j * 8 + 2 * q]) | ((uint32_t)f32_to_bf16_bits(f[j * 8 + 2 * q + 1]) << 16);
-            *reinterpret_cast<uint4*>(dst + col + j * 8) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        for (int it = 0; it < CHUNKS; ++it) {
+          const int at = it * 32 + lane, tk = at / CHUNKS, ch = at % CHUNKS;
+          const int dst = __shfl_sync(0xffffffffu, row, tk);
+          const uint4 u = lds128(stage + (uint32_t)(tk * DIMS * 2 + ((ch ^ (MODE == 1 ? (tk >> 2) & 1 : (tk >> 1) & 3)) * 16)));
+          const int col = n0 + 8 * ch;
+          if (c0 + tk < walk.cnt && col < p.N) {
+            __nv_bfloat16* out = p.c + (size_t)dst * p.ldc + col;
+            if (p.vec) {
+              *reinterpret_cast<uint4*>(out) = u;
+            } else {
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+              for (int j = 0; j < 8 && col + j < p.N; ++j) out[j] = __ushort_as_bfloat16((uint16_t)(w[j >> 1] >> (16 * (j & 1))));
+            }
           }
-        } else if (row_ok) {
-          for (int j = 0; j < 32 && col + j < N; ++j) dst[col + j] = __float2bfloat16_rn(f[j]);
         }
         __syncwarp();
       }
-      __syncwarp();
       tc_fence_before();
-      if (lane == 0) mbar_arrive(&acc_empty[i & 1]);
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[i & 1], 0));
     }
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_d, MT_TMEM_COLS);
+    pair_tmem_dealloc(tmem, 2 * MT_NMAX);
   }
 }
 
@@ -261,21 +314,49 @@ __global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, long long ld
   for (int i = threadIdx.x; i < k16; i += blockDim.x) dst[i] = src[i];
 }
 
+int mt_encode(const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) {
+    set_error("cuTensorMapEncodeTiled entry point not available");
+    return LL_ERR_CUDA;
+  }
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d) base=%p", (int)r, base);
+    return LL_ERR_CUDA;
+  }
+  return LL_OK;
+}
+
+// The weights' map: GLU as (k, eight rows, gate or up, groups of eight, expert), boxes of 128 rows; else (k, row, expert).
+int mt_weight_map(const void* w, int mode, int X, int N, int K, CUtensorMap* out) {
+  const cuuint64_t row = (cuuint64_t)K * 2;
+  if (mode == 1 && N % 8 == 0) {
+    const cuuint64_t dims[5] = {(cuuint64_t)K, 8, 2, (cuuint64_t)N / 8, (cuuint64_t)X}, strides[4] = {row, row * N, row * 8, row * 2 * N};
+    const cuuint32_t box[5] = {(cuuint32_t)BK, 8, 2, 8, 1};
+    return mt_encode(w, 5, dims, strides, box, out);
+  }
+  if (mode == 1) return make_map(w, X * 2 * N, K, 8, out);
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)N, (cuuint64_t)X}, strides[2] = {row, row * N};
+  const cuuint32_t box[3] = {(cuuint32_t)BK, 128, 1};
+  return mt_encode(w, 3, dims, strides, box, out);
+}
+
 template <int MODE>
-int launch_moe_tc(const CUtensorMap& ma, const CUtensorMap& mb, const int32_t* offsets, const int32_t* perm, int X, int N, int K,
-                  float limit, float alpha, float shift, void* c, int ldc, int n_rows, cudaStream_t st) {
-  constexpr size_t smem = (size_t)MT_STAGES * (MT_A_BYTES + MT_B_BYTES) + (2 * MT_STAGES + 5) * 8 + 32 + 1024;
+int launch_moe_pair(const CUtensorMap& mw, const CUtensorMap& m64, const CUtensorMap& m16, const MtParams& p, int n_rows, cudaStream_t st) {
   static PerDevice configured;
   if (!configured) {
-    LL_CUDA(cudaFuncSetAttribute(moe_gemm_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    LL_CUDA(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MT_SMEM));
     configured.mark();
   }
-  const int ncols = MODE == 1 ? MT_BN : MT_COLS;
-  const long long most = (long long)((N + ncols - 1) / ncols) * ((n_rows + BM - 1) / BM + X);
+  const int cols = MODE == 1 ? 128 : 256;
+  const long long most = (long long)((p.N + cols - 1) / cols) * (n_rows / MT_NMAX + std::min(n_rows, p.X));
   LL_CHECK_ARG(most < (1ll << 30), "moe_grouped_gemm_tc: too many tiles");
-  const int grid = (int)std::min<long long>(most, sm_count() > 0 ? sm_count() : 148);
-  moe_gemm_tc_kernel<MODE><<<grid, MT_THREADS, smem, st>>>(ma, mb, offsets, perm, X, N, K, limit, alpha, shift, (__nv_bfloat16*)c, ldc, wait_word());
-  LL_LAUNCH_OK("moe_gemm_tc_kernel");
+  const int pairs = sm_count() > 1 ? sm_count() / 2 : 1;
+  LL_CUDA(launch(moe_gemm_pair_kernel<MODE>, dim3(2 * (unsigned)std::min<long long>(most, pairs)), dim3(MT_THREADS), MT_SMEM, st, true, mw, m64, m16, p));
+  LL_LAUNCH_OK("moe_gemm_pair_kernel");
   return LL_OK;
 }
 
@@ -308,13 +389,16 @@ int ll_moe_grouped_gemm_tc(const void* a, const void* w, const int32_t* offsets,
   if (n_rows == 0) return LL_OK;
   const long long wrows = (long long)n_experts * (mode == 1 ? 2 : 1) * N;
   LL_CHECK_ARG(wrows < (1ll << 31), "moe_grouped_gemm_tc: weight stack too tall for one tensor map");
-  CUtensorMap ma, mb;
-  if (int r = make_map(a, n_rows, K, BM, &ma)) return r;
-  if (int r = make_map(w, (int)wrows, K, MT_BN, &mb)) return r;
+  CUtensorMap mw, m64, m16;
+  if (int r = mt_weight_map(w, mode, n_experts, N, K, &mw)) return r;
+  if (int r = make_map(a, n_rows, K, 64, &m64)) return r;
+  if (int r = make_map(a, n_rows, K, 16, &m16)) return r;
+  const MtParams p{offsets, perm, (__nv_bfloat16*)c, n_experts, N, (K + BK - 1) / BK, ldc, ldc % 8 == 0 && N % 8 == 0, N % 8 != 0, limit, alpha, shift,
+                   wait_word()};
   cudaStream_t st = (cudaStream_t)stream;
-  if (mode == 1) return launch_moe_tc<1>(ma, mb, offsets, perm, n_experts, N, K, limit, alpha, shift, c, ldc, n_rows, st);
-  if (mode == 3) return launch_moe_tc<3>(ma, mb, offsets, perm, n_experts, N, K, limit, alpha, shift, c, ldc, n_rows, st);
-  return launch_moe_tc<0>(ma, mb, offsets, perm, n_experts, N, K, limit, alpha, shift, c, ldc, n_rows, st);
+  if (mode == 1) return launch_moe_pair<1>(mw, m64, m16, p, n_rows, st);
+  if (mode == 3) return launch_moe_pair<3>(mw, m64, m16, p, n_rows, st);
+  return launch_moe_pair<0>(mw, m64, m16, p, n_rows, st);
 }
 
 // 0, or the code of the first bounded wait that ran out in a kernel of this file (1: ring slot, 2: operands, 3: accumulator,

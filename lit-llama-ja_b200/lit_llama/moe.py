@@ -34,8 +34,8 @@ from . import _native as N
 from .feed_forward import glu_unit, relu_squared_
 
 # the tcgen05 path: at least this many (token, choice) rows in the step, and on average per expert
-TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "1024"))
-TC_MIN_ROWS_PER_EXPERT = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "48"))
+TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "128"))
+TC_MIN_ROWS_PER_EXPERT = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "1"))
 
 
 STEP_MAX_TOKENS, STEP_SMALL_EXPERT = 8, 1 << 22       # tokens of a step; ff * width
