@@ -541,6 +541,16 @@ LL_API int ll_moe_step(const void* x, const float* w_router, const float* bias, 
                        int n_groups, int keep_groups, int group_top, const void* w_gu, const void* w_down, const void* ws_in, const void* ws_down,
                        int M, int width, int n_experts, int top, int ff, int shared_ff, int shared_gate, int mode, float limit, float alpha,
                        float shared_limit, void* out, void* scratch, ll_stream stream);
+/* Any number of tokens (x [M][width] bf16, dense rows, widths in multiples of 8) in six launches on the tcgen05 tensor cores: the router with the
+ * shared expert's gate logit, the sort of the (token, choice) pairs, their rows in that order, first projections with their unit, second ones, the combination.  Arguments as
+ * ll_moe_step; out on a 16-byte boundary.  h, the experts' and the shared expert's results are rounded to bf16 between the kernels, the gate's
+ * logit stays fp32.  scratch: ll_moe_prompt_scratch_bytes, of any contents, on a 16-byte boundary. */
+LL_API int ll_moe_prompt_supported(int M, int width, int n_experts, int ff, int shared_ff);
+LL_API size_t ll_moe_prompt_scratch_bytes(int M, int width, int n_experts, int top, int ff, int shared_ff);
+LL_API int ll_moe_prompt(const void* x, const float* w_router, const float* bias, const float* correction, int score, float out_scale,
+                         int n_groups, int keep_groups, int group_top, const void* w_gu, const void* w_down, const void* ws_in, const void* ws_down,
+                         int M, int width, int n_experts, int top, int ff, int shared_ff, int shared_gate, int mode, float limit, float alpha,
+                         float shared_limit, void* out, void* scratch, ll_stream stream);
 /* out[m] = sum_k expert_w[m][k] * y[m * top + k]  (+ sigmoid(shared_gate[m * gate_ld]) * shared_y[m], when shared_y is
  * given; shared_gate NULL: the shared expert is added as it is). */
 LL_API int ll_moe_combine(const void* y, const float* expert_w, int top, const void* shared_y, int shared_ld,

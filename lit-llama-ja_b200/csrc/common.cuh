@@ -209,6 +209,13 @@ __device__ __forceinline__ uint64_t policy_evict_first() {
 // wait until every kernel this one depends on has completed and flushed.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A pointer to what the kernels waited for have left: loads through it stay behind the wait.  (A load through a const __restrict__ parameter
+// may be taken for one of memory that never changes while the kernel runs, and moved ahead of it.)
+template <typename T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  asm volatile("" : "+l"(p) : : "memory");
+  return p;
+}
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;

@@ -18,6 +18,13 @@
 //   warps 2-9: epilogue, 32 tokens at a time: 16x256b loads from tensor memory, the unit, a transposing store into the warp's staging
 //              place (tokens of 32 or 64 bytes), whole sectors from there
 // Two accumulators of 256 TMEM columns alternate, so the epilogue of a tile runs under the main loop of the next.
+// What bounds it: with few tokens the weights' way from HBM (64 tokens, 32 experts of 2048 x 1024: 5.7 TB/s while all pairs have a tile, and
+// 3.6 rounds of tiles dealt out in four); with many the shared memory's 128 bytes a clock, which a stage of 64 k passes through twice
+// (written and read: about 256 + n clocks where the products take 2 n).  8192 rows of 32 experts, width 2048, ff 1024: first projections 97 us
+// with 128-row tiles of one CTA, 72 so; second ones 57 and 45.
+// ll_moe_prompt chains the whole layer by programmatic launches; the shared expert's tiles stand before the experts' in the same launch, which
+// fills rounds and starts while the router and the sort still run.  Rows brought by gather4 copies instead of a gathering kernel: 301 us a layer
+// where it takes 188 (2048 tokens; 128-byte pieces are too many copies).
 // Every wait on an mbarrier is bounded; a wait that runs out records a code in g_moe_tc_error, the roles of both CTAs
 // stop, copies and products in flight end, TMEM is freed.
 #include <algorithm>
@@ -25,6 +32,13 @@
 #include "tcgen05.cuh"
 
 namespace llb {
+
+// moe_ops.cu: the router alone, and the combination, as parts of a chain of launches
+int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
+                   cudaStream_t st);
+int moe_combine_rows(const void* y, const float* expert_w, int top, const void* shared_y, const float* gate, void* out, int M, int dim, cudaStream_t st);
+
 namespace {
 
 constexpr int MT_STAGES = 6, MT_NMAX = 256, MT_NSTEP = 32;
@@ -35,13 +49,20 @@ constexpr uint32_t MT_WAIT_LIMIT = 1u << 22;
 
 __device__ int g_moe_tc_error = 0;
 
+struct MtPart {                     // the experts' products, or the shared expert's
+  __nv_bfloat16* c;
+  int N, nkb, ldc, vec;             // vec: rows of c are whole 16-byte pieces
+  int boxes;                        // GLU with N no multiple of 8: gate and up rows come in boxes of eight from a flat map
+  float limit;
+};
 struct MtParams {
+  MtPart part[2];                   // experts, shared expert
   const int32_t* offsets;
   const int32_t* perm;
-  __nv_bfloat16* c;
-  int X, N, nkb, ldc, vec;          // vec: rows of c are whole 16-byte pieces
-  int boxes;                        // GLU with N no multiple of 8: gate and up rows come in boxes of eight from a flat map
-  float limit, alpha, shift;
+  const int32_t* order;             // experts by falling size of their tiles, or null: as they stand
+  int X, M;                         // M: rows of the shared expert (0: there is none)
+  int early;                        // the shared expert's operands are there before the kernels that this one waits for have ended
+  float alpha, shift;
   int* word;
 };
 struct MtFail {
@@ -63,21 +84,29 @@ __device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, const Mt
   return false;
 }
 
-// Walk over the tiles in rising order; every role keeps its own.  Tile: 256 weight rows (column tile `ct`) x `cnt` sorted rows from `r0` on,
-// `n` columns of the product.
+// Walk over the tiles: the shared expert's, then the experts'; every role keeps its own.  Tile: 256 weight rows (column tile `ct`) x `cnt`
+// rows from `r0` on, `n` columns of the product.
 struct MtWalk {
-  int e = -1, first = 0, next = 0;      // expert, its first tile, the one after its last
+  int k = -2, e = -1, first = 0, next = 0;      // place in the order, expert (-1: shared), its first tile, the one after its last
   int row = 0, count = 0, tiles = 1, step = 0;
   int ct = 0, r0 = 0, cnt = 0, n = 0;
-  __device__ __forceinline__ bool seek(const int32_t* __restrict__ offsets, int X, int ncol, int t) {
+  static __device__ __forceinline__ int columns(int count, int tiles) { return ((count + tiles - 1) / tiles + MT_NSTEP - 1) / MT_NSTEP * MT_NSTEP; }
+  template <int OUTS>
+  __device__ __forceinline__ bool seek(const MtParams& p, int t) {
     while (t >= next) {
-      if (++e >= X) return false;
-      row = __ldg(offsets + e);
-      count = __ldg(offsets + e + 1) - row;
+      if (++k >= p.X) return false;
+      if (k < 0) {
+        e = -1, row = 0, count = p.M;
+      } else {
+        if (k == 0 && p.early) pdl_wait();      // (offsets, order, perm: the first look at what the kernels before have left)
+        e = p.order != nullptr ? p.order[k] : k;
+        row = p.offsets[e];
+        count = p.offsets[e + 1] - row;
+      }
       tiles = (count + MT_NMAX - 1) / MT_NMAX;
       first = next;
-      next += tiles * ncol;
-      if (count > 0) step = ((count + tiles - 1) / tiles + MT_NSTEP - 1) / MT_NSTEP * MT_NSTEP;
+      next += tiles * ((p.part[k < 0].N + 2 * OUTS - 1) / (2 * OUTS));
+      if (count > 0) step = columns(count, tiles);
     }
     const int q = t - first;
     ct = q / tiles;
@@ -88,6 +117,8 @@ struct MtWalk {
     return true;
   }
 };
+// the i-th tile of a pair: to and fro, so that with tiles of falling size the pairs' sums are alike
+__device__ __forceinline__ int mt_tile(int i, int pair, int pairs) { return i * pairs + ((i & 1) ? pairs - 1 - pair : pair); }
 
 __device__ __forceinline__ void pair_box3(void* dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
   asm volatile(
@@ -126,10 +157,13 @@ __device__ __forceinline__ void store_tokens(uint32_t at, uint32_t a, uint32_t b
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+struct MtMaps {      // weights; tokens in boxes of 64 and of 16 rows
+  CUtensorMap w, t64, t16;
+};
+
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
-    moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_t64,
-                         const __grid_constant__ CUtensorMap map_t16, const MtParams p) {
+    moe_gemm_pair_kernel(const __grid_constant__ MtMaps experts, const __grid_constant__ MtMaps shared, const __grid_constant__ MtParams p) {
   constexpr int OUTS = MODE == 1 ? 64 : 128;             // outputs of a CTA's 128 rows
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
@@ -146,9 +180,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();
   if (threadIdx.x == 0) {
-    prefetch_tensormap(&map_w);
-    prefetch_tensormap(&map_t64);
-    prefetch_tensormap(&map_t16);
+    prefetch_tensormap(&experts.w);
+    prefetch_tensormap(&experts.t64);
+    prefetch_tensormap(&experts.t16);
+    prefetch_tensormap(&shared.w);
+    prefetch_tensormap(&shared.t64);
+    prefetch_tensormap(&shared.t16);
     for (int i = 0; i < MT_STAGES; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * MT_EPI_WARPS);
     *s_fail = 0;
@@ -161,9 +198,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const MtFail fail{s_fail, cluster_addr(s_fail, (uint32_t)(rank ^ 1)), p.word};
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, nkb = p.nkb;
-  const int ncol = (p.N + 2 * OUTS - 1) / (2 * OUTS);
-  pdl_wait();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  if (!p.early) pdl_wait();
   pdl_launch_dependents();
 
   if (warp == 0) {
@@ -172,27 +208,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
       int s = 0;
       uint32_t ph = 1;
       bool ok = true;
-      for (int t = pair; ok && walk.seek(p.offsets, p.X, ncol, t); t += pairs) {
-        const int half = walk.n / 2, r0 = walk.r0 + rank * half, n0 = (walk.ct * 2 + rank) * OUTS;
+      for (int i = 0; ok && walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+        const bool dense = walk.e < 0;
+        const MtPart& part = p.part[dense];
+        const MtMaps& maps = dense ? shared : experts;
+        const int half = walk.n / 2, r0 = walk.r0 + rank * half, n0 = (walk.ct * 2 + rank) * OUTS, e = dense ? 0 : walk.e, nkb = part.nkb;
         for (int kb = 0; kb < nkb; ++kb) {
           if (!(ok = mt_wait(&empty[s], ph, fail, 1))) break;
           if (rank == 0) mbar_expect_tx(&full[s], (uint32_t)(2 * (MT_A_BYTES + half * BK * 2)));      // both CTAs' operands
           const uint32_t bar = cluster_addr(&full[s], 0);
           uint8_t *da = sa + s * MT_A_BYTES, *db = sb + s * MT_B_BYTES;
           if (MODE != 1) {
-            pair_box3(da, &map_w, kb * BK, n0, walk.e, bar);
-          } else if (!p.boxes) {
-            pair_box5(da, &map_w, kb * BK, n0 / 8, walk.e, bar);
+            pair_box3(da, &maps.w, kb * BK, n0, e, bar);
+          } else if (!part.boxes) {
+            pair_box5(da, &maps.w, kb * BK, n0 / 8, e, bar);
           } else {
-            const int y = walk.e * 2 * p.N + n0;
+            const int y = e * 2 * part.N + n0;
             for (int j = 0; j < 8; ++j) {
-              pair_box(da + j * 2048, &map_w, kb * BK, y + 8 * j, bar);
-              pair_box(da + j * 2048 + 1024, &map_w, kb * BK, y + p.N + 8 * j, bar);
+              pair_box(da + j * 2048, &maps.w, kb * BK, y + 8 * j, bar);
+              pair_box(da + j * 2048 + 1024, &maps.w, kb * BK, y + part.N + 8 * j, bar);
             }
           }
           int r = 0;
-          for (; r + 64 <= half; r += 64) pair_box(db + r * BK * 2, &map_t64, kb * BK, r0 + r, bar);
-          for (; r < half; r += 16) pair_box(db + r * BK * 2, &map_t16, kb * BK, r0 + r, bar);
+          for (; r + 64 <= half; r += 64) pair_box(db + r * BK * 2, &maps.t64, kb * BK, r0 + r, bar);
+          for (; r < half; r += 16) pair_box(db + r * BK * 2, &maps.t16, kb * BK, r0 + r, bar);
           if (++s == MT_STAGES) s = 0, ph ^= 1u;
         }
       }
@@ -205,7 +244,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
       bool ok = true;
       int s = 0, i = 0;
       uint32_t ph = 0;
-      for (int t = pair; rank == 0 && ok && walk.seek(p.offsets, p.X, ncol, t); t += pairs, ++i) {
+      for (; rank == 0 && ok && walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+        const int nkb = p.part[walk.e < 0].nkb;
         const uint32_t d = tmem + (uint32_t)((i & 1) * MT_NMAX), idesc = instr_desc_bf16(256, 0) | ((uint32_t)(walk.n >> 3) << 17);
         if (!(ok = mt_wait(&acc_empty[i & 1], (uint32_t)((i >> 1) & 1) ^ 1u, fail, 4))) break;
         tc_fence_after();
@@ -231,7 +271,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
     const uint32_t mine = stage + (uint32_t)(lane * DIMS * 2);
     MtWalk walk;
     int i = 0;
-    for (int t = pair; walk.seek(p.offsets, p.X, ncol, t); t += pairs, ++i) {
+    for (; walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+      const MtPart& out = p.part[walk.e < 0];
+      const float limit = out.limit;
       const int n0 = (walk.ct * 2 + rank) * OUTS + quarter * DIMS;
       if (!__all_sync(0xffffffffu, mt_wait(&acc_full[i & 1], (uint32_t)(i >> 1) & 1u, fail, 3))) break;
       tc_fence_after();
@@ -240,7 +282,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
       for (int c0 = part * 32; c0 < walk.cnt; c0 += 64) {
         const int tok = c0 + lane;
         int row = walk.r0 + tok;
-        if (MODE == 0 && tok < walk.cnt) row = p.perm[row];
+        if (MODE == 0 && walk.e >= 0 && tok < walk.cnt) row = p.perm[row];
 #pragma unroll
         for (int hl = 0; hl < 2; ++hl) {
           uint32_t v[16];
@@ -252,8 +294,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
               float f[2];
 #pragma unroll
               for (int q = 0; q < 2; ++q) {
-                const float g = fminf(__uint_as_float(v[4 * j + q]), p.limit);
-                const float up = fminf(fmaxf(__uint_as_float(v[4 * j + 2 + q]), -p.limit), p.limit);
+                const float g = fminf(__uint_as_float(v[4 * j + q]), limit);
+                const float up = fminf(fmaxf(__uint_as_float(v[4 * j + 2 + q]), -limit), limit);
                 f[q] = g / (1.f + expf(-p.alpha * g)) * (up + p.shift);
               }
               o[j] = pack_bf16(f[0], f[1]);
@@ -280,13 +322,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
           const int dst = __shfl_sync(0xffffffffu, row, tk);
           const uint4 u = lds128(stage + (uint32_t)(tk * DIMS * 2 + ((ch ^ (MODE == 1 ? (tk >> 2) & 1 : (tk >> 1) & 3)) * 16)));
           const int col = n0 + 8 * ch;
-          if (c0 + tk < walk.cnt && col < p.N) {
-            __nv_bfloat16* out = p.c + (size_t)dst * p.ldc + col;
-            if (p.vec) {
-              *reinterpret_cast<uint4*>(out) = u;
+          if (c0 + tk < walk.cnt && col < out.N) {
+            __nv_bfloat16* at_c = out.c + (size_t)dst * out.ldc + col;
+            if (out.vec) {
+              *reinterpret_cast<uint4*>(at_c) = u;
             } else {
               const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-              for (int j = 0; j < 8 && col + j < p.N; ++j) out[j] = __ushort_as_bfloat16((uint16_t)(w[j >> 1] >> (16 * (j & 1))));
+              for (int j = 0; j < 8 && col + j < out.N; ++j) at_c[j] = __ushort_as_bfloat16((uint16_t)(w[j >> 1] >> (16 * (j & 1))));
             }
           }
         }
@@ -305,13 +347,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
   }
 }
 
-// xs[r][:] = x[perm[r] / top][:] for the sorted rows r (16-byte pieces)
-__global__ void moe_gather_rows_kernel(const uint4* __restrict__ x, long long ldx16, const int32_t* __restrict__ perm, int top,
-                                       uint4* __restrict__ out, int k16) {
-  const int r = blockIdx.x;
-  const uint4* src = x + (long long)(perm[r] / top) * ldx16;
+// xs[r][:] = x[perm[r] / top][:] for the sorted rows r (16-byte pieces): a warp a row, eight pieces a lane on their way
+constexpr int GR_WARPS = 8;
+__global__ void __launch_bounds__(32 * GR_WARPS) moe_gather_rows_kernel(const uint4* __restrict__ x, long long ldx16, const int32_t* perm,
+                                                                        int top, uint4* __restrict__ out, int k16, int n_rows) {
+  const int r = blockIdx.x * GR_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (r >= n_rows) return;
+  const uint4* src = x + (long long)(after_wait(perm)[r] / top) * ldx16;
   uint4* dst = out + (long long)r * k16;
-  for (int i = threadIdx.x; i < k16; i += blockDim.x) dst[i] = src[i];
+  for (int i0 = lane; i0 < k16; i0 += 256) {
+    uint4 u[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (i0 + 32 * j < k16) u[j] = src[i0 + 32 * j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (i0 + 32 * j < k16) dst[i0 + 32 * j] = u[j];
+  }
 }
 
 int mt_encode(const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, CUtensorMap* out) {
@@ -345,19 +399,104 @@ int mt_weight_map(const void* w, int mode, int X, int N, int K, CUtensorMap* out
 }
 
 template <int MODE>
-int launch_moe_pair(const CUtensorMap& mw, const CUtensorMap& m64, const CUtensorMap& m16, const MtParams& p, int n_rows, cudaStream_t st) {
+int launch_moe_pair(const MtMaps& experts, const MtMaps& shared, const MtParams& p, int n_rows, cudaStream_t st) {
   static PerDevice configured;
   if (!configured) {
     LL_CUDA(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MT_SMEM));
     configured.mark();
   }
   const int cols = MODE == 1 ? 128 : 256;
-  const long long most = (long long)((p.N + cols - 1) / cols) * (n_rows / MT_NMAX + std::min(n_rows, p.X));
+  const long long most = (long long)((p.part[0].N + cols - 1) / cols) * (n_rows / MT_NMAX + std::min(n_rows, p.X)) +
+                         (long long)((p.part[1].N + cols - 1) / cols) * ((p.M + MT_NMAX - 1) / MT_NMAX);
   LL_CHECK_ARG(most < (1ll << 30), "moe_grouped_gemm_tc: too many tiles");
   const int pairs = sm_count() > 1 ? sm_count() / 2 : 1;
-  LL_CUDA(launch(moe_gemm_pair_kernel<MODE>, dim3(2 * (unsigned)std::min<long long>(most, pairs)), dim3(MT_THREADS), MT_SMEM, st, true, mw, m64, m16, p));
+  LL_CUDA(launch(moe_gemm_pair_kernel<MODE>, dim3(2 * (unsigned)std::min<long long>(most, pairs)), dim3(MT_THREADS), MT_SMEM, st, true, experts,
+                 shared, p));
   LL_LAUNCH_OK("moe_gemm_pair_kernel");
   return LL_OK;
+}
+
+MtPart mt_part(void* c, int mode, int N, int K, int ldc, float limit) {
+  return MtPart{(__nv_bfloat16*)c, N, (K + BK - 1) / BK, ldc, ldc % 8 == 0 && N % 8 == 0, mode == 1 && N % 8 != 0, limit};
+}
+int mt_maps(const void* w, int mode, int X, int N, int K, const void* a, int rows, MtMaps* m) {
+  if (int r = mt_weight_map(w, mode, X, N, K, &m->w)) return r;
+  if (int r = make_map(a, rows, K, 64, &m->t64)) return r;
+  return make_map(a, rows, K, 16, &m->t16);
+}
+
+// The (token, choice) pairs of a prompt in the order of their experts, and the experts in the order of their tiles' size: one block, counts
+// and places in shared memory (8192 pairs of 32 experts: 4 us; the pairs of an expert come in no fixed order, which no result depends on).
+constexpr int SORT_THREADS = 1024, SORT_KEPT = 16;
+__global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const int32_t* expert_idx, int n_pairs, int X, int32_t* __restrict__ offsets,
+                                                                int32_t* __restrict__ order, int32_t* __restrict__ perm) {
+  extern __shared__ int32_t sort_smem[];
+  int32_t *count = sort_smem, *at = count + X, *size = at + X;      // [X] each
+  const int tid = threadIdx.x, lane = tid & 31;
+  pdl_launch_dependents();
+  for (int e = tid; e < X; e += SORT_THREADS) count[e] = 0;
+  __syncthreads();
+  pdl_wait();
+  expert_idx = after_wait(expert_idx);
+  int32_t mine[SORT_KEPT], rank[SORT_KEPT];      // the first pairs of a thread keep their places in registers
+#pragma unroll
+  for (int j = 0; j < SORT_KEPT; ++j) mine[j] = j * SORT_THREADS + tid < n_pairs ? expert_idx[j * SORT_THREADS + tid] : -1;
+#pragma unroll
+  for (int j = 0; j < SORT_KEPT; ++j)
+    if (mine[j] >= 0) rank[j] = atomicAdd(&count[mine[j]], 1);
+  __syncthreads();                               // (theirs are the first places; the rest fill an expert's rows from behind)
+  for (int i = SORT_KEPT * SORT_THREADS + tid; i < n_pairs; i += SORT_THREADS) atomicAdd(&count[expert_idx[i]], 1);
+  __syncthreads();
+  if (tid < 32) {
+    int before = 0;
+    for (int e0 = 0; e0 < X; e0 += 32) {
+      const int e = e0 + lane, c = e < X ? count[e] : 0;
+      int incl = c;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+      }
+      if (e < X) {
+        at[e] = offsets[e] = before + incl - c;
+        count[e] = before + incl;
+        const int tiles = (c + MT_NMAX - 1) / MT_NMAX;
+        size[e] = c > 0 ? MtWalk::columns(c, tiles) : 0;
+      }
+      before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) offsets[X] = before;
+  }
+  __syncthreads();
+  for (int e = tid; e < X; e += SORT_THREADS) {
+    int place = 0;
+    for (int o = 0; o < X; ++o) place += size[o] > size[e] || (size[o] == size[e] && o < e);
+    order[place] = e;
+  }
+#pragma unroll
+  for (int j = 0; j < SORT_KEPT; ++j)
+    if (mine[j] >= 0) perm[at[mine[j]] + rank[j]] = j * SORT_THREADS + tid;
+  for (int i = SORT_KEPT * SORT_THREADS + tid; i < n_pairs; i += SORT_THREADS) perm[atomicSub(&count[expert_idx[i]], 1) - 1] = i;
+}
+
+struct MpScratch {
+  int32_t *idx, *offsets, *order, *perm;
+  float *weight, *gate;
+  __nv_bfloat16 *xs, *h, *y, *hs, *ys;
+  size_t total;
+};
+MpScratch mp_carve(void* base, int M, int X, int top, int width, int ff, int sff) {
+  MpScratch s;
+  size_t o = 0;
+  auto take = [&](size_t b) { size_t r = o; o += (b + 127) & ~(size_t)127; return r; };
+  uint8_t* p = (uint8_t*)base;
+  const size_t n = (size_t)M * top;
+  s.idx = (int32_t*)(p + take(n * 4)), s.weight = (float*)(p + take(n * 4)), s.perm = (int32_t*)(p + take(n * 4));
+  s.offsets = (int32_t*)(p + take((size_t)(X + 1) * 4)), s.order = (int32_t*)(p + take((size_t)X * 4)), s.gate = (float*)(p + take((size_t)M * 4));
+  s.xs = (__nv_bfloat16*)(p + take(n * width * 2)), s.h = (__nv_bfloat16*)(p + take(n * ff * 2)), s.y = (__nv_bfloat16*)(p + take(n * width * 2));
+  s.hs = (__nv_bfloat16*)(p + take((size_t)M * sff * 2)), s.ys = (__nv_bfloat16*)(p + take(sff ? (size_t)M * width * 2 : 0));
+  s.total = o;
+  return s;
 }
 
 }  // namespace
@@ -372,8 +511,8 @@ int ll_moe_gather_rows(const void* x, int ldx, const int32_t* perm, int top, int
   LL_CHECK_ARG(K % 8 == 0 && ldx % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0,
                "moe_gather_rows: rows must be 16-byte aligned bf16");
   if (n_rows == 0) return LL_OK;
-  moe_gather_rows_kernel<<<n_rows, K / 8 >= 256 ? 256 : 128, 0, (cudaStream_t)stream>>>((const uint4*)x, ldx / 8, perm, top, (uint4*)out,
-                                                                                     K / 8);
+  moe_gather_rows_kernel<<<(n_rows + GR_WARPS - 1) / GR_WARPS, 32 * GR_WARPS, 0, (cudaStream_t)stream>>>((const uint4*)x, ldx / 8, perm, top, (uint4*)out,
+                                                                                                      K / 8, n_rows);
   LL_LAUNCH_OK("moe_gather_rows_kernel");
   return LL_OK;
 }
@@ -389,16 +528,71 @@ int ll_moe_grouped_gemm_tc(const void* a, const void* w, const int32_t* offsets,
   if (n_rows == 0) return LL_OK;
   const long long wrows = (long long)n_experts * (mode == 1 ? 2 : 1) * N;
   LL_CHECK_ARG(wrows < (1ll << 31), "moe_grouped_gemm_tc: weight stack too tall for one tensor map");
-  CUtensorMap mw, m64, m16;
-  if (int r = mt_weight_map(w, mode, n_experts, N, K, &mw)) return r;
-  if (int r = make_map(a, n_rows, K, 64, &m64)) return r;
-  if (int r = make_map(a, n_rows, K, 16, &m16)) return r;
-  const MtParams p{offsets, perm, (__nv_bfloat16*)c, n_experts, N, (K + BK - 1) / BK, ldc, ldc % 8 == 0 && N % 8 == 0, N % 8 != 0, limit, alpha, shift,
-                   wait_word()};
+  MtMaps maps;
+  if (int r = mt_maps(w, mode, n_experts, N, K, a, n_rows, &maps)) return r;
+  MtParams p{};
+  p.part[0] = p.part[1] = mt_part(c, mode, N, K, ldc, limit);
+  p.offsets = offsets, p.perm = perm, p.X = n_experts, p.alpha = alpha, p.shift = shift, p.word = wait_word();
   cudaStream_t st = (cudaStream_t)stream;
-  if (mode == 1) return launch_moe_pair<1>(mw, m64, m16, p, n_rows, st);
-  if (mode == 3) return launch_moe_pair<3>(mw, m64, m16, p, n_rows, st);
-  return launch_moe_pair<0>(mw, m64, m16, p, n_rows, st);
+  if (mode == 1) return launch_moe_pair<1>(maps, maps, p, n_rows, st);
+  if (mode == 3) return launch_moe_pair<3>(maps, maps, p, n_rows, st);
+  return launch_moe_pair<0>(maps, maps, p, n_rows, st);
+}
+
+int ll_moe_prompt_supported(int M, int width, int n_experts, int ff, int shared_ff) {
+  return M >= 1 && M < (1 << 24) && width > 0 && width % 8 == 0 && ff > 0 && ff % 8 == 0 && shared_ff >= 0 && shared_ff % 8 == 0 && n_experts <= 4096 &&
+         (long long)n_experts * 2 * ff < (1ll << 31) && (long long)n_experts * width < (1ll << 31);
+}
+
+size_t ll_moe_prompt_scratch_bytes(int M, int width, int n_experts, int top, int ff, int shared_ff) {
+  return mp_carve(nullptr, M, n_experts, top, width, ff, shared_ff).total;
+}
+
+int ll_moe_prompt(const void* x, const float* w_router, const float* bias, const float* correction, int score, float out_scale, int n_groups,
+                  int keep_groups, int group_top, const void* w_gu, const void* w_down, const void* ws_in, const void* ws_down, int M, int width,
+                  int n_experts, int top, int ff, int shared_ff, int shared_gate, int mode, float limit, float alpha, float shared_limit, void* out,
+                  void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_router && w_gu && w_down && out && scratch && (shared_ff == 0 || (ws_in && ws_down)), "moe_prompt: null pointer");
+  LL_CHECK_ARG(n_experts > 0 && top > 0 && top <= n_experts && mode >= 1 && mode <= 3 && (long long)M * top < (1ll << 30), "bad moe_prompt arguments");
+  if (!ll_moe_prompt_supported(M, width, n_experts, ff, shared_ff)) {
+    set_error("moe_prompt takes widths in multiples of 8 (M=%d width=%d experts=%d ff=%d shared=%d)", M, width, n_experts, ff, shared_ff);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)ws_in | (uintptr_t)ws_down | (uintptr_t)scratch | (uintptr_t)out) & 15) == 0,
+               "moe_prompt: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const MpScratch s = mp_carve(scratch, M, n_experts, top, width, ff, shared_ff);
+  const int n = M * top, up = mode == 2 ? 1 : mode;
+  const __nv_bfloat16* gate_row = shared_ff && shared_gate ? (const __nv_bfloat16*)ws_in + (size_t)(up == 1 ? 2 : 1) * shared_ff * width : nullptr;
+  if (int r = moe_route_only(x, w_router, bias, M, width, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, s.idx, s.weight,
+                             gate_row, s.gate, st))
+    return r;
+  LL_CUDA(launch(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), 3 * sizeof(int32_t) * n_experts, st, true, (const int32_t*)s.idx, n, n_experts, s.offsets,
+                 s.order, s.perm));
+  LL_LAUNCH_OK("moe_sort_kernel");
+  LL_CUDA(launch(moe_gather_rows_kernel, dim3((n + GR_WARPS - 1) / GR_WARPS), dim3(32 * GR_WARPS), 0, st, true, (const uint4*)x, (long long)(width / 8),
+                 (const int32_t*)s.perm, top, (uint4*)s.xs, width / 8, n));
+  LL_LAUNCH_OK("moe_gather_rows_kernel");
+  // first projections with their unit
+  MtMaps experts, shared;
+  if (int r = mt_maps(w_gu, up, n_experts, ff, width, s.xs, n, &experts)) return r;
+  shared = experts;
+  if (shared_ff)
+    if (int r = mt_maps(ws_in, up, 1, shared_ff, width, x, M, &shared)) return r;
+  MtParams p{};
+  p.part[0] = mt_part(s.h, up, ff, width, ff, limit), p.part[1] = mt_part(s.hs, up, shared_ff, width, shared_ff, shared_limit);
+  p.offsets = s.offsets, p.perm = s.perm, p.order = s.order, p.X = n_experts, p.M = shared_ff ? M : 0, p.early = 1;
+  p.alpha = alpha, p.shift = mode == 2 ? 0.f : 1.f, p.word = wait_word();
+  if (int r = up == 1 ? launch_moe_pair<1>(experts, shared, p, n, st) : launch_moe_pair<3>(experts, shared, p, n, st)) return r;
+  // second ones
+  if (int r = mt_maps(w_down, 0, n_experts, width, ff, s.h, n, &experts)) return r;
+  shared = experts;
+  if (shared_ff)
+    if (int r = mt_maps(ws_down, 0, 1, width, shared_ff, s.hs, M, &shared)) return r;
+  p.part[0] = mt_part(s.y, 0, width, ff, width, 0.f), p.part[1] = mt_part(s.ys, 0, width, shared_ff, width, 0.f);
+  p.early = 0;
+  if (int r = launch_moe_pair<0>(experts, shared, p, n, st)) return r;
+  return moe_combine_rows(s.y, s.weight, top, shared_ff ? s.ys : nullptr, gate_row ? s.gate : nullptr, out, M, width, st);
 }
 
 // 0, or the code of the first bounded wait that ran out in a kernel of this file (1: ring slot, 2: operands, 3: accumulator,

@@ -34,7 +34,8 @@ __global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kern
                                                                int score, const float* __restrict__ correction, float out_scale,
                                                                int n_groups, int keep_groups, int group_top,
                                                                int32_t* __restrict__ expert_idx, float* __restrict__ expert_w,
-                                                               int32_t* __restrict__ counts, int32_t* __restrict__ rank) {
+                                                               int32_t* __restrict__ counts, int32_t* __restrict__ rank,
+                                                               const T* __restrict__ gate_row, float* __restrict__ gate) {
   pdl_launch_dependents();             // (a step of a few tokens: the shared expert's blocks start beside this one)
   extern __shared__ float sm[];
   float* xs = sm;                      // [RT_TOK][dim]
@@ -57,6 +58,18 @@ __global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kern
   }
   for (int idx = nt * dim + tid; idx < RT_TOK * dim; idx += RT_THREADS) xs[idx] = 0.f;
   __syncthreads();
+  if (gate_row != nullptr && warp < nt) {      // the shared expert's gate logit of the warp's token (rows of whole 16-byte pieces)
+    const float* xt = xs + warp * dim;
+    float g = 0.f;
+#pragma unroll 4
+    for (int i = lane; i < dim / V; i += 32) {
+      const uint4 u = reinterpret_cast<const uint4*>(gate_row)[i];
+#pragma unroll
+      for (int j = 0; j < V; ++j) g += dt<T>::ld(reinterpret_cast<const T*>(&u), j) * xt[i * V + j];
+    }
+    g = warp_sum(g);
+    if (lane == 0) gate[m0 + warp] = g;
+  }
   const bool vec4 = (dim % 4 == 0) && (((uintptr_t)w_router & 15) == 0);
   // RT_EG experts at a time per warp and four columns per step: 16 independent weight loads in flight per lane
   for (int e0 = warp * RT_EG; e0 < X; e0 += (RT_THREADS / 32) * RT_EG) {
@@ -191,7 +204,7 @@ __global__ void __launch_bounds__(RT_THREADS, RT_TOK > 1 ? 2 : 1) moe_route_kern
     for (int k = lane; k < top; k += 32) {      // the places of all choices at once: one round trip to the counters
       const size_t at = (size_t)m * top + k;
       expert_w[at] = expert_w[at] / denom * out_scale;
-      rank[at] = atomicAdd(&counts[expert_idx[at]], 1);
+      if (counts != nullptr) rank[at] = atomicAdd(&counts[expert_idx[at]], 1);
     }
   }
 }
@@ -468,11 +481,11 @@ __global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restr
 }
 
 // 16 bytes per access, the same sums: 2048 tokens of width 2048 with four choices and a shared expert, 21 us -> 9 (40 MB).
-template <typename T>
-__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const T* __restrict__ y, const float* __restrict__ expert_w, int top,
-                                                              const T* __restrict__ shared_y, int shared_ld,
-                                                              const T* __restrict__ shared_gate, int gate_ld, T* __restrict__ out, int M,
-                                                              int dim) {
+template <typename T, typename GATE = T>
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const T* y, const float* expert_w, int top, const T* shared_y, int shared_ld,
+                                                              const GATE* shared_gate, int gate_ld, T* __restrict__ out, int M, int dim) {
+  pdl_wait();
+  y = after_wait(y), expert_w = after_wait(expert_w), shared_y = after_wait(shared_y), shared_gate = after_wait(shared_gate);
   constexpr int V = 16 / sizeof(T);
   const int pieces = dim / V;
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -489,7 +502,7 @@ __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const T* __restric
     for (int j = 0; j < V; ++j) v[j] += w * dt<T>::ld(reinterpret_cast<const T*>(&u), j);
   }
   if (shared_y) {
-    const float sg = shared_gate ? 1.f / (1.f + expf(-dt<T>::ld(shared_gate, (size_t)m * gate_ld))) : 1.f;
+    const float sg = shared_gate ? 1.f / (1.f + expf(-dt<GATE>::ld(shared_gate, (size_t)m * gate_ld))) : 1.f;
     const uint4 u = *reinterpret_cast<const uint4*>(shared_y + (size_t)m * shared_ld + c);
 #pragma unroll
     for (int j = 0; j < V; ++j) v[j] += sg * dt<T>::ld(reinterpret_cast<const T*>(&u), j);
@@ -547,10 +560,11 @@ static int route_check(int M, int dim, int n_experts, int top, int score, const 
   }
   return LL_OK;
 }
-// The router: choices and weights of every token (counts: how many choices an expert has, added to what is there; rank: a choice's place).
+// The router: choices and weights of every token (counts: how many choices an expert has, added to what is there, and rank, a choice's place, or
+// null), and with a gate row the shared expert's gate logit of every token.
 static int route_launch(const void* x, int dtype, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score,
                         const float* correction, float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx,
-                        float* expert_w, int32_t* counts, int32_t* rank, cudaStream_t st) {
+                        float* expert_w, int32_t* counts, int32_t* rank, const void* gate_row, float* gate, cudaStream_t st) {
   const size_t per_token = route_smem(dim, n_experts, score, n_groups);
   const int sms = sm_count();
   const int tok = M >= 8 * sms && 8 * per_token <= RT_WIDE_SMEM ? 8 : M <= sms ? 1 : 4;
@@ -565,7 +579,7 @@ static int route_launch(const void* x, int dtype, const float* w_router, const f
     }                                                                                                                                \
   }                                                                                                                                  \
   moe_route_kernel<T, TOK><<<blocks, RT_THREADS, smem, st>>>((const T*)x, w_router, bias, M, dim, n_experts, top, score, correction,  \
-                                                             out_scale, n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank)
+                                                             out_scale, n_groups, keep_groups, group_top, expert_idx, expert_w, counts, rank, (const T*)gate_row, gate)
 #define LL_RT(T)                                                                                                                     \
   if (tok == 8) { LL_RT_TOK(T, 8); } else if (tok == 4) { LL_RT_TOK(T, 4); } else { LL_RT_TOK(T, 1); }
   if (dtype == LL_F32) {
@@ -583,11 +597,21 @@ static int route_launch(const void* x, int dtype, const float* w_router, const f
 }
 
 int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
-                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
                    cudaStream_t st) {
   if (int r = route_check(M, dim, n_experts, top, score, correction, n_groups, keep_groups, group_top)) return r;
   return route_launch(x, LL_BF16, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
-                      expert_w, counts, rank, st);
+                      expert_w, nullptr, nullptr, gate_row, gate, st);
+}
+
+// The combination of a prompt's rows in one chain of programmatic launches: whole 16-byte pieces, the gate's logits in fp32.
+int moe_combine_rows(const void* y, const float* expert_w, int top, const void* shared_y, const float* gate, void* out, int M, int dim, cudaStream_t st) {
+  const size_t n = (size_t)M * (dim / 8);
+  typedef __nv_bfloat16 T;
+  LL_CUDA(launch(moe_combine_vec_kernel<T, float>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, true, (const T*)y, expert_w, top, (const T*)shared_y,
+                 dim, gate, 1, (T*)out, M, dim));
+  LL_LAUNCH_OK("moe_combine_kernel");
+  return LL_OK;
 }
 
 }  // namespace llb
@@ -620,7 +644,7 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
   if (M == 0) return LL_OK;
   LL_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * n_experts, st));
   if (int r = route_launch(x, dtype, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
-                           expert_w, counts, rank, st))
+                           expert_w, counts, rank, nullptr, nullptr, st))
     return r;
   const int n_pairs = M * top;
   moe_permute_kernel<<<(n_pairs + 255) / 256, 256, sizeof(int32_t) * (n_experts + 1), st>>>(expert_idx, rank, counts, n_pairs,

@@ -13,9 +13,9 @@
 
 namespace llb {
 
-// moe_ops.cu: the router alone (counts and rank are scratch)
+// moe_ops.cu: the router alone
 int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
-                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
                    cudaStream_t st);
 
 namespace {
@@ -152,20 +152,18 @@ __global__ void __launch_bounds__(MS_THREADS) moe_step_down_kernel(const MsParam
 }
 
 struct MsScratch {
-  int32_t *idx, *counts, *rank;
+  int32_t* idx;
   float* weight;
   __nv_bfloat16 *h, *hs, *gate;
   size_t total;
 };
-MsScratch ms_carve(void* base, int M, int X, int top, int ff, int sff) {
+MsScratch ms_carve(void* base, int M, int top, int ff, int sff) {
   MsScratch s;
   size_t o = 0;
   auto take = [&](size_t b) { size_t r = o; o += (b + 127) & ~(size_t)127; return r; };
   uint8_t* p = (uint8_t*)base;
   s.idx = (int32_t*)(p + take((size_t)M * top * 4));
   s.weight = (float*)(p + take((size_t)M * top * 4));
-  s.counts = (int32_t*)(p + take((size_t)X * 4));
-  s.rank = (int32_t*)(p + take((size_t)M * top * 4));
   s.h = (__nv_bfloat16*)(p + take((size_t)M * top * ff * 2));
   s.hs = (__nv_bfloat16*)(p + take((size_t)M * sff * 2));
   s.gate = (__nv_bfloat16*)(p + take((size_t)M * 2));
@@ -184,7 +182,7 @@ int ll_moe_step_supported(int M, int width, int ff, int shared_ff) {
   return M >= 1 && M <= 8 && width > 0 && width % 8 == 0 && ff > 0 && ff % 8 == 0 && shared_ff >= 0 && shared_ff % 8 == 0;
 }
 
-size_t ll_moe_step_scratch_bytes(int M, int n_experts, int top, int ff, int shared_ff) { return ms_carve(nullptr, M, n_experts, top, ff, shared_ff).total; }
+size_t ll_moe_step_scratch_bytes(int M, int n_experts, int top, int ff, int shared_ff) { return ms_carve(nullptr, M, top, ff, shared_ff).total; }
 
 int ll_moe_step(const void* x, const float* w_router, const float* bias, const float* correction, int score, float out_scale, int n_groups,
                 int keep_groups, int group_top, const void* w_gu, const void* w_down, const void* ws_in, const void* ws_down, int M, int width,
@@ -199,9 +197,9 @@ int ll_moe_step(const void* x, const float* w_router, const float* bias, const f
   LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)ws_in | (uintptr_t)ws_down | (uintptr_t)scratch) & 15) == 0,
                "moe_step: rows must be 16-byte aligned bf16");
   cudaStream_t st = (cudaStream_t)stream;
-  const MsScratch s = ms_carve(scratch, M, n_experts, top, ff, shared_ff);
+  const MsScratch s = ms_carve(scratch, M, top, ff, shared_ff);
   if (int r = moe_route_only(x, w_router, bias, M, width, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, s.idx, s.weight,
-                             s.counts, s.rank, st))
+                             nullptr, nullptr, st))
     return r;
   typedef const __nv_bfloat16* B;
   const MsParams p{(B)x, (B)w_gu, (B)w_down, shared_ff ? (B)ws_in : nullptr, shared_ff ? (B)ws_down : nullptr, s.idx, s.weight, s.h, s.hs, s.gate,

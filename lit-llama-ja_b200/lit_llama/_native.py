@@ -156,6 +156,10 @@ EXPORTS = {
     "ll_moe_step_scratch_bytes": ([i32, i32, i32, i32, i32], sz_t),
     "ll_moe_step": ([vp, vp, vp, vp, i32, C.c_float, i32, i32, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, C.c_float,
                      C.c_float, vp, vp, vp], C.c_int),
+    "ll_moe_prompt_supported": ([i32] * 5, C.c_int),
+    "ll_moe_prompt_scratch_bytes": ([i32] * 6, sz_t),
+    "ll_moe_prompt": ([vp, vp, vp, vp, i32, C.c_float, i32, i32, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, C.c_float,
+                       C.c_float, vp, vp, vp], C.c_int),
     "ll_moe_combine": ([vp, vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, vp], C.c_int),
     "ll_add_norm_pair": ([vp, vp, C.c_float, vp, C.c_float, vp, C.c_float, vp, vp, C.c_float, vp, i32, vp, i32, i32, i32, vp], C.c_int),
     "ll_add_layer_norm": ([vp, vp, C.c_float, vp, vp, C.c_float, vp, i32, i32, i32, vp], C.c_int),

@@ -14,10 +14,11 @@ squared-relu layers.
 
 The experts' weights are stacked ([X, 2 ff, width] for [gate; up] or [X, ff, width] for up alone, [X, width, ff] for down) and run as two grouped GEMMs
 over the (token, choice) pairs sorted by expert; counts, offsets and the permutation never leave the device, so a step
-is one fixed launch sequence.  Steps with many rows per expert (prefill in bfloat16) gather the rows into sorted order
-and run both GEMMs on the tcgen05 tensor cores (TMA-tiled operands, accumulators in TMEM, the activation as the first
-GEMM's epilogue); small steps use the mma.sync / FMA kernels that take rows in place.  The shared expert is dense
-(library GEMMs) with its gate logit as one more output row.
+is one fixed launch sequence.  More than a few bfloat16 tokens go through ``ll_moe_prompt``: the router, the sort, the gathered rows, both
+projections on the tcgen05 tensor cores with the shared expert's tiles among the experts' (the activation is the first one's epilogue), and the
+combination, six kernels under programmatic launches.  A few tokens go through ``ll_moe_step``.  What neither takes (fp32, other layouts, weights
+that want a gradient) runs as separate calls: grouped GEMMs that take rows in place or, with rows that TMA can tile, the tcgen05 ones, and
+the shared expert as dense library GEMMs with its gate logit as one more output row.
 """
 from __future__ import annotations
 
@@ -33,9 +34,11 @@ from torch.nn import functional as F
 from . import _native as N
 from .feed_forward import glu_unit, relu_squared_
 
-# the tcgen05 path: at least this many (token, choice) rows in the step, and on average per expert
-TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "128"))
-TC_MIN_ROWS_PER_EXPERT = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "1"))
+# the tcgen05 path: at least this many (token, choice) rows in the step, and on average per expert.  Graphed, us, mma.sync / tcgen05: 32 experts of
+# 2048 x 1024, four chosen, a shared one, 9 tokens 109 / 88, 64 119 / 104, 300 164 / 112, 2048 527 / 185; 16 of 1024 x 768, two chosen 49 / 39,
+# 51 / 42, 74 / 48, 165 / 77; 16 of 1024 x 1024, four chosen, none shared, 9 tokens 43 / 45, 64 69 / 44.  Fewer rows are the steps of a few tokens.
+TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "8"))
+TC_MIN_ROWS_PER_EXPERT = float(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "0.25"))
 
 
 STEP_MAX_TOKENS, STEP_SMALL_EXPERT = 8, 1 << 22       # tokens of a step; ff * width
@@ -173,8 +176,8 @@ class MoE(nn.Module):
         return (x_act.dtype == torch.bfloat16 and s.width % 8 == 0 and s.ff % 8 == 0 and x_act.stride(0) % 8 == 0
                 and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts and N.has("ll_moe_grouped_gemm_tc"))
 
-    def _step(self, at, x_act: torch.Tensor, M: int) -> torch.Tensor:
-        """A few tokens in three launches (``ll_moe_step``)."""
+    def _one_call(self, entry: str, at, x_act: torch.Tensor, M: int, scratch_bytes: int) -> torch.Tensor:
+        """The whole layer through ``ll_moe_step`` or ``ll_moe_prompt``."""
         s, p = self.spec, self._parameters
         sff = s.shared_ff or 0
         x, w_gu, w_down, ws_in, ws_down = at if sff else (*at, None, None)
@@ -182,19 +185,18 @@ class MoE(nn.Module):
         bias = p["b_router"] if "b_router" in p else self.b_router
         correction = p["correction"] if "correction" in p else self.correction
         out = torch.empty_like(x_act)
-        scratch = x_act.new_empty(_step_scratch_bytes(M, s.experts, s.top, s.ff, sff) // 2)          # (whole pieces of 128 bytes or more)
-        N.call("ll_moe_step", x, N.ptr(router), N.ptr(bias), N.ptr(correction), _SCORES[s.score], float(s.weight_scale), s.groups,
+        scratch = x_act.new_empty(scratch_bytes // 2)          # (whole pieces of 128 bytes)
+        N.call(entry, x, N.ptr(router), N.ptr(bias), N.ptr(correction), _SCORES[s.score], float(s.weight_scale), s.groups,
                s.keep_groups if s.groups > 1 else 1, s.group_top, w_gu, w_down, ws_in, ws_down, M, s.width, s.experts, s.top, s.ff, sff,
                1 if s.shared_gate else 0, self.up_mode, float(s.limit), float(s.alpha), float(s.shared_limit if s.shared_limit is not None else s.limit),
                N.ptr(out), N.ptr(scratch), N.stream())
         return out
 
-    def _takes_step(self, x_act: torch.Tensor, M: int):
-        """A few bf16 tokens (``step_pays``), and weights that are what the module was built with: their addresses, or ``None``."""
+    def _rows(self, x_act: torch.Tensor, M: int):
+        """The addresses of dense bf16 rows and of weights that are what the module was built with, or ``None``."""
         s = self.spec
         branches = 1 if s.unit == "relu2" else 2
-        if not (x_act.dtype is torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width)
-                and step_pays(M, s.width, s.ff, s.shared_ff or 0, s.experts, s.top, branches)):
+        if not (x_act.dtype is torch.bfloat16 and x_act.is_cuda and x_act.shape == (M, s.width)):
             return None
         p = self._parameters
         up, down = (s.experts, branches * s.ff, s.width), (s.experts, s.width, s.ff)
@@ -206,11 +208,30 @@ class MoE(nn.Module):
         return N.step_rows(x_act, (p.get("w_gu"), p.get("w_down"), w, p.get("w_shared_down")),
                            (up, down, (w.shape[0], s.width), (s.width, s.shared_ff)))
 
+    def _takes_step(self, x_act: torch.Tensor, M: int):
+        """A few bf16 tokens (``step_pays``) in three launches: the rows' addresses, or ``None``."""
+        s = self.spec
+        if not step_pays(M, s.width, s.ff, s.shared_ff or 0, s.experts, s.top, 1 if s.unit == "relu2" else 2):
+            return None
+        return self._rows(x_act, M)
+
+    def _takes_prompt(self, x_act: torch.Tensor, M: int):
+        """More of them on the tcgen05 kernels in one call: the rows' addresses, or ``None``."""
+        s = self.spec
+        if not (self.takes_tensor_cores(M * s.top, x_act) and N.has("ll_moe_prompt")
+                and N.call_ret("ll_moe_prompt_supported", M, s.width, s.experts, s.ff, s.shared_ff or 0)):
+            return None
+        return self._rows(x_act, M)
+
     def forward(self, x_act: torch.Tensor) -> torch.Tensor:
         s, M = self.spec, x_act.shape[0]
         at = self._takes_step(x_act, M) if M <= STEP_MAX_TOKENS else None
         if at:
-            return self._step(at, x_act, M)
+            return self._one_call("ll_moe_step", at, x_act, M, _step_scratch_bytes(M, s.experts, s.top, s.ff, s.shared_ff or 0))
+        at = self._takes_prompt(x_act, M)
+        if at:
+            return self._one_call("ll_moe_prompt", at, x_act, M, N.call_ret("ll_moe_prompt_scratch_bytes", M, s.width, s.experts, s.top, s.ff,
+                                                                             s.shared_ff or 0))
         dev, dtype = x_act.device, x_act.dtype
         dt, st = N.dtype_code(dtype), N.stream()
         _, w, offsets, perm = self.route(x_act)
