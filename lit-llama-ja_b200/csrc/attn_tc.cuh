@@ -1,8 +1,8 @@
 // Softmax attention of prompts on tcgen05: S = Q K^T and O += P V with fp32 accumulators in tensor memory.
 //
-// A block owns 256 consecutive queries of one head as two tiles of 128 and walks the keys they can see 64 at a time:
+// A block owns two tiles of 128 queries of one head (neighbours, or one from each end: at_apart) and walks the keys they can see 64 at a time:
 //   warps 0-7, 8-15 : softmax of tile 0 / tile 1; two threads share a query row, each 32 of its 64 scores: they read them from tensor
-//                     memory, scale, cap, mask, exponentiate, write the weights back over the scores as packed bf16 (one term, or
+//                     memory, scale, cap, mask, exponentiate, write the weights back over their own scores as packed bf16 (one term, or
 //                     two: hi and what hi left over) and keep the row's sum; at the end they normalise and store the row
 //   warp 16         : TMA producer (queries once, then key and value blocks into rings)
 //   warps 17, 18    : one thread each issues the MMAs of a tile: the scores of the next key block first, then P V of this one
@@ -10,12 +10,16 @@
 // Scores have two buffers per tile, so that the tensor cores form the next block's scores while a block's weights are made; the
 // weights lie where the scores were (MMAs of one thread run in issue order).  The running maximum only moves when a row's scores
 // outgrow it by 2^8: the accumulator is then rescaled in place, which after the first blocks of a row hardly ever happens; the
-// result does not depend on it.
+// result does not depend on it.  Capped scores have a bound of their own: where it is at most 2^80 they need no maximum, and the two threads
+// of a row nothing from one another before the end.
 // Keys are addressed by position in a ring (slot = position % ring): a block of keys ends where the ring wraps.  Rows past the
 // last key of the step may hold anything: their scores are masked and their value rows are cleared in shared memory.
 //
 // What bounds it is the softmax: a row's chain (load, maximum, exponent, split, store) runs at one instruction in four clocks
-// for a warp on its own, so a row has two threads and a scheduler four such warps.
+// for a warp on its own, so a row has two threads and a scheduler four such warps.  2048 queries, 16 heads of 128, two terms, us: 52 (capped 68)
+// with neighbouring tiles, one barrier of a tile's 256 threads a block of keys and a running maximum for capped scores as well; 40 (45) now.
+// Blocks of 128 keys with one buffer of scores a tile (no second one fits beside the accumulators): 53 and 60, a tile's chain of weights,
+// P V and the next scores being what it waits for.
 // Every wait is bounded; one that runs out records a code, all roles stop, copies in flight are waited for, tensor memory is freed.
 #pragma once
 #include <climits>
@@ -54,6 +58,7 @@ constexpr int AT_QBOX = AT_Q * 64 * 2, AT_KBOX = AT_K * 64 * 2;      // TMA boxe
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 constexpr float AT_LOG2E = 1.4426950408889634f;
 constexpr float AT_SLACK = 8.f;                       // a row's scores may outgrow its reference by 2^8 before it moves
+constexpr float AT_BOUND = 80.f;                      // scores that a cap keeps within 2^-80 .. 2^80 need no reference
 
 __device__ int g_attn_tc_error = 0;     // per file that instantiates the kernel: its entry asks for it (attn_tc_error)
 
@@ -65,6 +70,7 @@ struct AtParams {
   __nv_bfloat16* y;
   float scale, softcap;
   int T, H, group, vdim, window, chunk, ring, gate_ld, gate_per_head, gate_vec, y_ld;
+  int apart;                   // a block's two tiles: one from the end and one from the start (else neighbours)
   int* word;                   // wait_word()
 };
 
@@ -177,18 +183,23 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
-// Barrier `id` of the 256 threads of a tile; whether any of them says yes.
+// Barrier `id` of the 64 threads that share 32 rows; whether any of them says yes.
 __device__ __forceinline__ bool at_any(int id, bool yes) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %2, 0;\n\t"
-      "barrier.cta.red.or.pred q, %1, 256, p;\n\t"
+      "barrier.cta.red.or.pred q, %1, 64, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
       : "r"(id), "r"((uint32_t)yes)
       : "memory");
   return r != 0;
+}
+__device__ __forceinline__ float at_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 __device__ __forceinline__ int at_first_visible(int i, int window, int chunk) {
@@ -253,8 +264,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   float* s_x = reinterpret_cast<float*>(s_range + 4); // [tile][half][row]: what the two threads of a row tell one another
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // the last queries see the most keys: they go first, so that the long blocks do not end up as the tail
-  const int t0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * 2 * AT_Q, h = blockIdx.y, b = blockIdx.z, g = h / p.group;
+  // neighbours: the last queries see the most keys, so they go first, and the long blocks do not end up as the tail
+  const int q_tiles = (p.T + AT_Q - 1) / AT_Q, pair = (int)gridDim.x - 1 - (int)blockIdx.x;
+  const int tile0 = p.apart ? q_tiles - 1 - (int)blockIdx.x : 2 * pair, tile1 = p.apart ? (int)blockIdx.x : 2 * pair + 1;
+  const int tq0 = tile0 * AT_Q, tq1 = tile1 != tile0 ? tile1 * AT_Q : p.T;      // (the middle one of an odd number stands alone)
+  const int h = blockIdx.y, b = blockIdx.z, g = h / p.group;
 
   if (threadIdx.x == 0) {
     prefetch_tensormap(&map_q);
@@ -276,8 +290,17 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  if (warp == AT_WARPS && elect_one()) {                // the queries do not depend on the positions
+    const int tiles = tq1 < p.T ? 2 : 1;
+    mbar_expect_tx(q_full, (uint32_t)(tiles * NB * AT_QBOX));
+    for (int i = 0; i < tiles; ++i) {
+      for (int c = 0; c < NB1; ++c) tma_box4(sq + (i * NB + c) * AT_QBOX, &map_q, c * 64, h, i ? tq1 : tq0, b, q_full);
+      for (int c = 0; c < NB2; ++c) tma_box4(sq + (i * NB + NB1 + c) * AT_QBOX, &map_q2, c * 64, h, i ? tq1 : tq0, b, q_full);
+    }
+  }
+  __syncwarp();
   // positions of the tiles' queries
-  const int tile = warp >> 3, half = (warp >> 2) & 1, row = (int)(threadIdx.x & (AT_Q - 1)), t = t0 + tile * AT_Q + row;
+  const int tile = warp >> 3, half = (warp >> 2) & 1, row = (int)(threadIdx.x & (AT_Q - 1)), t = (tile ? tq1 : tq0) + row;
   int qp = 0;
   if (warp < AT_WARPS) {
     if (t < p.T) qp = p.pos_ids[t];
@@ -301,12 +324,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   if (warp == AT_WARPS) {
     // ===================== TMA producer =====================
     if (elect_one()) {
-      const int tiles = t0 + AT_Q < p.T ? 2 : 1;
-      mbar_expect_tx(q_full, (uint32_t)(tiles * NB * AT_QBOX));
-      for (int i = 0; i < tiles; ++i) {
-        for (int c = 0; c < NB1; ++c) tma_box4(sq + (i * NB + c) * AT_QBOX, &map_q, c * 64, h, t0 + i * AT_Q, b, q_full);
-        for (int c = 0; c < NB2; ++c) tma_box4(sq + (i * NB + NB1 + c) * AT_QBOX, &map_q2, c * 64, h, t0 + i * AT_Q, b, q_full);
-      }
       int n = 0;
       bool ok = true;
       for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next(), ++n) {
@@ -374,7 +391,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           for (int term = 0; term < TERMS; ++term)
 #pragma unroll
             for (int k = 0; k < AT_K / UMMA_K; ++k)            // 16 keys: 8 columns of packed weights, two groups of eight rows
-              umma_ts(tm_o, tm_s + 64u * buf + 32u * term + 8u * k, vdesc + (uint64_t)(128 * k), idesc_o,
+              umma_ts(tm_o, tm_s + 64u * buf + 32u * (k >> 1) + 16u * term + 8u * (k & 1), vdesc + (uint64_t)(128 * k), idesc_o,
                       (np != 0u || (term | k) != 0) ? 1u : 0u);
           umma_commit(&o_full[2 * i + (int)buf]);
           umma_commit(&v_empty[vs]);
@@ -418,11 +435,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     const float slope = BIAS ? p.slopes[h] * bias_unit : 0.f;
     float* const mine = s_x + (tile * 2 + half) * AT_Q + row;
     const float* const other = s_x + (tile * 2 + (half ^ 1)) * AT_Q + row;
-    float ref = -INFINITY;
+    const int bar = 1 + tile * 4 + (warp & 3);
+    const bool bounded = CAP && cap2 <= AT_BOUND;
+    float ref = bounded ? 0.f : -INFINITY;
     f2 sum2[2] = {f2_of(0.f, 0.f), f2_of(0.f, 0.f)};
     uint32_t n = 0;
     bool ok = true;
-    for (AtBlock blk(kt0, last, p.ring); blk.any(); blk.next()) {
+    for (AtBlock blk(kt0, last, p.ring); ok && blk.any(); blk.next()) {
       if (blk.meets(mylo, myhi)) {
         const uint32_t ts = ts0 + 64u * (n & 1u);
         ok = at_wait(&s_full[2 * tile + (int)(n & 1u)], (n >> 1) & 1u, s_fail, p.word, 7);
@@ -440,32 +459,29 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         }
         const int cmin = qlo - c0, cmax = min(blk.rows - 1 - AT_C * half, qp - c0);          // visible columns of this row
         const bool masked = __any_sync(0xffffffffu, cmin > 0 || cmax < AT_C - 1);
-        float amx = 0.f;
         if (masked) {
 #pragma unroll
           for (int e = 0; e < AT_C; ++e)
-            if (e < cmin || e > cmax) sr[e] = __float_as_uint(-INFINITY);
-        } else if (CAP) {
-          float a4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int e = 0; e < AT_C; ++e) a4[e & 3] = fmaxf(a4[e & 3], fabsf(__uint_as_float(sr[e])));
-          amx = fmaxf(fmaxf(a4[0], a4[1]), fmaxf(a4[2], a4[3]));
+            if (e < cmin || e > cmax) sr[e] = bounded ? 0u : __float_as_uint(-INFINITY);
         }
-        float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+        float mx = 0.f;
+        if (!bounded) {
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int e = 0; e < AT_C; ++e) m4[e & 3] = fmaxf(m4[e & 3], __uint_as_float(sr[e]));
-        float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-        // (a NaN among the scores is passed over by amx; NaN * P(NaN) stays NaN)
-        const bool poly = CAP && !masked && __all_sync(0xffffffffu, amx * mul < AT_TANH_SMALL);
-        if (mx != -INFINITY) {                                              // the row's largest score in units of log2
-          mx *= mul;
-          if (CAP) mx = cap2 * (1.f - 2.f * at_rcp(1.f + at_exp2(mx * (2.f * AT_LOG2E))));
+          for (int e = 0; e < AT_C; e += 2) m4[(e >> 1) & 3] = at_max3(m4[(e >> 1) & 3], __uint_as_float(sr[e]), __uint_as_float(sr[e + 1]));
+          mx = at_max3(m4[0], m4[1], fmaxf(m4[2], m4[3]));
+          if (mx != -INFINITY) {                                              // the row's largest score in units of log2
+            mx *= mul;
+            if (CAP) mx = cap2 * (1.f - 2.f * at_rcp(1.f + at_exp2(mx * (2.f * AT_LOG2E))));
+          }
         }
         __syncwarp();      // the stores to tensor memory below are the whole warp's: lanes part above this line and not between it and them
-        // one barrier of the tile's warps per block: does any row's reference have to move, has any wait run out?
-        if (at_any(1 + tile, !ok || mx > ref + AT_SLACK || (ref == -INFINITY && mx > -INFINITY))) {
+        if (bounded) {
+          if (!__all_sync(0xffffffffu, ok)) break;
+        } else if (at_any(bar, !ok || mx > ref + AT_SLACK || (ref == -INFINITY && mx > -INFINITY))) {
+          // (one barrier of the rows' two warps per block: does any row's reference have to move, has any wait run out?)
           *mine = mx;
-          ok = !at_any(1 + tile, !ok);
+          ok = !at_any(bar, !ok);
           if (!ok) break;
           const float mo = *other;
           const float nref = fmaxf(ref, fmaxf(mx, mo));
@@ -476,7 +492,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           if (n > 0) ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, p.word, 8);
           __syncwarp();
           tc_fence_after();
-          if (at_any(1 + tile, !ok)) {                                      // (also: both threads of a row have read the other's)
+          if (at_any(bar, !ok)) {                                      // (also: both threads of a row have read the other's)
             ok = false;
             break;
           }
@@ -505,23 +521,40 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             f2_split(a, a0, a1);
             sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
           }
-        } else if (poly) {
+        } else {
+          // tanh by its polynomial, looking on the way at how large the squares are; where some row's are too large the raw scores, taken from
+          // tensor memory again, go through the exponential form.  (A NaN is passed over; NaN * P(NaN) stays NaN.)
           const float m3 = mul * mul * mul, c0p = cap2 * AT_T0 * mul, c1p = cap2 * AT_T1 * m3, c2p = cap2 * AT_T2 * (m3 * mul * mul);
           const f2 p0c = f2_of(c0p, c0p), p1c = f2_of(c1p, c1p), p2c = f2_of(c2p, c2p);
+          float u4[4] = {0.f, 0.f, 0.f, 0.f};
+          if (bounded || !masked) {
 #pragma unroll
-          for (int e = 0; e < AT_C; e += 2) {
-            const f2 x = f2_of(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), u = f2_mul(x, x);
-            const f2 a = f2_fma(x, f2_fma(f2_fma(p2c, u, p1c), u, p0c), sub2);
-            float a0, a1;
-            f2_split(a, a0, a1);
-            sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
+            for (int e = 0; e < AT_C; e += 2) {
+              const f2 x = f2_of(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), u = f2_mul(x, x);
+              const f2 a = f2_fma(x, f2_fma(f2_fma(p2c, u, p1c), u, p0c), sub2);
+              float a0, a1, u0, u1;
+              f2_split(a, a0, a1);
+              f2_split(u, u0, u1);
+              u4[(e >> 1) & 3] = at_max3(u4[(e >> 1) & 3], u0, u1);
+              sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
+            }
           }
-        } else {
-          const float k2 = mul * (2.f * AT_LOG2E), top = cap2 + sub, two = -2.f * cap2;
+          if (!(bounded || !masked) || !__all_sync(0xffffffffu, at_max3(u4[0], u4[1], fmaxf(u4[2], u4[3])) * (mul * mul) < AT_TANH_SMALL * AT_TANH_SMALL)) {
+            const float k2 = mul * (2.f * AT_LOG2E), top = cap2 + sub, two = -2.f * cap2;
+            tmem_ld32_async(ts + (uint32_t)(AT_C * half), sr);
+            tmem_wait_ld();
+            tie32(sr);
 #pragma unroll
-          for (int e = 0; e < AT_C; ++e) {
-            const float a = fmaf(two, at_rcp(1.f + at_exp2(__uint_as_float(sr[e]) * k2)), top);
-            sr[e] = __float_as_uint(masked && (e < cmin || e > cmax) ? -INFINITY : a);
+            for (int e = 0; e < AT_C; ++e) {
+              float x = __uint_as_float(sr[e]);
+              if (BIAS) x = fmaf(slope, (float)(c0 + e - qp), x * (p.scale * bias_unit));
+              sr[e] = __float_as_uint(fmaf(two, at_rcp(1.f + at_exp2(x * k2)), top));
+            }
+          }
+          if (masked) {
+#pragma unroll
+            for (int e = 0; e < AT_C; ++e)
+              if (e < cmin || e > cmax) sr[e] = __float_as_uint(-INFINITY);
           }
         }
         // weights
@@ -540,9 +573,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             pl[e] = pack_bf16(l0, l1);
           }
         }
-        // the tile's warps have all read their scores (the barrier above): the weights go over them
-        tmem_st16(ts + 16u * half, ph);
-        if (TERMS == 2) tmem_st16(ts + 32u + 16u * half, pl);
+        // the weights go over the thread's own scores: 16 columns of the first term, 16 of the second
+        tmem_st16(ts + (uint32_t)(AT_C * half), ph);
+        if (TERMS == 2) tmem_st16(ts + (uint32_t)(AT_C * half) + 16u, pl);
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -550,50 +583,58 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         ++n;
       }
     }
-    if (ok && n > 0 && t0 + tile * AT_Q < p.T) {
-      ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, p.word, 9);
-      __syncwarp();
-      tc_fence_after();
-      float s0, s1;
-      f2_split(f2_add(sum2[0], sum2[1]), s0, s1);
-      *mine = s0 + s1;
-      if (!at_any(1 + tile, !ok)) {
-        float den = half == 0 ? *mine + *other : *other + *mine;            // the halves' sums in the order of the columns
-        if (p.sink) den += at_exp2(p.sink[h] * AT_LOG2E - ref);
-        float fin = den > 0.f ? 1.f / den : 0.f;
-        const size_t m = (size_t)b * p.T + t;
-        const bool live = t < p.T;
-        if (live && p.gate && p.gate_per_head) fin *= at_sigmoid(__bfloat162float(p.gate[m * p.gate_ld + h]));
-        __nv_bfloat16* dst = p.y + m * p.y_ld + (size_t)h * p.vdim;
-        const __nv_bfloat16* gt = p.gate && !p.gate_per_head ? p.gate + m * p.gate_ld + (size_t)h * p.vdim : nullptr;
-#pragma unroll 1
-        for (int c = 32 * half; c < DV; c += 64) {
-          // the row's gate numbers are asked for before the accumulator is waited for, 16 bytes at a time (two at a time, one after
-          // the other, took as long as half of the keys)
-          uint4 gu[4];
+    const bool store = n > 0 && (tile ? tq1 : tq0) < p.T, live = t < p.T;
+    const size_t m = (size_t)b * p.T + t;
+    const __nv_bfloat16* gt = p.gate && !p.gate_per_head ? p.gate + m * p.gate_ld + (size_t)h * p.vdim : nullptr;
+    // the row's gate numbers are asked for before the accumulator is waited for, 16 bytes at a time
+    uint4 gu[NBV][4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (gt && live && c + 8 * e < p.vdim) gu[e] = at_load8(gt + c + 8 * e, p.gate_vec);
-          __syncwarp();
-          uint32_t o[32];
-          tmem_ld32_async(to + (uint32_t)c, o);
-          tmem_wait_ld();
-          tie32(o);
+    for (int z = 0; z < NBV; ++z)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (!live || c + 8 * e >= p.vdim) continue;           // (vdim is a multiple of 8)
-            const uint32_t gw[4] = {gu[e].x, gu[e].y, gu[e].z, gu[e].w};
-            uint32_t w[4];
+      for (int e = 0; e < 4; ++e) {
+        const int c = 64 * z + 32 * half + 8 * e;
+        gu[z][e] = make_uint4(0u, 0u, 0u, 0u);
+        if (gt && live && c < p.vdim) gu[z][e] = at_load8(gt + c, p.gate_vec);
+      }
+    if (ok && store) ok = at_wait(&o_full[2 * tile + (int)((n - 1u) & 1u)], ((n - 1u) >> 1) & 1u, s_fail, p.word, 9);
+    __syncwarp();
+    tc_fence_after();
+    float s0, s1;
+    f2_split(f2_add(sum2[0], sum2[1]), s0, s1);
+    *mine = s0 + s1;
+    if (!at_any(bar, !ok) && store) {
+      float den = half == 0 ? *mine + *other : *other + *mine;            // the halves' sums in the order of the columns
+      float num = 1.f;
+      if (p.sink) {                                     // (scaled by whichever is larger, the reference or the sink)
+        const float sk = p.sink[h] * AT_LOG2E - ref, up = fmaxf(sk, 0.f);
+        num = at_exp2(-up);
+        den = den * num + at_exp2(sk - up);
+      }
+      float fin = den > 0.f ? num / den : 0.f;
+      if (live && p.gate && p.gate_per_head) fin *= at_sigmoid(__bfloat162float(p.gate[m * p.gate_ld + h]));
+      __nv_bfloat16* dst = p.y + m * p.y_ld + (size_t)h * p.vdim;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float a = __uint_as_float(o[8 * e + 2 * j]) * fin, z = __uint_as_float(o[8 * e + 2 * j + 1]) * fin;
-              if (gt) a *= at_sigmoid(bf16_bits_to_f32(gw[j] & 0xffffu)), z *= at_sigmoid(bf16_bits_to_f32(gw[j] >> 16));
-              w[j] = pack_bf16(a, z);
-            }
-            *reinterpret_cast<uint4*>(dst + c + 8 * e) = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int z = 0; z < NBV; ++z) {
+        const int c = 64 * z + 32 * half;
+        __syncwarp();
+        uint32_t o[32];
+        tmem_ld32_async(to + (uint32_t)c, o);
+        tmem_wait_ld();
+        tie32(o);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (!live || c + 8 * e >= p.vdim) continue;           // (vdim is a multiple of 8)
+          const uint32_t gw[4] = {gu[z][e].x, gu[z][e].y, gu[z][e].z, gu[z][e].w};
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float a = __uint_as_float(o[8 * e + 2 * j]) * fin, q = __uint_as_float(o[8 * e + 2 * j + 1]) * fin;
+            if (gt) a *= at_sigmoid(bf16_bits_to_f32(gw[j] & 0xffffu)), q *= at_sigmoid(bf16_bits_to_f32(gw[j] >> 16));
+            w[j] = pack_bf16(a, q);
           }
-          __syncwarp();
+          *reinterpret_cast<uint4*>(dst + c + 8 * e) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        __syncwarp();
       }
     }
     tc_fence_before();
@@ -660,13 +701,20 @@ bool attn_tc_supported(const AttnTcArgs& a) {
          a.y_ld % 8 == 0 && ((uintptr_t)a.y & 15) == 0 && (a.terms == 1 || a.terms == 2);
 }
 
+// Which tiles a block takes.  Queries that see all keys before them have very unequal walks: of neighbours the last two walk everything while the
+// first two are done at once, and with fewer blocks than SMs nothing evens that out; one tile from the end and one from the start make all
+// blocks alike (2048 queries, 16 heads of 128: 50 us -> 40, capped 57 -> 45; 32 heads 84 -> 74).  Tiles that a window keeps alike stay
+// neighbours, which share most of their keys (window 700 of 2048: 30.3, apart 31.3; chunks of 512: 21.7, apart 24.7; a window of half of the
+// queries is even at 33, one of 1500 of 1736 42 -> 40 apart).
+bool at_apart(const AttnTcArgs& a) { return a.chunk <= 0 && (a.window <= 0 || 2ll * a.window >= a.T); }
+
 enum AttnTcKind { AT_ROTARY, AT_LATENT };     // which forms a file instantiates
 
 template <AttnTcKind KIND>
 int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
   const AtParams p{a.pos_ids, a.sink, a.slopes, (const __nv_bfloat16*)a.gate, (__nv_bfloat16*)a.y, a.scale, a.softcap, a.T, a.H, a.H / a.G,
                    a.v.dim, a.window, a.chunk, a.ring, a.gate_ld, a.gate_per_head,
-                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, wait_word()};
+                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, at_apart(a), wait_word()};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
   const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \

@@ -47,6 +47,12 @@ CASES = [dict(T=t, past=0, ring=512) for t in (16, 63, 64, 65, 127, 128, 129, 25
 ]
 
 
+# a block's tiles from both ends: an even and an odd number of them, positions before the step, a window of most queries; caps with and without a bound
+APART = [dict(T=513, past=70, ring=583, cap=50.0, sink=True, gate=True), dict(T=640, past=0, ring=640), dict(T=385, past=0, ring=385, cap=100.0, sink=True),
+         dict(T=700, past=20, ring=720, window=400), dict(T=640, past=3, ring=700, cap=1.5, slopes=True, spoil=True)]
+CASES += APART
+
+
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
 def test_softmax_prompt_against_fp32_form(case):
     got, top = _softmax(**case)
