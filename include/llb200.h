@@ -653,6 +653,19 @@ LL_API size_t ll_decay_chunked_unit_scratch_bytes(int B, int T, int H, int n, in
 LL_API int ll_decay_chunked_unit(const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride, int dtype, const float* a,
                                  const float* ks, float qs, float* state, const int32_t* pos_ids, float* y, int B, int T, int H, int qk_heads,
                                  int n, int p, float* scratch, ll_stream stream);
+/* A matrix memory layer (ll_matrix_memory_gates, the recurrence with its constant column, ll_gated_group_norm_rows) with both projections in one
+ * call, bf16.  p: columns of a head with the constant one; chunks: ll_decay_chunked_unit (else ll_decay_scan). */
+LL_API size_t ll_matrix_memory_layer_scratch_bytes(int B, int T, int n_in, int H, int n, int p);
+LL_API int ll_matrix_memory_layer(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int g_col, int i_col, int f_col,
+                                  const float* bias_i, const float* bias_f, float gate_cap, const float* norm, float eps, float qs, float* memory,
+                                  float* stabiliser, const int32_t* pos_ids, int B, int T, int width, int H, int n, int p, int chunks, void* out,
+                                  void* scratch, ll_stream stream);
+/* y[m][n] = sum_k x[m][k] w[n][k], bf16 with fp32 sums, any number of rows; head_cols > 0: w is [N / head_cols][K][head_cols] instead of [N][K].  K, ldx
+ * in multiples of 8, head_cols of 64, x and w on 16-byte boundaries.  ll_dense_rows_error(): as ll_moe_tc_error. */
+LL_API int ll_dense_rows(const void* x, int ldx, const void* w, int head_cols, void* y, int ldy, int M, int N, int K, ll_stream stream);
+LL_API int ll_dense_rows_error(void);
+/* The same by the form that a layer of one call takes for this many rows. */
+LL_API int ll_rows_linear(const void* x, int ldx, const void* w, void* y, int ldy, int M, int N, int K, ll_stream stream);
 /* Gated delta rule (csrc/delta_rule.cu), per sequence b and head h with S an n x p matrix, q and k of head h / (H / qk_heads):
  *   k^ = k / sqrt(|k|^2 + unit_eps),  q^ = q / sqrt(|q|^2 + unit_eps) * qs
  *   g = exp(-exp(a_log[h]) * softplus(raw_a + dt_bias[h])),  beta = sigmoid(raw_b)
@@ -773,11 +786,25 @@ LL_API int ll_latent_step(const void* x, const void* w_in, int n_in, const void*
                           float eps, const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim,
                           int rot_dims, int v_dim, int kv_rank, int cache_len, int gate_col0, int kv_col0, int window, float scale, int splits,
                           int weight_terms, void* out, void* scratch, ll_stream stream);
+/* The same layer for B sequences of T tokens each, any number of rows.  rows > 0: attention over plain keys and values of the cache's first
+ * `rows` slots per sequence (all of them, or one sequence), formed per head (as ll_latent_prompt_attn; values of 64 or 128, splits 1); rows 0: in
+ * latent space. */
+LL_API size_t ll_latent_layer_scratch_bytes(int B, int T, int n_in, int heads, int nope, int rot_dim, int kv_rank, int v_dim, int rows, int splits);
+LL_API int ll_latent_layer(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm, float eps,
+                           const float* rope, const int32_t* pos_ids, void* cache, int B, int T, int width, int heads, int nope, int rot_dim, int rot_dims,
+                           int v_dim, int kv_rank, int cache_len, int rows, int gate_col0, int kv_col0, int window, float scale, int splits,
+                           int weight_terms, void* out, void* scratch, ll_stream stream);
 LL_API size_t ll_softmax_step_scratch_bytes(int B, int n_in, int H, int dim, int vdim, int splits);
 LL_API int ll_softmax_step(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col,
                            const float* q_norm, const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc,
                            void* vc, const float* sink, const float* slopes, float scale, float softcap, int B, int width, int H, int G, int dim,
                            int vdim, int window, int chunk, int ring, int splits, int form, void* out, void* scratch, ll_stream stream);
+/* The same layer for B sequences of T tokens each, any number of rows (x [B * T][width] bf16): projections of more than two rows by
+ * ll_dense_rows.  Scratch: ll_softmax_step_scratch_bytes of B * T rows. */
+LL_API int ll_softmax_layer(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col, const float* q_norm,
+                            const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc, void* vc, const float* sink,
+                            const float* slopes, float scale, float softcap, int B, int T, int width, int H, int G, int dim, int vdim, int window,
+                            int chunk, int ring, int splits, int form, void* out, void* scratch, ll_stream stream);
 
 #ifdef __cplusplus
 }

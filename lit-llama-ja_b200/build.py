@@ -29,6 +29,9 @@ FAMILY_SOURCES = {
     "Bumulix": ["quant_pack", "residual_ops", "rotary_attn", "latent_attn"],
 }
 
+# what kernels of a file call in another one
+DEPENDS = {"rotary_attn": ["dense_rows"], "latent_attn": ["dense_rows"], "decay_chunk": ["dense_rows"]}
+
 
 def sources():
     return sorted(CSRC.glob("*.cu"))
@@ -71,7 +74,7 @@ def build_only(name, stems, verbose=False):
     """A reduced library from the named sources only -> lit_llama/libllb200_<name>.so (select it with LLB200_LIB=<path>):
     what a model family needs, without waiting for the kernels of the others.  Rebuilt only when a source is newer."""
     out = HERE / "lit_llama" / f"libllb200_{name}.so"
-    srcs = [CSRC / f"{s}.cu" for s in stems]
+    srcs = [CSRC / f"{s}.cu" for s in dict.fromkeys(d for s in stems for d in (s, *DEPENDS.get(s, ())))]
     deps = srcs + list(CSRC.glob("*.cuh")) + [HERE.parent / "include" / "llb200.h"]
     if out.exists() and all(p.stat().st_mtime <= out.stat().st_mtime for p in deps):
         return out

@@ -241,6 +241,7 @@ template <int NB1, int NB2, int NBV, int TERMS, bool CAP, bool BIAS>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2,
                                                                const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_k2,
                                                                const __grid_constant__ CUtensorMap map_v, const AtParams p) {
+  pdl_launch_dependents();
   using Shape = AtShape<NB1, NB2, NBV>;
   constexpr int NB = Shape::NB, KS = Shape::KS, VS = Shape::VS, DV = NBV * 64;
   constexpr uint32_t TM_S = 0, TM_O = 256;            // per tile: two score buffers of 64 columns; 128 accumulator columns

@@ -17,6 +17,7 @@
 // 2048 tokens, 8 heads of 128 x 257: the walk took 496 us (a chain of 2048 steps), collect + pass + read take 24 + 14 + 51.  Column tiles of
 // 64: with three terms of the state a tile of 128 leaves one block per SM.
 #include "chunk_mma.cuh"
+#include "dense_rows.cuh"
 
 namespace llb {
 
@@ -415,6 +416,60 @@ int ll_decay_chunked_unit(const void* q, int q_stride, const void* k, int k_stri
   LL_DCU(16) LL_DCU(32) LL_DCU(64) LL_DCU(128)
 #undef LL_DCU
   return LL_ERR_UNSUPPORTED;
+}
+
+namespace {
+struct MatrixLayerScratch {
+  void *proj, *normed;
+  float *keep, *take, *stab, *y, *chunks;
+  size_t total;
+};
+MatrixLayerScratch matrix_layer_carve(void* base, int B, int T, int n_in, int H, int n, int p) {
+  MatrixLayerScratch s;
+  size_t o = 0;
+  auto take = [&](size_t b) { void* r = (uint8_t*)base + o; o += (b + 255) & ~(size_t)255; return r; };
+  const size_t M = (size_t)B * T;
+  s.proj = take(M * n_in * 2);
+  s.keep = (float*)take(M * H * 4), s.take = (float*)take(M * H * 4), s.stab = (float*)take(M * H * 4);
+  s.y = (float*)take(M * H * p * 4);
+  s.normed = take(M * H * (p - 1) * 2);
+  s.chunks = (float*)take(T >= DC_L ? ll_decay_chunked_unit_scratch_bytes(B, T, H, n, p) : 0);
+  s.total = o;
+  return s;
+}
+}  // namespace
+
+size_t ll_matrix_memory_layer_scratch_bytes(int B, int T, int n_in, int H, int n, int p) { return matrix_layer_carve(nullptr, B, T, n_in, H, n, p).total; }
+
+int ll_matrix_memory_layer(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int g_col, int i_col, int f_col,
+                           const float* bias_i, const float* bias_f, float gate_cap, const float* norm, float eps, float qs, float* memory, float* stabiliser,
+                           const int32_t* pos_ids, int B, int T, int width, int H, int n, int p, int chunks, void* out, void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_in && w_o && bias_i && bias_f && norm && memory && stabiliser && pos_ids && out && scratch, "matrix_memory_layer: null pointer");
+  LL_CHECK_ARG(B > 0 && T > 0 && H > 0 && n > 0 && p > 1 && q_col >= 0 && k_col >= 0 && v_col >= 0 && g_col >= 0 && i_col >= 0 && f_col >= 0,
+               "bad matrix_memory_layer arguments");
+  const int hv = H * (p - 1), M = B * T;
+  if (width % 8 != 0 || n_in % 8 != 0 || hv % 8 != 0) {
+    set_error("matrix_memory_layer takes widths in multiples of 8 (width=%d rows %d heads %d x %d)", width, n_in, H, p - 1);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0, "matrix_memory_layer: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const MatrixLayerScratch s = matrix_layer_carve(scratch, B, T, n_in, H, n, p);
+  const __nv_bfloat16* proj = (const __nv_bfloat16*)s.proj;
+  if (int r = rows_linear(x, width, w_in, s.proj, n_in, M, n_in, width, false, st)) return r;
+  if (int r = ll_matrix_memory_gates(proj + i_col, proj + f_col, LL_BF16, n_in, bias_i, bias_f, gate_cap, stabiliser, pos_ids, s.keep, s.take, s.stab, B, T, H,
+                                     stream))
+    return r;
+  if (chunks) {
+    if (int r = ll_decay_chunked_unit(proj + q_col, n_in, proj + k_col, n_in, proj + v_col, n_in, LL_BF16, s.keep, s.take, qs, memory, pos_ids, s.y, B, T, H, H, n,
+                                      p, s.chunks, stream))
+      return r;
+  } else if (int r = ll_decay_scan(proj + q_col, n_in, proj + k_col, n_in, proj + v_col, n_in, LL_BF16, s.keep, 0, s.take, nullptr, qs, memory, pos_ids, s.y, B,
+                                   T, H, H, n, p, 1, stream)) {
+    return r;
+  }
+  if (int r = ll_gated_group_norm_rows(s.y, p, s.stab, proj + g_col, n_in, norm, 0, eps, H, 0, 1, s.normed, hv, LL_BF16, M, hv, stream)) return r;
+  return rows_linear(s.normed, hv, w_o, out, width, M, width, hv, true, st);
 }
 
 }  // extern "C"

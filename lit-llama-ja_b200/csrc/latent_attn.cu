@@ -12,7 +12,7 @@
 // part; the (cos, sin) table is [positions][rot_dims / 2][2] fp32.  Scores, softmax weights and sums
 // are fp32; T is the dtype of activations and of the cache.
 #include "attn_tc.cuh"
-#include "small_rows.cuh"
+#include "dense_rows.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -744,37 +744,27 @@ LatentStepScratch latent_step_carve(void* base, int B, int n_in, int heads, int 
   s.total = o;
   return s;
 }
+struct LatentExpandScratch {
+  void *proj, *q_rot, *k, *v, *o;
+  size_t total;
+};
+LatentExpandScratch latent_expand_carve(void* base, int B, int T, int n_in, int heads, int nope, int rot_dim, int v_dim, int rows) {
+  LatentExpandScratch s;
+  size_t o = 0;
+  auto take = [&](size_t b) { void* r = (uint8_t*)base + o; o += (b + 255) & ~(size_t)255; return r; };
+  const size_t M = (size_t)B * T, R = (size_t)B * rows;
+  s.proj = take(M * n_in * 2);
+  s.q_rot = take(M * heads * rot_dim * 2);
+  s.k = take(R * heads * nope * 2);
+  s.v = take(R * heads * v_dim * 2);
+  s.o = take(M * heads * v_dim * 2);
+  s.total = o;
+  return s;
+}
 }  // namespace
 
 size_t ll_latent_step_scratch_bytes(int B, int n_in, int heads, int kv_rank, int v_dim, int splits) {
   return latent_step_carve(nullptr, B, n_in, heads, kv_rank, v_dim, splits).total;
-}
-
-int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm, float eps,
-                   const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim, int rot_dims, int v_dim,
-                   int kv_rank, int cache_len, int gate_col0, int kv_col0, int window, float scale, int splits, int weight_terms, void* out,
-                   void* scratch, ll_stream stream) {
-  LL_CHECK_ARG(x && w_in && w_uk && w_uv_t && w_o && rope && pos_ids && cache && out && scratch, "latent_step: null pointer");
-  LL_CHECK_ARG(heads > 0 && nope > 0 && kv_rank > 0 && v_dim > 0 && splits >= 1, "bad latent_step arguments");
-  if (B < 1 || B > SR_MAX || width % 8 != 0 || n_in % 8 != 0 || kv_rank % 8 != 0 || v_dim % 8 != 0 || kv_rank > 1024 || nope > 1024) {
-    set_error("latent_step takes 1 to %d sequences and sizes in multiples of 8 (B=%d width=%d rank=%d v=%d)", SR_MAX, B, width, kv_rank, v_dim);
-    return LL_ERR_UNSUPPORTED;
-  }
-  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_uk | (uintptr_t)w_uv_t | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0,
-               "latent_step: rows must be 16-byte aligned bf16");
-  cudaStream_t st = (cudaStream_t)stream;
-  const LatentStepScratch s = latent_step_carve(scratch, B, n_in, heads, kv_rank, v_dim, splits);
-  const long long lat_h = (long long)B * kv_rank, q_head = nope + rot_dim;
-  if (int r = small_linear(x, width, w_in, s.proj, n_in, B, n_in, width, st)) return r;
-  if (kv_norm != nullptr)
-    if (int r = ll_latent_kv_append(s.proj, LL_BF16, n_in, kv_col0, kv_norm, eps, rope, pos_ids, cache, B, 1, kv_rank, rot_dim, rot_dims, cache_len, stream))
-      return r;
-  if (int r = small_heads(s.proj, q_head, n_in, w_uk, s.q_lat, lat_h, kv_rank, heads, B, kv_rank, nope, st)) return r;
-  if (int r = ll_latent_attn_terms(s.q_lat, lat_h, kv_rank, s.proj, n_in, nope, (int)q_head, gate_col0, rope, pos_ids, cache, s.o_lat, lat_h, kv_rank,
-                                   LL_BF16, B, 1, heads, kv_rank, rot_dim, rot_dims, cache_len, window, scale, splits, weight_terms, s.split, stream))
-    return r;
-  if (int r = small_heads(s.o_lat, lat_h, kv_rank, w_uv_t, s.o, v_dim, (long long)heads * v_dim, heads, B, v_dim, kv_rank, st)) return r;
-  return small_linear(s.o, heads * v_dim, w_o, out, width, B, width, heads * v_dim, st);
 }
 
 int ll_latent_prompt_supported(int nope, int rot_dim, int v_dim, int kv_rank, int q_stride, int q_head_stride, int y_stride) {
@@ -809,6 +799,66 @@ int ll_latent_prompt_attn(const void* q, int q_stride, int nope, int q_head_stri
       (const __nv_bfloat16*)q, q_stride, nope, q_head_stride, rope, pos_ids, (__nv_bfloat16*)q_rot, T, n_head, rot_dim, rot_dims, pieces);
   LL_LAUNCH_OK("latent_rotate_q_kernel");
   return attn_tc_launch<AT_LATENT>(a, (cudaStream_t)stream);
+}
+
+int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm, float eps,
+                   const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim, int rot_dims, int v_dim,
+                   int kv_rank, int cache_len, int gate_col0, int kv_col0, int window, float scale, int splits, int weight_terms, void* out,
+                   void* scratch, ll_stream stream) {
+  if (B < 1 || B > SR_MAX) {
+    set_error("latent_step takes 1 to %d sequences (B=%d)", SR_MAX, B);
+    return LL_ERR_UNSUPPORTED;
+  }
+  return ll_latent_layer(x, w_in, n_in, w_uk, w_uv_t, w_o, kv_norm, eps, rope, pos_ids, cache, B, 1, width, heads, nope, rot_dim, rot_dims, v_dim, kv_rank,
+                         cache_len, 0, gate_col0, kv_col0, window, scale, splits, weight_terms, out, scratch, stream);
+}
+
+size_t ll_latent_layer_scratch_bytes(int B, int T, int n_in, int heads, int nope, int rot_dim, int kv_rank, int v_dim, int rows, int splits) {
+  return rows > 0 ? latent_expand_carve(nullptr, B, T, n_in, heads, nope, rot_dim, v_dim, rows).total
+                  : latent_step_carve(nullptr, B * T, n_in, heads, kv_rank, v_dim, splits).total;
+}
+
+int ll_latent_layer(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm, float eps,
+                    const float* rope, const int32_t* pos_ids, void* cache, int B, int T, int width, int heads, int nope, int rot_dim, int rot_dims, int v_dim,
+                    int kv_rank, int cache_len, int rows, int gate_col0, int kv_col0, int window, float scale, int splits, int weight_terms, void* out,
+                    void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_in && w_uk && w_uv_t && w_o && rope && pos_ids && cache && out && scratch, "latent_layer: null pointer");
+  LL_CHECK_ARG(B > 0 && T > 0 && heads > 0 && nope > 0 && kv_rank > 0 && v_dim > 0 && splits >= 1 && rows >= 0 && rows <= cache_len &&
+                   (rows == 0 || rows == cache_len || B == 1),
+               "bad latent_layer arguments");
+  if (width % 8 != 0 || n_in % 8 != 0 || kv_rank % 8 != 0 || v_dim % 8 != 0 || kv_rank > 1024 || nope > 1024 ||
+      (rows > 0 && (v_dim % 64 != 0 || !ll_latent_prompt_supported(nope, rot_dim, v_dim, kv_rank, n_in, nope + rot_dim, heads * v_dim)))) {
+    set_error("latent_layer takes sizes in multiples of 8, values of 64 or 128 where rows are expanded (B=%d T=%d width=%d rank=%d v=%d)", B, T, width, kv_rank,
+              v_dim);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_uk | (uintptr_t)w_uv_t | (uintptr_t)w_o | (uintptr_t)scratch | (rows ? (uintptr_t)cache : 0)) & 15) == 0,
+               "latent_layer: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const int M = B * T, q_head = nope + rot_dim, row = kv_rank + rot_dim;
+  const LatentExpandScratch e = latent_expand_carve(scratch, B, T, n_in, heads, nope, rot_dim, v_dim, rows);
+  const LatentStepScratch s = latent_step_carve(scratch, M, n_in, heads, kv_rank, v_dim, splits);      // (proj stands first in both)
+  if (int r = rows_linear(x, width, w_in, s.proj, n_in, M, n_in, width, false, st)) return r;
+  if (kv_norm != nullptr)
+    if (int r = ll_latent_kv_append(s.proj, LL_BF16, n_in, kv_col0, kv_norm, eps, rope, pos_ids, cache, B, T, kv_rank, rot_dim, rot_dims, cache_len, stream))
+      return r;
+  if (rows > 0) {                        // keys and values of the cache's first rows, per head
+    const int hk = heads * nope, hv = heads * v_dim;
+    if (int r = dense_rows(cache, row, w_uk, 0, e.k, hk, B * rows, hk, kv_rank, st)) return r;
+    if (int r = dense_rows(cache, row, w_uv_t, v_dim, e.v, hv, B * rows, hv, kv_rank, st)) return r;
+    const __nv_bfloat16* gate = gate_col0 >= 0 ? (const __nv_bfloat16*)s.proj + gate_col0 : nullptr;
+    if (int r = ll_latent_prompt_attn(s.proj, n_in, nope, q_head, gate, n_in, rope, pos_ids, e.k, hk, nope, e.v, hv, v_dim, cache, e.q_rot, e.o, hv, B, T, heads,
+                                      kv_rank, rot_dim, rot_dims, v_dim, rows, window, scale, weight_terms, stream))
+      return r;
+    return rows_linear(e.o, hv, w_o, out, width, M, width, hv, true, st);
+  }
+  const long long lat_h = (long long)M * kv_rank;
+  if (int r = small_heads(s.proj, q_head, n_in, w_uk, s.q_lat, lat_h, kv_rank, heads, M, kv_rank, nope, st)) return r;
+  if (int r = ll_latent_attn_terms(s.q_lat, lat_h, kv_rank, s.proj, n_in, nope, q_head, gate_col0, rope, pos_ids, cache, s.o_lat, lat_h, kv_rank,
+                                   LL_BF16, B, T, heads, kv_rank, rot_dim, rot_dims, cache_len, window, scale, splits, weight_terms, s.split, stream))
+    return r;
+  if (int r = small_heads(s.o_lat, lat_h, kv_rank, w_uv_t, s.o, v_dim, (long long)heads * v_dim, heads, M, v_dim, kv_rank, st)) return r;
+  return rows_linear(s.o, heads * v_dim, w_o, out, width, M, width, heads * v_dim, true, st);
 }
 
 int ll_latent_prompt_error(void) { return attn_tc_error(); }

@@ -401,6 +401,7 @@ template <typename TA>
 __global__ void gated_group_norm_kernel(const float* __restrict__ y, int y_gs, const float* __restrict__ stab,
                                         const TA* __restrict__ gate, int gate_stride, const float* __restrict__ w, int w_shared,
                                         float eps, int groups, int gate_first, int gate_sigmoid, TA* __restrict__ out, int out_stride, int C) {
+  pdl_launch_dependents();             // (a projection that follows sets itself up under this kernel)
   const int m = blockIdx.x;
   const int gs = C / groups;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -19,7 +19,7 @@
 //             combined as a difference, o = a_0 - lambda * a_1, then divided by the root mean square of o over the head's
 //             values (eps inside the root) and multiplied by `post`; the gate, if any, follows.
 #include "attn_tc.cuh"
-#include "small_rows.cuh"
+#include "dense_rows.cuh"
 #include "common.cuh"
 
 namespace llb {
@@ -420,6 +420,7 @@ __global__ void __launch_bounds__(SA_WARPS * 32) softmax_attn_kernel(
     const int32_t* __restrict__ pos_ids, const float* __restrict__ sink, const float* __restrict__ slopes, float scale, float softcap,
     int Tn, int H, int G, int dim, int vdim, int window, int chunk, int ring, int splits, int maps, int pairs, float* __restrict__ part_ml,
     float* __restrict__ part_acc, T* __restrict__ y, int y_stride) {
+  pdl_launch_dependents();             // (a projection that follows sets itself up under this kernel)
   // a warp owns one (query, head, map); with one map per head, h below is the head itself
   const int pair = blockIdx.x * SA_WARPS + (threadIdx.x >> 5);
   if (pair >= pairs) return;
@@ -575,6 +576,7 @@ __global__ void softmax_attn_merge_kernel(const float* __restrict__ part_ml, con
                                           const T* __restrict__ gate, int gate_stride, const float* __restrict__ sink, int H, int vdim,
                                           int splits, int maps, float lambda, float post, float eps, int pairs, T* __restrict__ y,
                                           int y_stride) {
+  pdl_launch_dependents();             // (a projection that follows sets itself up under this kernel)
   __shared__ float wsp[4][2][SA_MAX_SPLITS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = blockIdx.x * (blockDim.x >> 5) + warp;      // (query, head)
@@ -720,6 +722,7 @@ __global__ void __launch_bounds__(TM_THREADS, MAPS == 1 ? 3 : 2) softmax_attn_mm
     const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ vc, const int32_t* __restrict__ pos_ids,
     const float* __restrict__ sink, const float* __restrict__ slopes, float scale, float softcap, int Tn, int H, int G, int dim, int vdim,
     int window, int chunk, int ring, float lambda, float post, float eps, __nv_bfloat16* __restrict__ y, int y_stride) {
+  pdl_launch_dependents();             // (a projection that follows sets itself up under this kernel)
   constexpr int LD = DK + 8, CH = DK / 8, LV = DV + 8, CV = DV / 8, STAGE = TM_K * (LD + LV);      // a stage: 64 key rows, then 64 value rows
   extern __shared__ __align__(16) unsigned char tm_smem[];
   __nv_bfloat16* const stages = (__nv_bfloat16*)tm_smem;
@@ -1130,29 +1133,42 @@ size_t ll_softmax_step_scratch_bytes(int B, int n_in, int H, int dim, int vdim, 
   return softmax_step_carve(nullptr, B, n_in, H, dim, vdim, splits).total;
 }
 
+int ll_softmax_layer(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col, const float* q_norm,
+                     const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc, void* vc, const float* sink,
+                     const float* slopes, float scale, float softcap, int B, int T, int width, int H, int G, int dim, int vdim, int window, int chunk,
+                     int ring, int splits, int form, void* out, void* scratch, ll_stream stream) {
+  LL_CHECK_ARG(x && w_in && w_o && pos_ids && kc && vc && out && scratch, "softmax_layer: null pointer");
+  LL_CHECK_ARG(B > 0 && T > 0 && H > 0 && G > 0 && dim > 0 && vdim > 0 && splits >= 1 && q_col >= 0 && k_col >= 0, "bad softmax_layer arguments");
+  if (width % 8 != 0 || n_in % 8 != 0 || (H * vdim) % 8 != 0) {
+    set_error("softmax_layer takes widths in multiples of 8 (width=%d rows %d heads %d x %d)", width, n_in, H, vdim);
+    return LL_ERR_UNSUPPORTED;
+  }
+  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0, "softmax_layer: rows must be 16-byte aligned bf16");
+  cudaStream_t st = (cudaStream_t)stream;
+  const int M = B * T;
+  const SoftmaxStepScratch s = softmax_step_carve(scratch, M, n_in, H, dim, vdim, splits);
+  const __nv_bfloat16* proj = (const __nv_bfloat16*)s.proj;
+  if (int r = rows_linear(x, width, w_in, s.proj, n_in, M, n_in, width, false, st)) return r;
+  if (int r = ll_qk_rotary_append_maps(proj + q_col, n_in, proj + k_col, n_in, v_col >= 0 ? proj + v_col : nullptr, n_in, LL_BF16, q_norm, k_norm, eps, freq,
+                                       rot_dims, pos_ids, s.q, kc, vc, B, T, H, G, dim, vdim, ring, 1, stream))
+    return r;
+  if (int r = ll_softmax_attn_rows(s.q, H * dim, gate_col >= 0 ? proj + gate_col : nullptr, gate_col >= 0 ? n_in : 0, kc, vc, LL_BF16, pos_ids, sink, slopes,
+                                   scale, softcap, B, T, H, G, dim, vdim, window, chunk, ring, splits, form, 1, 0.f, 1.f, eps, splits > 1 ? s.split : nullptr,
+                                   s.y, H * vdim, stream))
+    return r;
+  return rows_linear(s.y, H * vdim, w_o, out, width, M, width, H * vdim, true, st);
+}
+
 int ll_softmax_step(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col, const float* q_norm,
                     const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc, void* vc, const float* sink,
                     const float* slopes, float scale, float softcap, int B, int width, int H, int G, int dim, int vdim, int window, int chunk, int ring,
                     int splits, int form, void* out, void* scratch, ll_stream stream) {
-  LL_CHECK_ARG(x && w_in && w_o && pos_ids && kc && vc && out && scratch, "softmax_step: null pointer");
-  LL_CHECK_ARG(H > 0 && G > 0 && dim > 0 && vdim > 0 && splits >= 1 && q_col >= 0 && k_col >= 0, "bad softmax_step arguments");
-  if (B < 1 || B > SR_MAX || width % 8 != 0 || n_in % 8 != 0 || (H * vdim) % 8 != 0) {
-    set_error("softmax_step takes 1 to %d sequences and widths in multiples of 8 (B=%d width=%d heads %d x %d)", SR_MAX, B, width, H, vdim);
+  if (B < 1 || B > SR_MAX) {
+    set_error("softmax_step takes 1 to %d sequences (B=%d)", SR_MAX, B);
     return LL_ERR_UNSUPPORTED;
   }
-  LL_CHECK_ARG((((uintptr_t)x | (uintptr_t)w_in | (uintptr_t)w_o | (uintptr_t)scratch) & 15) == 0, "softmax_step: rows must be 16-byte aligned bf16");
-  cudaStream_t st = (cudaStream_t)stream;
-  const SoftmaxStepScratch s = softmax_step_carve(scratch, B, n_in, H, dim, vdim, splits);
-  const __nv_bfloat16* proj = (const __nv_bfloat16*)s.proj;
-  if (int r = small_linear(x, width, w_in, s.proj, n_in, B, n_in, width, st)) return r;
-  if (int r = ll_qk_rotary_append_maps(proj + q_col, n_in, proj + k_col, n_in, v_col >= 0 ? proj + v_col : nullptr, n_in, LL_BF16, q_norm, k_norm, eps, freq,
-                                       rot_dims, pos_ids, s.q, kc, vc, B, 1, H, G, dim, vdim, ring, 1, stream))
-    return r;
-  if (int r = ll_softmax_attn_rows(s.q, H * dim, gate_col >= 0 ? proj + gate_col : nullptr, gate_col >= 0 ? n_in : 0, kc, vc, LL_BF16, pos_ids, sink, slopes,
-                                   scale, softcap, B, 1, H, G, dim, vdim, window, chunk, ring, splits, form, 1, 0.f, 1.f, eps, splits > 1 ? s.split : nullptr,
-                                   s.y, H * vdim, stream))
-    return r;
-  return small_linear(s.y, H * vdim, w_o, out, width, B, width, H * vdim, st);
+  return ll_softmax_layer(x, w_in, n_in, w_o, q_col, k_col, v_col, gate_col, q_norm, k_norm, eps, freq, rot_dims, pos_ids, kc, vc, sink, slopes, scale, softcap,
+                          B, 1, width, H, G, dim, vdim, window, chunk, ring, splits, form, out, scratch, stream);
 }
 
 int ll_softmax_attn_biased(const void* q, int q_stride, const void* gate, int gate_stride, const void* kc, const void* vc, int dtype,

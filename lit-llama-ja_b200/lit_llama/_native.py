@@ -152,6 +152,16 @@ EXPORTS = {
     "ll_softmax_step_scratch_bytes": ([i32] * 6, sz_t),
     "ll_softmax_step": ([vp, vp, i32, vp, i32, i32, i32, i32, vp, vp, C.c_float, vp, i32, vp, vp, vp, vp, vp, C.c_float, C.c_float] + [i32] * 11
                         + [vp, vp, vp], C.c_int),
+    "ll_dense_rows": ([vp, i32, vp, i32, vp, i32, i32, i32, i32, vp], C.c_int),
+    "ll_dense_rows_error": ([], C.c_int),
+    "ll_rows_linear": ([vp, i32, vp, vp, i32, i32, i32, i32, vp], C.c_int),
+    "ll_softmax_layer": ([vp, vp, i32, vp, i32, i32, i32, i32, vp, vp, C.c_float, vp, i32, vp, vp, vp, vp, vp, C.c_float, C.c_float] + [i32] * 12
+                         + [vp, vp, vp], C.c_int),
+    "ll_latent_layer_scratch_bytes": ([i32] * 10, sz_t),
+    "ll_latent_layer": ([vp, vp, i32, vp, vp, vp, vp, C.c_float, vp, vp, vp] + [i32] * 14 + [C.c_float, i32, i32, vp, vp, vp], C.c_int),
+    "ll_matrix_memory_layer_scratch_bytes": ([i32] * 6, sz_t),
+    "ll_matrix_memory_layer": ([vp, vp, i32, vp] + [i32] * 6 + [vp, vp, C.c_float, vp, C.c_float, C.c_float, vp, vp, vp] + [i32] * 7 + [vp, vp, vp],
+                               C.c_int),
     "ll_moe_step_supported": ([i32, i32, i32, i32], C.c_int),
     "ll_moe_step_scratch_bytes": ([i32, i32, i32, i32, i32], sz_t),
     "ll_moe_step": ([vp, vp, vp, vp, i32, C.c_float, i32, i32, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, C.c_float, C.c_float,
@@ -316,6 +326,22 @@ def gemv(args: GemvArgs) -> None:
     global LAUNCHES
     LAUNCHES += 1
     check(_fn["ll_int4_gemv"](C.byref(args), stream()), "ll_int4_gemv")
+
+
+FEW_ROWS, LARGE_WEIGHTS = 8, 1 << 25
+
+
+def layer_rows(M: int, weights: int, most: int, large: bool) -> bool:
+    """Whether a layer of ``M`` rows that could run in one call does.  A few rows of a layer that is not large: always, its products are as fast as
+    the library's (csrc/small_rows.cuh).  Else while rows times weights, which is what its kernels' time goes by, stays under ``most``, the work that
+    takes as long as the host takes to make the separate calls (``large``: also with weights whose way from memory is most of the time).  A step that
+    is being captured has no such calls to save, and there the library's products of more rows are the faster ones."""
+    if weights <= LARGE_WEIGHTS:
+        if M <= FEW_ROWS:
+            return True
+    elif not large:
+        return False
+    return M * weights <= most and not torch.cuda.is_current_stream_capturing()
 
 
 _PLAIN = (torch.nn.Parameter, torch.Tensor)

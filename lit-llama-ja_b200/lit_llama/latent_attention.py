@@ -46,11 +46,16 @@ EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
 # 48 / 43 and 50 / 44, 52 / 48 and 52 / 48, 66 / 63 and 66 / 62.
 # From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
+# Rows times weights of a layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 2048 rows 92 / 40,
+# 95 / 56, 95 / 76; 2048, 17, 400, 1024 and 2048 rows 93 / 43, 92 / 66, 92 / 76, 110 / 108; 4096, 3, 17, 120 and 700 rows 89 / 62, 92 / 62, 93 / 79, 101 / 114.  A
+# few rows, replayed as a graph: one token of four sequences over 1500 rows, widths 1024 and 2048: 37 / 34, 43 / 39 (4096: 55 / 59, so not there).
+LAYER_MAX_PRODUCTS = 12 << 30
+LATENT_MAX_ROW_HEADS = 512           # rows times heads of a step in one call whose queries stay in latent space: 18 rows, 16 heads 89 / 60, 32 heads 89 / 93
 
 
 @functools.lru_cache(maxsize=1024)
-def _step_scratch_bytes(B: int, n_in: int, heads: int, kv_rank: int, v_dim: int, splits: int) -> int:
-    return N.call_ret("ll_latent_step_scratch_bytes", B, n_in, heads, kv_rank, v_dim, splits)
+def _layer_scratch_bytes(*sizes: int) -> int:
+    return N.call_ret("ll_latent_layer_scratch_bytes", *sizes)
 
 
 @dataclass
@@ -193,21 +198,47 @@ class LatentAttention(nn.Module):
                 splits: int = 1, end: Optional[int] = None) -> torch.Tensor:
         """x_act ``[B*T, width]`` -> ``[B*T, width]``; ``cache`` ``[B, S, row]`` is this layer's or its source's (already
         appended to by the source in this step).  ``end``: as in ``attend``."""
-        if T == 1:
-            at = self._takes_step(x_act, B, cache)
-            if at:
-                return self._step(at, x_act, B, pos_ids, rope, cache, splits)
+        at, rows = (self._takes_step(x_act, B, cache), 0) if T == 1 else (None, 0)
+        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, True):
+            at, rows = self._takes_layer_rows(x_act, B, T, cache, splits, end)
+        if at:
+            return self._one_call(at, x_act, B, T, pos_ids, rope, cache, rows, splits)
         return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
 
     def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor):
-        """One bf16 token of one or two sequences, plain queries, at most a gate per head: the whole layer in one call, if its weights are
+        """One token of one or two sequences."""
+        return self._takes_layer(x_act, B, cache, "ll_latent_step") if 1 <= B <= STEP_MAX_ROWS else None
+
+    def _takes_layer_rows(self, x_act: torch.Tensor, B: int, T: int, cache: torch.Tensor, splits: int, end: Optional[int]):
+        """Several rows: (the weights' addresses or ``None``, cache rows per sequence that are expanded per head or 0).  The form of attention is
+        the one that the separate calls would take."""
+        s = self.spec
+        at = self._takes_layer(x_act, B * T, cache, "ll_latent_layer")
+        if not at:
+            return None, 0
+        S, n_in = cache.shape[1], self._parameters["w_in"].shape[0]
+        if T >= EXPAND_MIN_TOKENS and splits == 1:
+            first, rows = self._visible(T, S, end)
+            if (s.scale > 0 and self._expand_pays(B, T, rows)
+                    and N.call_ret("ll_latent_prompt_supported", s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, n_in, s.q_head, s.heads * s.v_dim)
+                    and cache.data_ptr() % 16 == 0):
+                whole = first is None or (first == 0 and (B == 1 or rows == S))
+                return (at, rows) if whole and s.v_dim % 64 == 0 else (None, 0)
+        return (at, 0) if B * T * s.heads <= LATENT_MAX_ROW_HEADS else (None, 0)
+
+    def _expand_pays(self, B: int, T: int, rows: int) -> bool:
+        s = self.spec
+        return rows <= EXPAND_MAX_SLOTS_PER_TOKEN * T and 2 * B * rows * s.heads * (s.nope_dim + s.v_dim) <= EXPAND_MAX_BYTES
+
+    def _takes_layer(self, x_act: torch.Tensor, M: int, cache: torch.Tensor, entry: str):
+        """``M`` bf16 rows, plain queries, at most a gate per head: the whole layer in one call, if its weights are
         what the layer was built with.  Their addresses, or ``None``."""
         s, p = self.spec, self._parameters
         w = p.get("w_in")
-        if not (1 <= B <= STEP_MAX_ROWS and w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
+        if not (w is not None and s.q_rank is None and s.gate != "element" and x_act.is_cuda
                 and x_act.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and cache.is_contiguous()
-                and cache.get_device() == x_act.get_device() and x_act.shape == (B, s.width) and s.kv_rank <= 1024 and s.nope_dim <= 1024
-                and N.has("ll_latent_step")):
+                and cache.get_device() == x_act.get_device() and x_act.shape == (M, s.width) and s.kv_rank <= 1024 and s.nope_dim <= 1024
+                and N.has(entry)):
             return None
         n_in = w.shape[0]
         if n_in < self.n_in or (s.width | s.kv_rank | s.v_dim | n_in) % 8:
@@ -215,15 +246,16 @@ class LatentAttention(nn.Module):
         return N.step_rows(x_act, (w, p.get("w_uk"), p.get("w_uv_t"), p.get("w_o")),
                            ((n_in, s.width), (s.heads, s.nope_dim, s.kv_rank), (s.heads, s.kv_rank, s.v_dim), (s.width, s.heads * s.v_dim)))
 
-    def _step(self, at, x_act: torch.Tensor, B: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, splits: int) -> torch.Tensor:
+    def _one_call(self, at, x_act: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, rope: torch.Tensor, cache: torch.Tensor, rows: int,
+                  splits: int) -> torch.Tensor:
         s, p = self.spec, self._parameters
         x, w_in, w_uk, w_uv_t, w_o = at
         n_in = p["w_in"].shape[0]
         norm = None if not self.owns_cache else p["kv_norm"] if "kv_norm" in p else self.kv_norm
         out = torch.empty_like(x_act)
-        scratch = x_act.new_empty(_step_scratch_bytes(B, n_in, s.heads, s.kv_rank, s.v_dim, splits) // 2)          # (whole pieces of 128 bytes or more)
-        N.call("ll_latent_step", x, w_in, n_in, w_uk, w_uv_t, w_o, N.ptr(norm), float(s.eps), N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), B, s.width,
-               s.heads, s.nope_dim, s.rot_dim, s.rot_dims, s.v_dim, s.kv_rank, cache.shape[1], self.gate_col0 if s.gate == "head" else -1,
+        scratch = x_act.new_empty(_layer_scratch_bytes(B, T, n_in, s.heads, s.nope_dim, s.rot_dim, s.kv_rank, s.v_dim, rows, splits) // 2)  # (whole pieces)
+        N.call("ll_latent_layer", x, w_in, n_in, w_uk, w_uv_t, w_o, N.ptr(norm), float(s.eps), N.ptr(rope), N.ptr(pos_ids), N.ptr(cache), B, T, s.width,
+               s.heads, s.nope_dim, s.rot_dim, s.rot_dims, s.v_dim, s.kv_rank, cache.shape[1], rows, self.gate_col0 if s.gate == "head" else -1,
                self.kv_col0, s.window if s.window is not None else 0, float(s.scale), splits, 2 if s.exact_weights else 1, N.ptr(out),
                N.ptr(scratch), N.stream())
         return out
@@ -275,8 +307,7 @@ class LatentAttention(nn.Module):
         48 / 574 -> 27 / 192, 2048 after 0 734 -> 68; 64 heads, 16 after 1000 102 -> 50, 200 after 7000 1679 -> 267.  Rows that no query
         sees are not worth forming: with all of 8192 slots expanded, 150 tokens at position 0 took 41 -> 60 (16 heads) and 76 -> 146 (64)."""
         s = self.spec
-        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0 and rows <= EXPAND_MAX_SLOTS_PER_TOKEN * T
-                and 2 * B * rows * s.heads * (s.nope_dim + s.v_dim) <= EXPAND_MAX_BYTES
+        return (q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and s.scale > 0 and self._expand_pays(B, T, rows)
                 and N.has("ll_latent_prompt_attn") and cache.is_contiguous() and (out is None or (out.stride(1) == 1 and out.data_ptr() % 16 == 0))
                 and bool(N.call_ret("ll_latent_prompt_supported", s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, q.stride(0), s.q_head,
                                     s.heads * s.v_dim if out is None else out.stride(0)))

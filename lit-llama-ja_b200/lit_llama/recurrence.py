@@ -30,6 +30,7 @@ the gates are in the activation dtype.  A sequence at position 0 starts from a z
 """
 from __future__ import annotations
 
+import functools
 import os
 from dataclasses import dataclass
 from typing import List, Tuple
@@ -44,6 +45,17 @@ from .short_conv import ShortConv
 
 def pad8(n: int) -> int:
     return (n + 7) // 8 * 8
+
+
+# Rows times weights of a matrix memory layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 1024
+# rows 66 / 30, 77 / 57, 79 / 74; 2048, 17, 400 and 700 rows 67 / 33, 78 / 70, 86 / 94; 4096, 17 and 400 rows 67 / 30, 78 / 68.  A few rows, replayed as a
+# graph: one token of three sequences, widths 1024, 2048, 4096: 20 / 13, 21 / 18, 26 / 17.
+LAYER_MAX_PRODUCTS = 6 << 30
+
+
+@functools.lru_cache(maxsize=1024)
+def _matrix_scratch_bytes(*sizes: int) -> int:
+    return N.call_ret("ll_matrix_memory_layer_scratch_bytes", *sizes)
 
 
 USE_CHUNKS = os.environ.get("LLB200_DECAY_CHUNKS", "1") != "0"       # 0: always walk token by token
@@ -298,11 +310,39 @@ class MatrixMemoryMixer(nn.Module):
         self.norm.copy_(get("norm").float())
         self.w_o.copy_(get("o"))
 
+    def _takes_layer(self, u: torch.Tensor, M: int):
+        """``M`` bf16 rows and weights that are what the layer was built with: their addresses, or ``None``."""
+        s, p = self.spec, self._parameters
+        w = p.get("w_in")
+        if not (w is not None and u.is_cuda and u.dtype is torch.bfloat16 and u.shape == (M, s.width) and N.has("ll_matrix_memory_layer")):
+            return None
+        n_in, hv = w.shape[0], s.heads * s.vdim
+        if n_in < self.n_in or (s.width | hv | n_in) % 8:
+            return None
+        return N.step_rows(u, (w, p.get("w_o")), ((n_in, s.width), (s.width, hv)))
+
+    def _one_call(self, at, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, states) -> torch.Tensor:
+        s, p, c = self.spec, self._parameters, self.cols
+        x, w_in, w_o = at
+        n_in = p["w_in"].shape[0]
+        out = torch.empty_like(u)
+        scratch = u.new_empty(_matrix_scratch_bytes(B, T, n_in, s.heads, s.dim, s.vdim + 1) // 2)          # (whole pieces of 128 bytes or more)
+        chunks = (USE_CHUNKS and N.has("ll_decay_chunked_unit") and (c["q"] | c["k"] | c["v"]) % 8 == 0
+                  and N.call_ret("ll_decay_chunked_supported", N.LL_BF16, T, s.dim, s.vdim, n_in, n_in, n_in))
+        bias_i, bias_f, norm = (p[n] if n in p else getattr(self, n) for n in ("bias_i", "bias_f", "norm"))
+        N.call("ll_matrix_memory_layer", x, w_in, n_in, w_o, c["q"], c["k"], c["v"], c["g"], c["i"], c["f"], N.ptr(bias_i), N.ptr(bias_f),
+               float(s.gate_cap), N.ptr(norm), float(s.eps), s.dim ** -0.5, N.ptr(states[0]), N.ptr(states[1]), N.ptr(pos_ids), B, T, s.width, s.heads,
+               s.dim, s.vdim + 1, 1 if chunks else 0, N.ptr(out), N.ptr(scratch), N.stream())
+        return out
+
     def forward(self, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, states) -> torch.Tensor:
         s = self.spec
         c = self.cols
         memory, stabiliser = states
         M = B * T
+        at = self._takes_layer(u, M) if N.layer_rows(M, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, True) else None
+        if at:
+            return self._one_call(at, u, B, T, pos_ids, states)
         proj = F.linear(u, self.w_in)
         keep = torch.empty((M, s.heads), dtype=torch.float32, device=u.device)
         take, stab = torch.empty_like(keep), torch.empty_like(keep)

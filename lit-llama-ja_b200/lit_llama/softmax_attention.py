@@ -57,6 +57,10 @@ def pad8(n: int) -> int:
 # 55 / 53, 37 / 32 to 59 / 57, 55 / 50 to 80 / 71; with 32 key heads of width 4096 62 / 61 (69 / 65) to 90 / 93 (99 / 100).
 # From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
+# Rows times weights of a layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 1024 rows 53 / 28,
+# 54 / 42, 54 / 50; 2048, 17, 120 and 400 rows 54 / 33, 55 / 44, 53 / 54; 4096, 17 and 60 rows 56 / 60, 62 / 66 (so not there).  A few rows, replayed as
+# a graph: one token of three sequences over 100 keys, widths 1024 and 2048: 29 / 24, 32 / 29.
+LAYER_MAX_PRODUCTS = 4 << 30
 
 
 @functools.lru_cache(maxsize=1024)
@@ -221,19 +225,24 @@ class SoftmaxAttention(nn.Module):
 
     def forward(self, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
                 form: int = 0) -> torch.Tensor:
-        if T == 1:
-            at = self._takes_step(u, B, caches)
-            if at:
-                return self._step(at, u, B, pos_ids, caches, splits, form)
+        at = self._takes_step(u, B, caches) if T == 1 else None
+        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, False):
+            at = self._takes_layer(u, B * T, caches, "ll_softmax_layer")
+        if at:
+            return self._one_call(at, u, B, T, pos_ids, caches, splits, form)
         return F.linear(self.attend(F.linear(u, self.w_in), B, T, pos_ids, caches, conv_state, splits, form), self.w_o)
 
     def _takes_step(self, u: torch.Tensor, B: int, caches):
-        """One bf16 token of one or two sequences on a layer with its own ring, one score map, no short convolution and nothing prepared head by
-        head: the whole layer in one call, if its weights are what the layer was built with.  Their addresses, or ``None``."""
+        """One token of one or two sequences."""
+        return self._takes_layer(u, B, caches, "ll_softmax_step") if 1 <= B <= STEP_MAX_ROWS else None
+
+    def _takes_layer(self, u: torch.Tensor, M: int, caches, entry: str):
+        """``M`` bf16 rows on a layer with its own ring, one score map, no short convolution and nothing prepared head by head: the whole layer in
+        one call, if its weights are what the layer was built with.  Their addresses, or ``None``."""
         s, p = self.spec, self._parameters
         w = p.get("w_in")
-        if not (1 <= B <= STEP_MAX_ROWS and w is not None and self.owner and s.conv_taps == 0 and s.maps == 1 and not s.by_head
-                and not self.plain_q and u.is_cuda and u.dtype is torch.bfloat16 and u.shape == (B, s.width) and N.has("ll_softmax_step")):
+        if not (w is not None and self.owner and s.conv_taps == 0 and s.maps == 1 and not s.by_head
+                and not self.plain_q and u.is_cuda and u.dtype is torch.bfloat16 and u.shape == (M, s.width) and N.has(entry)):
             return None
         dev, n_in = u.get_device(), w.shape[0]
         for c in caches:
@@ -244,7 +253,7 @@ class SoftmaxAttention(nn.Module):
             return None
         return N.step_rows(u, (w, p.get("w_o")), ((n_in, s.width), (s.width, hv)))
 
-    def _step(self, at, u: torch.Tensor, B: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
+    def _one_call(self, at, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, splits: int, form: int) -> torch.Tensor:
         s, p, c = self.spec, self._parameters, self.cols
         kc, vc = caches
         x, w_in, w_o = at
@@ -253,10 +262,10 @@ class SoftmaxAttention(nn.Module):
         k_norm = p["k_norm"] if "k_norm" in p else self.k_norm
         sink = p["sink"] if "sink" in p else self.sink
         out = torch.empty_like(u)
-        scratch = u.new_empty(_step_scratch_bytes(B, n_in, s.heads, s.dim, s.vdim, splits) // 2)          # (whole pieces of 128 bytes or more)
-        N.call("ll_softmax_step", x, w_in, n_in, w_o, c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1, N.ptr(q_norm), N.ptr(k_norm),
+        scratch = u.new_empty(_step_scratch_bytes(B * T, n_in, s.heads, s.dim, s.vdim, splits) // 2)          # (whole pieces of 128 bytes or more)
+        N.call("ll_softmax_layer", x, w_in, n_in, w_o, c["q"], c["k"], c.get("v", -1), c["g"] if s.gate else -1, N.ptr(q_norm), N.ptr(k_norm),
                float(s.eps), N.ptr(self.freq), s.rotary.dims, N.ptr(pos_ids), N.ptr(kc), N.ptr(vc), N.ptr(sink), N.ptr(self.slopes), float(s.scale),
-               float(s.softcap), B, s.width, s.heads, s.kv_heads, s.dim, s.vdim, s.window or 0, s.chunk or 0, kc.shape[1], splits, form, N.ptr(out),
+               float(s.softcap), B, T, s.width, s.heads, s.kv_heads, s.dim, s.vdim, s.window or 0, s.chunk or 0, kc.shape[1], splits, form, N.ptr(out),
                N.ptr(scratch), N.stream())
         return out
 
