@@ -336,6 +336,8 @@ LL_API int ll_tp_reduce_add(void* x, const void* recv, uint32_t* cnt, int32_t* e
 
 /* ref: RMSNorm.forward, model.py:276-283 - every intermediate rounded to the activation dtype. */
 LL_API int ll_rmsnorm(const void* x, const void* weight, void* y, int dtype, int rows, int dim, float eps, ll_stream stream);
+/* sum = x + h (rounded), y = the norm of that sum as ll_rmsnorm: bf16 rows on 16-byte boundaries, dim a multiple of 8 up to 32768. */
+LL_API int ll_add_rmsnorm(const void* x, const void* h, void* sum, const void* w, void* y, int rows, int dim, float eps, ll_stream stream);
 
 /* ref: wte lookup, model.py:110, fused with the sum-of-squares partials the first fused RMSNorm
  * consumes: x[m][:] = wte[idx[m]][:]; ssq (optional, may be NULL): ssq[m][p] = sum over 16-column tile p of
@@ -400,6 +402,9 @@ LL_API int ll_advance_pos(int32_t* pos, int cache_len, int max_pos, ll_stream st
  * Lets LLaMA.forward(idx, max_seq_length, input_pos) honour an arbitrary input_pos without a
  * host sync (ref: model.py:101-104 index_select by input_pos). */
 LL_API int ll_set_pos(int32_t* pos, const int64_t* input_pos, int cache_len, int max_pos, ll_stream stream);
+/* The same for T tokens at input_pos [T]: pos_ids, slots = pos % cache_len, seen = min(pos, cache_len - 1).  A position outside 0 .. max_pos - 1 is
+ * reported by a later launch or ll_wait_check (LL_ERR_WAIT). */
+LL_API int ll_prompt_pos(int32_t* pos_ids, int32_t* slots, int32_t* seen, const int64_t* input_pos, int T, int cache_len, int max_pos, ll_stream stream);
 
 /* ---------------------------------------------------------------------------------------
  * A residual stream kept in fp32 whatever the activation dtype (csrc/residual_ops.cu).
@@ -480,6 +485,11 @@ LL_API int ll_latent_prompt_attn(const void* q, int q_stride, int nope, int q_he
  * ll_latent_prompt_attn / ll_softmax_attn*.  Both synchronise the device. */
 LL_API int ll_latent_prompt_error(void);
 LL_API int ll_softmax_attn_tc_error(void);
+/* Softmax attention of several tokens over a cache of S slots, bf16: q [B][H][T][hs], k, v [B][H][S][hs], y [B][T][H * hs].  Query t sees the slots
+ * 0 .. pos_ids[t] (pos_ids < S), in any order; softmax weights carry 16 bits. */
+LL_API int ll_causal_attn_supported(int head_size, int T);
+LL_API int ll_causal_attn(const void* q, const void* k, const void* v, const int32_t* pos_ids, void* y, int B, int T, int H, int hs, int S, float scale,
+                          ll_stream stream);
 LL_API size_t ll_latent_attn_scratch_bytes(int M, int n_head, int kv_rank, int splits);
 
 /* ---------------------------------------------------------------------------------------

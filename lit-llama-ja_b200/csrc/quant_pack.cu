@@ -45,6 +45,10 @@ int wait_check() {
   if (code != 0) *p = 0;
   if (g_wait_host.load(std::memory_order_relaxed) != 0) code = g_wait_host.exchange(0, std::memory_order_relaxed);
   if (code == 0) return LL_OK;
+  if (code >= 700) {
+    set_error("an earlier launch was given a token position outside the rotary table: what it and the launches after it wrote is not valid");
+    return LL_ERR_WAIT;
+  }
   static const char* const where[] = {"", "prompt attention", "int4 rows", "llm.int8", "grouped experts", "delta rule in chunks", "dense products"};
   set_error("a bounded wait ran out in an earlier launch (%s, code %d): what it and the launches after it wrote is not valid",
             code >= 100 && code < 700 ? where[code / 100] : "?", code);

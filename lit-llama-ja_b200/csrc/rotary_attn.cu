@@ -1194,6 +1194,26 @@ int ll_softmax_attn(const void* q, int q_stride, const void* gate, int gate_stri
                               window, chunk, ring, splits, form, 1, 0.f, 1.f, 0.f, scratch, y, stream);
 }
 
+int ll_causal_attn_supported(int head_size, int T) { return T > 0 && head_size > 0 && head_size % 8 == 0 && head_size <= 128; }
+
+int ll_causal_attn(const void* q, const void* k, const void* v, const int32_t* pos_ids, void* y, int B, int T, int H, int hs, int S, float scale,
+                   ll_stream stream) {
+  LL_CHECK_ARG(q && k && v && pos_ids && y, "causal_attn: null pointer");
+  LL_CHECK_ARG(B > 0 && H > 0 && S > 0 && scale > 0.f, "bad causal_attn arguments");
+  AttnTcArgs a{};
+  a.q = {q, hs, (long long)T * hs, hs, (long long)H * T * hs};
+  a.k = {k, hs, (long long)S * hs, hs, (long long)H * S * hs};
+  a.v = {v, hs, (long long)S * hs, hs, (long long)H * S * hs};
+  a.pos_ids = pos_ids, a.scale = scale;
+  a.B = B, a.T = T, a.H = H, a.G = H, a.ring = S, a.terms = 2;
+  a.y = y, a.y_ld = H * hs;
+  if (!ll_causal_attn_supported(hs, T) || !attn_tc_supported(a)) {
+    set_error("causal_attn: bf16 heads of up to 128 numbers in multiples of 8, on 16-byte boundaries (T=%d, head of %d)", T, hs);
+    return LL_ERR_UNSUPPORTED;
+  }
+  return attn_tc_launch<AT_ROTARY>(a, (cudaStream_t)stream);
+}
+
 int ll_softmax_attn_tc_error(void) { return attn_tc_error(); }
 
 }  // extern "C"

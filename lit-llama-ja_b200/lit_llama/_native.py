@@ -111,6 +111,9 @@ EXPORTS = {
     "ll_tp_ll_recv_bytes": ([i32, i32], sz_t),
     "ll_tp_ll_allreduce_add": ([vp, vp, vp, vp, i32, i32, i32, i32, vp], C.c_int),
     "ll_rmsnorm": ([vp, vp, vp, i32, i32, i32, C.c_float, vp], C.c_int),
+    "ll_add_rmsnorm": ([vp, vp, vp, vp, vp, i32, i32, C.c_float, vp], C.c_int),
+    "ll_causal_attn_supported": ([i32, i32], C.c_int),
+    "ll_causal_attn": ([vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, C.c_float, vp], C.c_int),
     "ll_embed_ssq": ([vp, vp, vp, vp, i32, i32, vp], C.c_int),
     "ll_rope_kv_append": ([vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_decode_attn": ([vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, i32, vp], C.c_int),
@@ -123,6 +126,7 @@ EXPORTS = {
     "ll_add": ([vp, vp, vp, i32, sz_t, vp], C.c_int),
     "ll_advance_pos": ([vp, i32, i32, vp], C.c_int),
     "ll_set_pos": ([vp, vp, i32, i32, vp], C.c_int),
+    "ll_prompt_pos": ([vp, vp, vp, vp, i32, i32, i32, vp], C.c_int),
     "ll_apply_rope": ([vp, vp, vp, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_embed_scaled": ([vp, i32, vp, C.c_float, vp, vp, i32, i32, i32, vp], C.c_int),
     "ll_gain_norm_add_mix": ([vp, vp, i32, vp, C.c_float, vp, vp, sz_t, vp, i32, vp, vp, i32, i32, i32, vp], C.c_int),

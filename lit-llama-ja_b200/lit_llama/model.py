@@ -22,7 +22,7 @@ import torch.nn as nn
 from torch.nn import functional as F
 
 from . import _native as N
-from .quantization import gated_pair
+from .quantization import gated_pair, is_plain
 from .stepping import graph_capture
 from .utils import find_multiple
 
@@ -118,6 +118,8 @@ class _Step:
     mask: Optional[torch.Tensor]       # bool mask for T > 1 with cache
     max_seq_length: int
     use_cache: bool
+    seen: Optional[torch.Tensor] = None   # int32 [T] last slot that a token of a multi-token step sees (what ``mask`` says: a position past the
+                                          # cache sees every slot)
 
 
 class CausalSelfAttention(nn.Module):
@@ -161,10 +163,17 @@ class CausalSelfAttention(nn.Module):
             N.call("ll_decode_attn", N.ptr(q), N.ptr(k_cache), N.ptr(v_cache), N.ptr(step.pos3), N.ptr(y),
                    N.dtype_code(x.dtype), B, nh, hs, S, splits, N.ptr(ws.attn_scratch), N.ptr(ws.attn_counters), 0,
                    N.stream())
+        elif step.seen is not None and x.dtype is torch.bfloat16:
+            # multi-token (prefill / no-cache) attention on the tcgen05 kernel, straight into the projection's rows
+            y = torch.empty((B, T, C), device=x.device, dtype=x.dtype)
+            N.call("ll_causal_attn", N.ptr(q), N.ptr(k_cache), N.ptr(v_cache), N.ptr(step.seen), N.ptr(y), B, T, nh, hs, S, hs ** -0.5, N.stream())
         else:
-            # multi-token (prefill / no-cache) attention: library SDPA, as the reference (model.py:237)
+            # library SDPA, as the reference (model.py:237): other types and head sizes
             if step.use_cache:
-                y = F.scaled_dot_product_attention(q, k_cache, v_cache, attn_mask=step.mask, dropout_p=0.0)
+                mask = step.mask
+                if mask is None:
+                    mask = (torch.arange(S, device=x.device)[None] <= step.seen[:, None])[None, None]
+                y = F.scaled_dot_product_attention(q, k_cache, v_cache, attn_mask=mask, dropout_p=0.0)
             else:
                 y = F.scaled_dot_product_attention(q, k_cache, v_cache, is_causal=True, dropout_p=0.0)
             y = y.transpose(1, 2).contiguous().view(B, T, C)
@@ -197,6 +206,20 @@ def _residual(x: torch.Tensor, h: torch.Tensor) -> torch.Tensor:
     return y
 
 
+def _residual_norm(x: torch.Tensor, h: torch.Tensor, norm: RMSNorm):
+    """``x + h`` and the norm of it, rounded as the two kernels round them."""
+    w = norm.scale
+    if not (is_plain(norm, RMSNorm) and x.dtype is torch.bfloat16 and h.dtype is x.dtype and w.dtype is x.dtype and x.is_cuda and x.shape == h.shape
+            and x.is_contiguous() and h.is_contiguous() and w.is_contiguous() and w.shape == x.shape[-1:] and norm.dim in (-1, x.dim() - 1)
+            and x.shape[-1] % 8 == 0 and x.shape[-1] <= 32768 and (x.data_ptr() | h.data_ptr() | w.data_ptr()) % 16 == 0
+            and not (torch.is_grad_enabled() and (x.requires_grad or h.requires_grad or w.requires_grad))):
+        x = _residual(x, h)
+        return x, norm(x)
+    s, y = torch.empty_like(x), torch.empty_like(x)
+    N.call("ll_add_rmsnorm", N.ptr(x), N.ptr(h), N.ptr(s), N.ptr(w), N.ptr(y), x.numel() // x.shape[-1], x.shape[-1], float(norm.eps), N.stream())
+    return s, y
+
+
 class Block(nn.Module):
     """ref: model.py:154-175"""
 
@@ -209,8 +232,8 @@ class Block(nn.Module):
 
     def forward(self, x: torch.Tensor, step: _Step, kv_cache: Optional[KVCache] = None):
         h, kv_cache = self.attn(self.rms_1(x), step, kv_cache)
-        x = _residual(x, h)
-        x = _residual(x, self.mlp(self.rms_2(x)))
+        x, h = _residual_norm(x, h, self.rms_2)
+        x = _residual(x, self.mlp(h))
         return x, kv_cache
 
 
@@ -337,8 +360,17 @@ class LLaMA(nn.Module):
         block_size = self.config.block_size
         use_cache = input_pos is not None
         dev = idx.device
-        pos3 = mask = None
-        if use_cache:
+        pos3 = mask = seen = None
+        kernel = (T > 1 or not use_cache) and self.transformer.wte.weight.dtype is torch.bfloat16 and N.has("ll_causal_attn") \
+            and bool(N.call_ret("ll_causal_attn_supported", self.config.head_size, T))
+        if use_cache and kernel:
+            N.require_cuda(input_pos)
+            if input_pos.shape != (T,):
+                raise RuntimeError(f"{T} tokens at positions of shape {tuple(input_pos.shape)}")
+            pos_ids, slots, seen = torch.empty((3, T), dtype=torch.int32, device=dev).unbind(0)
+            N.call("ll_prompt_pos", N.ptr(pos_ids), N.ptr(slots), N.ptr(seen), N.ptr(input_pos.to(torch.int64).contiguous()), T, max_seq_length, block_size,
+                   N.stream())
+        elif use_cache:
             pos_ids = input_pos.to(torch.int32)
             if T == 1:
                 pos3 = torch.empty(3, dtype=torch.int32, device=dev)
@@ -351,7 +383,8 @@ class LLaMA(nn.Module):
                 mask = self.mask_cache.index_select(2, input_pos)[:, :, :, :max_seq_length]
         else:
             pos_ids = slots = torch.arange(T, dtype=torch.int32, device=dev)
-        step = _Step(self._rope_f32, pos_ids.contiguous(), slots.contiguous(), pos3, mask, max_seq_length, use_cache)
+            seen = pos_ids if kernel else None
+        step = _Step(self._rope_f32, pos_ids.contiguous(), slots.contiguous(), pos3, mask, max_seq_length, use_cache, seen)
 
         x = self.transformer.wte(idx)
         if use_cache and not self.kv_caches:
@@ -383,8 +416,7 @@ class LLaMA(nn.Module):
             kv = self._kv_pool[key] = [(torch.zeros(shape, device=dev, dtype=dtype), torch.zeros(shape, device=dev, dtype=dtype))
                                        for _ in range(self.config.n_layer)]
         else:
-            for k, v in kv:
-                k.zero_(); v.zero_()
+            torch._foreach_zero_([t for pair in kv for t in pair])
         return list(kv)
 
     def _fused_engine(self, B: int, max_seq_length: int):
