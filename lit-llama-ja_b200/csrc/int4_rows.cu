@@ -7,8 +7,8 @@
 // activations are the B operand, tiles of bn rows x 128 k loaded by TMA.  A pair of CTAs forms one product of 256 weight columns (128 = the
 // TMEM lanes of each) x bn rows, and each CTA brings half of the rows: of a CTA of its own x takes 72 KB a step of 128 k at 256 rows from L2,
 // 46 bytes a clock and SM; the pair needs 40 KB.  Unpacking reads the bytes by transposing loads (64 single-byte loads a thread before) and
-// the scales from shared memory; the loop's registers may not spill or miss in what is left of L1 (that doubled a step's time; of the plain form
-// ptxas spills one register, stored and loaded once each).
+// the scales from shared memory; the loop's registers may not spill or miss in what is left of L1 (that doubled a step's time; of the gated form
+// ptxas spills three registers, stored and loaded once each).
 // us, one CTA a tile / pairs: 11008 x 4096 at 150, 512, 1100 rows 28 / 24, 51 / 46, 82 / 69; 4096 x 11008 at 150, 512 rows 53 / 48, 87 / 54;
 // 32000 x 4096 at 512 rows 140 / 103.  Bound by products at 256 rows a tile (0.84 us a step with all SMs busy, 0.76 at the rate of a large
 // dense product), below that by unpacking.
@@ -20,6 +20,8 @@
 //                long however many warps share it); then the epilogue, every fourth 16 rows per group
 // Gated form: a CTA's 128 columns are 64 of W1 and the same 64 of W2; the warps of the first hand their sums, rounded, to those of the
 // second through shared memory.  (13824 x 5120, 1100 rows: 241 us; two layers and their product 274 before.)
+// The tiles of a last wave that would leave pairs idle are cut along k (r4_plan); a second small kernel adds their parts, in fp32 and in the order of
+// k.  (A prompt of 512 tokens has 32 tiles of its 4096 x 11008 layer for 74 pairs, and 24 in the third wave of the gated one.)
 // Persistent: a pair walks tiles with a stride of the grid; a group drains a tile after its first step of the next one, and gives the
 // accumulator back as soon as it is in registers, so that the tensor cores wait for the drain alone.
 // Every wait is bounded; one that runs out records a code, all roles of both CTAs stop, copies in flight are waited for, tensor memory is
@@ -45,9 +47,36 @@ struct R4Params {
   const __nv_bfloat16* zeros[2];
   const __nv_bfloat16* bias[2];
   __nv_bfloat16* y;
-  int M, N, steps, G, steps_per_group, wide, bn, xst, mtiles, tiles;
+  float* part;                   // [(tiles - full) * parts][2 CTAs][bn][128]: sums of parts of tiles
+  int M, N, steps, G, steps_per_group, wide, bn, xst, mtiles, tiles, full, parts;      // the tiles from `full` on are cut along k into `parts`
   int* word;                     // wait_word()
 };
+
+// What a pair takes: of the tiles before p.full every `pairs`th, whole, then of the parts of the others every `pairs`th, two at most.
+struct R4Unit {
+  int tile, k0, len;             // `len` steps of a tile from step k0 on (none: 0)
+};
+struct R4Share {
+  int whole, part[2];            // how many whole tiles; which parts
+  R4Unit unit[2];
+};
+__device__ __forceinline__ R4Share r4_share(const R4Params& p, int pair, int pairs) {
+  R4Share q{p.full > pair ? (p.full - pair + pairs - 1) / pairs : 0, {pair, pair + pairs}, {{0, 0, 0}, {0, 0, 0}}};
+  for (int i = 0; i < 2; ++i) {
+    const int t = p.parts > 0 ? q.part[i] / p.parts : 0, c = q.part[i] - t * p.parts;
+    if (p.parts == 0 || p.full + t >= p.tiles) continue;
+    const int k0 = (int)((long long)p.steps * c / p.parts);
+    q.unit[i] = {p.full + t, k0, (int)((long long)p.steps * (c + 1) / p.parts) - k0};
+  }
+  return q;
+}
+// its nth unit
+__device__ __forceinline__ R4Unit r4_unit(const volatile R4Share* q, int steps, int pair, int pairs, int nth) {
+  const int o = nth - q->whole;
+  if (o < 0) return {pair + nth * pairs, 0, steps};
+  if (o > 1) return {0, 0, 0};
+  return {q->unit[o].tile, q->unit[o].k0, q->unit[o].len};
+}
 
 struct R4Fail {                  // the flag that stops all roles, here and in the other CTA
   volatile int* here;
@@ -110,6 +139,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
   uint64_t* g_empty = g_full + R4_GROUPS;              // and have been taken
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(g_empty + R4_GROUPS);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
+  R4Share* share = reinterpret_cast<R4Share*>(s_fail + 1);
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();
   if (threadIdx.x == 0) {
@@ -123,6 +153,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
     mbar_init(d_full, 1);
     mbar_init(d_empty, 2 * 4 * R4_GROUPS);
     *s_fail = 0;
+    *share = r4_share(p, blockIdx.x >> 1, gridDim.x >> 1);
     fence_barrier_init();
   }
   if (warp == 1) pair_tmem_alloc(tmem_ptr, 512);
@@ -142,10 +173,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
       bool ok = true;
       int s = 0;
       uint32_t ph = 1;
-      for (int tile = pair; ok && tile < p.tiles; tile += pairs) {
-        const int n0 = (tile / p.mtiles) * TILE_N, m0 = (tile % p.mtiles) * bn + rank * (bn >> 1);
+      for (int nth = 0; ok; ++nth) {
+        const R4Unit u = r4_unit(share, steps, pair, pairs, nth);
+        if (u.len == 0) break;
+        const int n0 = (u.tile / p.mtiles) * TILE_N, m0 = (u.tile % p.mtiles) * bn + rank * (bn >> 1);
         if (warp == 0) {
-          for (int kb = 0; kb < steps; ++kb) {
+          for (int kb = u.k0; kb < u.k0 + u.len; ++kb) {
             if (!(ok = r4_wait(&x_empty[s], ph, fail, 1))) break;
             if (rank == 0) mbar_expect_tx(&x_full[s], 2u * (uint32_t)xb);      // both CTAs' rows
             const uint32_t bar = cluster_addr(&x_full[s], 0);
@@ -155,7 +188,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
           }
         } else {
           const int c0 = n0 + rank * (TILE_N / 2);
-          for (int kb = 0; kb < steps; ++kb) {
+          for (int kb = u.k0; kb < u.k0 + u.len; ++kb) {
             if (!(ok = r4_wait(&w_empty[s], ph, fail, 2))) break;
             mbar_expect_tx(&w_full[s], R4_WBYTES);
             r4_box(sw + s * R4_WBYTES, &map_w0, c0, kb * (R4_K / 2), &w_full[s]);
@@ -173,9 +206,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
       bool ok = true;
       int s = 0, tl = 0;
       uint32_t ph = 0, blk = 0;
-      for (int tile = pair; rank == 0 && ok && tile < p.tiles; tile += pairs, ++tl) {
+      for (; rank == 0 && ok; ++tl) {
+        const int len = r4_unit(share, steps, pair, pairs, tl).len;
+        if (len == 0) break;
         if (tl > 0 && !(ok = r4_wait(d_empty, (uint32_t)(tl - 1) & 1u, fail, 3))) break;
-        for (int kb = 0; ok && kb < steps; ++kb, ++blk) {
+        for (int kb = 0; ok && kb < len; ++kb, ++blk) {
           const uint32_t buf = blk % R4_GROUPS;
           if (!(ok = r4_spin(&x_full[s], ph, fail, 5) && r4_spin(&a_ready[buf], (blk / R4_GROUPS) & 1u, fail, 4))) break;
           tc_fence_after();
@@ -209,15 +244,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
       }
     };
     uint2 sv[4], zv[4];
-    fetch(pair, 0, sv, zv);
-    for (int tile = pair; ok && tile < p.tiles; tile += pairs) {
-      for (int kb = 0; ok && kb < steps; kb += 4) {
+    R4Unit u = r4_unit(share, steps, pair, pairs, 0);
+    if (u.len > 0) fetch(u.tile, u.k0 & ~3, sv, zv);
+    for (int nth = 1; ok && u.len > 0; ++nth) {
+      const R4Unit next = r4_unit(share, steps, pair, pairs, nth);
+      const int end = u.k0 + u.len;
+      for (int kb = u.k0 & ~3; ok && kb < end; kb += 4) {
         uint2 sn[4], zn[4];
-        const bool last = kb + 4 >= steps;
-        if (!last || tile + pairs < p.tiles) fetch(last ? tile + pairs : tile, last ? 0 : kb + 4, sn, zn);
+        const bool last = kb + 4 >= end;
+        if (!last || next.len > 0) fetch(last ? next.tile : u.tile, last ? next.k0 & ~3 : kb + 4, sn, zn);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          if (kb + j >= steps) break;
+          if (kb + j < u.k0 || kb + j >= end) continue;
           ok = __all_sync(0xffffffffu, r4_wait(&w_empty[s], ph, fail, 11));
           if (!ok) break;
 #pragma unroll
@@ -229,6 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
 #pragma unroll
         for (int q = 0; q < 4; ++q) sv[q] = sn[q], zv[q] = zn[q];
       }
+      u = next;
     }
   } else {
     const int quarter = warp & 3, grp = (warp - 4) >> 2, half = quarter >> 1;        // half: the CTA's first or last 64 columns
@@ -238,14 +277,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
     const uint32_t a_ready0 = cluster_addr(&a_ready[grp], 0), d_empty0 = cluster_addr(d_empty, 0);
     bool ok = true;
     uint32_t boxes = 0, swaps = 0;
-    // a finished tile: its sums leave tensor memory, then the accumulator is given back, then they are stored
-    auto drain = [&](int tile, uint32_t nth) {
+    // a finished unit: its sums leave tensor memory, then the accumulator is given back, then they are stored
+    auto drain = [&](uint32_t nth) {
+      const R4Unit u = r4_unit(share, steps, pair, pairs, (int)nth);
       ok = __all_sync(0xffffffffu, r4_wait(d_full, nth & 1u, fail, 6));
       if (!ok) return;
       tc_fence_after();
-      const int n = (tile / p.mtiles) * TILE_N + col, m0 = (tile % p.mtiles) * bn;
+      const int n = (u.tile / p.mtiles) * TILE_N + col, m0 = (u.tile % p.mtiles) * bn;
       const __nv_bfloat16* b = second ? p.bias[1] : p.bias[0];
       const float bias = b != nullptr && n < p.N ? __bfloat162float(b[n]) : 0.f;
+      if (u.tile >= p.full) {                // a part of a tile: its sums go to L2 as they are
+        float* const dst = p.part + ((size_t)share->part[(int)nth - share->whole] * 2 + rank) * (size_t)(bn * 128) + quarter * 32 + lane;
+#pragma unroll 1
+        for (int r = grp * 16; r < bn; r += 16 * R4_GROUPS) {
+          uint32_t v[16];
+          r4_ld16(tmem + lanes + (uint32_t)r, v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < 16; ++e) asm volatile("" : "+r"(v[e]));
+#pragma unroll
+          for (int e = 0; e < 16; ++e) __stcg(dst + (r + e) * 128, __uint_as_float(v[e]));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(d_empty0);
+        return;
+      }
       uint32_t w[4][8];
 #pragma unroll
       for (int c = 0; c < 4; c += 2) {       // (bn is a multiple of 32 above 64: pairs of chunks, and only the last chunk of a group can be missing)
@@ -322,21 +379,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
         }
       }
     };
-    // the group's steps: every fourth of all steps of all of the pair's tiles
-    int tile = pair, kb = grp, drained = pair, s = grp;
-    uint32_t nth = 0, round = 0, wph = 0;    // round: the group's how-many-th step
-    while (kb >= steps && tile < p.tiles) kb -= steps, tile += pairs;
+    // the group's steps: every fourth of all steps of all of the pair's units
+    int len = r4_unit(share, steps, pair, pairs, 0).len, kb = grp, s = grp;
+    uint32_t unit = 0, drained = 0, round = 0, wph = 0;    // unit: of the group's next step; round: its how-many-th step
+    while (len > 0 && kb >= len) kb -= len, len = r4_unit(share, steps, pair, pairs, (int)++unit).len;
     constexpr int WIDTH = GATED ? 64 : 128;
     const R4Row<WIDTH> row(lane);
-    while (ok && drained < p.tiles) {
-      const int upto = min(tile, p.tiles);   // tiles before this one can be drained
-      bool step = tile < p.tiles;
+    while (ok && (len > 0 || drained < unit)) {
+      bool step = len > 0;
+      const uint32_t upto = unit;            // units before this one can be drained
       if (step) {
         ok = r4_wait(&w_full[s], wph, fail, 7);
         if (ok && round > 0) ok = r4_wait(&a_free[grp], (round - 1u) & 1u, fail, 8);
         if (!(ok = __all_sync(0xffffffffu, ok))) break;
-        // a tile that is done already (for the group whose step was its last) is drained before the step, others after it
-        step = drained >= upto || !__any_sync(0xffffffffu, mbar_test_wait(d_full, nth & 1u));
+        // a unit that is done already (for the group whose step was its last) is drained before the step, others after it
+        step = drained >= upto || !__any_sync(0xffffffffu, mbar_test_wait(d_full, drained & 1u));
       }
       if (step) {
         tc_fence_after();
@@ -347,14 +404,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(R4_THREADS, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&w_empty[s]), mbar_arrive_cluster(a_ready0);
         kb += R4_GROUPS;
-        while (kb >= steps && tile < p.tiles) kb -= steps, tile += pairs;
+        while (len > 0 && kb >= len) kb -= len, len = r4_unit(share, steps, pair, pairs, (int)++unit).len;
         ++round;
         if ((s += R4_GROUPS) >= R4_WST) s -= R4_WST, wph ^= 1u;
       }
-      while (ok && drained < upto) {
-        drain(drained, nth++);
-        drained += pairs;
-      }
+      while (ok && drained < upto) drain(drained++);
     }
     tc_fence_before();
     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -386,24 +440,107 @@ int r4_out_map(const void* y, int M, int N, CUtensorMap* out) {
 }
 
 // Clocks of a launch with tiles of bn rows: waves of the persistent grid, 128 k at a time, plus the drain.  A step costs its products, or, with
-// few rows, its unpacking (us a step of 13824 x 5120, 900 rows, tiles of 128 / 160 / 192 / 224 / 256 rows: .54 / .56 / .61 / .66 / .78, the last with six pairs idle in its third wave).
+// few rows, its unpacking (us a step of 13824 x 5120, 900 rows, tiles of 128 / 160 / 192 / 224 / 256 rows: .54 / .56 / .61 / .66 / .78, the last with
+// six pairs idle in its third wave).
+int r4_step(int bn) { return 4 * bn > 530 + 7 * bn / 5 ? 4 * bn : 530 + 7 * bn / 5; }
 long long r4_cost(int M, int N, int tile_n, int steps, int bn, int pairs) {
   const long long tiles = (long long)((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n);
-  const int products = 4 * bn, unpack = 530 + 7 * bn / 5;
-  return (tiles + pairs - 1) / pairs * ((long long)steps * (products > unpack ? products : unpack) + 1500);
+  return (tiles + pairs - 1) / pairs * ((long long)steps * r4_step(bn) + 1500);
+}
+// The same of `tiles` tiles cut into `parts` along k each: their steps, the launch that adds the parts up (5 us) and their way through L2 (6 MB a us).
+// us on the device, every tile whole / by this rule: 4096 x 11008 at 130, 300, 512 rows 48 / 24, 50 / 34, 50 / 43, from 700 on all whole (53; in the
+// parts nearest to paying 58); 2048 x 5632 at 130, 512, 700 rows 27 / 15, 27 / 21, 29 / 24; 4096 x 4096 at 130, 300 rows 22 / 16, 23 / 20, 512 whole
+// (24; 26); the gated 11008 x 4096 at 130, 300, 512, 700 rows 45 / 37, 63 / 56, 80 / 74, 109 / 106.  Ranges of one length for all pairs, that cross
+// tile ends, were 2 to 4 us slower (two drains a pair, more parts); the last pair to arrive adding up in the kernel itself made the loop spill (whole
+// tiles a fifth slower).
+constexpr int R4_PARTS = 8;
+long long r4_parts_cost(int steps, int bn, int tiles, int parts, int pairs) {
+  return (long long)((tiles * parts + pairs - 1) / pairs) * ((long long)((steps + parts - 1) / parts) * r4_step(bn) + 1500) + 7000 + tiles * parts * bn / 4;
+}
+
+// How the work is laid out: whole tiles in whole waves; those of a last wave that would leave pairs idle are cut along k, if that pays.
+struct R4Plan {
+  int bn, full, parts;           // (parts 0: every tile whole)
+};
+R4Plan r4_plan(int M, int N, int steps, int tile_n, int pairs, int tile_rows, int parts, bool scratch) {
+  R4Plan best{};
+  long long least = 0;
+  for (int bn = tile_rows ? tile_rows : 256; bn >= (tile_rows ? tile_rows : 128); bn -= 32) {
+    const int tiles = ((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n), full = tiles / pairs * pairs, rest = tiles - full;
+    const long long whole = r4_cost(M, N, tile_n, steps, bn, pairs);
+    if (best.bn == 0 || whole < least) best = {bn, tiles, 0}, least = whole;
+    if (!scratch || rest == 0) continue;
+    const long long before = r4_cost(full / pairs * bn, tile_n, tile_n, steps, bn, 1);
+    for (int s = parts > 0 ? parts : 2; s <= (parts > 0 ? parts : R4_PARTS) && s <= steps && rest * s <= 2 * pairs; ++s) {
+      const long long cost = before + r4_parts_cost(steps, bn, rest, s, pairs);
+      if (parts > 0 || cost < least) best = {bn, full, s}, least = cost;
+    }
+  }
+  return best;
+}
+int r4_pairs(int grid) {
+  const int sms = grid > 0 ? grid : sm_count() > 0 ? sm_count() : 148;
+  return sms > 1 ? (grid > 0 ? (sms + 1) / 2 : sms / 2) : 1;
+}
+int r4_tiles(int M, int N, int tile_n, int bn) { return ((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n); }
+size_t r4_scratch_bytes(const R4Plan& q, int tiles) {
+  return (size_t)(tiles - q.full) * q.parts * 2 * q.bn * 128 * sizeof(float);
+}
+
+bool r4_form_ok(int tile_rows, int grid) { return (tile_rows == 0 || (tile_rows % 32 == 0 && tile_rows >= 128 && tile_rows <= 256)) && grid >= 0; }
+
+// The tiles that were cut: their parts in the order of k, then what the epilogue of a whole tile does.  A block: four rows of a tile; a thread: four
+// columns (of both layers) of a row.
+template <bool GATED>
+__global__ void __launch_bounds__(GATED ? 128 : 256) int4_rows_sum_kernel(const float* part, const __nv_bfloat16* __restrict__ b0,
+                                                                          const __nv_bfloat16* __restrict__ b1, __nv_bfloat16* y, int M, int N, int bn,
+                                                                          int mtiles, int full, int parts) {
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int OUT = GATED ? 64 : 128, L = GATED ? 2 : 1;              // outputs of a CTA of the pair, layers
+  const int t = blockIdx.x, tile = full + t, col = (threadIdx.x & (OUT / 4 - 1)) * 4, rank = (threadIdx.x / (OUT / 4)) & 1;
+  const int n = tile / mtiles * (2 * OUT) + rank * OUT + col, r = blockIdx.y * 4 + threadIdx.x / (OUT / 2), m = tile % mtiles * bn + r;
+  if (n >= N || m >= M) return;
+  const size_t size = (size_t)bn * 256;
+  const float* src = part + (size_t)t * parts * size + ((size_t)rank * bn + r) * 128 + col;
+  float4 s[L];
+#pragma unroll
+  for (int h = 0; h < L; ++h) s[h] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int c = 0; c < parts; c += 4) {
+    float4 v[L][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < L; ++h) v[h][i] = __ldcg(reinterpret_cast<const float4*>(src + (size_t)min(c + i, parts - 1) * size + h * 64));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < L; ++h)
+        if (c + i < parts) s[h].x += v[h][i].x, s[h].y += v[h][i].y, s[h].z += v[h][i].z, s[h].w += v[h][i].w;
+  }
+  uint32_t w[L][2];
+#pragma unroll
+  for (int h = 0; h < L; ++h) {
+    const __nv_bfloat16* b = h ? b1 : b0;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (b != nullptr) a = make_float4(__bfloat162float(b[n]), __bfloat162float(b[n + 1]), __bfloat162float(b[n + 2]), __bfloat162float(b[n + 3]));
+    w[h][0] = pack_bf16(s[h].x + a.x, s[h].y + a.y), w[h][1] = pack_bf16(s[h].z + a.z, s[h].w + a.w);
+  }
+  if (GATED) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      w[0][e] = r4_mul2(pack_bf16(silu_fast(__uint_as_float(w[0][e] << 16)), silu_fast(__uint_as_float(w[0][e] & 0xffff0000u))), w[L - 1][e]);
+  }
+  *reinterpret_cast<uint2*>(y + (size_t)m * N + n) = make_uint2(w[0][0], w[0][1]);
 }
 
 template <bool GATED>
-int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p, int K, int tile_rows, int grid, cudaStream_t st) {
+int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p, int K, void* scratch, int tile_rows, int grid, int parts, cudaStream_t st) {
   constexpr int TILE_N = GATED ? 128 : 256;
-  const int sms = grid > 0 ? grid : sm_count();
-  const int pairs = sms > 1 ? (grid > 0 ? (sms + 1) / 2 : sms / 2) : 1;
-  p.bn = tile_rows;
-  if (tile_rows == 0) {
-    p.bn = 256;
-    for (int bn = 224; bn >= 128; bn -= 32)
-      if (r4_cost(p.M, p.N, TILE_N, p.steps, bn, pairs) < r4_cost(p.M, p.N, TILE_N, p.steps, p.bn, pairs)) p.bn = bn;
-  }
+  const int pairs = r4_pairs(grid);
+  LL_CHECK_ARG((long long)((p.M + 127) / 128) * ((p.N + TILE_N - 1) / TILE_N) < (1ll << 30), "int4_rows: too many tiles");
+  const R4Plan q = r4_plan(p.M, p.N, p.steps, TILE_N, pairs, tile_rows, parts, scratch != nullptr);
+  p.bn = q.bn, p.full = q.full, p.parts = q.parts;
   p.xst = R4_XBYTES / (p.bn * 128);
   p.wide = r4_wide(p.scales[0], p.zeros[0], p.scales[1], p.zeros[1], p.G, p.steps_per_group);
   CUtensorMap mw0, mw1, mx, my;
@@ -417,12 +554,18 @@ int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p,
     configured.mark();
   }
   p.mtiles = (p.M + p.bn - 1) / p.bn;
-  const long long tiles = (long long)p.mtiles * ((p.N + TILE_N - 1) / TILE_N);
-  LL_CHECK_ARG(tiles < (1ll << 30), "int4_rows: too many tiles");
-  p.tiles = (int)tiles;
+  p.tiles = r4_tiles(p.M, p.N, TILE_N, p.bn);
   p.word = wait_word();
-  LL_CUDA(launch(int4_rows_kernel<GATED>, dim3(2 * (p.tiles < pairs ? p.tiles : pairs)), dim3(R4_THREADS), R4_SMEM, st, true, mw0, mw1, mx, my, p));
+  int blocks = p.tiles < pairs ? p.tiles : pairs;
+  const int cut = p.tiles - q.full;
+  if (cut > 0) p.part = (float*)scratch, blocks = q.full > 0 || cut * q.parts > pairs ? pairs : cut * q.parts;
+  LL_CUDA(launch(int4_rows_kernel<GATED>, dim3(2 * blocks), dim3(R4_THREADS), R4_SMEM, st, true, mw0, mw1, mx, my, p));
   LL_LAUNCH_OK("int4_rows_kernel");
+  if (cut > 0) {
+    LL_CUDA(launch(int4_rows_sum_kernel<GATED>, dim3(cut, p.bn / 4), dim3(GATED ? 128 : 256), 0, st, true, (const float*)p.part, p.bias[0], p.bias[1], p.y,
+                   p.M, p.N, p.bn, p.mtiles, p.full, p.parts));
+    LL_LAUNCH_OK("int4_rows_sum_kernel");
+  }
   return LL_OK;
 }
 
@@ -442,39 +585,57 @@ int ll_int4_rows(const uint8_t* qw, const void* scales, const void* zeros, const
 
 int ll_int4_rows_form(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, int M, int N, int K,
                       int group, int tile_rows, int grid, ll_stream stream) {
+  return ll_int4_rows_split(qw, scales, zeros, x, bias, y, nullptr, M, N, K, group, tile_rows, grid, 0, stream);
+}
+
+size_t ll_int4_rows_scratch_bytes(int M, int N, int K, int layers, int tile_rows, int grid, int parts) {
+  if (M < 1 || N < 1 || K < R4_K || layers < 1 || layers > 2 || grid < 0 || parts < 0 || !r4_form_ok(tile_rows, grid)) return 0;
+  const int tile_n = layers == 2 ? 128 : 256;
+  if ((long long)((M + 127) / 128) * ((N + tile_n - 1) / tile_n) >= (1ll << 30)) return 0;
+  const R4Plan q = r4_plan(M, N, K / R4_K, tile_n, r4_pairs(grid), tile_rows, parts, true);
+  return r4_scratch_bytes(q, r4_tiles(M, N, tile_n, q.bn));
+}
+
+int ll_int4_rows_split(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch, int M, int N,
+                       int K, int group, int tile_rows, int grid, int parts, ll_stream stream) {
   LL_CHECK_ARG(qw && scales && zeros && x && y && M > 0, "int4_rows: null pointer or no rows");
   if (!ll_int4_rows_supported(N, K, group)) {
     set_error("int4_rows needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
     return LL_ERR_UNSUPPORTED;
   }
-  LL_CHECK_ARG((((uintptr_t)qw | (uintptr_t)x | (uintptr_t)y) & 15) == 0, "int4_rows: packed weights, x and y must be 16-byte aligned");
-  LL_CHECK_ARG((tile_rows == 0 || (tile_rows % 32 == 0 && tile_rows >= 128 && tile_rows <= 256)) && grid >= 0,
-               "int4_rows: tiles of 128 to 256 rows, a multiple of 32");
+  LL_CHECK_ARG((((uintptr_t)qw | (uintptr_t)x | (uintptr_t)y | (uintptr_t)scratch) & 15) == 0,
+               "int4_rows: packed weights, x, y and scratch must be 16-byte aligned");
+  LL_CHECK_ARG(r4_form_ok(tile_rows, grid) && parts >= 0, "int4_rows: tiles of 128 to 256 rows, a multiple of 32");
   R4Params p{};
   p.scales[0] = p.scales[1] = (const __nv_bfloat16*)scales, p.zeros[0] = p.zeros[1] = (const __nv_bfloat16*)zeros;
   p.bias[0] = p.bias[1] = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
-  return r4_launch<false>(qw, qw, x, p, K, tile_rows, grid, (cudaStream_t)stream);
+  return r4_launch<false>(qw, qw, x, p, K, scratch, tile_rows, grid, parts, (cudaStream_t)stream);
 }
 
 int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
                        const void* zeros2, const void* bias2, const void* x, void* h, int M, int N, int K, int group, int tile_rows, int grid,
                        ll_stream stream) {
+  return ll_int4_rows_gated_split(qw1, scales1, zeros1, bias1, qw2, scales2, zeros2, bias2, x, h, nullptr, M, N, K, group, tile_rows, grid, 0, stream);
+}
+
+int ll_int4_rows_gated_split(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
+                             const void* zeros2, const void* bias2, const void* x, void* h, void* scratch, int M, int N, int K, int group,
+                             int tile_rows, int grid, int parts, ll_stream stream) {
   LL_CHECK_ARG(qw1 && scales1 && zeros1 && qw2 && scales2 && zeros2 && x && h && M > 0, "int4_rows_gated: null pointer or no rows");
   if (!ll_int4_rows_supported(N, K, group)) {
     set_error("int4_rows_gated needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
     return LL_ERR_UNSUPPORTED;
   }
-  LL_CHECK_ARG((((uintptr_t)qw1 | (uintptr_t)qw2 | (uintptr_t)x | (uintptr_t)h) & 15) == 0,
-               "int4_rows_gated: packed weights, x and h must be 16-byte aligned");
-  LL_CHECK_ARG((tile_rows == 0 || (tile_rows % 32 == 0 && tile_rows >= 128 && tile_rows <= 256)) && grid >= 0,
-               "int4_rows_gated: tiles of 128 to 256 rows, a multiple of 32");
+  LL_CHECK_ARG((((uintptr_t)qw1 | (uintptr_t)qw2 | (uintptr_t)x | (uintptr_t)h | (uintptr_t)scratch) & 15) == 0,
+               "int4_rows_gated: packed weights, x, h and scratch must be 16-byte aligned");
+  LL_CHECK_ARG(r4_form_ok(tile_rows, grid) && parts >= 0, "int4_rows_gated: tiles of 128 to 256 rows, a multiple of 32");
   R4Params p{};
   p.scales[0] = (const __nv_bfloat16*)scales1, p.zeros[0] = (const __nv_bfloat16*)zeros1, p.bias[0] = (const __nv_bfloat16*)bias1;
   p.scales[1] = (const __nv_bfloat16*)scales2, p.zeros[1] = (const __nv_bfloat16*)zeros2, p.bias[1] = (const __nv_bfloat16*)bias2;
   p.y = (__nv_bfloat16*)h;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
-  return r4_launch<true>(qw1, qw2, x, p, K, tile_rows, grid, (cudaStream_t)stream);
+  return r4_launch<true>(qw1, qw2, x, p, K, scratch, tile_rows, grid, parts, (cudaStream_t)stream);
 }
 
 // 0, or the code of the first bounded wait that ran out in this file's kernel.  Synchronises the device.

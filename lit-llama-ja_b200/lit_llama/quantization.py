@@ -34,6 +34,11 @@ def _batch_scratch_bytes(M: int, Nout: int, K: int, layers: int) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
+def _rows_scratch_bytes(M: int, Nout: int, K: int, layers: int) -> int:
+    return N.call_ret("ll_int4_rows_scratch_bytes", M, Nout, K, layers, 0, 0, 0)
+
+
+@functools.lru_cache(maxsize=4096)
 def _gemv_supported(bits: int, Nout: int, K: int, group: int, nmat: int, M: int) -> bool:
     if bits == 8:
         return bool(N.call_ret("ll_q8_gemv_supported", Nout, K, group, nmat, M))
@@ -251,8 +256,14 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         elif M <= self.FUSED_GEMM_MAX_M and self._fused_gemm_eligible(x) and self._fused_gemm(x, y):
             pass
         elif self.ROWS_MIN_M <= M <= self.ROWS_MAX_M and self._rows_eligible(x):
-            N.call("ll_int4_rows", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), M, Nout, K,
-                   self.tile_cols, N.stream())
+            nbytes = _rows_scratch_bytes(M, Nout, K, 1)
+            if nbytes:                         # (a last wave of tiles that pays to be cut along k)
+                scratch = _int8_workspace(x.device, nbytes)
+                N.call("ll_int4_rows_split", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y),
+                       N.ptr(scratch), M, Nout, K, self.tile_cols, 0, 0, 0, N.stream())
+            else:
+                N.call("ll_int4_rows", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), M, Nout, K,
+                       self.tile_cols, N.stream())
         elif M <= 16:
             assert inp.dtype in (torch.float32, torch.bfloat16)
             N.call("ll_qlinear_simt", N.ptr(x), N.dtype_code(x.dtype), M, N.ptr(qw), N.ptr(self.scales.contiguous()),
@@ -350,8 +361,10 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
     if rows:
         q1, q2 = fc1._packed_ptr_ok(), fc2._packed_ptr_ok()
         N.require_cuda(q1, q2)
-        N.call("ll_int4_rows_gated", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
-               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), M, Nout, K, fc1.tile_cols, 0, 0, N.stream())
+        nbytes = _rows_scratch_bytes(M, Nout, K, 2)
+        scratch = _int8_workspace(x.device, nbytes) if nbytes else None
+        N.call("ll_int4_rows_gated_split", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
+               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), N.ptr(scratch), M, Nout, K, fc1.tile_cols, 0, 0, 0, N.stream())
     else:
         w1, w2 = fc1.get_weight(dtype=x.dtype), fc2.get_weight(dtype=x.dtype)
         N.call("ll_gemm_bf16_gated", N.ptr(x), N.ptr(w1), N.ptr(fc1.bias), N.ptr(w2), N.ptr(fc2.bias), N.ptr(h), M, Nout, K, N.stream())
