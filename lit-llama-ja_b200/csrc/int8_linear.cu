@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(256, 4) int8_finish_rows_kernel(const int32_t*
   constexpr int ROWS = 16, SL = 4, L = 64, NW = L * 16 / 256, NA = L * ROWS / 256, AS = 256 / ROWS;   // SL: shares of the list
   __shared__ __align__(16) float w_s[L][64], a_s[L][ROWS];
   const int tid = threadIdx.x, n0 = blockIdx.x * 64, m0 = blockIdx.y * ROWS, blk = m0 / 64, col = (tid & 15) * 4;
+  pdl_launch_dependents();
   const int cnt = count[blk];
   float first[4];                                          // GATED: the first layer's outputs
 #pragma unroll 1
@@ -305,12 +306,13 @@ constexpr int I8P_THREADS = 512, I8P_HELD = 4;
 template <typename T>
 __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restrict__ x, int8_t* __restrict__ ca, float* __restrict__ sca,
                                                                uint8_t* __restrict__ flag, int32_t* __restrict__ idx, int32_t* __restrict__ count,
-                                                               int32_t* __restrict__ arrive, int K, float thr, int vec) {
+                                                               int32_t* __restrict__ arrive, int K, float thr, int vec, int early) {
   constexpr int WARPS = I8P_THREADS / 32, STEP = I8P_THREADS * 8;
   __shared__ float s_max[WARPS];
   __shared__ int s_warp[WARPS], s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, blk = blockIdx.x / 64, m0 = blk * 64, M = min(64, (int)gridDim.x - m0);
   flag += (size_t)blk * K, idx += (size_t)blk * K;
+  if (early) pdl_launch_dependents();
   const T* row = x + (size_t)blockIdx.x * K;
   float held[I8P_HELD][8], mx = 0.f;
 #pragma unroll
@@ -362,8 +364,8 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
   __syncthreads();
   if (tid == 0) s_last = atomicAdd(arrive + blk, 1) == M - 1;
   __syncthreads();
-  // The next kernel's CTAs come while the lists are made.  (Let in from the start on they pile up on the SMs that have no row: 130 rows with long
-  // lists 2300 us instead of 1280.)
+  // Of prompts the next kernel's CTAs come while the lists are made.  (Let in from the start on they pile up on the SMs that have no row: 130 rows
+  // with long lists 2300 us instead of 1280.)
   pdl_launch_dependents();
   if (!s_last) return;
   __threadfence();
@@ -411,6 +413,114 @@ __global__ void __launch_bounds__(I8P_THREADS) int8_prep_kernel(const T* __restr
   }
 }
 
+// The same for few rows in one cluster of eight CTAs, every eighth row a CTA: the columns that stand out are bits in shared memory, each CTA marks
+// those of its rows, and past one cluster barrier ORs all eight CTAs' (CTAs of a cluster run at the same time).  Codes are written once, nothing has
+// to be cleared before, and the kernel starts under the one before it.  Bound by the arithmetic of eight SMs, 2 us a row of 11008.  us a layer of
+// 11008 x 4096 and of 4096 x 11008, clearing and a CTA per row / here: 1 row 17 / 12 and 18 / 14, 8 rows 17 / 13 and 18 / 15; 24 rows of 4096 features
+// 17 / 15.  Against a CTA per row with the weights ahead of it, without and with 30 outliers, 32 rows of 4096 features 14.9 / 15.8 and 21.1 / 19.5,
+// 48 rows 16.9 / 18.7 and 23.5 / 23.8, 16 rows of 11008 16.3 / 16.8 and 19.6 / 19.1.
+constexpr int I8F_THREADS = 1024, I8F_CTAS = 8, I8F_MOST = 16384;          // features a CTA takes
+__device__ __forceinline__ uint32_t int8_peer_word(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+template <typename T>
+__global__ void __cluster_dims__(I8F_CTAS, 1, 1) __launch_bounds__(I8F_THREADS, 1)
+    int8_prep_few_kernel(const T* x, int8_t* __restrict__ ca, float* __restrict__ sca, int32_t* __restrict__ idx, int32_t* __restrict__ count,
+                         int M, int K, float thr, int vec) {
+  constexpr int WARPS = I8F_THREADS / 32;
+  extern __shared__ __align__(16) uint32_t i8p_smem[];
+  __shared__ float s_max[WARPS];
+  __shared__ int s_warp[WARPS];
+  const int words = K / 32;
+  uint32_t *own = i8p_smem, *all = own + words;        // a bit per column: of this CTA's rows, of the block's
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)cluster_rank();
+  const int held = (M + I8F_CTAS - 1) / I8F_CTAS;        // rows of a CTA at most
+  const int per = held <= 1 ? 32 : held <= 2 ? 16 : held <= 4 ? 8 : 4, m = rank + warp / per * I8F_CTAS, step = per * 256;   // warps of a row
+  const int k0 = (tid - warp / per * per * 32) * 8;
+  const bool mine = m < M;
+  const size_t at = (size_t)m * K;
+  for (int i = tid; i < words; i += I8F_THREADS) own[i] = 0u;
+  __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
+  const T* row = after_wait(x) + at;
+  float mx = 0.f;
+  if (mine) {
+#pragma unroll 4
+    for (int k = k0; k < K; k += step) {                 // (K is a multiple of 128)
+      float v[8];
+      int8_load8<T>(row + k, v, vec);
+      uint32_t bits = 0u;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float a = fabsf(v[e]);
+        if (a >= thr) bits |= 1u << e;
+        else mx = fmaxf(mx, a);
+      }
+      if (bits) atomicOr(&own[k >> 5], bits << (k & 31));
+    }
+  }
+  mx = warp_max(mx);
+  if (lane == 0) s_max[warp] = mx;
+  cluster_sync();                                        // (of this CTA's threads too)
+  for (int i = tid; i < words; i += I8F_THREADS) {
+    uint32_t w = 0u;
+#pragma unroll
+    for (int r = 0; r < I8F_CTAS; ++r) w |= int8_peer_word(cluster_addr(own + i, (uint32_t)r));
+    all[i] = w;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // waited for at the end: no CTA leaves while its bits are read
+  __syncthreads();
+  if (mine) {
+    mx = s_max[warp / per * per];
+    for (int w = 1; w < per; ++w) mx = fmaxf(mx, s_max[warp / per * per + w]);
+    if (k0 == 0) sca[m] = mx;
+    const float inv = __fdiv_rn(127.f, mx == 0.f ? 1.f : mx);
+#pragma unroll 4
+    for (int k = k0; k < K; k += step) {
+      float v[8];
+      int8_load8<T>(row + k, v, vec);
+      const uint32_t bits = all[k >> 5] >> (k & 31);
+      uint32_t o[2] = {0u, 0u};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float q = 0.f;
+        if (fabsf(v[e]) < thr && !((bits >> e) & 1u)) q = fminf(fmaxf(rintf(__fmul_rn(v[e], inv)), -127.f), 127.f);
+        o[e >> 2] |= ((uint32_t)(int)q & 0xffu) << (8 * (e & 3));
+      }
+      *reinterpret_cast<uint2*>(ca + at + k) = make_uint2(o[0], o[1]);
+    }
+  }
+  if (rank == I8F_CTAS - 1) {                            // (the CTA with the fewest rows)
+    int base = 0;
+    for (int i0 = 0; i0 < words; i0 += I8F_THREADS) {
+      const uint32_t w = i0 + tid < words ? all[i0 + tid] : 0u;
+      const int n = __popc(w);
+      int incl = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += u;
+      }
+      if (lane == 31) s_warp[warp] = incl;
+      __syncthreads();
+      int to = base + incl - n, total = 0;
+      for (int u = 0; u < WARPS; ++u) {
+        const int c = s_warp[u];
+        if (u < warp) to += c;
+        total += c;
+      }
+      for (uint32_t left = w; left; left &= left - 1u) idx[to++] = (i0 + tid) * 32 + __ffs((int)left) - 1;
+      base += total;
+      __syncthreads();
+    }
+    if (tid == 0) *count = base;
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ================================================================================================== up to 64 rows
 // part[range][m][n] = the sum over the range's k of CA[m][k] CB[n][k]: the weights are the A operand (128 output columns a CTA), streamed
 // through a ring of 16 KB boxes; two CTAs share an SM.  MP: rows rounded up to 16, 32, 48 or 64.
@@ -453,10 +563,20 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
       bool ok = true;
       int s = 0;
       uint32_t ph = 1;
+      // the weights of the first stages come while the rows are prepared (the preparation waits for all before it and only then lets this kernel in:
+      // whoever made the weights is done).  us a layer of 4096 x 11008 that a CTA per row prepares, 32 and 64 rows: 19 / 17, 21 / 19.
+      const int ahead = min(STAGES, kb1 - kb0);
+      for (int i = 0; i < ahead; ++i) {
+        mbar_expect_tx(&full[i], I8_BOX + XB);
+        i8_box(sw + i * I8_BOX, map_w, (kb0 + i) * 128, n0, &full[i]);
+      }
+      pdl_wait();
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!(ok = i8_wait(&empty[s], ph, s_fail, word, 5))) break;
-        mbar_expect_tx(&full[s], I8_BOX + XB);
-        i8_box(sw + s * I8_BOX, map_w, kb * 128, n0, &full[s]);
+        if (kb - kb0 >= ahead) {
+          if (!(ok = i8_wait(&empty[s], ph, s_fail, word, 5))) break;
+          mbar_expect_tx(&full[s], I8_BOX + XB);
+          i8_box(sw + s * I8_BOX, map_w, kb * 128, n0, &full[s]);
+        }
         i8_box(sx + s * XB, &map_x, kb * 128, 0, &full[s]);
         if (++s == STAGES) s = 0, ph ^= 1u;
       }
@@ -483,6 +603,7 @@ __global__ void __launch_bounds__(192, 2) int8_columns_tc_kernel(const __grid_co
     }
   } else {
     const int quarter = warp & 3, n = n0 + quarter * 32 + lane;
+    pdl_wait();                      // (the partial sums' place may be the kernel's before)
     const bool ok = __all_sync(0xffffffffu, i8_wait(done, 0, s_fail, word, 7) && *(volatile int*)s_fail == 0);
     tc_fence_after();
     if (ok) {
@@ -546,8 +667,14 @@ Ws carve(void* base, int M, int N, int K, int layers, bool partial) {
 
 template <typename T>
 int int8_prepare(const T* x, const Ws& w, void* base, int M, int K, float thr, cudaStream_t st) {
+  const int vec = ((uintptr_t)x & 15) == 0 ? 1 : 0;
+  if (M <= 64 && (long long)((M + I8F_CTAS - 1) / I8F_CTAS) * K <= I8F_MOST) {
+    LL_CUDA(launch(int8_prep_few_kernel<T>, dim3(I8F_CTAS), dim3(I8F_THREADS), K / 32 * 8, st, true, x, w.ca, w.sca, w.idx, w.count, M, K, thr, vec));
+    LL_LAUNCH_OK("int8_prep_few_kernel");
+    return LL_OK;
+  }
   LL_CUDA(cudaMemsetAsync((uint8_t*)base + w.zero_off, 0, w.zero_bytes, st));
-  int8_prep_kernel<T><<<M, I8P_THREADS, 0, st>>>(x, w.ca, w.sca, w.flag, w.idx, w.count, w.arrive, K, thr, ((uintptr_t)x & 15) == 0);
+  int8_prep_kernel<T><<<M, I8P_THREADS, 0, st>>>(x, w.ca, w.sca, w.flag, w.idx, w.count, w.arrive, K, thr, vec, M <= 64 ? 1 : 0);
   LL_LAUNCH_OK("int8_prep_kernel");
   return LL_OK;
 }
@@ -562,8 +689,8 @@ int i8c_launch(const CUtensorMap& m0, const CUtensorMap& m1, const Ws& w, int M,
     configured.mark();
   }
   const int tiles = (N + 127) / 128;
-  int8_columns_tc_kernel<MP><<<dim3(layers * tiles, ranges), 192, i8c_smem(MP), st>>>(m0, m1, mx, w.part, M, N, K / 128, per, tiles, (size_t)ranges * M * N,
-                                                                                    wait_word());
+  LL_CUDA(launch(int8_columns_tc_kernel<MP>, dim3(layers * tiles, ranges), dim3(192), i8c_smem(MP), st, true, m0, m1, mx, w.part, M, N, K / 128, per, tiles,
+                 (size_t)ranges * M * N, wait_word()));
   LL_LAUNCH_OK("int8_columns_tc_kernel");
   return LL_OK;
 }
@@ -584,6 +711,7 @@ int int8_pass(const T* x, const I8Layer<T>& l0, const I8Layer<T>& l1, T* y, int 
   else if (M <= 48) r = i8c_launch<48>(m0, m1, w, M, N, K, layers, per, ranges, st);
   else r = i8c_launch<64>(m0, m1, w, M, N, K, layers, per, ranges, st);
   if (r) return r;
+  // (Not under the product: its CTAs would pile up on the SMs that are done first, 24 rows with long lists 43 us instead of 33.)
   int8_finish_rows_kernel<T, GATED><<<dim3((N + 63) / 64, (M + 15) / 16), 256, 0, st>>>(w.part, ranges, (size_t)M * N, (size_t)ranges * M * N, w.sca, l0, l1, x,
                                                                                      w.idx, w.count, y, M, N, K);
   LL_LAUNCH_OK("int8_finish_rows_kernel");

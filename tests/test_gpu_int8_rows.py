@@ -256,3 +256,45 @@ def test_prompts_with_long_and_short_lists(M, N, transposed, dtype):
             bound = bound + ((want + odd).abs() * 2.0 ** -8 * 1.01 if dtype == torch.bfloat16 else 0.0)
             assert ((y[rows].double() - want - odd).abs() <= bound).all()
     assert NV.call_ret("ll_int8_tc_error") == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 64, 128), (7, 64, 256), (8, 33, 16384), (8, 33, 16512), (9, 64, 8192), (9, 64, 8320), (24, 64, 1152), (40, 64, 256),
+                                   (63, 130, 512), (64, 64, 2048), (64, 64, 2176)])
+def test_rows_of_a_cluster(M, N, K):
+    """Few rows are prepared by a cluster of eight CTAs: every number of rows a CTA can have, and both sides of the line to a CTA per row."""
+    test_small_batches_against_64_bits(M, N, K, 0)
+
+
+@pytest.mark.parametrize("M", [5, 12, 64, 130])
+def test_columns_that_stand_out_once(M):
+    """Column 97 m stands out in row m alone; infinities stand out, NaN does not and counts as nothing; the rows around keep their own scales."""
+    from lit_llama import _native as NV
+
+    N, K = 16, 16384
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn((M, K), generator=g, device="cuda").clamp(-4, 4).half()
+    r = torch.arange(M, device="cuda")
+    x[r, 97 * r] = 8.0
+    x[M - 1, 5] = float("nan")
+    cb = torch.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=torch.int8)
+    scb = torch.rand(N, generator=g, device="cuda") + 0.5
+    ys = []
+    for v in (x, torch.where(x.isnan(), torch.zeros_like(x), x)):
+        ws = torch.full((NV.call_ret("ll_int8_workspace_bytes", M, N, K),), 0x5A, dtype=torch.uint8, device="cuda")
+        y = torch.empty((M, N), dtype=torch.float16, device="cuda")
+        NV.call("ll_int8_linear", NV.ptr(v), NV.LL_F16, NV.ptr(cb), None, NV.ptr(scb), None, NV.ptr(y), M, N, K, 6.0, NV.ptr(ws), ws.numel(), NV.stream())
+        ys.append(y)
+    torch.cuda.synchronize()
+    assert NV.call_ret("ll_int8_tc_error") == 0
+    assert torch.equal(ys[0], ys[1])
+    a = torch.where(x.isnan(), torch.zeros_like(x), x).double()
+    for b0 in range(0, M, 64):                                 # a column is taken out for a block of 64 rows
+        v = a[b0:b0 + 64]
+        big = v >= 6.0
+        cols, sca = big.any(0), v.masked_fill(big, 0.0).abs().amax(1)
+        ca = torch.round(v.masked_fill(big, 0.0).float() * (torch.full_like(sca, 127.0).float() / sca.float())[:, None]).double().masked_fill(cols[None], 0.0)
+        wo = (cb.double()[:, cols] * scb.double()[:, None] / 127.0).half().double()
+        main, odd, size = (ca @ cb.double().t()) * sca[:, None] * scb.double()[None] / 127.0 ** 2, v[:, cols] @ wo.t(), v[:, cols].abs() @ wo.abs().t()
+        # both parts and their sum rounded to fp16 (2^-11 of each); an outlier's weight may round to the other fp16 neighbour (2^-10 of the term)
+        err = (ys[0][b0:b0 + 64].double() - (main + odd)).abs()
+        assert (err <= 2.0 ** -11 * (main.abs() + odd.abs() + (main + odd).abs()) + 2.0 ** -10 * size + 1e-6).all()
