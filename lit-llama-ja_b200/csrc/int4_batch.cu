@@ -272,6 +272,7 @@ __global__ void __launch_bounds__(256) int4_batch_sum_kernel(const float* __rest
                                                              int steps, int ntiles, int total, int ranges, int slots, int mp) {
   pdl_wait();
   pdl_launch_dependents();
+  part = after_wait(part);
   const int m = blockIdx.y * 8 + (threadIdx.x >> 5), col = (threadIdx.x & 31) * 4, n = blockIdx.x * 128 + col;
   if (m >= M || n >= N) return;
   auto sum = [&](int tile) {

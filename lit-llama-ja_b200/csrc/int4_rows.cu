@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(GATED ? 128 : 256) int4_rows_sum_kernel(const 
                                                                           int mtiles, int full, int parts) {
   pdl_wait();
   pdl_launch_dependents();
+  part = after_wait(part);
   constexpr int OUT = GATED ? 64 : 128, L = GATED ? 2 : 1;              // outputs of a CTA of the pair, layers
   const int t = blockIdx.x, tile = full + t, col = (threadIdx.x & (OUT / 4 - 1)) * 4, rank = (threadIdx.x / (OUT / 4)) & 1;
   const int n = tile / mtiles * (2 * OUT) + rank * OUT + col, r = blockIdx.y * 4 + threadIdx.x / (OUT / 2), m = tile % mtiles * bn + r;
