@@ -1,6 +1,6 @@
 // Softmax attention of prompts on tcgen05: S = Q K^T and O += P V with fp32 accumulators in tensor memory.
 //
-// A block owns two tiles of 128 queries of one head (neighbours, or one from each end: at_apart) and walks the keys they can see 64 at a time:
+// A block owns two tiles of 128 queries of one head, or one (neighbours, one from each end, alone: at_tiles) and walks the keys they can see 64 at a time:
 //   warps 0-7, 8-15 : softmax of tile 0 / tile 1; two threads share a query row, each 32 of its 64 scores: they read them from tensor
 //                     memory, scale, cap, mask, exponentiate, write the weights back over their own scores as packed bf16 (one term, or
 //                     two: hi and what hi left over) and keep the row's sum; at the end they normalise and store the row
@@ -62,6 +62,7 @@ constexpr float AT_BOUND = 80.f;                      // scores that a cap keeps
 
 __device__ int g_attn_tc_error = 0;     // per file that instantiates the kernel: its entry asks for it (attn_tc_error)
 
+enum AtTiles { AT_NEIGHBOURS, AT_APART, AT_ALONE };     // two next to one another, one from the end and one from the start, one
 struct AtParams {
   const int32_t* pos_ids;
   const float* sink;
@@ -70,7 +71,7 @@ struct AtParams {
   __nv_bfloat16* y;
   float scale, softcap;
   int T, H, group, vdim, window, chunk, ring, gate_ld, gate_per_head, gate_vec, y_ld;
-  int apart;                   // a block's two tiles: one from the end and one from the start (else neighbours)
+  int tiles;                   // a block's tiles: AtTiles
   int* word;                   // wait_word()
 };
 
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // neighbours: the last queries see the most keys, so they go first, and the long blocks do not end up as the tail
   const int q_tiles = (p.T + AT_Q - 1) / AT_Q, pair = (int)gridDim.x - 1 - (int)blockIdx.x;
-  const int tile0 = p.apart ? q_tiles - 1 - (int)blockIdx.x : 2 * pair, tile1 = p.apart ? (int)blockIdx.x : 2 * pair + 1;
+  const int tile0 = p.tiles != AT_NEIGHBOURS ? q_tiles - 1 - (int)blockIdx.x : 2 * pair;
+  const int tile1 = p.tiles == AT_ALONE ? tile0 : p.tiles == AT_APART ? (int)blockIdx.x : 2 * pair + 1;
   const int tq0 = tile0 * AT_Q, tq1 = tile1 != tile0 ? tile1 * AT_Q : p.T;      // (the middle one of an odd number stands alone)
   const int h = blockIdx.y, b = blockIdx.z, g = h / p.group;
 
@@ -686,7 +688,8 @@ int at_launch(const AttnTcArgs& a, const AtParams& p, cudaStream_t st) {
     if (int r = at_map(a.q2, a.H, a.T, a.B, AT_Q, &mq2)) return r;
     if (int r = at_map(a.k2, 1, a.ring, a.B, AT_K, &mk2)) return r;
   }
-  const dim3 grid((a.T + 2 * AT_Q - 1) / (2 * AT_Q), a.H, a.B);
+  const int tiles = (a.T + AT_Q - 1) / AT_Q;
+  const dim3 grid(p.tiles == AT_ALONE ? tiles : (tiles + 1) / 2, a.H, a.B);
   kernel<<<grid, AT_THREADS, smem, st>>>(mq, mq2, mk, mk2, mv, p);
   LL_LAUNCH_OK("attn_tc_kernel");
   return LL_OK;
@@ -707,7 +710,13 @@ bool attn_tc_supported(const AttnTcArgs& a) {
 // blocks alike (2048 queries, 16 heads of 128: 50 us -> 40, capped 57 -> 45; 32 heads 84 -> 74).  Tiles that a window keeps alike stay
 // neighbours, which share most of their keys (window 700 of 2048: 30.3, apart 31.3; chunks of 512: 21.7, apart 24.7; a window of half of the
 // queries is even at 33, one of 1500 of 1736 42 -> 40 apart).
-bool at_apart(const AttnTcArgs& a) { return a.chunk <= 0 && (a.window <= 0 || 2ll * a.window >= a.T); }
+// With no more tiles than SMs a block takes one (us, two a block / one: 32 heads, 300 and 512 queries 15.4 / 13.6, 18.6 / 16.3; 16 heads, 130, 512, 1024,
+// 1152 queries 13.3 / 11.0, 17.8 / 14.4, 24.4 / 21.8, 26.8 / 23.7, with a window of 200 of 1024 19.7 / 14.8; 8 heads, 2048 queries 37.8 / 35.1).
+int at_tiles(const AttnTcArgs& a) {
+  const int sms = sm_count();
+  if ((long long)((a.T + AT_Q - 1) / AT_Q) * a.H * a.B <= (sms > 0 ? sms : 148)) return AT_ALONE;
+  return a.chunk <= 0 && (a.window <= 0 || 2ll * a.window >= a.T) ? AT_APART : AT_NEIGHBOURS;
+}
 
 enum AttnTcKind { AT_ROTARY, AT_LATENT };     // which forms a file instantiates
 
@@ -715,7 +724,7 @@ template <AttnTcKind KIND>
 int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
   const AtParams p{a.pos_ids, a.sink, a.slopes, (const __nv_bfloat16*)a.gate, (__nv_bfloat16*)a.y, a.scale, a.softcap, a.T, a.H, a.H / a.G,
                    a.v.dim, a.window, a.chunk, a.ring, a.gate_ld, a.gate_per_head,
-                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, at_apart(a), wait_word()};
+                   a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, at_tiles(a), wait_word()};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
   const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \

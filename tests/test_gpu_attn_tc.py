@@ -51,6 +51,10 @@ CASES = [dict(T=t, past=0, ring=512) for t in (16, 63, 64, 65, 127, 128, 129, 25
 APART = [dict(T=513, past=70, ring=583, cap=50.0, sink=True, gate=True), dict(T=640, past=0, ring=640), dict(T=385, past=0, ring=385, cap=100.0, sink=True),
          dict(T=700, past=20, ring=720, window=400), dict(T=640, past=3, ring=700, cap=1.5, slopes=True, spoil=True)]
 CASES += APART
+# with no more tiles than SMs a block takes one of them; the same walks with more: two tiles a block, from both ends or neighbours
+CASES += [dict(c, B=149 // (-(-c["T"] // 128) * 4) + 1) for c in APART + [
+    dict(T=300, past=33, ring=512, chunk=50), dict(T=513, past=77, ring=650, window=64, spoil=True), dict(T=257, past=3, ring=260, cap=50.0),
+    dict(T=129, past=0, ring=129, dim=128, vdim=128, gate=True), dict(T=40, past=250, ring=256, window=20)]]
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(f"{k}{v}" for k, v in c.items()))
@@ -193,3 +197,34 @@ def test_models_say_where_a_step_ends(family, monkeypatch, tmp_path):
     util.run_schedule(m, list(range(9)), [5, 3, 1], 64)
     assert {e for t, e in ends if t == 5} == {5} and {e for t, e in ends if t == 3} == {8}
     assert {e for t, e in ends if t == 1} <= {None}              # a captured step's position is known to the device alone
+
+
+@pytest.mark.parametrize("T,past,S,window,terms", [(129, 0, 200, 50, False), (257, 100, 400, None, True), (385, 20, 420, None, False)])
+def test_latent_tiles_of_many_sequences(T, past, S, window, terms):
+    """More tiles than SMs (two a block, neighbours or from both ends) against the same sequences two at a time (a tile a block): a row meets the same
+    keys in the same order, in blocks that may start elsewhere (its weights round apart by 2^-9 at most, and the row once more)."""
+    from lit_llama import _native as N
+    from lit_llama.latent_attention import LatentAttention, LatentAttentionSpec
+
+    B, H, nope, rot, v = 28, 3, 64, 32, 64
+    spec = LatentAttentionSpec(width=64, heads=H, nope_dim=nope, rot_dim=rot, v_dim=v, kv_rank=256, window=window, scale=(nope + rot) ** -0.5,
+                               gate="head", exact_weights=terms)
+    m = LatentAttention(spec, torch.bfloat16, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(T)
+    for p in m.parameters():
+        if p.dim() > 1:
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") / math.sqrt(p.shape[-1]))
+    proj = torch.randn((B * T, m.w_in.shape[0]), generator=g, device="cuda").to(torch.bfloat16)
+    pos = torch.arange(past, past + T, dtype=torch.int32, device="cuda")
+    rope = spec.rope_table(past + T, "cuda")
+    cache = torch.randn((B, S, spec.row), generator=g, device="cuda").to(torch.bfloat16)
+    m._takes_expanded = lambda *a: True
+    both = []
+    for n in (B, 2):
+        outs = []
+        for b in range(0, B, n):
+            out = torch.zeros((n * T, H * v), dtype=torch.bfloat16, device="cuda")
+            outs.append(m.attend(proj[b * T:(b + n) * T], n, T, pos, rope, cache[b:b + n].clone(), 1, out).double())
+        both.append(torch.cat(outs))
+    assert N.call_ret("ll_latent_prompt_error") == 0
+    assert torch.isfinite(both[0]).all() and (both[0] - both[1]).norm() <= 2.0 ** -7.5 * both[1].norm()
