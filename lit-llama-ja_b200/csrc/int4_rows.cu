@@ -449,10 +449,12 @@ long long r4_cost(int M, int N, int tile_n, int steps, int bn, int pairs) {
 }
 // The same of `tiles` tiles cut into `parts` along k each: their steps, the launch that adds the parts up (5 us) and their way through L2 (6 MB a us).
 // us on the device, every tile whole / by this rule: 4096 x 11008 at 130, 300, 512 rows 48 / 24, 50 / 34, 50 / 43, from 700 on all whole (53; in the
-// parts nearest to paying 58); 2048 x 5632 at 130, 512, 700 rows 27 / 15, 27 / 21, 29 / 24; 4096 x 4096 at 130, 300 rows 22 / 16, 23 / 20, 512 whole
-// (24; 26); the gated 11008 x 4096 at 130, 300, 512, 700 rows 45 / 37, 63 / 56, 80 / 74, 109 / 106.  Ranges of one length for all pairs, that cross
-// tile ends, were 2 to 4 us slower (two drains a pair, more parts); the last pair to arrive adding up in the kernel itself made the loop spill (whole
-// tiles a fifth slower).
+// parts nearest to paying 58); the gated 11008 x 4096 at 130, 300, 512, 700 rows 45 / 37, 63 / 56, 80 / 74, 109 / 106.  Short layers (R4_SHORT) stay
+// whole: 2048 x 5632 of 130 rows would take 15 instead of 27, but calls of its size are bound by the host, for which a second launch and its scratch
+// are 2 us (228 rows through a feed-forward of width 2048, a call 49 whole, 51 cut).  Ranges of one length for all pairs, that cross tile ends, were
+// 2 to 4 us slower (two drains a pair, more parts); the last pair to arrive adding up in the kernel itself made the loop spill (whole tiles a fifth
+// slower).
+constexpr long long R4_SHORT = 40000;
 constexpr int R4_PARTS = 8;
 long long r4_parts_cost(int steps, int bn, int tiles, int parts, int pairs) {
   return (long long)((tiles * parts + pairs - 1) / pairs) * ((long long)((steps + parts - 1) / parts) * r4_step(bn) + 1500) + 7000 + tiles * parts * bn / 4;
@@ -465,11 +467,15 @@ struct R4Plan {
 R4Plan r4_plan(int M, int N, int steps, int tile_n, int pairs, int tile_rows, int parts, bool scratch) {
   R4Plan best{};
   long long least = 0;
-  for (int bn = tile_rows ? tile_rows : 256; bn >= (tile_rows ? tile_rows : 128); bn -= 32) {
-    const int tiles = ((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n), full = tiles / pairs * pairs, rest = tiles - full;
+  const int most = tile_rows ? tile_rows : 256, fewest = tile_rows ? tile_rows : 128;
+  for (int bn = most; bn >= fewest; bn -= 32) {
     const long long whole = r4_cost(M, N, tile_n, steps, bn, pairs);
-    if (best.bn == 0 || whole < least) best = {bn, tiles, 0}, least = whole;
-    if (!scratch || rest == 0) continue;
+    if (best.bn == 0 || whole < least) best = {bn, ((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n), 0}, least = whole;
+  }
+  if (!scratch || (parts == 0 && least < R4_SHORT)) return best;
+  for (int bn = most; bn >= fewest; bn -= 32) {
+    const int tiles = ((M + bn - 1) / bn) * ((N + tile_n - 1) / tile_n), full = tiles / pairs * pairs, rest = tiles - full;
+    if (rest == 0) continue;
     const long long before = r4_cost(full / pairs * bn, tile_n, tile_n, steps, bn, 1);
     for (int s = parts > 0 ? parts : 2; s <= (parts > 0 ? parts : R4_PARTS) && s <= steps && rest * s <= 2 * pairs; ++s) {
       const long long cost = before + r4_parts_cost(steps, bn, rest, s, pairs);
