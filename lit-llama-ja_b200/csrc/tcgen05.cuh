@@ -27,6 +27,11 @@ EncodeTiledFn encode_fn() {
         qres == cudaDriverEntryPointSuccess)
       fn = (EncodeTiledFn)p;
   });
+  // The driver's call wants a context.  A thread whose first call this is may have none: memory that the caller's pool serves binds none, and a
+  // layer's first launch comes after its maps (error 201 in every new thread).
+  thread_local bool bound = false;
+  int dev = 0;
+  if (!bound) bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
   return fn;
 }
 
