@@ -33,6 +33,12 @@ def _batch_scratch_bytes(M: int, Nout: int, K: int, layers: int) -> int:
     return N.call_ret("ll_int4_batch_scratch_bytes", M, Nout, K, layers, 0)
 
 
+def _call_scratch(x: torch.Tensor, nbytes: int) -> torch.Tensor:
+    """Scratch of one call alone.  A call is several launches and the interpreter is let go during it, so the launches of two threads on one stream
+    can alternate, and graphs captured on one stream can be replayed on two: neither may meet the other's partial sums."""
+    return x.new_empty(nbytes, dtype=torch.uint8)
+
+
 @functools.lru_cache(maxsize=4096)
 def _rows_scratch_bytes(M: int, Nout: int, K: int, layers: int) -> int:
     return N.call_ret("ll_int4_rows_scratch_bytes", M, Nout, K, layers, 0, 0, 0)
@@ -258,7 +264,7 @@ class ColBlockQuantizedLinear(torch.nn.Module):
         elif self.ROWS_MIN_M <= M <= self.ROWS_MAX_M and self._rows_eligible(x):
             nbytes = _rows_scratch_bytes(M, Nout, K, 1)
             if nbytes:                         # (a last wave of tiles that pays to be cut along k)
-                scratch = _int8_workspace(x.device, nbytes)
+                scratch = _call_scratch(x, nbytes)
                 N.call("ll_int4_rows_split", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y),
                        N.ptr(scratch), M, Nout, K, self.tile_cols, 0, 0, 0, N.stream())
             else:
@@ -362,7 +368,7 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
         q1, q2 = fc1._packed_ptr_ok(), fc2._packed_ptr_ok()
         N.require_cuda(q1, q2)
         nbytes = _rows_scratch_bytes(M, Nout, K, 2)
-        scratch = _int8_workspace(x.device, nbytes) if nbytes else None
+        scratch = _call_scratch(x, nbytes) if nbytes else None
         N.call("ll_int4_rows_gated_split", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
                N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), N.ptr(scratch), M, Nout, K, fc1.tile_cols, 0, 0, 0, N.stream())
     else:

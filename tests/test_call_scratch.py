@@ -1,0 +1,63 @@
+"""Scratch of quantized layers, on the host: the library's launches are recorded instead of made.  A call that begins while another one is still in the
+library (two threads: the interpreter is let go there) must not be given the other's scratch."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+# entry -> where its scratch stands among the arguments
+SCRATCH = {"ll_int4_rows_split": 6, "ll_int4_rows_gated_split": 10}
+
+
+@pytest.fixture
+def library(monkeypatch):
+    from lit_llama import quantization as q
+
+    class Library:
+        depth, inner, seen = 0, None, []
+
+        def call(self, name, *a):
+            if name not in SCRATCH:
+                return
+            self.seen.append((name, a[SCRATCH[name]]))
+            if self.depth == 0 and self.inner is not None:
+                self.depth = 1
+                self.inner()
+                self.depth = 0
+
+    lib = Library()
+    lib.seen = []
+    monkeypatch.setattr(q.N, "require_cuda", lambda *t: None)
+    monkeypatch.setattr(q.N, "stream", lambda: 0)
+    monkeypatch.setattr(q.N, "call", lib.call)
+    monkeypatch.setattr(q, "_INT8_WS", {})
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    return lib
+
+
+def _int4(N, K):
+    from lit_llama.quantization import ColBlockQuantizedLinear
+
+    lin = ColBlockQuantizedLinear(K, N, False, bits=4, tile_cols=128).to(torch.bfloat16)
+    lin.quant_weight.zero_(), lin.scales.fill_(1.0), lin.zeros.zero_()
+    return lin
+
+
+def _two_at_once(library, call):
+    library.inner = call
+    call()
+    assert len(library.seen) == 2 and all(at for _, at in library.seen)
+    return library.seen[0][1] != library.seen[1][1]
+
+
+def test_cut_tiles_of_prompts(library):
+    lin, x = _int4(1024, 11008), torch.zeros((300, 11008), dtype=torch.bfloat16)
+    assert _two_at_once(library, lambda: lin(x))
+
+
+def test_cut_tiles_of_gated_prompts(library):
+    from lit_llama.quantization import gated_pair
+
+    l1, l2, x = _int4(11008, 4096), _int4(11008, 4096), torch.zeros((300, 4096), dtype=torch.bfloat16)
+    rows = SimpleNamespace(shape=x.shape, device=SimpleNamespace(type="cuda"), reshape=x.reshape)
+    assert _two_at_once(library, lambda: gated_pair(l1, l2, rows))
