@@ -7,6 +7,7 @@ call fails.  Build the library with ``python lit-llama-ja_b200/build.py``.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from pathlib import Path
 
 import torch
@@ -348,7 +349,23 @@ def layer_rows(M: int, weights: int, most: int, large: bool) -> bool:
             return True
     elif not large:
         return False
-    return M * weights <= most and not torch.cuda.is_current_stream_capturing()
+    if M * weights > most or torch.cuda.is_current_stream_capturing():
+        return False
+    _ready_library()
+    return True
+
+
+_made = threading.local()
+
+
+def _ready_library() -> None:
+    """The library's handle of this thread and device, made outside a capture: a step that takes one call here takes the library's products when it is
+    captured, and a handle cannot be made there (the calls before it, which made one, no longer do)."""
+    dev = torch.cuda.current_device() if _current_device is None else _current_device()
+    devices = _made.__dict__.setdefault("devices", set())
+    if dev not in devices:
+        torch.cuda.current_blas_handle()
+        devices.add(dev)
 
 
 _PLAIN = (torch.nn.Parameter, torch.Tensor)
