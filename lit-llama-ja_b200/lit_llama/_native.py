@@ -339,17 +339,14 @@ def gemv(args: GemvArgs) -> None:
 FEW_ROWS, LARGE_WEIGHTS = 8, 1 << 25
 
 
-def layer_rows(M: int, weights: int, most: int, large: bool) -> bool:
+def layer_rows(M: int, weights: int, most: int, largest: int) -> bool:
     """Whether a layer of ``M`` rows that could run in one call does.  A few rows of a layer that is not large: always, its products are as fast as
     the library's (csrc/small_rows.cuh).  Else while rows times weights, which is what its kernels' time goes by, stays under ``most``, the work that
-    takes as long as the host takes to make the separate calls (``large``: also with weights whose way from memory is most of the time).  A step that
-    is being captured has no such calls to save, and there the library's products of more rows are the faster ones."""
-    if weights <= LARGE_WEIGHTS:
-        if M <= FEW_ROWS:
-            return True
-    elif not large:
-        return False
-    if M * weights > most or torch.cuda.is_current_stream_capturing():
+    takes as long as the host takes to make the separate calls, and the weights, whose way from memory the library's products are the faster for, under
+    ``largest``.  A step that is being captured has no such calls to save, and there the library's products of more rows are the faster ones."""
+    if M <= FEW_ROWS and weights <= LARGE_WEIGHTS:
+        return True
+    if M * weights > most or weights > largest or torch.cuda.is_current_stream_capturing():
         return False
     _ready_library()
     return True

@@ -44,18 +44,28 @@ EXPAND_MAX_BYTES = 512 << 20         # of the expanded rows of a step
 # 4096 over 300 104 / 58, two sequences 102 / 61; replayed as a graph 40.5 / 33.2, 53.9 / 51.2 and 60.4 / 55.4.  Graphed, every layer's weights
 # and rows from memory, over 300 and 2000 rows: width 1024 48 / 42 and 47 / 41, 2048 50 / 46 and 50 / 45, 4096 63 / 59 and 63 / 58; two sequences
 # 48 / 43 and 50 / 44, 52 / 48 and 52 / 48, 66 / 63 and 66 / 62.
-# From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
-# Rows times weights of a layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 2048 rows 92 / 40,
-# 95 / 56, 95 / 76; 2048, 17, 400, 1024 and 2048 rows 93 / 43, 92 / 66, 92 / 76, 110 / 108; 4096, 3, 17, 120 and 700 rows 89 / 62, 92 / 62, 93 / 79, 101 / 114.  A
-# few rows, replayed as a graph: one token of four sequences over 1500 rows, widths 1024 and 2048: 37 / 34, 43 / 39 (4096: 55 / 59, so not there).
-LAYER_MAX_PRODUCTS = 12 << 30
-LATENT_MAX_ROW_HEADS = 512           # rows times heads of a step in one call whose queries stay in latent space: 18 rows, 16 heads 89 / 60, 32 heads 89 / 93
+# More rows: rows times weights of a layer that runs in one call, and its weights (_native.layer_rows).  us a call, separate / one, keys and values expanded
+# per head: width 1024, 17, 400 and 2048 rows 92 / 40, 95 / 56, 95 / 76; 2048, 17, 400, 1024 and 2048 rows 93 / 43, 92 / 66, 92 / 76, 110 / 108; 4096 (44M
+# weights), 17, 120, 300 and 700 rows 99 / 76, 98 / 70, 95 / 83, 101 / 114; 69M, 17, 120 and 300 rows 96 / 88, 101 / 83, 97 / 93; 98M, 17, 120 and 200
+# rows 101 / 97, 95 / 92, 99 / 104; 173M, 17, 60 and 200 rows 120 / 126, 106 / 109, 121 / 126.  A few rows, replayed as a graph: one token of four
+# sequences over 1500 rows, widths 1024 and 2048: 37 / 34, 43 / 39 (4096: 55 / 59, so not there).
+LAYER_MAX_PRODUCTS, LAYER_MAX_WEIGHTS = 12 << 30, 100 << 20
+# Rows times heads of a step in one call whose queries stay in latent space (every four rows read the heads' weights again, and long walks leave no host
+# time to save), and its weights.  us, separate / one: 24 heads, 3, 8 and 16 tokens over 300 rows 89 / 66, 89 / 71, 87 / 83, over 2000 rows 4, 8 and 16
+# tokens 203 / 197, 202 / 200, 203 / 214; 32 heads (44M weights) 92 / 82, 90 / 85, 92 / 104, 219 / 213, 220 / 216, 219 / 236, one sequence's 8 and 12
+# tokens 100 / 100, 100 / 109; 40 heads (69M) 3 and 8 tokens 97 / 97, 98 / 102, over 2000 rows 223 / 227, 224 / 232.
+LATENT_MAX_ROW_HEADS, LATENT_MAX_WEIGHTS = 256, 3 << 24
 
 
 @functools.lru_cache(maxsize=1024)
 def _layer_scratch_bytes(*sizes: int) -> int:
     return N.call_ret("ll_latent_layer_scratch_bytes", *sizes)
+
+
+@functools.lru_cache(maxsize=1024)
+def _expanded_supported(*sizes: int) -> bool:
+    return N.has("ll_latent_layer") and bool(N.call_ret("ll_latent_prompt_supported", *sizes))
 
 
 @dataclass
@@ -199,8 +209,10 @@ class LatentAttention(nn.Module):
         """x_act ``[B*T, width]`` -> ``[B*T, width]``; ``cache`` ``[B, S, row]`` is this layer's or its source's (already
         appended to by the source in this step).  ``end``: as in ``attend``."""
         at, rows = (self._takes_step(x_act, B, cache), 0) if T == 1 else (None, 0)
-        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, True):
-            at, rows = self._takes_layer_rows(x_act, B, T, cache, splits, end)
+        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None:
+            rows = self._layer_form(B, T, cache, splits, end)
+            if rows is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, LAYER_MAX_WEIGHTS):
+                at = self._takes_layer(x_act, B * T, cache, "ll_latent_layer")
         if at:
             return self._one_call(at, x_act, B, T, pos_ids, rope, cache, rows, splits)
         return F.linear(self.attend(F.linear(x_act, self.w_in), B, T, pos_ids, rope, cache, splits, end=end), self.w_o)
@@ -209,22 +221,18 @@ class LatentAttention(nn.Module):
         """One token of one or two sequences."""
         return self._takes_layer(x_act, B, cache, "ll_latent_step") if 1 <= B <= STEP_MAX_ROWS else None
 
-    def _takes_layer_rows(self, x_act: torch.Tensor, B: int, T: int, cache: torch.Tensor, splits: int, end: Optional[int]):
-        """Several rows: (the weights' addresses or ``None``, cache rows per sequence that are expanded per head or 0).  The form of attention is
+    def _layer_form(self, B: int, T: int, cache: torch.Tensor, splits: int, end: Optional[int]) -> Optional[int]:
+        """Cache rows per sequence that a call of several rows expands per head, 0: queries stay in latent space; ``None``: not in one call.  The form is
         the one that the separate calls would take."""
-        s = self.spec
-        at = self._takes_layer(x_act, B * T, cache, "ll_latent_layer")
-        if not at:
-            return None, 0
-        S, n_in = cache.shape[1], self._parameters["w_in"].shape[0]
+        s, S = self.spec, cache.shape[1]
         if T >= EXPAND_MIN_TOKENS and splits == 1:
             first, rows = self._visible(T, S, end)
-            if (s.scale > 0 and self._expand_pays(B, T, rows)
-                    and N.call_ret("ll_latent_prompt_supported", s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, n_in, s.q_head, s.heads * s.v_dim)
-                    and cache.data_ptr() % 16 == 0):
-                whole = first is None or (first == 0 and (B == 1 or rows == S))
-                return (at, rows) if whole and s.v_dim % 64 == 0 else (None, 0)
-        return (at, 0) if B * T * s.heads <= LATENT_MAX_ROW_HEADS else (None, 0)
+            if s.v_dim % 64 or not (first is None or (first == 0 and (B == 1 or rows == S))):
+                return None
+            if s.scale > 0 and self._expand_pays(B, T, rows) and cache.data_ptr() % 16 == 0 and _expanded_supported(
+                    s.nope_dim, s.rot_dim, s.v_dim, s.kv_rank, self.w_in.shape[0], s.q_head, s.heads * s.v_dim):
+                return rows
+        return 0 if B * T * s.heads <= LATENT_MAX_ROW_HEADS and self.w_in.numel() + self.w_o.numel() <= LATENT_MAX_WEIGHTS else None
 
     def _expand_pays(self, B: int, T: int, rows: int) -> bool:
         s = self.spec

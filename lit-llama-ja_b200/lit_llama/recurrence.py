@@ -47,10 +47,12 @@ def pad8(n: int) -> int:
     return (n + 7) // 8 * 8
 
 
-# Rows times weights of a matrix memory layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 1024
-# rows 66 / 30, 77 / 57, 79 / 74; 2048, 17, 400 and 700 rows 67 / 33, 78 / 70, 86 / 94; 4096, 17 and 400 rows 67 / 30, 78 / 68.  A few rows, replayed as a
+# Rows times weights of a matrix memory layer that runs in one call, and its weights (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400
+# and 1024 rows 66 / 30, 77 / 57, 79 / 74; 2048, 17, 400 and 700 rows 67 / 33, 78 / 70, 86 / 94; 34M weights, 17, 120, 200 and 300 rows 66 / 38, 79 / 60,
+# 77 / 71, 77 / 78; 53M, 17, 60, 120 and 200 rows 67 / 52, 66 / 67, 78 / 72, 79 / 86; 67M, 3, 17, 60 and 200 rows 66 / 46, 65 / 54, 66 / 66, 84 / 87; 76M,
+# 3, 17 and 60 rows 66 / 52, 65 / 64, 70 / 78; 134M, 3, 8 and 120 rows 74 / 80, 83 / 93, 99 / 108.  A few rows, replayed as a
 # graph: one token of three sequences, widths 1024, 2048, 4096: 20 / 13, 21 / 18, 26 / 17.
-LAYER_MAX_PRODUCTS = 6 << 30
+LAYER_MAX_PRODUCTS, LAYER_MAX_WEIGHTS = 6 << 30, 1 << 26
 
 
 @functools.lru_cache(maxsize=1024)
@@ -340,7 +342,7 @@ class MatrixMemoryMixer(nn.Module):
         c = self.cols
         memory, stabiliser = states
         M = B * T
-        at = self._takes_layer(u, M) if N.layer_rows(M, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, True) else None
+        at = self._takes_layer(u, M) if N.layer_rows(M, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, LAYER_MAX_WEIGHTS) else None
         if at:
             return self._one_call(at, u, B, T, pos_ids, states)
         proj = F.linear(u, self.w_in)

@@ -226,7 +226,7 @@ class SoftmaxAttention(nn.Module):
     def forward(self, u: torch.Tensor, B: int, T: int, pos_ids: torch.Tensor, caches, conv_state=None, splits: int = 1,
                 form: int = 0) -> torch.Tensor:
         at = self._takes_step(u, B, caches) if T == 1 else None
-        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, False):
+        if not at and (T > 1 or B > STEP_MAX_ROWS) and self.w_in is not None and N.layer_rows(B * T, self.w_in.numel() + self.w_o.numel(), LAYER_MAX_PRODUCTS, N.LARGE_WEIGHTS):
             at = self._takes_layer(u, B * T, caches, "ll_softmax_layer")
         if at:
             return self._one_call(at, u, B, T, pos_ids, caches, splits, form)
