@@ -171,10 +171,11 @@ class MoE(nn.Module):
 
     def takes_tensor_cores(self, n_rows: int, x_act: torch.Tensor) -> bool:
         """Whether a step of ``n_rows`` (token, choice) rows runs its expert GEMMs on the tcgen05 kernels: bfloat16, rows
-        that TMA can tile (16-byte multiples), and enough rows per expert to fill 128-row tiles."""
+        that TMA can tile (16-byte multiples on 16-byte boundaries, the other kernels read any), and enough of them."""
         s = self.spec
         return (x_act.dtype == torch.bfloat16 and s.width % 8 == 0 and s.ff % 8 == 0 and x_act.stride(0) % 8 == 0
-                and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts and N.has("ll_moe_grouped_gemm_tc"))
+                and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts
+                and (x_act.data_ptr() | self.w_gu.data_ptr() | self.w_down.data_ptr()) % 16 == 0 and N.has("ll_moe_grouped_gemm_tc"))
 
     def _one_call(self, entry: str, at, x_act: torch.Tensor, M: int, scratch_bytes: int) -> torch.Tensor:
         """The whole layer through ``ll_moe_step`` or ``ll_moe_prompt``."""
