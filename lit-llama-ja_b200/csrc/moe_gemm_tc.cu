@@ -18,8 +18,9 @@ namespace llb {
 
 // moe_ops.cu: the router alone, and the combination, as parts of a chain of launches
 int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
-                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
-                   cudaStream_t st);
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   const void* gate_row, float* gate, cudaStream_t st);
+int moe_permute(const int32_t* expert_idx, const int32_t* rank, const int32_t* counts, int n_pairs, int X, int32_t* offsets, int32_t* perm, cudaStream_t st);
 int moe_combine_rows(const void* y, const float* expert_w, int top, const void* shared_y, const float* gate, void* out, int M, int dim, cudaStream_t st);
 
 namespace {
@@ -45,11 +46,15 @@ __global__ void __launch_bounds__(32 * GR_WARPS) moe_gather_rows_kernel(const ui
   }
 }
 
-// The (token, choice) pairs of a prompt in the order of their experts, and the experts in the order of their tiles' size: one block, counts
-// and places in shared memory (8192 pairs of 32 experts: 4 us; the pairs of an expert come in no fixed order, which no result depends on).
-constexpr int SORT_THREADS = 1024, SORT_KEPT = 16;
-__global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const int32_t* expert_idx, int n_pairs, int X, int32_t* __restrict__ offsets,
-                                                                int32_t* __restrict__ order, int32_t* __restrict__ perm) {
+// The (token, choice) pairs of a prompt in the order of their experts, the experts in the order of their tiles' size, and how many row tiles stand before
+// each of them in that order: one block, counts and places in shared memory (8192 pairs of 32 experts: 4 us; the pairs of an expert come in no
+// fixed order, which no result depends on).  Pairs in registers: up to SORT_PAIRS.  More are counted by the router and placed by a grid of their own
+// (moe_permute; counts not null), which leaves the experts to this kernel: in one block
+// the rest of 131072 pairs of four experts took a layer of 64 x 64 358 us instead of 282.
+constexpr int SORT_THREADS = 1024, SORT_KEPT = 16, SORT_PAIRS = SORT_THREADS * SORT_KEPT, SORT_EXPERTS = 4;      // SORT_EXPERTS: of a thread
+__global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const int32_t* expert_idx, const int32_t* counts, int n_pairs, int X,
+                                                                int32_t* __restrict__ offsets, int32_t* __restrict__ order, int32_t* __restrict__ first,
+                                                                int32_t* __restrict__ perm) {
   extern __shared__ int32_t sort_smem[];
   int32_t *count = sort_smem, *at = count + X, *size = at + X;      // [X] each
   const int tid = threadIdx.x, lane = tid & 31;
@@ -57,50 +62,68 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(const int32_t* e
   for (int e = tid; e < X; e += SORT_THREADS) count[e] = 0;
   __syncthreads();
   pdl_wait();
-  expert_idx = after_wait(expert_idx);
-  int32_t mine[SORT_KEPT], rank[SORT_KEPT];      // the first pairs of a thread keep their places in registers
+  int32_t mine[SORT_KEPT], rank[SORT_KEPT];
+  if (counts == nullptr) {
+    expert_idx = after_wait(expert_idx);
 #pragma unroll
-  for (int j = 0; j < SORT_KEPT; ++j) mine[j] = j * SORT_THREADS + tid < n_pairs ? expert_idx[j * SORT_THREADS + tid] : -1;
+    for (int j = 0; j < SORT_KEPT; ++j) mine[j] = j * SORT_THREADS + tid < n_pairs ? expert_idx[j * SORT_THREADS + tid] : -1;
 #pragma unroll
-  for (int j = 0; j < SORT_KEPT; ++j)
-    if (mine[j] >= 0) rank[j] = atomicAdd(&count[mine[j]], 1);
-  __syncthreads();                               // (theirs are the first places; the rest fill an expert's rows from behind)
-  for (int i = SORT_KEPT * SORT_THREADS + tid; i < n_pairs; i += SORT_THREADS) atomicAdd(&count[expert_idx[i]], 1);
+    for (int j = 0; j < SORT_KEPT; ++j)
+      if (mine[j] >= 0) rank[j] = atomicAdd(&count[mine[j]], 1);
+  } else {
+    counts = after_wait(counts);
+    for (int e = tid; e < X; e += SORT_THREADS) count[e] = counts[e];
+  }
   __syncthreads();
-  if (tid < 32) {
+  // exclusive sums of numbers in shared memory, by the first warp
+  auto sums = [&](const int32_t* v, int32_t* keep, int32_t* out) {
     int before = 0;
     for (int e0 = 0; e0 < X; e0 += 32) {
-      const int e = e0 + lane, c = e < X ? count[e] : 0;
+      const int e = e0 + lane, c = e < X ? v[e] : 0;
       int incl = c;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
+        const int u = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += u;
       }
       if (e < X) {
-        at[e] = offsets[e] = before + incl - c;
-        count[e] = before + incl;
-        const int tiles = (c + MT_NMAX - 1) / MT_NMAX;
-        size[e] = c > 0 ? MtWalk::columns(c, tiles) : 0;
+        out[e] = before + incl - c;
+        if (keep != nullptr) keep[e] = before + incl - c;
       }
       before += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) offsets[X] = before;
+    if (lane == 0) out[X] = before;
+  };
+  auto row_tiles = [&](int e) { return (count[e] + MT_NMAX - 1) / MT_NMAX; };
+  for (int e = tid; e < X; e += SORT_THREADS) size[e] = count[e] > 0 ? MtWalk::columns(count[e], row_tiles(e)) : 0;
+  if (tid < 32) sums(count, at, offsets);
+  __syncthreads();
+  int place[SORT_EXPERTS];
+#pragma unroll
+  for (int j = 0; j < SORT_EXPERTS; ++j) {
+    const int e = j * SORT_THREADS + tid;
+    if (e >= X) break;
+    const int own = size[e];
+    int n = 0;
+#pragma unroll 4
+    for (int o = 0; o < X; ++o) n += size[o] > own || (size[o] == own && o < e);
+    order[n] = e;
+    place[j] = n;
   }
   __syncthreads();
-  for (int e = tid; e < X; e += SORT_THREADS) {
-    int place = 0;
-    for (int o = 0; o < X; ++o) place += size[o] > size[e] || (size[o] == size[e] && o < e);
-    order[place] = e;
-  }
 #pragma unroll
-  for (int j = 0; j < SORT_KEPT; ++j)
-    if (mine[j] >= 0) perm[at[mine[j]] + rank[j]] = j * SORT_THREADS + tid;
-  for (int i = SORT_KEPT * SORT_THREADS + tid; i < n_pairs; i += SORT_THREADS) perm[atomicSub(&count[expert_idx[i]], 1) - 1] = i;
+  for (int j = 0; j < SORT_EXPERTS; ++j)
+    if (j * SORT_THREADS + tid < X) size[place[j]] = row_tiles(j * SORT_THREADS + tid);
+  __syncthreads();
+  if (tid < 32) sums(size, nullptr, first);
+  if (counts == nullptr)
+#pragma unroll
+    for (int j = 0; j < SORT_KEPT; ++j)
+      if (mine[j] >= 0) perm[at[mine[j]] + rank[j]] = j * SORT_THREADS + tid;
 }
 
 struct MpScratch {
-  int32_t *idx, *offsets, *order, *perm;
+  int32_t *idx, *offsets, *order, *first, *perm, *counts, *rank;      // counts, rank: of more pairs than the sort keeps
   float *weight, *gate;
   __nv_bfloat16 *xs, *h, *y, *hs, *ys;
   size_t total;
@@ -113,6 +136,8 @@ MpScratch mp_carve(void* base, int M, int X, int top, int width, int ff, int sff
   const size_t n = (size_t)M * top;
   s.idx = (int32_t*)(p + take(n * 4)), s.weight = (float*)(p + take(n * 4)), s.perm = (int32_t*)(p + take(n * 4));
   s.offsets = (int32_t*)(p + take((size_t)(X + 1) * 4)), s.order = (int32_t*)(p + take((size_t)X * 4)), s.gate = (float*)(p + take((size_t)M * 4));
+  s.first = (int32_t*)(p + take((size_t)(X + 1) * 4));
+  s.counts = (int32_t*)(p + take(n > SORT_PAIRS ? (size_t)X * 4 : 0)), s.rank = (int32_t*)(p + take(n > SORT_PAIRS ? n * 4 : 0));
   s.xs = (__nv_bfloat16*)(p + take(n * width * 2)), s.h = (__nv_bfloat16*)(p + take(n * ff * 2)), s.y = (__nv_bfloat16*)(p + take(n * width * 2));
   s.hs = (__nv_bfloat16*)(p + take((size_t)M * sff * 2)), s.ys = (__nv_bfloat16*)(p + take(sff ? (size_t)M * width * 2 : 0));
   s.total = o;
@@ -160,7 +185,8 @@ int ll_moe_grouped_gemm_tc(const void* a, const void* w, const int32_t* offsets,
 }
 
 int ll_moe_prompt_supported(int M, int width, int n_experts, int ff, int shared_ff) {
-  return M >= 1 && M < (1 << 24) && width > 0 && width % 8 == 0 && ff > 0 && ff % 8 == 0 && shared_ff >= 0 && shared_ff % 8 == 0 && n_experts <= 4096 &&
+  return M >= 1 && M < (1 << 24) && width > 0 && width % 8 == 0 && ff > 0 && ff % 8 == 0 && shared_ff >= 0 && shared_ff % 8 == 0 &&
+         n_experts <= SORT_THREADS * SORT_EXPERTS &&
          (long long)n_experts * 2 * ff < (1ll << 31) && (long long)n_experts * width < (1ll << 31);
 }
 
@@ -184,11 +210,15 @@ int ll_moe_prompt(const void* x, const float* w_router, const float* bias, const
   const MpScratch s = mp_carve(scratch, M, n_experts, top, width, ff, shared_ff);
   const int n = M * top, up = mode == 2 ? 1 : mode;
   const __nv_bfloat16* gate_row = shared_ff && shared_gate ? (const __nv_bfloat16*)ws_in + (size_t)(up == 1 ? 2 : 1) * shared_ff * width : nullptr;
+  int32_t* const counts = n > SORT_PAIRS ? s.counts : nullptr;
+  if (counts != nullptr) LL_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * n_experts, st));
   if (int r = moe_route_only(x, w_router, bias, M, width, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, s.idx, s.weight,
-                             gate_row, s.gate, st))
+                             counts, counts != nullptr ? s.rank : nullptr, gate_row, s.gate, st))
     return r;
-  LL_CUDA(launch(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), 3 * sizeof(int32_t) * n_experts, st, true, (const int32_t*)s.idx, n, n_experts, s.offsets,
-                 s.order, s.perm));
+  if (counts != nullptr)
+    if (int r = moe_permute(s.idx, s.rank, counts, n, n_experts, s.offsets, s.perm, st)) return r;
+  LL_CUDA(launch(moe_sort_kernel, dim3(1), dim3(SORT_THREADS), 3 * sizeof(int32_t) * n_experts, st, true, (const int32_t*)s.idx, (const int32_t*)counts, n,
+                 n_experts, s.offsets, s.order, s.first, s.perm));
   LL_LAUNCH_OK("moe_sort_kernel");
   LL_CUDA(launch(moe_gather_rows_kernel, dim3((n + GR_WARPS - 1) / GR_WARPS), dim3(32 * GR_WARPS), 0, st, true, (const uint4*)x, (long long)(width / 8),
                  (const int32_t*)s.perm, top, (uint4*)s.xs, width / 8, n));
@@ -201,7 +231,7 @@ int ll_moe_prompt(const void* x, const float* w_router, const float* bias, const
     if (int r = mt_maps(ws_in, up, 1, shared_ff, width, x, M, &shared)) return r;
   MtParams p{};
   p.part[0] = mt_part(s.h, up, ff, width, ff, limit), p.part[1] = mt_part(s.hs, up, shared_ff, width, shared_ff, shared_limit);
-  p.offsets = s.offsets, p.perm = s.perm, p.order = s.order, p.X = n_experts, p.M = shared_ff ? M : 0, p.cuts = (p.M + MT_NMAX - 1) / MT_NMAX, p.early = 1;
+  p.offsets = s.offsets, p.perm = s.perm, p.order = s.order, p.first = s.first, p.X = n_experts, p.M = shared_ff ? M : 0, p.cuts = (p.M + MT_NMAX - 1) / MT_NMAX, p.early = 1;
   p.alpha = alpha, p.shift = mode == 2 ? 0.f : 1.f, p.word = wait_word();
   if (int r = up == 1 ? launch_moe_pair<1>(experts, shared, p, n, st) : launch_moe_pair<3>(experts, shared, p, n, st)) return r;
   // second ones

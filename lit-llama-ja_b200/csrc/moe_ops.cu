@@ -597,11 +597,17 @@ static int route_launch(const void* x, int dtype, const float* w_router, const f
 }
 
 int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
-                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
-                   cudaStream_t st) {
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   const void* gate_row, float* gate, cudaStream_t st) {
   if (int r = route_check(M, dim, n_experts, top, score, correction, n_groups, keep_groups, group_top)) return r;
   return route_launch(x, LL_BF16, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
-                      expert_w, nullptr, nullptr, gate_row, gate, st);
+                      expert_w, counts, rank, gate_row, gate, st);
+}
+
+int moe_permute(const int32_t* expert_idx, const int32_t* rank, const int32_t* counts, int n_pairs, int X, int32_t* offsets, int32_t* perm, cudaStream_t st) {
+  moe_permute_kernel<<<(n_pairs + 255) / 256, 256, sizeof(int32_t) * (X + 1), st>>>(expert_idx, rank, counts, n_pairs, X, offsets, perm);
+  LL_LAUNCH_OK("moe_permute_kernel");
+  return LL_OK;
 }
 
 // The combination of a prompt's rows in one chain of programmatic launches: whole 16-byte pieces, the gate's logits in fp32.
@@ -646,11 +652,7 @@ int ll_moe_route_choice(const void* x, int dtype, const float* w_router, const f
   if (int r = route_launch(x, dtype, w_router, bias, M, dim, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, expert_idx,
                            expert_w, counts, rank, nullptr, nullptr, st))
     return r;
-  const int n_pairs = M * top;
-  moe_permute_kernel<<<(n_pairs + 255) / 256, 256, sizeof(int32_t) * (n_experts + 1), st>>>(expert_idx, rank, counts, n_pairs,
-                                                                                          n_experts, offsets, perm);
-  LL_LAUNCH_OK("moe_permute_kernel");
-  return LL_OK;
+  return moe_permute(expert_idx, rank, counts, M * top, n_experts, offsets, perm, st);
 }
 
 int ll_moe_grouped_gemm(const void* a, int lda, const void* w, const int32_t* offsets, const int32_t* perm, int mode, int dtype,

@@ -15,8 +15,8 @@ namespace llb {
 
 // moe_ops.cu: the router alone
 int moe_route_only(const void* x, const float* w_router, const float* bias, int M, int dim, int n_experts, int top, int score, const float* correction,
-                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, const void* gate_row, float* gate,
-                   cudaStream_t st);
+                   float out_scale, int n_groups, int keep_groups, int group_top, int32_t* expert_idx, float* expert_w, int32_t* counts, int32_t* rank,
+                   const void* gate_row, float* gate, cudaStream_t st);
 
 namespace {
 
@@ -199,7 +199,7 @@ int ll_moe_step(const void* x, const float* w_router, const float* bias, const f
   cudaStream_t st = (cudaStream_t)stream;
   const MsScratch s = ms_carve(scratch, M, top, ff, shared_ff);
   if (int r = moe_route_only(x, w_router, bias, M, width, n_experts, top, score, correction, out_scale, n_groups, keep_groups, group_top, s.idx, s.weight,
-                             nullptr, nullptr, st))
+                             nullptr, nullptr, nullptr, nullptr, st))
     return r;
   typedef const __nv_bfloat16* B;
   const MsParams p{(B)x, (B)w_gu, (B)w_down, shared_ff ? (B)ws_in : nullptr, shared_ff ? (B)ws_down : nullptr, s.idx, s.weight, s.h, s.hs, s.gate,

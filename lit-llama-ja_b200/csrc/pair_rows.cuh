@@ -27,6 +27,8 @@ constexpr int MT_STAGES = 6, MT_NMAX = 256, MT_NSTEP = 32;
 constexpr int MT_A_BYTES = 128 * BK * 2, MT_B_BYTES = MT_NMAX / 2 * BK * 2;
 constexpr int MT_EPI_WARPS = 8, MT_THREADS = 64 + 32 * MT_EPI_WARPS, MT_OUT = 32 * 64;      // staging of a warp: 32 tokens of 64 bytes
 constexpr size_t MT_SMEM = (size_t)MT_STAGES * (MT_A_BYTES + MT_B_BYTES) + MT_EPI_WARPS * MT_OUT + (2 * MT_STAGES + 4) * 8 + 32 + 1024;
+constexpr int MT_TABLE = 2048;      // entries of a CTA's table of where experts' tiles begin
+constexpr size_t MT_TABLE_SMEM = (MT_TABLE + 1 + MT_THREADS / 32) * sizeof(int32_t);
 constexpr uint32_t MT_WAIT_LIMIT = 1u << 22;
 
 __device__ int g_pair_rows_error = 0;      // per file that instantiates the kernel
@@ -43,7 +45,9 @@ struct MtParams {
   const int32_t* offsets;
   const int32_t* perm;
   const int32_t* order;             // experts by falling size of their tiles, or null: as they stand
+  const int32_t* first;             // [X + 1] in that order: row tiles (of up to MT_NMAX rows) before an expert's, or null: every CTA makes a table
   int X, M;                         // M: rows of the shared expert (0: there is none)
+  int group, groups;                // experts of an entry of that table, and entries (launch_moe_pair)
   int cuts;                         // tiles that these rows are cut into
   int early;                        // the shared expert's operands are there before the kernels that this one waits for have ended
   float alpha, shift;
@@ -69,28 +73,43 @@ __device__ __forceinline__ bool mt_wait(uint64_t* bar, uint32_t parity, const Mt
 }
 
 // Walk over the tiles: the shared expert's, then the experts'; every role keeps its own.  Tile: 256 weight rows (column tile `ct`) x `cnt`
-// rows from `r0` on, `n` columns of the product.
+// rows from `r0` on, `n` columns of the product.  The expert of a tile is looked up in the table of where experts' row tiles begin, from the last one
+// on in steps that double.  (Expert by expert, two dependent loads and two divisions each, every role took half a us an expert: 2048 tokens, 256 experts of
+// 256 x 64, 219 us a layer where it takes 92; 700 tokens, 512 experts of 512 x 64 415 and 170.)
 struct MtWalk {
-  int k = -2, e = -1, first = 0, next = 0;      // place in the order, expert (-1: shared), its first tile, the one after its last
+  int k = -2, e = -1, base = 0, first = 0, next = 0;      // place in the order, expert (-1: shared), tiles before the experts', its first tile, the one after
   int row = 0, count = 0, tiles = 1, step = 0;
   int ct = 0, r0 = 0, cnt = 0, n = 0;
   static __host__ __device__ __forceinline__ int columns(int count, int tiles) { return ((count + tiles - 1) / tiles + MT_NSTEP - 1) / MT_NSTEP * MT_NSTEP; }
   template <int OUTS>
-  __device__ __forceinline__ bool seek(const MtParams& p, int t) {
-    while (t >= next) {
-      if (++k >= p.X) return false;
-      if (k < 0) {
-        e = -1, row = 0, count = p.M, tiles = p.cuts;
-      } else {
-        if (k == 0 && p.early) pdl_wait();      // (offsets, order, perm: the first look at what the kernels before have left)
+  static __device__ __forceinline__ int column_tiles(const MtPart& part) { return (part.N + 2 * OUTS - 1) / (2 * OUTS); }
+  template <int OUTS>
+  __device__ __forceinline__ bool seek(const MtParams& p, const int32_t* table, int t) {
+    if (k == -2) {
+      k = -1, count = p.M, tiles = p.cuts;
+      base = next = tiles * column_tiles<OUTS>(p.part[1]);
+      if (count > 0) step = columns(count, tiles);
+    }
+    if (t >= next) {
+      if (p.X == 0) return false;
+      if (k < 0 && p.early) pdl_wait();      // (offsets, order, first, perm: the first look at what the kernels before have left)
+      const int cols = column_tiles<OUTS>(p.part[0]), q = (t - base) / cols;
+      if (q >= table[p.groups]) return false;
+      int lo = k < 0 ? 0 : k / p.group, hop = 1;
+      for (; lo + hop < p.groups && table[lo + hop] <= q; hop *= 2) lo += hop;
+      for (; hop > 0; hop /= 2)
+        if (lo + hop < p.groups && table[lo + hop] <= q) lo += hop;
+      int f = table[lo];
+      for (k = lo * p.group;; ++k, f += tiles) {
         e = p.order != nullptr ? p.order[k] : k;
         row = p.offsets[e];
         count = p.offsets[e + 1] - row;
         tiles = (count + MT_NMAX - 1) / MT_NMAX;
+        if (q < f + tiles) break;
       }
-      first = next;
-      next += tiles * ((p.part[k < 0].N + 2 * OUTS - 1) / (2 * OUTS));
-      if (count > 0) step = columns(count, tiles);
+      first = base + f * cols;
+      next = first + tiles * cols;
+      step = columns(count, tiles);
     }
     const int q = t - first;
     ct = q / tiles;
@@ -101,6 +120,34 @@ struct MtWalk {
     return true;
   }
 };
+// The table of a CTA: row tiles before the experts of every entry, and of all; `sums`: a place per warp.  Ends with a barrier of the CTA.
+__device__ __forceinline__ void mt_make_table(const MtParams& p, int32_t* table, int32_t* sums) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = (p.groups + MT_THREADS - 1) / MT_THREADS, g0 = min(tid * per, p.groups);
+  const int g1 = min(g0 + per, p.groups);
+  auto row_tiles = [&](int g) {
+    int n = 0;
+    for (int e = g * p.group; e < min((g + 1) * p.group, p.X); ++e) n += (p.offsets[e + 1] - p.offsets[e] + MT_NMAX - 1) / MT_NMAX;
+    return n;
+  };
+  int own = 0;
+  for (int g = g0; g < g1; ++g) own += row_tiles(g);
+  int incl = own;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  if (lane == 31) sums[warp] = incl;
+  __syncthreads();
+  int before = incl - own;
+  for (int w = 0; w < MT_THREADS / 32; ++w) before += w < warp ? sums[w] : 0;
+  for (int g = g0; g < g1; ++g) {
+    table[g] = before;
+    before += row_tiles(g);
+  }
+  if (tid == MT_THREADS - 1) table[p.groups] = before;      // (the last thread: all entries stand before its own end)
+  __syncthreads();
+}
 // the i-th tile of a pair: to and fro, so that with tiles of falling size the pairs' sums are alike
 __device__ __forceinline__ int mt_tile(int i, int pair, int pairs) { return i * pairs + ((i & 1) ? pairs - 1 - pair : pair); }
 
@@ -177,6 +224,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
   uint64_t* acc_empty = acc_full + 2;              // [2], used in rank 0: both CTAs' warps arrive
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(acc_empty + 2);
   int* s_fail = reinterpret_cast<int*>(tmem_ptr + 1);
+  int32_t* s_table = reinterpret_cast<int32_t*>(s_fail + 1);      // [MT_TABLE + 1], then a place per warp
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = (int)cluster_rank();
@@ -202,6 +250,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   if (!p.early) pdl_wait();
   pdl_launch_dependents();
+  const int32_t* table = p.first;
+  if (p.X > 0 && p.first == nullptr) {
+    mt_make_table(p, s_table, s_table + MT_TABLE + 1);
+    table = s_table;
+  }
 
   if (warp == 0) {
     if (elect_one()) {
@@ -209,7 +262,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
       int s = 0;
       uint32_t ph = 1;
       bool ok = true;
-      for (int i = 0; ok && walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+      for (int i = 0; ok && walk.seek<OUTS>(p, table, mt_tile(i, pair, pairs)); ++i) {
         const bool dense = walk.e < 0;
         const MtPart& part = p.part[dense];
         const MtMaps& maps = dense ? shared : experts;
@@ -250,7 +303,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
       bool ok = true;
       int s = 0, i = 0;
       uint32_t ph = 0;
-      for (; rank == 0 && ok && walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+      for (; rank == 0 && ok && walk.seek<OUTS>(p, table, mt_tile(i, pair, pairs)); ++i) {
         const int nkb = p.part[walk.e < 0].nkb;
         const bool across = MODE == 0 && p.part[walk.e < 0].across != 0;      // 16 k are 16 rows of 128 bytes then, not 32 bytes of a row
         const uint64_t ad = across ? mt_desc_across(smem_u32(sa)) : smem_desc_sw128(smem_u32(sa)), astep = across ? 128 : 2;
@@ -279,7 +332,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MT_THREADS, 1)
     const uint32_t mine = stage + (uint32_t)(lane * DIMS * 2);
     MtWalk walk;
     int i = 0;
-    for (; walk.seek<OUTS>(p, mt_tile(i, pair, pairs)); ++i) {
+    for (; walk.seek<OUTS>(p, table, mt_tile(i, pair, pairs)); ++i) {
       const MtPart& out = p.part[walk.e < 0];
       const float limit = out.limit;
       const int n0 = (walk.ct * 2 + rank) * OUTS + quarter * DIMS;
@@ -386,18 +439,22 @@ int mt_weight_map(const void* w, int mode, int X, int N, int K, CUtensorMap* out
 }
 
 template <int MODE>
-int launch_moe_pair(const MtMaps& experts, const MtMaps& shared, const MtParams& p, int n_rows, cudaStream_t st) {
+int launch_moe_pair(const MtMaps& experts, const MtMaps& shared, MtParams p, int n_rows, cudaStream_t st) {
+  constexpr size_t smem = MT_SMEM + MT_TABLE_SMEM;
+  static_assert(smem <= 227 * 1024, "shared memory of a block");
   static PerDevice configured;
   if (!configured) {
-    LL_CUDA(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MT_SMEM));
+    LL_CUDA(cudaFuncSetAttribute(moe_gemm_pair_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured.mark();
   }
+  p.group = p.first != nullptr || p.X == 0 ? 1 : (p.X + MT_TABLE - 1) / MT_TABLE;
+  p.groups = (p.X + p.group - 1) / p.group;
   const int cols = MODE == 1 ? 128 : 256;
   const long long most = (long long)((p.part[0].N + cols - 1) / cols) * (n_rows / MT_NMAX + std::min(n_rows, p.X)) +
                          (long long)((p.part[1].N + cols - 1) / cols) * p.cuts;
   LL_CHECK_ARG(most < (1ll << 30), "moe_grouped_gemm_tc: too many tiles");
   const int pairs = sm_count() > 1 ? sm_count() / 2 : 1;
-  LL_CUDA(launch(moe_gemm_pair_kernel<MODE>, dim3(2 * (unsigned)std::min<long long>(most, pairs)), dim3(MT_THREADS), MT_SMEM, st, true, experts,
+  LL_CUDA(launch(moe_gemm_pair_kernel<MODE>, dim3(2 * (unsigned)std::min<long long>(most, pairs)), dim3(MT_THREADS), smem, st, true, experts,
                  shared, p));
   LL_LAUNCH_OK("moe_gemm_pair_kernel");
   return LL_OK;

@@ -41,6 +41,19 @@ TC_MIN_ROWS = int(os.environ.get("LLB200_MOE_TC_MIN_ROWS", "8"))
 TC_MIN_ROWS_PER_EXPERT = float(os.environ.get("LLB200_MOE_TC_MIN_ROWS_PER_EXPERT", "0.25"))
 
 
+def tc_least_rows(size: int, experts: int, shared: bool) -> int:
+    """Rows per expert from which the tcgen05 kernels take experts of ``size`` = width x ff numbers.  A tile is 256 weight rows whatever the tokens, so
+    many small experts with a few rows each are the mma.sync kernels' (16-row tiles, a CTA each) unless a shared expert's products come with them.
+    Graphed, us, mma.sync / tcgen05 at 2, 8, 16 and 64 rows an expert, four chosen, none shared: 32 experts of 512 x 256 25 / 28, 28 / 28, 37 / 28, 44 / 31,
+    of 1024 x 512 40 / 46, 42 / 46, 64 / 47, 83 / 53, of 1024 x 768 56 / 57, 59 / 58, 79 / 58, 91 / 64; 128 of 512 x 256 48 / 48, 58 / 68, 72 / 68,
+    105 / 82, of 1024 x 256 73 / 76, 87 / 95, 106 / 96, 165 / 114, of 1024 x 768 135 / 128, 163 / 155, 203 / 157, 292 / 180; with a shared one of 256,
+    128 of 1024 x 256 85 / 81, 98 / 95, 116 / 97, 174 / 120.  Smaller still, 256 of 256 x 64: 39 / 52, 48 / 68, 59 / 73, 114 / 132 (through the separate
+    calls 156 from 48 rows on), with a shared one 47 / 53, 57 / 69, 69 / 74, 125 / 136.  Eight experts: 23 / 24 to 29 / 27 at 8 rows."""
+    if experts > 64 and size <= 1 << 16:
+        return 48
+    return 16 if experts >= 16 and size < 3 << 18 and not shared else 0
+
+
 STEP_MAX_TOKENS, STEP_SMALL_EXPERT = 8, 1 << 22       # tokens of a step; ff * width
 STEP_REPEAT_BYTES = 300 << 20                         # of weights that a step reads for one token after another
 
@@ -171,10 +184,10 @@ class MoE(nn.Module):
 
     def takes_tensor_cores(self, n_rows: int, x_act: torch.Tensor) -> bool:
         """Whether a step of ``n_rows`` (token, choice) rows runs its expert GEMMs on the tcgen05 kernels: bfloat16, rows
-        that TMA can tile (16-byte multiples on 16-byte boundaries, the other kernels read any), and enough of them."""
+        that TMA can tile (16-byte multiples on 16-byte boundaries, the other kernels read any), and enough of them (``tc_least_rows``)."""
         s = self.spec
         return (x_act.dtype == torch.bfloat16 and s.width % 8 == 0 and s.ff % 8 == 0 and x_act.stride(0) % 8 == 0
-                and n_rows >= TC_MIN_ROWS and n_rows >= TC_MIN_ROWS_PER_EXPERT * s.experts
+                and n_rows >= TC_MIN_ROWS and n_rows >= max(TC_MIN_ROWS_PER_EXPERT, tc_least_rows(s.width * s.ff, s.experts, bool(s.shared_ff))) * s.experts
                 and (x_act.data_ptr() | self.w_gu.data_ptr() | self.w_down.data_ptr()) % 16 == 0 and N.has("ll_moe_grouped_gemm_tc"))
 
     def _one_call(self, entry: str, at, x_act: torch.Tensor, M: int, scratch_bytes: int) -> torch.Tensor:
@@ -217,10 +230,9 @@ class MoE(nn.Module):
         return self._rows(x_act, M)
 
     def _takes_prompt(self, x_act: torch.Tensor, M: int):
-        """More of them on the tcgen05 kernels in one call: the rows' addresses, or ``None``."""
+        """More of them, that take the tcgen05 kernels, in one call: the rows' addresses, or ``None``."""
         s = self.spec
-        if not (self.takes_tensor_cores(M * s.top, x_act) and N.has("ll_moe_prompt")
-                and N.call_ret("ll_moe_prompt_supported", M, s.width, s.experts, s.ff, s.shared_ff or 0)):
+        if not (N.has("ll_moe_prompt") and N.call_ret("ll_moe_prompt_supported", M, s.width, s.experts, s.ff, s.shared_ff or 0)):
             return None
         return self._rows(x_act, M)
 
@@ -229,7 +241,8 @@ class MoE(nn.Module):
         at = self._takes_step(x_act, M) if M <= STEP_MAX_TOKENS else None
         if at:
             return self._one_call("ll_moe_step", at, x_act, M, _step_scratch_bytes(M, s.experts, s.top, s.ff, s.shared_ff or 0))
-        at = self._takes_prompt(x_act, M)
+        tensor_cores = self.takes_tensor_cores(M * s.top, x_act)
+        at = self._takes_prompt(x_act, M) if tensor_cores else None
         if at:
             return self._one_call("ll_moe_prompt", at, x_act, M, N.call_ret("ll_moe_prompt_scratch_bytes", M, s.width, s.experts, s.top, s.ff,
                                                                              s.shared_ff or 0))
@@ -239,7 +252,7 @@ class MoE(nn.Module):
         n = M * s.top
         h = torch.empty((n, s.ff), dtype=dtype, device=dev)
         y = torch.empty((n, s.width), dtype=dtype, device=dev)
-        if self.takes_tensor_cores(n, x_act):
+        if tensor_cores:
             xs = torch.empty((n, s.width), dtype=dtype, device=dev)
             N.call("ll_moe_gather_rows", N.ptr(x_act), x_act.stride(0), N.ptr(perm), s.top, n, s.width, N.ptr(xs), st)
             N.call("ll_moe_grouped_gemm_tc", N.ptr(xs), N.ptr(self.w_gu), N.ptr(offsets), N.ptr(perm), self.up_mode, n, s.experts, s.ff,

@@ -36,3 +36,10 @@ def test_form_of_a_latent_layer_in_one_call(native, B, T, S, end, v, width, want
     cache = torch.zeros((B, S, m.spec.row), dtype=torch.bfloat16)
     assert m._layer_form(B, T, cache, 1, end) == want
 
+
+def test_rows_from_which_experts_take_the_tensor_cores():
+    from lit_llama.moe import tc_least_rows
+
+    assert tc_least_rows(2048 * 1024, 32, False) == 0 == tc_least_rows(1024 * 768, 256, False) == tc_least_rows(512 * 256, 128, True)
+    assert tc_least_rows(1024 * 512, 32, False) == 16 and tc_least_rows(64 * 24, 8, False) == 0
+    assert tc_least_rows(256 * 256, 128, True) == 48 == tc_least_rows(256 * 64, 256, False)
