@@ -365,8 +365,8 @@ class LLaMA(nn.Module):
             and bool(N.call_ret("ll_causal_attn_supported", self.config.head_size, T))
         if use_cache and kernel:
             N.require_cuda(input_pos)
-            if input_pos.shape != (T,):
-                raise RuntimeError(f"{T} tokens at positions of shape {tuple(input_pos.shape)}")
+            if input_pos.shape != (T,) or input_pos.dtype not in (torch.int32, torch.int64):
+                raise RuntimeError(f"{T} tokens at positions of shape {tuple(input_pos.shape)} in {input_pos.dtype} (int32 or int64)")
             pos_ids, slots, seen = torch.empty((3, T), dtype=torch.int32, device=dev).unbind(0)
             N.call("ll_prompt_pos", N.ptr(pos_ids), N.ptr(slots), N.ptr(seen), N.ptr(input_pos.to(torch.int64).contiguous()), T, max_seq_length, block_size,
                    N.stream())
