@@ -367,6 +367,10 @@ class LLaMA(nn.Module):
             N.require_cuda(input_pos)
             if input_pos.shape != (T,) or input_pos.dtype not in (torch.int32, torch.int64):
                 raise RuntimeError(f"{T} tokens at positions of shape {tuple(input_pos.shape)} in {input_pos.dtype} (int32 or int64)")
+            if self.kv_caches:                 # the kernels take their strides from the call: nothing else looks whether the caches are those
+                k = self.kv_caches[0][0]
+                if k.shape != (B, self.transformer.h[0].attn.n_head, max_seq_length, self.config.head_size) or k.dtype is not torch.bfloat16:
+                    raise RuntimeError(f"{B} sequences of up to {max_seq_length} tokens over a cache of shape {tuple(k.shape)} in {k.dtype}")
             pos_ids, slots, seen = torch.empty((3, T), dtype=torch.int32, device=dev).unbind(0)
             N.call("ll_prompt_pos", N.ptr(pos_ids), N.ptr(slots), N.ptr(seen), N.ptr(input_pos.to(torch.int64).contiguous()), T, max_seq_length, block_size,
                    N.stream())

@@ -26,3 +26,20 @@ def test_positions_are_whole_numbers_of_32_or_64_bits(dtype):
     m.reset_cache()
     with pytest.raises(RuntimeError):
         m(idx, 16, torch.arange(5, device="cuda").to(dtype))
+
+
+@torch.no_grad()
+def test_caches_of_another_shape_are_refused():
+    """Caches made for another length, batch or dtype than a prompt's, before anything is written to them."""
+    m, idx, pos = _model(), torch.arange(6, device="cuda")[None], torch.arange(6, device="cuda")
+    m(idx, 16, pos)
+    held = [[t.clone() for t in kv] for kv in m.kv_caches]
+    for args in ((idx, 32, pos), (idx, 12, pos), (idx.repeat(2, 1), 16, pos)):
+        with pytest.raises(RuntimeError, match="cache"):
+            m(*args)
+    assert all(torch.equal(a, b) for kv, kv0 in zip(m.kv_caches, held) for a, b in zip(kv, kv0))
+    m.kv_caches = [tuple(t.float() for t in kv) for kv in m.kv_caches]
+    with pytest.raises(RuntimeError, match="cache"):
+        m(idx, 16, pos)
+    m.reset_cache()
+    m(idx, 32, pos)
