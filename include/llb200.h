@@ -412,7 +412,8 @@ LL_API int ll_advance_pos(int32_t* pos, int cache_len, int max_pos, ll_stream st
  * host sync (ref: model.py:101-104 index_select by input_pos). */
 LL_API int ll_set_pos(int32_t* pos, const int64_t* input_pos, int cache_len, int max_pos, ll_stream stream);
 /* The same for T tokens at input_pos [T]: pos_ids, slots = pos % cache_len, seen = min(pos, cache_len - 1).  A position outside 0 .. max_pos - 1 is
- * reported by a later launch or ll_wait_check (LL_ERR_WAIT). */
+ * reported by a later launch or ll_wait_check (LL_ERR_WAIT); its token gets pos_ids 0, slots -1, seen 0, with which ll_rope_kv_append stores no key and
+ * no value and makes queries that are no numbers. */
 LL_API int ll_prompt_pos(int32_t* pos_ids, int32_t* slots, int32_t* seen, const int64_t* input_pos, int T, int cache_len, int max_pos, ll_stream stream);
 
 /* ---------------------------------------------------------------------------------------

@@ -147,6 +147,7 @@ __global__ void embed_ssq_kernel(const __nv_bfloat16* __restrict__ wte, const in
 }
 
 // ---------------------------------------------------------------- RoPE + KV append (rows R, A)
+// A token without a slot (-1: its position was reported, prompt_pos_kernel) stores no key and no value, and its queries are no numbers.
 // grid (T, B*n_head), block head_size/2 threads
 template <typename T>
 __global__ void rope_kv_kernel(const T* __restrict__ qkv, const float* __restrict__ rope,
@@ -164,6 +165,11 @@ __global__ void rope_kv_kernel(const T* __restrict__ qkv, const float* __restric
   {
     const float x0 = dt<T>::ld(row, head * hs + d), x1 = dt<T>::ld(row, head * hs + d + 1);
     T* o = q_out + (((size_t)b * n_head + head) * Tn + t) * hs;
+    if (slot < 0) {
+      dt<T>::st(o, d, NAN);
+      dt<T>::st(o, d + 1, NAN);
+      return;
+    }
     dt<T>::st(o, d, __fsub_rn(__fmul_rn(x0, cs.x), __fmul_rn(x1, cs.y)));
     dt<T>::st(o, d + 1, __fadd_rn(__fmul_rn(x1, cs.x), __fmul_rn(x0, cs.y)));
   }
@@ -189,11 +195,14 @@ __global__ void __launch_bounds__(256) rope_kv_vec_kernel(const __nv_bfloat16* _
   const uint4* row = reinterpret_cast<const uint4*>(qkv + (((size_t)b * Tn + t) * 3 + which) * E);
   const float* cs = rope + (size_t)pos_ids[t] * hs;
   const int slot = slots[t];
+  if (slot < 0 && which > 0) return;
 #pragma unroll 2
   for (int i = threadIdx.x; i < per; i += blockDim.x) {
     const int e = i * 8, head = e / hs, d = e - head * hs;
     uint4 u = row[i];
-    if (which < 2) {
+    if (slot < 0) {
+      u = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+    } else if (which < 2) {
       const float4 c0 = *reinterpret_cast<const float4*>(cs + d), c1 = *reinterpret_cast<const float4*>(cs + d + 4);
       const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
       uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -790,16 +799,16 @@ __global__ void apply_rope_kernel(const T* __restrict__ x, const float* __restri
 }
 
 // Positions of a prompt's tokens: rotary rows, cache slots, and the last slot that each token sees.  A position outside the table is reported where
-// the next launch looks (and kept inside, so that nothing is read or written out of range).
+// the next launch looks; its token gets row 0 and no slot, so that no other token's row of the cache is written for it.
 __global__ void prompt_pos_kernel(int32_t* __restrict__ pos_ids, int32_t* __restrict__ slots, int32_t* __restrict__ seen, const int64_t* __restrict__ input_pos,
                                   int T, int S, int max_pos, int* word) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
     const int64_t p = input_pos[t];
-    if (p < 0 || p >= (int64_t)max_pos) wait_ran_out(word, 700);
-    const int q = (int)(p < 0 ? 0 : p >= (int64_t)max_pos ? max_pos - 1 : p);
-    pos_ids[t] = q;
-    slots[t] = q % S;
-    seen[t] = min(q, S - 1);
+    const bool in = p >= 0 && p < (int64_t)max_pos;
+    if (!in) wait_ran_out(word, 700);
+    pos_ids[t] = in ? (int)p : 0;
+    slots[t] = in ? (int)p % S : -1;
+    seen[t] = in ? min((int)p, S - 1) : 0;
   }
 }
 

@@ -298,6 +298,9 @@ class LLaMA(nn.Module):
     # ------------------------------------------------------------------ forward (row M)
     def forward(self, idx: torch.Tensor, max_seq_length: Optional[int] = None,
                 input_pos: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """ref: model.py:84-151.  Positions are looked at on the device: one of a prompt that lies outside 0 .. block_size - 1 raises at a later launch,
+        or, where the caller has synchronised, at ``_native.check_waits()``.  Until then its token's logits are no numbers; the cache's rows are those of
+        the other tokens."""
         N.require_cuda(idx)
         B, T = idx.size()
         block_size = self.config.block_size
