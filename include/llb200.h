@@ -215,9 +215,15 @@ LL_API int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const voi
                               const void* scales2, const void* zeros2, const void* bias2, const void* x, void* h, int M, int N, int K, int group,
                               int tile_rows, int grid, ll_stream stream);
 /* Both with scratch (ll_int4_rows_scratch_bytes, layers: 1, or 2 for the gated form; on a 16-byte boundary, of any contents; null where that is
- * 0): the tiles that would leave pairs of SMs idle in a last wave are cut along k into `parts` (0: as many as pay; more than two
- * parts a pair: none), whose sums meet in fp32, in the order of k.  tile_rows, grid and parts the same for the size and the launch. */
+ * 0; one call's alone until its kernels have ended): the tiles that would leave pairs of SMs idle in a last wave are cut along k into `parts` (0: as
+ * many as pay; more than two parts a pair: none), whose sums meet in fp32, in the order of k.  tile_rows, grid and parts the same for the size and the
+ * launch; a scratch of fewer bytes than the launch needs is refused.  The forms without a size take it on trust. */
 LL_API size_t ll_int4_rows_scratch_bytes(int M, int N, int K, int layers, int tile_rows, int grid, int parts);
+LL_API int ll_int4_rows_sized(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch,
+                              size_t scratch_bytes, int M, int N, int K, int group, int tile_rows, int grid, int parts, ll_stream stream);
+LL_API int ll_int4_rows_gated_sized(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2,
+                                    const void* scales2, const void* zeros2, const void* bias2, const void* x, void* h, void* scratch,
+                                    size_t scratch_bytes, int M, int N, int K, int group, int tile_rows, int grid, int parts, ll_stream stream);
 LL_API int ll_int4_rows_split(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch,
                               int M, int N, int K, int group, int tile_rows, int grid, int parts, ll_stream stream);
 LL_API int ll_int4_rows_gated_split(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2,

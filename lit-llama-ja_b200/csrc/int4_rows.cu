@@ -542,12 +542,17 @@ __global__ void __launch_bounds__(GATED ? 128 : 256) int4_rows_sum_kernel(const 
 }
 
 template <bool GATED>
-int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p, int K, void* scratch, int tile_rows, int grid, int parts, cudaStream_t st) {
+int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p, int K, void* scratch, size_t scratch_bytes, int tile_rows, int grid,
+              int parts, cudaStream_t st) {
   constexpr int TILE_N = GATED ? 128 : 256;
   const int pairs = r4_pairs(grid);
   LL_CHECK_ARG((long long)((p.M + 127) / 128) * ((p.N + TILE_N - 1) / TILE_N) < (1ll << 30), "int4_rows: too many tiles");
   const R4Plan q = r4_plan(p.M, p.N, p.steps, TILE_N, pairs, tile_rows, parts, scratch != nullptr);
   p.bn = q.bn, p.full = q.full, p.parts = q.parts;
+  p.mtiles = (p.M + p.bn - 1) / p.bn;
+  p.tiles = r4_tiles(p.M, p.N, TILE_N, p.bn);
+  LL_CHECK_ARG(scratch == nullptr || scratch_bytes >= r4_scratch_bytes(q, p.tiles), "int4_rows: scratch of %zu bytes, %zu are needed", scratch_bytes,
+               r4_scratch_bytes(q, p.tiles));
   p.xst = R4_XBYTES / (p.bn * 128);
   p.wide = r4_wide(p.scales[0], p.zeros[0], p.scales[1], p.zeros[1], p.G, p.steps_per_group);
   CUtensorMap mw0, mw1, mx, my;
@@ -560,8 +565,6 @@ int r4_launch(const uint8_t* qw0, const uint8_t* qw1, const void* x, R4Params p,
     LL_CUDA(cudaFuncSetAttribute(int4_rows_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, R4_SMEM));
     configured.mark();
   }
-  p.mtiles = (p.M + p.bn - 1) / p.bn;
-  p.tiles = r4_tiles(p.M, p.N, TILE_N, p.bn);
   p.word = wait_word();
   int blocks = p.tiles < pairs ? p.tiles : pairs;
   const int cut = p.tiles - q.full;
@@ -605,6 +608,11 @@ size_t ll_int4_rows_scratch_bytes(int M, int N, int K, int layers, int tile_rows
 
 int ll_int4_rows_split(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch, int M, int N,
                        int K, int group, int tile_rows, int grid, int parts, ll_stream stream) {
+  return ll_int4_rows_sized(qw, scales, zeros, x, bias, y, scratch, SIZE_MAX, M, N, K, group, tile_rows, grid, parts, stream);
+}
+
+int ll_int4_rows_sized(const uint8_t* qw, const void* scales, const void* zeros, const void* x, const void* bias, void* y, void* scratch,
+                       size_t scratch_bytes, int M, int N, int K, int group, int tile_rows, int grid, int parts, ll_stream stream) {
   LL_CHECK_ARG(qw && scales && zeros && x && y && M > 0, "int4_rows: null pointer or no rows");
   if (!ll_int4_rows_supported(N, K, group)) {
     set_error("int4_rows needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
@@ -617,7 +625,7 @@ int ll_int4_rows_split(const uint8_t* qw, const void* scales, const void* zeros,
   p.scales[0] = p.scales[1] = (const __nv_bfloat16*)scales, p.zeros[0] = p.zeros[1] = (const __nv_bfloat16*)zeros;
   p.bias[0] = p.bias[1] = (const __nv_bfloat16*)bias, p.y = (__nv_bfloat16*)y;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
-  return r4_launch<false>(qw, qw, x, p, K, scratch, tile_rows, grid, parts, (cudaStream_t)stream);
+  return r4_launch<false>(qw, qw, x, p, K, scratch, scratch_bytes, tile_rows, grid, parts, (cudaStream_t)stream);
 }
 
 int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
@@ -629,6 +637,13 @@ int ll_int4_rows_gated(const uint8_t* qw1, const void* scales1, const void* zero
 int ll_int4_rows_gated_split(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
                              const void* zeros2, const void* bias2, const void* x, void* h, void* scratch, int M, int N, int K, int group,
                              int tile_rows, int grid, int parts, ll_stream stream) {
+  return ll_int4_rows_gated_sized(qw1, scales1, zeros1, bias1, qw2, scales2, zeros2, bias2, x, h, scratch, SIZE_MAX, M, N, K, group, tile_rows, grid, parts,
+                                  stream);
+}
+
+int ll_int4_rows_gated_sized(const uint8_t* qw1, const void* scales1, const void* zeros1, const void* bias1, const uint8_t* qw2, const void* scales2,
+                             const void* zeros2, const void* bias2, const void* x, void* h, void* scratch, size_t scratch_bytes, int M, int N, int K,
+                             int group, int tile_rows, int grid, int parts, ll_stream stream) {
   LL_CHECK_ARG(qw1 && scales1 && zeros1 && qw2 && scales2 && zeros2 && x && h && M > 0, "int4_rows_gated: null pointer or no rows");
   if (!ll_int4_rows_supported(N, K, group)) {
     set_error("int4_rows_gated needs N %% 16 == 0 and group %% 128 == 0 (N=%d K=%d group=%d)", N, K, group);
@@ -642,7 +657,7 @@ int ll_int4_rows_gated_split(const uint8_t* qw1, const void* scales1, const void
   p.scales[1] = (const __nv_bfloat16*)scales2, p.zeros[1] = (const __nv_bfloat16*)zeros2, p.bias[1] = (const __nv_bfloat16*)bias2;
   p.y = (__nv_bfloat16*)h;
   p.M = M, p.N = N, p.steps = K / R4_K, p.G = K / group, p.steps_per_group = group / R4_K;
-  return r4_launch<true>(qw1, qw2, x, p, K, scratch, tile_rows, grid, parts, (cudaStream_t)stream);
+  return r4_launch<true>(qw1, qw2, x, p, K, scratch, scratch_bytes, tile_rows, grid, parts, (cudaStream_t)stream);
 }
 
 // 0, or the code of the first bounded wait that ran out in this file's kernel.  Synchronises the device.

@@ -91,6 +91,8 @@ EXPORTS = {
     "ll_int4_rows_form": ([vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_gated": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_scratch_bytes": ([i32, i32, i32, i32, i32, i32, i32], C.c_size_t),
+    "ll_int4_rows_sized": ([vp, vp, vp, vp, vp, vp, vp, sz_t, i32, i32, i32, i32, i32, i32, i32, vp], C.c_int),
+    "ll_int4_rows_gated_sized": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, sz_t, i32, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_split": ([vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_gated_split": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp], C.c_int),
     "ll_int4_rows_error": ([], C.c_int),

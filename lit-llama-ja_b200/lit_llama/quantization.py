@@ -265,8 +265,8 @@ class ColBlockQuantizedLinear(torch.nn.Module):
             nbytes = _rows_scratch_bytes(M, Nout, K, 1)
             if nbytes:                         # (a last wave of tiles that pays to be cut along k)
                 scratch = _call_scratch(x, nbytes)
-                N.call("ll_int4_rows_split", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y),
-                       N.ptr(scratch), M, Nout, K, self.tile_cols, 0, 0, 0, N.stream())
+                N.call("ll_int4_rows_sized", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y),
+                       N.ptr(scratch), nbytes, M, Nout, K, self.tile_cols, 0, 0, 0, N.stream())
             else:
                 N.call("ll_int4_rows", N.ptr(qw), N.ptr(self.scales), N.ptr(self.zeros), N.ptr(x), N.ptr(self.bias), N.ptr(y), M, Nout, K,
                        self.tile_cols, N.stream())
@@ -369,8 +369,9 @@ def gated_pair(fc1: torch.nn.Module, fc2: torch.nn.Module, inp: torch.Tensor):
         N.require_cuda(q1, q2)
         nbytes = _rows_scratch_bytes(M, Nout, K, 2)
         scratch = _call_scratch(x, nbytes) if nbytes else None
-        N.call("ll_int4_rows_gated_split", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
-               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), N.ptr(scratch), M, Nout, K, fc1.tile_cols, 0, 0, 0, N.stream())
+        N.call("ll_int4_rows_gated_sized", N.ptr(q1), N.ptr(fc1.scales), N.ptr(fc1.zeros), N.ptr(fc1.bias), N.ptr(q2), N.ptr(fc2.scales),
+               N.ptr(fc2.zeros), N.ptr(fc2.bias), N.ptr(x), N.ptr(h), N.ptr(scratch), nbytes, M, Nout, K, fc1.tile_cols, 0, 0, 0,
+               N.stream())
     else:
         w1, w2 = fc1.get_weight(dtype=x.dtype), fc2.get_weight(dtype=x.dtype)
         N.call("ll_gemm_bf16_gated", N.ptr(x), N.ptr(w1), N.ptr(fc1.bias), N.ptr(w2), N.ptr(fc2.bias), N.ptr(h), M, Nout, K, N.stream())

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 # entry -> where its scratch stands among the arguments
-SCRATCH = {"ll_int4_rows_split": 6, "ll_int4_rows_gated_split": 10}
+SCRATCH = {"ll_int4_rows_sized": 6, "ll_int4_rows_gated_sized": 10}
 
 
 @pytest.fixture
@@ -61,3 +61,16 @@ def test_cut_tiles_of_gated_prompts(library):
     l1, l2, x = _int4(11008, 4096), _int4(11008, 4096), torch.zeros((300, 4096), dtype=torch.bfloat16)
     rows = SimpleNamespace(shape=x.shape, device=SimpleNamespace(type="cuda"), reshape=x.reshape)
     assert _two_at_once(library, lambda: gated_pair(l1, l2, rows))
+
+
+@pytest.mark.parametrize("layers", [1, 2])
+def test_a_scratch_that_is_too_small_is_refused(layers):
+    """One byte less than the launch needs: nothing is launched (the addresses are never used)."""
+    from lit_llama import _native as N
+
+    M, Nout, K = 300, 11008 if layers == 2 else 1024, 4096 if layers == 2 else 11008
+    need = N.call_ret("ll_int4_rows_scratch_bytes", M, Nout, K, layers, 0, 0, 0)
+    assert need > 0
+    entry, pointers = ("ll_int4_rows_gated_sized", 11) if layers == 2 else ("ll_int4_rows_sized", 7)
+    with pytest.raises(RuntimeError, match=f"scratch of {need - 1} bytes"):
+        N.call(entry, *([1 << 20] * pointers), need - 1, M, Nout, K, 128, 0, 0, 0, None)
