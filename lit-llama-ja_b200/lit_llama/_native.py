@@ -278,7 +278,7 @@ def call_ret(name: str, *args):
 
 def require_cuda(*tensors: torch.Tensor) -> None:
     for t in tensors:
-        if t is not None and t.device.type != "cuda":
+        if t is not None and not t.is_cuda:
             raise RuntimeError(
                 "lit-llama-ja_b200 computes on CUDA (sm_100a) only - there is no CPU fallback; "
                 f"got a tensor on {t.device}"

@@ -9,6 +9,8 @@ from __future__ import annotations
 
 import functools
 import math
+import threading
+import weakref
 
 import torch
 
@@ -514,18 +516,22 @@ def _int8_gated_pair(fc1: Linear8bitLt, fc2: Linear8bitLt, inp: torch.Tensor):
     return h.view(inp.shape[:-1] + (Nout,))
 
 
-_INT8_WS: dict = {}
+_INT8_WS: dict = {}                            # (thread, device, stream) -> buffer
 
 
 def _int8_workspace(device, nbytes: int) -> torch.Tensor:
-    """Per-(device, stream) scratch of the int8 linear (kernels on one stream are ordered).  An outgrown buffer stays: a graph captured with
-    its address writes to it at every replay.  Each is at least twice the one before, so that together they stay below twice the largest."""
-    key = (device.index, N.stream())
-    held = _INT8_WS.get(key)
-    if held is None or held[-1].numel() < nbytes:
-        held = _INT8_WS.setdefault(key, [])
-        held.append(torch.empty(max(nbytes + 256, 2 * held[-1].numel() if held else 0), dtype=torch.uint8, device=device))
-    return held[-1]
+    """Scratch of llm.int8 layers and of int4 batches, kept from call to call: one buffer for what a thread launches on a stream, since that runs in
+    order.  (The launches of two threads on one stream can alternate: a call is several, and the interpreter is let go during it.)  A captured call
+    has memory of its graph's own: graphs captured on one stream can be replayed on two."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    key = (threading.get_ident(), device.index, N.stream())
+    ws = _INT8_WS.get(key)
+    if ws is None:
+        weakref.finalize(threading.current_thread(), _INT8_WS.pop, key, None)      # a thread's buffers go with it
+    if ws is None or ws.numel() < nbytes:      # (an outgrown one goes back to the stream that it was made on, behind the calls that used it)
+        ws = _INT8_WS[key] = torch.empty(max(nbytes + 256, 2 * ws.numel() if ws is not None else 0), dtype=torch.uint8, device=device)
+    return ws
 
 
 # --------------------------------------------------------------------------------------- row Z

@@ -6,7 +6,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-KINDS = ["rows", "gated_rows"]
+KINDS = ["rows", "gated_rows", "batch", "gated_batch", "int8", "gated_int8", "int8_prompt"]
 
 
 def _int4(N, K, seed):
@@ -20,14 +20,24 @@ def _int4(N, K, seed):
     return lin
 
 
+def _int8(N, K, seed):
+    from lit_llama.quantization import Linear8bitLt
+
+    lin = Linear8bitLt(K, N, bias=False, device="cuda", dtype=torch.bfloat16)
+    lin.load_state_dict({"weight": torch.randn((N, K), generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda") * 0.05})
+    return lin
+
+
 def _calls(kind):
     """Two calls of the same sizes on different rows."""
     from lit_llama.quantization import gated_pair
 
     g = torch.Generator(device="cuda").manual_seed(1)
-    M, N, K = {"rows": (300, 1024, 11008), "gated_rows": (300, 11008, 4096)}[kind]
-    layers = [_int4(N, K, i) for i in range(2 if "gated" in kind else 1)]
+    M, N, K = {"rows": (300, 1024, 11008), "gated_rows": (300, 11008, 4096), "int8_prompt": (130, 1024, 2048)}.get(kind, (32, 1024, 2048))
+    layers = [(_int8 if "int8" in kind else _int4)(N, K, i) for i in range(2 if "gated" in kind else 1)]
     xs = [torch.randn((M, K), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    for i, x in enumerate(xs):
+        x[:, 7 * i: 7 * i + 3] *= 30.0                    # outlier features, others in either call
     run = (lambda x: gated_pair(*layers, x)) if "gated" in kind else layers[0]
     return [lambda x=x: run(x) for x in xs]
 
