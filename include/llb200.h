@@ -757,7 +757,9 @@ LL_API int ll_qk_rotary_append(const void* q, int q_stride, const void* k, int k
 /* s_h(i,j) = scale q_h(i).k_g(j), then cap tanh(s / cap) (softcap 0: none); j visible when j <= i, (window 0 or i - j < window),
  * (chunk 0 or j / chunk == i / chunk); softmax with exp(sink[h]) added to the denominator (sink NULL: none); o_h = sum_j w v_g(j),
  * times sigmoid(gate[m][h*vdim + c]) (gate NULL: none) -> y [B*T][H*vdim].  form 0: chosen by shape and dtype; 1: the fp32
- * form.  splits > 1 cuts every query's keys into that many ranges (fp32 form; scratch: ll_softmax_attn_scratch_bytes). */
+ * form.  splits > 1 cuts every query's keys into that many ranges (fp32 form; scratch: ll_softmax_attn_scratch_bytes).  Several bf16 queries under
+ * a cap of up to 55 (the tensor-core form, whose weights the cap then bounds instead of a running maximum) take values below
+ * 2^(127 - 1.45 cap) / keys: 2^43 with a cap of 50 and 2048 keys. */
 LL_API size_t ll_softmax_attn_scratch_bytes(int M, int H, int vdim, int splits);
 LL_API int ll_softmax_attn(const void* q, int q_stride, const void* gate, int gate_stride, const void* kc, const void* vc, int dtype,
                            const int32_t* pos_ids, const float* sink, float scale, float softcap, int B, int T, int H, int G, int dim,

@@ -11,7 +11,8 @@
 // weights lie where the scores were (MMAs of one thread run in issue order).  The running maximum only moves when a row's scores
 // outgrow it by 2^8: the accumulator is then rescaled in place, which after the first blocks of a row hardly ever happens; the
 // result does not depend on it.  Capped scores have a bound of their own: where it is at most 2^80 they need no maximum, and the two threads
-// of a row nothing from one another before the end.
+// of a row nothing from one another before the end.  Weights are then up to 2^c (c = cap * log2(e)) and not 2^8, which the fp32 sums hold while values are
+// below 2^(127 - c) / keys and (what is not lost) above 2^(c - 118): with a cap of 50 and 2048 keys 2^44 and 2^-46, with the largest of 55 2^36 and 2^-38.
 // Keys are addressed by position in a ring (slot = position % ring): a block of keys ends where the ring wraps.  Rows past the
 // last key of the step may hold anything: their scores are masked and their value rows are cleared in shared memory.
 //
@@ -58,7 +59,7 @@ constexpr int AT_QBOX = AT_Q * 64 * 2, AT_KBOX = AT_K * 64 * 2;      // TMA boxe
 constexpr uint32_t AT_WAIT_LIMIT = 1u << 20;
 constexpr float AT_LOG2E = 1.4426950408889634f;
 constexpr float AT_SLACK = 8.f;                       // a row's scores may outgrow its reference by 2^8 before it moves
-constexpr float AT_BOUND = 80.f;                      // scores that a cap keeps within 2^-80 .. 2^80 need no reference
+constexpr float AT_BOUND = 80.f;                      // scores that a cap keeps within 2^-80 .. 2^80 need no reference (what that leaves to values: above)
 
 __device__ int g_attn_tc_error = 0;     // per file that instantiates the kernel: its entry asks for it (attn_tc_error)
 
