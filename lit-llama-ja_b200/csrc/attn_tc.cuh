@@ -243,7 +243,6 @@ template <int NB1, int NB2, int NBV, int TERMS, bool CAP, bool BIAS>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2,
                                                                const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_k2,
                                                                const __grid_constant__ CUtensorMap map_v, const AtParams p) {
-  pdl_launch_dependents();
   using Shape = AtShape<NB1, NB2, NBV>;
   constexpr int NB = Shape::NB, KS = Shape::KS, VS = Shape::VS, DV = NBV * 64;
   constexpr uint32_t TM_S = 0, TM_O = 256;            // per tile: two score buffers of 64 columns; 128 accumulator columns
@@ -294,6 +293,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
+  // (Not before the block has its tensor memory: a kernel let in that fits beside it could take that first, and then waits for this one's end.)
+  pdl_launch_dependents();
   if (warp == AT_WARPS && elect_one()) {                // the queries do not depend on the positions
     const int tiles = tq1 < p.T ? 2 : 1;
     mbar_expect_tx(q_full, (uint32_t)(tiles * NB * AT_QBOX));
