@@ -17,8 +17,9 @@
 // last key of the step may hold anything: their scores are masked and their value rows are cleared in shared memory.
 //
 // What bounds it is the softmax: a row's chain (load, maximum, exponent, split, store) runs at one instruction in four clocks
-// for a warp on its own, so a row has two threads and a scheduler four such warps.  2048 queries, 16 heads of 128, two terms, us: 52 (capped 68)
-// with neighbouring tiles, one barrier of a tile's 256 threads a block of keys and a running maximum for capped scores as well; 40 (45) now.
+// for a warp on its own, so a row has two threads and a scheduler four such warps.  2048 queries, 16 heads of 128, two terms, us: 46 (capped at 50 64, at 80
+// 65) with neighbouring tiles, one barrier of a tile's 256 threads a block of keys and a running maximum for all capped scores; 37 (40, 47) now.  Bounded and
+// other capped scores are two kernels: one for both was a tenth slower for either.
 // Blocks of 128 keys with one buffer of scores a tile (no second one fits beside the accumulators): 53 and 60, a tile's chain of weights,
 // P V and the next scores being what it waits for.
 // Every wait is bounded; one that runs out records a code, all roles stop, copies in flight are waited for, tensor memory is freed.
@@ -238,8 +239,9 @@ struct AtShape {
   static constexpr int SMEM = 2 * NB * AT_QBOX + KS * NB * AT_KBOX + VS * NBV * AT_KBOX + 512 + 4 * AT_Q * 4 + 1024;
 };
 
-// TERMS: bf16 terms of a weight.  CAP: capped scores; BIAS: distance bias.
-template <int NB1, int NB2, int NBV, int TERMS, bool CAP, bool BIAS>
+// TERMS: bf16 terms of a weight.  CAP: scores are capped, and the cap bounds their weights (AT_BOUNDED) or does not; BIAS: distance bias.
+enum AtCap { AT_UNCAPPED, AT_BOUNDED, AT_CAPPED };
+template <int NB1, int NB2, int NBV, int TERMS, AtCap CAP, bool BIAS>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2,
                                                                const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_k2,
                                                                const __grid_constant__ CUtensorMap map_v, const AtParams p) {
@@ -441,7 +443,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     float* const mine = s_x + (tile * 2 + half) * AT_Q + row;
     const float* const other = s_x + (tile * 2 + (half ^ 1)) * AT_Q + row;
     const int bar = 1 + tile * 4 + (warp & 3);
-    const bool bounded = CAP && cap2 <= AT_BOUND;
+    constexpr bool bounded = CAP == AT_BOUNDED;
     float ref = bounded ? 0.f : -INFINITY;
     f2 sum2[2] = {f2_of(0.f, 0.f), f2_of(0.f, 0.f)};
     uint32_t n = 0;
@@ -470,11 +472,19 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             if (e < cmin || e > cmax) sr[e] = bounded ? 0u : __float_as_uint(-INFINITY);
         }
         float mx = 0.f;
+        bool poly = bounded;
         if (!bounded) {
           float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
           for (int e = 0; e < AT_C; e += 2) m4[(e >> 1) & 3] = at_max3(m4[(e >> 1) & 3], __uint_as_float(sr[e]), __uint_as_float(sr[e + 1]));
           mx = at_max3(m4[0], m4[1], fmaxf(m4[2], m4[3]));
+          if (CAP && !masked) {
+            float a4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int e = 0; e < AT_C; e += 2)
+              a4[(e >> 1) & 3] = at_max3(a4[(e >> 1) & 3], fabsf(__uint_as_float(sr[e])), fabsf(__uint_as_float(sr[e + 1])));
+            poly = __all_sync(0xffffffffu, at_max3(a4[0], a4[1], fmaxf(a4[2], a4[3])) * mul < AT_TANH_SMALL);
+          }
           if (mx != -INFINITY) {                                              // the row's largest score in units of log2
             mx *= mul;
             if (CAP) mx = cap2 * (1.f - 2.f * at_rcp(1.f + at_exp2(mx * (2.f * AT_LOG2E))));
@@ -527,12 +537,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
           }
         } else {
-          // tanh by its polynomial, looking on the way at how large the squares are; where some row's are too large the raw scores, taken from
-          // tensor memory again, go through the exponential form.  (A NaN is passed over; NaN * P(NaN) stays NaN.)
+          // tanh by its polynomial while all scores are small.  Of bounded ones that is seen on the way: where some row's are too large the raw scores,
+          // taken from tensor memory again, go through the exponential form.  (A NaN is passed over; NaN * P(NaN) stays NaN.)
           const float m3 = mul * mul * mul, c0p = cap2 * AT_T0 * mul, c1p = cap2 * AT_T1 * m3, c2p = cap2 * AT_T2 * (m3 * mul * mul);
           const f2 p0c = f2_of(c0p, c0p), p1c = f2_of(c1p, c1p), p2c = f2_of(c2p, c2p);
           float u4[4] = {0.f, 0.f, 0.f, 0.f};
-          if (bounded || !masked) {
+          if (poly) {
 #pragma unroll
             for (int e = 0; e < AT_C; e += 2) {
               const f2 x = f2_of(__uint_as_float(sr[e]), __uint_as_float(sr[e + 1])), u = f2_mul(x, x);
@@ -540,23 +550,31 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
               float a0, a1, u0, u1;
               f2_split(a, a0, a1);
               f2_split(u, u0, u1);
-              u4[(e >> 1) & 3] = at_max3(u4[(e >> 1) & 3], u0, u1);
+              if (bounded) u4[(e >> 1) & 3] = at_max3(u4[(e >> 1) & 3], u0, u1);
               sr[e] = __float_as_uint(a0), sr[e + 1] = __float_as_uint(a1);
             }
           }
-          if (!(bounded || !masked) || !__all_sync(0xffffffffu, at_max3(u4[0], u4[1], fmaxf(u4[2], u4[3])) * (mul * mul) < AT_TANH_SMALL * AT_TANH_SMALL)) {
-            const float k2 = mul * (2.f * AT_LOG2E), top = cap2 + sub, two = -2.f * cap2;
-            tmem_ld32_async(ts + (uint32_t)(AT_C * half), sr);
-            tmem_wait_ld();
-            tie32(sr);
+          if (bounded) {
+            poly = __all_sync(0xffffffffu, at_max3(u4[0], u4[1], fmaxf(u4[2], u4[3])) * (mul * mul) < AT_TANH_SMALL * AT_TANH_SMALL);
+            if (!poly) {
+              tmem_ld32_async(ts + (uint32_t)(AT_C * half), sr);
+              tmem_wait_ld();
+              tie32(sr);
+              if (BIAS) {
 #pragma unroll
-            for (int e = 0; e < AT_C; ++e) {
-              float x = __uint_as_float(sr[e]);
-              if (BIAS) x = fmaf(slope, (float)(c0 + e - qp), x * (p.scale * bias_unit));
-              sr[e] = __float_as_uint(fmaf(two, at_rcp(1.f + at_exp2(x * k2)), top));
+                for (int e = 0; e < AT_C; ++e) sr[e] = __float_as_uint(fmaf(slope, (float)(c0 + e - qp), __uint_as_float(sr[e]) * (p.scale * bias_unit)));
+              }
             }
           }
-          if (masked) {
+          if (!poly) {
+            const float k2 = mul * (2.f * AT_LOG2E), top = cap2 + sub, two = -2.f * cap2;
+#pragma unroll
+            for (int e = 0; e < AT_C; ++e) {
+              const float a = fmaf(two, at_rcp(1.f + at_exp2(__uint_as_float(sr[e]) * k2)), top);
+              sr[e] = __float_as_uint(!bounded && masked && (e < cmin || e > cmax) ? -INFINITY : a);
+            }
+          }
+          if (bounded && masked) {
 #pragma unroll
             for (int e = 0; e < AT_C; ++e)
               if (e < cmin || e > cmax) sr[e] = __float_as_uint(-INFINITY);
@@ -675,7 +693,7 @@ bool at_operand_ok(const AttnTcOperand& o) {
          o.row % 8 == 0 && o.batch % 8 == 0;
 }
 
-template <int NB1, int NB2, int NBV, int TERMS, bool CAP, bool BIAS>
+template <int NB1, int NB2, int NBV, int TERMS, AtCap CAP, bool BIAS>
 int at_launch(const AttnTcArgs& a, const AtParams& p, cudaStream_t st) {
   constexpr int smem = AtShape<NB1, NB2, NBV>::SMEM;
   static_assert(smem <= 227 * 1024, "shared memory of a block");
@@ -707,17 +725,20 @@ bool attn_tc_supported(const AttnTcArgs& a) {
          a.y_ld % 8 == 0 && ((uintptr_t)a.y & 15) == 0 && (a.terms == 1 || a.terms == 2);
 }
 
-// Which tiles a block takes.  Queries that see all keys before them have very unequal walks: of neighbours the last two walk everything while the
-// first two are done at once, and with fewer blocks than SMs nothing evens that out; one tile from the end and one from the start make all
-// blocks alike (2048 queries, 16 heads of 128: 50 us -> 40, capped 57 -> 45; 32 heads 84 -> 74).  Tiles that a window keeps alike stay
-// neighbours, which share most of their keys (window 700 of 2048: 30.3, apart 31.3; chunks of 512: 21.7, apart 24.7; a window of half of the
-// queries is even at 33, one of 1500 of 1736 42 -> 40 apart).
-// With no more tiles than SMs a block takes one (us, two a block / one: 32 heads, 300 and 512 queries 15.4 / 13.6, 18.6 / 16.3; 16 heads, 130, 512, 1024,
-// 1152 queries 13.3 / 11.0, 17.8 / 14.4, 24.4 / 21.8, 26.8 / 23.7, with a window of 200 of 1024 19.7 / 14.8; 8 heads, 2048 queries 37.8 / 35.1).
+// Which tiles a block takes.  With no more tiles than SMs one (us, two a block / one: 32 heads, 300 and 512 queries 15.4 / 13.6, 18.6 / 16.3; 16 heads, 130,
+// 512, 1024, 1152 queries 13.3 / 11.0, 17.8 / 14.4, 24.4 / 21.8, 26.8 / 23.7, with a window of 200 of 1024 19.7 / 14.8; 8 heads, 2048 queries 37.8 / 35.1).
+// Two neighbours share most of their keys, and with blocks for several rounds of the SMs the long ones, which come first, even out by themselves.  Queries
+// that see all keys before them have very unequal walks, though: while the blocks fit the SMs at once, or their second round is more than half full, one tile
+// from the end and one from the start make all blocks alike.  neighbours / apart, of heads of 128, by tiles and blocks per SM: 4, 8, 16, 32 tiles at up to
+// one 1.10, 1.21, 1.27, 1.28, three 0.90; eight to 64 tiles at 1.08 and 1.3 0.81 - 1.01, at 1.5 - 2 1.02 - 1.15, at 2.2 - 3 0.91 - 1.06, at 3.5 - 7
+// 0.87 - 1.00.  Under a window of two thirds, a half and a third of the queries at up to one 1.05 - 1.20 (three tiles 0.87), 0.99 - 1.11, 0.81 - 1.05, at 1.7
+// 0.98 - 1.12, 0.94 - 1.07, 0.78 - 1.01.  Chunks stay neighbours (512 of 2048: 21.7, apart 24.7 us).
 int at_tiles(const AttnTcArgs& a) {
-  const int sms = sm_count();
-  if ((long long)((a.T + AT_Q - 1) / AT_Q) * a.H * a.B <= (sms > 0 ? sms : 148)) return AT_ALONE;
-  return a.chunk <= 0 && (a.window <= 0 || 2ll * a.window >= a.T) ? AT_APART : AT_NEIGHBOURS;
+  const long long tiles = (a.T + AT_Q - 1) / AT_Q, blocks = (tiles + 1) / 2 * a.H * a.B, sms = sm_count() > 0 ? sm_count() : 148;
+  if (tiles * a.H * a.B <= sms) return AT_ALONE;
+  if (a.chunk > 0 || tiles < 4) return AT_NEIGHBOURS;
+  if (blocks <= sms) return a.window <= 0 || 2ll * a.window >= a.T ? AT_APART : AT_NEIGHBOURS;
+  return 2 * blocks >= 3 * sms && blocks <= 2 * sms && (a.window <= 0 || a.window >= a.T) ? AT_APART : AT_NEIGHBOURS;
 }
 
 enum AttnTcKind { AT_ROTARY, AT_LATENT };     // which forms a file instantiates
@@ -728,14 +749,16 @@ int attn_tc_launch(const AttnTcArgs& a, cudaStream_t st) {
                    a.v.dim, a.window, a.chunk, a.ring, a.gate_ld, a.gate_per_head,
                    a.gate_ld % 8 == 0 && ((uintptr_t)a.gate & 15) == 0, a.y_ld, at_tiles(a), wait_word()};
   const int nb = (a.q.dim + 63) / 64, nbv = (a.v.dim + 63) / 64;
-  const bool cap = a.softcap > 0.f, bias = a.slopes != nullptr, two = a.q2.base != nullptr;
+  const AtCap cap = a.softcap <= 0.f ? AT_UNCAPPED : a.softcap * AT_LOG2E <= AT_BOUND ? AT_BOUNDED : AT_CAPPED;
+  const bool bias = a.slopes != nullptr, two = a.q2.base != nullptr;
 #define LL_AT(N1, N2, NV, TERMS, CC, BB) \
   if (nb == N1 && two == (N2 > 0) && nbv == NV && a.terms == TERMS && cap == CC && bias == BB) return at_launch<N1, N2, NV, TERMS, CC, BB>(a, p, st);
 #define LL_AT_SIZES(N2, TERMS, CC, BB) LL_AT(1, N2, 1, TERMS, CC, BB) LL_AT(1, N2, 2, TERMS, CC, BB) LL_AT(2, N2, 1, TERMS, CC, BB) LL_AT(2, N2, 2, TERMS, CC, BB)
   if constexpr (KIND == AT_ROTARY) {
-    LL_AT_SIZES(0, 2, false, false) LL_AT_SIZES(0, 2, true, false) LL_AT_SIZES(0, 2, false, true) LL_AT_SIZES(0, 2, true, true)
+    LL_AT_SIZES(0, 2, AT_UNCAPPED, false) LL_AT_SIZES(0, 2, AT_BOUNDED, false) LL_AT_SIZES(0, 2, AT_CAPPED, false)
+    LL_AT_SIZES(0, 2, AT_UNCAPPED, true) LL_AT_SIZES(0, 2, AT_BOUNDED, true) LL_AT_SIZES(0, 2, AT_CAPPED, true)
   } else {
-    LL_AT_SIZES(1, 1, false, false) LL_AT_SIZES(1, 2, false, false)
+    LL_AT_SIZES(1, 1, AT_UNCAPPED, false) LL_AT_SIZES(1, 2, AT_UNCAPPED, false)
   }
 #undef LL_AT_SIZES
 #undef LL_AT
