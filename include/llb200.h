@@ -808,7 +808,8 @@ LL_API int ll_softmax_attn_rows(const void* q, int q_stride, const void* gate, i
  * Latent: w_uk [heads][nope][kv_rank], w_uv_t [heads][kv_rank][v_dim]; columns of the projection: queries first, gate_col0 (one logit a head;
  * < 0: none), kv_col0; kv_norm NULL: the cache is another layer's and already holds the rows.  Softmax (one score map, queries and keys that
  * turn or are normed): columns of queries, keys, values (< 0: the un-rotated keys) and gate (< 0: none).  Widths, ranks and value sizes in
- * multiples of 8, kv_rank and nope up to 1024; scratch of the given bytes, any contents, 256-byte aligned.  Other sizes: LL_ERR_UNSUPPORTED. */
+ * multiples of 8, kv_rank and nope up to 1024; scratch of the given bytes, any contents, 256-byte aligned.  Other sizes: LL_ERR_UNSUPPORTED.
+ * The calls for one token are the layers' below with T = 1. */
 LL_API size_t ll_latent_step_scratch_bytes(int B, int n_in, int heads, int kv_rank, int v_dim, int splits);
 LL_API int ll_latent_step(const void* x, const void* w_in, int n_in, const void* w_uk, const void* w_uv_t, const void* w_o, const float* kv_norm,
                           float eps, const float* rope, const int32_t* pos_ids, void* cache, int B, int width, int heads, int nope, int rot_dim,
@@ -827,8 +828,8 @@ LL_API int ll_softmax_step(const void* x, const void* w_in, int n_in, const void
                            const float* q_norm, const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc,
                            void* vc, const float* sink, const float* slopes, float scale, float softcap, int B, int width, int H, int G, int dim,
                            int vdim, int window, int chunk, int ring, int splits, int form, void* out, void* scratch, ll_stream stream);
-/* The same layer for B sequences of T tokens each, any number of rows (x [B * T][width] bf16): projections of more than two rows by
- * ll_dense_rows.  Scratch: ll_softmax_step_scratch_bytes of B * T rows. */
+/* The same layer for B sequences of T tokens each, any number of rows (x [B * T][width] bf16): projections of 3 to 16 rows, and to 32
+ * of up to 4096 columns, in blocks of 16 weight rows (ll_rows_linear), of more by ll_dense_rows.  Scratch: ll_softmax_step_scratch_bytes of B * T rows. */
 LL_API int ll_softmax_layer(const void* x, const void* w_in, int n_in, const void* w_o, int q_col, int k_col, int v_col, int gate_col, const float* q_norm,
                             const float* k_norm, float eps, const float* freq, int rot_dims, const int32_t* pos_ids, void* kc, void* vc, const float* sink,
                             const float* slopes, float scale, float softcap, int B, int T, int width, int H, int G, int dim, int vdim, int window,

@@ -19,7 +19,7 @@ struct SpParams {
   int* word;
 };
 constexpr int SP_PITCH = 132;      // floats from one token's sums to the next: a quarter's rows and four pairs of tokens fall on 32 banks
-constexpr int SP_ROWS = MT_STAGES * (MT_A_BYTES + MT_B_BYTES) / (SP_PITCH * 4);      // tokens that fit the ring's place
+static_assert(MT_NMAX * SP_PITCH * 4 <= MT_STAGES * (MT_A_BYTES + MT_B_BYTES), "a tile's sums in the ring's place (two pairs a tile)");
 
 // 32 lanes x 32 columns to the same place of another CTA's shared memory: v[c] of lane l at (c * SP_PITCH + l) floats
 __device__ __forceinline__ void sp_store(uint32_t at, const uint32_t (&v)[32]) {
@@ -225,7 +225,7 @@ int dense_rows(const void* x, long long ldx, const void* w, int head_cols, void*
     for (int sp = 1; sp <= 2; ++sp) {
       // (clusters of four CTAs: an eighth of the pairs is left for what does not fit a GPC.  Four pairs a tile: clusters of eight ran in two waves,
       // 2048 x 2048 with 64 rows 13.0 where two pairs take 8.8 and one 10.3)
-      if (sp > 1 && ((long long)wt * c * sp > pairs - pairs / 8 || nkb < 8 || step > SP_ROWS)) continue;
+      if (sp > 1 && ((long long)wt * c * sp > pairs - pairs / 8 || nkb < 8)) continue;
       const long long rounds = ((long long)wt * c + pairs - 1) / pairs, cost = rounds * (256 + step) * ((nkb + sp - 1) / sp) + (sp > 1 ? 2000 + 16 * step : 0);
       if (best < 0 || cost < best) best = cost, cuts = c, split = sp;
     }

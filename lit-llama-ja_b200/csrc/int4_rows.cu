@@ -11,7 +11,8 @@
 // ptxas spills three registers, stored and loaded once each).
 // us, one CTA a tile / pairs: 11008 x 4096 at 150, 512, 1100 rows 28 / 24, 51 / 46, 82 / 69; 4096 x 11008 at 150, 512 rows 53 / 48, 87 / 54;
 // 32000 x 4096 at 512 rows 140 / 103.  Bound by products at 256 rows a tile (0.84 us a step with all SMs busy, 0.76 at the rate of a large
-// dense product), below that by unpacking.
+// dense product), below that by unpacking.  Counters, 512 rows of the gated 11008 x 4096 and of 4096 x 11008 cut along k: tensor pipe 53 and 46 % of the
+// time, issue slots 36 and 33, L2 16, HBM 8 and 9.
 //   warps 0, 2 : TMA producers: 128 k of bn / 2 rows of x; 64 x 128 packed bytes
 //   warp 1     : in the CTA of rank 0, one thread issues 256 x bn x 16 MMAs (A from tensor memory) for both
 //   warp 3     : scales and zeros, several steps ahead
@@ -451,7 +452,8 @@ long long r4_cost(int M, int N, int tile_n, int steps, int bn, int pairs) {
 // us on the device, every tile whole / by this rule: 4096 x 11008 at 130, 300, 512 rows 48 / 24, 50 / 34, 50 / 43, from 700 on all whole (53; in the
 // parts nearest to paying 58); the gated 11008 x 4096 at 130, 300, 512, 700 rows 45 / 37, 63 / 56, 80 / 74, 109 / 106.  Short layers (R4_SHORT) stay
 // whole: 2048 x 5632 of 130 rows would take 15 instead of 27, but calls of its size are bound by the host, for which a second launch and its scratch
-// are 2 us (228 rows through a feed-forward of width 2048, a call 49 whole, 51 cut).  Ranges of one length for all pairs, that cross tile ends, were
+// are 2 us (228 rows through a feed-forward of width 2048, a call 49 whole, 51 cut).  The rule goes by sizes alone: such a layer stays whole in a captured
+// step as well, where no host is in the way.  Ranges of one length for all pairs, that cross tile ends, were
 // 2 to 4 us slower (two drains a pair, more parts); the last pair to arrive adding up in the kernel itself made the loop spill (whole tiles a fifth
 // slower).
 constexpr long long R4_SHORT = 40000;

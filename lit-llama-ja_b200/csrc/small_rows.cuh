@@ -1,6 +1,7 @@
-// Products of a few rows (decoding: one or two) with bf16 weights that are read once, on CUDA cores: bound by the weights' way from memory, so what
-// counts is 16-byte loads in flight.  Two forms: weights [N][K] (a warp per output row), and weights [K][N] per head (partial sums over
-// k in a block).  Both start under the kernel before them and wait for it before they read anything.
+// Products of a few rows with bf16 weights that are read once: bound by the weights' way from memory, so what counts is 16-byte loads in flight.  Three
+// forms: one or two rows with weights [N][K] on CUDA cores (a warp per output row), 3 to 32 rows with the same weights on mma.sync (few_rows_kernel), and
+// weights [K][N] per head on CUDA cores (partial sums over k in a block, four rows at most).  All start under the kernel before them and wait for it before
+// they read what it makes; few_rows_kernel reads weights before that wait where its caller knows whoever wrote them to have ended (early).
 // The first form takes one or two rows only: every weight meets every row's sums in registers, and from three rows on the conversions cost more than the loads.  Both
 // projections of an attention layer, us, here / the library's products: one row of width 2048 12.7 / 12.7, of 4096 21.7 / 27.3; four rows (when
 // this form still took them) 21.4 / 11.4 and 51.9 / 27.1.  Two rows of w a warp halve the warps in flight: 8.4 for the first projection against 5.5.

@@ -219,7 +219,7 @@ class LatentAttention(nn.Module):
 
     def _takes_step(self, x_act: torch.Tensor, B: int, cache: torch.Tensor):
         """One token of one or two sequences."""
-        return self._takes_layer(x_act, B, cache, "ll_latent_step") if 1 <= B <= STEP_MAX_ROWS else None
+        return self._takes_layer(x_act, B, cache, "ll_latent_layer") if 1 <= B <= STEP_MAX_ROWS else None
 
     def _layer_form(self, B: int, T: int, cache: torch.Tensor, splits: int, end: Optional[int]) -> Optional[int]:
         """Cache rows per sequence that a call of several rows expands per head, 0: queries stay in latent space; ``None``: not in one call.  The form is

@@ -55,9 +55,8 @@ def pad8(n: int) -> int:
 # memory, one token over 100, 1000 and 4000 keys in ranges of 64: width 1024 34 / 26 (70 / 36), 36 / 29 (56 / 35), 56 / 52 (67 / 55); 2048
 # 38 / 31 (50 / 35), 42 / 35 (56 / 40), 60 / 53 (72 / 58); 4096 55 / 45 (63 / 50), 58 / 49 (71 / 56), 77 / 62 (87 / 68).  Two sequences 33 / 27 to
 # 55 / 53, 37 / 32 to 59 / 57, 55 / 50 to 80 / 71; with 32 key heads of width 4096 62 / 61 (69 / 65) to 90 / 93 (99 / 100).
-# From three sequences on the library's products are the faster ones (csrc/small_rows.cuh), so larger batches keep the separate calls.
 STEP_MAX_ROWS = 2
-# Rows times weights of a layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 1024 rows 53 / 28,
+# More rows: rows times weights of a layer that runs in one call (_native.layer_rows).  us a call, separate / one: width 1024, 17, 400 and 1024 rows 53 / 28,
 # 54 / 42, 54 / 50; 2048, 17, 120 and 400 rows 54 / 33, 55 / 44, 53 / 54; 4096, 17 and 60 rows 56 / 60, 62 / 66 (so not there).  A few rows, replayed as
 # a graph: one token of three sequences over 100 keys, widths 1024 and 2048: 29 / 24, 32 / 29.
 LAYER_MAX_PRODUCTS = 4 << 30
@@ -234,7 +233,7 @@ class SoftmaxAttention(nn.Module):
 
     def _takes_step(self, u: torch.Tensor, B: int, caches):
         """One token of one or two sequences."""
-        return self._takes_layer(u, B, caches, "ll_softmax_step") if 1 <= B <= STEP_MAX_ROWS else None
+        return self._takes_layer(u, B, caches, "ll_softmax_layer") if 1 <= B <= STEP_MAX_ROWS else None
 
     def _takes_layer(self, u: torch.Tensor, M: int, caches, entry: str):
         """``M`` bf16 rows on a layer with its own ring, one score map, no short convolution and nothing prepared head by head: the whole layer in
